@@ -1,11 +1,14 @@
-"""ctypes binding of libegs_b200.so (the C-ABI library declared in include/egs_b200.h).
+"""Loads the native libraries: libegs_b200.so (the C ABI declared in include/egs_b200.h, bound with ctypes) and
+_egs_host.so (the host path built on it, an extension module).
 
-There is no CPU fallback: if the library cannot be loaded (and cannot be built because nvcc is absent)
+There is no CPU fallback: if a library cannot be loaded (and cannot be built because the compilers are absent)
 importing the operators raises.
 """
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import threading
 
@@ -27,6 +30,7 @@ EXPORTS = (
     "egs_gather_scatter_pair", "egs_fused_pair_eligible", "egs_dweight_prezeroed", "egs_selftest_wait_timeout",
     "egs_describe_plan", "egs_gather_gemm_bias", "egs_gemm_scatter_bias", "egs_route_topk", "egs_index_csr",
     "egs_index_csr_scratch_bytes", "egs_index_compact", "egs_gemm_scatter_prepared", "egs_gemm_scatter_csr",
+    "egs_set_status_mirror",
 )
 
 
@@ -39,8 +43,9 @@ class PlanInfo(ctypes.Structure):
                                             "expert_fastest", "splits", "rows_per_split")]
 
 
-_lock = threading.Lock()
+_lock = threading.RLock()
 _lib = None
+_host = None
 
 
 def _declare(lib: ctypes.CDLL) -> None:
@@ -89,6 +94,8 @@ def _declare(lib: ctypes.CDLL) -> None:
     lib.egs_gemm_scatter_csr.argtypes = [vp, vp, vp, vp, vp, vp, ctypes.POINTER(Dims), i, i, i, vp]
     lib.egs_describe_plan.restype = i
     lib.egs_describe_plan.argtypes = [i, ctypes.POINTER(Dims), i, i, i, ctypes.POINTER(PlanInfo)]
+    lib.egs_set_status_mirror.restype = i
+    lib.egs_set_status_mirror.argtypes = [vp, vp]
     lib.egs_fill_zero.restype = i
     lib.egs_fill_zero.argtypes = [vp, sz, vp]
     lib.egs_launch_count.restype = i64
@@ -103,28 +110,49 @@ def library_path() -> str:
     return os.environ.get("EGS_B200_LIBRARY", _build.LIB_PATH)
 
 
+def _up_to_date(path: str, stale: bool) -> None:
+    """Builds ``path`` when it is missing or older than its sources; an old library stands in where nothing can be built."""
+    if stale:
+        try:
+            _build.build()
+        except Exception as exc:  # a compiler is absent, or a compile error
+            if not os.path.exists(path):
+                raise RuntimeError(f"{os.path.basename(path)} is not built and could not be built here ({exc}); run "
+                                   "`python -m expertscattergather_b200.build` where nvcc and g++ are available") from exc
+    if not os.path.exists(path):
+        raise RuntimeError(f"{os.path.basename(path)} not found at {path}")
+
+
 def load() -> ctypes.CDLL:
-    """Loads (building first when the sources are newer and nvcc is present) and returns the library."""
+    """Loads (building first when the sources are newer and nvcc is present) and returns the C-ABI library."""
     global _lib
-    with _lock:
-        if _lib is not None:
-            return _lib
-        path = library_path()
-        if path == _build.LIB_PATH:
-            try:
-                if _build.needs_build():
-                    _build.build()
-            except Exception as exc:  # nvcc absent or compile error
-                if not os.path.exists(path):
-                    raise RuntimeError(
-                        "libegs_b200.so is not built and could not be built here "
-                        f"({exc}); run `python -m expertscattergather_b200.build` where nvcc is available") from exc
-        if not os.path.exists(path):
-            raise RuntimeError(f"libegs_b200.so not found at {path}")
-        lib = ctypes.CDLL(path)
-        _declare(lib)
-        _lib = lib
-        return lib
+    if _lib is None:
+        with _lock:
+            if _lib is None:
+                path = library_path()
+                _up_to_date(path, path == _build.LIB_PATH and _build.needs_build())
+                lib = ctypes.CDLL(path)
+                _declare(lib)
+                _lib = lib
+    return _lib
+
+
+def host():
+    """Loads (building first when needed) and returns the native host module, bound to the library of :func:`load`."""
+    global _host
+    if _host is None:
+        with _lock:
+            if _host is None:
+                load()
+                import torch  # noqa: F401  (the module's own dependencies)
+                path = _build.HOST_PATH
+                _up_to_date(path, _build.host_needs_build())
+                loader = importlib.machinery.ExtensionFileLoader("_egs_host", path)
+                module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_egs_host", path, loader=loader))
+                loader.exec_module(module)
+                module.init(library_path())
+                _host = module
+    return _host
 
 
 def check(code: int, what: str) -> None:

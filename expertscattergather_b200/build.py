@@ -1,23 +1,29 @@
-"""Builds libegs_b200.so (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Builds the two native libraries in-tree: libegs_b200.so (kernels behind the C ABI, nvcc for sm_100a) and _egs_host.so (the
+host path: operators, autograd functions and the training step over that ABI, g++ against the installed torch).
 
     python -m expertscattergather_b200.build [--force] [--verbose]
 
-The library is written to ``expertscattergather_b200/_lib/libegs_b200.so``.  It is rebuilt when a source
-file is newer than the library.  nvcc cross-compiles without a GPU.
+Both are written to ``expertscattergather_b200/_lib/`` and rebuilt when a source file is newer.  No GPU is needed.
 """
 from __future__ import annotations
 
+import concurrent.futures
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 OUT_DIR = os.path.join(PKG, "_lib")
+OBJ_DIR = os.path.join(OUT_DIR, "obj")
 LIB_PATH = os.path.join(OUT_DIR, "libegs_b200.so")
+HOST_PATH = os.path.join(OUT_DIR, "_egs_host.so")
 SOURCES = ["egs_api.cu", "egs_generic.cu", "egs_tensor.cu", "egs_pair16.cu", "egs_gather2.cu", "egs_index.cu"]
-HEADERS = [os.path.join(CSRC, "egs_internal.cuh"), os.path.join(CSRC, "egs_tcgen05.cuh"), os.path.join(PKG, "..", "include", "egs_b200.h")]
+HOST_SOURCE = os.path.join(CSRC, "egs_host.cpp")
+API_HEADER = os.path.join(PKG, "..", "include", "egs_b200.h")
+HEADERS = [os.path.join(CSRC, "egs_internal.cuh"), os.path.join(CSRC, "egs_tcgen05.cuh"), API_HEADER]
 
 
 def _nvcc() -> str:
@@ -27,28 +33,65 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found (set NVCC or put it on PATH)")
 
 
+def _newer(target: str, deps) -> bool:
+    return not os.path.exists(target) or any(os.path.getmtime(d) > os.path.getmtime(target) for d in deps)
+
+
 def needs_build() -> bool:
-    if not os.path.exists(LIB_PATH):
-        return True
-    t = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(CSRC, s) for s in SOURCES] + HEADERS
-    return any(os.path.getmtime(d) > t for d in deps)
+    return _newer(LIB_PATH, [os.path.join(CSRC, s) for s in SOURCES] + HEADERS)
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and not needs_build():
-        return LIB_PATH
-    os.makedirs(OUT_DIR, exist_ok=True)
-    cmd = [_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
-           "-shared", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2"]
-    if verbose:
-        cmd += ["-Xptxas", "-v"]
-    cmd += [os.path.join(CSRC, s) for s in SOURCES] + ["-o", LIB_PATH, "-lcudart"]
+def host_needs_build() -> bool:
+    return _newer(HOST_PATH, [HOST_SOURCE, API_HEADER])
+
+
+def _run(cmd, verbose: bool) -> None:
     res = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or res.returncode != 0:
         sys.stderr.write(res.stdout + res.stderr)
     if res.returncode != 0:
-        raise RuntimeError("nvcc failed building libegs_b200.so")
+        raise RuntimeError(f"{os.path.basename(cmd[0])} failed building {cmd[cmd.index('-o') + 1]}")
+
+
+def _build_kernels(force: bool, verbose: bool) -> None:
+    os.makedirs(OBJ_DIR, exist_ok=True)
+    flags = [_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
+             "-Xcompiler", "-O2"] + (["-Xptxas", "-v"] if verbose else [])
+    objs, jobs = [], []
+    with concurrent.futures.ThreadPoolExecutor(max_workers=len(SOURCES)) as pool:
+        for s in SOURCES:
+            src, obj = os.path.join(CSRC, s), os.path.join(OBJ_DIR, s + ".o")
+            objs.append(obj)
+            if force or _newer(obj, [src] + HEADERS):
+                jobs.append(pool.submit(_run, flags + ["-c", src, "-o", obj], verbose))
+        for j in jobs:
+            j.result()
+    _run(flags + ["-shared"] + objs + ["-o", LIB_PATH, "-lcudart"], False)
+
+
+def _build_host(verbose: bool) -> None:
+    import torch
+    from torch.utils import cpp_extension
+    os.makedirs(OUT_DIR, exist_ok=True)
+    cuda_home = os.path.dirname(os.path.dirname(_nvcc()))
+    incs = cpp_extension.include_paths() + [os.path.join(cuda_home, "include"), sysconfig.get_paths()["include"]]
+    lib_dirs = cpp_extension.library_paths() + [os.path.join(cuda_home, "lib64")]
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           "-DTORCH_EXTENSION_NAME=_egs_host", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
+    cmd += [f for d in incs for f in ("-isystem", d)] + [HOST_SOURCE, "-o", HOST_PATH]
+    cmd += [f"-L{d}" for d in lib_dirs] + [f"-Wl,-rpath,{d}" for d in lib_dirs[:1]]
+    cmd += ["-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lcudart", "-ldl"]
+    _run(cmd, verbose)
+
+
+def build(force: bool = False, verbose: bool = False) -> str:
+    """Builds what is out of date; returns the path of the kernel library."""
+    kernels, host = force or needs_build(), force or host_needs_build()
+    with concurrent.futures.ThreadPoolExecutor(max_workers=2) as pool:
+        jobs = ([pool.submit(_build_kernels, force, verbose)] if kernels else []) + ([pool.submit(_build_host, verbose)] if host else [])
+        for j in jobs:
+            j.result()
     return LIB_PATH
 
 

@@ -3,6 +3,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 
 #include <cuda.h>   // types of the driver API only (CUtensorMap); the entry point is looked up at run time, libcuda is not linked
 
@@ -39,6 +40,22 @@ static std::atomic<long long> g_launches{0};
 static thread_local char g_cuda_error[256] = "";
 
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
+
+// Registered (status word, host mirror) pairs: written under the lock, read without it.
+static constexpr int kMaxMirrors = 64;
+static std::mutex g_mirror_mutex;
+static std::atomic<int32_t*> g_mirror_word[kMaxMirrors];
+static std::atomic<int32_t*> g_mirror_host[kMaxMirrors];
+
+StatusRef status_ref(int32_t* status_word) {
+  if (status_word)
+    for (int i = 0; i < kMaxMirrors; ++i) {
+      int32_t* w = g_mirror_word[i].load(std::memory_order_acquire);
+      if (w == status_word) return {status_word, g_mirror_host[i].load(std::memory_order_relaxed)};
+      if (!w) break;
+    }
+  return {status_word, nullptr};
+}
 
 namespace {
 
@@ -171,7 +188,7 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
   }
 
   RowGemmParams p{};
-  p.A = A; p.W = W; p.bias = bias; p.Ind = Ind; p.Out = Out; p.acc = acc; p.plan = plan; p.status = status;
+  p.A = A; p.W = W; p.bias = bias; p.Ind = Ind; p.Out = Out; p.acc = acc; p.plan = plan; p.status = status_ref(status);
   p.B = static_cast<int>(d.B); p.T = static_cast<int>(d.T); p.E = static_cast<int>(d.E); p.K = static_cast<int>(d.K);
   p.C = static_cast<int>(d.C); p.N = static_cast<int>(d.N);
   p.M = static_cast<int>(d.B * d.K);
@@ -219,6 +236,19 @@ const char* egs_status_string(int code) {
 const char* egs_last_cuda_error(void) { return g_cuda_error; }
 
 int64_t egs_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
+
+int egs_set_status_mirror(int32_t* status_word, int32_t* host_mirror) {
+  if (!status_word) return EGS_ERR_INVALID_ARGUMENT;
+  std::lock_guard<std::mutex> lock(g_mirror_mutex);
+  for (int i = 0; i < kMaxMirrors; ++i) {
+    int32_t* w = g_mirror_word[i].load(std::memory_order_relaxed);
+    if (w && w != status_word) continue;
+    g_mirror_host[i].store(host_mirror, std::memory_order_relaxed);
+    g_mirror_word[i].store(status_word, std::memory_order_release);
+    return EGS_OK;
+  }
+  return EGS_ERR_TOO_LARGE;
+}
 
 int egs_gather_gemm(const void* X, const void* W, const void* Ind, void* Y, const egs_dims* dims, int w_layout,
                     int dtype, int index_dtype, int precision, int path, int32_t* status_word, void* cuda_stream) {
@@ -348,7 +378,7 @@ int egs_gather_scatter_pair(const void* Src, const void* W1, const void* W2, con
   if (!no_work && (!aligned16(Src) || !aligned16(W1) || !aligned16(W2) || !aligned16(Mid) || !aligned16(Dst)))
     return EGS_ERR_UNSUPPORTED;
   FusedParams p{};
-  p.Src = Src; p.W1 = W1; p.W2 = W2; p.Ind = Ind; p.Mid = Mid; p.status = status_word;
+  p.Src = Src; p.W1 = W1; p.W2 = W2; p.Ind = Ind; p.Mid = Mid; p.status = status_ref(status_word);
   p.B = static_cast<int>(B); p.T = static_cast<int>(T); p.E = static_cast<int>(E); p.K = static_cast<int>(K);
   p.C1 = static_cast<int>(C1); p.N1 = static_cast<int>(N1); p.N2 = static_cast<int>(N2);
   p.M = static_cast<int>(B * K);
@@ -441,7 +471,7 @@ static int dweight_impl(const void* Xsrc, const void* Ysrc, const void* Ind, voi
   if (!Xsrc || !Ysrc || !Ind) return EGS_ERR_INVALID_ARGUMENT;
 
   DWeightParams p{};
-  p.Xsrc = Xsrc; p.Ysrc = Ysrc; p.Ind = Ind; p.out = out; p.status = status_word;
+  p.Xsrc = Xsrc; p.Ysrc = Ysrc; p.Ind = Ind; p.out = out; p.status = status_ref(status_word);
   p.B = static_cast<int>(B); p.T = static_cast<int>(T); p.E = static_cast<int>(E); p.K = static_cast<int>(K);
   p.FG = static_cast<int>(FG); p.FD = static_cast<int>(FD);
   p.M = static_cast<int>(B * K);

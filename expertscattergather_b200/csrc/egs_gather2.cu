@@ -179,10 +179,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kG2Threads, 1) tenso
     }
     mbar_init(smem_u32(&hdr->drain), 1);
     fence_mbar_init();
-    hdr->abort_flag = (p.status && (*reinterpret_cast<volatile int32_t*>(p.status) & EGS_STATUS_PIPELINE_TIMEOUT)) ? 1u : 0u;
+    hdr->abort_flag = p.status.timed_out() ? 1u : 0u;
     if (smem_misaligned(smem_raw)) {
       hdr->abort_flag = 1u;
-      if (p.status) atomicOr(p.status, EGS_STATUS_INTERNAL);
+      p.status.report(EGS_STATUS_INTERNAL);
     }
   }
   __syncthreads();
@@ -215,7 +215,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kG2Threads, 1) tenso
       tiles.locate(t, e, rb);
       // this thread's token rows, looked up by the index warp while the previous tile was loading
       const uint32_t rbuf = tcnt & 1u;
-      alive = mbar_wait_warp(smem_u32(&hdr->rows_full[rbuf]), (tcnt >> 1) & 1, abort_flag, p.status, lane);
+      alive = mbar_wait_warp(smem_u32(&hdr->rows_full[rbuf]), (tcnt >> 1) & 1, abort_flag, p.status.word, lane);
       if (!alive) break;
       bool all_rows = true;
 #pragma unroll
@@ -226,7 +226,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kG2Threads, 1) tenso
       mbar_arrive(smem_u32(&hdr->rows_empty[rbuf]));
       const char* a0 = A + cc * 16;
       for (int kt = 0; kt < nk && alive; ++kt) {
-        if (round > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[slot]), (round - 1) & 1, abort_flag, p.status, lane);
+        if (round > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[slot]), (round - 1) & 1, abort_flag, p.status.word, lane);
         if (!alive) break;
         const uint32_t base = ring0 + static_cast<uint32_t>(slot) * stage_bytes;
         const uint32_t bar = smem_u32(&hdr->full[slot]);
@@ -281,12 +281,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kG2Threads, 1) tenso
         // the buffer has been read out in both CTAs by the epilogue warps of the tile that used it last
         const uint32_t buf = (nbuf == 2u) ? (tcnt & 1u) : 0u;
         const uint32_t use = (nbuf == 2u) ? (tcnt >> 1) : tcnt;          // how often the buffer has been used before
-        if (use > 0) ok = mbar_wait(smem_u32(&hdr->acc_empty[buf]), (use - 1) & 1, abort_flag, p.status);
+        if (use > 0) ok = mbar_wait(smem_u32(&hdr->acc_empty[buf]), (use - 1) & 1, abort_flag, p.status.word);
         if (!ok) break;
         tc_fence_after();
         for (int ks = 0; ks < nk && ok; ++ks) {
-          ok = mbar_wait(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status);
-          if (ok) ok = mbar_wait(smem_u32(&hdr->peer_full[slot]), round & 1, abort_flag, p.status);
+          ok = mbar_wait(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status.word);
+          if (ok) ok = mbar_wait(smem_u32(&hdr->peer_full[slot]), round & 1, abort_flag, p.status.word);
           if (!ok) break;
           tc_fence_after();
           const uint32_t base = (ring0 + static_cast<uint32_t>(slot) * stage_bytes) & 0x3FFFFu;   // offset inside the CTA
@@ -326,7 +326,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kG2Threads, 1) tenso
       uint32_t round = 0;
       for (int t = pair; t < tiles.ntiles && ok; t += npairs) {
         for (int ks = 0; ks < nk && ok; ++ks) {
-          ok = mbar_wait(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status);
+          ok = mbar_wait(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status.word);
           if (!ok) break;
           fence_proxy_async_smem();
           mbar_arrive_cluster(leader_peer_full0 + static_cast<uint32_t>(slot) * 8u);
@@ -344,7 +344,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kG2Threads, 1) tenso
     uint32_t tcnt = 0;
     for (int t = pair; t < tiles.ntiles && alive; t += npairs, ++tcnt) {
       const uint32_t rbuf = tcnt & 1u, use = tcnt >> 1;
-      if (use > 0) alive = mbar_wait_warp(smem_u32(&hdr->rows_empty[rbuf]), (use - 1) & 1, abort_flag, p.status, lane);
+      if (use > 0) alive = mbar_wait_warp(smem_u32(&hdr->rows_empty[rbuf]), (use - 1) & 1, abort_flag, p.status.word, lane);
       if (!alive) break;
       int e, rb;
       tiles.locate(t, e, rb);
@@ -364,7 +364,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kG2Threads, 1) tenso
         int row = -1;
         if (base_row[i] >= 0) {
           if (tk[i] >= 0 && tk[i] < p.T) row = base_row[i] + static_cast<int>(tk[i]);
-          else if (p.status) atomicOr(p.status, EGS_STATUS_INDEX_OUT_OF_RANGE);
+          else p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
         }
         hdr->rows[rbuf][lane + 32 * i] = row;
       }
@@ -394,7 +394,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kG2Threads, 1) tenso
       const T* bias_row = p.bias ? static_cast<const T*>(p.bias) + static_cast<long long>(e) * p.N : nullptr;
       const uint32_t buf = (nbuf == 2u) ? (tcnt & 1u) : 0u;
       const uint32_t use = (nbuf == 2u) ? (tcnt >> 1) : tcnt;
-      alive = mbar_wait_warp(smem_u32(&hdr->acc_full[buf]), use & 1, abort_flag, p.status, lane);
+      alive = mbar_wait_warp(smem_u32(&hdr->acc_full[buf]), use & 1, abort_flag, p.status.word, lane);
       if (!alive) break;
       tc_fence_after();
       const uint32_t trow = tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + (buf * 2u + static_cast<uint32_t>(mt)) * acc_cols;
@@ -459,6 +459,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kG2Threads, 1) tenso
   if (warp == kG2MmaWarp && *abort_flag) {
     if (lane == 0) {
       uint32_t ignore_abort = 0u;
+      p.status.tell_host();
       umma2_commit(smem_u32(&hdr->drain));
       safe = mbar_wait(smem_u32(&hdr->drain), 0u, &ignore_abort, nullptr) ? 1u : 0u;
     }

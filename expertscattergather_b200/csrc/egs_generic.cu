@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(NTHREADS) generic_rowgemm_kernel(RowGemmParams
         ra = (SCATTER ? slot : tok) * p.C;
         ro = (SCATTER ? tok : slot) * p.N;
       } else {
-        if (p.status) atomicOr(p.status, EGS_STATUS_INDEX_OUT_OF_RANGE);
+        p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
         if (!SCATTER) ro = slot * p.N;   // gather: the row is still written (zeros)
       }
     }
@@ -155,8 +155,8 @@ __global__ void __launch_bounds__(NTHREADS) generic_dweight_kernel(DWeightParams
         if (t >= 0 && t < p.T) {
           rg = (static_cast<long long>(b) * p.T + t) * p.FG;
           rd = slot * p.FD;
-        } else if (p.status) {
-          atomicOr(p.status, EGS_STATUS_INDEX_OUT_OF_RANGE);
+        } else {
+          p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
         }
       }
       row_g[tid] = rg;

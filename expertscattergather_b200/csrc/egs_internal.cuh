@@ -36,6 +36,26 @@ __device__ __forceinline__ long long load_index(const void* ind, int index_dtype
   return static_cast<const short*>(ind)[pos];
 }
 
+// The caller's status word and, where one was registered for it (egs_set_status_mirror), its mapped host mirror.  A CTA that
+// gives up (a wait that ran out, misaligned shared memory) stores the reason there on its way out - rare, and the host looks
+// before its next call, so that no copy of the word has to be queued behind every pass.
+struct StatusRef {
+  int32_t* word = nullptr;
+  int32_t* mirror = nullptr;
+  __device__ __forceinline__ bool timed_out() const {
+    return word && (*reinterpret_cast<volatile int32_t*>(word) & EGS_STATUS_PIPELINE_TIMEOUT);
+  }
+  __device__ __forceinline__ void report(int bits) const {
+    if (word) atomicOr(word, bits);
+  }
+  __device__ __forceinline__ void tell_host() const {
+    if (word && mirror)
+      *reinterpret_cast<volatile int32_t*>(mirror) =
+          *reinterpret_cast<volatile int32_t*>(word) & (EGS_STATUS_PIPELINE_TIMEOUT | EGS_STATUS_INTERNAL);
+  }
+};
+StatusRef status_ref(int32_t* status_word);
+
 // ------------------------------------------------------------------------------------------------
 // parameter blocks (validated on the host: every product below fits in int32 unless typed int64)
 // ------------------------------------------------------------------------------------------------
@@ -49,7 +69,7 @@ struct RowGemmParams {
                       // zero = add directly into the 16-bit output; NULL = always the float32 rows
   const void* bias;   // optional [E, N] in the tensors' dtype: bias[e, :] is added to every produced row of expert e
                       // (G: to the stored row; S: to the row before it is added to its token row); NULL = none
-  int32_t* status;    // optional device status word
+  StatusRef status;    // optional device status word
   int B, T, E, K, C, N;
   int M;              // expert rows per expert = B*K
   int w_layout;
@@ -68,7 +88,7 @@ struct DWeightParams {
   const void* Ind;
   void* out;          // final output in the tensors' dtype
   float* acc;         // fp32 accumulation buffer when splits > 1 (may alias out for fp32), else unused
-  int32_t* status;
+  StatusRef status;
   int B, T, E, K, FG, FD;
   int M;              // B*K
   int out_layout;
@@ -91,7 +111,7 @@ struct FusedParams {
   float* Dst;          // float32 token rows [B*T, N2], added to (16-bit tensors: the accumulation rows of the scratch)
   void* Out16;         // 16-bit tensors: the output token rows [B*T, N2] that direct 16-bit additions go to
   const int* plan;     // 16-bit tensors: device flag, see RowGemmParams::plan
-  int32_t* status;
+  StatusRef status;
   int B, T, E, K, C1, N1, N2;
   int M;               // B*K
   int w_layout;        // of both weights

@@ -89,7 +89,7 @@ __device__ __forceinline__ void p16_rows(const FusedParams& p, int e, int m, int
   slot = (b * p.E + e) * p.K + k;
   const long long t = load_index(p.Ind, p.index_dtype, slot);
   if (t >= 0 && t < p.T) tok = b * p.T + static_cast<int>(t);
-  else if (report && p.status) atomicOr(p.status, EGS_STATUS_INDEX_OUT_OF_RANGE);
+  else if (report) p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
 }
 
 // Position in the stage ring; advanced once per stage by every role that follows the ring order.
@@ -141,10 +141,10 @@ __global__ void __launch_bounds__(kP16Threads, 1) tensor_pair16_persistent_kerne
     for (int b = 0; b < 2; ++b) mbar_init(smem_u32(&hdr->acc2_empty[b]), kP16ScatterWarps / 2);
     mbar_init(smem_u32(&hdr->drain), 1);
     fence_mbar_init();
-    hdr->abort_flag = (p.status && (*reinterpret_cast<volatile int32_t*>(p.status) & EGS_STATUS_PIPELINE_TIMEOUT)) ? 1u : 0u;
+    hdr->abort_flag = p.status.timed_out() ? 1u : 0u;
     if (smem_misaligned(smem_raw)) {
       hdr->abort_flag = 1u;
-      if (p.status) atomicOr(p.status, EGS_STATUS_INTERNAL);
+      p.status.report(EGS_STATUS_INTERNAL);
     }
   }
   if (warp == kP16WarpG) {
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kP16Threads, 1) tensor_pair16_persistent_kerne
     };
     auto acquire = [&]() -> uint32_t {           // waits for the next ring slot; returns its address (0 = aborting)
       if (ring.round > 0)
-        alive = mbar_wait_warp(smem_u32(&hdr->empty[ring.slot]), (ring.round - 1) & 1, abort_flag, p.status, lane);
+        alive = mbar_wait_warp(smem_u32(&hdr->empty[ring.slot]), (ring.round - 1) & 1, abort_flag, p.status.word, lane);
       return alive ? ring0 + static_cast<uint32_t>(ring.slot) * slot_bytes : 0u;
     };
     auto publish = [&]() {
@@ -272,8 +272,8 @@ __global__ void __launch_bounds__(kP16Threads, 1) tensor_pair16_persistent_kerne
       int tok, slot;
       p16_rows(p, blk.e, blk.m0 + q * 32 + lane, tok, slot, true);
       // acc1 of this row block is complete, and the S tiles of the previous one no longer read Y
-      alive = mbar_wait_warp(smem_u32(&hdr->acc1_full), tcnt & 1, abort_flag, p.status, lane);
-      if (alive && tcnt > 0) alive = mbar_wait_warp(smem_u32(&hdr->s_done), (tcnt - 1) & 1, abort_flag, p.status, lane);
+      alive = mbar_wait_warp(smem_u32(&hdr->acc1_full), tcnt & 1, abort_flag, p.status.word, lane);
+      if (alive && tcnt > 0) alive = mbar_wait_warp(smem_u32(&hdr->s_done), (tcnt - 1) & 1, abort_flag, p.status.word, lane);
       if (!alive) break;
       tc_fence_after();
       T* dst = mid + static_cast<long long>(slot >= 0 ? slot : 0) * p.N1;
@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(kP16Threads, 1) tensor_pair16_persistent_kerne
         const int n0 = nt * kP16NT;
         const int bn = min(kP16NT, ((p.N2 - n0) + 15) & ~15);
         // a barrier of its own per (group, buffer): this group sees every one of its completions, in order
-        alive = mbar_wait_warp(smem_u32(&hdr->acc2_full[2 * grp + buf]), (seen >> buf) & 1u, abort_flag, p.status, lane);
+        alive = mbar_wait_warp(smem_u32(&hdr->acc2_full[2 * grp + buf]), (seen >> buf) & 1u, abort_flag, p.status.word, lane);
         seen ^= 1u << buf;
         if (!alive) break;
         tc_fence_after();
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(kP16Threads, 1) tensor_pair16_persistent_kerne
       P16Ring ring;
       int tcnt = 0;
       auto mma_g = [&](int ks) {                 // one G stage into acc1
-        ok = mbar_wait(smem_u32(&hdr->full[ring.slot]), ring.round & 1, abort_flag, p.status);
+        ok = mbar_wait(smem_u32(&hdr->full[ring.slot]), ring.round & 1, abort_flag, p.status.word);
         if (!ok) return;
         const uint32_t base = ring0 + static_cast<uint32_t>(ring.slot) * slot_bytes;
         const uint64_t ad = a_desc0 + (base >> 4);
@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(kP16Threads, 1) tensor_pair16_persistent_kerne
       // only tell the current phase of a barrier from the one before, so a lane that skipped phases of full[slot] could
       // mistake an older completion for its own stage's.
       auto pass_foreign = [&]() {
-        ok = mbar_wait(smem_u32(&hdr->full[ring.slot]), ring.round & 1, abort_flag, p.status);
+        ok = mbar_wait(smem_u32(&hdr->full[ring.slot]), ring.round & 1, abort_flag, p.status.word);
         ring.advance(stages);
       };
       if (static_cast<int>(blockIdx.x) < row_blocks) {
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kP16Threads, 1) tensor_pair16_persistent_kerne
         const bool has_next = rb + static_cast<int>(gridDim.x) < row_blocks;
         if (has_next) {
           // acc1 has been read (Y(t) is complete) before G(t+1) overwrites it
-          ok = mbar_wait(smem_u32(&hdr->y_ready), tcnt & 1, abort_flag, p.status);
+          ok = mbar_wait(smem_u32(&hdr->y_ready), tcnt & 1, abort_flag, p.status.word);
           if (!ok) break;
           tc_fence_after();
         }
@@ -452,26 +452,26 @@ __global__ void __launch_bounds__(kP16Threads, 1) tensor_pair16_persistent_kerne
       uint32_t used = 0, par_e = 0;              // per accumulator: used before; parity of the release to wait for next
       // (see the G lane: stages of the other lane are waited for too, so that no phase of full[slot] is skipped)
       auto pass_foreign = [&]() {
-        ok = mbar_wait(smem_u32(&hdr->full[ring.slot]), ring.round & 1, abort_flag, p.status);
+        ok = mbar_wait(smem_u32(&hdr->full[ring.slot]), ring.round & 1, abort_flag, p.status.word);
         ring.advance(stages);
       };
       for (int ks = 0; ks < nk1 && ok; ++ks) pass_foreign();           // the G stages of the first row block
       for (int rb = blockIdx.x; rb < row_blocks && ok; rb += gridDim.x, ++tcnt) {
         const bool has_next = rb + static_cast<int>(gridDim.x) < row_blocks;
-        ok = mbar_wait(smem_u32(&hdr->y_ready), tcnt & 1, abort_flag, p.status);
+        ok = mbar_wait(smem_u32(&hdr->y_ready), tcnt & 1, abort_flag, p.status.word);
         if (!ok) break;
         tc_fence_after();
         for (int i = 0; i < steps && ok; ++i) {
           if (i < n2) {
             const int buf = i & 1, gb = 2 * ((i >> 1) & 1) + buf;
             if ((used >> buf) & 1u) {                      // the previous tile in this accumulator has been read
-              ok = mbar_wait(smem_u32(&hdr->acc2_empty[buf]), (par_e >> buf) & 1u, abort_flag, p.status);
+              ok = mbar_wait(smem_u32(&hdr->acc2_empty[buf]), (par_e >> buf) & 1u, abort_flag, p.status.word);
               if (!ok) break;
               par_e ^= 1u << buf;
               tc_fence_after();
             }
             used |= 1u << buf;
-            ok = mbar_wait(smem_u32(&hdr->full[ring.slot]), ring.round & 1, abort_flag, p.status);
+            ok = mbar_wait(smem_u32(&hdr->full[ring.slot]), ring.round & 1, abort_flag, p.status.word);
             if (!ok) break;
             const uint32_t base = ring0 + static_cast<uint32_t>(ring.slot) * slot_bytes;
             const int bn = min(kP16NT, ((p.N2 - i * kP16NT) + 15) & ~15);
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(kP16Threads, 1) tensor_pair16_persistent_kerne
   // ---- common exit ----
   tc_fence_before();
   __syncthreads();
-  if (warp == kP16WarpG) tmem_release(tmem_base, kP16TmemCols, smem_u32(&hdr->drain), abort_flag, lane);
+  if (warp == kP16WarpG) tmem_release(tmem_base, kP16TmemCols, smem_u32(&hdr->drain), abort_flag, p.status, lane);
 }
 
 constexpr size_t kP16SmemMax = 227 * 1024;

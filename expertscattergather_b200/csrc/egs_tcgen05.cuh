@@ -453,10 +453,11 @@ __device__ __forceinline__ bool smem_misaligned(const void* raw) { return (smem_
 // the columns are released; if even that wait runs out the columns stay allocated until the CTA exits rather than
 // being released under running MMAs.
 __device__ __forceinline__ void tmem_release(uint32_t tmem_base, uint32_t ncols, uint32_t drain_bar, volatile uint32_t* abort_flag,
-                                             int lane) {
+                                             const StatusRef& status, int lane) {
   uint32_t safe = 1u;
   if (*abort_flag) {
     if (lane == 0) {
+      status.tell_host();
       uint32_t ignore_abort = 0u;      // the CTA's abort flag is already up: this wait must not return early on it
       umma_commit(drain_bar);
       safe = mbar_wait(drain_bar, 0u, &ignore_abort, nullptr) ? 1u : 0u;

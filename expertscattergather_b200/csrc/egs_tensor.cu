@@ -44,7 +44,7 @@ namespace {
 struct Pipe {
   SmemHeader* hdr;
   volatile uint32_t* abort_flag;
-  int32_t* status;
+  StatusRef status;
   uint32_t tiles0;        // shared-window address of stage 0
   uint32_t stage_bytes;
   int stages;
@@ -65,10 +65,10 @@ __device__ __forceinline__ uint32_t pipe_setup(const Pipe& pp, uint32_t full_cou
     // A launch that follows a timed-out one on the same status word does no work (keeps a broken pipeline
     // from costing one wait limit per wave of CTAs).
     hdr->abort_flag =
-        (pp.status && (*reinterpret_cast<volatile int32_t*>(pp.status) & EGS_STATUS_PIPELINE_TIMEOUT)) ? 1u : 0u;
+        pp.status.timed_out() ? 1u : 0u;
     if (smem_misaligned(hdr)) {
       hdr->abort_flag = 1u;
-      if (pp.status) atomicOr(pp.status, EGS_STATUS_INTERNAL);
+      pp.status.report(EGS_STATUS_INTERNAL);
     }
   }
   if (warp == kProducerWarps) {
@@ -84,7 +84,7 @@ __device__ __forceinline__ uint32_t pipe_setup(const Pipe& pp, uint32_t full_cou
 __device__ __forceinline__ void pipe_teardown(const Pipe& pp, uint32_t tmem_base, uint32_t tmem_cols, int warp) {
   tc_fence_before();
   __syncthreads();
-  if (warp == kProducerWarps) tmem_release(tmem_base, tmem_cols, smem_u32(&pp.hdr->drain), pp.abort_flag, threadIdx.x & 31);
+  if (warp == kProducerWarps) tmem_release(tmem_base, tmem_cols, smem_u32(&pp.hdr->drain), pp.abort_flag, pp.status, threadIdx.x & 31);
 }
 
 // Common end of every producer variant: drain own copies, then wait (warp-uniformly) for the accumulator.
@@ -92,7 +92,7 @@ __device__ __forceinline__ bool producer_finish(const Pipe& pp, int lane, bool a
   cp_async_wait_all();
   // all lanes of a warp must take the tcgen05.ld of the epilogue together: the decision is warp-uniform
   alive = __all_sync(0xffffffffu, alive);
-  if (alive && pp.nk > 0) alive = mbar_wait_warp(smem_u32(&pp.hdr->done), 0u, pp.abort_flag, pp.status, lane);
+  if (alive && pp.nk > 0) alive = mbar_wait_warp(smem_u32(&pp.hdr->done), 0u, pp.abort_flag, pp.status.word, lane);
   if (alive) tc_fence_after();
   return alive;
 }
@@ -107,7 +107,7 @@ __device__ __forceinline__ bool run_producer(const Pipe& pp, int lane, Issue&& i
   if (!STRICT) {
     for (int kt = 0; kt < nk; ++kt) {
       const int slot = kt % stages, use = kt / stages;
-      if (use > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[slot]), (use - 1) & 1, pp.abort_flag, pp.status, lane);
+      if (use > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[slot]), (use - 1) & 1, pp.abort_flag, pp.status.word, lane);
       if (!alive) break;
       issue(kt, pp.tiles0 + slot * pp.stage_bytes);
       cp_async_mbar_arrive_noinc(smem_u32(&hdr->full[slot]));
@@ -129,7 +129,7 @@ __device__ __forceinline__ bool run_producer(const Pipe& pp, int lane, Issue&& i
       const int kt = kc + dist;
       if (kt < nk && alive) {
         const int use = kt / stages;
-        if (use > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[kt % stages]), (use - 1) & 1, pp.abort_flag, pp.status, lane);
+        if (use > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[kt % stages]), (use - 1) & 1, pp.abort_flag, pp.status.word, lane);
         if (alive) issue(kt, pp.tiles0 + (kt % stages) * pp.stage_bytes);
       }
       cp_async_commit();
@@ -165,7 +165,7 @@ __device__ __forceinline__ void run_mma_lane(const Pipe& pp, Mma&& mma) {
   bool ok = true;
   for (int ks = 0; ks < pp.nk; ++ks) {
     const int slot = ks % pp.stages;
-    ok = mbar_wait(smem_u32(&hdr->full[slot]), (ks / pp.stages) & 1, pp.abort_flag, pp.status);
+    ok = mbar_wait(smem_u32(&hdr->full[slot]), (ks / pp.stages) & 1, pp.abort_flag, pp.status.word);
     if (!ok) break;
     tc_fence_after();
     mma(ks, pp.tiles0 + slot * pp.stage_bytes);
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_rowgemm_kern
         ra = SCATTER ? slot : tok;
         ro = SCATTER ? tok : slot;
       } else {
-        if (p.status) atomicOr(p.status, EGS_STATUS_INDEX_OUT_OF_RANGE);
+        p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
         if (!SCATTER) ro = slot;      // gather: the row is still written (zeros)
       }
     }
@@ -608,7 +608,7 @@ __device__ __forceinline__ void lookup_rows(const RowGemmParams& p, int e, int m
     src_row = SCATTER ? slot : tok;
     dst_row = SCATTER ? tok : slot;
   } else {
-    if (report && p.status) atomicOr(p.status, EGS_STATUS_INDEX_OUT_OF_RANGE);
+    if (report) p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
     if (!SCATTER) dst_row = slot;      // gather: the row is still written (zeros)
   }
 }
@@ -661,10 +661,10 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
     }
     mbar_init(smem_u32(&hdr->drain), 1);
     fence_mbar_init();
-    hdr->abort_flag = (p.status && (*reinterpret_cast<volatile int32_t*>(p.status) & EGS_STATUS_PIPELINE_TIMEOUT)) ? 1u : 0u;
+    hdr->abort_flag = p.status.timed_out() ? 1u : 0u;
     if (smem_misaligned(smem_raw)) {
       hdr->abort_flag = 1u;
-      if (p.status) atomicOr(p.status, EGS_STATUS_INTERNAL);
+      p.status.report(EGS_STATUS_INTERNAL);
     }
   }
   const int mma_warp = kPersistProducerWarps + kPersistEpilogueWarps;
@@ -752,7 +752,7 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
         const bool tile_full = a_full && (nc_full || cn_full);
         for (int kt = 0; kt < nk; ++kt, ++g) {
           const int slot = g % stages, use = g / stages;
-          if (use > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[slot]), (use - 1) & 1, abort_flag, p.status, lane);
+          if (use > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[slot]), (use - 1) & 1, abort_flag, p.status.word, lane);
           if (!alive) break;
           const uint32_t base = tiles0 + slot * stage_bytes;
           const int k0 = kt * KE;
@@ -827,7 +827,7 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
         const int n0 = nt * p.BN;
         const int bn = min(p.BN, ((p.N - n0) + 15) & ~15);
         const int buf = t & 1;
-        alive = mbar_wait_warp(smem_u32(&hdr->acc_full[buf]), (t >> 1) & 1, abort_flag, p.status, lane);
+        alive = mbar_wait_warp(smem_u32(&hdr->acc_full[buf]), (t >> 1) & 1, abort_flag, p.status.word, lane);
         if (!alive) break;
         tc_fence_after();
         const int nblk = (bn + 31) >> 5;
@@ -902,14 +902,14 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
           const uint32_t idesc = make_idesc(Elem<T>::fmt, 0u, w_nc ? 0u : 1u, kTileM, static_cast<uint32_t>(bn));
           const int buf = t & 1;
           if (t >= 2) {
-            ok = mbar_wait(smem_u32(&hdr->acc_empty[buf]), ((t >> 1) - 1) & 1, abort_flag, p.status);
+            ok = mbar_wait(smem_u32(&hdr->acc_empty[buf]), ((t >> 1) - 1) & 1, abort_flag, p.status.word);
             if (!ok) break;
             tc_fence_after();
           }
           const uint32_t d = tmem_base + buf * acc_cols;
           for (int ks = 0; ks < nk; ++ks, ++g) {
             const int slot = g % stages;
-            ok = mbar_wait(smem_u32(&hdr->full[slot]), (g / stages) & 1, abort_flag, p.status);
+            ok = mbar_wait(smem_u32(&hdr->full[slot]), (g / stages) & 1, abort_flag, p.status.word);
             if (!ok) break;
             tc_fence_after();
             const uint32_t a_hi = tiles0 + slot * stage_bytes;
@@ -934,7 +934,7 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
   // ---- common exit ----
   tc_fence_before();
   __syncthreads();
-  if (warp == mma_warp) tmem_release(tmem_base, tmem_cols, smem_u32(&hdr->drain), abort_flag, lane);
+  if (warp == mma_warp) tmem_release(tmem_base, tmem_cols, smem_u32(&hdr->drain), abort_flag, p.status, lane);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1010,7 +1010,7 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_dweight_kern
       if (brow[j] >= 0) {
         int tok = -1;
         if (tk[j] >= 0 && tk[j] < p.T) tok = brow[j] + static_cast<int>(tk[j]);
-        else if (p.status) atomicOr(p.status, EGS_STATUS_INDEX_OUT_OF_RANGE);
+        else p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
         row_tok[i0 + j * kThreads] = tok;
       }
     }
@@ -1324,7 +1324,7 @@ __global__ void __launch_bounds__(17 * 32, 1) tensor_fused_pair_kernel(FusedPara
       slot = (b * p.E + e) * p.K + k;
       const long long t = load_index(p.Ind, p.index_dtype, slot);
       if (t >= 0 && t < p.T) tok = b * p.T + static_cast<int>(t);
-      else if (p.status) atomicOr(p.status, EGS_STATUS_INDEX_OUT_OF_RANGE);
+      else p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
     }
     hdr->row_tok[tid] = tok;
     hdr->row_slot[tid] = slot;
@@ -1339,10 +1339,10 @@ __global__ void __launch_bounds__(17 * 32, 1) tensor_fused_pair_kernel(FusedPara
     mbar_init(smem_u32(&hdr->acc2_done), 1);
     mbar_init(smem_u32(&hdr->drain), 1);
     fence_mbar_init();
-    hdr->abort_flag = (p.status && (*reinterpret_cast<volatile int32_t*>(p.status) & EGS_STATUS_PIPELINE_TIMEOUT)) ? 1u : 0u;
+    hdr->abort_flag = p.status.timed_out() ? 1u : 0u;
     if (smem_misaligned(smem_raw)) {
       hdr->abort_flag = 1u;
-      if (p.status) atomicOr(p.status, EGS_STATUS_INTERNAL);
+      p.status.report(EGS_STATUS_INTERNAL);
     }
   }
   const int mma_warp = kProdWarps + kEpiWarps;
@@ -1420,7 +1420,7 @@ __global__ void __launch_bounds__(17 * 32, 1) tensor_fused_pair_kernel(FusedPara
     if (!STRICT) {
       for (int g = 0; g < ntot; ++g) {
         const int slot = g % stages, use = g / stages;
-        if (use > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[slot]), (use - 1) & 1, abort_flag, p.status, lane);
+        if (use > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[slot]), (use - 1) & 1, abort_flag, p.status.word, lane);
         if (!alive) break;
         issue(g, tiles0 + slot * stage_bytes);
         cp_async_mbar_arrive_noinc(smem_u32(&hdr->full[slot]));
@@ -1443,7 +1443,7 @@ __global__ void __launch_bounds__(17 * 32, 1) tensor_fused_pair_kernel(FusedPara
         const int g = gc + dist;
         if (g < ntot && alive) {
           const int use = g / stages;
-          if (use > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[g % stages]), (use - 1) & 1, abort_flag, p.status, lane);
+          if (use > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[g % stages]), (use - 1) & 1, abort_flag, p.status.word, lane);
           if (alive) issue(g, tiles0 + (g % stages) * stage_bytes);
         }
         cp_async_commit();
@@ -1457,7 +1457,7 @@ __global__ void __launch_bounds__(17 * 32, 1) tensor_fused_pair_kernel(FusedPara
     const int row = lg * 32 + lane;               // tile row this thread owns in tensor memory
     const uint32_t lane_base = static_cast<uint32_t>(lg * 32) << 16;
     bool alive = true;
-    if (nk1 > 0) alive = mbar_wait_warp(smem_u32(&hdr->acc1_done), 0u, abort_flag, p.status, lane);
+    if (nk1 > 0) alive = mbar_wait_warp(smem_u32(&hdr->acc1_done), 0u, abort_flag, p.status.word, lane);
     if (alive) {
       tc_fence_after();
       // (1) Mid tile: tensor memory -> shared memory in the K-major operand format (segment = 32 columns)
@@ -1503,7 +1503,7 @@ __global__ void __launch_bounds__(17 * 32, 1) tensor_fused_pair_kernel(FusedPara
       }
       // (3) scatter epilogue: the stage ring is idle once acc2_done has completed; its first 32 KB are the
       //     warps' transpose tiles
-      alive = mbar_wait_warp(smem_u32(&hdr->acc2_done), 0u, abort_flag, p.status, lane);
+      alive = mbar_wait_warp(smem_u32(&hdr->acc2_done), 0u, abort_flag, p.status.word, lane);
       if (alive) {
         tc_fence_after();
         const uint32_t tile = tiles0 + static_cast<uint32_t>(ew) * 4096u;
@@ -1532,10 +1532,10 @@ __global__ void __launch_bounds__(17 * 32, 1) tensor_fused_pair_kernel(FusedPara
         const int slot = g % stages;
         if (g == nk1) {
           // the Mid operand tile must be complete before the second contraction starts
-          ok = mbar_wait(smem_u32(&hdr->mid_ready), 0u, abort_flag, p.status);
+          ok = mbar_wait(smem_u32(&hdr->mid_ready), 0u, abort_flag, p.status.word);
           if (!ok) break;
         }
-        ok = mbar_wait(smem_u32(&hdr->full[slot]), (g / stages) & 1, abort_flag, p.status);
+        ok = mbar_wait(smem_u32(&hdr->full[slot]), (g / stages) & 1, abort_flag, p.status.word);
         if (!ok) break;
         tc_fence_after();
         const uint32_t base = tiles0 + slot * stage_bytes;
@@ -1578,7 +1578,7 @@ __global__ void __launch_bounds__(17 * 32, 1) tensor_fused_pair_kernel(FusedPara
   // ---- common exit ----
   tc_fence_before();
   __syncthreads();
-  if (warp == mma_warp) tmem_release(tmem_base, tmem_cols, smem_u32(&hdr->drain), abort_flag, lane);
+  if (warp == mma_warp) tmem_release(tmem_base, tmem_cols, smem_u32(&hdr->drain), abort_flag, p.status, lane);
 }
 
 // ------------------------------------------------------------------------------------------------

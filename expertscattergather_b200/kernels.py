@@ -7,6 +7,9 @@ dispatcher ops in namespace ``mylib`` with the same schemas (``:362,395,444,478`
 ``torch.autograd.Function`` classes (``:581-639``).  The bodies call the sm_100a kernels of
 ``libegs_b200.so`` instead of Triton; there is no autotuning and no CPU path.
 
+The modules (``torch_interface.py``) run the same functions natively (``csrc/egs_host.cpp``) on plain tensors in eager
+mode; the Python classes and dispatcher ops here serve direct callers, ``torch.compile`` and fake tensors.
+
 Differences from the reference, on purpose:
 * the scatter forward output is zero-filled (the reference allocates it with ``torch.empty`` and only
   adds to it, ``:457``);
@@ -41,34 +44,9 @@ def _gather_forward(X, W, Ind, out_dtype):
     return ops.gather_gemm(X, W, Ind, w_layout="cn")
 
 
-def _weight_grad_on_side_stream(Xsrc, Ysrc, Ind, out_layout):
-    """Enqueues operator D on the helper stream (it is independent of the dX / dY kernel of the same backward
-    call, and the two co-reside on the SMs); the caller joins with ``_join_side``."""
-    dev = Xsrc.device
-    main = torch.cuda.current_stream(dev)
-    side = ops.side_stream(dev)
-    side.wait_stream(main)
-    with torch.cuda.stream(side):
-        grad_W = ops.dweight(Xsrc, Ysrc, Ind, out_layout=out_layout)
-        grad_W.record_stream(main)
-    return grad_W
-
-
-def _join_side(t):
-    """Joins the helper stream and queues the copy of the status word to its host mirror: once per backward call, after
-    its kernels, so that the next operator call raises if one of them reported invalid results."""
-    torch.cuda.current_stream(t.device).wait_stream(ops.side_stream(t.device))
-    ops.publish_status(t.device)
-
-
 def _gather_backward(X, W, Ind, grad_output, out_dtype):
     # dX = scatter(dY @ W_g^T), dW_g = gather(X)^T @ dY        (reference: egs/triton_kernels.py:400-441)
-    T = X.shape[1]
-    grad_output = grad_output.contiguous()
-    grad_W = _weight_grad_on_side_stream(X, grad_output, Ind, "gathered_rows")
-    grad_X = ops.gemm_scatter(grad_output, W, Ind, T, w_layout="nc")
-    _join_side(grad_X)
-    return grad_X, grad_W
+    return ops._host().gather_backward(X, W, Ind, grad_output)
 
 
 def _scatter_forward(Y, W, Ind, T, out_dtype):
@@ -78,11 +56,7 @@ def _scatter_forward(Y, W, Ind, T, out_dtype):
 
 def _scatter_backward(Y, W, Ind, grad_X, out_dtype):
     # dY = gather(dOut) @ W_s^T, dW_s = Y^T @ gather(dOut)     (reference: egs/triton_kernels.py:483-525)
-    grad_X = grad_X.contiguous()
-    grad_W = _weight_grad_on_side_stream(grad_X, Y, Ind, "direct_rows")
-    grad_Y = ops.gather_gemm(grad_X, W, Ind, w_layout="nc")
-    _join_side(grad_Y)
-    return grad_Y, grad_W
+    return ops._host().scatter_backward(Y, W, Ind, grad_X)
 
 
 # ---- fake (meta) implementations: shapes and dtypes only --------------------------------------------
@@ -222,10 +196,9 @@ class ExpertGatherBiasFunction(torch.autograd.Function):
         X, W, Ind = ctx.saved_tensors
         need_x, need_w, need_b = ctx.needs_input_grad[:3]
         grad_output = grad_output.contiguous()
-        grad_W = _weight_grad_on_side_stream(X, grad_output, Ind, "gathered_rows") if need_w else None
+        grad_W = ops.dweight(X, grad_output, Ind, out_layout="gathered_rows") if need_w else None
         grad_X = ops.gemm_scatter(grad_output, W, Ind, X.shape[1], w_layout="nc") if need_x else None
         grad_b = grad_output.sum(dim=(0, 2)).reshape(ctx.bias_shape) if need_b else None
-        _join_side(grad_output)
         return grad_X, grad_W, grad_b, None
 
 
@@ -247,13 +220,12 @@ class ExpertScatterBiasFunction(torch.autograd.Function):
         Y, W, Ind = ctx.saved_tensors
         need_y, need_w, need_b = ctx.needs_input_grad[:3]
         grad_X = grad_X.contiguous()
-        grad_W = _weight_grad_on_side_stream(grad_X, Y, Ind, "direct_rows") if need_w else None
+        grad_W = ops.dweight(grad_X, Y, Ind, out_layout="direct_rows") if need_w else None
         grad_Y = ops.gather_gemm(grad_X, W, Ind, w_layout="nc") if need_y else None
         grad_b = None
         if need_b:
             ones = torch.ones(Y.shape[0], Y.shape[1], Y.shape[2], 8, device=Y.device, dtype=Y.dtype)
             grad_b = ops.dweight(grad_X, ones, Ind, out_layout="gathered_rows")[:, :, 0].reshape(ctx.bias_shape)
-        _join_side(grad_X)
         return grad_Y, grad_W, grad_b, None, None
 
 
@@ -265,8 +237,7 @@ class ExpertGatherScatterFunction(torch.autograd.Function):
     Where the fused kernel pays (float32, single-wave grids: ``ops.fused_pair_preferred``) the forward pass is one
     kernel (Y is written once, for the backward pass, and consumed from shared memory) and so is dY -> dX of the
     backward pass; otherwise each pass runs the two separate operators.  The weight gradients are the same two
-    contractions as in ``ExpertGatherFunction`` / ``ExpertScatterFunction`` and run next to dY -> dX on the helper
-    stream.  backward returns ``(grad_X, grad_W_g, grad_W_s, None)``; gradients autograd does not ask for are skipped.
+    contractions as in ``ExpertGatherFunction`` / ``ExpertScatterFunction``.  backward returns ``(grad_X, grad_W_g, grad_W_s, None)``; gradients autograd does not ask for are skipped.
     """
 
     @staticmethod
@@ -288,15 +259,13 @@ class ExpertGatherScatterFunction(torch.autograd.Function):
         grad_out = grad_out.contiguous()
         grad_X = grad_Wg = grad_Ws = dY = None
         if need_ws:
-            grad_Ws = _weight_grad_on_side_stream(grad_out, Y, Ind, "direct_rows")   # needs only dOut and Y
+            grad_Ws = ops.dweight(grad_out, Y, Ind, out_layout="direct_rows")
         if need_x and ctx.fused:
             dY, grad_X = ops.gather_scatter_pair(grad_out, Ws, Wg, Ind, w_layout="nc")
         elif need_x or need_wg:
             dY = ops.gather_gemm(grad_out, Ws, Ind, w_layout="nc")
         if need_wg:
-            grad_Wg = _weight_grad_on_side_stream(X, dY, Ind, "gathered_rows")
+            grad_Wg = ops.dweight(X, dY, Ind, out_layout="gathered_rows")
         if need_x and grad_X is None:
             grad_X = ops.gemm_scatter(dY, Wg, Ind, X.shape[1], w_layout="nc")
-        if need_ws or need_wg:
-            _join_side(grad_out)
         return grad_X, grad_Wg, grad_Ws, None

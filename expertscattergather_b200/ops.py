@@ -1,8 +1,9 @@
 """Tensor-level host API over the C ABI: the three operators G, S, D on torch CUDA tensors.
 
-The functions allocate outputs with torch (so every buffer belongs to torch's caching allocator, as in the
-reference's launch wrappers, ``egs/triton_kernels.py:375,408-409,457,491-492``), pass raw pointers, sizes
-and the current CUDA stream to ``libegs_b200.so`` and return without synchronising.
+The operators run in the native host module (``csrc/egs_host.cpp``): it checks the arguments, allocates outputs with torch
+(so every buffer belongs to torch's caching allocator, as in the reference's launch wrappers,
+``egs/triton_kernels.py:375,408-409,457,491-492``), passes raw pointers, sizes and the current CUDA stream to
+``libegs_b200.so`` and returns without synchronising.
 """
 from __future__ import annotations
 
@@ -19,15 +20,27 @@ __all__ = ["gather_gemm", "gemm_scatter", "gather_scatter_pair", "fused_pair_eli
 _PRECISIONS = {"strict": _lib.PREC_STRICT, "fp32": _lib.PREC_STRICT, "tf32": _lib.PREC_TF32}
 _PATHS = {"auto": _lib.PATH_AUTO, "generic": _lib.PATH_GENERIC, "tensor": _lib.PATH_TENSOR,
           "paired": _lib.PATH_PAIRED}     # "paired": per-call only, operator G on 16-bit tensors (see gather_gemm)
-_SM_COUNT = 148     # B200
 
 _state = {
     "precision": os.environ.get("EGS_B200_PRECISION", "strict").lower(),
     "path": os.environ.get("EGS_B200_PATH", "auto").lower(),
     "debug": os.environ.get("EGS_B200_DEBUG", "0") not in ("0", "", "false"),
 }
-_status_words: dict[int, torch.Tensor] = {}
-_status_mirrors: dict[int, torch.Tensor] = {}     # pinned host copies of the status words (see publish_status)
+_native = None
+
+
+def _push_state() -> None:
+    """Tells the native host module the defaults in force."""
+    if _native is not None:
+        _native.configure(_PRECISIONS[_state["precision"]], _PATHS[_state["path"]], _state["debug"])
+
+
+def _host():
+    global _native
+    if _native is None:
+        _native = _lib.host()
+        _push_state()
+    return _native
 
 
 def set_precision(mode: str) -> None:
@@ -36,6 +49,7 @@ def set_precision(mode: str) -> None:
     if mode not in _PRECISIONS:
         raise ValueError(f"unknown precision {mode!r}")
     _state["precision"] = mode
+    _push_state()
 
 
 def get_precision() -> str:
@@ -47,6 +61,7 @@ def set_path(path: str) -> None:
     if path not in _PATHS or path == "paired":
         raise ValueError(f"unknown path {path!r}")
     _state["path"] = path
+    _push_state()
 
 
 def get_path() -> str:
@@ -78,75 +93,30 @@ def _index_tensor(Ind: torch.Tensor):
 
 
 def _status_word(device: torch.device) -> torch.Tensor:
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    w = _status_words.get(idx)
-    if w is None:
-        w = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
-        _status_words[idx] = w
-    return w
+    dev = torch.device(device)
+    return _host().status_word(dev.index if dev.index is not None else torch.cuda.current_device())
+
+
+def _status_devices(device) -> int:
+    """Device index for the host module's status calls; -1 = every device in use."""
+    index = None if device is None else torch.device(device).index
+    return -1 if index is None else index
 
 
 def reset_status(device=None) -> None:
-    for idx, w in _status_words.items():
-        if device is None or torch.device(device).index in (None, idx):
-            w.zero_()
-            m = _status_mirrors.get(idx)
-            if m is not None:
-                m.zero_()
-
-
-def _status_text(idx: int, v: int) -> str:
-    msgs = []
-    if v & _lib.STATUS_INDEX_OUT_OF_RANGE:
-        msgs.append("an Ind value outside [0, T) was met (slot skipped)")
-    if v & _lib.STATUS_PIPELINE_TIMEOUT:
-        msgs.append("a bounded wait inside a tensor-core kernel ran out (results invalid)")
-    if v & _lib.STATUS_INTERNAL:
-        msgs.append("a tensor-core kernel found its shared memory misaligned and did no work (results invalid)")
-    return f"egs kernels on cuda:{idx} reported: " + "; ".join(msgs)
+    _host().reset_status(_status_devices(device))
 
 
 def publish_status(device) -> None:
-    """Queues, on the current stream, a 4-byte copy of the device status word into a pinned host mirror.  No
-    synchronisation: the mirror shows the word as of the last copy that has completed, and every operator call looks
-    at it first (see ``_raise_if_flagged``).  The autograd functions and ``train_step`` call this once per backward
-    pass / step, so a kernel that flagged a problem (above all a timed-out pipeline wait, after which the kernels skip
-    their work) makes the next call raise instead of returning uninitialised memory."""
-    dev = torch.device(device)
-    idx = dev.index if dev.index is not None else torch.cuda.current_device()
-    m = _status_mirrors.get(idx)
-    if m is None:
-        m = torch.zeros(1, dtype=torch.int32).pin_memory()
-        _status_mirrors[idx] = m
-    m.copy_(_status_word(torch.device("cuda", idx)), non_blocking=True)
-
-
-def _raise_if_flagged(dev: torch.device) -> None:
-    """Host-side look at the pinned mirror (no synchronisation).  Invalid-result bits raise and are cleared on both
-    sides; an out-of-range index alone is left for ``check_status`` (the slot was skipped, results are defined)."""
-    idx = dev.index if dev.index is not None else torch.cuda.current_device()
-    m = _status_mirrors.get(idx)
-    if m is None:
-        return
-    v = int(m[0])
-    if v & (_lib.STATUS_PIPELINE_TIMEOUT | _lib.STATUS_INTERNAL):
-        m.zero_()
-        _status_words[idx].zero_()
-        raise RuntimeError(_status_text(idx, v))
+    """Kept for callers of earlier versions: nothing has to be queued any more.  Kernels that report invalid results (above
+    all a timed-out pipeline wait, after which the kernels skip their work) store the report in a mapped host word as well,
+    and every operator call looks at that word first and raises instead of returning uninitialised memory."""
+    _status_word(device)
 
 
 def check_status(device=None) -> None:
     """Reads the device status word(s) (synchronises) and raises if a kernel flagged a problem."""
-    for idx, w in list(_status_words.items()):
-        if device is not None and torch.device(device).index not in (None, idx):
-            continue
-        v = int(w.item())
-        if v:
-            w.zero_()
-            m = _status_mirrors.get(idx)
-            if m is not None:
-                m.zero_()
-            raise RuntimeError(_status_text(idx, v))
+    _host().check_status(_status_devices(device))
 
 
 _side_streams: dict[int, "torch.cuda.Stream"] = {}
@@ -181,11 +151,7 @@ def fill_stream(device) -> "torch.cuda.Stream":
 
 def fill_zero(t: torch.Tensor) -> torch.Tensor:
     """Zero-fills a contiguous CUDA tensor with the library's fill kernel on the current stream."""
-    if not t.is_cuda or not t.is_contiguous():
-        raise ValueError("fill_zero needs a contiguous CUDA tensor")
-    with torch.cuda.device(t.device):
-        rc = _lib.load().egs_fill_zero(t.data_ptr(), t.numel() * t.element_size(), _stream_ptr(t.device))
-    _lib.check(rc, "egs_fill_zero")
+    _host().fill_zero(t)
     return t
 
 
@@ -201,7 +167,7 @@ def _require_cuda(*tensors) -> torch.device:
             raise RuntimeError("expert gather/scatter kernels need CUDA tensors (there is no CPU path)")
         if t.device != dev:
             raise RuntimeError("all tensors must be on the same CUDA device")
-    _raise_if_flagged(dev)
+    _host().raise_if_flagged(tensors[0])
     return dev
 
 
@@ -209,10 +175,29 @@ def _stream_ptr(dev) -> int:
     return torch.cuda.current_stream(dev).cuda_stream
 
 
+_DEFAULT = -1     # the host module's "whatever set_precision / set_path say"
+
+
+def _prec(precision) -> int:
+    return _DEFAULT if precision is None else _PRECISIONS[precision]
+
+
+def _path(path) -> int:
+    return _DEFAULT if path is None else _PATHS[path]
+
+
 def _enums(precision, path):
     prec = _PRECISIONS[precision if precision is not None else _state["precision"]]
     pth = _PATHS[path if path is not None else _state["path"]]
     return prec, pth
+
+
+def _layout(w_layout: str) -> int:
+    if w_layout == "cn":
+        return _lib.W_CN
+    if w_layout == "nc":
+        return _lib.W_NC
+    raise ValueError("w_layout must be 'cn' ([E,C,N]) or 'nc' ([E,N,C])")
 
 
 def _w_dims(W: torch.Tensor, w_layout: str):
@@ -239,36 +224,7 @@ def gather_gemm(X, W, Ind, *, w_layout="cn", precision=None, path=None, bias=Non
     ``W^T`` per expert ('nc', W is [E,N,C]).  X [B,T,C] -> Y [B,E,K,N], dtype of X.  ``bias`` ([E,N] or [E,1,N]) is
     added in the kernel's epilogue.  ``path="paired"`` (16-bit tensors, N a multiple of 32 up to 256) runs the kernel on
     pairs of SMs (``EGS_PATH_PAIRED``); it raises for shapes that kernel does not take."""
-    lib = _lib.load()
-    if X.dim() != 3 or W.dim() != 3 or Ind.dim() != 3:
-        raise ValueError("expected X[B,T,C], W[E,.,.], Ind[B,E,K]")
-    dev = _require_cuda(X, W, Ind)
-    if W.dtype != X.dtype:
-        raise ValueError("X and W must have the same dtype")
-    dt = dtype_to_type_id(X.dtype)
-    E, C, N, wl = _w_dims(W, w_layout)
-    B, T, Cx = X.shape
-    Bi, Ei, K = Ind.shape
-    if Cx != C or Ei != E or Bi != B:
-        raise ValueError(f"shape mismatch: X{tuple(X.shape)} W{tuple(W.shape)} Ind{tuple(Ind.shape)} ({w_layout})")
-    Xc, Wc = X.contiguous(), W.contiguous()
-    Ic, it = _index_tensor(Ind)
-    prec, pth = _enums(precision, path)
-    with torch.cuda.device(dev):
-        Y = torch.empty((B, E, K, N), device=dev, dtype=X.dtype)
-        dims = _lib.Dims(B, T, E, K, C, N)
-        bias_c = _bias_rows(bias, E, N, X.dtype, dev)
-        if bias_c is None:
-            rc = lib.egs_gather_gemm(Xc.data_ptr(), Wc.data_ptr(), Ic.data_ptr(), Y.data_ptr(), ctypes.byref(dims), wl, dt,
-                                     it, prec, pth, _status_word(dev).data_ptr(), _stream_ptr(dev))
-        else:
-            rc = lib.egs_gather_gemm_bias(Xc.data_ptr(), Wc.data_ptr(), bias_c.data_ptr(), Ic.data_ptr(), Y.data_ptr(),
-                                          ctypes.byref(dims), wl, dt, it, prec, pth, _status_word(dev).data_ptr(),
-                                          _stream_ptr(dev))
-    _lib.check(rc, "egs_gather_gemm")
-    if _state["debug"]:
-        check_status(dev)
-    return Y
+    return _host().gather_gemm(X, W, Ind, _layout(w_layout), _prec(precision), _path(path), bias)
 
 
 def gemm_scatter(Y, W, Ind, T, *, w_layout="cn", out=None, precision=None, path=None, bias=None, csr=None):
@@ -277,53 +233,13 @@ def gemm_scatter(Y, W, Ind, T, *, w_layout="cn", out=None, precision=None, path=
     [E,1,N]) is added to every routed slot's product before it is scattered.  ``csr``: an :class:`IndexCSR` of this
     ``Ind`` - the 16-bit scatter then takes its choice between direct additions and float32 rows from it instead of
     counting the contributions per token row again."""
-    lib = _lib.load()
-    if Y.dim() != 4 or W.dim() != 3 or Ind.dim() != 3:
-        raise ValueError("expected Y[B,E,K,C], W[E,.,.], Ind[B,E,K]")
-    dev = _require_cuda(Y, W, Ind)
-    if W.dtype != Y.dtype:
-        raise ValueError("Y and W must have the same dtype")
-    dt = dtype_to_type_id(Y.dtype)
-    E, C, N, wl = _w_dims(W, w_layout)
-    B, Ey, K, Cy = Y.shape
-    if Cy != C or Ey != E or tuple(Ind.shape) != (B, E, K):
-        raise ValueError(f"shape mismatch: Y{tuple(Y.shape)} W{tuple(W.shape)} Ind{tuple(Ind.shape)} ({w_layout})")
     T = int(T)
-    Yc, Wc = Y.contiguous(), W.contiguous()
-    Ic, it = _index_tensor(Ind)
-    prec, pth = _enums(precision, path)
-    with torch.cuda.device(dev):
-        zero = 1
-        if out is None:
-            out = torch.empty((B, T, N), device=dev, dtype=Y.dtype)
-        else:
-            if tuple(out.shape) != (B, T, N) or out.dtype != Y.dtype or not out.is_contiguous():
-                raise ValueError("out must be a contiguous [B,T,N] tensor of Y's dtype")
-            zero = 0
-        dims = _lib.Dims(B, T, E, K, C, N)
-        ws_bytes = int(lib.egs_scatter_workspace_bytes(B, T, N, dt))
-        ws = torch.empty(ws_bytes // 4, device=dev, dtype=torch.float32) if ws_bytes else None
-        bias_c = _bias_rows(bias, E, N, Y.dtype, dev)
-        if csr is not None:
-            if (csr.B, csr.T, csr.E, csr.K) != (B, T, E, K):
-                raise ValueError("the CSR was built for another Ind shape or T")
-            rc = lib.egs_gemm_scatter_prepared(Yc.data_ptr(), Wc.data_ptr(), bias_c.data_ptr() if bias_c is not None else None,
-                                               Ic.data_ptr(), csr.info.data_ptr(), out.data_ptr(), ctypes.byref(dims), wl, zero,
-                                               dt, it, prec, pth, ws.data_ptr() if ws is not None else None, ws_bytes,
-                                               _status_word(dev).data_ptr(), _stream_ptr(dev))
-        elif bias_c is None:
-            rc = lib.egs_gemm_scatter(Yc.data_ptr(), Wc.data_ptr(), Ic.data_ptr(), out.data_ptr(), ctypes.byref(dims), wl,
-                                      zero, dt, it, prec, pth, ws.data_ptr() if ws is not None else None, ws_bytes,
-                                      _status_word(dev).data_ptr(), _stream_ptr(dev))
-        else:
-            rc = lib.egs_gemm_scatter_bias(Yc.data_ptr(), Wc.data_ptr(), bias_c.data_ptr(), Ic.data_ptr(), out.data_ptr(),
-                                           ctypes.byref(dims), wl, zero, dt, it, prec, pth,
-                                           ws.data_ptr() if ws is not None else None, ws_bytes,
-                                           _status_word(dev).data_ptr(), _stream_ptr(dev))
-    _lib.check(rc, "egs_gemm_scatter")
-    if _state["debug"]:
-        check_status(dev)
-    return out
+    info = None
+    if csr is not None:
+        if Y.dim() != 4 or (csr.B, csr.T, csr.E, csr.K) != (Y.shape[0], T, Y.shape[1], Y.shape[2]):
+            raise ValueError("the CSR was built for another Ind shape or T")
+        info = csr.info
+    return _host().gemm_scatter(Y, W, Ind, T, _layout(w_layout), out, _prec(precision), _path(path), bias, info)
 
 
 def fused_pair_eligible(C1: int, N1: int, N2: int, dtype: torch.dtype, *, w_layout="cn", precision=None) -> bool:
@@ -334,8 +250,7 @@ def fused_pair_eligible(C1: int, N1: int, N2: int, dtype: torch.dtype, *, w_layo
         return False
     lib = _lib.load()
     prec, _ = _enums(precision, None)
-    wl = _lib.W_CN if w_layout == "cn" else _lib.W_NC
-    return bool(lib.egs_fused_pair_eligible(int(C1), int(N1), int(N2), wl, dtype_to_type_id(dtype), prec))
+    return bool(lib.egs_fused_pair_eligible(int(C1), int(N1), int(N2), _layout(w_layout), dtype_to_type_id(dtype), prec))
 
 
 def fused_pair_preferred(X: torch.Tensor, Wg: torch.Tensor, Ind: torch.Tensor) -> bool:
@@ -347,14 +262,7 @@ def fused_pair_preferred(X: torch.Tensor, Wg: torch.Tensor, Ind: torch.Tensor) -
     tensor, but both it and the separate kernels are bound by the bytes the SMs pull from L2 per 128-row tile, and
     the separate gather kernel halves those with 256-row tiles: whole steps measured 2 % faster to 14 % slower with
     the fused kernel (B200, bf16 configurations).  ``gather_scatter_pair`` runs it on request."""
-    if not X.is_cuda or X.dtype != torch.float32:
-        return False
-    I, J = X.shape[2], Wg.shape[2]
-    pair_ctas = Wg.shape[0] * ((X.shape[0] * Ind.shape[2] + 127) // 128)
-    if pair_ctas > _SM_COUNT:
-        return False
-    return (fused_pair_eligible(I, J, I, X.dtype, w_layout="cn")
-            and fused_pair_eligible(I, J, I, X.dtype, w_layout="nc"))
+    return _host().fused_pair_preferred(X, Wg, Ind)
 
 
 def gather_scatter_pair(Src, W1, W2, Ind, *, w_layout="cn", out=None, precision=None):
@@ -364,42 +272,7 @@ def gather_scatter_pair(Src, W1, W2, Ind, *, w_layout="cn", out=None, precision=
     Forward: ``gather_scatter_pair(X, W_g, W_s, Ind)`` -> (Y, Out).  Backward: ``gather_scatter_pair(dOut, W_s, W_g,
     Ind, w_layout="nc")`` -> (dY, dX).  ``out=None`` allocates and zero-fills Dst; a given ``out`` is added to.
     Raises when the shape is not eligible (see :func:`fused_pair_eligible`): callers then use the two operators."""
-    lib = _lib.load()
-    if Src.dim() != 3 or W1.dim() != 3 or W2.dim() != 3 or Ind.dim() != 3:
-        raise ValueError("expected Src[B,T,C1], W1[E,.,.], W2[E,.,.], Ind[B,E,K]")
-    dev = _require_cuda(Src, W1, W2, Ind)
-    if W1.dtype != Src.dtype or W2.dtype != Src.dtype:
-        raise ValueError("Src, W1 and W2 must have the same dtype")
-    dt = dtype_to_type_id(Src.dtype)
-    E, C1, N1, wl = _w_dims(W1, w_layout)
-    E2, N1b, N2, _ = _w_dims(W2, w_layout)
-    B, T, Cx = Src.shape
-    Bi, Ei, K = Ind.shape
-    if Cx != C1 or E2 != E or N1b != N1 or Ei != E or Bi != B:
-        raise ValueError(f"shape mismatch: Src{tuple(Src.shape)} W1{tuple(W1.shape)} W2{tuple(W2.shape)} "
-                         f"Ind{tuple(Ind.shape)} ({w_layout})")
-    Sc, W1c, W2c = Src.contiguous(), W1.contiguous(), W2.contiguous()
-    Ic, it = _index_tensor(Ind)
-    prec, _ = _enums(precision, None)
-    with torch.cuda.device(dev):
-        Mid = torch.empty((B, E, K, N1), device=dev, dtype=Src.dtype)
-        zero = 1
-        if out is None:
-            out = torch.empty((B, T, N2), device=dev, dtype=Src.dtype)
-        else:
-            if tuple(out.shape) != (B, T, N2) or out.dtype != Src.dtype or not out.is_contiguous():
-                raise ValueError("out must be a contiguous [B,T,N2] tensor of Src's dtype")
-            zero = 0
-        ws_bytes = int(lib.egs_scatter_workspace_bytes(B, T, N2, dt))
-        ws = torch.empty(ws_bytes // 4, device=dev, dtype=torch.float32) if ws_bytes else None
-        rc = lib.egs_gather_scatter_pair(Sc.data_ptr(), W1c.data_ptr(), W2c.data_ptr(), Ic.data_ptr(), Mid.data_ptr(),
-                                         out.data_ptr(), B, T, E, K, C1, N1, N2, wl, zero, dt, it, prec,
-                                         ws.data_ptr() if ws is not None else None, ws_bytes,
-                                         _status_word(dev).data_ptr(), _stream_ptr(dev))
-    _lib.check(rc, "egs_gather_scatter_pair")
-    if _state["debug"]:
-        check_status(dev)
-    return Mid, out
+    return _host().gather_scatter_pair(Src, W1, W2, Ind, _layout(w_layout), out, _prec(precision))
 
 
 def dweight(Xsrc, Ysrc, Ind, *, out_layout="gathered_rows", precision=None, path=None, zeroed_out=None):
@@ -407,44 +280,13 @@ def dweight(Xsrc, Ysrc, Ind, *, out_layout="gathered_rows", precision=None, path
     'gathered_rows' returns P [E,FG,FD]; 'direct_rows' returns P^T [E,FD,FG].
     ``zeroed_out``: an output tensor the caller has already zero-filled (float32 only) - the library then skips its
     own fill, which lets a caller issue the fill early, off the critical path."""
-    lib = _lib.load()
-    if Xsrc.dim() != 3 or Ysrc.dim() != 4 or Ind.dim() != 3:
-        raise ValueError("expected Xsrc[B,T,FG], Ysrc[B,E,K,FD], Ind[B,E,K]")
-    dev = _require_cuda(Xsrc, Ysrc, Ind)
-    if Xsrc.dtype != Ysrc.dtype:
-        raise ValueError("Xsrc and Ysrc must have the same dtype")
-    dt = dtype_to_type_id(Xsrc.dtype)
-    B, T, FG = Xsrc.shape
-    By, E, K, FD = Ysrc.shape
-    if By != B or tuple(Ind.shape) != (B, E, K):
-        raise ValueError(f"shape mismatch: Xsrc{tuple(Xsrc.shape)} Ysrc{tuple(Ysrc.shape)} Ind{tuple(Ind.shape)}")
     if out_layout == "gathered_rows":
-        ol, shape = _lib.DW_GATHERED_ROWS, (E, FG, FD)
+        layout = _lib.DW_GATHERED_ROWS
     elif out_layout == "direct_rows":
-        ol, shape = _lib.DW_DIRECT_ROWS, (E, FD, FG)
+        layout = _lib.DW_DIRECT_ROWS
     else:
         raise ValueError("out_layout must be 'gathered_rows' or 'direct_rows'")
-    Xc, Yc = Xsrc.contiguous(), Ysrc.contiguous()
-    Ic, it = _index_tensor(Ind)
-    prec, pth = _enums(precision, path)
-    with torch.cuda.device(dev):
-        fn = lib.egs_dweight
-        if zeroed_out is not None:
-            if (tuple(zeroed_out.shape) != shape or zeroed_out.dtype != torch.float32 or Xsrc.dtype != torch.float32
-                    or not zeroed_out.is_contiguous()):
-                raise ValueError("zeroed_out must be a contiguous float32 tensor of the output's shape")
-            out, fn = zeroed_out, lib.egs_dweight_prezeroed
-        else:
-            out = torch.empty(shape, device=dev, dtype=Xsrc.dtype)
-        ws_bytes = int(lib.egs_dw_workspace_bytes(E, FG, FD, dt))
-        ws = torch.empty(ws_bytes // 4, device=dev, dtype=torch.float32) if ws_bytes else None
-        rc = fn(Xc.data_ptr(), Yc.data_ptr(), Ic.data_ptr(), out.data_ptr(), B, T, E, K, FG, FD, ol, dt, it,
-                             prec, pth, ws.data_ptr() if ws is not None else None, ws_bytes,
-                             _status_word(dev).data_ptr(), _stream_ptr(dev))
-    _lib.check(rc, "egs_dweight")
-    if _state["debug"]:
-        check_status(dev)
-    return out
+    return _host().dweight(Xsrc, Ysrc, Ind, layout, _prec(precision), _path(path), zeroed_out)
 
 
 def describe_plan(op: str, B, T, E, K, C, N, dtype, *, w_layout="cn", precision=None) -> dict:
@@ -467,19 +309,7 @@ def route_topk(scores: torch.Tensor, K: int, *, index_dtype: torch.dtype = torch
     """Expert-choice routing on the device: ``scores`` [B,T,E] -> ``Ind`` [B,E,K], for every (b, e) the K tokens with the
     highest score, best first (equal scores: lower token id first).  K <= min(T, 1024).  The producer of the ``Ind`` the
     gather and scatter modules take; the reference has none (its tests draw Ind at random, ``test_all.py:16``)."""
-    lib = _lib.load()
-    if scores.dim() != 3:
-        raise ValueError("expected scores[B,T,E]")
-    dev = _require_cuda(scores)
-    if index_dtype not in _TORCH_INDEX:
-        raise ValueError("index_dtype must be int64, int32 or int16")
-    B, T, E = scores.shape
-    sc = scores.float().contiguous()
-    with torch.cuda.device(dev):
-        Ind = torch.empty((B, E, int(K)), device=dev, dtype=index_dtype)
-        rc = lib.egs_route_topk(sc.data_ptr(), Ind.data_ptr(), B, T, E, int(K), _TORCH_INDEX[index_dtype], _stream_ptr(dev))
-    _lib.check(rc, "egs_route_topk")
-    return Ind
+    return _host().route_topk(scores, int(K), index_dtype)
 
 
 class IndexCSR:
@@ -500,23 +330,9 @@ class IndexCSR:
 def build_index_csr(Ind: torch.Tensor, T: int) -> IndexCSR:
     """Counting sort of the routed slots by token row (see :class:`IndexCSR`).  Build it once per step: it serves both
     scatters of the step (``gemm_scatter(..., csr=...)`` skips its own counting pass) and :func:`gemm_scatter_csr`."""
-    lib = _lib.load()
-    if Ind.dim() != 3:
-        raise ValueError("expected Ind[B,E,K]")
-    dev = _require_cuda(Ind)
-    B, E, K = Ind.shape
     T = int(T)
-    Ic, it = _index_tensor(Ind)
-    with torch.cuda.device(dev):
-        counts = torch.empty(B * T, device=dev, dtype=torch.int32)
-        offsets = torch.empty(B * T + 1, device=dev, dtype=torch.int32)
-        entries = torch.empty(B * E * K, device=dev, dtype=torch.int32)
-        info = torch.empty(4, device=dev, dtype=torch.int32)
-        sb = int(lib.egs_index_csr_scratch_bytes(B, T))
-        scratch = torch.empty((sb + 3) // 4, device=dev, dtype=torch.int32)
-        rc = lib.egs_index_csr(Ic.data_ptr(), it, B, T, E, K, counts.data_ptr(), offsets.data_ptr(), entries.data_ptr(),
-                               info.data_ptr(), scratch.data_ptr(), sb, _stream_ptr(dev))
-    _lib.check(rc, "egs_index_csr")
+    counts, offsets, entries, info = _host().build_index_csr(Ind, T)
+    B, E, K = Ind.shape
     return IndexCSR(counts, offsets, entries, info, B, T, E, K)
 
 

@@ -14,10 +14,15 @@ import math
 import torch
 from torch import nn
 
+from . import ops
 from .kernels import (ExpertGatherBiasFunction, ExpertGatherFunction, ExpertGatherScatterFunction, ExpertScatterBiasFunction,
                       ExpertScatterFunction, create_kernels)
 
 __all__ = ["ExpertGather", "ExpertScatter", "ExpertGatherScatter"]
+
+# Eager calls go to the native autograd functions of csrc/egs_host.cpp.  They return None for tensors they do not take (fake
+# tensors, tensor subclasses, functorch wrappers); those, and traced calls, run the Python functions of kernels.py.
+_tracing = torch.compiler.is_compiling
 
 
 class ExpertGather(nn.Module):
@@ -44,6 +49,10 @@ class ExpertGather(nn.Module):
             nn.init.uniform_(self.bias, -bound, bound)
 
     def forward(self, x: torch.Tensor, Ind: torch.Tensor) -> torch.Tensor:
+        if not _tracing():
+            y = ops._host().gather_autograd(x, self.W, self.bias, Ind)
+            if y is not None:
+                return y
         if self.bias is not None:
             # y + bias ([E,1,J] broadcast over batch and slot, the reference's expression at :55-56), fused into the kernel
             return ExpertGatherBiasFunction.apply(x, self.W, self.bias, Ind)
@@ -84,6 +93,11 @@ class ExpertScatter(nn.Module):
             nn.init.uniform_(self.bias, -bound, bound)
 
     def forward(self, Y: torch.Tensor, Ind: torch.Tensor, T: int) -> torch.Tensor:
+        if not _tracing():
+            per_slot = self.bias if self.bias_mode == "per_slot" else None
+            out = ops._host().scatter_autograd(Y, self.W, per_slot, Ind, int(T))
+            if out is not None:
+                return out if self.bias is None or per_slot is not None else out + self.bias
         if self.bias is not None and self.bias_mode == "per_slot":
             return ExpertScatterBiasFunction.apply(Y, self.W, self.bias, Ind, T)
         out = ExpertScatterFunction.apply(Y, self.W, Ind, T)
@@ -111,4 +125,8 @@ class ExpertGatherScatter(nn.Module):
     def forward(self, x: torch.Tensor, Ind: torch.Tensor) -> torch.Tensor:
         if self.gather.bias is not None or self.scatter.bias is not None:
             return self.scatter(self.gather(x, Ind), Ind, x.shape[1])
+        if not _tracing():
+            out = ops._host().gather_scatter_autograd(x, self.gather.W, self.scatter.W, Ind)
+            if out is not None:
+                return out
         return ExpertGatherScatterFunction.apply(x, self.gather.W, self.scatter.W, Ind)

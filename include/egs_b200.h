@@ -77,6 +77,14 @@ const char* egs_status_string(int code);
 const char* egs_last_cuda_error(void);
 
 /*
+ * Registers a host mirror for a status word: kernels that report invalid results (EGS_STATUS_PIPELINE_TIMEOUT,
+ * EGS_STATUS_INTERNAL) on this word also store the bits there, so that the host sees them without a copy.  host_mirror is
+ * mapped (pinned) host memory the device can write, or NULL to stop mirroring.  At most 64 status words have a mirror
+ * (EGS_ERR_TOO_LARGE beyond).  Neither pointer is touched here; both must outlive the launches that follow.
+ */
+int egs_set_status_mirror(int32_t* status_word, int32_t* host_mirror);
+
+/*
  * Operator G:  Y[b,e,k,n] = sum_c X[b, Ind[b,e,k], c] * W(e,c,n)
  * Replaces expert_gather_kernel + its launch wrappers:
  *   gather forward       egs/triton_kernels.py:367-392  (X=X, W=W_g [E,I,J], w_layout=EGS_W_CN, C=I, N=J)
