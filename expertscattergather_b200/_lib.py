@@ -30,7 +30,7 @@ EXPORTS = (
     "egs_gather_scatter_pair", "egs_fused_pair_eligible", "egs_dweight_prezeroed", "egs_selftest_wait_timeout",
     "egs_describe_plan", "egs_gather_gemm_bias", "egs_gemm_scatter_bias", "egs_route_topk", "egs_index_csr",
     "egs_index_csr_scratch_bytes", "egs_index_compact", "egs_gemm_scatter_prepared", "egs_gemm_scatter_csr",
-    "egs_set_status_mirror",
+    "egs_set_status_mirror", "egs_expert_row_sum",
 )
 
 
@@ -96,6 +96,8 @@ def _declare(lib: ctypes.CDLL) -> None:
     lib.egs_describe_plan.argtypes = [i, ctypes.POINTER(Dims), i, i, i, ctypes.POINTER(PlanInfo)]
     lib.egs_set_status_mirror.restype = i
     lib.egs_set_status_mirror.argtypes = [vp, vp]
+    lib.egs_expert_row_sum.restype = i
+    lib.egs_expert_row_sum.argtypes = [vp, vp, vp, i64, i64, i64, i64, i64, i, i, vp, vp]
     lib.egs_fill_zero.restype = i
     lib.egs_fill_zero.argtypes = [vp, sz, vp]
     lib.egs_launch_count.restype = i64

@@ -486,16 +486,7 @@ static int dweight_impl(const void* Xsrc, const void* Ysrc, const void* Ind, voi
   if (tensor) {
     smem = configure_tensor_dweight(p, dtype, precision);
   } else {
-    // generic kernel: 64x64 tiles, contraction split so that the grid covers the SMs about twice
-    const long long tiles = ((FG + 63) / 64) * ((FD + 63) / 64) * E;
-    long long want = (2 * 148 + tiles - 1) / tiles;
-    const long long max_splits = (p.M + 15) / 16;
-    if (want > max_splits) want = max_splits;
-    if (want < 1) want = 1;
-    long long rows = (p.M + want - 1) / want;
-    rows = (rows + 15) / 16 * 16;
-    p.rows_per_split = static_cast<int>(rows);
-    p.splits = static_cast<int>((p.M + rows - 1) / rows);
+    configure_generic_dweight(p);
   }
   if (static_cast<long long>(p.E) * p.splits > 65535) return EGS_ERR_TOO_LARGE;   // grid.z limit
 
@@ -617,6 +608,24 @@ int egs_tensor_path_eligible(int op, const egs_dims* dims, int dtype, const void
   for (int i = 0; i < n_pointers; ++i)
     if (pointers && pointers[i] && !aligned16(pointers[i])) return 0;
   return 1;
+}
+
+int egs_expert_row_sum(const void* Src, const void* Ind, void* out, int64_t B, int64_t T, int64_t E, int64_t K, int64_t N, int dtype,
+                       int index_dtype, int32_t* status_word, void* cuda_stream) {
+  egs_dims d{B, T, E, K, 0, N};
+  if (int rc = check_dims(&d)) return rc;
+  if (!valid_dtype(dtype) || (Ind && !valid_index(index_dtype))) return EGS_ERR_INVALID_ARGUMENT;
+  if (E * N == 0) return EGS_OK;
+  if (!out) return EGS_ERR_INVALID_ARGUMENT;
+  cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
+  if (B * K == 0) {
+    cudaError_t err = launch_fill_zero(out, static_cast<size_t>(E) * N * elem_size(dtype), st);
+    return err == cudaSuccess ? EGS_OK : fail_cuda(err, "fill_zero");
+  }
+  if (!Src) return EGS_ERR_INVALID_ARGUMENT;
+  cudaError_t err = launch_expert_row_sum(Src, Ind, index_dtype, out, static_cast<int>(B), static_cast<int>(T), static_cast<int>(E),
+                                          static_cast<int>(K), static_cast<int>(N), dtype, status_ref(status_word), st);
+  return err == cudaSuccess ? EGS_OK : fail_cuda(err, "expert_row_sum launch");
 }
 
 int egs_fill_zero(void* p, size_t n_bytes, void* cuda_stream) {

@@ -9,29 +9,38 @@ namespace egs {
 
 namespace {
 
-constexpr int TM = 64;       // output tile rows
-constexpr int TN = 64;       // output tile columns
-constexpr int TK = 16;       // contraction step
-constexpr int PAD = 4;
-constexpr int NTHREADS = 256;  // 16 x 16 threads, 4 x 4 outputs each
+// Both kernels: 128 threads as 16 (ty) x 8 (tx), operands converted to float32 in shared memory, contraction steps of 32.
+// What bounds them is the chain of a step - load, barrier, multiply - so the next step's elements are fetched into registers
+// while the current one is multiplied, lanes run along the contiguous direction of every row (whole 128-byte segments), and
+// several CTAs share an SM.  Results leave through shared memory for the same reason: rows are written (or added to) 32
+// consecutive elements per instruction.  Tile widths are multiples of 32 chosen on the host so that little of a tile is
+// padding: the widths that come here are mostly odd and below 128.
+// 54855 routed rows, 83 -> 29 features, float32 (gather): 45 us with the former 64x64x16 tiles without prefetch.
+constexpr int NTHREADS = 128;
+constexpr int TM = 64;          // rows per CTA of the row kernel
+constexpr int TK = 32;          // contraction step
+constexpr int APITCH = TK + 4;  // floats; rows 16-byte aligned, consecutive rows 4 banks apart
 
 // ------------------------------------------------------------------------------------------------
 // G and S:  tile[m, n] = sum_c A[row_a(m), c] * W(e, c, n);   G stores it, S adds it atomically
 // (operator G: egs/triton_kernels.py:48-143, operator S: :156-247 in the reference)
+// NJ: tile width in units of 32 columns.  Thread (ty, tx) owns rows ty + 16 i and columns 32 j + 4 tx .. + 3.
 // ------------------------------------------------------------------------------------------------
-template <typename T, bool SCATTER>
-__global__ void __launch_bounds__(NTHREADS) generic_rowgemm_kernel(RowGemmParams p) {
-  __shared__ float As[TK][TM + PAD];
-  __shared__ float Bs[TK][TN + PAD];
+template <typename T, bool SCATTER, int NJ>
+__global__ void __launch_bounds__(NTHREADS, NJ == 4 ? 3 : 4) generic_rowgemm_kernel(RowGemmParams p) {
+  constexpr int BN = 32 * NJ, BPITCH = BN + 4;
+  __shared__ __align__(16) float As[TM * APITCH];
+  __shared__ __align__(16) float Bs[TK * BPITCH];
   __shared__ long long row_a[TM];   // element offset of the A row, -1 when masked
   __shared__ long long row_o[TM];   // element offset of the output row, -1 when masked
 
   const int e = blockIdx.z;
   const int m0 = blockIdx.x * TM;
-  const int n0 = blockIdx.y * TN;
-  const int tid = threadIdx.x;
+  const int n0 = blockIdx.y * BN;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tx = tid & 7, ty = tid >> 3;
   const T* __restrict__ A = static_cast<const T*>(p.A);
-  const T* __restrict__ W = static_cast<const T*>(p.W);
+  const T* __restrict__ W = static_cast<const T*>(p.W) + static_cast<long long>(e) * p.C * p.N;
   T* __restrict__ Out = static_cast<T*>(p.Out);
 
   if (tid < TM) {
@@ -55,158 +64,325 @@ __global__ void __launch_bounds__(NTHREADS) generic_rowgemm_kernel(RowGemmParams
   }
   __syncthreads();
 
-  const int tx = tid & 15, ty = tid >> 4;
-  float acc[4][4] = {};
-  const long long wbase = static_cast<long long>(e) * p.C * p.N;
-
-  for (int c0 = 0; c0 < p.C; c0 += TK) {
+  float ra[TM / 4], rb[8 * NJ];
+  auto fetch = [&](int c0) {
+    const int c = c0 + lane;
 #pragma unroll
-    for (int i = 0; i < (TM * TK) / NTHREADS; ++i) {
-      const int idx = tid + i * NTHREADS;
-      const int kk = idx & (TK - 1), m = idx >> 4;
-      const long long ra = row_a[m];
-      const int c = c0 + kk;
-      As[kk][m] = (ra >= 0 && c < p.C) ? to_f32<T>(A[ra + c]) : 0.f;
+    for (int i = 0; i < TM / 4; ++i) {
+      const long long off = row_a[warp + 4 * i];
+      ra[i] = (off >= 0 && c < p.C) ? to_f32<T>(A[off + c]) : 0.f;
     }
     if (p.w_layout == EGS_W_CN) {
 #pragma unroll
-      for (int i = 0; i < (TN * TK) / NTHREADS; ++i) {
-        const int idx = tid + i * NTHREADS;
-        const int n = idx & (TN - 1), kk = idx >> 6;
-        const int c = c0 + kk, nn = n0 + n;
-        Bs[kk][n] = (c < p.C && nn < p.N) ? to_f32<T>(W[wbase + static_cast<long long>(c) * p.N + nn]) : 0.f;
+      for (int i = 0; i < 8; ++i) {
+        const int cc = c0 + warp + 4 * i;
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          const int n = n0 + 32 * j + lane;
+          rb[i * NJ + j] = (cc < p.C && n < p.N) ? to_f32<T>(W[static_cast<long long>(cc) * p.N + n]) : 0.f;
+        }
       }
     } else {
 #pragma unroll
-      for (int i = 0; i < (TN * TK) / NTHREADS; ++i) {
-        const int idx = tid + i * NTHREADS;
-        const int kk = idx & (TK - 1), n = idx >> 4;
-        const int c = c0 + kk, nn = n0 + n;
-        Bs[kk][n] = (c < p.C && nn < p.N) ? to_f32<T>(W[wbase + static_cast<long long>(nn) * p.C + c]) : 0.f;
+      for (int i = 0; i < 8 * NJ; ++i) {
+        const int n = n0 + warp + 4 * i;
+        rb[i] = (c < p.C && n < p.N) ? to_f32<T>(W[static_cast<long long>(n) * p.C + c]) : 0.f;
       }
     }
+  };
+  auto stage = [&]() {
+#pragma unroll
+    for (int i = 0; i < TM / 4; ++i) As[(warp + 4 * i) * APITCH + lane] = ra[i];
+    if (p.w_layout == EGS_W_CN) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) Bs[(warp + 4 * i) * BPITCH + 32 * j + lane] = rb[i * NJ + j];
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8 * NJ; ++i) Bs[lane * BPITCH + warp + 4 * i] = rb[i];
+    }
+  };
+
+  float acc[4][4 * NJ] = {};
+  fetch(0);
+  for (int c0 = 0; c0 < p.C; c0 += TK) {
+    stage();
     __syncthreads();
+    if (c0 + TK < p.C) fetch(c0 + TK);
+#pragma unroll 1
+    for (int kk = 0; kk < TK; kk += 4) {
+      if (c0 + kk >= p.C) break;
+      float4 a[4];
 #pragma unroll
-    for (int kk = 0; kk < TK; ++kk) {
-      float a[4], b[4];
+      for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(&As[(ty + 16 * i) * APITCH + kk]);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
+      for (int q = 0; q < 4; ++q) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
+        for (int j = 0; j < NJ; ++j) {
+          const float4 b = *reinterpret_cast<const float4*>(&Bs[(kk + q) * BPITCH + 32 * j + 4 * tx]);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+          for (int i = 0; i < 4; ++i) {
+            const float av = q == 0 ? a[i].x : q == 1 ? a[i].y : q == 2 ? a[i].z : a[i].w;
+            acc[i][4 * j] = fmaf(av, b.x, acc[i][4 * j]);
+            acc[i][4 * j + 1] = fmaf(av, b.y, acc[i][4 * j + 1]);
+            acc[i][4 * j + 2] = fmaf(av, b.z, acc[i][4 * j + 2]);
+            acc[i][4 * j + 3] = fmaf(av, b.w, acc[i][4 * j + 3]);
+          }
+        }
+      }
     }
     __syncthreads();
   }
 
+  // 32 columns at a time through As: lanes then cover 32 consecutive elements of one row
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const long long ro = row_o[ty * 4 + i];
-    if (ro < 0) continue;
+  for (int j = 0; j < NJ; ++j) {
+    if (n0 + 32 * j >= p.N) break;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int nn = n0 + tx * 4 + j;
-      if (nn >= p.N) continue;
-      const float v = acc[i][j] + (p.bias ? to_f32<T>(static_cast<const T*>(p.bias)[static_cast<long long>(e) * p.N + nn]) : 0.f);
-      if (SCATTER) {
-        if (sizeof(T) == 2) atomicAdd(p.acc + ro + nn, v);   // 16-bit: float32 accumulation rows
-        else atomicAdd(reinterpret_cast<float*>(Out) + ro + nn, v);
-      } else {
-        Out[ro + nn] = from_f32<T>(v);
+    for (int i = 0; i < 4; ++i)
+      *reinterpret_cast<float4*>(&As[(ty + 16 * i) * APITCH + 4 * tx]) =
+          make_float4(acc[i][4 * j], acc[i][4 * j + 1], acc[i][4 * j + 2], acc[i][4 * j + 3]);
+    __syncthreads();
+    const int n = n0 + 32 * j + lane;
+    if (n < p.N) {
+      const float bias = p.bias ? to_f32<T>(static_cast<const T*>(p.bias)[static_cast<long long>(e) * p.N + n]) : 0.f;
+#pragma unroll 4
+      for (int r = warp; r < TM; r += 4) {
+        const long long ro = row_o[r];
+        if (ro < 0) continue;
+        const float v = As[r * APITCH + lane] + bias;
+        if (SCATTER) {
+          if (sizeof(T) == 2) atomicAdd(p.acc + ro + n, v);   // 16-bit: float32 accumulation rows
+          else atomicAdd(reinterpret_cast<float*>(Out) + ro + n, v);
+        } else {
+          Out[ro + n] = from_f32<T>(v);
+        }
       }
     }
+    __syncthreads();
   }
 }
 
 // ------------------------------------------------------------------------------------------------
 // D:  P[e, f, g] = sum_m Xsrc[token row(m), f] * Ysrc[slot row(m), g]
 // (operator D: egs/triton_kernels.py:261-356 in the reference)
+// FI, GJ: tile size in units of 32 gathered / direct features.  Thread (ty, tx) owns features f = 32 i + 2 ty + {0, 1} and
+// g = 32 j + 4 tx .. + 3.  A tile is summed over `rows_per_split` rows and added to the float32 result where there are several.
 // ------------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(NTHREADS) generic_dweight_kernel(DWeightParams p) {
-  __shared__ float As[TK][TM + PAD];
-  __shared__ float Bs[TK][TN + PAD];
-  __shared__ long long row_g[TK];
-  __shared__ long long row_d[TK];
+constexpr int kRowTable = 256;   // rows whose offsets are looked up at a time
+template <typename T, int FI, int GJ>
+__global__ void __launch_bounds__(NTHREADS, FI * GJ > 4 ? 3 : 4) generic_dweight_kernel(DWeightParams p) {
+  constexpr int FP = 32 * FI + 4, GP = 32 * GJ + 4, XP = 33;
+  constexpr int kTile = TK * (FP + GP) > 32 * XP ? TK * (FP + GP) : 32 * XP;
+  __shared__ __align__(16) float tile[kTile];
+  __shared__ long long row_g[kRowTable];
+  __shared__ long long row_d[kRowTable];
+  float* Fs = tile;
+  float* Gs = tile + TK * FP;
 
   const int e = blockIdx.z / p.splits;
   const int split = blockIdx.z - e * p.splits;
-  const int f0 = blockIdx.x * TM;
-  const int g0 = blockIdx.y * TN;
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
+  const int f0 = blockIdx.x * 32 * FI;
+  const int g0 = blockIdx.y * 32 * GJ;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tx = tid & 7, ty = tid >> 3;
   const T* __restrict__ Xs = static_cast<const T*>(p.Xsrc);
   const T* __restrict__ Ys = static_cast<const T*>(p.Ysrc);
 
   const int m_begin = split * p.rows_per_split;
   const int m_end = min(p.M, m_begin + p.rows_per_split);
-  float acc[4][4] = {};
+  float acc[2 * FI][4 * GJ] = {};
+  float rf[8 * FI], rg[8 * GJ];
+  auto fetch = [&](int r0) {       // r0: first row of the step within the table
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const long long og = row_g[r0 + warp + 4 * k], od = row_d[r0 + warp + 4 * k];
+#pragma unroll
+      for (int i = 0; i < FI; ++i) {
+        const int f = f0 + 32 * i + lane;
+        rf[k * FI + i] = (og >= 0 && f < p.FG) ? to_f32<T>(Xs[og + f]) : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < GJ; ++j) {
+        const int g = g0 + 32 * j + lane;
+        rg[k * GJ + j] = (od >= 0 && g < p.FD) ? to_f32<T>(Ys[od + g]) : 0.f;
+      }
+    }
+  };
 
-  for (int mc = m_begin; mc < m_end; mc += TK) {
-    if (tid < TK) {
-      const int m = mc + tid;
-      long long rg = -1, rd = -1;
+  for (int mt = m_begin; mt < m_end; mt += kRowTable) {
+    __syncthreads();
+    for (int i = tid; i < kRowTable; i += NTHREADS) {
+      const int m = mt + i;
+      long long og = -1, od = -1;
       if (m < m_end) {
         const int b = m / p.K, k = m - b * p.K;
         const long long slot = (static_cast<long long>(b) * p.E + e) * p.K + k;
         const long long t = load_index(p.Ind, p.index_dtype, slot);
         if (t >= 0 && t < p.T) {
-          rg = (static_cast<long long>(b) * p.T + t) * p.FG;
-          rd = slot * p.FD;
+          og = (static_cast<long long>(b) * p.T + t) * p.FG;
+          od = slot * p.FD;
         } else {
           p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
         }
       }
-      row_g[tid] = rg;
-      row_d[tid] = rd;
+      row_g[i] = og;
+      row_d[i] = od;
     }
     __syncthreads();
+    const int nrows = min(kRowTable, m_end - mt);
+    fetch(0);
+    for (int r0 = 0; r0 < nrows; r0 += TK) {
 #pragma unroll
-    for (int i = 0; i < (TM * TK) / NTHREADS; ++i) {
-      const int idx = tid + i * NTHREADS;
-      const int f = idx & (TM - 1), kk = idx >> 6;
-      const long long rg = row_g[kk];
-      As[kk][f] = (rg >= 0 && f0 + f < p.FG) ? to_f32<T>(Xs[rg + f0 + f]) : 0.f;
-      const long long rd = row_d[kk];
-      Bs[kk][f] = (rd >= 0 && g0 + f < p.FD) ? to_f32<T>(Ys[rd + g0 + f]) : 0.f;
+      for (int k = 0; k < 8; ++k) {
+#pragma unroll
+        for (int i = 0; i < FI; ++i) Fs[(warp + 4 * k) * FP + 32 * i + lane] = rf[k * FI + i];
+#pragma unroll
+        for (int j = 0; j < GJ; ++j) Gs[(warp + 4 * k) * GP + 32 * j + lane] = rg[k * GJ + j];
+      }
+      __syncthreads();
+      if (r0 + TK < nrows) fetch(r0 + TK);
+#pragma unroll 4
+      for (int kk = 0; kk < TK; ++kk) {
+        float2 a[FI];
+        float4 b[GJ];
+#pragma unroll
+        for (int i = 0; i < FI; ++i) a[i] = *reinterpret_cast<const float2*>(&Fs[kk * FP + 32 * i + 2 * ty]);
+#pragma unroll
+        for (int j = 0; j < GJ; ++j) b[j] = *reinterpret_cast<const float4*>(&Gs[kk * GP + 32 * j + 4 * tx]);
+#pragma unroll
+        for (int i = 0; i < FI; ++i)
+#pragma unroll
+          for (int j = 0; j < GJ; ++j) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const float av = u ? a[i].y : a[i].x;
+              acc[2 * i + u][4 * j] = fmaf(av, b[j].x, acc[2 * i + u][4 * j]);
+              acc[2 * i + u][4 * j + 1] = fmaf(av, b[j].y, acc[2 * i + u][4 * j + 1]);
+              acc[2 * i + u][4 * j + 2] = fmaf(av, b[j].z, acc[2 * i + u][4 * j + 2]);
+              acc[2 * i + u][4 * j + 3] = fmaf(av, b[j].w, acc[2 * i + u][4 * j + 3]);
+            }
+          }
+      }
+      __syncthreads();
     }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < TK; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
   }
 
+  // 32 x 32 blocks through shared memory, lanes along the contiguous direction of the output
   T* __restrict__ out = static_cast<T*>(p.out);
+  const bool fg = p.out_layout == EGS_DW_GATHERED_ROWS;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int f = f0 + ty * 4 + i;
-    if (f >= p.FG) continue;
+  for (int i = 0; i < FI; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int g = g0 + tx * 4 + j;
-      if (g >= p.FD) continue;
-      const long long off = (p.out_layout == EGS_DW_GATHERED_ROWS)
-                                ? (static_cast<long long>(e) * p.FG + f) * p.FD + g
-                                : (static_cast<long long>(e) * p.FD + g) * p.FG + f;
-      if (p.splits > 1) {
-        atomicAdd(p.acc + off, acc[i][j]);
-      } else {
-        out[off] = from_f32<T>(acc[i][j]);
+    for (int j = 0; j < GJ; ++j) {
+      if (f0 + 32 * i >= p.FG || g0 + 32 * j >= p.FD) continue;
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) tile[(2 * ty + u) * XP + 4 * tx + v] = acc[2 * i + u][4 * j + v];
+      __syncthreads();
+#pragma unroll
+      for (int r = warp; r < 32; r += 4) {
+        const int f = f0 + 32 * i + (fg ? r : lane), g = g0 + 32 * j + (fg ? lane : r);
+        if (f < p.FG && g < p.FD) {
+          const float v = fg ? tile[r * XP + lane] : tile[lane * XP + r];
+          const long long off = fg ? (static_cast<long long>(e) * p.FG + f) * p.FD + g : (static_cast<long long>(e) * p.FD + g) * p.FG + f;
+          if (p.splits > 1) atomicAdd(p.acc + off, v);
+          else out[off] = from_f32<T>(v);
+        }
       }
     }
+}
+
+// ------------------------------------------------------------------------------------------------
+// Row sums per expert (the bias gradients):  out[e, n] = sum over the slots of expert e of row[n] of a token row (through Ind)
+// or of the slot row itself (Ind == NULL).  Eight lanes cover 128 bytes of a row; a cluster of CTAs shares the rows of one
+// (expert, 128-byte column block) and adds its partial sums through distributed shared memory, so that there is neither a
+// scratch buffer nor a second pass and the order of the additions is fixed.  Memory-bound: four rows in flight per thread.
+// 65536 routed rows of 768 bf16 features: 40 us as the weight-gradient contraction against ones, 26 us as a library reduction
+// of 192 features.
+// ------------------------------------------------------------------------------------------------
+constexpr int kSumThreads = 256;
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(kSumThreads) expert_row_sum_kernel(const T* __restrict__ Src, const void* __restrict__ Ind,
+                                                                     int index_dtype, T* __restrict__ out, int T_, int E, int K, int N,
+                                                                     int M, StatusRef status) {
+  constexpr int PER = VEC ? 16 / static_cast<int>(sizeof(T)) : 1;   // columns per lane
+  constexpr int COLS = 8 * PER;                                     // columns per CTA
+  constexpr int ROWS = kSumThreads / 8;                             // rows a CTA reads at a time
+  __shared__ float part[ROWS][COLS + 1];
+  __shared__ float total[COLS];
+  const int rank = blockIdx.x, nranks = gridDim.x;                  // the cluster spans gridDim.x
+  const int e = blockIdx.z, c0 = blockIdx.y * COLS;
+  const int tid = threadIdx.x, cl = tid & 7, rl = tid >> 3;
+  const int col = c0 + cl * PER;
+  const int per = (M + nranks - 1) / nranks, m_end = min(M, (rank + 1) * per);
+  float acc[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) acc[i] = 0.f;
+  constexpr int U = 4;
+  for (int m0 = rank * per + rl; m0 < m_end; m0 += U * ROWS) {
+    long long row[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int m = m0 + u * ROWS;
+      row[u] = -1;
+      if (m < m_end) {
+        const int b = m / K, k = m - b * K;
+        const long long slot = (static_cast<long long>(b) * E + e) * K + k;
+        row[u] = slot;
+        if (Ind) {
+          const long long t = load_index(Ind, index_dtype, slot);
+          if (t >= 0 && t < T_) {
+            row[u] = static_cast<long long>(b) * T_ + t;
+          } else {
+            row[u] = -1;
+            status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
+          }
+        }
+      }
+    }
+    if (VEC) {
+      uint4 x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        x[u] = (row[u] >= 0 && col < N) ? *reinterpret_cast<const uint4*>(Src + row[u] * N + col) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const T* v = reinterpret_cast<const T*>(&x[u]);
+#pragma unroll
+        for (int i = 0; i < PER; ++i) acc[i] += to_f32<T>(v[i]);
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (row[u] >= 0 && col < N) acc[0] += to_f32<T>(Src[row[u] * N + col]);
+    }
   }
+#pragma unroll
+  for (int i = 0; i < PER; ++i) part[rl][cl * PER + i] = acc[i];
+  __syncthreads();
+  if (tid < COLS) {
+    float s = 0.f;
+    for (int r = 0; r < ROWS; ++r) s += part[r][tid];
+    total[tid] = s;
+  }
+  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+  if (rank == 0 && tid < COLS && c0 + tid < N) {
+    float s = 0.f;
+    const uint32_t mine = static_cast<uint32_t>(__cvta_generic_to_shared(&total[tid]));
+    for (int r = 0; r < nranks; ++r) {
+      uint32_t addr;
+      float v;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(mine), "r"(r));
+      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+      s += v;
+    }
+    out[static_cast<long long>(e) * N + c0 + tid] = from_f32<T>(s);
+  }
+  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");   // nobody's shared memory goes before it is read
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -320,30 +496,118 @@ int grid_for(size_t work_items, int per_block) {
 
 }  // namespace
 
+// Tile width over n features in units of 32, at most `most`: the least padding, the widest of equals.
+static int width_in_32s(int n, int most) {
+  int best = 1, best_pad = 1 << 30;
+  for (int w = 1; w <= most; ++w) {
+    const int tile = 32 * w, pad = (n + tile - 1) / tile * tile - n;
+    if (pad <= best_pad) {
+      best = w;
+      best_pad = pad;
+    }
+  }
+  return best;
+}
+
 cudaError_t launch_generic_rowgemm(const RowGemmParams& p, bool scatter, int dtype, cudaStream_t st) {
-  dim3 grid((p.M + TM - 1) / TM, (p.N + TN - 1) / TN, p.E);
-  dim3 block(NTHREADS);
-#define EGS_LAUNCH(TY)                                                            \
-  do {                                                                            \
-    if (scatter) generic_rowgemm_kernel<TY, true><<<grid, block, 0, st>>>(p);     \
-    else generic_rowgemm_kernel<TY, false><<<grid, block, 0, st>>>(p);            \
+  const int nj = width_in_32s(p.N, 4);
+  dim3 grid((p.M + TM - 1) / TM, (p.N + 32 * nj - 1) / (32 * nj), p.E);
+#define EGS_LAUNCH_NJ(TY, NJV)                                                             \
+  do {                                                                                     \
+    if (scatter) generic_rowgemm_kernel<TY, true, NJV><<<grid, NTHREADS, 0, st>>>(p);      \
+    else generic_rowgemm_kernel<TY, false, NJV><<<grid, NTHREADS, 0, st>>>(p);             \
+  } while (0)
+#define EGS_LAUNCH(TY)                       \
+  do {                                       \
+    if (nj == 1) EGS_LAUNCH_NJ(TY, 1);       \
+    else if (nj == 2) EGS_LAUNCH_NJ(TY, 2);  \
+    else if (nj == 3) EGS_LAUNCH_NJ(TY, 3);  \
+    else EGS_LAUNCH_NJ(TY, 4);               \
   } while (0)
   if (dtype == EGS_F32) EGS_LAUNCH(float);
   else if (dtype == EGS_F16) EGS_LAUNCH(__half);
   else EGS_LAUNCH(__nv_bfloat16);
 #undef EGS_LAUNCH
+#undef EGS_LAUNCH_NJ
   count_launch();
   return cudaGetLastError();
 }
 
+// Tile over FG x FD and the split of the contraction: about four CTAs per SM, and no fewer than 64 rows in a range, below which
+// adding the partial tile costs more than multiplying it.
+void configure_generic_dweight(DWeightParams& p) {
+  p.row_tiles = width_in_32s(p.FG, 4);
+  p.BN = 32 * width_in_32s(p.FD, 2);
+  const long long tiles = static_cast<long long>((p.FG + 32 * p.row_tiles - 1) / (32 * p.row_tiles)) * ((p.FD + p.BN - 1) / p.BN) * p.E;
+  long long want = (4 * 148 + tiles - 1) / tiles;
+  const long long most = (p.M + 63) / 64;
+  if (want > most) want = most;
+  if (want < 1) want = 1;
+  long long rows = (p.M + want - 1) / want;
+  rows = (rows + TK - 1) / TK * TK;
+  p.rows_per_split = static_cast<int>(rows);
+  p.splits = static_cast<int>((p.M + rows - 1) / rows);
+}
+
 cudaError_t launch_generic_dweight(const DWeightParams& p, int dtype, cudaStream_t st) {
-  dim3 grid((p.FG + TM - 1) / TM, (p.FD + TN - 1) / TN, p.E * p.splits);
-  dim3 block(NTHREADS);
-  if (dtype == EGS_F32) generic_dweight_kernel<float><<<grid, block, 0, st>>>(p);
-  else if (dtype == EGS_F16) generic_dweight_kernel<__half><<<grid, block, 0, st>>>(p);
-  else generic_dweight_kernel<__nv_bfloat16><<<grid, block, 0, st>>>(p);
+  const int fi = p.row_tiles, gj = p.BN / 32;
+  dim3 grid((p.FG + 32 * fi - 1) / (32 * fi), (p.FD + p.BN - 1) / p.BN, p.E * p.splits);
+#define EGS_LAUNCH_FI(TY, FIV)                                                           \
+  do {                                                                                   \
+    if (gj == 1) generic_dweight_kernel<TY, FIV, 1><<<grid, NTHREADS, 0, st>>>(p);       \
+    else generic_dweight_kernel<TY, FIV, 2><<<grid, NTHREADS, 0, st>>>(p);               \
+  } while (0)
+#define EGS_LAUNCH(TY)                       \
+  do {                                       \
+    if (fi == 1) EGS_LAUNCH_FI(TY, 1);       \
+    else if (fi == 2) EGS_LAUNCH_FI(TY, 2);  \
+    else if (fi == 3) EGS_LAUNCH_FI(TY, 3);  \
+    else EGS_LAUNCH_FI(TY, 4);               \
+  } while (0)
+  if (dtype == EGS_F32) EGS_LAUNCH(float);
+  else if (dtype == EGS_F16) EGS_LAUNCH(__half);
+  else EGS_LAUNCH(__nv_bfloat16);
+#undef EGS_LAUNCH
+#undef EGS_LAUNCH_FI
   count_launch();
   return cudaGetLastError();
+}
+
+template <typename T, bool VEC>
+static cudaError_t launch_row_sum(const void* Src, const void* Ind, int index_dtype, void* out, int B, int T_, int E, int K, int N,
+                                  StatusRef status, cudaStream_t st) {
+  constexpr int cols = 8 * (VEC ? 16 / static_cast<int>(sizeof(T)) : 1);
+  const int M = B * K, blocks = (N + cols - 1) / cols;
+  // CTAs per cluster: enough for about two per SM, at least 128 rows each
+  int ranks = 1;
+  while (ranks < 8 && static_cast<long long>(blocks) * E * ranks < 2 * 148 && M >= 128 * 2 * ranks) ranks *= 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ranks, blocks, E);
+  cfg.blockDim = dim3(kSumThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = ranks;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, expert_row_sum_kernel<T, VEC>, static_cast<const T*>(Src), Ind, index_dtype, static_cast<T*>(out), T_, E, K,
+                            N, M, status);
+}
+
+cudaError_t launch_expert_row_sum(const void* Src, const void* Ind, int index_dtype, void* out, int B, int T, int E, int K, int N,
+                                  int dtype, StatusRef status, cudaStream_t st) {
+  const bool vec = (reinterpret_cast<uintptr_t>(Src) & 15u) == 0 && (N * (dtype == EGS_F32 ? 4ll : 2ll)) % 16 == 0;
+  cudaError_t err;
+#define EGS_SUM(TY) \
+  err = vec ? launch_row_sum<TY, true>(Src, Ind, index_dtype, out, B, T, E, K, N, status, st) : launch_row_sum<TY, false>(Src, Ind, index_dtype, out, B, T, E, K, N, status, st)
+  if (dtype == EGS_F32) EGS_SUM(float);
+  else if (dtype == EGS_F16) EGS_SUM(__half);
+  else EGS_SUM(__nv_bfloat16);
+#undef EGS_SUM
+  count_launch();
+  return err;
 }
 
 cudaError_t launch_fill_zero(void* ptr, size_t bytes, cudaStream_t st) {

@@ -41,7 +41,7 @@ struct Api {
   X(egs_status_string) X(egs_last_cuda_error) X(egs_gather_gemm_bias) X(egs_gemm_scatter_bias) X(egs_gemm_scatter_prepared) \
   X(egs_scatter_workspace_bytes) X(egs_dweight) X(egs_dweight_prezeroed) X(egs_dw_workspace_bytes)                          \
   X(egs_gather_scatter_pair) X(egs_fused_pair_eligible) X(egs_route_topk) X(egs_index_csr) X(egs_index_csr_scratch_bytes)   \
-  X(egs_fill_zero) X(egs_set_status_mirror)
+  X(egs_fill_zero) X(egs_set_status_mirror) X(egs_expert_row_sum)
 #define EGS_FIELD(name) decltype(&::name) name = nullptr;
   EGS_API(EGS_FIELD)
 #undef EGS_FIELD
@@ -459,6 +459,17 @@ void fill_zero(const Tensor& t) {
   check(api.egs_fill_zero(t.data_ptr(), t.numel() * t.element_size(), c10::cuda::getCurrentCUDAStream(t.get_device()).stream()), "egs_fill_zero");
 }
 
+// [E, N]: per expert, the sum of its slot rows of Src (no Ind) or of the token rows of Src that Ind names
+Tensor expert_row_sum(const Tensor& Src, const OptTensor& Ind, int64_t B, int64_t T, int64_t E, int64_t K) {
+  Call c(Src);
+  const int64_t N = Src.size(-1);
+  Tensor out = empty({E, N}, Src.scalar_type(), c.idx);
+  const Index I = Ind ? index_tensor(*Ind) : Index{Tensor(), EGS_I64};
+  check(api.egs_expert_row_sum(ptr(Src), ptr(I.t), ptr(out), B, T, E, K, N, type_id(Src.scalar_type()), I.type, c.status(), c.stream),
+        "egs_expert_row_sum");
+  return out;
+}
+
 // ---- backward passes of the two operators ------------------------------------------------------------------------------------
 // The weight gradient runs on the helper stream next to the dX / dY kernel: the two are independent and share the SMs.
 struct Grads {
@@ -479,7 +490,7 @@ Grads gather_backward(const Tensor& X_, const Tensor& W, const Tensor& Ind_, con
     g.w = dweight_on(X, dY, Ind, EGS_DW_GATHERED_ROWS, -1, -1, std::nullopt, on, &ws);
   }
   if (need_x) g.in = gemm_scatter(dY, W, Ind, X.size(1), EGS_W_NC, std::nullopt, -1, -1, std::nullopt, std::nullopt);
-  if (need_b) g.b = dY.sum(at::IntArrayRef{0, 2});
+  if (need_b) g.b = expert_row_sum(dY, std::nullopt, dY.size(0), X.size(1), dY.size(1), dY.size(2));
   return g;
 }
 
@@ -497,11 +508,7 @@ Grads scatter_backward(const Tensor& Y_, const Tensor& W, const Tensor& Ind_, co
     g.w = dweight_on(dOut, Y, Ind, EGS_DW_DIRECT_ROWS, -1, -1, std::nullopt, on, &ws);
   }
   if (need_y) g.in = gather_gemm(dOut, W, Ind, EGS_W_NC, -1, -1, std::nullopt);
-  if (need_b) {
-    // sum over the slots of expert e of the gathered rows of dOut: operator D against ones
-    const Tensor ones = at::ones({Y.size(0), Y.size(1), Y.size(2), 8}, Y.options());
-    g.b = dweight_on(dOut, ones, Ind, EGS_DW_GATHERED_ROWS, -1, -1, std::nullopt, std::nullopt, nullptr).select(2, 0);
-  }
+  if (need_b) g.b = expert_row_sum(dOut, Ind, Y.size(0), dOut.size(1), Y.size(1), Y.size(2));
   return g;
 }
 

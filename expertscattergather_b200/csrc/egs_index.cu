@@ -27,6 +27,174 @@ __device__ __forceinline__ uint32_t float_key(float f) {
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
+// ---- route_topk, keys in registers ---------------------------------------------------------------------------------------
+// A CTA serves EG neighbouring experts of one batch element, WPE warps each.  The [T, EG] block of scores is read in whole
+// sectors (the experts are the contiguous direction: one expert alone would fetch eight times its bytes) and turned through
+// shared memory so that every thread ends up with R keys of its expert in registers.  The K-th largest key is then built bit
+// by bit - R compares and a reduction per bit - and the search stops as soon as exactly K keys lie at or above the candidate,
+// after about 20 of 32 bits for scores without ties.  What bounds it is that chain of reductions, not the bytes.
+// B=32, T=2048, E=64, K=128: 127 us with one CTA per expert column and shared-memory histograms.
+constexpr int kSelChunk = 8;          // keys per thread and chunk of the turn through shared memory
+constexpr int kSelMaxKeys = 64;       // keys per thread
+
+template <int WPE>
+__device__ __forceinline__ void expert_sync(int eg) {
+  if (WPE == 1) __syncwarp();
+  else asm volatile("bar.sync %0, %1;" ::"r"(eg + 1), "r"(WPE * 32) : "memory");
+}
+// sum over the expert's threads; red: WPE slots of this expert
+template <int WPE>
+__device__ __forceinline__ unsigned expert_sum(unsigned v, unsigned* red, int eg, int w, int lane) {
+  v = __reduce_add_sync(0xffffffffu, v);
+  if (WPE == 1) return v;
+  expert_sync<WPE>(eg);                      // the slots of the previous sum have been read
+  if (lane == 0) red[w] = v;
+  expert_sync<WPE>(eg);
+  v = 0;
+#pragma unroll
+  for (int i = 0; i < WPE; ++i) v += red[i];
+  return v;
+}
+
+template <int WPE, int R>
+__global__ void __launch_bounds__(512) route_topk_regs_kernel(const float* __restrict__ scores, void* __restrict__ ind, int index_dtype,
+                                                              int T, int E, int K, int eg_log2, int P) {
+  constexpr int CT = WPE * 32 * kSelChunk;   // tokens per chunk
+  extern __shared__ __align__(16) unsigned char sel_smem[];
+  __shared__ unsigned red_s[16], count_s[8];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int eg = warp / WPE, w = warp - eg * WPE;       // expert within the CTA, warp within the expert
+  const int EG = 1 << eg_log2;
+  const int pitch = CT + 4;                             // words; neighbouring experts 4 banks apart
+  uint32_t* turn = reinterpret_cast<uint32_t*>(sel_smem);                       // [EG][pitch], later the lists
+  unsigned long long* sel = reinterpret_cast<unsigned long long*>(sel_smem) + static_cast<size_t>(eg) * P;
+  const int groups = (E + EG - 1) / EG;
+  const int b = blockIdx.x / groups, e0 = (blockIdx.x - b * groups) * EG;
+  const float* base = scores + static_cast<long long>(b) * T * E + e0;
+  const int nthreads = EG * WPE * 32;
+
+  uint32_t key[R];
+  float v[kSelChunk];
+  auto fetch = [&](int t0) {
+#pragma unroll
+    for (int i = 0; i < kSelChunk; ++i) {
+      const int idx = tid + i * nthreads, t = t0 + (idx >> eg_log2), g = idx & (EG - 1);
+      v[i] = (t < T && e0 + g < E) ? base[static_cast<long long>(t) * E + g] : 0.f;
+    }
+  };
+  fetch(0);
+#pragma unroll
+  for (int c = 0; c < R / kSelChunk; ++c) {
+    if (c * CT < T) {                                   // (uniform over the CTA)
+#pragma unroll
+      for (int i = 0; i < kSelChunk; ++i) {
+        const int idx = tid + i * nthreads;
+        turn[(idx & (EG - 1)) * pitch + (idx >> eg_log2)] = float_key(v[i]);
+      }
+      __syncthreads();
+      if ((c + 1) * CT < T) fetch((c + 1) * CT);
+    }
+#pragma unroll
+    for (int i = 0; i < kSelChunk; ++i) {
+      const int tl = i * (WPE * 32) + w * 32 + lane;
+      key[c * kSelChunk + i] = (c * CT + tl < T) ? turn[eg * pitch + tl] : 0u;      // 0: below every candidate
+    }
+    if (c * CT < T) __syncthreads();
+  }
+  if (e0 + eg >= E) return;       // no CTA-wide barrier below
+
+  unsigned* red = red_s + eg * WPE;
+  uint32_t th = 0;
+  bool exact = false;             // exactly K keys are >= th
+  for (int bit = 31; bit >= 0 && !exact; --bit) {
+    const uint32_t cand = th | (1u << bit);
+    unsigned n = 0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) n += (key[i] >= cand) ? 1u : 0u;
+    n = expert_sum<WPE>(n, red, eg, w, lane);
+    if (n >= static_cast<unsigned>(K)) th = cand;
+    exact = n == static_cast<unsigned>(K);
+  }
+  // collect all keys above the threshold (at it, too, when they are exactly K), in any order: a thread's keys go to consecutive
+  // places, behind those of the lanes before it and of the warps that got there first
+  const uint32_t from = exact ? th : th + 1u;            // th is the largest key only if exact or tied at it: no wrap matters
+  const bool all_ones = !exact && th == 0xFFFFFFFFu;
+  if (w == 0 && lane == 0) count_s[eg] = 0;
+  expert_sync<WPE>(eg);
+  unsigned mine = 0;
+#pragma unroll
+  for (int i = 0; i < R; ++i) mine += (key[i] >= from) ? 1u : 0u;
+  if (all_ones) mine = 0;
+  unsigned incl = mine;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const unsigned o = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += o;
+  }
+  unsigned pos = 0;
+  if (lane == 31) pos = atomicAdd(&count_s[eg], incl);
+  pos = __shfl_sync(0xffffffffu, pos, 31) + incl - mine;
+  if (mine) {
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      if (key[i] >= from) {
+        const int t = (i / kSelChunk) * CT + (i % kSelChunk) * (WPE * 32) + w * 32 + lane;
+        sel[pos++] = (static_cast<unsigned long long>(key[i]) << 32) | (0xFFFFFFFFu - static_cast<unsigned>(t));
+      }
+    }
+  }
+  expert_sync<WPE>(eg);
+  if (!exact) {
+    // keys equal to the K-th: the lowest token ids fill the list (tokens ascend with the register index, then with the thread)
+    unsigned n_gt = count_s[eg];
+    for (int i = 0; i < R && n_gt < static_cast<unsigned>(K); ++i) {
+      uint32_t k = 0;
+#pragma unroll
+      for (int j = 0; j < R; ++j)
+        if (j == i) k = key[j];
+      const int t = (i / kSelChunk) * CT + (i % kSelChunk) * (WPE * 32) + w * 32 + lane;
+      const bool eq = t < T && k == th;
+      const unsigned m = __ballot_sync(0xffffffffu, eq);
+      unsigned before = __popc(m & ((1u << lane) - 1u)), total = __popc(m);
+      if (WPE > 1) {
+        expert_sync<WPE>(eg);
+        if (lane == 0) red[w] = __popc(m);
+        expert_sync<WPE>(eg);
+        total = 0;
+#pragma unroll
+        for (int j = 0; j < WPE; ++j) {
+          if (j < w) before += red[j];
+          total += red[j];
+        }
+      }
+      if (eq && n_gt + before < static_cast<unsigned>(K))
+        sel[n_gt + before] = (static_cast<unsigned long long>(k) << 32) | (0xFFFFFFFFu - static_cast<unsigned>(t));
+      n_gt += total;
+    }
+  }
+  // bitonic sort of the K selected (padded to a power of two with zeros, which sort last), descending
+  const int me = w * 32 + lane;
+  for (int i = K + me; i < P; i += WPE * 32) sel[i] = 0ull;
+  expert_sync<WPE>(eg);
+  for (int size = 2; size <= P; size <<= 1)
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      for (int i = me; i < P / 2; i += WPE * 32) {
+        const int lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
+        const unsigned long long x = sel[lo], y = sel[hi];
+        if ((x < y) == ((lo & size) == 0)) { sel[lo] = y; sel[hi] = x; }
+      }
+      expert_sync<WPE>(eg);
+    }
+  const long long out0 = (static_cast<long long>(b) * E + e0 + eg) * K;
+  for (int k = me; k < K; k += WPE * 32) {
+    const long long tok = static_cast<long long>(0xFFFFFFFFu - static_cast<unsigned>(sel[k] & 0xFFFFFFFFull));
+    if (index_dtype == EGS_I64) static_cast<long long*>(ind)[out0 + k] = tok;
+    else if (index_dtype == EGS_I32) static_cast<int*>(ind)[out0 + k] = static_cast<int>(tok);
+    else static_cast<short*>(ind)[out0 + k] = static_cast<short>(tok);
+  }
+}
+
+// ---- route_topk for sequences beyond the registers -----------------------------------------------------------------------
 constexpr int kTopkThreads = 256;
 constexpr int kTopkMaxK = 1024;
 
@@ -127,7 +295,148 @@ __global__ void __launch_bounds__(kTopkThreads) route_topk_kernel(const float* _
   }
 }
 
-// ---- CSR by counting sort ----------------------------------------------------------------------------------------------
+// ---- CSR by counting sort, one CTA per batch element ----------------------------------------------------------------------
+// A batch element's token rows and slots fit in shared memory for ordinary sizes: counting, the scan and the placement then need
+// no global atomics, and two launches do what the general path below does in nine.  The first counts; the second knows how many
+// valid slots the batch elements before its own have and places the entries.  Slots of one row come out in ascending order: an
+// entry's place is the number of smaller slots in its row (counted among the row's own entries, which are few; every entry is
+// ranked by a thread of its own, so a heavy row does not serialise).
+// B=32, T=2048, E=64, K=128: nine launches, 38 us of kernels.
+constexpr int kCsrBatchThreads = 1024;
+
+// sums over the CTA's threads, every thread gets the totals; red: 32 entries
+__device__ __forceinline__ int cta_sum(int v, int* red) {
+  v = __reduce_add_sync(0xffffffffu, v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  int s = red[threadIdx.x & 31];
+  return __reduce_add_sync(0xffffffffu, s);
+}
+
+__global__ void __launch_bounds__(kCsrBatchThreads) csr_batch_count_kernel(const void* __restrict__ ind, int index_dtype, int T, int EK,
+                                                                           int* __restrict__ counts, int4* __restrict__ partial) {
+  extern __shared__ int cnt[];          // [T]
+  __shared__ int red[32];
+  const int b = blockIdx.x, tid = threadIdx.x;
+  for (int t = tid; t < T; t += kCsrBatchThreads) cnt[t] = 0;
+  __syncthreads();
+  int valid = 0, bad = 0;
+  for (int s = tid; s < EK; s += kCsrBatchThreads) {
+    const long long t = load_index(ind, index_dtype, static_cast<long long>(b) * EK + s);
+    if (t >= 0 && t < T) {
+      atomicAdd(&cnt[t], 1);
+      ++valid;
+    } else {
+      bad = 1;
+    }
+  }
+  __syncthreads();
+  int most = 0, rows = 0;
+  for (int t = tid; t < T; t += kCsrBatchThreads) {
+    const int c = cnt[t];
+    counts[static_cast<long long>(b) * T + t] = c;
+    most = max(most, c);
+    rows += c > 0;
+  }
+  valid = cta_sum(valid, red);
+  rows = cta_sum(rows, red);
+  bad = __syncthreads_or(bad);
+  most = __reduce_max_sync(0xffffffffu, most);
+  if ((tid & 31) == 0) red[tid >> 5] = most;
+  __syncthreads();
+  if (tid == 0) {
+    for (int i = 0; i < 32; ++i) most = max(most, red[i]);
+    partial[b] = make_int4(most, rows, bad ? 1 : 0, valid);
+  }
+}
+
+__global__ void __launch_bounds__(kCsrBatchThreads) csr_batch_place_kernel(const void* __restrict__ ind, int index_dtype, int T, int EK,
+                                                                           const int* __restrict__ counts, const int4* __restrict__ partial,
+                                                                           int* __restrict__ offsets, int* __restrict__ entries,
+                                                                           int* __restrict__ info) {
+  extern __shared__ int csr_smem[];
+  __shared__ int red[32];
+  int* start = csr_smem;                // [T + 1] first entry of every row, local
+  int* cursor = csr_smem + T + 1;       // [T]
+  int* list = cursor + T;               // [EK] slots grouped by row, unordered inside a row
+  const int b = blockIdx.x, nb = gridDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+
+  int before = 0;
+  for (int i = tid; i < b; i += kCsrBatchThreads) before += partial[i].w;
+  before = cta_sum(before, red);
+  if (b == 0 && warp == 0) {            // the summary over all batch elements
+    int most = 0, rows = 0, bad = 0, valid = 0;
+    for (int i = lane; i < nb; i += 32) {
+      const int4 q = partial[i];
+      most = max(most, q.x);
+      rows += q.y;
+      bad |= q.z;
+      valid += q.w;
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    rows = __reduce_add_sync(0xffffffffu, rows);
+    bad = __reduce_or_sync(0xffffffffu, bad);
+    valid = __reduce_add_sync(0xffffffffu, valid);
+    if (lane == 0) {
+      info[0] = most;
+      info[1] = rows;
+      info[2] = bad;
+      info[3] = valid;
+    }
+  }
+  // exclusive scan of the counts: a contiguous run of rows per thread, then a scan of the threads' sums
+  const int per = (T + kCsrBatchThreads - 1) / kCsrBatchThreads, t0 = min(T, tid * per), t1 = min(T, t0 + per);
+  const int* row_counts = counts + static_cast<long long>(b) * T;
+  for (int t = tid; t < T; t += kCsrBatchThreads) cursor[t] = row_counts[t];
+  __syncthreads();
+  int sum = 0;
+  for (int t = t0; t < t1; ++t) sum += cursor[t];
+  int incl = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int o = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += o;
+  }
+  __syncthreads();
+  if (lane == 31) red[warp] = incl;
+  __syncthreads();
+  int wsum = red[lane];
+  const int mine = wsum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int o = __shfl_up_sync(0xffffffffu, wsum, d);
+    if (lane >= d) wsum += o;
+  }
+  const int wbase = __shfl_sync(0xffffffffu, wsum - mine, warp);
+  const int total = __shfl_sync(0xffffffffu, wsum, 31);
+  int run = wbase + incl - sum;
+  for (int t = t0; t < t1; ++t) {
+    const int c = cursor[t];
+    start[t] = run;
+    cursor[t] = run;
+    run += c;
+  }
+  if (tid == 0) start[T] = total;
+  __syncthreads();
+  for (int t = tid; t < T; t += kCsrBatchThreads) offsets[static_cast<long long>(b) * T + t] = before + start[t];
+  if (b == nb - 1 && tid == 0) offsets[static_cast<long long>(nb) * T] = before + total;
+  for (int s = tid; s < EK; s += kCsrBatchThreads) {
+    const long long t = load_index(ind, index_dtype, static_cast<long long>(b) * EK + s);
+    if (t >= 0 && t < T) list[atomicAdd(&cursor[t], 1)] = s;
+  }
+  __syncthreads();
+  for (int s = tid; s < EK; s += kCsrBatchThreads) {
+    const long long t = load_index(ind, index_dtype, static_cast<long long>(b) * EK + s);
+    if (t < 0 || t >= T) continue;
+    const int lo = start[t], hi = start[t + 1];
+    int rank = 0;
+    for (int i = lo; i < hi; ++i) rank += list[i] < s;
+    entries[before + lo + rank] = b * EK + s;
+  }
+}
+
+// ---- CSR by counting sort, any size ---------------------------------------------------------------------------------------
 // info[0] = heaviest row, info[1] = rows touched, info[2] = 1 if an id was out of range, info[3] = valid slots
 __global__ void __launch_bounds__(256) csr_count_kernel(const void* __restrict__ ind, int index_dtype, int B, int T, int E, int K,
                                                        int* __restrict__ counts, int* __restrict__ info) {
@@ -328,10 +637,36 @@ int grid_1d(long long items, int per_block, int cap) {
 
 }  // namespace
 
-cudaError_t launch_route_topk(const float* scores, void* ind, int index_dtype, int B, int T, int E, int K, cudaStream_t st) {
-  route_topk_kernel<<<B * E, kTopkThreads, 0, st>>>(scores, ind, index_dtype, B, T, E, K);
-  count_launch();
+template <int WPE, int R>
+static cudaError_t launch_topk_regs(const float* scores, void* ind, int index_dtype, int B, int T, int E, int K, cudaStream_t st) {
+  // experts per CTA: whole 32-byte sectors of scores, but no fewer CTAs than SMs where there are that many (batch, expert) pairs
+  int eg = 16 / WPE < 8 ? 16 / WPE : 8;
+  while (eg > 1 && (eg / 2 >= E || static_cast<long long>(B) * ((E + eg - 1) / eg) < 148)) eg /= 2;
+  int P = 1, eg_log2 = 0;
+  while (P < K) P <<= 1;
+  while ((1 << eg_log2) < eg) ++eg_log2;
+  const size_t turn = static_cast<size_t>(eg) * (WPE * 32 * kSelChunk + 4) * 4, lists = static_cast<size_t>(eg) * P * 8;
+  const size_t smem = turn > lists ? turn : lists;
+  if (smem > 48 * 1024) {      // at most 8 lists of kTopkMaxK entries
+    cudaError_t err = ensure_smem_optin<route_topk_regs_kernel<WPE, R>>(8 * kTopkMaxK * 8);
+    if (err != cudaSuccess) return err;
+  }
+  route_topk_regs_kernel<WPE, R><<<B * ((E + eg - 1) / eg), eg * WPE * 32, smem, st>>>(scores, ind, index_dtype, T, E, K, eg_log2, P);
   return cudaGetLastError();
+}
+
+cudaError_t launch_route_topk(const float* scores, void* ind, int index_dtype, int B, int T, int E, int K, cudaStream_t st) {
+  cudaError_t err = cudaSuccess;
+  // fewest warps per expert that hold its T keys in registers
+  if (T <= 1 * 32 * 8) err = launch_topk_regs<1, 8>(scores, ind, index_dtype, B, T, E, K, st);
+  else if (T <= 1 * 32 * 32) err = launch_topk_regs<1, 32>(scores, ind, index_dtype, B, T, E, K, st);
+  else if (T <= 1 * 32 * kSelMaxKeys) err = launch_topk_regs<1, kSelMaxKeys>(scores, ind, index_dtype, B, T, E, K, st);
+  else if (T <= 2 * 32 * kSelMaxKeys) err = launch_topk_regs<2, kSelMaxKeys>(scores, ind, index_dtype, B, T, E, K, st);
+  else if (T <= 4 * 32 * kSelMaxKeys) err = launch_topk_regs<4, kSelMaxKeys>(scores, ind, index_dtype, B, T, E, K, st);
+  else if (T <= 8 * 32 * kSelMaxKeys) err = launch_topk_regs<8, kSelMaxKeys>(scores, ind, index_dtype, B, T, E, K, st);
+  else route_topk_kernel<<<B * E, kTopkThreads, 0, st>>>(scores, ind, index_dtype, B, T, E, K);
+  count_launch();
+  return err != cudaSuccess ? err : cudaGetLastError();
 }
 
 size_t index_csr_scratch_ints(long long rows) { return static_cast<size_t>(rows) + static_cast<size_t>((rows + kScanBlock - 1) / kScanBlock) + 8; }
@@ -345,6 +680,19 @@ cudaError_t launch_index_csr(const void* ind, int index_dtype, int B, int T, int
   int* cursor = scratch;
   int* block_sums = scratch + rows;
   int* total = block_sums + nblocks;
+  // one CTA per batch element where its rows and slots fit in shared memory and the partial figures in the scratch
+  const long long ek = static_cast<long long>(E) * K;
+  const size_t place_smem = (2 * static_cast<size_t>(T) + 1 + static_cast<size_t>(ek)) * sizeof(int);
+  int4* partial = reinterpret_cast<int4*>((reinterpret_cast<uintptr_t>(scratch) + 15) & ~static_cast<uintptr_t>(15));
+  if (n > 0 && rows > 0 && place_smem <= 200 * 1024 && (4ll * B + 4) * static_cast<long long>(sizeof(int)) <= static_cast<long long>(index_csr_scratch_ints(rows) * sizeof(int))) {
+    cudaError_t err = ensure_smem_optin<csr_batch_place_kernel>(200 * 1024);
+    if (err == cudaSuccess) err = ensure_smem_optin<csr_batch_count_kernel>(200 * 1024);
+    if (err != cudaSuccess) return err;
+    csr_batch_count_kernel<<<B, kCsrBatchThreads, static_cast<size_t>(T) * sizeof(int), st>>>(ind, index_dtype, T, static_cast<int>(ek), counts, partial);
+    csr_batch_place_kernel<<<B, kCsrBatchThreads, place_smem, st>>>(ind, index_dtype, T, static_cast<int>(ek), counts, partial, offsets, entries, info);
+    count_launch(2);
+    return cudaGetLastError();
+  }
   cudaError_t err = launch_fill_zero(counts, static_cast<size_t>(rows) * sizeof(int), st);
   if (err == cudaSuccess) err = launch_fill_zero(info, 4 * sizeof(int), st);
   if (err == cudaSuccess) err = launch_fill_zero(cursor, static_cast<size_t>(rows) * sizeof(int), st);

@@ -126,7 +126,11 @@ struct FusedParams {
 // launchers implemented in the kernel files; each returns a cudaError_t from the launch
 // ------------------------------------------------------------------------------------------------
 cudaError_t launch_generic_rowgemm(const RowGemmParams& p, bool scatter, int dtype, cudaStream_t st);
+void configure_generic_dweight(DWeightParams& p);   // tile (BN, row_tiles in units of 32 features) and row ranges
 cudaError_t launch_generic_dweight(const DWeightParams& p, int dtype, cudaStream_t st);
+// out[e, n] = sum over the slots of expert e of a row of Src: token rows through Ind, or slot rows where Ind is NULL
+cudaError_t launch_expert_row_sum(const void* Src, const void* Ind, int index_dtype, void* out, int B, int T, int E, int K, int N,
+                                  int dtype, StatusRef status, cudaStream_t st);
 cudaError_t launch_fill_zero(void* ptr, size_t bytes, cudaStream_t st);
 cudaError_t launch_convert_from_f32(const float* src, void* dst, size_t n, int dtype, cudaStream_t st);
 cudaError_t launch_convert_to_f32(const void* src, float* dst, size_t n, int dtype, cudaStream_t st);
@@ -181,5 +185,18 @@ cudaError_t launch_plan_from_info(const int* info, int limit, int* plan, int32_t
 cudaError_t launch_wait_timeout_selftest(int32_t* status, int* out, long long limit_cycles, cudaStream_t st);
 
 void count_launch(int n = 1);
+
+// The opt-in to large dynamic shared memory is per kernel function and device: done once per thread and device, for `bytes`.
+template <auto kernel>
+cudaError_t ensure_smem_optin(int bytes) {
+  static thread_local int done_device = -1;
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  if (done_device == dev) return cudaSuccess;
+  err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (err == cudaSuccess) done_device = dev;
+  return err;
+}
 
 }  // namespace egs

@@ -437,6 +437,20 @@ __device__ __forceinline__ void add_bias4(const T* bias, uint32_t& x0, uint32_t&
   x3 = __float_as_uint(__uint_as_float(x3) + to_f32<T>(bias[3]));
 }
 
+// Adds bias[0..31] to 32 consecutive columns of a row (every lane of the warp reads the same 64 bytes); `left`: columns up to
+// the end of the row, a multiple of 8.  16-bit rows, 16-byte aligned.
+template <typename T>
+__device__ __forceinline__ void add_bias32(const T* bias, int left, uint32_t (&v)[32]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (8 * j >= left) break;
+    const uint4 x = *reinterpret_cast<const uint4*>(bias + 8 * j);
+    const T* b = reinterpret_cast<const T*>(&x);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[8 * j + i] = __float_as_uint(__uint_as_float(v[8 * j + i]) + to_f32<T>(b[i]));
+  }
+}
+
 __device__ __forceinline__ uint32_t tmem_cols_for(int bn) {
   uint32_t c = 32;
   while (c < static_cast<uint32_t>(bn)) c <<= 1;

@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_rowgemm_kern
       // direct 16-bit adds as bulk reductions: every lane stages 128 bytes (64 columns) of its own row in the idle
       // ring and hands them to the copy engine (see the persistent variant)
       static_assert(2u * kBulkBufBytes <= 16384u, "two staging buffers per warp");
-      const bool bulk16 = direct16 && p.bulk_epilogue && p.bias == nullptr && (pp.stages * pp.stage_bytes >= 8u * 2u * kBulkBufBytes);
+      const bool bulk16 = direct16 && p.bulk_epilogue && (pp.stages * pp.stage_bytes >= 8u * 2u * kBulkBufBytes);
       const T* bias_row = p.bias ? static_cast<const T*>(p.bias) + static_cast<long long>(e) * p.N : nullptr;
       if (bulk16) {
         if constexpr (ES == 2 && SCATTER) {
@@ -432,6 +432,7 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_rowgemm_kern
                   uint32_t v[32];
                   tmem_ld32(acc0 + static_cast<uint32_t>(c * 64 + h * 32), v);
                   tmem_ld_wait();
+                  if (bias_row) add_bias32<T>(bias_row + n0 + c * 64 + h * 32, p.N - (n0 + c * 64 + h * 32), v);
 #pragma unroll
                   for (int j = 0; j < 4; ++j)
                     asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(srow + h * 64u + j * 16u),
@@ -814,7 +815,7 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
     // bulk adds (direct 16-bit scatter): every lane stages 128 bytes of its own row and hands them to the copy
     // engine - no transpose, no shuffles, and the warp does not wait on the load/store unit.  (For float32 rows
     // the same scheme needs twice the operations per column and measured slower than the transposed reds.)
-    const bool bulk = direct16 && p.bulk_epilogue && p.bias == nullptr;
+    const bool bulk = direct16 && p.bulk_epilogue;
     const uint32_t my_stage = tile + static_cast<uint32_t>(lane) * kBulkRowPitch;
     int q = 0;                                           // bulk groups committed so far by this thread
     bool alive = true;
@@ -844,6 +845,9 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
                   uint32_t v[32];
                   tmem_ld32(acc0 + static_cast<uint32_t>(c * 64 + h * 32), v);
                   tmem_ld_wait();
+                  if (p.bias)
+                    add_bias32<T>(static_cast<const T*>(p.bias) + static_cast<long long>(blk.e) * p.N + n0 + c * 64 + h * 32,
+                                  p.N - (n0 + c * 64 + h * 32), v);
 #pragma unroll
                   for (int j = 0; j < 4; ++j)
                     asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(srow + h * 64u + j * 16u),
@@ -1751,19 +1755,6 @@ size_t configure_tensor_fused_pair(FusedParams& p, int precision) {
   return fixed + ns * stage_bytes;
 }
 
-// The opt-in to large dynamic shared memory is per kernel function: done once, for the maximum.
-template <auto kernel>
-static cudaError_t ensure_smem_optin() {
-  static thread_local int done_device = -1;
-  int dev = 0;
-  cudaError_t err = cudaGetDevice(&dev);
-  if (err != cudaSuccess) return err;
-  if (done_device == dev) return cudaSuccess;
-  err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMaxPerCta));
-  if (err == cudaSuccess) done_device = dev;
-  return err;
-}
-
 cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, int dtype, int precision, size_t smem_bytes,
                                   cudaStream_t st) {
   if (p.persistent) {
@@ -1774,10 +1765,10 @@ cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, int dtyp
 #define EGS_LAUNCH_P(TY)                                                                                     \
   do {                                                                                                       \
     if (scatter) {                                                                                           \
-      perr = (ensure_smem_optin<tensor_rowgemm_persistent_kernel<TY, true>>());                              \
+      perr = (ensure_smem_optin<tensor_rowgemm_persistent_kernel<TY, true>>(static_cast<int>(kSmemMaxPerCta)));                              \
       if (perr == cudaSuccess) tensor_rowgemm_persistent_kernel<TY, true><<<pgrid, pblock, smem_bytes, st>>>(p);  \
     } else {                                                                                                 \
-      perr = (ensure_smem_optin<tensor_rowgemm_persistent_kernel<TY, false>>());                             \
+      perr = (ensure_smem_optin<tensor_rowgemm_persistent_kernel<TY, false>>(static_cast<int>(kSmemMaxPerCta)));                             \
       if (perr == cudaSuccess) tensor_rowgemm_persistent_kernel<TY, false><<<pgrid, pblock, smem_bytes, st>>>(p); \
     }                                                                                                        \
   } while (0)
@@ -1796,7 +1787,7 @@ cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, int dtyp
   cudaError_t err = cudaSuccess;
 #define EGS_LAUNCH2(TY, STRICT, SC, MTV)                                                              \
   do {                                                                                                \
-    err = (ensure_smem_optin<tensor_rowgemm_kernel<TY, STRICT, SC, MTV>>());                          \
+    err = (ensure_smem_optin<tensor_rowgemm_kernel<TY, STRICT, SC, MTV>>(static_cast<int>(kSmemMaxPerCta)));                          \
     if (err == cudaSuccess) tensor_rowgemm_kernel<TY, STRICT, SC, MTV><<<grid, block, smem_bytes, st>>>(p); \
   } while (0)
 #define EGS_LAUNCH(TY, STRICT)                                        \
@@ -1831,7 +1822,7 @@ cudaError_t launch_tensor_dweight(const DWeightParams& p, int dtype, int precisi
   cudaError_t err = cudaSuccess;
 #define EGS_LAUNCH_D(TY, STRICT, MTV)                                                           \
   do {                                                                                          \
-    err = (ensure_smem_optin<tensor_dweight_kernel<TY, STRICT, MTV>>());                        \
+    err = (ensure_smem_optin<tensor_dweight_kernel<TY, STRICT, MTV>>(static_cast<int>(kSmemMaxPerCta)));                        \
     if (err == cudaSuccess) tensor_dweight_kernel<TY, STRICT, MTV><<<grid, block, smem_bytes, st>>>(p); \
   } while (0)
 #define EGS_LAUNCH(TY, STRICT)                                   \
@@ -1865,10 +1856,10 @@ cudaError_t launch_tensor_fused_pair(const FusedParams& p, int precision, size_t
   dim3 block(17 * 32);
   cudaError_t err;
   if (precision == EGS_PREC_STRICT) {
-    err = ensure_smem_optin<tensor_fused_pair_kernel<true>>();
+    err = ensure_smem_optin<tensor_fused_pair_kernel<true>>(static_cast<int>(kSmemMaxPerCta));
     if (err == cudaSuccess) tensor_fused_pair_kernel<true><<<grid, block, smem_bytes, st>>>(p);
   } else {
-    err = ensure_smem_optin<tensor_fused_pair_kernel<false>>();
+    err = ensure_smem_optin<tensor_fused_pair_kernel<false>>(static_cast<int>(kSmemMaxPerCta));
     if (err == cudaSuccess) tensor_fused_pair_kernel<false><<<grid, block, smem_bytes, st>>>(p);
   }
   if (err != cudaSuccess) return err;

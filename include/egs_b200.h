@@ -280,6 +280,14 @@ typedef struct egs_plan_info {
 } egs_plan_info;
 int egs_describe_plan(int op, const egs_dims* dims, int w_layout, int dtype, int precision, egs_plan_info* out);
 
+/*
+ * Row sums per expert:  out[e, n] = sum over (b, k) of a row of Src.  Ind given: the token row Ind[b,e,k] of Src [B,T,N] (the
+ * gradient of a per-slot scatter bias); Ind NULL: the slot row of Src [B,E,K,N] (the gradient of a gather bias).  Summed in
+ * float32 in a fixed order, rounded once to the tensors' dtype; out-of-range ids add nothing and set the status bit.
+ */
+int egs_expert_row_sum(const void* Src, const void* Ind, void* out, int64_t B, int64_t T, int64_t E, int64_t K, int64_t N, int dtype,
+                       int index_dtype, int32_t* status_word, void* cuda_stream);
+
 /* Zero-fills n bytes at p on the stream with the library's own fill kernel (what zero_output uses).
  * Replaces the torch.zeros_like calls of the reference's wrappers (egs/triton_kernels.py:408-409). */
 int egs_fill_zero(void* p, size_t n_bytes, void* cuda_stream);

@@ -1,0 +1,77 @@
+"""Kernel variants at the sizes where their dispatch or their tiles change over: remainders, the smallest and largest of each
+range, ties.  Integer-valued or index results are compared bit for bit, sums against float64."""
+import numpy as np
+import pytest
+import torch
+
+from expertscattergather_b200 import _lib, ops, workloads
+from expertscattergather_b200.workloads import Workload
+from gpu_util import STEP_KEYS, gpu_step
+from oracle import egs_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+# keys per thread and warps per expert change at T = 256, 1024, 2048, 4096, 8192, 16384 (beyond: the shared-memory kernel);
+# E around the eight experts of a CTA; few (batch, expert) pairs: fewer experts per CTA
+@pytest.mark.parametrize("B,T,E,K", [(1, 1, 1, 1), (2, 256, 9, 256), (40, 257, 33, 31), (3, 1024, 8, 1000), (20, 1025, 65, 3),
+                                     (20, 2049, 70, 1024), (2, 4097, 12, 77), (1, 8193, 5, 1024), (1, 16385, 3, 200)])
+@pytest.mark.parametrize("ties", [False, True])
+def test_route_topk_edges(cuda_device, B, T, E, K, ties):
+    g = torch.Generator().manual_seed(T + E)
+    scores = torch.randint(-3, 4, (B, T, E), generator=g).float() if ties else torch.randn(B, T, E, generator=g)
+    Ind = ops.route_topk(scores.to(cuda_device), K).cpu()
+    order = torch.sort(scores.permute(0, 2, 1), dim=-1, descending=True, stable=True).indices      # ties: lower token first
+    assert torch.equal(Ind, order[..., :K])
+
+
+@pytest.mark.parametrize("B,T,E,K", [(3, 1, 2, 5), (2, 1023, 7, 9), (5, 1025, 300, 20), (1, 20000, 11, 13), (1, 30000, 4, 9)])
+@pytest.mark.parametrize("one_row", [False, True])
+def test_index_csr_edges(cuda_device, B, T, E, K, one_row):
+    g = torch.Generator().manual_seed(T)
+    Ind = torch.randint(0, T, (B, E, K), generator=g)
+    if one_row:
+        Ind[:, : E // 2] = T - 1            # half of all slots in one row
+    Ind[B - 1, E - 1, K - 1] = T            # out of range: left out
+    csr = ops.build_index_csr(Ind.to(cuda_device), T)
+    flat = Ind + torch.arange(B).view(-1, 1, 1) * T
+    valid = (Ind < T).reshape(-1)
+    rows, slots = flat.reshape(-1)[valid], torch.arange(Ind.numel())[valid]
+    counts = torch.bincount(rows, minlength=B * T)
+    assert torch.equal(csr.counts.cpu().long(), counts)
+    assert torch.equal(csr.offsets.cpu().long(), torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)]))
+    assert torch.equal(csr.entries.cpu().long()[: slots.numel()], slots[torch.sort(rows, stable=True).indices])
+    assert csr.summary() == {"max_per_row": int(counts.max()), "rows_touched": int((counts > 0).sum()), "out_of_range": True,
+                             "valid_slots": int(valid.sum())}
+
+
+# generic kernels: tile widths of 32, 64, 96 and 128 columns, remainders in rows (B*K around 64), features and contraction steps
+@pytest.mark.parametrize("B,T,E,K,I,J", [(1, 3, 1, 1, 1, 1), (7, 40, 2, 9, 31, 33), (5, 33, 3, 13, 65, 95), (9, 70, 2, 29, 127, 97),
+                                         (3, 50, 2, 21, 161, 5), (2, 20, 1, 150, 33, 257)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_generic_kernels_edges(cuda_device, B, T, E, K, I, J, dtype):
+    w = Workload("gen", B, T, E, K, I, J, dtype, "replace", 77)
+    ins = workloads.make_inputs(w, integer_valued=True)
+    ref = orc.np_step(ins["X"], ins["Wg"], ins["Ws"], ins["Ind"], ins["G"])
+    got = gpu_step(ins, cuda_device, "generic")
+    for k in STEP_KEYS:         # small integers: exact in float32; 16-bit results are the float32 sums rounded once
+        if dtype == torch.float32:
+            assert np.array_equal(got[k].double().numpy(), ref[k]), k
+        elif k in ("Y", "dY"):
+            assert torch.equal(got[k], torch.from_numpy(ref[k]).to(dtype)), k
+
+
+@pytest.mark.parametrize("B,T,E,K,N", [(1, 5, 1, 1, 1), (3, 40, 4, 50, 24), (16, 64, 2, 100, 72), (70, 33, 3, 30, 33)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("gathered", [False, True])
+def test_expert_row_sum(cuda_device, B, T, E, K, N, dtype, gathered):
+    g = torch.Generator().manual_seed(N)
+    Ind = torch.randint(0, T, (B, E, K), generator=g)
+    src = torch.randint(-4, 5, (B, T, N) if gathered else (B, E, K, N), generator=g).to(dtype)
+    out = torch.full((E, N), float("nan"), dtype=dtype, device=cuda_device)
+    d_src, d_ind = src.to(cuda_device), Ind.to(cuda_device)
+    rc = _lib.load().egs_expert_row_sum(d_src.data_ptr(), d_ind.data_ptr() if gathered else None, out.data_ptr(), B, T, E, K, N,
+                                        ops.dtype_to_type_id(dtype), _lib.I64, None, torch.cuda.current_stream().cuda_stream)
+    assert rc == _lib.OK
+    rows = torch.gather(src.double(), 1, Ind.reshape(B, -1, 1).expand(-1, -1, N)).reshape(B, E, K, N) if gathered else src.double()
+    assert torch.equal(out.cpu(), rows.sum((0, 2)).to(dtype))       # integers: exact in float32, rounded once
