@@ -71,8 +71,10 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 constexpr long long kInt32Max = 2147483647LL;
 // 16-bit scatter adds directly into the output while no token row receives more contributions than this.
 constexpr int kDirect16Limit = 32;
-// Longest contraction strict float32 runs on the tensor cores under EGS_PATH_AUTO (see run_rowgemm).
-constexpr long long kStrictMaxContraction = 512;
+// Longest contraction strict float32 runs on the tensor cores under EGS_PATH_AUTO (see run_rowgemm), and longest that one
+// accumulator of the fused pair kernel sees.
+constexpr long long kStrictMaxContraction = 2048;
+constexpr long long kStrictMaxFusedContraction = 512;
 
 bool device_is_sm100() {
   static thread_local int cached_dev = -1;
@@ -139,8 +141,8 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
   const bool eligible = device_is_sm100() && rowgemm_tensor_ok(d, dtype, A, W, Out);
   if ((path == EGS_PATH_TENSOR || path == EGS_PATH_PAIRED) && !eligible) return EGS_ERR_UNSUPPORTED;
   // Strict float32 on long contractions: the tensor core's accumulator additions truncate, and the error grows with the
-  // contraction length (3.3e-5 of max|ref| at C = 4096 against the 1e-5 bar).  EGS_PATH_AUTO therefore keeps strict
-  // float32 on the tensor cores only up to kStrictMaxContraction and takes the FFMA kernels beyond.
+  // contraction length (3.3e-5 of max|ref| at C = 4096 against the 1e-5 bar).  The strict kernels sum chunks of 512 elements with
+  // correct rounding; EGS_PATH_AUTO takes them up to kStrictMaxContraction and the FFMA kernels beyond.
   const bool strict_long = (dtype == EGS_F32 && precision == EGS_PREC_STRICT && d.C > kStrictMaxContraction);
   const bool tensor = ((path == EGS_PATH_TENSOR || path == EGS_PATH_PAIRED) || (path == EGS_PATH_AUTO && eligible && !strict_long)) && !(d.C == 0) &&
                       (bias == nullptr || aligned16(bias));
@@ -197,13 +199,16 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
   cudaError_t err;
   if (tensor) {
     p.expert_fastest = pick_expert_fastest(d, scatter, dtype);
-    if (path == EGS_PATH_PAIRED) {
+    if (dtype == EGS_F32 && precision == EGS_PREC_STRICT) {
+      configure_strict_rowgemm(p);
+      err = launch_strict_rowgemm(p, scatter, st);
+    } else if (path == EGS_PATH_PAIRED) {
       const size_t smem2 = configure_tensor_gather2(p);
       if (smem2 == 0) return EGS_ERR_UNSUPPORTED;
       err = launch_tensor_gather2(p, dtype, smem2, st);
     } else {
-      const size_t smem = configure_tensor_rowgemm(p, scatter, dtype, precision);
-      err = launch_tensor_rowgemm(p, scatter, dtype, precision, smem, st);
+      const size_t smem = configure_tensor_rowgemm(p, scatter, dtype);
+      err = launch_tensor_rowgemm(p, scatter, dtype, smem, st);
     }
   } else {
     err = launch_generic_rowgemm(p, scatter, dtype, st);
@@ -354,7 +359,7 @@ int egs_fused_pair_eligible(int64_t C1, int64_t N1, int64_t N2, int w_layout, in
   FusedParams p{};
   p.C1 = static_cast<int>(C1); p.N1 = static_cast<int>(N1); p.N2 = static_cast<int>(N2); p.w_layout = w_layout;
   if (dtype != EGS_F32) return configure_tensor_pair16(p) != 0 ? 1 : 0;
-  if (precision == EGS_PREC_STRICT && C1 > kStrictMaxContraction) return 0;     // see run_rowgemm
+  if (precision == EGS_PREC_STRICT && C1 > kStrictMaxFusedContraction) return 0;     // see run_rowgemm
   return configure_tensor_fused_pair(p, precision) != 0 ? 1 : 0;
 }
 
@@ -483,12 +488,15 @@ static int dweight_impl(const void* Xsrc, const void* Ysrc, const void* Ind, voi
   const bool tensor = (path == EGS_PATH_TENSOR) || (path == EGS_PATH_AUTO && eligible);
 
   size_t smem = 0;
-  if (tensor) {
-    smem = configure_tensor_dweight(p, dtype, precision);
+  const bool strict = tensor && dtype == EGS_F32 && precision == EGS_PREC_STRICT;
+  if (strict) {
+    configure_strict_dweight(p);
+  } else if (tensor) {
+    smem = configure_tensor_dweight(p, dtype);
   } else {
     configure_generic_dweight(p);
   }
-  if (static_cast<long long>(p.E) * p.splits > 65535) return EGS_ERR_TOO_LARGE;   // grid.z limit
+  if (!strict && static_cast<long long>(p.E) * p.splits > 65535) return EGS_ERR_TOO_LARGE;   // grid.z limit
 
   cudaError_t err;
   if (p.splits > 1) {
@@ -503,7 +511,7 @@ static int dweight_impl(const void* Xsrc, const void* Ysrc, const void* Ind, voi
       if (err != cudaSuccess) return fail_cuda(err, "fill_zero");
     }
   }
-  err = tensor ? launch_tensor_dweight(p, dtype, precision, smem, st) : launch_generic_dweight(p, dtype, st);
+  err = strict ? launch_strict_dweight(p, st) : tensor ? launch_tensor_dweight(p, dtype, smem, st) : launch_generic_dweight(p, dtype, st);
   if (err != cudaSuccess) return fail_cuda(err, "dweight launch");
   if (p.splits > 1 && dtype != EGS_F32) {
     err = launch_convert_from_f32(p.acc, out, n_out, dtype, st);
@@ -584,7 +592,8 @@ int egs_describe_plan(int op, const egs_dims* dims, int w_layout, int dtype, int
     DWeightParams p{};
     p.B = static_cast<int>(d.B); p.T = static_cast<int>(d.T); p.E = static_cast<int>(d.E); p.K = static_cast<int>(d.K);
     p.FG = static_cast<int>(d.C); p.FD = static_cast<int>(d.N); p.M = static_cast<int>(d.B * d.K);
-    configure_tensor_dweight(p, dtype, precision);
+    if (dtype == EGS_F32 && precision == EGS_PREC_STRICT) configure_strict_dweight(p);
+    else configure_tensor_dweight(p, dtype);
     out->tile_n = p.BN; out->stages = p.stages; out->row_tiles = p.row_tiles; out->splits = p.splits;
     out->rows_per_split = p.rows_per_split;
     return EGS_OK;
@@ -594,7 +603,8 @@ int egs_describe_plan(int op, const egs_dims* dims, int w_layout, int dtype, int
   p.C = static_cast<int>(d.C); p.N = static_cast<int>(d.N); p.M = static_cast<int>(d.B * d.K);
   p.w_layout = w_layout;
   p.expert_fastest = pick_expert_fastest(d, op == 1, dtype);
-  configure_tensor_rowgemm(p, op == 1, dtype, precision);
+  if (dtype == EGS_F32 && precision == EGS_PREC_STRICT) configure_strict_rowgemm(p);
+  else configure_tensor_rowgemm(p, op == 1, dtype);
   out->tile_n = p.BN; out->stages = p.stages; out->row_tiles = p.row_tiles; out->persistent = p.persistent;
   out->bulk_epilogue = (p.persistent || op == 1) ? p.bulk_epilogue : 0; out->expert_fastest = p.expert_fastest;
   return EGS_OK;

@@ -143,12 +143,16 @@ cudaError_t launch_scatter_init(const int* plan, float* acc, void* out16, size_t
 cudaError_t launch_scatter_finish(const int* plan, const float* acc, void* out16, size_t n, int dtype, cudaStream_t st);
 
 // Tensor-core (tcgen05) family.  `configure_*` fills BN/stages and returns the dynamic shared memory size.
-size_t configure_tensor_rowgemm(RowGemmParams& p, bool scatter, int dtype, int precision);
-size_t configure_tensor_dweight(DWeightParams& p, int dtype, int precision);
-cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, int dtype, int precision,
-                                  size_t smem_bytes, cudaStream_t st);
-cudaError_t launch_tensor_dweight(const DWeightParams& p, int dtype, int precision, size_t smem_bytes,
-                                  cudaStream_t st);
+size_t configure_tensor_rowgemm(RowGemmParams& p, bool scatter, int dtype);
+size_t configure_tensor_dweight(DWeightParams& p, int dtype);
+cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, int dtype, size_t smem_bytes, cudaStream_t st);
+cudaError_t launch_tensor_dweight(const DWeightParams& p, int dtype, size_t smem_bytes, cudaStream_t st);
+
+// Strict float32 (egs_strict.cu).  Long contractions are fine up to kStrictMaxContraction (see run_rowgemm).
+void configure_strict_rowgemm(RowGemmParams& p);
+cudaError_t launch_strict_rowgemm(const RowGemmParams& p, bool scatter, cudaStream_t st);
+void configure_strict_dweight(DWeightParams& p);
+cudaError_t launch_strict_dweight(const DWeightParams& p, cudaStream_t st);
 
 // Fused pair: `configure` returns 0 when the shape does not fit the kernel (the caller then runs G and S).
 size_t configure_tensor_fused_pair(FusedParams& p, int precision);

@@ -282,22 +282,6 @@ __device__ __forceinline__ uint32_t tile_addr(uint32_t base, uint32_t seg_stride
   return row + (static_cast<uint32_t>((c & 7) ^ (r & 7)) << 4);
 }
 
-// In-place hi/lo split of one 16-byte chunk of float32 values (strict mode).
-__device__ __forceinline__ void split_chunk(uint32_t addr, uint32_t lo_offset) {
-  uint32_t v[4], lo[4];
-  asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr) : "memory");
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t hi = v[i] & 0xFFFFE000u;
-    const float rem = __uint_as_float(v[i]) - __uint_as_float(hi);
-    lo[i] = (__float_as_uint(rem) + 0x1000u) & 0xFFFFE000u;   // round to tf32 (nearest, ties away) with integer ops
-    v[i] = hi;
-  }
-  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
-  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr + lo_offset), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3])
-               : "memory");
-}
-
 template <typename T> struct Elem;
 template <> struct Elem<float> { static constexpr uint32_t fmt = 2; static constexpr bool tf32 = true; };
 template <> struct Elem<__half> { static constexpr uint32_t fmt = 0; static constexpr bool tf32 = false; };
@@ -319,15 +303,7 @@ __device__ __forceinline__ uint32_t pack2(__nv_bfloat16*, uint32_t a, uint32_t b
 // per instruction; for red.global.add that pattern measured ~3x the throughput of the row-per-thread one.
 //   emit(row_in_block, first_column, x0, x1, x2, x3) is called 8 times per lane.
 template <class Emit>
-__device__ __forceinline__ void warp_block_emit(uint32_t taddr, uint32_t tile, int lane, bool have_acc, Emit&& emit) {
-  uint32_t v[32];
-  if (have_acc) {
-    tmem_ld32(taddr, v);
-    tmem_ld_wait();
-  } else {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = 0u;
-  }
+__device__ __forceinline__ void warp_regs_emit(const uint32_t (&v)[32], uint32_t tile, int lane, Emit&& emit) {
 #pragma unroll
   for (int j = 0; j < 8; ++j)
     asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(tile + lane * 128u + (static_cast<uint32_t>(j ^ (lane & 7)) << 4)),
@@ -347,6 +323,19 @@ __device__ __forceinline__ void warp_block_emit(uint32_t taddr, uint32_t tile, i
   __syncwarp();                         // the tile may be overwritten from here on
 #pragma unroll
   for (int it = 0; it < 8; ++it) emit(it * 4 + (lane >> 3), j * 4, x[it][0], x[it][1], x[it][2], x[it][3]);
+}
+// The same straight from the accumulator (zeros where nothing was accumulated).
+template <class Emit>
+__device__ __forceinline__ void warp_block_emit(uint32_t taddr, uint32_t tile, int lane, bool have_acc, Emit&& emit) {
+  uint32_t v[32];
+  if (have_acc) {
+    tmem_ld32(taddr, v);
+    tmem_ld_wait();
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = 0u;
+  }
+  warp_regs_emit(v, tile, lane, emit);
 }
 // Same transpose for a 32-row x 64-column block (8 KB tile): every lane ends up with 8 consecutive columns of
 // one row, so 8 lanes cover 64 columns - 128 contiguous bytes of a 16-bit row per instruction.

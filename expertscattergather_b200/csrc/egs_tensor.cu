@@ -9,9 +9,7 @@
 // Stage hand-over uses mbarriers only: empty[s] (MMA completion -> producers), full[s] (data landed ->
 // MMA lane), done (all MMAs -> epilogue).  Producers never wait for their own copies: after issuing a
 // stage each thread executes cp.async.mbarrier.arrive.noinc, so the hardware arrives on full[s] when that
-// thread's copies have landed and the producers run ahead by the whole ring.  (Strict float32 is the
-// exception: it must pass the landed data through registers to split it, so there the producers wait for
-// the copy group, split in place and arrive themselves.)  Every wait is bounded: when it runs out the
+// thread's copies have landed and the producers run ahead by the whole ring.  Every wait is bounded: when it runs out the
 // thread sets the CTA's abort flag and EGS_STATUS_PIPELINE_TIMEOUT in the caller's status word, and all
 // roles fall through to the common exit, where tensor memory is released.
 //
@@ -28,10 +26,8 @@
 // whose XOR acts on 32-byte pairs with the row index modulo 4 (atoms of 4 rows; SBO = 512); float32 tiles
 // that are consumed MN-major are written in that variant.
 //
-// float32 tensors: kind::tf32.  EGS_PREC_STRICT splits every operand chunk in shared memory into
-// hi = top 19 bits and lo = tf32(x - hi) and issues lo*hi + hi*lo + hi*hi into the same accumulator, which
-// restores ~fp32 product accuracy (the reference computes fp32 dots with allow_tf32=False,
-// egs/triton_kernels.py:389).  16-bit tensors: kind::f16 with fp32 accumulation.
+// float32 tensors: kind::tf32, one TF32 product per element.  Strict float32 (three products) has its own kernels in
+// egs_strict.cu, except for the fused pair below.  16-bit tensors: kind::f16 with fp32 accumulation.
 #include "egs_tcgen05.cuh"
 
 namespace egs {
@@ -97,43 +93,18 @@ __device__ __forceinline__ bool producer_finish(const Pipe& pp, int lane, bool a
   return alive;
 }
 
-// Producer main loop.  issue(kt, stage_base) enqueues this thread's cp.async copies of stage kt;
-// split(kt, stage_base) is the strict-mode in-place hi/lo pass over the same chunks.
-template <bool STRICT, class Issue, class Split>
-__device__ __forceinline__ bool run_producer(const Pipe& pp, int lane, Issue&& issue, Split&& split) {
+// Producer main loop.  issue(kt, stage_base) enqueues this thread's cp.async copies of stage kt.
+template <class Issue>
+__device__ __forceinline__ bool run_producer(const Pipe& pp, int lane, Issue&& issue) {
   SmemHeader* hdr = pp.hdr;
   const int stages = pp.stages, nk = pp.nk;
   bool alive = true;
-  if (!STRICT) {
-    for (int kt = 0; kt < nk; ++kt) {
-      const int slot = kt % stages, use = kt / stages;
-      if (use > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[slot]), (use - 1) & 1, pp.abort_flag, pp.status.word, lane);
-      if (!alive) break;
-      issue(kt, pp.tiles0 + slot * pp.stage_bytes);
-      cp_async_mbar_arrive_noinc(smem_u32(&hdr->full[slot]));
-    }
-  } else {
-    const int dist = stages - 1;
-    for (int kt = 0; kt < dist; ++kt) {
-      if (kt < nk) issue(kt, pp.tiles0 + (kt % stages) * pp.stage_bytes);
-      cp_async_commit();
-    }
-    for (int kc = 0; kc < nk; ++kc) {
-      cp_async_wait_pending(dist - 1);
-      if (alive) {
-        split(kc, pp.tiles0 + (kc % stages) * pp.stage_bytes);
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&hdr->full[kc % stages]));
-      }
-      const int kt = kc + dist;
-      if (kt < nk && alive) {
-        const int use = kt / stages;
-        if (use > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[kt % stages]), (use - 1) & 1, pp.abort_flag, pp.status.word, lane);
-        if (alive) issue(kt, pp.tiles0 + (kt % stages) * pp.stage_bytes);
-      }
-      cp_async_commit();
-    }
+  for (int kt = 0; kt < nk; ++kt) {
+    const int slot = kt % stages, use = kt / stages;
+    if (use > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[slot]), (use - 1) & 1, pp.abort_flag, pp.status.word, lane);
+    if (!alive) break;
+    issue(kt, pp.tiles0 + slot * pp.stage_bytes);
+    cp_async_mbar_arrive_noinc(smem_u32(&hdr->full[slot]));
   }
   return producer_finish(pp, lane, alive);
 }
@@ -186,7 +157,7 @@ __device__ __forceinline__ void run_mma_lane(const Pipe& pp, Mma&& mma) {
 // MT = number of 128-row accumulator tiles per CTA (1 or 2).  With MT = 2 the CTA owns 256 expert rows: both
 // accumulators are fed from the same W tile, which cuts the bytes loaded per flop by a third and lets a
 // three-stage ring of one CTA per SM cover the load latency that two 2-stage CTAs cannot.
-template <typename T, bool STRICT, bool SCATTER, int MT>
+template <typename T, bool SCATTER, int MT>
 __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_rowgemm_kernel(RowGemmParams p) {
   constexpr int kRows = kTileM * MT;        // expert rows per CTA
   constexpr int ES = sizeof(T);
@@ -209,16 +180,14 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_rowgemm_kern
   const uint32_t a_bytes = kRows * 128u;
   const int nseg_b = (p.BN * ES + 127) / 128;
   const uint32_t b_bytes = w_nc ? static_cast<uint32_t>(p.BN) * 128u : static_cast<uint32_t>(nseg_b) * KE * 128u;
-  const uint32_t a_lo_off = a_bytes;                                   // strict: A_hi | A_lo | B_hi | B_lo
-  const uint32_t b_off = STRICT ? 2u * a_bytes : a_bytes;
-  const uint32_t b_lo_off = b_bytes;
+  const uint32_t b_off = a_bytes;
 
   Pipe pp;
   pp.hdr = hdr;
   pp.abort_flag = &hdr->abort_flag;
   pp.status = p.status;
   pp.tiles0 = smem_u32(smem) + kHeaderBytes;
-  pp.stage_bytes = (a_bytes + b_bytes) * (STRICT ? 2u : 1u);
+  pp.stage_bytes = a_bytes + b_bytes;
   pp.stages = p.stages;
   pp.nk = (p.C + KE - 1) / KE;
 
@@ -244,7 +213,7 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_rowgemm_kern
   }
   const uint32_t acc_cols = tmem_cols_for(p.BN);      // columns of one accumulator
   const uint32_t tmem_cols = acc_cols * MT;
-  const uint32_t tmem_base = pipe_setup(pp, STRICT ? kProducerWarps : kProducerThreads, tmem_cols, tid, warp);
+  const uint32_t tmem_base = pipe_setup(pp, kProducerThreads, tmem_cols, tid, warp);
   const bool run = (hdr->abort_flag == 0u);
 
   if (!run) {
@@ -345,34 +314,6 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_rowgemm_kern
           cp_async16_full(db + static_cast<uint32_t>(r) * 128u + cn_swz(r), src);
       }
     };
-    // strict float32: when this thread's chunk list has the fixed 4 + 4 shape the in-place hi/lo split reads all
-    // of its chunks first (the loads pipeline) and only then splits and stores them
-    const bool split_batched = STRICT && MT == 1 && (w_nc ? nb_iters <= 4 : (cn_fast && KE % cn_rstep == 0 && KE / cn_rstep <= 4));
-    auto split_stage_batched = [&](int, uint32_t base) {
-      uint32_t dst[8];
-      bool on[8];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        dst[i] = base + rc_dst0 + i * 4096u;
-        on[i] = true;
-        if (w_nc) {
-          dst[4 + i] = base + b_off + rc_dst0 + i * 4096u;
-          on[4 + i] = i < nb_iters && r0 + 32 * i < p.BN;
-        } else {
-          const int rr = cn_r0 + i * cn_rstep;
-          dst[4 + i] = base + b_off + cn_dst_seg + static_cast<uint32_t>(rr) * 128u +
-                       (static_cast<uint32_t>(((cn_c & 7) >> 1) ^ (rr & 3)) << 5) + (static_cast<uint32_t>(cn_c & 1) << 4);
-          on[4 + i] = rr < KE;
-        }
-      }
-      uint4 r[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (on[i]) r[i] = lds16(dst[i]);
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (on[i]) split_store(dst[i], i < 4 ? a_lo_off : b_lo_off, r[i]);
-    };
     auto issue_stage = [&](int kt, uint32_t base) {
       if (tile_full && (kt + 1) * KE <= p.C) {
         issue_full(kt, base);
@@ -380,23 +321,7 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_rowgemm_kern
         for_each_chunk(kt, base, [&](uint32_t dst, const char* src, bool v, bool) { cp_async16(dst, v ? src : W, v ? 16u : 0u); });
       }
     };
-    bool alive;
-    if (split_batched) alive = run_producer<STRICT>(pp, lane, issue_stage, split_stage_batched);
-    else
-    alive = run_producer<STRICT>(
-        pp, lane,
-        [&](int kt, uint32_t base) {
-          if (tile_full && (kt + 1) * KE <= p.C) {
-            issue_full(kt, base);
-          } else {
-            for_each_chunk(kt, base, [&](uint32_t dst, const char* src, bool v, bool) { cp_async16(dst, v ? src : W, v ? 16u : 0u); });
-          }
-        },
-        [&](int kc, uint32_t base) {
-          for_each_chunk(kc, base, [&](uint32_t dst, const char*, bool, bool is_b) {
-            split_chunk(dst, is_b ? b_lo_off : a_lo_off);
-          });
-        });
+    const bool alive = run_producer(pp, lane, issue_stage);
 
     // =========================== epilogue ===========================
     // The stage ring is idle once `done` has completed: its first 32 KB serve as the warps' transpose tiles.
@@ -510,32 +435,19 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_rowgemm_kern
       const uint64_t a_adv = 32u >> 4, b_adv = b_step >> 4;
       run_mma_lane(pp, [&](int ks, uint32_t a_hi) {
         const uint32_t b_hi = a_hi + b_off;
-        const int kq0 = 0, kq1 = min(KE / UK, (p.C - ks * KE + UK - 1) / UK);
-        uint64_t ad[MT], adl[MT];
+        const int kq1 = min(KE / UK, (p.C - ks * KE + UK - 1) / UK);
+        uint64_t ad[MT];
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          ad[mt] = make_smem_desc(a_hi + mt * (kTileM * 128u), 16u, 1024u) + kq0 * a_adv;
-          adl[mt] = STRICT ? make_smem_desc(a_hi + mt * (kTileM * 128u) + a_lo_off, 16u, 1024u) + kq0 * a_adv : 0ull;
-        }
-        uint64_t bd = make_smem_desc(b_hi, b_lbo, b_sbo, b_lay) + kq0 * b_adv;
-        uint64_t bdl = STRICT ? make_smem_desc(b_hi + b_lo_off, b_lbo, b_sbo, b_lay) + kq0 * b_adv : 0ull;
-        for (int kq = kq0; kq < kq1; ++kq) {
+        for (int mt = 0; mt < MT; ++mt) ad[mt] = make_smem_desc(a_hi + mt * (kTileM * 128u), 16u, 1024u);
+        uint64_t bd = make_smem_desc(b_hi, b_lbo, b_sbo, b_lay);
+        for (int kq = 0; kq < kq1; ++kq) {
           const uint32_t acc = (ks > 0 || kq > 0) ? 1u : 0u;
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt) {
-            const uint32_t d = tmem_base + mt * acc_cols;
-            if (STRICT) {
-              umma<Elem<T>::tf32>(d, adl[mt], bd, idesc, acc);
-              umma<Elem<T>::tf32>(d, ad[mt], bdl, idesc, 1u);
-              umma<Elem<T>::tf32>(d, ad[mt], bd, idesc, 1u);
-            } else {
-              umma<Elem<T>::tf32>(d, ad[mt], bd, idesc, acc);
-            }
+            umma<Elem<T>::tf32>(tmem_base + mt * acc_cols, ad[mt], bd, idesc, acc);
             ad[mt] += a_adv;
-            adl[mt] += a_adv;
           }
           bd += b_adv;
-          bdl += b_adv;
         }
       });
     }
@@ -951,7 +863,7 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
 //   the same B tile: a third fewer bytes loaded per flop, which is what bounds this kernel once the contraction
 //   is long (the loads of two 128 x 256 CTAs per SM top out well below the tensor rate).
 // ------------------------------------------------------------------------------------------------
-template <typename T, bool STRICT, int MT>
+template <typename T, int MT>
 __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_dweight_kernel(DWeightParams p) {
   constexpr int ES = sizeof(T);
   constexpr int KR = 128 / ES;          // contraction rows per stage (4 MMAs of UK rows)
@@ -981,16 +893,14 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_dweight_kern
   const uint32_t seg_stride = KR * 128u;
   const uint32_t a_bytes = NSEG_A * seg_stride;
   const uint32_t b_bytes = static_cast<uint32_t>(nseg_b) * seg_stride;
-  const uint32_t a_lo_off = a_bytes;
-  const uint32_t b_off = STRICT ? 2u * a_bytes : a_bytes;
-  const uint32_t b_lo_off = b_bytes;
+  const uint32_t b_off = a_bytes;
 
   Pipe pp;
   pp.hdr = hdr;
   pp.abort_flag = &hdr->abort_flag;
   pp.status = p.status;
   pp.tiles0 = smem_u32(smem) + kHeaderBytesD + table_bytes;
-  pp.stage_bytes = (a_bytes + b_bytes) * (STRICT ? 2u : 1u);
+  pp.stage_bytes = a_bytes + b_bytes;
   pp.stages = p.stages;
   pp.nk = (rows + KR - 1) / KR;
 
@@ -1021,7 +931,7 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_dweight_kern
   }
   const uint32_t acc_cols = tmem_cols_for(p.BN);
   const uint32_t tmem_cols = acc_cols * MT;
-  const uint32_t tmem_base = pipe_setup(pp, STRICT ? kProducerWarps : kProducerThreads, tmem_cols, tid, warp);
+  const uint32_t tmem_base = pipe_setup(pp, kProducerThreads, tmem_cols, tid, warp);
   const bool run = (hdr->abort_flag == 0u);
 
   if (!run) {
@@ -1130,26 +1040,6 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_dweight_kern
       }
       b_next_kt = kt + 1;
     };
-    const bool split_batched = STRICT && MT == 1 && KR / a_rstep <= 4 && b_fast && KR % b_rstep == 0 && KR / b_rstep <= 4;
-    auto split_stage_batched = [&](int, uint32_t base) {
-      uint32_t dst[8];
-      bool on[8];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int ra = a_r0 + i * a_rstep, rb = b_r0 + i * b_rstep;
-        dst[i] = base + a_dst_seg + static_cast<uint32_t>(ra) * 128u + swz(a_c, ra);
-        on[i] = ra < KR;
-        dst[4 + i] = base + b_off + b_dst_seg + static_cast<uint32_t>(rb) * 128u + swz(b_c, rb);
-        on[4 + i] = rb < KR;
-      }
-      uint4 r[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (on[i]) r[i] = lds16(dst[i]);
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (on[i]) split_store(dst[i], i < 4 ? a_lo_off : b_lo_off, r[i]);
-    };
     auto issue_stage = [&](int kt, uint32_t base) {
       // the lean path walks b_ptr stage by stage, so it serves a prefix of consecutive full stages
       if (tile_full && kt == b_next_kt && (kt + 1) * KR <= rows) {
@@ -1158,24 +1048,7 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_dweight_kern
         for_each_chunk(kt, base, true, [&](uint32_t dst, const char* src, bool v, bool) { cp_async16(dst, v ? src : Xs, v ? 16u : 0u); });
       }
     };
-    bool alive;
-    if (split_batched) alive = run_producer<STRICT>(pp, lane, issue_stage, split_stage_batched);
-    else
-    alive = run_producer<STRICT>(
-        pp, lane,
-        [&](int kt, uint32_t base) {
-          // the lean path walks b_ptr stage by stage, so it serves a prefix of consecutive full stages
-          if (tile_full && kt == b_next_kt && (kt + 1) * KR <= rows) {
-            issue_full(kt, base);
-          } else {
-            for_each_chunk(kt, base, true, [&](uint32_t dst, const char* src, bool v, bool) { cp_async16(dst, v ? src : Xs, v ? 16u : 0u); });
-          }
-        },
-        [&](int kc, uint32_t base) {
-          for_each_chunk(kc, base, false, [&](uint32_t dst, const char*, bool, bool is_b) {
-            split_chunk(dst, is_b ? b_lo_off : a_lo_off);
-          });
-        });
+    const bool alive = run_producer(pp, lane, issue_stage);
 
     // epilogue
     if (alive) {
@@ -1238,21 +1111,13 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_dweight_kern
         const int nkq = min(KR / UK, (rrem + UK - 1) / UK);
         uint64_t ad = make_smem_desc(a_hi, seg_stride, kMnSbo, kMnLayout);
         uint64_t bd = make_smem_desc(b_hi, seg_stride, kMnSbo, kMnLayout);
-        uint64_t adl = STRICT ? make_smem_desc(a_hi + a_lo_off, seg_stride, kMnSbo, kMnLayout) : 0ull;
-        uint64_t bdl = STRICT ? make_smem_desc(b_hi + b_lo_off, seg_stride, kMnSbo, kMnLayout) : 0ull;
         // second accumulator (MT = 2): features 128..255 of the A tile, ES segments further on
         const uint64_t a_mt_adv = (static_cast<uint32_t>(ES) * seg_stride) >> 4;
         for (int kq = 0; kq < nkq; ++kq) {
           const uint32_t acc = (ks > 0 || kq > 0) ? 1u : 0u;
-          if (STRICT) {
-            umma<Elem<T>::tf32>(tmem_base, adl, bd, idesc, acc);
-            umma<Elem<T>::tf32>(tmem_base, ad, bdl, idesc, 1u);
-            umma<Elem<T>::tf32>(tmem_base, ad, bd, idesc, 1u);
-          } else {
-            umma<Elem<T>::tf32>(tmem_base, ad, bd, idesc, acc);
-            if (MT == 2) umma<Elem<T>::tf32>(tmem_base + acc_cols, ad + a_mt_adv, bd, idesc, acc);
-          }
-          ad += k_adv; bd += k_adv; adl += k_adv; bdl += k_adv;
+          umma<Elem<T>::tf32>(tmem_base, ad, bd, idesc, acc);
+          if (MT == 2) umma<Elem<T>::tf32>(tmem_base + acc_cols, ad + a_mt_adv, bd, idesc, acc);
+          ad += k_adv; bd += k_adv;
         }
       });
     }
@@ -1630,18 +1495,11 @@ int pick_stages(size_t fixed_bytes, size_t stage_bytes, long long ctas, bool all
 
 }  // namespace
 
-size_t configure_tensor_rowgemm(RowGemmParams& p, bool scatter, int dtype, int precision) {
+size_t configure_tensor_rowgemm(RowGemmParams& p, bool scatter, int dtype) {
   const int es = (dtype == EGS_F32) ? 4 : 2;
-  const bool strict = (dtype == EGS_F32 && precision == EGS_PREC_STRICT);
   const int ke = 128 / es;
   int bn = (p.N + 15) & ~15;
-  const int cap = strict ? 128 : 256;
-  if (bn > cap) bn = cap;
-  // strict float32 doubles every tile (hi + lo): when the grid is larger than one wave, 64-wide tiles keep a
-  // 2-stage ring under half an SM's shared memory so that two CTAs share an SM
-  if (strict && bn > 64 &&
-      static_cast<long long>((p.M + kTileM - 1) / kTileM) * ((p.N + bn - 1) / bn) * p.E > kSmCount)
-    bn = 64;
+  if (bn > 256) bn = 256;
   p.BN = bn;
   const size_t nseg_b = (static_cast<size_t>(bn) * es + 127) / 128;
   const size_t b_bytes = (p.w_layout == EGS_W_NC) ? static_cast<size_t>(bn) * 128 : nseg_b * ke * 128;
@@ -1651,10 +1509,10 @@ size_t configure_tensor_rowgemm(RowGemmParams& p, bool scatter, int dtype, int p
   // enough for the deeper ring to matter, and the two accumulators fit in tensor memory
   const long long ctas2 = static_cast<long long>((p.M + 2 * kTileM - 1) / (2 * kTileM)) * n_tiles * p.E;
   // (the scatter epilogue dominates short contractions and profits from two CTAs per SM instead)
-  const bool want2 = !strict && p.M >= 2 * kTileM && ctas2 >= kSmCount && p.C * es >= (scatter ? 4096 : 1024);
+  const bool want2 = p.M >= 2 * kTileM && ctas2 >= kSmCount && p.C * es >= (scatter ? 4096 : 1024);
   p.row_tiles = want2 ? 2 : 1;
   const size_t a_bytes = static_cast<size_t>(kTileM) * p.row_tiles * 128;
-  const size_t stage_bytes = (a_bytes + b_bytes) * (strict ? 2 : 1);
+  const size_t stage_bytes = a_bytes + b_bytes;
   const long long ctas = static_cast<long long>((p.M + kTileM * p.row_tiles - 1) / (kTileM * p.row_tiles)) * n_tiles * p.E;
   // persistent variant (see its kernel): scatter problems with many tiles, non-strict arithmetic
   const long long tiles1 = static_cast<long long>((p.M + kTileM - 1) / kTileM) * n_tiles * p.E;
@@ -1662,7 +1520,7 @@ size_t configure_tensor_rowgemm(RowGemmParams& p, bool scatter, int dtype, int p
   // direct 16-bit scatter adds go out as bulk reductions
   p.bulk_epilogue = (scatter && es == 2) ? 1 : 0;
   // (measured: it wins for contractions of up to four stages - the scatter of cfg4 and cfg2 - and loses for longer ones)
-  if (!strict && scatter && p.C * es <= 512 && tiles1 >= 2 * kSmCount) {
+  if (scatter && p.C * es <= 512 && tiles1 >= 2 * kSmCount) {
     const size_t st1 = static_cast<size_t>(kTileM) * 128 + b_bytes;
     size_t fixed_p = kPersistHeaderBytes + kPersistMaxEpilogueWarps * 4096;
     // 16-bit scatter: staging buffers for the bulk adds when the ring keeps three stages
@@ -1683,33 +1541,27 @@ size_t configure_tensor_rowgemm(RowGemmParams& p, bool scatter, int dtype, int p
   return fixed + p.stages * stage_bytes;
 }
 
-size_t configure_tensor_dweight(DWeightParams& p, int dtype, int precision) {
+size_t configure_tensor_dweight(DWeightParams& p, int dtype) {
   const int es = (dtype == EGS_F32) ? 4 : 2;
-  const bool strict = (dtype == EGS_F32 && precision == EGS_PREC_STRICT);
   const int kr = 128 / es;
   int bn = (p.FD + 15) & ~15;
-  const int cap = strict ? 64 : 256;   // strict: 64-wide tiles so that two CTAs share an SM
-  if (bn > cap) bn = cap;
+  if (bn > 256) bn = 256;
   p.BN = bn;
   const size_t seg_stride = static_cast<size_t>(kr) * 128;
   const size_t nseg_b = (static_cast<size_t>(bn) * es + 127) / 128;
   // 256-feature CTAs (two accumulators): long contractions whose grid still covers the SMs, non-strict only
   const long long tiles2 = static_cast<long long>((p.FG + 2 * kTileM - 1) / (2 * kTileM)) * ((p.FD + bn - 1) / bn) * p.E;
-  const bool want2 = !strict && p.FG > kTileM && tiles2 >= kSmCount && p.M >= 16 * kr && bn * 2 <= 512;
+  const bool want2 = p.FG > kTileM && tiles2 >= kSmCount && p.M >= 16 * kr && bn * 2 <= 512;
   p.row_tiles = want2 ? 2 : 1;
   const size_t a_bytes = es * seg_stride * p.row_tiles;
-  const size_t stage_bytes = (a_bytes + nseg_b * seg_stride) * (strict ? 2 : 1);
+  const size_t stage_bytes = a_bytes + nseg_b * seg_stride;
   // split the contraction so that the grid fills one wave of CTAs and no CTA owns more rows than the
   // shared-memory row table holds
   const int f_tile = kTileM * p.row_tiles;
   const long long tiles = static_cast<long long>((p.FG + f_tile - 1) / f_tile) * ((p.FD + bn - 1) / bn) * p.E;
   // as many row ranges as still fit in one wave of CTAs (two CTAs per SM with 128-feature tiles)
   long long want = (static_cast<long long>(kSmCount) * (p.row_tiles == 2 ? 1 : 2)) / tiles;
-  // Strict float32: the tensor core adds every product group into the float32 accumulator with truncation, an error that
-  // grows with the number of accumulation steps (measured 1.5e-5 of max|ref| after 8192 contraction rows, against a
-  // 1e-5 bar).  Ranges of at most 1024 rows keep it near 3e-6; the partial tiles are then summed by float32 atomics,
-  // which round correctly.
-  const int max_rows = strict ? 1024 : kMaxRowsPerSplit;
+  const int max_rows = kMaxRowsPerSplit;
   const long long min_splits = (p.M + max_rows - 1) / max_rows;
   if (want < min_splits) want = min_splits;
   const long long max_splits = (p.M + kr - 1) / kr;
@@ -1755,8 +1607,7 @@ size_t configure_tensor_fused_pair(FusedParams& p, int precision) {
   return fixed + ns * stage_bytes;
 }
 
-cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, int dtype, int precision, size_t smem_bytes,
-                                  cudaStream_t st) {
+cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, int dtype, size_t smem_bytes, cudaStream_t st) {
   if (p.persistent) {
     const int row_blocks = p.E * ((p.M + kTileM - 1) / kTileM);
     dim3 pgrid(row_blocks < kSmCount ? row_blocks : kSmCount);
@@ -1785,29 +1636,24 @@ cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, int dtyp
   dim3 grid(p.expert_fastest ? p.E : row_tiles, (p.N + p.BN - 1) / p.BN, p.expert_fastest ? row_tiles : p.E);
   dim3 block(kThreads);
   cudaError_t err = cudaSuccess;
-#define EGS_LAUNCH2(TY, STRICT, SC, MTV)                                                              \
-  do {                                                                                                \
-    err = (ensure_smem_optin<tensor_rowgemm_kernel<TY, STRICT, SC, MTV>>(static_cast<int>(kSmemMaxPerCta)));                          \
-    if (err == cudaSuccess) tensor_rowgemm_kernel<TY, STRICT, SC, MTV><<<grid, block, smem_bytes, st>>>(p); \
+#define EGS_LAUNCH2(TY, SC, MTV)                                                                                \
+  do {                                                                                                          \
+    err = (ensure_smem_optin<tensor_rowgemm_kernel<TY, SC, MTV>>(static_cast<int>(kSmemMaxPerCta)));            \
+    if (err == cudaSuccess) tensor_rowgemm_kernel<TY, SC, MTV><<<grid, block, smem_bytes, st>>>(p);             \
   } while (0)
-#define EGS_LAUNCH(TY, STRICT)                                        \
-  do {                                                                \
-    if (scatter) {                                                    \
-      if (p.row_tiles == 2 && !STRICT) EGS_LAUNCH2(TY, false, true, 2);  \
-      else EGS_LAUNCH2(TY, STRICT, true, 1);                          \
-    } else {                                                          \
-      if (p.row_tiles == 2 && !STRICT) EGS_LAUNCH2(TY, false, false, 2); \
-      else EGS_LAUNCH2(TY, STRICT, false, 1);                         \
-    }                                                                 \
+#define EGS_LAUNCH(TY)                                  \
+  do {                                                  \
+    if (scatter) {                                      \
+      if (p.row_tiles == 2) EGS_LAUNCH2(TY, true, 2);   \
+      else EGS_LAUNCH2(TY, true, 1);                    \
+    } else {                                            \
+      if (p.row_tiles == 2) EGS_LAUNCH2(TY, false, 2);  \
+      else EGS_LAUNCH2(TY, false, 1);                   \
+    }                                                   \
   } while (0)
-  if (dtype == EGS_F32) {
-    if (precision == EGS_PREC_STRICT) EGS_LAUNCH(float, true);
-    else EGS_LAUNCH(float, false);
-  } else if (dtype == EGS_F16) {
-    EGS_LAUNCH(__half, false);
-  } else {
-    EGS_LAUNCH(__nv_bfloat16, false);
-  }
+  if (dtype == EGS_F32) EGS_LAUNCH(float);
+  else if (dtype == EGS_F16) EGS_LAUNCH(__half);
+  else EGS_LAUNCH(__nv_bfloat16);
 #undef EGS_LAUNCH
 #undef EGS_LAUNCH2
   if (err != cudaSuccess) return err;
@@ -1815,29 +1661,24 @@ cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, int dtyp
   return cudaGetLastError();
 }
 
-cudaError_t launch_tensor_dweight(const DWeightParams& p, int dtype, int precision, size_t smem_bytes, cudaStream_t st) {
+cudaError_t launch_tensor_dweight(const DWeightParams& p, int dtype, size_t smem_bytes, cudaStream_t st) {
   const int f_tile = kTileM * p.row_tiles;
   dim3 grid((p.FG + f_tile - 1) / f_tile, (p.FD + p.BN - 1) / p.BN, p.E * p.splits);
   dim3 block(kThreads);
   cudaError_t err = cudaSuccess;
-#define EGS_LAUNCH_D(TY, STRICT, MTV)                                                           \
-  do {                                                                                          \
-    err = (ensure_smem_optin<tensor_dweight_kernel<TY, STRICT, MTV>>(static_cast<int>(kSmemMaxPerCta)));                        \
-    if (err == cudaSuccess) tensor_dweight_kernel<TY, STRICT, MTV><<<grid, block, smem_bytes, st>>>(p); \
+#define EGS_LAUNCH_D(TY, MTV)                                                                                   \
+  do {                                                                                                          \
+    err = (ensure_smem_optin<tensor_dweight_kernel<TY, MTV>>(static_cast<int>(kSmemMaxPerCta)));                \
+    if (err == cudaSuccess) tensor_dweight_kernel<TY, MTV><<<grid, block, smem_bytes, st>>>(p);                 \
   } while (0)
-#define EGS_LAUNCH(TY, STRICT)                                   \
-  do {                                                           \
-    if (p.row_tiles == 2 && !STRICT) EGS_LAUNCH_D(TY, false, 2); \
-    else EGS_LAUNCH_D(TY, STRICT, 1);                            \
+#define EGS_LAUNCH(TY)                          \
+  do {                                          \
+    if (p.row_tiles == 2) EGS_LAUNCH_D(TY, 2);  \
+    else EGS_LAUNCH_D(TY, 1);                   \
   } while (0)
-  if (dtype == EGS_F32) {
-    if (precision == EGS_PREC_STRICT) EGS_LAUNCH(float, true);
-    else EGS_LAUNCH(float, false);
-  } else if (dtype == EGS_F16) {
-    EGS_LAUNCH(__half, false);
-  } else {
-    EGS_LAUNCH(__nv_bfloat16, false);
-  }
+  if (dtype == EGS_F32) EGS_LAUNCH(float);
+  else if (dtype == EGS_F16) EGS_LAUNCH(__half);
+  else EGS_LAUNCH(__nv_bfloat16);
 #undef EGS_LAUNCH
 #undef EGS_LAUNCH_D
   if (err != cudaSuccess) return err;

@@ -75,3 +75,38 @@ def test_expert_row_sum(cuda_device, B, T, E, K, N, dtype, gathered):
     assert rc == _lib.OK
     rows = torch.gather(src.double(), 1, Ind.reshape(B, -1, 1).expand(-1, -1, N)).reshape(B, E, K, N) if gathered else src.double()
     assert torch.equal(out.cpu(), rows.sum((0, 2)).to(dtype))       # integers: exact in float32, rounded once
+
+
+# strict float32 kernels: tile widths 32 / 64 / 96 / 128 with partial last tiles, contractions around one step (32), one chunk
+# (512) and several, rows around one block of 128, one and several row ranges of D (1024 rows each)
+@pytest.mark.parametrize("B,T,E,K,I,J", [(1, 4, 1, 1, 4, 4), (3, 60, 2, 43, 36, 28), (5, 90, 3, 51, 516, 68), (4, 200, 2, 65, 1028, 136),
+                                         (2, 300, 1, 128, 2048, 200), (9, 400, 2, 230, 544, 96), (2, 50, 70, 9, 260, 140)])
+def test_strict_float32_edges(cuda_device, B, T, E, K, I, J):
+    w = Workload("strict", B, T, E, K, I, J, torch.float32, "replace", 78)
+    exact = workloads.make_inputs(w, integer_valued=True)           # every product and sum is exact: bit for bit
+    exact["Ind"][B - 1, E - 1, K - 1] = T                           # out of range: skipped
+    ref = orc.np_step(exact["X"], exact["Wg"], exact["Ws"], exact["Ind"].clamp(0, T - 1), exact["G"])
+    ops.reset_status()
+    d = {k: v.to(cuda_device) for k, v in exact.items()}
+    Y = ops.gather_gemm(d["X"], d["Wg"], d["Ind"], path="tensor")
+    dY = ops.gather_gemm(d["G"], d["Ws"], d["Ind"], w_layout="nc", path="tensor")
+    ref["Y"][B - 1, E - 1, K - 1] = 0
+    ref["dY"][B - 1, E - 1, K - 1] = 0
+    assert np.array_equal(Y.cpu().double().numpy(), ref["Y"]) and np.array_equal(dY.cpu().double().numpy(), ref["dY"])
+    safe = exact["Ind"].clamp(0, T - 1)                             # the masked slot's row of Y is zero: it adds nothing
+    Yc, dYc = Y.cpu(), dY.cpu()
+    Out = ops.gemm_scatter(Y, d["Ws"], d["Ind"], T, path="tensor")
+    dX = ops.gemm_scatter(dY, d["Wg"], d["Ind"], T, w_layout="nc", path="tensor")
+    assert np.array_equal(Out.cpu().double().numpy(), orc.np_scatter(Yc, exact["Ws"], safe, T))
+    assert np.array_equal(dX.cpu().double().numpy(), orc.np_scatter(dYc, exact["Wg"].transpose(1, 2).contiguous(), safe, T))
+    dWg = ops.dweight(d["X"], dY, d["Ind"], path="tensor")
+    dWs = ops.dweight(d["G"], Y, d["Ind"], out_layout="direct_rows", path="tensor")
+    assert np.array_equal(dWg.cpu().double().numpy(), orc.np_dweight(exact["X"], dYc, safe))
+    assert np.array_equal(dWs.cpu().double().numpy(), orc.np_dweight(exact["G"], Yc, safe).transpose(0, 2, 1))
+    with pytest.raises(RuntimeError, match="outside"):
+        ops.check_status()
+    real = workloads.make_inputs(w)                                 # and the float32 bar of the parity tests on real values
+    truth = orc.np_step(real["X"], real["Wg"], real["Ws"], real["Ind"], real["G"])
+    got = gpu_step(real, cuda_device, "tensor")
+    for k in STEP_KEYS:
+        assert orc.rel_err(got[k], truth[k]) <= 1e-5, k
