@@ -131,13 +131,14 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
   const bool no_work = (d.B * d.E * d.K == 0);
   if (!no_work && (!A || !W || !Ind) && d.C > 0) return EGS_ERR_INVALID_ARGUMENT;
 
-  // 16-bit scatter.  Workspace layout: [plan flag, 256 B][per-token counters, B*T ints][float32 rows, B*T*N].
-  // Generic kernels always sum in the float32 rows; the tensor-core path lets a planning kernel decide per call
-  // between those and direct 16-bit additions (see egs_generic.cu).
+  // 16-bit scatter.  Workspace layout: [256 B unused][planning flags, B ints in room for B*T][float32 rows, B*T*N].  Generic
+  // kernels always sum in the float32 rows; the tensor-core path decides per batch element between those and direct 16-bit
+  // additions (see egs_generic.cu).
   const bool f32_rows = scatter && dtype != EGS_F32;
   const size_t n_out = static_cast<size_t>(out_rows) * d.N;
   float* acc = nullptr;
   int* plan = nullptr;
+  bool own = false;                       // the call's previous launch is a kernel of ours that triggers its dependents early
   const bool eligible = device_is_sm100() && rowgemm_tensor_ok(d, dtype, A, W, Out);
   if ((path == EGS_PATH_TENSOR || path == EGS_PATH_PAIRED) && !eligible) return EGS_ERR_UNSUPPORTED;
   // Strict float32 on long contractions: the tensor core's accumulator additions truncate, and the error grows with the
@@ -152,20 +153,14 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
     if (!workspace || workspace_bytes < need || !aligned16(workspace)) return EGS_ERR_WORKSPACE;
     char* ws = static_cast<char*>(workspace);
     const size_t counter_bytes = (static_cast<size_t>(out_rows) * sizeof(int) + 255) & ~static_cast<size_t>(255);
-    int* counters = reinterpret_cast<int*>(ws + 256);
     acc = reinterpret_cast<float*>(ws + 256 + counter_bytes);
     cudaError_t err;
     if (tensor && !no_work && d.C > 0) {
-      plan = reinterpret_cast<int*>(ws);
-      if (csr_info) {   // a CSR of this Ind has been built: its heaviest-row figure decides, no pass over Ind
-        err = launch_plan_from_info(csr_info, kDirect16Limit, plan, status, st);
-      } else {
-        err = launch_fill_zero(ws, 256 + counter_bytes, st);
-        if (err == cudaSuccess)
-          err = launch_scatter_plan(Ind, index_dtype, static_cast<int>(d.B), static_cast<int>(d.T), static_cast<int>(d.E),
-                                    static_cast<int>(d.K), counters, plan, kDirect16Limit, status, st);
-      }
-      if (err == cudaSuccess) err = launch_scatter_init(plan, acc, Out, n_out, zero_output, dtype, st);
+      plan = reinterpret_cast<int*>(ws + 256);
+      err = launch_scatter_prepare(Ind, index_dtype, static_cast<int>(d.B), static_cast<int>(d.T), static_cast<int>(d.E),
+                                   static_cast<int>(d.K), csr_info, kDirect16Limit, plan, acc, Out, static_cast<int>(d.N),
+                                   zero_output, dtype, status_ref(status), st);
+      own = true;
     } else {
       err = zero_output ? launch_fill_zero(acc, n_out * sizeof(float), st) : launch_convert_to_f32(Out, acc, n_out, dtype, st);
     }
@@ -173,10 +168,11 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
   } else if (scatter && zero_output) {
     cudaError_t err = launch_fill_zero(Out, out_bytes, st);
     if (err != cudaSuccess) return fail_cuda(err, "fill_zero");
+    own = true;
   }
   auto finish_rows = [&]() -> int {
     if (!f32_rows) return EGS_OK;
-    cudaError_t err = plan ? launch_scatter_finish(plan, acc, Out, n_out, dtype, st)
+    cudaError_t err = plan ? launch_scatter_finish(plan, acc, Out, static_cast<int>(d.B), static_cast<size_t>(d.T) * d.N, dtype, st)
                            : launch_convert_from_f32(acc, Out, n_out, dtype, st);
     return err == cudaSuccess ? EGS_OK : fail_cuda(err, "scatter scratch convert");
   };
@@ -195,6 +191,7 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
   p.C = static_cast<int>(d.C); p.N = static_cast<int>(d.N);
   p.M = static_cast<int>(d.B * d.K);
   p.w_layout = w_layout; p.index_dtype = index_dtype;
+  p.after_own = own ? 1 : 0;
 
   cudaError_t err;
   if (tensor) {
@@ -393,6 +390,7 @@ int egs_gather_scatter_pair(const void* Src, const void* W1, const void* W2, con
     if (zero_output && dst_bytes > 0) {
       cudaError_t err = launch_fill_zero(Dst, dst_bytes, st);
       if (err != cudaSuccess) return fail_cuda(err, "fill_zero");
+      p.after_own = 1;
     }
     if (no_work) return EGS_OK;
     p.Dst = static_cast<float*>(Dst);
@@ -416,14 +414,12 @@ int egs_gather_scatter_pair(const void* Src, const void* W1, const void* W2, con
   if (!workspace || workspace_bytes < need || !aligned16(workspace)) return EGS_ERR_WORKSPACE;
   char* ws = static_cast<char*>(workspace);
   const size_t counter_bytes = (static_cast<size_t>(B) * T * sizeof(int) + 255) & ~static_cast<size_t>(255);
-  int* plan = reinterpret_cast<int*>(ws);
-  int* counters = reinterpret_cast<int*>(ws + 256);
+  int* plan = reinterpret_cast<int*>(ws + 256);
   float* acc = reinterpret_cast<float*>(ws + 256 + counter_bytes);
-  cudaError_t err = launch_fill_zero(ws, 256 + counter_bytes, st);
-  if (err == cudaSuccess)
-    err = launch_scatter_plan(Ind, index_dtype, p.B, p.T, p.E, p.K, counters, plan, kDirect16Limit, status_word, st);
-  if (err == cudaSuccess) err = launch_scatter_init(plan, acc, Dst, n_dst, zero_output, dtype, st);
-  if (err != cudaSuccess) return fail_cuda(err, "scatter scratch init");
+  cudaError_t err = launch_scatter_prepare(Ind, index_dtype, p.B, p.T, p.E, p.K, nullptr, kDirect16Limit, plan, acc, Dst, p.N2, zero_output,
+                                           dtype, status_ref(status_word), st);
+  if (err != cudaSuccess) return fail_cuda(err, "scatter preparation");
+  p.after_own = 1;
   p.Dst = acc; p.Out16 = Dst; p.plan = plan;
   const double act_bytes = static_cast<double>(B) * T * N2 * 4.0;
   const double w_bytes = static_cast<double>(E) * N1 * (static_cast<double>(C1) + N2) * elem_size(dtype);
@@ -435,7 +431,7 @@ int egs_gather_scatter_pair(const void* Src, const void* W1, const void* W2, con
   if (smem == 0) return EGS_ERR_UNSUPPORTED;
   err = launch_tensor_pair16(p, dtype, smem, st);
   if (err != cudaSuccess) return fail_cuda(err, "gather_scatter_pair launch");
-  err = launch_scatter_finish(plan, acc, Dst, n_dst, dtype, st);
+  err = launch_scatter_finish(plan, acc, Dst, p.B, static_cast<size_t>(p.T) * p.N2, dtype, st);
   return err == cudaSuccess ? EGS_OK : fail_cuda(err, "scatter scratch convert");
 }
 
@@ -509,12 +505,13 @@ static int dweight_impl(const void* Xsrc, const void* Ysrc, const void* Ind, voi
     if (!(out_is_zero && dtype == EGS_F32)) {
       err = launch_fill_zero(p.acc, n_out * sizeof(float), st);
       if (err != cudaSuccess) return fail_cuda(err, "fill_zero");
+      p.after_own = 1;
     }
   }
   err = strict ? launch_strict_dweight(p, st) : tensor ? launch_tensor_dweight(p, dtype, smem, st) : launch_generic_dweight(p, dtype, st);
   if (err != cudaSuccess) return fail_cuda(err, "dweight launch");
   if (p.splits > 1 && dtype != EGS_F32) {
-    err = launch_convert_from_f32(p.acc, out, n_out, dtype, st);
+    err = launch_convert_from_f32(p.acc, out, n_out, dtype, st, tensor);   // (the tensor-core kernel triggers its dependents)
     if (err != cudaSuccess) return fail_cuda(err, "convert launch");
   }
   return EGS_OK;

@@ -390,6 +390,7 @@ __global__ void __launch_bounds__(kSumThreads) expert_row_sum_kernel(const T* __
 // ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) fill_zero_kernel(uint4* __restrict__ p16, size_t n16, unsigned char* tail,
                                                        size_t ntail) {
+  pdl_trigger();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   const uint4 z = make_uint4(0, 0, 0, 0);
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n16; i += stride) p16[i] = z;
@@ -397,6 +398,7 @@ __global__ void __launch_bounds__(256) fill_zero_kernel(uint4* __restrict__ p16,
 }
 
 __global__ void __launch_bounds__(256) fill_zero_bytes_kernel(unsigned char* p, size_t n) {
+  pdl_trigger();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) p[i] = 0;
 }
@@ -406,6 +408,7 @@ template <typename T> __device__ __forceinline__ void convert8(const float* __re
 template <typename T>
 __global__ void __launch_bounds__(256) convert_from_f32_kernel(const float* __restrict__ src, T* __restrict__ dst,
                                                               size_t n) {
+  pdl_wait();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   const size_t i0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const bool vec = sizeof(T) == 2 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0;
@@ -422,43 +425,57 @@ __global__ void __launch_bounds__(256) convert_to_f32_kernel(const T* __restrict
     dst[i] = to_f32<T>(src[i]);
 }
 
-// ---- 16-bit scatter planning -------------------------------------------------------------------
+// ---- 16-bit scatter: preparation and finish -------------------------------------------------------
 // Adding straight into a bf16/fp16 output rounds at every addition, which is accurate enough only while few
 // contributions meet in one token row; summing in float32 rows and rounding once is always accurate but costs
 // a float32 fill, float32 atomics on a buffer twice the size and a conversion pass.  The choice is made on the
-// device, per call, from the actual indices: plan != 0 selects the float32 rows.
-__global__ void __launch_bounds__(256) scatter_plan_kernel(const void* __restrict__ ind, int index_dtype, int B, int T, int E,
-                                                          int K, int* __restrict__ counters, int* __restrict__ plan,
-                                                          int limit) {
-  const long long n = static_cast<long long>(B) * E * K;
-  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-  for (long long s = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; s < n; s += stride) {
-    const long long t = load_index(ind, index_dtype, s);
-    if (t < 0 || t >= T) continue;
-    const long long b = s / (static_cast<long long>(E) * K);
-    if (atomicAdd(counters + b * T + t, 1) + 1 > limit) *plan = 1;
-  }
-}
-
+// device, per call and batch element, from the actual indices: plan[b] != 0 selects the float32 rows.
+// One kernel counts and zeroes: every CTA counts the slots of its batch element in shared memory (4096 ids: about 2 us, under
+// the stores of the other CTAs) and zeroes its share of the buffer the additions of that batch element go to.  A chain of a
+// counter fill, a counting pass over global atomics and an init pass took three launches and 10-14 us of gaps and kernels
+// (with the dependent launches, a serving pass of one 64-token prompt went from 37 to 27 us).
+// Sequences beyond kPrepCounters tokens share counters (token id modulo kPrepCounters): that can choose the float32 rows where
+// they are not needed, never the reverse.
+constexpr int kPrepThreads = 512;
+constexpr int kPrepCounters = 50 * 1024;
 template <typename T>
-__global__ void __launch_bounds__(256) scatter_init_kernel(const int* __restrict__ plan, float* __restrict__ acc,
-                                                          T* __restrict__ out, size_t n, int zero_output) {
-  const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-  const size_t i0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (*plan) {   // float32 rows: zero them, or seed them with what the output holds
-    if (zero_output) {
-      float4* a4 = reinterpret_cast<float4*>(acc);
-      const size_t n4 = n / 4;
-      for (size_t i = i0; i < n4; i += stride) a4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (size_t i = n4 * 4 + i0; i < n; i += stride) acc[i] = 0.f;
-    } else {
-      for (size_t i = i0; i < n; i += stride) acc[i] = to_f32<T>(out[i]);
+__global__ void __launch_bounds__(kPrepThreads) scatter_prepare_kernel(const void* __restrict__ ind, int index_dtype, int B, int T_, int EK,
+                                                                       const int* __restrict__ info, int limit,
+                                                                       int* __restrict__ plan, float* __restrict__ acc, T* __restrict__ out,
+                                                                       size_t per_batch, int zero_output, StatusRef status) {
+  extern __shared__ int prep_cnt[];      // [min(T_, kPrepCounters)] without `info`
+  pdl_trigger();
+  const int tid = threadIdx.x;
+  for (int b = blockIdx.y; b < B; b += gridDim.y) {
+    int flag = 0;
+    if (info) {
+      flag = info[0] > limit;
+      if (info[2] && blockIdx.x == 0 && b == 0 && tid == 0) status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
+    } else if (EK > limit) {
+      const int nc = min(T_, kPrepCounters);
+      for (int t = tid; t < nc; t += kPrepThreads) prep_cnt[t] = 0;
+      __syncthreads();
+      int over = 0;
+      for (int s = tid; s < EK; s += kPrepThreads) {
+        const long long t = load_index(ind, index_dtype, static_cast<long long>(b) * EK + s);
+        if (t >= 0 && t < T_) over |= atomicAdd(&prep_cnt[static_cast<int>(t) % nc], 1) >= limit;
+      }
+      flag = __syncthreads_or(over);
     }
-  } else if (zero_output) {   // direct adds: only the 16-bit output needs zeroing
-    uint4* o16 = reinterpret_cast<uint4*>(out);
-    const size_t n8 = n / 8;
-    for (size_t i = i0; i < n8; i += stride) o16[i] = make_uint4(0, 0, 0, 0);
-    for (size_t i = n8 * 8 + i0; i < n; i += stride) out[i] = from_f32<T>(0.f);
+    if (blockIdx.x == 0 && tid == 0) plan[b] = flag;
+    const size_t base = static_cast<size_t>(b) * per_batch;
+    const size_t stride = static_cast<size_t>(gridDim.x) * kPrepThreads, i0 = static_cast<size_t>(blockIdx.x) * kPrepThreads + tid;
+    // (per_batch is a multiple of 8 elements and both buffers are 16-byte aligned: tensor-core path only)
+    if (flag && zero_output) {
+      float4* a4 = reinterpret_cast<float4*>(acc + base);
+      for (size_t i = i0; i < per_batch / 4; i += stride) a4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    } else if (flag) {                   // seed the float32 rows with what the output holds
+      for (size_t i = i0; i < per_batch; i += stride) acc[base + i] = to_f32<T>(out[base + i]);
+    } else if (zero_output) {
+      uint4* o16 = reinterpret_cast<uint4*>(out + base);
+      for (size_t i = i0; i < per_batch / 8; i += stride) o16[i] = make_uint4(0, 0, 0, 0);
+    }
+    __syncthreads();                     // the counters of this batch element have been used
   }
 }
 
@@ -473,16 +490,14 @@ __device__ __forceinline__ void convert8(const float* __restrict__ src, T* __res
 
 template <typename T>
 __global__ void __launch_bounds__(256) scatter_finish_kernel(const int* __restrict__ plan, const float* __restrict__ acc,
-                                                            T* __restrict__ out, size_t n) {
-  if (!*plan) return;
+                                                            T* __restrict__ out, int B, size_t per_batch) {
+  pdl_wait();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-  const size_t i0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (sizeof(T) == 2) {          // (both buffers are 16-byte aligned: checked on the host)
-    const size_t n8 = n / 8;
-    for (size_t i = i0; i < n8; i += stride) convert8<T>(acc + 8 * i, out + 8 * i);
-    for (size_t i = n8 * 8 + i0; i < n; i += stride) out[i] = from_f32<T>(acc[i]);
-  } else {
-    for (size_t i = i0; i < n; i += stride) out[i] = from_f32<T>(acc[i]);
+  for (int b = blockIdx.y; b < B; b += gridDim.y) {
+    if (!plan[b]) continue;
+    const size_t base = static_cast<size_t>(b) * per_batch;
+    for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < per_batch / 8; i += stride)
+      convert8<T>(acc + base + 8 * i, out + base + 8 * i);
   }
 }
 
@@ -624,47 +639,65 @@ cudaError_t launch_fill_zero(void* ptr, size_t bytes, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_convert_from_f32(const float* src, void* dst, size_t n, int dtype, cudaStream_t st) {
+cudaError_t launch_convert_from_f32(const float* src, void* dst, size_t n, int dtype, cudaStream_t st, bool after_own) {
   if (n == 0) return cudaSuccess;
   const int grid = grid_for(n, 256 * 4);
-  if (dtype == EGS_F16) convert_from_f32_kernel<__half><<<grid, 256, 0, st>>>(src, static_cast<__half*>(dst), n);
+  cudaError_t err;
+  if (dtype == EGS_F16) err = launch_kernel(convert_from_f32_kernel<__half>, grid, 256, 0, st, after_own, src, static_cast<__half*>(dst), n);
   else if (dtype == EGS_BF16)
-    convert_from_f32_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(src, static_cast<__nv_bfloat16*>(dst), n);
+    err = launch_kernel(convert_from_f32_kernel<__nv_bfloat16>, grid, 256, 0, st, after_own, src, static_cast<__nv_bfloat16*>(dst), n);
   else return cudaErrorInvalidValue;
+  count_launch();
+  return err;
+}
+
+template <typename T>
+static cudaError_t prepare(const void* Ind, int index_dtype, int B, int T_, int EK, const int* info, int limit, int* plan, float* acc,
+                           void* out16, size_t per_batch, int zero_output, StatusRef status, cudaStream_t st) {
+  // CTAs per batch element: four per SM in all, each with at least 4 KB to zero and no more ids to count than half the elements
+  // it zeroes
+  const bool count = info == nullptr && EK > limit;
+  size_t per = (4 * 148 + B - 1) / B;
+  const size_t by_bytes = per_batch * sizeof(T) / 4096, by_count = count ? per_batch / (2 * static_cast<size_t>(EK)) : per;
+  if (per > by_bytes) per = by_bytes;
+  if (per > by_count) per = by_count;
+  if (per < 1) per = 1;
+  const size_t smem = count ? static_cast<size_t>(T_ < kPrepCounters ? T_ : kPrepCounters) * sizeof(int) : 0;
+  if (smem > 48 * 1024) {
+    cudaError_t err = ensure_smem_optin<scatter_prepare_kernel<T>>(kPrepCounters * static_cast<int>(sizeof(int)));
+    if (err != cudaSuccess) return err;
+  }
+  scatter_prepare_kernel<T><<<dim3(static_cast<unsigned>(per), B < 65535 ? B : 65535), kPrepThreads, smem, st>>>(
+      Ind, index_dtype, B, T_, EK, info, limit, plan, acc, static_cast<T*>(out16), per_batch, zero_output, status);
   count_launch();
   return cudaGetLastError();
 }
 
-cudaError_t launch_scatter_plan(const void* Ind, int index_dtype, int B, int T, int E, int K, int* counters, int* plan,
-                                int limit, int32_t*, cudaStream_t st) {
-  const size_t n = static_cast<size_t>(B) * E * K;
-  if (n == 0) return cudaSuccess;
-  scatter_plan_kernel<<<grid_for(n, 256), 256, 0, st>>>(Ind, index_dtype, B, T, E, K, counters, plan, limit);
-  count_launch();
-  return cudaGetLastError();
+cudaError_t launch_scatter_prepare(const void* Ind, int index_dtype, int B, int T, int E, int K, const int* csr_info, int limit, int* plan,
+                                   float* acc, void* out16, int N, int zero_output, int dtype, StatusRef status, cudaStream_t st) {
+  const size_t per_batch = static_cast<size_t>(T) * N;
+  if (B == 0 || per_batch == 0) return cudaSuccess;
+  const int ek = E * K;      // B*E*K fits in 32 bits
+  if (dtype == EGS_F16) return prepare<__half>(Ind, index_dtype, B, T, ek, csr_info, limit, plan, acc, out16, per_batch, zero_output, status, st);
+  if (dtype == EGS_BF16)
+    return prepare<__nv_bfloat16>(Ind, index_dtype, B, T, ek, csr_info, limit, plan, acc, out16, per_batch, zero_output, status, st);
+  return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_scatter_init(const int* plan, float* acc, void* out16, size_t n, int zero_output, int dtype,
-                                cudaStream_t st) {
-  if (n == 0) return cudaSuccess;
-  const int grid = grid_for(n, 256 * 8);
-  if (dtype == EGS_F16) scatter_init_kernel<__half><<<grid, 256, 0, st>>>(plan, acc, static_cast<__half*>(out16), n, zero_output);
+cudaError_t launch_scatter_finish(const int* plan, const float* acc, void* out16, int B, size_t per_batch, int dtype, cudaStream_t st) {
+  if (B == 0 || per_batch == 0) return cudaSuccess;
+  size_t per = per_batch / (256 * 8 * 4);                // four vectors per thread, a few waves of CTAs at most
+  const size_t most = (148 * 8 + B - 1) / B;
+  if (per > most) per = most;
+  if (per < 1) per = 1;
+  const dim3 grid(static_cast<unsigned>(per), B < 65535 ? B : 65535);
+  cudaError_t err;
+  if (dtype == EGS_F16) err = launch_kernel(scatter_finish_kernel<__half>, grid, 256, 0, st, true, plan, acc, static_cast<__half*>(out16), B, per_batch);
   else if (dtype == EGS_BF16)
-    scatter_init_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(plan, acc, static_cast<__nv_bfloat16*>(out16), n, zero_output);
+    err = launch_kernel(scatter_finish_kernel<__nv_bfloat16>, grid, 256, 0, st, true, plan, acc, static_cast<__nv_bfloat16*>(out16), B, per_batch);
   else return cudaErrorInvalidValue;
   count_launch();
-  return cudaGetLastError();
-}
-
-cudaError_t launch_scatter_finish(const int* plan, const float* acc, void* out16, size_t n, int dtype, cudaStream_t st) {
-  if (n == 0) return cudaSuccess;
-  const int grid = grid_for(n, 256 * 4);
-  if (dtype == EGS_F16) scatter_finish_kernel<__half><<<grid, 256, 0, st>>>(plan, acc, static_cast<__half*>(out16), n);
-  else if (dtype == EGS_BF16)
-    scatter_finish_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(plan, acc, static_cast<__nv_bfloat16*>(out16), n);
-  else return cudaErrorInvalidValue;
-  count_launch();
-  return cudaGetLastError();
+  return err;
 }
 
 cudaError_t launch_convert_to_f32(const void* src, float* dst, size_t n, int dtype, cudaStream_t st) {

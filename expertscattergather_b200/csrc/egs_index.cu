@@ -623,11 +623,6 @@ __global__ void __launch_bounds__(kCsrThreads) csr_scatter_kernel(const T* __res
   }
 }
 
-__global__ void plan_from_info_kernel(const int* __restrict__ info, int limit, int* __restrict__ plan, int32_t* status) {
-  *plan = (info[0] > limit) ? 1 : 0;
-  if (info[2] && status) atomicOr(status, EGS_STATUS_INDEX_OUT_OF_RANGE);
-}
-
 int grid_1d(long long items, int per_block, int cap) {
   long long blocks = (items + per_block - 1) / per_block;
   if (blocks > cap) blocks = cap;
@@ -711,12 +706,6 @@ cudaError_t launch_index_csr(const void* ind, int index_dtype, int B, int T, int
     csr_sort_rows_kernel<<<static_cast<int>((rows + 255) / 256), 256, 0, st>>>(offsets, entries, rows);
   }
   count_launch(n > 0 ? 6 : 3);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_plan_from_info(const int* info, int limit, int* plan, int32_t* status, cudaStream_t st) {
-  plan_from_info_kernel<<<1, 1, 0, st>>>(info, limit, plan, status);
-  count_launch();
   return cudaGetLastError();
 }
 

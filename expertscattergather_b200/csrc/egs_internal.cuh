@@ -65,8 +65,8 @@ struct RowGemmParams {
   const void* Ind;    // [B, E, K]
   void* Out;          // G: slot rows [B*E*K, N]     S: token rows [B*T, N]
   float* acc;         // S with 16-bit tensors: float32 accumulation rows [B*T, N]; otherwise unused
-  const int* plan;    // S with 16-bit tensors: device flag, non-zero = accumulate in the float32 rows,
-                      // zero = add directly into the 16-bit output; NULL = always the float32 rows
+  const int* plan;    // S with 16-bit tensors: a device flag per batch element, non-zero = its token rows accumulate in the
+                      // float32 rows, zero = direct additions into the 16-bit output; NULL = always the float32 rows
   const void* bias;   // optional [E, N] in the tensors' dtype: bias[e, :] is added to every produced row of expert e
                       // (G: to the stored row; S: to the row before it is added to its token row); NULL = none
   StatusRef status;    // optional device status word
@@ -79,6 +79,7 @@ struct RowGemmParams {
   int expert_fastest; // tensor path: grid order (1: experts vary fastest, row tiles slowest)
   int row_tiles;      // tensor path: 128-row accumulator tiles per CTA (1 or 2)
   int persistent;     // tensor path: 1 = persistent warp-specialised variant
+  int after_own;      // launched behind a kernel of the same call (fill, preparation): see launch_kernel
   int bulk_epilogue;  // persistent scatter: rows staged in shared memory and added with bulk asynchronous reductions
 };
 
@@ -98,6 +99,7 @@ struct DWeightParams {
   int BN;             // tensor path: tile width over FD
   int stages;
   int row_tiles;      // tensor path: 128-feature accumulator tiles per CTA over FG (1 or 2)
+  int after_own;      // launched behind the fill of `acc`: see launch_kernel
 };
 
 // Fused pair G -> S (tensor path only):  Mid = gather(Src) x W1[e] is stored as slot rows AND fed, without leaving the
@@ -110,7 +112,7 @@ struct FusedParams {
   void* Mid;           // slot rows [B*E*K, N1], overwritten
   float* Dst;          // float32 token rows [B*T, N2], added to (16-bit tensors: the accumulation rows of the scratch)
   void* Out16;         // 16-bit tensors: the output token rows [B*T, N2] that direct 16-bit additions go to
-  const int* plan;     // 16-bit tensors: device flag, see RowGemmParams::plan
+  const int* plan;     // 16-bit tensors: device flags, see RowGemmParams::plan
   StatusRef status;
   int B, T, E, K, C1, N1, N2;
   int M;               // B*K
@@ -119,6 +121,7 @@ struct FusedParams {
   int BN1, BN2;        // MMA widths (multiples of 16)
   int stages;
   int expert_fastest;  // 16-bit kernel: order of the row blocks a CTA walks (1: experts vary fastest)
+  int after_own;       // launched behind a kernel of the same call (fill, preparation): see launch_kernel
   uint32_t slot_bytes; // 16-bit kernel: bytes of one ring slot
 };
 
@@ -132,15 +135,14 @@ cudaError_t launch_generic_dweight(const DWeightParams& p, int dtype, cudaStream
 cudaError_t launch_expert_row_sum(const void* Src, const void* Ind, int index_dtype, void* out, int B, int T, int E, int K, int N,
                                   int dtype, StatusRef status, cudaStream_t st);
 cudaError_t launch_fill_zero(void* ptr, size_t bytes, cudaStream_t st);
-cudaError_t launch_convert_from_f32(const float* src, void* dst, size_t n, int dtype, cudaStream_t st);
+cudaError_t launch_convert_from_f32(const float* src, void* dst, size_t n, int dtype, cudaStream_t st, bool after_own = false);
 cudaError_t launch_convert_to_f32(const void* src, float* dst, size_t n, int dtype, cudaStream_t st);
-// 16-bit scatter planning (see egs_generic.cu): counts contributions per token row and raises *plan when any
-// row receives more than `limit`; the init / finish kernels then act on the float32 rows or on the 16-bit output.
-cudaError_t launch_scatter_plan(const void* Ind, int index_dtype, int B, int T, int E, int K, int* counters, int* plan,
-                                int limit, int32_t* status, cudaStream_t st);
-cudaError_t launch_scatter_init(const int* plan, float* acc, void* out16, size_t n, int zero_output, int dtype,
-                                cudaStream_t st);
-cudaError_t launch_scatter_finish(const int* plan, const float* acc, void* out16, size_t n, int dtype, cudaStream_t st);
+// 16-bit scatter (see egs_generic.cu): prepare decides, per batch element, between direct additions (no token row gets more than
+// `limit` contributions) and float32 rows, and zeroes (or seeds) what the additions go to; finish rounds the float32 rows.
+// csr_info: the summary of a prepared CSR, whose heaviest row decides for all batch elements; NULL = the ids are counted.
+cudaError_t launch_scatter_prepare(const void* Ind, int index_dtype, int B, int T, int E, int K, const int* csr_info, int limit, int* plan,
+                                   float* acc, void* out16, int N, int zero_output, int dtype, StatusRef status, cudaStream_t st);
+cudaError_t launch_scatter_finish(const int* plan, const float* acc, void* out16, int B, size_t per_batch, int dtype, cudaStream_t st);
 
 // Tensor-core (tcgen05) family.  `configure_*` fills BN/stages and returns the dynamic shared memory size.
 size_t configure_tensor_rowgemm(RowGemmParams& p, bool scatter, int dtype);
@@ -182,13 +184,36 @@ cudaError_t launch_compact_index(const void* ind, int index_dtype, long long n, 
 cudaError_t launch_csr_scatter(const void* Y, const void* W, const void* bias, const int* offsets, const int* entries, void* Out,
                                long long rows, int E, int K, int C, int N, int w_layout, int accumulate, int dtype,
                                cudaStream_t st);
-// *plan = (info[0] > limit): the 16-bit scatter's choice taken from a prepared CSR instead of a pass over Ind
-cudaError_t launch_plan_from_info(const int* info, int limit, int* plan, int32_t* status, cudaStream_t st);
 
 // Bounded-wait self-test (see the kernel): out = two ints on the device.
 cudaError_t launch_wait_timeout_selftest(int32_t* status, int* out, long long limit_cycles, cudaStream_t st);
 
 void count_launch(int n = 1);
+
+// ------------------------------------------------------------------------------------------------
+// Programmatic dependent launch, for pairs of kernels that one entry point issues back to back on one stream.  The first kernel
+// (a fill, the scatter's preparation, a kernel whose result is still to be rounded) is launched normally, so that everything
+// before it has finished when it runs, and calls pdl_trigger at its start; the second then becomes resident while the first
+// runs, does all that does not depend on it (the contraction), and calls pdl_wait before it touches what the first wrote.
+// A kernel launched without the attribute returns from pdl_wait at once.
+// ------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... Params, class... Args>
+cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool after_own, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = after_own ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
 
 // The opt-in to large dynamic shared memory is per kernel function and device: done once per thread and device, for `bytes`.
 template <auto kernel>

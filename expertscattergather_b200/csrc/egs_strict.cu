@@ -163,6 +163,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(StrictParams 
   tc_fence_after();
   const uint32_t tmem_base = hdr->tmem_base;
 
+  pdl_trigger();
   if (hdr->abort_flag != 0u) {
     // fall through to the common exit
   } else if (warp < kProdWarps) {
@@ -341,6 +342,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(StrictParams 
     const uint32_t lane_base = static_cast<uint32_t>(lg * 32) << 16;
     const uint32_t sums = tmem_base + lane_base + 2u * acc_cols;
     bool alive = true;
+    pdl_wait();                                          // the zeros the results are added to
     int t = 0;                                           // accumulators taken so far
     for (int un = blockIdx.x; un < p.units && alive; un += gridDim.x) {
       const Unit u = unit_of<OP>(p, un);
@@ -514,14 +516,14 @@ int strict_raw_stages(int bn) {
 }
 
 template <int OP>
-cudaError_t launch(const StrictParams& p, cudaStream_t st) {
+cudaError_t launch(const StrictParams& p, bool after_own, cudaStream_t st) {
   const size_t stage = kATile + static_cast<size_t>(p.BN) * 128;
   const size_t smem = kStrictHeader + kXposeBytes + (p.raw + kLoStages) * stage;
   cudaError_t err = ensure_smem_optin<strict_kernel<OP>>(static_cast<int>(kSmemMax));
   if (err != cudaSuccess) return err;
-  strict_kernel<OP><<<p.units < kSms ? p.units : kSms, kStrictThreads, smem, st>>>(p);
+  err = launch_kernel(strict_kernel<OP>, p.units < kSms ? p.units : kSms, kStrictThreads, smem, st, after_own, p);
   count_launch();
-  return cudaGetLastError();
+  return err;
 }
 
 }  // namespace
@@ -546,7 +548,7 @@ cudaError_t launch_strict_rowgemm(const RowGemmParams& r, bool scatter, cudaStre
   const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.E;
   if (units > 2147483647ll) return cudaErrorInvalidValue;
   p.units = static_cast<int>(units);
-  return scatter ? launch<kOpScatter>(p, st) : launch<kOpGather>(p, st);
+  return scatter ? launch<kOpScatter>(p, r.after_own != 0, st) : launch<kOpGather>(p, r.after_own != 0, st);
 }
 
 void configure_strict_dweight(DWeightParams& p) {
@@ -578,7 +580,7 @@ cudaError_t launch_strict_dweight(const DWeightParams& r, cudaStream_t st) {
   const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.E * p.splits;
   if (units > 2147483647ll) return cudaErrorInvalidValue;
   p.units = static_cast<int>(units);
-  return launch<kOpDweight>(p, st);
+  return launch<kOpDweight>(p, r.after_own != 0, st);
 }
 
 }  // namespace egs

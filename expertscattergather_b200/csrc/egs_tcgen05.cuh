@@ -337,49 +337,6 @@ __device__ __forceinline__ void warp_block_emit(uint32_t taddr, uint32_t tile, i
   }
   warp_regs_emit(v, tile, lane, emit);
 }
-// Same transpose for a 32-row x 64-column block (8 KB tile): every lane ends up with 8 consecutive columns of
-// one row, so 8 lanes cover 64 columns - 128 contiguous bytes of a 16-bit row per instruction.
-//   emit(row_in_block, first_column, x[8]) is called 8 times per lane.
-template <class Emit>
-__device__ __forceinline__ void warp_block_emit64(uint32_t taddr, uint32_t tile, int lane, Emit&& emit) {
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    uint32_t v[32];
-    tmem_ld32(taddr + h * 32, v);
-    tmem_ld_wait();
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(tile + lane * 256u + (static_cast<uint32_t>((h * 8 + j) ^ (lane & 7)) << 4)),
-                   "r"(v[4 * j]), "r"(v[4 * j + 1]), "r"(v[4 * j + 2]), "r"(v[4 * j + 3])
-                   : "memory");
-  }
-  __syncwarp();
-  const int j = lane & 7;
-#pragma unroll
-  for (int it = 0; it < 8; ++it) {
-    const int row = it * 4 + (lane >> 3);
-    uint32_t x[8];
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-      asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];"
-                   : "=r"(x[4 * q]), "=r"(x[4 * q + 1]), "=r"(x[4 * q + 2]), "=r"(x[4 * q + 3])
-                   : "r"(tile + row * 256u + (static_cast<uint32_t>((2 * j + q) ^ (row & 7)) << 4))
-                   : "memory");
-    emit(row, j * 8, x);
-  }
-  __syncwarp();
-}
-__device__ __forceinline__ void red8(__nv_bfloat16* dst, const uint32_t (&x)[8]) {
-  asm volatile("red.global.add.noftz.v4.bf16x2 [%0], {%1,%2,%3,%4};" ::"l"(dst), "r"(pack2(dst, x[0], x[1])),
-               "r"(pack2(dst, x[2], x[3])), "r"(pack2(dst, x[4], x[5])), "r"(pack2(dst, x[6], x[7]))
-               : "memory");
-}
-__device__ __forceinline__ void red8(__half* dst, const uint32_t (&x)[8]) {
-  asm volatile("red.global.add.noftz.v4.f16x2 [%0], {%1,%2,%3,%4};" ::"l"(dst), "r"(pack2(dst, x[0], x[1])),
-               "r"(pack2(dst, x[2], x[3])), "r"(pack2(dst, x[4], x[5])), "r"(pack2(dst, x[6], x[7]))
-               : "memory");
-}
-__device__ __forceinline__ void red8(float*, const uint32_t (&)[8]) {}   // never taken: direct adds are 16-bit only
 // Bulk asynchronous reduction: adds `bytes` (multiple of 16) of elements staged in shared memory to global memory.
 // The copy engine reads the shared memory after the instruction has issued: the staging buffer may be rewritten
 // only after bulk_wait_read, and the issuing thread's own writes need fence.proxy.async before the instruction.

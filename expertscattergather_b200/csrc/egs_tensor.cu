@@ -74,6 +74,7 @@ __device__ __forceinline__ uint32_t pipe_setup(const Pipe& pp, uint32_t full_cou
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();
   return hdr->tmem_base;
 }
 
@@ -90,6 +91,7 @@ __device__ __forceinline__ bool producer_finish(const Pipe& pp, int lane, bool a
   alive = __all_sync(0xffffffffu, alive);
   if (alive && pp.nk > 0) alive = mbar_wait_warp(smem_u32(&pp.hdr->done), 0u, pp.abort_flag, pp.status.word, lane);
   if (alive) tc_fence_after();
+  pdl_wait();                            // what the results are added to
   return alive;
 }
 
@@ -324,26 +326,30 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_rowgemm_kern
     const bool alive = run_producer(pp, lane, issue_stage);
 
     // =========================== epilogue ===========================
-    // The stage ring is idle once `done` has completed: its first 32 KB serve as the warps' transpose tiles.
+    // The stage ring is idle once `done` has completed: it holds, per warp, a 4 KB transpose tile or, where the ring has room, the
+    // two staging buffers of the bulk reductions (the tile fits in them; warps of one CTA may differ in which they use).
     if (alive) {
       const int lg = warp & 3, half = warp >> 2;
-      const uint32_t tile = pp.tiles0 + static_cast<uint32_t>(warp) * 4096u;
+      const bool bulk_room = SCATTER && ES == 2 && p.bulk_epilogue && (pp.stages * pp.stage_bytes >= 8u * 2u * kBulkBufBytes);
+      const uint32_t area = pp.tiles0 + static_cast<uint32_t>(warp) * (bulk_room ? 2u * kBulkBufBytes : 4096u);
       T* out = static_cast<T*>(p.Out);
       float* acc_rows = (ES == 2) ? p.acc : reinterpret_cast<float*>(p.Out);   // S: float32 rows being added to
-      // 16-bit S: the planning flag says whether to add into the float32 rows or straight into the output
-      const bool direct16 = SCATTER && ES == 2 && p.plan != nullptr && *p.plan == 0;
+      // 16-bit S: the planning flags say, per batch element, whether to add into the float32 rows or straight into the output.
+      // f32_rows(mt): which of this warp's 32 rows of accumulator mt go to the float32 rows.
+      auto f32_rows = [&](int mt) -> uint32_t {
+        const int m = m0 + mt * kTileM + lg * 32 + lane;
+        return __ballot_sync(0xffffffffu, p.plan == nullptr || (m < p.M && p.plan[m / p.K] != 0));
+      };
+      // direct 16-bit adds go out as bulk reductions: every lane stages 128 bytes (64 columns) of its own row and hands them to the
+      // copy engine (see the persistent variant)
+      bool bulk16 = bulk_room;
+      if (bulk_room)
+        for (int mt = 0; mt < MT; ++mt) bulk16 = bulk16 && f32_rows(mt) == 0u;
       const int nblk = (bn + 31) >> 5;
-      // direct 16-bit adds go out in 64-column blocks (128-byte row segments) when the ring has room for the
-      // eight 8 KB transpose tiles and the tile width is a multiple of 64
-      const bool wide16 = direct16 && (bn % 64 == 0) && (pp.stages * pp.stage_bytes >= 8u * 8192u);
-      // direct 16-bit adds as bulk reductions: every lane stages 128 bytes (64 columns) of its own row in the idle
-      // ring and hands them to the copy engine (see the persistent variant)
-      static_assert(2u * kBulkBufBytes <= 16384u, "two staging buffers per warp");
-      const bool bulk16 = direct16 && p.bulk_epilogue && (pp.stages * pp.stage_bytes >= 8u * 2u * kBulkBufBytes);
       const T* bias_row = p.bias ? static_cast<const T*>(p.bias) + static_cast<long long>(e) * p.N : nullptr;
       if (bulk16) {
         if constexpr (ES == 2 && SCATTER) {
-          const uint32_t my_stage = pp.tiles0 + static_cast<uint32_t>(warp) * (2u * kBulkBufBytes) + static_cast<uint32_t>(lane) * kBulkRowPitch;
+          const uint32_t my_stage = area + static_cast<uint32_t>(lane) * kBulkRowPitch;
           int q = 0;
           for (int mt = 0; mt < MT; ++mt) {
             const int ro = hdr->row_o[mt * kTileM + lg * 32 + lane];
@@ -376,35 +382,12 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_rowgemm_kern
           }
           bulk_wait_all();                               // shared memory must outlive the copy engine's reads
         }
-      } else if (wide16) {
-        const uint32_t tile8 = pp.tiles0 + static_cast<uint32_t>(warp) * 8192u;
-        for (int mt = 0; mt < MT; ++mt) {
-          for (int c = half; c < (bn >> 6); c += 2) {
-            const int col0 = n0 + c * 64;
-            warp_block_emit64(tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + mt * acc_cols + static_cast<uint32_t>(c * 64), tile8,
-                              lane, [&](int row, int cj, const uint32_t (&x)[8]) {
-                                const int ro = hdr->row_o[mt * kTileM + lg * 32 + row];
-                                const int col = col0 + cj;
-                                if (ro >= 0 && col < p.N) {
-                                  if (bias_row) {
-                                    uint32_t y[8];
-#pragma unroll
-                                    for (int i = 0; i < 8; ++i) y[i] = x[i];
-                                    add_bias4<T>(bias_row + col, y[0], y[1], y[2], y[3]);
-                                    add_bias4<T>(bias_row + col + 4, y[4], y[5], y[6], y[7]);
-                                    red8(out + static_cast<long long>(ro) * p.N + col, y);
-                                  } else {
-                                    red8(out + static_cast<long long>(ro) * p.N + col, x);
-                                  }
-                                }
-                              });
-          }
-        }
       } else
       for (int mt = 0; mt < MT; ++mt) {
+        const uint32_t to_f32 = (SCATTER && ES == 2) ? f32_rows(mt) : 0xffffffffu;
         for (int c = half; c < nblk; c += 2) {
           const int col0 = n0 + c * 32;
-          warp_block_emit(tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + mt * acc_cols + static_cast<uint32_t>(c * 32), tile,
+          warp_block_emit(tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + mt * acc_cols + static_cast<uint32_t>(c * 32), area,
                           lane, true, [&](int row, int cj, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3) {
                             const int ro = hdr->row_o[mt * kTileM + lg * 32 + row];
                             const int col = col0 + cj;
@@ -412,8 +395,8 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_rowgemm_kern
                               const long long off = static_cast<long long>(ro) * p.N + col;
                               if (bias_row) add_bias4<T>(bias_row + col, x0, x1, x2, x3);
                               if (SCATTER) {
-                                if (direct16) red4(out + off, x0, x1, x2, x3);
-                                else red4(acc_rows + off, x0, x1, x2, x3);
+                                if ((to_f32 >> row) & 1u) red4(acc_rows + off, x0, x1, x2, x3);
+                                else red4(out + off, x0, x1, x2, x3);
                               } else {
                                 store4(out + off, x0, x1, x2, x3);   // masked source rows were zero-filled: zeros
                               }
@@ -589,6 +572,7 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = hdr->tmem_base;
+  pdl_trigger();
   const bool run = (hdr->abort_flag == 0u);
 
   if (!run) {
@@ -723,19 +707,24 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
     const uint32_t tile = xpose0 + static_cast<uint32_t>(ew) * xpose_tile;
     T* out = static_cast<T*>(p.Out);
     float* acc_rows = (ES == 2) ? p.acc : reinterpret_cast<float*>(p.Out);   // S: float32 rows being added to
-    const bool direct16 = SCATTER && ES == 2 && p.plan != nullptr && *p.plan == 0;
     // bulk adds (direct 16-bit scatter): every lane stages 128 bytes of its own row and hands them to the copy
     // engine - no transpose, no shuffles, and the warp does not wait on the load/store unit.  (For float32 rows
     // the same scheme needs twice the operations per column and measured slower than the transposed reds.)
-    const bool bulk = direct16 && p.bulk_epilogue;
     const uint32_t my_stage = tile + static_cast<uint32_t>(lane) * kBulkRowPitch;
     int q = 0;                                           // bulk groups committed so far by this thread
     bool alive = true;
+    if (SCATTER) pdl_wait();                             // the planning flags and the zeros the rows are added to
     int t = 0;                                           // tiles finished so far by this CTA
     for (int rb = blockIdx.x; rb < row_blocks && alive; rb += gridDim.x) {
       const RowBlock blk = row_block_of(p, rb, m_tiles);
       int src_row, my_ro;                                // destination row of tile row lg*32 + lane
-      lookup_rows<SCATTER>(p, blk.e, blk.m0 + lg * 32 + lane, src_row, my_ro, half == 0);
+      const int my_m = blk.m0 + lg * 32 + lane;
+      lookup_rows<SCATTER>(p, blk.e, my_m, src_row, my_ro, half == 0);
+      // rows of this warp whose batch element sums in float32 rows (bits), see RowGemmParams::plan
+      const uint32_t to_f32 = (SCATTER && ES == 2) ? __ballot_sync(0xffffffffu, p.plan == nullptr || (my_m < p.M && p.plan[my_m / p.K] != 0))
+                                                   : 0xffffffffu;
+      const bool bulk = SCATTER && ES == 2 && p.bulk_epilogue && to_f32 == 0u;
+      if (SCATTER && ES == 2 && !bulk) bulk_wait_all();  // the transposes below reuse the staging buffers
       for (int nt = 0; nt < n_tiles && alive; ++nt, ++t) {
         const int n0 = nt * p.BN;
         const int bn = min(p.BN, ((p.N - n0) + 15) & ~15);
@@ -787,8 +776,8 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
                               const long long off = static_cast<long long>(ro) * p.N + col;
                               if (p.bias) add_bias4<T>(static_cast<const T*>(p.bias) + static_cast<long long>(blk.e) * p.N + col, x0, x1, x2, x3);
                               if (SCATTER) {
-                                if (direct16) red4(out + off, x0, x1, x2, x3);
-                                else red4(acc_rows + off, x0, x1, x2, x3);
+                                if ((to_f32 >> row) & 1u) red4(acc_rows + off, x0, x1, x2, x3);
+                                else red4(out + off, x0, x1, x2, x3);
                               } else {
                                 store4(out + off, x0, x1, x2, x3);
                               }
@@ -801,7 +790,7 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
         if (lane == 0) mbar_arrive(smem_u32(&hdr->acc_empty[buf]));
       }
     }
-    if (bulk) bulk_wait_all();                           // shared memory must outlive the copy engine's reads
+    if (SCATTER && ES == 2) bulk_wait_all();             // shared memory must outlive the copy engine's reads
   } else {
     // =========================== MMA issuer ===========================
     if (lane == 0) {
@@ -1224,6 +1213,7 @@ __global__ void __launch_bounds__(17 * 32, 1) tensor_fused_pair_kernel(FusedPara
   tc_fence_after();
   const uint32_t tmem_base = hdr->tmem_base;
   const uint32_t acc1 = tmem_base, acc2 = tmem_base + acc1_cols;
+  pdl_trigger();
   const bool run = (hdr->abort_flag == 0u);
   const int ntot = nk1 + nk2;
   if (!run) {
@@ -1374,6 +1364,7 @@ __global__ void __launch_bounds__(17 * 32, 1) tensor_fused_pair_kernel(FusedPara
       //     warps' transpose tiles
       alive = mbar_wait_warp(smem_u32(&hdr->acc2_done), 0u, abort_flag, p.status.word, lane);
       if (alive) {
+        pdl_wait();                      // the zeros the rows are added to
         tc_fence_after();
         const uint32_t tile = tiles0 + static_cast<uint32_t>(ew) * 4096u;
         const int nblk = (p.BN2 + 31) >> 5;
@@ -1617,10 +1608,10 @@ cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, int dtyp
   do {                                                                                                       \
     if (scatter) {                                                                                           \
       perr = (ensure_smem_optin<tensor_rowgemm_persistent_kernel<TY, true>>(static_cast<int>(kSmemMaxPerCta)));                              \
-      if (perr == cudaSuccess) tensor_rowgemm_persistent_kernel<TY, true><<<pgrid, pblock, smem_bytes, st>>>(p);  \
+      if (perr == cudaSuccess) perr = launch_kernel(tensor_rowgemm_persistent_kernel<TY, true>, pgrid, pblock, smem_bytes, st, p.after_own != 0, p);  \
     } else {                                                                                                 \
       perr = (ensure_smem_optin<tensor_rowgemm_persistent_kernel<TY, false>>(static_cast<int>(kSmemMaxPerCta)));                             \
-      if (perr == cudaSuccess) tensor_rowgemm_persistent_kernel<TY, false><<<pgrid, pblock, smem_bytes, st>>>(p); \
+      if (perr == cudaSuccess) perr = launch_kernel(tensor_rowgemm_persistent_kernel<TY, false>, pgrid, pblock, smem_bytes, st, false, p); \
     }                                                                                                        \
   } while (0)
     if (dtype == EGS_F32) EGS_LAUNCH_P(float);
@@ -1639,7 +1630,7 @@ cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, int dtyp
 #define EGS_LAUNCH2(TY, SC, MTV)                                                                                \
   do {                                                                                                          \
     err = (ensure_smem_optin<tensor_rowgemm_kernel<TY, SC, MTV>>(static_cast<int>(kSmemMaxPerCta)));            \
-    if (err == cudaSuccess) tensor_rowgemm_kernel<TY, SC, MTV><<<grid, block, smem_bytes, st>>>(p);             \
+    if (err == cudaSuccess) err = launch_kernel(tensor_rowgemm_kernel<TY, SC, MTV>, grid, block, smem_bytes, st, p.after_own != 0, p); \
   } while (0)
 #define EGS_LAUNCH(TY)                                  \
   do {                                                  \
@@ -1669,7 +1660,7 @@ cudaError_t launch_tensor_dweight(const DWeightParams& p, int dtype, size_t smem
 #define EGS_LAUNCH_D(TY, MTV)                                                                                   \
   do {                                                                                                          \
     err = (ensure_smem_optin<tensor_dweight_kernel<TY, MTV>>(static_cast<int>(kSmemMaxPerCta)));                \
-    if (err == cudaSuccess) tensor_dweight_kernel<TY, MTV><<<grid, block, smem_bytes, st>>>(p);                 \
+    if (err == cudaSuccess) err = launch_kernel(tensor_dweight_kernel<TY, MTV>, grid, block, smem_bytes, st, p.after_own != 0, p); \
   } while (0)
 #define EGS_LAUNCH(TY)                          \
   do {                                          \
@@ -1698,10 +1689,10 @@ cudaError_t launch_tensor_fused_pair(const FusedParams& p, int precision, size_t
   cudaError_t err;
   if (precision == EGS_PREC_STRICT) {
     err = ensure_smem_optin<tensor_fused_pair_kernel<true>>(static_cast<int>(kSmemMaxPerCta));
-    if (err == cudaSuccess) tensor_fused_pair_kernel<true><<<grid, block, smem_bytes, st>>>(p);
+    if (err == cudaSuccess) err = launch_kernel(tensor_fused_pair_kernel<true>, grid, block, smem_bytes, st, p.after_own != 0, p);
   } else {
     err = ensure_smem_optin<tensor_fused_pair_kernel<false>>(static_cast<int>(kSmemMaxPerCta));
-    if (err == cudaSuccess) tensor_fused_pair_kernel<false><<<grid, block, smem_bytes, st>>>(p);
+    if (err == cudaSuccess) err = launch_kernel(tensor_fused_pair_kernel<false>, grid, block, smem_bytes, st, p.after_own != 0, p);
   }
   if (err != cudaSuccess) return err;
   count_launch();

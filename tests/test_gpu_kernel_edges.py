@@ -110,3 +110,35 @@ def test_strict_float32_edges(cuda_device, B, T, E, K, I, J):
     got = gpu_step(real, cuda_device, "tensor")
     for k in STEP_KEYS:
         assert orc.rel_err(got[k], truth[k]) <= 1e-5, k
+
+
+# 16-bit scatter: the choice between direct additions and float32 rows is made per batch element; tiles of 128 expert rows here
+# span batch elements of both kinds (K = 48), the persistent kernel (N = 1032) and the one-tile kernel (long contraction)
+@pytest.mark.parametrize("C,N", [(40, 72), (256, 1032), (520, 64)])
+@pytest.mark.parametrize("pair", [False, True])
+def test_scatter16_mixes_both_kinds_of_batch_elements(cuda_device, C, N, pair):
+    if pair and (C % 16 or C > 256):
+        pytest.skip("shape the pair kernel does not take")
+    B, T, E, K = 9, 130, 40, 48
+    g = torch.Generator().manual_seed(C)
+    Ind = torch.randint(0, T, (B, E, K), generator=g)              # about 15 per row
+    Ind[2, :, 0] = 7                                               # 40 more on one row of batch elements 2 and 5
+    Ind[5, :, 1] = 129
+    most = torch.stack([torch.bincount(Ind[b].reshape(-1), minlength=T).max() for b in range(B)])
+    assert (most[[2, 5]] > 32).all() and (most <= 32).sum() >= 5
+    Y = torch.randint(-2, 3, (B, E, K, C), generator=g).to(torch.bfloat16)
+    W = torch.randint(-1, 2, (E, C, N), generator=g).to(torch.bfloat16)
+    if pair:
+        X = torch.randint(-1, 2, (B, T, 32), generator=g).to(torch.bfloat16)
+        W1 = torch.randint(-1, 2, (E, 32, C), generator=g).to(torch.bfloat16)
+        Mid, Out = ops.gather_scatter_pair(X.to(cuda_device), W1.to(cuda_device), W.to(cuda_device), Ind.to(cuda_device))
+        Y = Mid.cpu()
+    else:
+        Out = ops.gemm_scatter(Y.to(cuda_device), W.to(cuda_device), Ind.to(cuda_device), T)
+    ref = orc.np_scatter(Y, W, Ind, T)
+    err = np.abs(Out.cpu().double().numpy() - ref).max((1, 2)) / np.abs(ref).max()
+    assert err.max() <= 3e-2, err
+    # sums in float32 rows are rounded once: half a unit in the last of bf16's eight bits
+    for b in (2, 5):
+        exact = torch.from_numpy(ref[b]).to(torch.bfloat16).double().numpy()
+        assert np.abs(Out[b].cpu().double().numpy() - exact).max() <= 2.0 ** -8 * np.abs(ref[b]).max()
