@@ -20,7 +20,7 @@ OUT_DIR = os.path.join(PKG, "_lib")
 OBJ_DIR = os.path.join(OUT_DIR, "obj")
 LIB_PATH = os.path.join(OUT_DIR, "libegs_b200.so")
 HOST_PATH = os.path.join(OUT_DIR, "_egs_host.so")
-SOURCES = ["egs_api.cu", "egs_generic.cu", "egs_tensor.cu", "egs_strict.cu", "egs_pair16.cu", "egs_gather2.cu", "egs_index.cu"]
+SOURCES = ["egs_api.cu", "egs_generic.cu", "egs_tensor.cu", "egs_strict.cu", "egs_dense16.cu", "egs_pair16.cu", "egs_gather2.cu", "egs_index.cu"]
 HOST_SOURCE = os.path.join(CSRC, "egs_host.cpp")
 API_HEADER = os.path.join(PKG, "..", "include", "egs_b200.h")
 HEADERS = [os.path.join(CSRC, "egs_internal.cuh"), os.path.join(CSRC, "egs_tcgen05.cuh"), API_HEADER]

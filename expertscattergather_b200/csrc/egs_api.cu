@@ -11,7 +11,7 @@
 
 namespace egs {
 
-bool encode_tensor_map_16bit(TensorMap3* out, const void* base, const unsigned long long dims[3], const unsigned box[3]) {
+bool encode_tensor_map_16bit(TensorMap3* out, const void* base, int rank, const unsigned long long* dims, const unsigned* box) {
   using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -24,13 +24,18 @@ bool encode_tensor_map_16bit(TensorMap3* out, const void* base, const unsigned l
     return reinterpret_cast<EncodeFn>(fn);
   }();
   static_assert(sizeof(TensorMap3) == sizeof(CUtensorMap), "tensor map size");
-  if (!encode || !out || !base) return false;
-  const cuuint64_t gdim[3] = {dims[0], dims[1], dims[2]};
-  const cuuint64_t gstride[2] = {dims[0] * 2ull, dims[0] * dims[1] * 2ull};      // bytes, dimensions 1 and 2
-  const cuuint32_t bdim[3] = {box[0], box[1], box[2]};
-  const cuuint32_t estride[3] = {1u, 1u, 1u};
+  if (!encode || !out || !base || rank < 2 || rank > 4) return false;
+  cuuint64_t gdim[4], gstride[3];
+  cuuint32_t bdim[4], estride[4] = {1u, 1u, 1u, 1u};
+  cuuint64_t pitch = 2;                                  // bytes from one element of dimension i to the next
+  for (int i = 0; i < rank; ++i) {
+    gdim[i] = dims[i];
+    bdim[i] = box[i];
+    pitch *= dims[i];
+    if (i + 1 < rank) gstride[i] = pitch;
+  }
   // CU_TENSOR_MAP_DATA_TYPE_UINT16: the loads only move bits, so one map type serves bf16 and fp16
-  const CUresult rc = encode(reinterpret_cast<CUtensorMap*>(out), CU_TENSOR_MAP_DATA_TYPE_UINT16, 3u, const_cast<void*>(base), gdim,
+  const CUresult rc = encode(reinterpret_cast<CUtensorMap*>(out), CU_TENSOR_MAP_DATA_TYPE_UINT16, static_cast<cuuint32_t>(rank), const_cast<void*>(base), gdim,
                              gstride, bdim, estride, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return rc == CUDA_SUCCESS;
@@ -203,6 +208,9 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
       const size_t smem2 = configure_tensor_gather2(p);
       if (smem2 == 0) return EGS_ERR_UNSUPPORTED;
       err = launch_tensor_gather2(p, dtype, smem2, st);
+    } else if (dtype != EGS_F32) {
+      configure_dense16_rowgemm(p, scatter);
+      err = launch_dense16_rowgemm(p, scatter, dtype, st);
     } else {
       const size_t smem = configure_tensor_rowgemm(p, scatter, dtype);
       err = launch_tensor_rowgemm(p, scatter, dtype, smem, st);
@@ -485,14 +493,17 @@ static int dweight_impl(const void* Xsrc, const void* Ysrc, const void* Ind, voi
 
   size_t smem = 0;
   const bool strict = tensor && dtype == EGS_F32 && precision == EGS_PREC_STRICT;
+  const bool dense16 = tensor && dtype != EGS_F32;
   if (strict) {
     configure_strict_dweight(p);
+  } else if (dense16) {
+    configure_dense16_dweight(p);
   } else if (tensor) {
     smem = configure_tensor_dweight(p, dtype);
   } else {
     configure_generic_dweight(p);
   }
-  if (!strict && static_cast<long long>(p.E) * p.splits > 65535) return EGS_ERR_TOO_LARGE;   // grid.z limit
+  if (!strict && !dense16 && static_cast<long long>(p.E) * p.splits > 65535) return EGS_ERR_TOO_LARGE;   // grid.z limit
 
   cudaError_t err;
   if (p.splits > 1) {
@@ -508,7 +519,7 @@ static int dweight_impl(const void* Xsrc, const void* Ysrc, const void* Ind, voi
       p.after_own = 1;
     }
   }
-  err = strict ? launch_strict_dweight(p, st) : tensor ? launch_tensor_dweight(p, dtype, smem, st) : launch_generic_dweight(p, dtype, st);
+  err = strict ? launch_strict_dweight(p, st) : dense16 ? launch_dense16_dweight(p, dtype, st) : tensor ? launch_tensor_dweight(p, dtype, smem, st) : launch_generic_dweight(p, dtype, st);
   if (err != cudaSuccess) return fail_cuda(err, "dweight launch");
   if (p.splits > 1 && dtype != EGS_F32) {
     err = launch_convert_from_f32(p.acc, out, n_out, dtype, st, tensor);   // (the tensor-core kernel triggers its dependents)
@@ -589,7 +600,8 @@ int egs_describe_plan(int op, const egs_dims* dims, int w_layout, int dtype, int
     DWeightParams p{};
     p.B = static_cast<int>(d.B); p.T = static_cast<int>(d.T); p.E = static_cast<int>(d.E); p.K = static_cast<int>(d.K);
     p.FG = static_cast<int>(d.C); p.FD = static_cast<int>(d.N); p.M = static_cast<int>(d.B * d.K);
-    if (dtype == EGS_F32 && precision == EGS_PREC_STRICT) configure_strict_dweight(p);
+    if (dtype != EGS_F32) configure_dense16_dweight(p);
+    else if (precision == EGS_PREC_STRICT) configure_strict_dweight(p);
     else configure_tensor_dweight(p, dtype);
     out->tile_n = p.BN; out->stages = p.stages; out->row_tiles = p.row_tiles; out->splits = p.splits;
     out->rows_per_split = p.rows_per_split;
@@ -600,7 +612,8 @@ int egs_describe_plan(int op, const egs_dims* dims, int w_layout, int dtype, int
   p.C = static_cast<int>(d.C); p.N = static_cast<int>(d.N); p.M = static_cast<int>(d.B * d.K);
   p.w_layout = w_layout;
   p.expert_fastest = pick_expert_fastest(d, op == 1, dtype);
-  if (dtype == EGS_F32 && precision == EGS_PREC_STRICT) configure_strict_rowgemm(p);
+  if (dtype != EGS_F32) configure_dense16_rowgemm(p, op == 1);
+  else if (precision == EGS_PREC_STRICT) configure_strict_rowgemm(p);
   else configure_tensor_rowgemm(p, op == 1, dtype);
   out->tile_n = p.BN; out->stages = p.stages; out->row_tiles = p.row_tiles; out->persistent = p.persistent;
   out->bulk_epilogue = (p.persistent || op == 1) ? p.bulk_epilogue : 0; out->expert_fastest = p.expert_fastest;

@@ -1,0 +1,763 @@
+// Operators G, S and D for 16-bit tensors as one persistent, warp-specialised kernel (sm_100a).
+//
+//   warps 0..7    gather producers: index-driven 16-byte cp.async row copies into the stage ring
+//   warps 8..15   read-out: tensor memory -> stores (G, D) / bulk reductions or red.global.add (S)
+//   warp  16      tensor-memory allocation; one lane issues tcgen05.mma, four per stage as straight-line code
+//   warp  17      one lane issues the TMA box loads of everything that is not gathered
+//   warps 18, 19  (D) look up the token rows of the contraction rows to come into a table in shared memory
+//
+// A unit of work is one 128 x BN accumulator tile; CTAs (one per SM) walk the units, the stage ring runs on across them and the
+// accumulator is double-buffered in tensor memory, so neither set-up nor read-out stands between two tiles.
+//   G  rows = expert rows, token rows through Ind (cp.async);     columns = W[e] (TMA)
+//   S  rows = expert rows, slot rows (TMA where 128 rows are whole batch elements or parts of one, else cp.async);  columns = W[e]
+//   D  contraction = expert rows; one operand the gathered token rows (cp.async), the other the slot rows (TMA under the same
+//      condition for 64 rows, else cp.async).  Either may be the one whose features are the accumulator's rows.
+//
+// What bounds the main loop is shared-memory bandwidth: a stage (64 contraction elements) of a 128 x 256 tile is 48 KB written
+// and 48 KB read by its four MMAs, 750 clocks at 128 bytes per clock against 512 clocks of tensor work.  The two copy paths have
+// to stay below that, and neither does alone: 16-byte cp.async costs about 10 clocks per warp instruction (960 for such a stage),
+// a TMA box about 2 clocks per 128-byte row.  Split between them, a stage of G costs the load/store unit 320 and the TMA unit
+// 550 clocks, side by side.  A lone issuing lane needs 7-10 clocks per instruction: nothing on the per-stage paths of the TMA and
+// MMA lanes divides or multiplies.
+#include <type_traits>
+
+#include "egs_tcgen05.cuh"
+
+namespace egs {
+
+namespace {
+
+constexpr int kProdWarps = 8, kProdThreads = kProdWarps * 32;
+constexpr int kEpiWarps = 8;
+constexpr int kMmaWarp = kProdWarps + kEpiWarps, kTmaWarp = kMmaWarp + 1;
+constexpr int kIndexWarp = kTmaWarp + 1, kIndexWarps = 2;      // D only
+template <int OP> constexpr int kDenseThreads = (OP == 2 ? kIndexWarp + kIndexWarps : kTmaWarp + 1) * 32;
+constexpr int kStep = 64;                          // contraction elements per stage
+constexpr uint32_t kDenseHeader = 1024;
+constexpr int kBatch = 256;                        // D: contraction rows whose ids are looked up at a time (four steps)
+// D: two batches of token rows; without TMA boxes for the slot rows two of those as well.  (Sized so that four stages of a
+// 128 x 256 tile still fit beside it with TMA boxes: three stages cost a quarter of the rate.)
+__host__ __device__ constexpr uint32_t table_bytes(bool slots) { return (slots ? 4u : 2u) * kBatch * 4u; }
+constexpr uint32_t kMTile = 16384;                 // bytes of the 128-wide operand: 128 rows x 64 elements, or 64 rows x 128
+constexpr uint32_t kSeg = kStep * 128u;            // one 64-column segment of a 64-row tile
+constexpr uint32_t kEpiPlain = kEpiWarps * 4096u;
+constexpr uint32_t kEpiBulk = (kEpiWarps * 2u * kBulkBufBytes + 1023u) & ~1023u;
+constexpr size_t kSmemMax = 227 * 1024;
+constexpr int kSms = 148;
+
+enum { kOpGather = 0, kOpScatter = 1, kOpDweight = 2 };
+
+struct __align__(16) DenseHeader {
+  unsigned long long full[kMaxStages];
+  unsigned long long empty[kMaxStages];
+  unsigned long long acc_full[2];
+  unsigned long long acc_empty[2];
+  unsigned long long ids_full[2];
+  unsigned long long ids_empty[2];
+  unsigned long long drain;
+  uint32_t tmem_base;
+  uint32_t abort_flag;
+};
+static_assert(sizeof(DenseHeader) <= kDenseHeader, "header does not fit");
+
+struct DenseParams {
+  const void* Rows;   // G, D: token rows; S: slot rows
+  const void* Slot;   // D: slot rows
+  const void* bias;   // G, S: [E, N] or NULL
+  const void* Ind;
+  void* Out;          // G: slot rows; S: token rows; D: the gradient
+  float* acc;         // S: float32 rows; D: float32 sums when splits > 1
+  const int* plan;    // S: see RowGemmParams::plan
+  StatusRef status;
+  int B, T, E, K, M;
+  int C, N;           // G, S: contraction and produced width; D: features of the operand along the accumulator's rows / columns
+  int nc;             // G, S: 1 = weights [E, N, C]
+  int index_dtype;
+  int BN, stages;
+  int tiles_m, tiles_n, units, order;    // order: 1 = experts vary faster than row blocks
+  int splits, rows_per_split;            // D
+  int swap;           // D: 1 = the slot rows' features are the accumulator's rows
+  int lane_rows;      // D: 1 = the output's rows are the accumulator's rows
+  int tma_rows;       // S, D: slot rows come by TMA
+  int bulk;           // S
+};
+
+struct Unit {
+  int e, m0, n0, split;
+};
+template <int OP>
+__device__ __forceinline__ Unit unit_of(const DenseParams& p, int u) {
+  Unit r;
+  const int nt = u % p.tiles_n;
+  u /= p.tiles_n;
+  int mt;
+  r.split = 0;
+  if (OP == kOpDweight) {
+    mt = u % p.tiles_m;
+    u /= p.tiles_m;
+    r.split = u % p.splits;
+    r.e = u / p.splits;
+  } else if (p.order) {
+    r.e = u % p.E;
+    mt = u / p.E;
+  } else {
+    mt = u % p.tiles_m;
+    r.e = u / p.tiles_m;
+  }
+  r.m0 = mt * kTileM;
+  r.n0 = nt * p.BN;
+  return r;
+}
+template <int OP>
+__device__ __forceinline__ int unit_steps(const DenseParams& p, const Unit& u) {
+  if (OP != kOpDweight) return (p.C + kStep - 1) / kStep;
+  return (min(p.rows_per_split, p.M - u.split * p.rows_per_split) + kStep - 1) / kStep;
+}
+
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* map, int x, int y, int z, int w, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
+      : "memory");
+}
+
+template <typename T, int OP>
+__global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __grid_constant__ DenseParams p, const __grid_constant__ TensorMap3 map_w,
+                                                                   const __grid_constant__ TensorMap3 map_rows) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  DenseHeader* hdr = reinterpret_cast<DenseHeader*>(smem_raw);
+  const uint32_t smem0 = smem_u32(smem_raw);
+  const uint32_t epi0 = smem0 + kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : 0u);
+  const uint32_t ring0 = epi0 + ((OP == kOpScatter && p.bulk) ? kEpiBulk : kEpiPlain);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nseg = (p.BN + 63) >> 6;
+  const uint32_t n_bytes = (OP != kOpDweight && p.nc) ? static_cast<uint32_t>(p.BN) * 128u : static_cast<uint32_t>(nseg) * kSeg;
+  const uint32_t stage_bytes = kMTile + n_bytes;
+  const int stages = p.stages;
+  const uint32_t acc_cols = tmem_cols_for(p.BN);
+  const uint32_t tmem_cols = 2u * acc_cols;
+  volatile uint32_t* abort_flag = &hdr->abort_flag;
+  const bool has_cp = OP != kOpScatter || !p.tma_rows;
+  const bool has_tma = OP != kOpDweight || p.tma_rows;
+
+  if (tid == 0) {
+    for (int s = 0; s < kMaxStages; ++s) {
+      mbar_init(smem_u32(&hdr->full[s]), (has_cp ? kProdThreads : 0) + (has_tma ? 1 : 0));
+      mbar_init(smem_u32(&hdr->empty[s]), 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_u32(&hdr->acc_full[b]), 1);
+      mbar_init(smem_u32(&hdr->acc_empty[b]), kEpiWarps);
+      mbar_init(smem_u32(&hdr->ids_full[b]), kIndexWarps * 32);
+      mbar_init(smem_u32(&hdr->ids_empty[b]), kProdWarps);
+    }
+    mbar_init(smem_u32(&hdr->drain), 1);
+    fence_mbar_init();
+    hdr->abort_flag = p.status.timed_out() ? 1u : 0u;
+    if (smem_misaligned(smem_raw)) {
+      hdr->abort_flag = 1u;
+      p.status.report(EGS_STATUS_INTERNAL);
+    }
+  }
+  if (warp == kMmaWarp) {
+    tmem_alloc(smem_u32(&hdr->tmem_base), tmem_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = hdr->tmem_base;
+  pdl_trigger();
+
+  if (hdr->abort_flag != 0u) {
+    // fall through to the common exit
+  } else if (warp < kProdWarps) {
+    // =========================== gather producers ===========================
+    if (has_cp) {
+      const char* Rows = static_cast<const char*>(p.Rows);
+      const int cc = tid & 7, r0 = tid >> 3;
+      const uint32_t rc_dst = static_cast<uint32_t>(r0) * 128u + (static_cast<uint32_t>(cc ^ (r0 & 7)) << 4);
+      const long long pitch_c = static_cast<long long>(p.C) * 2;
+      int slot = 0, round = 0;
+      bool alive = true;
+      if constexpr (OP != kOpDweight) {
+        long long ahead_t[4];              // G: token ids of the next unit's rows, loaded a unit ahead
+        auto fetch_ids = [&](int v) {
+          const Unit w = unit_of<OP>(p, v);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int m = min(w.m0 + r0 + 32 * i, p.M - 1), b = m / p.K;
+            ahead_t[i] = load_index(p.Ind, p.index_dtype, static_cast<long long>(b * p.E + w.e) * p.K + (m - b * p.K));
+          }
+        };
+        if (OP == kOpGather && static_cast<int>(blockIdx.x) < p.units) fetch_ids(blockIdx.x);
+        for (int un = blockIdx.x; un < p.units && alive; un += gridDim.x) {
+          const Unit u = unit_of<OP>(p, un);
+          const int steps = unit_steps<OP>(p, u);
+          const char* src[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int m = u.m0 + r0 + 32 * i, b = m / p.K;
+            int row = -1;
+            if (OP == kOpScatter) row = m < p.M ? (b * p.E + u.e) * p.K + (m - b * p.K) : -1;
+            else if (m < p.M && ahead_t[i] >= 0 && ahead_t[i] < p.T) row = b * p.T + static_cast<int>(ahead_t[i]);
+            src[i] = row >= 0 ? Rows + static_cast<long long>(row) * pitch_c + cc * 16 : nullptr;
+          }
+          if (OP == kOpGather && un + static_cast<int>(gridDim.x) < p.units) fetch_ids(un + gridDim.x);
+          for (int k = 0; k < steps; ++k) {
+            if (round > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[slot]), (round - 1) & 1, abort_flag, p.status.word, lane);
+            if (!alive) break;
+            const uint32_t base = ring0 + static_cast<uint32_t>(slot) * stage_bytes + rc_dst;
+            const bool kvalid = k * kStep + cc * 8 < p.C;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const bool v = kvalid && src[i];
+              cp_async16(base + i * 4096u, v ? src[i] : Rows, v ? 16u : 0u);
+              if (src[i]) src[i] += 128;
+            }
+            cp_async_mbar_arrive_noinc(smem_u32(&hdr->full[slot]));
+            if (++slot == stages) { slot = 0; ++round; }
+          }
+        }
+      } else {
+        // A 64-row tile is walked with a fixed 16-byte chunk per thread: 16 threads per row of the 128-wide operand (4 rows per
+        // thread, 16 apart), 4 * RN threads per row of the BN-wide one (RN rows per thread).  Rows are whole multiples of eight
+        // apart, so the swizzle of a thread's chunk is the same in all of them.  A warp must not spend more than some 60
+        // instructions on a step (two producer warps share a scheduler, and a step is 500-1000 clocks): the counts are template
+        // parameters, the products 32-bit.  Generic loops took 390 instructions and twice the kernel's time.
+        // The index warps keep the token (and slot) rows of two batches of kBatch contraction rows in shared memory.  A step's ids
+        // are read one step ahead, before the copies of the step before it are issued: a read behind a copy waits for it.
+        auto run = [&](auto rn_tag, auto swap_tag, auto tma_tag) {
+          constexpr int RN = decltype(rn_tag)::value, kBatchSteps = kBatch / kStep;
+          constexpr bool SWAP = decltype(swap_tag)::value, TMA = decltype(tma_tag)::value;
+          constexpr int RG = SWAP ? RN : 4, RS = SWAP ? 4 : RN;                      // rows per thread: gathered, slot operand
+          constexpr int TN = 4 * RN;                                                 // threads per row of the BN-wide operand
+          const int m_c = tid & 15, m_r = tid >> 4, n_c = tid & (TN - 1), n_r = tid / TN;
+          const bool n_on = n_c * 8 < p.BN;
+          const int g_c = SWAP ? n_c : m_c, g_r = SWAP ? n_r : m_r, s_c = SWAP ? m_c : n_c, s_r = SWAP ? m_r : n_r;
+          const bool g_on = !SWAP || n_on, s_on = !TMA && (SWAP || n_on);
+          constexpr uint32_t GSTEP = kStep / RG, SSTEP = kStep / RS;                 // rows from one of a thread's copies to the next
+          const uint32_t g_dst = ring0 + (SWAP ? kMTile : 0u) + static_cast<uint32_t>(g_c >> 3) * kSeg + g_r * 128u + (((g_c & 7) ^ (g_r & 7)) << 4);
+          const uint32_t s_dst = ring0 + (SWAP ? 0u : kMTile) + static_cast<uint32_t>(s_c >> 3) * kSeg + s_r * 128u + (((s_c & 7) ^ (s_r & 7)) << 4);
+          const unsigned g_pitch = static_cast<unsigned>(SWAP ? p.N : p.C) * 2u, s_pitch = static_cast<unsigned>(SWAP ? p.C : p.N) * 2u;
+          const uint32_t table = smem0 + kDenseHeader;                               // [2][token][kBatch], then [2][slot][kBatch]
+          auto get = [](uint32_t a) -> int {
+            int v;
+            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+            return v;
+          };
+          int tg[RG], ts[RS];
+          auto read_ids = [&](uint32_t at) {             // the ids of one step: its first entry in the token table
+#pragma unroll
+            for (int j = 0; j < RG; ++j) tg[j] = get(at + (g_r + j * GSTEP) * 4u);
+            if (!TMA) {
+#pragma unroll
+              for (int j = 0; j < RS; ++j) ts[j] = get(at + 2u * kBatch * 4u + (s_r + j * SSTEP) * 4u);
+            }
+          };
+          int batch = 0;                                                             // batches begun by this CTA
+          if (static_cast<int>(blockIdx.x) < p.units) {
+            alive = mbar_wait_warp(smem_u32(&hdr->ids_full[0]), 0u, abort_flag, p.status.word, lane);
+            read_ids(table);
+          }
+          for (int un = blockIdx.x; un < p.units && alive; un += gridDim.x) {
+            const Unit u = unit_of<OP>(p, un);
+            const int steps = unit_steps<OP>(p, u);
+            const int f0 = (SWAP ? u.n0 : u.m0) + g_c * 8, s0 = (SWAP ? u.m0 : u.n0) + s_c * 8;     // first feature of the chunk
+            const bool g_in = f0 < (SWAP ? p.N : p.C), s_in = s0 < (SWAP ? p.C : p.N);
+            const char* g_col = Rows + (g_in ? static_cast<long long>(f0) * 2 : 0ll);
+            const char* s_col = static_cast<const char*>(p.Slot) + (s_in ? static_cast<long long>(s0) * 2 : 0ll);
+            for (int k = 0; k < steps; ++k) {
+              if (round > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[slot]), (round - 1) & 1, abort_flag, p.status.word, lane);
+              if (!alive) break;
+              int cg[RG], cs[RS];
+#pragma unroll
+              for (int j = 0; j < RG; ++j) cg[j] = tg[j];
+              if (!TMA) {
+#pragma unroll
+                for (int j = 0; j < RS; ++j) cs[j] = ts[j];
+              }
+              const bool unit_end = k + 1 == steps;
+              if (!unit_end && (k + 1) % kBatchSteps != 0) {
+                read_ids(table + static_cast<uint32_t>(batch & 1) * (kBatch * 4u) + static_cast<uint32_t>((k + 1) % kBatchSteps) * (kStep * 4u));
+              } else {                                   // the next batch: of this unit or of the next one
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&hdr->ids_empty[batch & 1]));    // this warp has read the batch
+                ++batch;
+                if (!unit_end || un + static_cast<int>(gridDim.x) < p.units) {
+                  alive = mbar_wait_warp(smem_u32(&hdr->ids_full[batch & 1]), (batch >> 1) & 1, abort_flag, p.status.word, lane);
+                  if (!alive) break;
+                  read_ids(table + static_cast<uint32_t>(batch & 1) * (kBatch * 4u));
+                }
+              }
+              const uint32_t base = static_cast<uint32_t>(slot) * stage_bytes;
+              if (g_on && (RG > 1 || g_r < kStep)) {
+#pragma unroll
+                for (int j = 0; j < RG; ++j)
+                  cp_async16(base + g_dst + j * GSTEP * 128u, g_col + static_cast<unsigned long long>(static_cast<unsigned>(max(cg[j], 0))) * g_pitch,
+                             (g_in && cg[j] >= 0) ? 16u : 0u);
+              }
+              if (s_on && (RS > 1 || s_r < kStep)) {
+#pragma unroll
+                for (int j = 0; j < RS; ++j)
+                  cp_async16(base + s_dst + j * SSTEP * 128u, s_col + static_cast<unsigned long long>(static_cast<unsigned>(max(cs[j], 0))) * s_pitch,
+                             (s_in && cs[j] >= 0) ? 16u : 0u);
+              }
+              cp_async_mbar_arrive_noinc(smem_u32(&hdr->full[slot]));
+              if (++slot == stages) { slot = 0; ++round; }
+            }
+          }
+        };
+        auto pick_rn = [&](auto swap_tag, auto tma_tag) {
+          if (p.BN > 128) run(std::integral_constant<int, 8>{}, swap_tag, tma_tag);
+          else if (p.BN > 64) run(std::integral_constant<int, 4>{}, swap_tag, tma_tag);
+          else if (p.BN > 32) run(std::integral_constant<int, 2>{}, swap_tag, tma_tag);
+          else run(std::integral_constant<int, 1>{}, swap_tag, tma_tag);
+        };
+        if (p.swap) {
+          if (p.tma_rows) pick_rn(std::true_type{}, std::true_type{});
+          else pick_rn(std::true_type{}, std::false_type{});
+        } else {
+          if (p.tma_rows) pick_rn(std::false_type{}, std::true_type{});
+          else pick_rn(std::false_type{}, std::false_type{});
+        }
+      }
+      cp_async_wait_all();
+    }
+  } else if (warp < kMmaWarp) {
+    // =========================== read-out ===========================
+    const int ew = warp - kProdWarps;
+    const int lg = ew & 3, half = ew >> 2;               // TMEM lane group, share of the column blocks
+    const uint32_t area = epi0 + static_cast<uint32_t>(ew) * ((OP == kOpScatter && p.bulk) ? 2u * kBulkBufBytes : 4096u);
+    const uint32_t lane_base = static_cast<uint32_t>(lg * 32) << 16;
+    T* out = static_cast<T*>(p.Out);
+    int q = 0;                                           // bulk groups committed so far by this thread
+    bool alive = true;
+    pdl_wait();                                          // planning flags, zeros the results are added to
+    // G, S: destination of tile row lg * 32 + lane of the next unit - token id, slot, planning flag - loaded a unit ahead
+    long long next_t = 0;
+    int next_slot = -1, next_b = 0, next_flag = 0;
+    auto look_up = [&](int v) {
+      if (OP == kOpDweight || v >= p.units) return;
+      const Unit w = unit_of<OP>(p, v);
+      const int m = w.m0 + lg * 32 + lane;
+      next_slot = -1;
+      next_flag = 0;
+      if (m < p.M) {
+        next_b = m / p.K;
+        next_slot = (next_b * p.E + w.e) * p.K + (m - next_b * p.K);
+        next_t = load_index(p.Ind, p.index_dtype, next_slot);
+        if (OP == kOpScatter) next_flag = p.plan[next_b];
+      }
+    };
+    look_up(blockIdx.x);
+    int t = 0;
+    for (int un = blockIdx.x; un < p.units && alive; un += gridDim.x, ++t) {
+      const Unit u = unit_of<OP>(p, un);
+      const int bn = min(p.BN, p.N - u.n0);              // columns of this tile (a multiple of 8)
+      const int n_end = u.n0 + bn;
+      int my_ro = -1;                                    // G, S: destination row of tile row lg * 32 + lane
+      uint32_t to_f32 = 0u;
+      if (OP != kOpDweight) {
+        if (next_slot >= 0) {
+          const bool ok = next_t >= 0 && next_t < p.T;
+          if (!ok && half == 0 && u.n0 == 0) p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
+          my_ro = OP == kOpGather ? next_slot : (ok ? next_b * p.T + static_cast<int>(next_t) : -1);
+        }
+        if (OP == kOpScatter) to_f32 = __ballot_sync(0xffffffffu, next_flag != 0);
+        look_up(un + gridDim.x);
+      }
+      const T* bias_row = (OP != kOpDweight && p.bias) ? static_cast<const T*>(p.bias) + static_cast<long long>(u.e) * p.N + u.n0 : nullptr;
+      const bool bulk = OP == kOpScatter && p.bulk && to_f32 == 0u;
+      if (OP == kOpScatter && p.bulk && !bulk) bulk_wait_all();    // the transposes below reuse the staging buffers
+      const int buf = t & 1;
+      alive = mbar_wait_warp(smem_u32(&hdr->acc_full[buf]), (t >> 1) & 1, abort_flag, p.status.word, lane);
+      if (!alive) break;
+      tc_fence_after();
+      const uint32_t acc = tmem_base + lane_base + static_cast<uint32_t>(buf) * acc_cols;
+      const bool packed = OP == kOpGather || bulk || (OP == kOpDweight && p.splits == 1 && p.lane_rows);
+      if (packed) {
+        // 64 columns = 128 bytes of a 16-bit row at a time
+        for (int c = half; c * 64 < bn; c += 2, ++q) {
+          const uint32_t srow = OP == kOpScatter ? area + static_cast<uint32_t>(q & 1) * kBulkBufBytes + static_cast<uint32_t>(lane) * kBulkRowPitch
+                                                 : area + static_cast<uint32_t>(lane) * 128u;
+          if (OP == kOpScatter && q >= 2) bulk_wait_read_1();      // the group that used this buffer two blocks ago has been read
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (c * 64 + h * 32 < bn) {
+              uint32_t v[32];
+              tmem_ld32(acc + static_cast<uint32_t>(c * 64 + h * 32), v);
+              tmem_ld_wait();
+              if (OP != kOpDweight && bias_row) add_bias32<T>(bias_row + c * 64 + h * 32, bn - (c * 64 + h * 32), v);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const int ch = h * 4 + j;
+                asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(
+                                 srow + static_cast<uint32_t>(OP == kOpScatter ? ch : ch ^ (lane & 7)) * 16u),
+                             "r"(pack2(out, v[8 * j], v[8 * j + 1])), "r"(pack2(out, v[8 * j + 2], v[8 * j + 3])),
+                             "r"(pack2(out, v[8 * j + 4], v[8 * j + 5])), "r"(pack2(out, v[8 * j + 6], v[8 * j + 7]))
+                             : "memory");
+              }
+            }
+          }
+          const int col0 = u.n0 + c * 64;
+          if (OP == kOpScatter) {
+            fence_proxy_async_smem();
+            const int ncols = min(64, bn - c * 64);
+            if (my_ro >= 0) bulk_reduce_add(out + static_cast<long long>(my_ro) * p.N + col0, srow, static_cast<uint32_t>(ncols) * 2u);
+            bulk_commit();
+          } else {
+            // eight lanes cover the 128 bytes of one row
+            __syncwarp();
+            const int j = lane & 7, col = col0 + j * 8;
+            uint4 x[8];
+#pragma unroll
+            for (int it = 0; it < 8; ++it) {
+              const int row = it * 4 + (lane >> 3);
+              asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];"
+                           : "=r"(x[it].x), "=r"(x[it].y), "=r"(x[it].z), "=r"(x[it].w)
+                           : "r"(area + row * 128u + (static_cast<uint32_t>(j ^ (row & 7)) << 4))
+                           : "memory");
+            }
+            __syncwarp();
+#pragma unroll
+            for (int it = 0; it < 8; ++it) {
+              const int row = it * 4 + (lane >> 3);
+              long long ro;
+              if (OP == kOpGather) {
+                ro = __shfl_sync(0xffffffffu, my_ro, row);
+              } else {
+                const int f = u.m0 + lg * 32 + row;
+                ro = f < p.C ? static_cast<long long>(u.e) * p.C + f : -1;
+              }
+              if (ro >= 0 && col < n_end) *reinterpret_cast<uint4*>(out + ro * p.N + col) = x[it];
+            }
+          }
+        }
+      } else {
+        for (int c = half; c * 32 < bn; c += 2) {
+          const int col0 = u.n0 + c * 32;
+          uint32_t v[32];
+          tmem_ld32(acc + static_cast<uint32_t>(c * 32), v);
+          tmem_ld_wait();
+          if (OP == kOpScatter) {
+            warp_regs_emit(v, area, lane, [&](int row, int cj, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3) {
+              const int ro = __shfl_sync(0xffffffffu, my_ro, row);
+              const int col = col0 + cj;
+              if (ro >= 0 && col < n_end) {
+                const long long off = static_cast<long long>(ro) * p.N + col;
+                if (bias_row) add_bias4<T>(bias_row + c * 32 + cj, x0, x1, x2, x3);
+                if ((to_f32 >> row) & 1u) red4(p.acc + off, x0, x1, x2, x3);
+                else red4(out + off, x0, x1, x2, x3);
+              }
+            });
+          } else if (OP == kOpDweight && p.lane_rows) {  // partial sums, output rows = accumulator rows
+            warp_regs_emit(v, area, lane, [&](int row, int cj, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3) {
+              const int f = u.m0 + lg * 32 + row, col = col0 + cj;
+              if (f < p.C && col < n_end) red4(p.acc + (static_cast<long long>(u.e) * p.C + f) * p.N + col, x0, x1, x2, x3);
+            });
+          } else if (OP == kOpDweight) {                 // output rows = accumulator columns
+            warp_cols_emit(v, area, lane, [&](int ci, int f4, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3) {
+              const int f = u.m0 + lg * 32 + f4;
+              if (f < p.C && col0 + ci < n_end) {
+                const long long off = (static_cast<long long>(u.e) * p.N + col0 + ci) * p.C + f;
+                if (p.splits > 1) red4(p.acc + off, x0, x1, x2, x3);
+                else store4(out + off, x0, x1, x2, x3);
+              }
+            });
+          }
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&hdr->acc_empty[buf]));
+    }
+    if (OP == kOpScatter) bulk_wait_all();               // shared memory must outlive the copy engine's reads
+  } else if (warp == kMmaWarp) {
+    // =========================== MMA issuer ===========================
+    if (lane == 0) {
+      const bool a_mn = OP == kOpDweight, b_mn = OP == kOpDweight || !p.nc;
+      const uint64_t a_desc = a_mn ? make_smem_desc(0u, kSeg, 1024u) : make_smem_desc(0u, 16u, 1024u);
+      const uint64_t b_desc = b_mn ? make_smem_desc(0u, kSeg, 1024u) : make_smem_desc(0u, 16u, 1024u);
+      const uint32_t a_adv = (a_mn ? 16u * 128u : 32u) >> 4, b_adv = (b_mn ? 16u * 128u : 32u) >> 4;
+      bool ok = true;
+      int t = 0, slot = 0, round = 0;
+      uint32_t addr = ring0 >> 4;                        // descriptors: 14 address bits in 16-byte units (shared memory is smaller)
+      for (int un = blockIdx.x; un < p.units && ok; un += gridDim.x, ++t) {
+        const Unit u = unit_of<OP>(p, un);
+        const int steps = unit_steps<OP>(p, u);
+        const int bn = min(p.BN, ((p.N - u.n0) + 15) & ~15);
+        const uint32_t idesc = make_idesc(Elem<T>::fmt, a_mn ? 1u : 0u, b_mn ? 1u : 0u, kTileM, static_cast<uint32_t>(bn));
+        const int buf = t & 1;
+        if (t >= 2) {
+          ok = mbar_wait(smem_u32(&hdr->acc_empty[buf]), ((t >> 1) - 1) & 1, abort_flag, p.status.word);
+          if (!ok) break;
+          tc_fence_after();
+        }
+        const uint32_t d = tmem_base + static_cast<uint32_t>(buf) * acc_cols;
+        for (int ks = 0; ks < steps; ++ks) {
+          ok = mbar_wait(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status.word);
+          if (!ok) break;
+          tc_fence_after();
+          umma_ss_f16_x4(d, a_desc + addr, b_desc + addr + (kMTile >> 4), a_adv, b_adv, idesc, ks > 0 ? 1u : 0u);
+          umma_commit(smem_u32(&hdr->empty[slot]));
+          addr += stage_bytes >> 4;
+          if (++slot == stages) {
+            slot = 0;
+            ++round;
+            addr = ring0 >> 4;
+          }
+        }
+        if (ok) umma_commit(smem_u32(&hdr->acc_full[buf]));
+      }
+    }
+    __syncwarp();
+  } else if (warp >= kIndexWarp) {
+    // =========================== index warps (D) ===========================
+    const uint32_t table = smem0 + kDenseHeader;
+    const int it = tid - kIndexWarp * 32;
+    constexpr int kPer = kBatch / (kIndexWarps * 32);
+    bool alive = true;
+    int batch = 0;
+    for (int un = blockIdx.x; un < p.units && alive; un += gridDim.x) {
+      const Unit u = unit_of<OP>(p, un);
+      const int m_begin = u.split * p.rows_per_split, m_end = min(p.M, m_begin + p.rows_per_split);
+      const bool report = u.m0 == 0 && u.n0 == 0;
+      for (int m0 = m_begin; m0 < m_end && alive; m0 += kBatch, ++batch) {
+        int tok[kPer], slot_row[kPer];
+        long long t[kPer];
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {                 // all loads first
+          const int m = m0 + it + i * kIndexWarps * 32;
+          const bool on = m < m_end;
+          tok[i] = on ? m / p.K : 0;
+          const int s = (tok[i] * p.E + u.e) * p.K + (on ? m - tok[i] * p.K : 0);
+          t[i] = load_index(p.Ind, p.index_dtype, s);
+          slot_row[i] = on ? s : -1;
+        }
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+          const bool known = t[i] >= 0 && t[i] < p.T;
+          if (slot_row[i] >= 0 && !known && report) p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
+          tok[i] = (slot_row[i] >= 0 && known) ? tok[i] * p.T + static_cast<int>(t[i]) : -1;
+        }
+        if (batch >= 2) alive = mbar_wait_warp(smem_u32(&hdr->ids_empty[batch & 1]), ((batch >> 1) - 1) & 1, abort_flag, p.status.word, lane);
+        if (!alive) break;
+        const uint32_t dst = table + static_cast<uint32_t>(batch & 1) * (kBatch * 4u) + static_cast<uint32_t>(it) * 4u;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+          asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + i * kIndexWarps * 128u), "r"(tok[i]) : "memory");
+          if (!p.tma_rows) asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + 2u * kBatch * 4u + i * kIndexWarps * 128u), "r"(slot_row[i]) : "memory");
+        }
+        mbar_arrive(smem_u32(&hdr->ids_full[batch & 1]));
+      }
+    }
+  } else if (has_tma) {
+    // =========================== TMA issuer ===========================
+    if (lane == 0) {
+      const uint32_t bytes = (OP != kOpDweight ? n_bytes : (p.swap ? kMTile : n_bytes)) + ((OP == kOpScatter && p.tma_rows) ? kMTile : 0u);
+      bool ok = true;
+      int slot = 0, round = 0;
+      uint32_t base = ring0;
+      for (int un = blockIdx.x; un < p.units && ok; un += gridDim.x) {
+        const Unit u = unit_of<OP>(p, un);
+        const int steps = unit_steps<OP>(p, u);
+        int m = OP == kOpDweight ? u.split * p.rows_per_split : u.m0;
+        int b = m / p.K, k = m - b * p.K;                // first slot row of the step
+        for (int ks = 0, c0 = 0; ks < steps; ++ks, c0 += kStep) {
+          if (round > 0) {
+            ok = mbar_wait(smem_u32(&hdr->empty[slot]), (round - 1) & 1, abort_flag, p.status.word);
+            if (!ok) break;
+          }
+          const uint32_t bar = smem_u32(&hdr->full[slot]);
+          mbar_arrive_expect_tx(bar, bytes);
+          if (OP != kOpDweight) {
+            if (OP == kOpScatter && p.tma_rows) tma_load_4d(base, &map_rows, c0, k, u.e, b, bar);
+            if (p.nc) {
+              tma_load_3d(base + kMTile, &map_w, c0, u.n0, u.e, bar);
+            } else {
+              for (int s = 0; s < nseg; ++s) tma_load_3d(base + kMTile + s * kSeg, &map_w, u.n0 + s * 64, c0, u.e, bar);
+            }
+          } else {
+            const int ns = p.swap ? 2 : nseg, x0 = p.swap ? u.m0 : u.n0;
+            const uint32_t dst = base + (p.swap ? 0u : kMTile);
+            for (int s = 0; s < ns; ++s) tma_load_4d(dst + s * kSeg, &map_rows, x0 + s * 64, k, u.e, b, bar);
+            k += kStep;                                  // 64 rows are parts of one batch element or whole ones
+            while (k >= p.K) { k -= p.K; ++b; }
+          }
+          base += stage_bytes;
+          if (++slot == stages) {
+            slot = 0;
+            ++round;
+            base = ring0;
+          }
+        }
+      }
+    }
+    __syncwarp();
+  }
+
+  // ---- common exit ----
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kMmaWarp) tmem_release(tmem_base, tmem_cols, smem_u32(&hdr->drain), abort_flag, p.status, lane);
+}
+
+// Slot rows can come as one TMA box per 64-element column segment when `rows` consecutive expert rows starting at a multiple of
+// `rows` are whole batch elements or lie inside one.
+bool rows_fit_boxes(int K, int rows) { return K % rows == 0 || rows % K == 0; }
+bool encode_slot_rows(TensorMap3* map, const void* base, int B, int E, int K, int width, int rows) {
+  const unsigned kk = static_cast<unsigned>(K < rows ? K : rows);
+  const unsigned long long dims[4] = {static_cast<unsigned long long>(width), static_cast<unsigned long long>(K),
+                                      static_cast<unsigned long long>(E), static_cast<unsigned long long>(B)};
+  const unsigned box[4] = {64u, kk, 1u, static_cast<unsigned>(rows) / kk};
+  return encode_tensor_map_16bit(map, base, 4, dims, box);
+}
+
+// Tile width over n columns.  Per step the shared memory moves 2 * (128 + BN) * 128 bytes at 128 bytes per clock; the load/store
+// unit needs lsu0 + lsu1 * BN clocks for its share of the copies; read-out takes epi clocks per column beside the next tile's
+// main loop; units go out in waves of one per SM.
+int pick_bn(int n, long long unit_rows, int steps, double lsu0, double lsu1, double epi) {
+  int best = 256;
+  double best_cost = 1e30;
+  const int top = n < 256 ? (n + 15) / 16 * 16 : 256;
+  for (int bn = top; bn >= 16; bn -= 16) {
+    const long long tiles = (n + bn - 1) / bn;
+    const long long units = unit_rows * tiles, waves = (units + kSms - 1) / kSms;
+    double step = 2.0 * (128 + bn);
+    const double lsu = lsu0 + lsu1 * bn;
+    if (lsu > step) step = lsu;
+    double unit = steps * step;
+    if (epi * bn > unit) unit = epi * bn;
+    const double cost = waves * (unit + 1000) + epi * bn;
+    if (cost < best_cost * 0.98) {
+      best = bn;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
+int ring_stages(int BN, bool nc_tile, uint32_t epi_bytes) {
+  const size_t n_bytes = nc_tile ? static_cast<size_t>(BN) * 128 : static_cast<size_t>((BN + 63) / 64) * kSeg;
+  const size_t s = (kSmemMax - kDenseHeader - epi_bytes) / (kMTile + n_bytes);      // epi_bytes: all that is not ring
+  return static_cast<int>(s > kMaxStages ? kMaxStages : s);
+}
+
+template <typename T, int OP>
+cudaError_t launch(const DenseParams& p, const TensorMap3& mw, const TensorMap3& mr, bool after_own, cudaStream_t st) {
+  const size_t n_bytes = (OP != kOpDweight && p.nc) ? static_cast<size_t>(p.BN) * 128 : static_cast<size_t>((p.BN + 63) / 64) * kSeg;
+  const size_t smem = kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : 0u) + ((OP == kOpScatter && p.bulk) ? kEpiBulk : kEpiPlain) + p.stages * (kMTile + n_bytes);
+  cudaError_t err = ensure_smem_optin<dense16_kernel<T, OP>>(static_cast<int>(kSmemMax));
+  if (err != cudaSuccess) return err;
+  err = launch_kernel(dense16_kernel<T, OP>, p.units < kSms ? p.units : kSms, kDenseThreads<OP>, smem, st, after_own, p, mw, mr);
+  count_launch();
+  return err;
+}
+
+}  // namespace
+
+void configure_dense16_rowgemm(RowGemmParams& p, bool scatter) {
+  const long long row_blocks = static_cast<long long>((p.M + kTileM - 1) / kTileM) * p.E;
+  const int steps = (p.C + kStep - 1) / kStep;
+  const bool cp_rows = !scatter || !rows_fit_boxes(p.K, 128);
+  p.BN = pick_bn(p.N, row_blocks, steps, cp_rows ? 340.0 : 0.0, 0.0, scatter ? 28.0 : 16.0);
+  p.bulk_epilogue = scatter ? 1 : 0;
+  p.stages = ring_stages(p.BN, p.w_layout == EGS_W_NC, scatter ? kEpiBulk : kEpiPlain);
+  p.row_tiles = 2;        // two 128-row accumulators per CTA
+  p.persistent = (scatter && steps <= 4) ? 1 : 0;        // (for egs_describe_plan) the additions outlast the contraction
+}
+
+cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dtype, cudaStream_t st) {
+  DenseParams p{};
+  p.Rows = r.A; p.bias = r.bias; p.Ind = r.Ind; p.Out = r.Out; p.acc = r.acc; p.plan = r.plan; p.status = r.status;
+  p.B = r.B; p.T = r.T; p.E = r.E; p.K = r.K; p.M = r.M; p.C = r.C; p.N = r.N;
+  p.nc = r.w_layout == EGS_W_NC;
+  p.index_dtype = r.index_dtype;
+  p.BN = r.BN; p.stages = r.stages;
+  p.tiles_m = (r.M + kTileM - 1) / kTileM;
+  p.tiles_n = (r.N + r.BN - 1) / r.BN;
+  p.order = r.expert_fastest;
+  p.bulk = r.bulk_epilogue;
+  const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.E;
+  if (units > 2147483647ll - kSms) return cudaErrorInvalidValue;
+  p.units = static_cast<int>(units);
+  TensorMap3 mw{}, mr{};
+  const unsigned long long inner = p.nc ? r.C : r.N, outer = p.nc ? r.N : r.C;
+  const unsigned long long dims[3] = {inner, outer, static_cast<unsigned long long>(r.E)};
+  const unsigned box[3] = {64u, p.nc ? static_cast<unsigned>(r.BN) : static_cast<unsigned>(kStep), 1u};
+  if (!encode_tensor_map_16bit(&mw, r.W, 3, dims, box)) return cudaErrorInvalidValue;
+  p.tma_rows = scatter && rows_fit_boxes(r.K, 128) && encode_slot_rows(&mr, r.A, r.B, r.E, r.K, r.C, 128);
+  const bool half = dtype == EGS_F16;
+  if (scatter) return half ? launch<__half, kOpScatter>(p, mw, mr, r.after_own != 0, st) : launch<__nv_bfloat16, kOpScatter>(p, mw, mr, r.after_own != 0, st);
+  return half ? launch<__half, kOpGather>(p, mw, mr, false, st) : launch<__nv_bfloat16, kOpGather>(p, mw, mr, false, st);
+}
+
+// D: which operand's features are the accumulator's rows, the tile width, and the row ranges.
+static void plan_dweight(const DWeightParams& p, bool& swap, int& bn, int& splits, int& rows) {
+  const bool slot_cp = !rows_fit_boxes(p.K, kStep);
+  double best = 1e30;
+  const long long steps_all = (p.M + kStep - 1) / kStep;
+  // the orientation whose accumulator rows are the output's rows first: its read-out stores whole row segments
+  const bool pref = p.out_layout == EGS_DW_DIRECT_ROWS;
+  for (int o = 0; o < 2; ++o) {
+    const bool sw = o == 0 ? pref : !pref;
+    const int mf = sw ? p.FD : p.FG, nf = sw ? p.FG : p.FD;
+    const long long tm = (mf + kTileM - 1) / kTileM;
+    // load/store clocks per step: 10 per 512 bytes; the gathered operand always, the slot operand where it has no boxes
+    const double lsu0 = (!sw ? 320.0 : 0.0) + (sw && slot_cp ? 320.0 : 0.0), lsu1 = (sw ? 2.5 : 0.0) + (!sw && slot_cp ? 2.5 : 0.0);
+    const double epi = o == 0 ? 16.0 : 24.0;
+    for (int s = 1; s <= 64 && s <= steps_all; s = s < 4 ? s + 1 : s + s / 2) {
+      const long long sp_steps = (steps_all + s - 1) / s;
+      const long long real = (steps_all + sp_steps - 1) / sp_steps;      // ranges of whole steps
+      const double e = real > 1 ? 32.0 : epi;                            // partial tiles are added atomically
+      const int w = pick_bn(nf, tm * p.E * real, static_cast<int>(sp_steps), lsu0, lsu1, e);
+      const long long units = tm * p.E * real * ((nf + w - 1) / w), waves = (units + kSms - 1) / kSms;
+      double step = 2.0 * (128 + w);
+      if (lsu0 + lsu1 * w > step) step = lsu0 + lsu1 * w;
+      double unit = sp_steps * step;
+      if (e * w > unit) unit = e * w;
+      // more than one range: zero fill and rounding of the float32 sums, two launches and 10 bytes an element
+      double cost = waves * (unit + 1000) + e * w;
+      if (real > 1) cost += 9000 + static_cast<double>(p.E) * p.FG * p.FD * 10 / (148 * 20.0);
+      if (cost < best * (o == 0 ? 1.0 : 0.97)) {
+        best = cost;
+        swap = sw;
+        bn = w;
+        splits = static_cast<int>(real);
+        rows = static_cast<int>(sp_steps * kStep);
+      }
+    }
+  }
+}
+
+void configure_dense16_dweight(DWeightParams& p) {
+  bool swap = false;
+  plan_dweight(p, swap, p.BN, p.splits, p.rows_per_split);
+  p.swap = swap ? 1 : 0;
+  p.stages = ring_stages(p.BN, false, table_bytes(!rows_fit_boxes(p.K, kStep)) + kEpiPlain);
+  p.row_tiles = 2;        // two 128-row accumulators per CTA
+}
+
+cudaError_t launch_dense16_dweight(const DWeightParams& r, int dtype, cudaStream_t st) {
+  DenseParams p{};
+  p.Rows = r.Xsrc; p.Slot = r.Ysrc; p.Ind = r.Ind; p.Out = r.out; p.acc = r.acc; p.status = r.status;
+  p.B = r.B; p.T = r.T; p.E = r.E; p.K = r.K; p.M = r.M;
+  p.swap = r.swap;
+  p.C = r.swap ? r.FD : r.FG;
+  p.N = r.swap ? r.FG : r.FD;
+  p.lane_rows = (r.out_layout == EGS_DW_DIRECT_ROWS) == (r.swap != 0);
+  p.index_dtype = r.index_dtype;
+  p.BN = r.BN; p.stages = r.stages; p.splits = r.splits; p.rows_per_split = r.rows_per_split;
+  p.tiles_m = (p.C + kTileM - 1) / kTileM;
+  p.tiles_n = (p.N + r.BN - 1) / r.BN;
+  const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.E * p.splits;
+  if (units > 2147483647ll - kSms) return cudaErrorInvalidValue;
+  p.units = static_cast<int>(units);
+  TensorMap3 mw{}, mr{};
+  p.tma_rows = rows_fit_boxes(r.K, kStep) && encode_slot_rows(&mr, r.Ysrc, r.B, r.E, r.K, r.FD, kStep);
+  return dtype == EGS_F16 ? launch<__half, kOpDweight>(p, mw, mr, r.after_own != 0, st)
+                          : launch<__nv_bfloat16, kOpDweight>(p, mw, mr, r.after_own != 0, st);
+}
+
+}  // namespace egs

@@ -502,7 +502,7 @@ cudaError_t launch_tensor_gather2(const RowGemmParams& p, int dtype, size_t smem
   const unsigned long long dims[3] = {static_cast<unsigned long long>(nc ? p.C : p.N), static_cast<unsigned long long>(nc ? p.N : p.C),
                                       static_cast<unsigned long long>(p.E)};
   const unsigned box[3] = {64u, nc ? static_cast<unsigned>(p.BN / 2) : 64u, 1u};
-  if (!encode_tensor_map_16bit(&m, p.W, dims, box)) return cudaErrorInvalidValue;
+  if (!encode_tensor_map_16bit(&m, p.W, 3, dims, box)) return cudaErrorInvalidValue;
   const long long ntiles = static_cast<long long>((p.M + 2 * kG2Rows - 1) / (2 * kG2Rows)) * p.E;      // 512 expert rows each
   dim3 grid(2 * static_cast<unsigned>(ntiles < kG2Pairs ? ntiles : kG2Pairs));
   dim3 block(kG2Threads);

@@ -100,6 +100,7 @@ struct DWeightParams {
   int stages;
   int row_tiles;      // tensor path: 128-feature accumulator tiles per CTA over FG (1 or 2)
   int after_own;      // launched behind the fill of `acc`: see launch_kernel
+  int swap;           // 16-bit: the slot rows' features run along the accumulator's rows
 };
 
 // Fused pair G -> S (tensor path only):  Mid = gather(Src) x W1[e] is stored as slot rows AND fed, without leaving the
@@ -150,6 +151,12 @@ size_t configure_tensor_dweight(DWeightParams& p, int dtype);
 cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, int dtype, size_t smem_bytes, cudaStream_t st);
 cudaError_t launch_tensor_dweight(const DWeightParams& p, int dtype, size_t smem_bytes, cudaStream_t st);
 
+// 16-bit tensors (egs_dense16.cu): persistent kernels for G, S and D.
+void configure_dense16_rowgemm(RowGemmParams& p, bool scatter);
+cudaError_t launch_dense16_rowgemm(const RowGemmParams& p, bool scatter, int dtype, cudaStream_t st);
+void configure_dense16_dweight(DWeightParams& p);
+cudaError_t launch_dense16_dweight(const DWeightParams& p, int dtype, cudaStream_t st);
+
 // Strict float32 (egs_strict.cu).  Long contractions are fine up to kStrictMaxContraction (see run_rowgemm).
 void configure_strict_rowgemm(RowGemmParams& p);
 cudaError_t launch_strict_rowgemm(const RowGemmParams& p, bool scatter, cudaStream_t st);
@@ -166,13 +173,13 @@ cudaError_t launch_tensor_gather2(const RowGemmParams& p, int dtype, size_t smem
 size_t configure_tensor_pair16(FusedParams& p);
 cudaError_t launch_tensor_pair16(const FusedParams& p, int dtype, size_t smem_bytes, cudaStream_t st);
 
-// Opaque 128-byte TMA tensor map (CUtensorMap of the driver API) and its encoder for a dense 3-D tensor of 16-bit
-// elements, dims[0] innermost, 128-byte swizzle, out-of-range elements read as zero.  Returns false when the driver
+// Opaque 128-byte TMA tensor map (CUtensorMap of the driver API) and its encoder for a dense tensor of 16-bit elements of up to
+// four dimensions, dims[0] innermost, 128-byte swizzle, out-of-range elements read as zero.  Returns false when the driver
 // refuses the geometry (strides must be multiples of 16 bytes, box sides at most 256).
 struct alignas(64) TensorMap3 {
   unsigned char bytes[128];
 };
-bool encode_tensor_map_16bit(TensorMap3* out, const void* base, const unsigned long long dims[3], const unsigned box[3]);
+bool encode_tensor_map_16bit(TensorMap3* out, const void* base, int rank, const unsigned long long* dims, const unsigned* box);
 
 // Index preparation (egs_index.cu).  All index arrays are int32 on the device.
 cudaError_t launch_route_topk(const float* scores, void* ind, int index_dtype, int B, int T, int E, int K, cudaStream_t st);

@@ -563,7 +563,7 @@ cudaError_t launch_tensor_pair16(const FusedParams& p, int dtype, size_t smem_by
   const unsigned b1[3] = {64u, nc ? static_cast<unsigned>(p.N1) : 64u, 1u};
   const unsigned long long d2[3] = {static_cast<unsigned long long>(nc ? p.N1 : p.N2), static_cast<unsigned long long>(nc ? p.N2 : p.N1), e};
   const unsigned b2[3] = {64u, nc ? 64u : static_cast<unsigned>(p.N1), 1u};
-  if (!encode_tensor_map_16bit(&m1, p.W1, d1, b1) || !encode_tensor_map_16bit(&m2, p.W2, d2, b2)) return cudaErrorInvalidValue;
+  if (!encode_tensor_map_16bit(&m1, p.W1, 3, d1, b1) || !encode_tensor_map_16bit(&m2, p.W2, 3, d2, b2)) return cudaErrorInvalidValue;
   const int row_blocks = p.E * ((p.M + kTileM - 1) / kTileM);
   dim3 grid(row_blocks < kP16SmCount ? row_blocks : kP16SmCount);
   dim3 block(kP16Threads);

@@ -324,6 +324,24 @@ __device__ __forceinline__ void warp_regs_emit(const uint32_t (&v)[32], uint32_t
 #pragma unroll
   for (int it = 0; it < 8; ++it) emit(it * 4 + (lane >> 3), j * 4, x[it][0], x[it][1], x[it][2], x[it][3]);
 }
+// The transposed counterpart: 8 lanes cover 32 rows (lanes) of one column, four consecutive rows each.
+//   emit(column, first_row_in_block, x0, x1, x2, x3) is called 8 times per lane.
+template <class Emit>
+__device__ __forceinline__ void warp_cols_emit(const uint32_t (&v)[32], uint32_t tile, int lane, Emit&& emit) {
+#pragma unroll
+  for (int i = 0; i < 32; ++i) asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + i * 128u + lane * 4u), "r"(v[i]) : "memory");
+  __syncwarp();
+  uint32_t x[8][4];
+#pragma unroll
+  for (int it = 0; it < 8; ++it)
+    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(x[it][0]), "=r"(x[it][1]), "=r"(x[it][2]), "=r"(x[it][3])
+                 : "r"(tile + (it * 4 + (lane >> 3)) * 128u + (lane & 7) * 16u)
+                 : "memory");
+  __syncwarp();
+#pragma unroll
+  for (int it = 0; it < 8; ++it) emit(it * 4 + (lane >> 3), (lane & 7) * 4, x[it][0], x[it][1], x[it][2], x[it][3]);
+}
 // The same straight from the accumulator (zeros where nothing was accumulated).
 template <class Emit>
 __device__ __forceinline__ void warp_block_emit(uint32_t taddr, uint32_t tile, int lane, bool have_acc, Emit&& emit) {

@@ -271,8 +271,9 @@ typedef struct egs_plan_info {
   int tensor_path;    /* 1: tcgen05 tensor-core kernels, 0: generic CUDA-core kernels (the fields below are then 0) */
   int tile_n;         /* tile width over the produced features */
   int stages;         /* depth of the shared-memory stage ring */
-  int row_tiles;      /* 128-row accumulator tiles per CTA: 1 or 2 */
-  int persistent;     /* G / S: 1 = the persistent warp-specialised kernel */
+  int row_tiles;      /* 128-row accumulators a CTA holds: 1 or 2 */
+  int persistent;     /* float32 S: 1 = the persistent kernel.  16-bit tensors (all kernels are persistent): 1 = a scatter whose
+                       * tiles are bound by their additions, not by their contraction */
   int bulk_epilogue;  /* S with 16-bit tensors: direct additions go out as bulk reductions */
   int expert_fastest; /* G / S: grid order, 1 = experts vary fastest */
   int splits;         /* D: row ranges the contraction is split into */
