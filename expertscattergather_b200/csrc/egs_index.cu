@@ -32,7 +32,8 @@ __device__ __forceinline__ uint32_t float_key(float f) {
 // sectors (the experts are the contiguous direction: one expert alone would fetch eight times its bytes) and turned through
 // shared memory so that every thread ends up with R keys of its expert in registers.  The K-th largest key is then built bit
 // by bit - R compares and a reduction per bit - and the search stops as soon as exactly K keys lie at or above the candidate,
-// after about 20 of 32 bits for scores without ties.  What bounds it is that chain of reductions, not the bytes.
+// after about 20 of 32 bits for scores without ties.  What bounds it is that chain of reductions and, before it, of chunks read one
+// after the other, not the bytes: few (batch, expert) pairs get more warps each (see launch_route_topk).
 // B=32, T=2048, E=64, K=128: 127 us with one CTA per expert column and shared-memory histograms.
 constexpr int kSelChunk = 8;          // keys per thread and chunk of the turn through shared memory
 constexpr int kSelMaxKeys = 64;       // keys per thread
@@ -42,12 +43,12 @@ __device__ __forceinline__ void expert_sync(int eg) {
   if (WPE == 1) __syncwarp();
   else asm volatile("bar.sync %0, %1;" ::"r"(eg + 1), "r"(WPE * 32) : "memory");
 }
-// sum over the expert's threads; red: WPE slots of this expert
+// sum over the expert's threads; red: two sets of WPE slots of this expert, used in turn (par), so that one barrier is enough
 template <int WPE>
-__device__ __forceinline__ unsigned expert_sum(unsigned v, unsigned* red, int eg, int w, int lane) {
+__device__ __forceinline__ unsigned expert_sum(unsigned v, unsigned* red, int par, int eg, int w, int lane) {
   v = __reduce_add_sync(0xffffffffu, v);
   if (WPE == 1) return v;
-  expert_sync<WPE>(eg);                      // the slots of the previous sum have been read
+  red += (par & 1) * WPE;
   if (lane == 0) red[w] = v;
   expert_sync<WPE>(eg);
   v = 0;
@@ -61,7 +62,7 @@ __global__ void __launch_bounds__(512) route_topk_regs_kernel(const float* __res
                                                               int T, int E, int K, int eg_log2, int P) {
   constexpr int CT = WPE * 32 * kSelChunk;   // tokens per chunk
   extern __shared__ __align__(16) unsigned char sel_smem[];
-  __shared__ unsigned red_s[16], count_s[8];
+  __shared__ unsigned red_s[32], count_s[8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int eg = warp / WPE, w = warp - eg * WPE;       // expert within the CTA, warp within the expert
   const int EG = 1 << eg_log2;
@@ -103,7 +104,7 @@ __global__ void __launch_bounds__(512) route_topk_regs_kernel(const float* __res
   }
   if (e0 + eg >= E) return;       // no CTA-wide barrier below
 
-  unsigned* red = red_s + eg * WPE;
+  unsigned* red = red_s + eg * 2 * WPE;
   uint32_t th = 0;
   bool exact = false;             // exactly K keys are >= th
   for (int bit = 31; bit >= 0 && !exact; --bit) {
@@ -111,7 +112,7 @@ __global__ void __launch_bounds__(512) route_topk_regs_kernel(const float* __res
     unsigned n = 0;
 #pragma unroll
     for (int i = 0; i < R; ++i) n += (key[i] >= cand) ? 1u : 0u;
-    n = expert_sum<WPE>(n, red, eg, w, lane);
+    n = expert_sum<WPE>(n, red, bit, eg, w, lane);
     if (n >= static_cast<unsigned>(K)) th = cand;
     exact = n == static_cast<unsigned>(K);
   }
@@ -652,14 +653,28 @@ static cudaError_t launch_topk_regs(const float* scores, void* ind, int index_dt
 
 cudaError_t launch_route_topk(const float* scores, void* ind, int index_dtype, int B, int T, int E, int K, cudaStream_t st) {
   cudaError_t err = cudaSuccess;
-  // fewest warps per expert that hold its T keys in registers
-  if (T <= 1 * 32 * 8) err = launch_topk_regs<1, 8>(scores, ind, index_dtype, B, T, E, K, st);
-  else if (T <= 1 * 32 * 32) err = launch_topk_regs<1, 32>(scores, ind, index_dtype, B, T, E, K, st);
-  else if (T <= 1 * 32 * kSelMaxKeys) err = launch_topk_regs<1, kSelMaxKeys>(scores, ind, index_dtype, B, T, E, K, st);
-  else if (T <= 2 * 32 * kSelMaxKeys) err = launch_topk_regs<2, kSelMaxKeys>(scores, ind, index_dtype, B, T, E, K, st);
-  else if (T <= 4 * 32 * kSelMaxKeys) err = launch_topk_regs<4, kSelMaxKeys>(scores, ind, index_dtype, B, T, E, K, st);
-  else if (T <= 8 * 32 * kSelMaxKeys) err = launch_topk_regs<8, kSelMaxKeys>(scores, ind, index_dtype, B, T, E, K, st);
-  else route_topk_kernel<<<B * E, kTopkThreads, 0, st>>>(scores, ind, index_dtype, B, T, E, K);
+  if (T > 8 * 32 * kSelMaxKeys) {
+    route_topk_kernel<<<B * E, kTopkThreads, 0, st>>>(scores, ind, index_dtype, B, T, E, K);
+  } else {
+    // Warps per expert: enough for 32 warps per SM in all while every thread still has eight keys, and no fewer than hold the T
+    // keys.  B=1, T=8965, E=34: 23 us with one expert per CTA of eight warps and 64 keys each.
+    int wpe = 1;
+    while (wpe < 8 && (T > wpe * 32 * kSelMaxKeys || (T > wpe * 32 * 8 && static_cast<long long>(B) * E * wpe < 148 * 32))) wpe *= 2;
+    int r = 8;
+    while (T > wpe * 32 * r) r *= 2;
+#define EGS_TOPK_R(W)                                                                          \
+  do {                                                                                         \
+    if (r == 8) err = launch_topk_regs<W, 8>(scores, ind, index_dtype, B, T, E, K, st);        \
+    else if (r == 16) err = launch_topk_regs<W, 16>(scores, ind, index_dtype, B, T, E, K, st); \
+    else if (r == 32) err = launch_topk_regs<W, 32>(scores, ind, index_dtype, B, T, E, K, st); \
+    else err = launch_topk_regs<W, 64>(scores, ind, index_dtype, B, T, E, K, st);              \
+  } while (0)
+    if (wpe == 1) EGS_TOPK_R(1);
+    else if (wpe == 2) EGS_TOPK_R(2);
+    else if (wpe == 4) EGS_TOPK_R(4);
+    else EGS_TOPK_R(8);
+#undef EGS_TOPK_R
+  }
   count_launch();
   return err != cudaSuccess ? err : cudaGetLastError();
 }
