@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(kSumThreads) expert_row_sum_kernel(const T* __
   float acc[PER];
 #pragma unroll
   for (int i = 0; i < PER; ++i) acc[i] = 0.f;
-  constexpr int U = 4;
+  constexpr int U = 8;
   for (int m0 = rank * per + rl; m0 < m_end; m0 += U * ROWS) {
     long long row[U];
 #pragma unroll
@@ -593,9 +593,9 @@ static cudaError_t launch_row_sum(const void* Src, const void* Ind, int index_dt
                                   StatusRef status, cudaStream_t st) {
   constexpr int cols = 8 * (VEC ? 16 / static_cast<int>(sizeof(T)) : 1);
   const int M = B * K, blocks = (N + cols - 1) / cols;
-  // CTAs per cluster: enough for about two per SM, at least 128 rows each
+  // CTAs per cluster: up to eight per SM in all (they are latency chains: id, row, sum), at least 128 rows each
   int ranks = 1;
-  while (ranks < 8 && static_cast<long long>(blocks) * E * ranks < 2 * 148 && M >= 128 * 2 * ranks) ranks *= 2;
+  while (ranks < 8 && static_cast<long long>(blocks) * E * ranks < 8 * 148 && M >= 128 * 2 * ranks) ranks *= 2;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(ranks, blocks, E);
   cfg.blockDim = dim3(kSumThreads);

@@ -471,7 +471,13 @@ Tensor expert_row_sum(const Tensor& Src, const OptTensor& Ind, int64_t B, int64_
 }
 
 // ---- backward passes of the two operators ------------------------------------------------------------------------------------
-// The weight gradient runs on the helper stream next to the dX / dY kernel: the two are independent and share the SMs.
+// The weight gradient runs on the helper stream next to the dX / dY kernel: the two are independent and share the SMs.  Below
+// kSmallWork multiply-adds (kernels of under 10 us) a backward pass is bound by the host, and the fork and join are left out.
+constexpr double kSmallWork = 1 << 27;
+bool worth_a_side_stream(const Tensor& slot_rows, const Tensor& W) {      // [B,E,K,J] and a weight tensor of E * I * J elements
+  const double slots = static_cast<double>(slot_rows.size(0)) * slot_rows.size(2);
+  return slots * W.numel() > kSmallWork;
+}
 struct Grads {
   Tensor in, w, b;
 };
@@ -483,7 +489,7 @@ Grads gather_backward(const Tensor& X_, const Tensor& W, const Tensor& Ind_, con
   std::optional<SideStream> side;
   if (need_w) {
     std::optional<cudaStream_t> on;
-    if (need_x || need_b) {
+    if ((need_x || need_b) && worth_a_side_stream(dY, W)) {
       side.emplace(Call(X, dY));
       on = side->stream();
     }
@@ -501,7 +507,7 @@ Grads scatter_backward(const Tensor& Y_, const Tensor& W, const Tensor& Ind_, co
   std::optional<SideStream> side;
   if (need_w) {
     std::optional<cudaStream_t> on;
-    if (need_y || need_b) {
+    if ((need_y || need_b) && worth_a_side_stream(Y, W)) {
       side.emplace(Call(Y, dOut));
       on = side->stream();
     }
@@ -595,18 +601,27 @@ struct GatherScatterFunction : torch::autograd::Function<GatherScatterFunction> 
     const Tensor dOut = grads[0].contiguous();
     Tensor dX, dWg, dWs, dY, ws;
     std::optional<SideStream> side;
+    const bool fork = worth_a_side_stream(Y, Wg);
+    std::optional<cudaStream_t> on;
     if (need_ws) {                                     // needs only dOut and Y
-      side.emplace(Call(X, dOut));
-      dWs = dweight_on(dOut, Y, Ind, EGS_DW_DIRECT_ROWS, -1, -1, std::nullopt, side->stream(), &ws);
+      if (fork) {
+        side.emplace(Call(X, dOut));
+        on = side->stream();
+      }
+      dWs = dweight_on(dOut, Y, Ind, EGS_DW_DIRECT_ROWS, -1, -1, std::nullopt, on, &ws);
     }
     if (need_x && ctx->saved_data["fused"].toBool())
       std::tie(dY, dX) = gather_scatter_pair(dOut, Ws, Wg, Ind, EGS_W_NC, std::nullopt, -1);
     else if (need_x || need_wg)
       dY = gather_gemm(dOut, Ws, Ind, EGS_W_NC, -1, -1, std::nullopt);
     if (need_wg) {
-      if (side) side->sync_from_main();
-      else side.emplace(Call(X, dOut));
-      dWg = dweight_on(X, dY, Ind, EGS_DW_GATHERED_ROWS, -1, -1, std::nullopt, side->stream(), &ws);
+      if (side) {
+        side->sync_from_main();
+      } else if (fork) {
+        side.emplace(Call(X, dOut));
+        on = side->stream();
+      }
+      dWg = dweight_on(X, dY, Ind, EGS_DW_GATHERED_ROWS, -1, -1, std::nullopt, on, &ws);
     }
     if (need_x && !dX.defined()) dX = gemm_scatter(dY, Wg, Ind, X.size(1), EGS_W_NC, std::nullopt, -1, -1, std::nullopt, std::nullopt);
     return {dX, dWg, dWs, Tensor()};
