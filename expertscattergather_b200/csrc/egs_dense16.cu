@@ -50,6 +50,7 @@ enum { kOpGather = 0, kOpScatter = 1, kOpDweight = 2 };
 struct __align__(16) DenseHeader {
   unsigned long long full[kMaxStages];
   unsigned long long empty[kMaxStages];
+  unsigned long long peer_full[kMaxStages];          // pairs: the peer's half of a stage has landed (the leader's copy is used)
   unsigned long long acc_full[2];
   unsigned long long acc_empty[2];
   unsigned long long ids_full[2];
@@ -80,12 +81,13 @@ struct DenseParams {
   int lane_rows;      // D: 1 = the output's rows are the accumulator's rows
   int tma_rows;       // S, D: slot rows come by TMA
   int bulk;           // S
+  int half;           // columns of a tile one CTA stages: BN, or BN / 2 in a pair
 };
 
 struct Unit {
   int e, m0, n0, split;
 };
-template <int OP>
+template <int OP, bool PAIR>
 __device__ __forceinline__ Unit unit_of(const DenseParams& p, int u) {
   Unit r;
   const int nt = u % p.tiles_n;
@@ -104,9 +106,19 @@ __device__ __forceinline__ Unit unit_of(const DenseParams& p, int u) {
     mt = u % p.tiles_m;
     r.e = u / p.tiles_m;
   }
-  r.m0 = mt * kTileM;
+  r.m0 = PAIR ? mt * 2 * kTileM + static_cast<int>(blockIdx.x & 1) * kTileM : mt * kTileM;     // this CTA's 128 rows
   r.n0 = nt * p.BN;
   return r;
+}
+// width of a tile's MMA (the last tile of a row may be narrower), and the first column this CTA stages
+template <bool PAIR>
+__device__ __forceinline__ int mma_width(const DenseParams& p, const Unit& u) {
+  const int left = p.N - u.n0;
+  return min(p.BN, PAIR ? (left + 31) & ~31 : (left + 15) & ~15);
+}
+template <bool PAIR>
+__device__ __forceinline__ int first_column(const DenseParams& p, const Unit& u) {
+  return PAIR && (blockIdx.x & 1) ? u.n0 + mma_width<true>(p, u) / 2 : u.n0;
 }
 template <int OP>
 __device__ __forceinline__ int unit_steps(const DenseParams& p, const Unit& u) {
@@ -121,8 +133,8 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* map, int x
       : "memory");
 }
 
-template <typename T, int OP>
-__global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __grid_constant__ DenseParams p, const __grid_constant__ TensorMap3 map_w,
+template <typename T, int OP, bool PAIR>
+__global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __grid_constant__ DenseParams p, const __grid_constant__ TensorMap3 map_w,
                                                                    const __grid_constant__ TensorMap3 map_rows) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   DenseHeader* hdr = reinterpret_cast<DenseHeader*>(smem_raw);
@@ -130,8 +142,10 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
   const uint32_t epi0 = smem0 + kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : 0u);
   const uint32_t ring0 = epi0 + ((OP == kOpScatter && p.bulk) ? kEpiBulk : kEpiPlain);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int nseg = (p.BN + 63) >> 6;
-  const uint32_t n_bytes = (OP != kOpDweight && p.nc) ? static_cast<uint32_t>(p.BN) * 128u : static_cast<uint32_t>(nseg) * kSeg;
+  const int first = PAIR ? blockIdx.x >> 1 : blockIdx.x, stride = PAIR ? gridDim.x >> 1 : gridDim.x;    // units of this CTA or pair
+  const bool leader = !PAIR || (blockIdx.x & 1) == 0;
+  const int nseg = (p.half + 63) >> 6;
+  const uint32_t n_bytes = (OP != kOpDweight && p.nc) ? static_cast<uint32_t>(p.half) * 128u : static_cast<uint32_t>(nseg) * kSeg;
   const uint32_t stage_bytes = kMTile + n_bytes;
   const int stages = p.stages;
   const uint32_t acc_cols = tmem_cols_for(p.BN);
@@ -144,10 +158,11 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
     for (int s = 0; s < kMaxStages; ++s) {
       mbar_init(smem_u32(&hdr->full[s]), (has_cp ? kProdThreads : 0) + (has_tma ? 1 : 0));
       mbar_init(smem_u32(&hdr->empty[s]), 1);
+      mbar_init(smem_u32(&hdr->peer_full[s]), 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&hdr->acc_full[b]), 1);
-      mbar_init(smem_u32(&hdr->acc_empty[b]), kEpiWarps);
+      mbar_init(smem_u32(&hdr->acc_empty[b]), PAIR ? 2 * kEpiWarps : kEpiWarps);       // (a pair's: the leader's copy is used)
       mbar_init(smem_u32(&hdr->ids_full[b]), kIndexWarps * 32);
       mbar_init(smem_u32(&hdr->ids_empty[b]), kProdWarps);
     }
@@ -159,12 +174,19 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
       p.status.report(EGS_STATUS_INTERNAL);
     }
   }
+  if (PAIR) __syncthreads();
   if (warp == kMmaWarp) {
-    tmem_alloc(smem_u32(&hdr->tmem_base), tmem_cols);
-    tmem_relinquish();
+    if (PAIR) {
+      tmem_alloc2(smem_u32(&hdr->tmem_base), tmem_cols);
+      tmem_relinquish2();
+    } else {
+      tmem_alloc(smem_u32(&hdr->tmem_base), tmem_cols);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();          // both CTAs' barriers are initialised before anything crosses the pair
   tc_fence_after();
   const uint32_t tmem_base = hdr->tmem_base;
   pdl_trigger();
@@ -183,16 +205,16 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
       if constexpr (OP != kOpDweight) {
         long long ahead_t[4];              // G: token ids of the next unit's rows, loaded a unit ahead
         auto fetch_ids = [&](int v) {
-          const Unit w = unit_of<OP>(p, v);
+          const Unit w = unit_of<OP, PAIR>(p, v);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int m = min(w.m0 + r0 + 32 * i, p.M - 1), b = m / p.K;
             ahead_t[i] = load_index(p.Ind, p.index_dtype, static_cast<long long>(b * p.E + w.e) * p.K + (m - b * p.K));
           }
         };
-        if (OP == kOpGather && static_cast<int>(blockIdx.x) < p.units) fetch_ids(blockIdx.x);
-        for (int un = blockIdx.x; un < p.units && alive; un += gridDim.x) {
-          const Unit u = unit_of<OP>(p, un);
+        if (OP == kOpGather && first < p.units) fetch_ids(first);
+        for (int un = first; un < p.units && alive; un += stride) {
+          const Unit u = unit_of<OP, PAIR>(p, un);
           const int steps = unit_steps<OP>(p, u);
           const char* src[4];
 #pragma unroll
@@ -203,7 +225,7 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
             else if (m < p.M && ahead_t[i] >= 0 && ahead_t[i] < p.T) row = b * p.T + static_cast<int>(ahead_t[i]);
             src[i] = row >= 0 ? Rows + static_cast<long long>(row) * pitch_c + cc * 16 : nullptr;
           }
-          if (OP == kOpGather && un + static_cast<int>(gridDim.x) < p.units) fetch_ids(un + gridDim.x);
+          if (OP == kOpGather && un + stride < p.units) fetch_ids(un + stride);
           for (int k = 0; k < steps; ++k) {
             if (round > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[slot]), (round - 1) & 1, abort_flag, p.status.word, lane);
             if (!alive) break;
@@ -233,7 +255,7 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
           constexpr int RG = SWAP ? RN : 4, RS = SWAP ? 4 : RN;                      // rows per thread: gathered, slot operand
           constexpr int TN = 4 * RN;                                                 // threads per row of the BN-wide operand
           const int m_c = tid & 15, m_r = tid >> 4, n_c = tid & (TN - 1), n_r = tid / TN;
-          const bool n_on = n_c * 8 < p.BN;
+          const bool n_on = n_c * 8 < p.half;
           const int g_c = SWAP ? n_c : m_c, g_r = SWAP ? n_r : m_r, s_c = SWAP ? m_c : n_c, s_r = SWAP ? m_r : n_r;
           const bool g_on = !SWAP || n_on, s_on = !TMA && (SWAP || n_on);
           constexpr uint32_t GSTEP = kStep / RG, SSTEP = kStep / RS;                 // rows from one of a thread's copies to the next
@@ -256,14 +278,15 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
             }
           };
           int batch = 0;                                                             // batches begun by this CTA
-          if (static_cast<int>(blockIdx.x) < p.units) {
+          if (first < p.units) {
             alive = mbar_wait_warp(smem_u32(&hdr->ids_full[0]), 0u, abort_flag, p.status.word, lane);
             read_ids(table);
           }
-          for (int un = blockIdx.x; un < p.units && alive; un += gridDim.x) {
-            const Unit u = unit_of<OP>(p, un);
+          for (int un = first; un < p.units && alive; un += stride) {
+            const Unit u = unit_of<OP, PAIR>(p, un);
             const int steps = unit_steps<OP>(p, u);
-            const int f0 = (SWAP ? u.n0 : u.m0) + g_c * 8, s0 = (SWAP ? u.m0 : u.n0) + s_c * 8;     // first feature of the chunk
+            const int nc0 = first_column<PAIR>(p, u);
+            const int f0 = (SWAP ? nc0 : u.m0) + g_c * 8, s0 = (SWAP ? u.m0 : nc0) + s_c * 8;       // first feature of the chunk
             const bool g_in = f0 < (SWAP ? p.N : p.C), s_in = s0 < (SWAP ? p.C : p.N);
             const char* g_col = Rows + (g_in ? static_cast<long long>(f0) * 2 : 0ll);
             const char* s_col = static_cast<const char*>(p.Slot) + (s_in ? static_cast<long long>(s0) * 2 : 0ll);
@@ -284,7 +307,7 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&hdr->ids_empty[batch & 1]));    // this warp has read the batch
                 ++batch;
-                if (!unit_end || un + static_cast<int>(gridDim.x) < p.units) {
+                if (!unit_end || un + stride < p.units) {
                   alive = mbar_wait_warp(smem_u32(&hdr->ids_full[batch & 1]), (batch >> 1) & 1, abort_flag, p.status.word, lane);
                   if (!alive) break;
                   read_ids(table + static_cast<uint32_t>(batch & 1) * (kBatch * 4u));
@@ -309,9 +332,9 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
           }
         };
         auto pick_rn = [&](auto swap_tag, auto tma_tag) {
-          if (p.BN > 128) run(std::integral_constant<int, 8>{}, swap_tag, tma_tag);
-          else if (p.BN > 64) run(std::integral_constant<int, 4>{}, swap_tag, tma_tag);
-          else if (p.BN > 32) run(std::integral_constant<int, 2>{}, swap_tag, tma_tag);
+          if (p.half > 128) run(std::integral_constant<int, 8>{}, swap_tag, tma_tag);
+          else if (p.half > 64) run(std::integral_constant<int, 4>{}, swap_tag, tma_tag);
+          else if (p.half > 32) run(std::integral_constant<int, 2>{}, swap_tag, tma_tag);
           else run(std::integral_constant<int, 1>{}, swap_tag, tma_tag);
         };
         if (p.swap) {
@@ -339,7 +362,7 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
     int next_slot = -1, next_b = 0, next_flag = 0;
     auto look_up = [&](int v) {
       if (OP == kOpDweight || v >= p.units) return;
-      const Unit w = unit_of<OP>(p, v);
+      const Unit w = unit_of<OP, PAIR>(p, v);
       const int m = w.m0 + lg * 32 + lane;
       next_slot = -1;
       next_flag = 0;
@@ -350,10 +373,10 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
         if (OP == kOpScatter) next_flag = p.plan[next_b];
       }
     };
-    look_up(blockIdx.x);
+    look_up(first);
     int t = 0;
-    for (int un = blockIdx.x; un < p.units && alive; un += gridDim.x, ++t) {
-      const Unit u = unit_of<OP>(p, un);
+    for (int un = first; un < p.units && alive; un += stride, ++t) {
+      const Unit u = unit_of<OP, PAIR>(p, un);
       const int bn = min(p.BN, p.N - u.n0);              // columns of this tile (a multiple of 8)
       const int n_end = u.n0 + bn;
       int my_ro = -1;                                    // G, S: destination row of tile row lg * 32 + lane
@@ -365,7 +388,7 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
           my_ro = OP == kOpGather ? next_slot : (ok ? next_b * p.T + static_cast<int>(next_t) : -1);
         }
         if (OP == kOpScatter) to_f32 = __ballot_sync(0xffffffffu, next_flag != 0);
-        look_up(un + gridDim.x);
+        look_up(un + stride);
       }
       const T* bias_row = (OP != kOpDweight && p.bias) ? static_cast<const T*>(p.bias) + static_cast<long long>(u.e) * p.N + u.n0 : nullptr;
       const bool bulk = OP == kOpScatter && p.bulk && to_f32 == 0u;
@@ -470,12 +493,15 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&hdr->acc_empty[buf]));
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(&hdr->acc_empty[buf]), 0));
+        else mbar_arrive(smem_u32(&hdr->acc_empty[buf]));
+      }
     }
     if (OP == kOpScatter) bulk_wait_all();               // shared memory must outlive the copy engine's reads
   } else if (warp == kMmaWarp) {
     // =========================== MMA issuer ===========================
-    if (lane == 0) {
+    if (lane == 0 && leader) {
       const bool a_mn = OP == kOpDweight, b_mn = OP == kOpDweight || !p.nc;
       const uint64_t a_desc = a_mn ? make_smem_desc(0u, kSeg, 1024u) : make_smem_desc(0u, 16u, 1024u);
       const uint64_t b_desc = b_mn ? make_smem_desc(0u, kSeg, 1024u) : make_smem_desc(0u, 16u, 1024u);
@@ -483,11 +509,11 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
       bool ok = true;
       int t = 0, slot = 0, round = 0;
       uint32_t addr = ring0 >> 4;                        // descriptors: 14 address bits in 16-byte units (shared memory is smaller)
-      for (int un = blockIdx.x; un < p.units && ok; un += gridDim.x, ++t) {
-        const Unit u = unit_of<OP>(p, un);
+      for (int un = first; un < p.units && ok; un += stride, ++t) {
+        const Unit u = unit_of<OP, PAIR>(p, un);
         const int steps = unit_steps<OP>(p, u);
-        const int bn = min(p.BN, ((p.N - u.n0) + 15) & ~15);
-        const uint32_t idesc = make_idesc(Elem<T>::fmt, a_mn ? 1u : 0u, b_mn ? 1u : 0u, kTileM, static_cast<uint32_t>(bn));
+        const uint32_t idesc =
+            make_idesc(Elem<T>::fmt, a_mn ? 1u : 0u, b_mn ? 1u : 0u, PAIR ? 2 * kTileM : kTileM, static_cast<uint32_t>(mma_width<PAIR>(p, u)));
         const int buf = t & 1;
         if (t >= 2) {
           ok = mbar_wait(smem_u32(&hdr->acc_empty[buf]), ((t >> 1) - 1) & 1, abort_flag, p.status.word);
@@ -497,10 +523,16 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
         const uint32_t d = tmem_base + static_cast<uint32_t>(buf) * acc_cols;
         for (int ks = 0; ks < steps; ++ks) {
           ok = mbar_wait(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status.word);
+          if (PAIR && ok) ok = mbar_wait(smem_u32(&hdr->peer_full[slot]), round & 1, abort_flag, p.status.word);
           if (!ok) break;
           tc_fence_after();
-          umma_ss_f16_x4(d, a_desc + addr, b_desc + addr + (kMTile >> 4), a_adv, b_adv, idesc, ks > 0 ? 1u : 0u);
-          umma_commit(smem_u32(&hdr->empty[slot]));
+          if (PAIR) {
+            umma2_ss_f16_x4(d, a_desc + addr, b_desc + addr + (kMTile >> 4), a_adv, b_adv, idesc, ks > 0 ? 1u : 0u);
+            umma2_commit_both(smem_u32(&hdr->empty[slot]));
+          } else {
+            umma_ss_f16_x4(d, a_desc + addr, b_desc + addr + (kMTile >> 4), a_adv, b_adv, idesc, ks > 0 ? 1u : 0u);
+            umma_commit(smem_u32(&hdr->empty[slot]));
+          }
           addr += stage_bytes >> 4;
           if (++slot == stages) {
             slot = 0;
@@ -508,7 +540,27 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
             addr = ring0 >> 4;
           }
         }
-        if (ok) umma_commit(smem_u32(&hdr->acc_full[buf]));
+        if (ok) {
+          if (PAIR) {
+            umma2_commit_both(smem_u32(&hdr->acc_full[buf]));
+          } else {
+            umma_commit(smem_u32(&hdr->acc_full[buf]));
+          }
+        }
+      }
+    } else if (PAIR && lane == 0) {
+      // the peer tells the leader of every stage that has landed here
+      const uint32_t to_leader = map_to_cta(smem_u32(&hdr->peer_full[0]), 0);
+      bool ok = true;
+      int slot = 0, round = 0;
+      for (int un = first; un < p.units && ok; un += stride) {
+        const int steps = unit_steps<OP>(p, unit_of<OP, PAIR>(p, un));
+        for (int ks = 0; ks < steps; ++ks) {
+          ok = mbar_wait(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status.word);
+          if (!ok) break;
+          mbar_arrive_cluster_relaxed(to_leader + slot * 8u);
+          if (++slot == stages) { slot = 0; ++round; }
+        }
       }
     }
     __syncwarp();
@@ -519,8 +571,8 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
     constexpr int kPer = kBatch / (kIndexWarps * 32);
     bool alive = true;
     int batch = 0;
-    for (int un = blockIdx.x; un < p.units && alive; un += gridDim.x) {
-      const Unit u = unit_of<OP>(p, un);
+    for (int un = first; un < p.units && alive; un += stride) {
+      const Unit u = unit_of<OP, PAIR>(p, un);
       const int m_begin = u.split * p.rows_per_split, m_end = min(p.M, m_begin + p.rows_per_split);
       const bool report = u.m0 == 0 && u.n0 == 0;
       for (int m0 = m_begin; m0 < m_end && alive; m0 += kBatch, ++batch) {
@@ -559,9 +611,10 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
       bool ok = true;
       int slot = 0, round = 0;
       uint32_t base = ring0;
-      for (int un = blockIdx.x; un < p.units && ok; un += gridDim.x) {
-        const Unit u = unit_of<OP>(p, un);
+      for (int un = first; un < p.units && ok; un += stride) {
+        const Unit u = unit_of<OP, PAIR>(p, un);
         const int steps = unit_steps<OP>(p, u);
+        const int n0 = first_column<PAIR>(p, u);
         int m = OP == kOpDweight ? u.split * p.rows_per_split : u.m0;
         int b = m / p.K, k = m - b * p.K;                // first slot row of the step
         for (int ks = 0, c0 = 0; ks < steps; ++ks, c0 += kStep) {
@@ -574,12 +627,12 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
           if (OP != kOpDweight) {
             if (OP == kOpScatter && p.tma_rows) tma_load_4d(base, &map_rows, c0, k, u.e, b, bar);
             if (p.nc) {
-              tma_load_3d(base + kMTile, &map_w, c0, u.n0, u.e, bar);
+              tma_load_3d(base + kMTile, &map_w, c0, n0, u.e, bar);
             } else {
-              for (int s = 0; s < nseg; ++s) tma_load_3d(base + kMTile + s * kSeg, &map_w, u.n0 + s * 64, c0, u.e, bar);
+              for (int s = 0; s < nseg; ++s) tma_load_3d(base + kMTile + s * kSeg, &map_w, n0 + s * 64, c0, u.e, bar);
             }
           } else {
-            const int ns = p.swap ? 2 : nseg, x0 = p.swap ? u.m0 : u.n0;
+            const int ns = p.swap ? 2 : nseg, x0 = p.swap ? u.m0 : n0;
             const uint32_t dst = base + (p.swap ? 0u : kMTile);
             for (int s = 0; s < ns; ++s) tma_load_4d(dst + s * kSeg, &map_rows, x0 + s * 64, k, u.e, b, bar);
             k += kStep;                                  // 64 rows are parts of one batch element or whole ones
@@ -600,7 +653,27 @@ __global__ void __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __g
   // ---- common exit ----
   tc_fence_before();
   __syncthreads();
-  if (warp == kMmaWarp) tmem_release(tmem_base, tmem_cols, smem_u32(&hdr->drain), abort_flag, p.status, lane);
+  if (!PAIR) {
+    if (warp == kMmaWarp) tmem_release(tmem_base, tmem_cols, smem_u32(&hdr->drain), abort_flag, p.status, lane);
+  } else {
+    // nobody leaves while the partner may still read its shared memory, write its tensor memory or signal its barriers; after an
+    // abort MMAs of the pair may still be in flight, and the leader waits for them (bounded) before the pair meets
+    uint32_t safe = 1u;
+    if (warp == kMmaWarp && *abort_flag) {
+      if (lane == 0) {
+        uint32_t ignore_abort = 0u;
+        p.status.tell_host();
+        umma2_commit(smem_u32(&hdr->drain));
+        safe = mbar_wait(smem_u32(&hdr->drain), 0u, &ignore_abort, nullptr) ? 1u : 0u;
+      }
+      safe = __shfl_sync(0xffffffffu, safe, 0);
+    }
+    cluster_sync_all();
+    if (warp == kMmaWarp && safe) {
+      tc_fence_after();
+      tmem_dealloc2(tmem_base, tmem_cols);
+    }
+  }
 }
 
 // Slot rows can come as one TMA box per 64-element column segment when `rows` consecutive expert rows starting at a multiple of
@@ -614,56 +687,76 @@ bool encode_slot_rows(TensorMap3* map, const void* base, int B, int E, int K, in
   return encode_tensor_map_16bit(map, base, 4, dims, box);
 }
 
-// Tile width over n columns.  Per step the shared memory moves 2 * (128 + BN) * 128 bytes at 128 bytes per clock; the load/store
-// unit needs lsu0 + lsu1 * BN clocks for its share of the copies; read-out takes epi clocks per column beside the next tile's
-// main loop; units go out in waves of one per SM.
-int pick_bn(int n, long long unit_rows, int steps, double lsu0, double lsu1, double epi) {
-  int best = 256;
-  double best_cost = 1e30;
-  const int top = n < 256 ? (n + 15) / 16 * 16 : 256;
-  for (int bn = top; bn >= 16; bn -= 16) {
-    const long long tiles = (n + bn - 1) / bn;
-    const long long units = unit_rows * tiles, waves = (units + kSms - 1) / kSms;
-    double step = 2.0 * (128 + bn);
-    const double lsu = lsu0 + lsu1 * bn;
-    if (lsu > step) step = lsu;
-    double unit = steps * step;
-    if (epi * bn > unit) unit = epi * bn;
-    const double cost = waves * (unit + 1000) + epi * bn;
-    if (cost < best_cost * 0.98) {
-      best = bn;
-      best_cost = cost;
+// One CTA per tile of 128 x BN or a pair of CTAs per tile of 256 x BN, and BN.  Per step a CTA's shared memory moves
+// 2 * (128 + columns it stages) * 128 bytes at 128 bytes per clock and the tensor core multiplies BN columns in 2 * BN clocks; the
+// load/store unit needs lsu0 + lsu1 * (columns staged) clocks for its share of the copies; read-out takes epi clocks per column
+// (counted in blocks of `block` columns) beside the next tile's main loop; units go out in waves of one per SM or pair of SMs.
+struct Tile {
+  int bn = 256;
+  bool pair = false;
+  double cost = 1e30;
+};
+Tile pick_tile(int n, int m, long long groups, int steps, double lsu0, double lsu1, double epi, int block, bool may_pair) {
+  Tile best;
+  for (int pair = 0; pair <= (may_pair ? 1 : 0); ++pair) {
+    const int rows = pair ? 2 * kTileM : kTileM, sms = pair ? kSms / 2 : kSms, unit16 = pair ? 32 : 16;
+    const long long row_units = (m + rows - 1) / rows * groups;
+    const int top = n < 256 ? (n + unit16 - 1) / unit16 * unit16 : 256;
+    for (int bn = top; bn >= unit16; bn -= unit16) {
+      const long long tiles = (n + bn - 1) / bn;
+      const long long units = row_units * tiles, waves = (units + sms - 1) / sms;
+      const int staged = pair ? bn / 2 : bn;
+      double step = 2.0 * (128 + staged);
+      if (2.0 * bn > step) step = 2.0 * bn;
+      if (lsu0 + lsu1 * staged > step) step = lsu0 + lsu1 * staged;
+      double unit = steps * step;
+      const double out = epi * ((bn + block - 1) / block * block);
+      if (out > unit) unit = out;
+      const double cost = waves * (unit + 1000) + out;
+      if (cost < best.cost * (pair && !best.pair ? 0.95 : 0.98)) {
+        best.bn = bn;
+        best.pair = pair != 0;
+        best.cost = cost;
+      }
     }
   }
   return best;
 }
 
-int ring_stages(int BN, bool nc_tile, uint32_t epi_bytes) {
-  const size_t n_bytes = nc_tile ? static_cast<size_t>(BN) * 128 : static_cast<size_t>((BN + 63) / 64) * kSeg;
-  const size_t s = (kSmemMax - kDenseHeader - epi_bytes) / (kMTile + n_bytes);      // epi_bytes: all that is not ring
+int ring_stages(int half, bool nc_tile, uint32_t not_ring) {
+  const size_t n_bytes = nc_tile ? static_cast<size_t>(half) * 128 : static_cast<size_t>((half + 63) / 64) * kSeg;
+  const size_t s = (kSmemMax - kDenseHeader - not_ring) / (kMTile + n_bytes);
   return static_cast<int>(s > kMaxStages ? kMaxStages : s);
 }
 
-template <typename T, int OP>
+template <typename T, int OP, bool PAIR>
 cudaError_t launch(const DenseParams& p, const TensorMap3& mw, const TensorMap3& mr, bool after_own, cudaStream_t st) {
-  const size_t n_bytes = (OP != kOpDweight && p.nc) ? static_cast<size_t>(p.BN) * 128 : static_cast<size_t>((p.BN + 63) / 64) * kSeg;
-  const size_t smem = kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : 0u) + ((OP == kOpScatter && p.bulk) ? kEpiBulk : kEpiPlain) + p.stages * (kMTile + n_bytes);
-  cudaError_t err = ensure_smem_optin<dense16_kernel<T, OP>>(static_cast<int>(kSmemMax));
+  const size_t n_bytes = (OP != kOpDweight && p.nc) ? static_cast<size_t>(p.half) * 128 : static_cast<size_t>((p.half + 63) / 64) * kSeg;
+  const size_t smem = kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : 0u) + ((OP == kOpScatter && p.bulk) ? kEpiBulk : kEpiPlain) +
+                      p.stages * (kMTile + n_bytes);
+  cudaError_t err = ensure_smem_optin<dense16_kernel<T, OP, PAIR>>(static_cast<int>(kSmemMax));
   if (err != cudaSuccess) return err;
-  err = launch_kernel(dense16_kernel<T, OP>, p.units < kSms ? p.units : kSms, kDenseThreads<OP>, smem, st, after_own, p, mw, mr);
+  const int grid = PAIR ? 2 * (p.units < kSms / 2 ? p.units : kSms / 2) : (p.units < kSms ? p.units : kSms);
+  err = launch_kernel(dense16_kernel<T, OP, PAIR>, grid, kDenseThreads<OP>, smem, st, after_own, p, mw, mr);
   count_launch();
   return err;
+}
+template <int OP, bool PAIR>
+cudaError_t launch_typed(const DenseParams& p, int dtype, const TensorMap3& mw, const TensorMap3& mr, bool after_own, cudaStream_t st) {
+  return dtype == EGS_F16 ? launch<__half, OP, PAIR>(p, mw, mr, after_own, st) : launch<__nv_bfloat16, OP, PAIR>(p, mw, mr, after_own, st);
 }
 
 }  // namespace
 
 void configure_dense16_rowgemm(RowGemmParams& p, bool scatter) {
-  const long long row_blocks = static_cast<long long>((p.M + kTileM - 1) / kTileM) * p.E;
   const int steps = (p.C + kStep - 1) / kStep;
   const bool cp_rows = !scatter || !rows_fit_boxes(p.K, 128);
-  p.BN = pick_bn(p.N, row_blocks, steps, cp_rows ? 340.0 : 0.0, 0.0, scatter ? 28.0 : 16.0);
+  // (a scatter is bound by its additions: no pairs; bulk reductions go out in blocks of 64 columns)
+  const Tile t = pick_tile(p.N, p.M, p.E, steps, cp_rows ? 340.0 : 0.0, 0.0, scatter ? 28.0 : 16.0, scatter ? 64 : 1, !scatter);
+  p.BN = t.bn;
+  p.pair = t.pair ? 1 : 0;
   p.bulk_epilogue = scatter ? 1 : 0;
-  p.stages = ring_stages(p.BN, p.w_layout == EGS_W_NC, scatter ? kEpiBulk : kEpiPlain);
+  p.stages = ring_stages(p.pair ? p.BN / 2 : p.BN, p.w_layout == EGS_W_NC, scatter ? kEpiBulk : kEpiPlain);
   p.row_tiles = 2;        // two 128-row accumulators per CTA
   p.persistent = (scatter && steps <= 4) ? 1 : 0;        // (for egs_describe_plan) the additions outlast the contraction
 }
@@ -675,7 +768,9 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
   p.nc = r.w_layout == EGS_W_NC;
   p.index_dtype = r.index_dtype;
   p.BN = r.BN; p.stages = r.stages;
-  p.tiles_m = (r.M + kTileM - 1) / kTileM;
+  p.half = r.pair ? r.BN / 2 : r.BN;
+  const int rows = r.pair ? 2 * kTileM : kTileM;
+  p.tiles_m = (r.M + rows - 1) / rows;
   p.tiles_n = (r.N + r.BN - 1) / r.BN;
   p.order = r.expert_fastest;
   p.bulk = r.bulk_epilogue;
@@ -685,16 +780,15 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
   TensorMap3 mw{}, mr{};
   const unsigned long long inner = p.nc ? r.C : r.N, outer = p.nc ? r.N : r.C;
   const unsigned long long dims[3] = {inner, outer, static_cast<unsigned long long>(r.E)};
-  const unsigned box[3] = {64u, p.nc ? static_cast<unsigned>(r.BN) : static_cast<unsigned>(kStep), 1u};
+  const unsigned box[3] = {64u, p.nc ? static_cast<unsigned>(p.half) : static_cast<unsigned>(kStep), 1u};
   if (!encode_tensor_map_16bit(&mw, r.W, 3, dims, box)) return cudaErrorInvalidValue;
   p.tma_rows = scatter && rows_fit_boxes(r.K, 128) && encode_slot_rows(&mr, r.A, r.B, r.E, r.K, r.C, 128);
-  const bool half = dtype == EGS_F16;
-  if (scatter) return half ? launch<__half, kOpScatter>(p, mw, mr, r.after_own != 0, st) : launch<__nv_bfloat16, kOpScatter>(p, mw, mr, r.after_own != 0, st);
-  return half ? launch<__half, kOpGather>(p, mw, mr, false, st) : launch<__nv_bfloat16, kOpGather>(p, mw, mr, false, st);
+  if (scatter) return launch_typed<kOpScatter, false>(p, dtype, mw, mr, r.after_own != 0, st);
+  return r.pair ? launch_typed<kOpGather, true>(p, dtype, mw, mr, false, st) : launch_typed<kOpGather, false>(p, dtype, mw, mr, false, st);
 }
 
-// D: which operand's features are the accumulator's rows, the tile width, and the row ranges.
-static void plan_dweight(const DWeightParams& p, bool& swap, int& bn, int& splits, int& rows) {
+// D: which operand's features are the accumulator's rows, the tile, and the row ranges.
+void configure_dense16_dweight(DWeightParams& p) {
   const bool slot_cp = !rows_fit_boxes(p.K, kStep);
   double best = 1e30;
   const long long steps_all = (p.M + kStep - 1) / kStep;
@@ -703,39 +797,27 @@ static void plan_dweight(const DWeightParams& p, bool& swap, int& bn, int& split
   for (int o = 0; o < 2; ++o) {
     const bool sw = o == 0 ? pref : !pref;
     const int mf = sw ? p.FD : p.FG, nf = sw ? p.FG : p.FD;
-    const long long tm = (mf + kTileM - 1) / kTileM;
     // load/store clocks per step: 10 per 512 bytes; the gathered operand always, the slot operand where it has no boxes
     const double lsu0 = (!sw ? 320.0 : 0.0) + (sw && slot_cp ? 320.0 : 0.0), lsu1 = (sw ? 2.5 : 0.0) + (!sw && slot_cp ? 2.5 : 0.0);
-    const double epi = o == 0 ? 16.0 : 24.0;
     for (int s = 1; s <= 64 && s <= steps_all; s = s < 4 ? s + 1 : s + s / 2) {
       const long long sp_steps = (steps_all + s - 1) / s;
       const long long real = (steps_all + sp_steps - 1) / sp_steps;      // ranges of whole steps
-      const double e = real > 1 ? 32.0 : epi;                            // partial tiles are added atomically
-      const int w = pick_bn(nf, tm * p.E * real, static_cast<int>(sp_steps), lsu0, lsu1, e);
-      const long long units = tm * p.E * real * ((nf + w - 1) / w), waves = (units + kSms - 1) / kSms;
-      double step = 2.0 * (128 + w);
-      if (lsu0 + lsu1 * w > step) step = lsu0 + lsu1 * w;
-      double unit = sp_steps * step;
-      if (e * w > unit) unit = e * w;
+      const double epi = real > 1 ? 32.0 : o == 0 ? 16.0 : 20.0;         // (partial tiles are added atomically)
+      const Tile t = pick_tile(nf, mf, p.E * real, static_cast<int>(sp_steps), lsu0, lsu1, epi, 1, true);
+      double cost = t.cost;
       // more than one range: zero fill and rounding of the float32 sums, two launches and 10 bytes an element
-      double cost = waves * (unit + 1000) + e * w;
       if (real > 1) cost += 9000 + static_cast<double>(p.E) * p.FG * p.FD * 10 / (148 * 20.0);
       if (cost < best * (o == 0 ? 1.0 : 0.97)) {
         best = cost;
-        swap = sw;
-        bn = w;
-        splits = static_cast<int>(real);
-        rows = static_cast<int>(sp_steps * kStep);
+        p.swap = sw ? 1 : 0;
+        p.BN = t.bn;
+        p.pair = t.pair ? 1 : 0;
+        p.splits = static_cast<int>(real);
+        p.rows_per_split = static_cast<int>(sp_steps * kStep);
       }
     }
   }
-}
-
-void configure_dense16_dweight(DWeightParams& p) {
-  bool swap = false;
-  plan_dweight(p, swap, p.BN, p.splits, p.rows_per_split);
-  p.swap = swap ? 1 : 0;
-  p.stages = ring_stages(p.BN, false, table_bytes(!rows_fit_boxes(p.K, kStep)) + kEpiPlain);
+  p.stages = ring_stages(p.pair ? p.BN / 2 : p.BN, false, table_bytes(slot_cp) + kEpiPlain);
   p.row_tiles = 2;        // two 128-row accumulators per CTA
 }
 
@@ -749,15 +831,17 @@ cudaError_t launch_dense16_dweight(const DWeightParams& r, int dtype, cudaStream
   p.lane_rows = (r.out_layout == EGS_DW_DIRECT_ROWS) == (r.swap != 0);
   p.index_dtype = r.index_dtype;
   p.BN = r.BN; p.stages = r.stages; p.splits = r.splits; p.rows_per_split = r.rows_per_split;
-  p.tiles_m = (p.C + kTileM - 1) / kTileM;
+  p.half = r.pair ? r.BN / 2 : r.BN;
+  const int rows = r.pair ? 2 * kTileM : kTileM;
+  p.tiles_m = (p.C + rows - 1) / rows;
   p.tiles_n = (p.N + r.BN - 1) / r.BN;
   const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.E * p.splits;
   if (units > 2147483647ll - kSms) return cudaErrorInvalidValue;
   p.units = static_cast<int>(units);
   TensorMap3 mw{}, mr{};
   p.tma_rows = rows_fit_boxes(r.K, kStep) && encode_slot_rows(&mr, r.Ysrc, r.B, r.E, r.K, r.FD, kStep);
-  return dtype == EGS_F16 ? launch<__half, kOpDweight>(p, mw, mr, r.after_own != 0, st)
-                          : launch<__nv_bfloat16, kOpDweight>(p, mw, mr, r.after_own != 0, st);
+  return r.pair ? launch_typed<kOpDweight, true>(p, dtype, mw, mr, r.after_own != 0, st)
+                : launch_typed<kOpDweight, false>(p, dtype, mw, mr, r.after_own != 0, st);
 }
 
 }  // namespace egs

@@ -61,59 +61,12 @@ struct __align__(16) G2Header {
 };
 static_assert(sizeof(G2Header) <= kG2HeaderBytes, "header does not fit");
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// shared::cluster address of `local_addr` (an address in this CTA's shared memory) in the CTA of rank `rank`
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void tmem_alloc2(uint32_t smem_dst, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish2() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
 // one 32-byte store (a whole sector); the address must be 32-byte aligned
 __device__ __forceinline__ void store_32bytes(void* dst, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t a4, uint32_t a5,
                                               uint32_t a6, uint32_t a7) {
   asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(a4), "r"(a5),
                "r"(a6), "r"(a7)
                : "memory");
-}
-// commit of the pair's MMAs issued so far to ONE barrier, which may live in either CTA (shared::cluster address)
-__device__ __forceinline__ void umma2_commit(uint32_t cluster_bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar) : "memory");
-}
-// four contraction steps of the pair's MMA (M = 256: 128 rows of each CTA; B = N/2 columns from each CTA)
-__device__ __forceinline__ void umma2_ss_f16_x4(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t a_adv, uint32_t b_adv,
-                                                uint32_t idesc, uint32_t accumulate_first) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 aa, bb, a, b;\n\t"
-      "setp.ne.b32 p, %6, 0;\n\tsetp.eq.b32 q, 0, 0;\n\t"
-      "cvt.u64.u32 aa, %3;\n\tcvt.u64.u32 bb, %4;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %5, p;\n\t"
-      "add.u64 a, %1, aa;\n\tadd.u64 b, %2, bb;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %5, q;\n\t"
-      "add.u64 a, a, aa;\n\tadd.u64 b, b, bb;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %5, q;\n\t"
-      "add.u64 a, a, aa;\n\tadd.u64 b, b, bb;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %5, q;\n\t}" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(a_adv), "r"(b_adv), "r"(idesc), "r"(accumulate_first)
-      : "memory");
 }
 __device__ __forceinline__ void umma2_ss_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(

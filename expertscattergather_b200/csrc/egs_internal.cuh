@@ -79,6 +79,7 @@ struct RowGemmParams {
   int expert_fastest; // tensor path: grid order (1: experts vary fastest, row tiles slowest)
   int row_tiles;      // tensor path: 128-row accumulator tiles per CTA (1 or 2)
   int persistent;     // tensor path: 1 = persistent warp-specialised variant
+  int pair;           // 16-bit G: tiles of 256 rows on pairs of SMs
   int after_own;      // launched behind a kernel of the same call (fill, preparation): see launch_kernel
   int bulk_epilogue;  // persistent scatter: rows staged in shared memory and added with bulk asynchronous reductions
 };
@@ -101,6 +102,7 @@ struct DWeightParams {
   int row_tiles;      // tensor path: 128-feature accumulator tiles per CTA over FG (1 or 2)
   int after_own;      // launched behind the fill of `acc`: see launch_kernel
   int swap;           // 16-bit: the slot rows' features run along the accumulator's rows
+  int pair;           // 16-bit: tiles of 256 rows on pairs of SMs
 };
 
 // Fused pair G -> S (tensor path only):  Mid = gather(Src) x W1[e] is stored as slot rows AND fed, without leaving the
