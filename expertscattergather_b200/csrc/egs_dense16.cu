@@ -501,10 +501,10 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     if (OP == kOpScatter) bulk_wait_all();               // shared memory must outlive the copy engine's reads
   } else if (warp == kMmaWarp) {
     // =========================== MMA issuer ===========================
-    if (lane == 0 && leader) {
+    if (leader) {
       const bool a_mn = OP == kOpDweight, b_mn = OP == kOpDweight || !p.nc;
       const uint64_t a_desc = a_mn ? make_smem_desc(0u, kSeg, 1024u) : make_smem_desc(0u, 16u, 1024u);
-      const uint64_t b_desc = b_mn ? make_smem_desc(0u, kSeg, 1024u) : make_smem_desc(0u, 16u, 1024u);
+      const uint64_t b_desc = (b_mn ? make_smem_desc(0u, kSeg, 1024u) : make_smem_desc(0u, 16u, 1024u)) + (kMTile >> 4);
       const uint32_t a_adv = (a_mn ? 16u * 128u : 32u) >> 4, b_adv = (b_mn ? 16u * 128u : 32u) >> 4;
       bool ok = true;
       int t = 0, slot = 0, round = 0;
@@ -516,22 +516,19 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
             make_idesc(Elem<T>::fmt, a_mn ? 1u : 0u, b_mn ? 1u : 0u, PAIR ? 2 * kTileM : kTileM, static_cast<uint32_t>(mma_width<PAIR>(p, u)));
         const int buf = t & 1;
         if (t >= 2) {
-          ok = mbar_wait(smem_u32(&hdr->acc_empty[buf]), ((t >> 1) - 1) & 1, abort_flag, p.status.word);
+          ok = mbar_wait_all(smem_u32(&hdr->acc_empty[buf]), ((t >> 1) - 1) & 1, abort_flag, p.status.word);
           if (!ok) break;
-          tc_fence_after();
         }
         const uint32_t d = tmem_base + static_cast<uint32_t>(buf) * acc_cols;
         for (int ks = 0; ks < steps; ++ks) {
-          ok = mbar_wait(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status.word);
-          if (PAIR && ok) ok = mbar_wait(smem_u32(&hdr->peer_full[slot]), round & 1, abort_flag, p.status.word);
+          ok = mbar_wait_all(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status.word);
+          if (PAIR && ok) ok = mbar_wait_all(smem_u32(&hdr->peer_full[slot]), round & 1, abort_flag, p.status.word);
           if (!ok) break;
           tc_fence_after();
-          if (PAIR) {
-            umma2_ss_f16_x4(d, a_desc + addr, b_desc + addr + (kMTile >> 4), a_adv, b_adv, idesc, ks > 0 ? 1u : 0u);
-            umma2_commit_both(smem_u32(&hdr->empty[slot]));
-          } else {
-            umma_ss_f16_x4(d, a_desc + addr, b_desc + addr + (kMTile >> 4), a_adv, b_adv, idesc, ks > 0 ? 1u : 0u);
-            umma_commit(smem_u32(&hdr->empty[slot]));
+          if (elect_one()) {
+            umma_f16_x4<PAIR>(d, a_desc + addr, b_desc + addr, a_adv, b_adv, idesc, ks > 0 ? 1u : 0u);
+            umma_done<PAIR>(smem_u32(&hdr->empty[slot]));
+            if (ks + 1 == steps) umma_done<PAIR>(smem_u32(&hdr->acc_full[buf]));
           }
           addr += stage_bytes >> 4;
           if (++slot == stages) {
@@ -540,15 +537,8 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
             addr = ring0 >> 4;
           }
         }
-        if (ok) {
-          if (PAIR) {
-            umma2_commit_both(smem_u32(&hdr->acc_full[buf]));
-          } else {
-            umma_commit(smem_u32(&hdr->acc_full[buf]));
-          }
-        }
       }
-    } else if (PAIR && lane == 0) {
+    } else if (PAIR) {
       // the peer tells the leader of every stage that has landed here
       const uint32_t to_leader = map_to_cta(smem_u32(&hdr->peer_full[0]), 0);
       bool ok = true;
@@ -556,9 +546,9 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       for (int un = first; un < p.units && ok; un += stride) {
         const int steps = unit_steps<OP>(p, unit_of<OP, PAIR>(p, un));
         for (int ks = 0; ks < steps; ++ks) {
-          ok = mbar_wait(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status.word);
+          ok = mbar_wait_all(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status.word);
           if (!ok) break;
-          mbar_arrive_cluster_relaxed(to_leader + slot * 8u);
+          if (elect_one()) mbar_arrive_cluster_relaxed(to_leader + slot * 8u);
           if (++slot == stages) { slot = 0; ++round; }
         }
       }
@@ -606,44 +596,50 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     }
   } else if (has_tma) {
     // =========================== TMA issuer ===========================
-    if (lane == 0) {
-      const uint32_t bytes = (OP != kOpDweight ? n_bytes : (p.swap ? kMTile : n_bytes)) + ((OP == kOpScatter && p.tma_rows) ? kMTile : 0u);
-      bool ok = true;
-      int slot = 0, round = 0;
-      uint32_t base = ring0;
-      for (int un = first; un < p.units && ok; un += stride) {
-        const Unit u = unit_of<OP, PAIR>(p, un);
-        const int steps = unit_steps<OP>(p, u);
-        const int n0 = first_column<PAIR>(p, u);
-        int m = OP == kOpDweight ? u.split * p.rows_per_split : u.m0;
-        int b = m / p.K, k = m - b * p.K;                // first slot row of the step
-        for (int ks = 0, c0 = 0; ks < steps; ++ks, c0 += kStep) {
-          if (round > 0) {
-            ok = mbar_wait(smem_u32(&hdr->empty[slot]), (round - 1) & 1, abort_flag, p.status.word);
-            if (!ok) break;
-          }
-          const uint32_t bar = smem_u32(&hdr->full[slot]);
+    const uint32_t bytes = (OP != kOpDweight ? n_bytes : (p.swap ? kMTile : n_bytes)) + ((OP == kOpScatter && p.tma_rows) ? kMTile : 0u);
+    bool ok = true;
+    int slot = 0, round = 0;
+    uint32_t base = ring0;
+    for (int un = first; un < p.units && ok; un += stride) {
+      const Unit u = unit_of<OP, PAIR>(p, un);
+      const int steps = unit_steps<OP>(p, u);
+      const int n0 = first_column<PAIR>(p, u);
+      int m = OP == kOpDweight ? u.split * p.rows_per_split : u.m0;
+      int b = m / p.K, k = m - b * p.K;                // first slot row of the step
+      for (int ks = 0, c0 = 0; ks < steps; ++ks, c0 += kStep) {
+        if (round > 0) {
+          ok = mbar_wait_all(smem_u32(&hdr->empty[slot]), (round - 1) & 1, abort_flag, p.status.word);
+          if (!ok) break;
+        }
+        const uint32_t bar = smem_u32(&hdr->full[slot]);
+        if (elect_one()) {
           mbar_arrive_expect_tx(bar, bytes);
           if (OP != kOpDweight) {
             if (OP == kOpScatter && p.tma_rows) tma_load_4d(base, &map_rows, c0, k, u.e, b, bar);
             if (p.nc) {
               tma_load_3d(base + kMTile, &map_w, c0, n0, u.e, bar);
             } else {
-              for (int s = 0; s < nseg; ++s) tma_load_3d(base + kMTile + s * kSeg, &map_w, n0 + s * 64, c0, u.e, bar);
+#pragma unroll
+              for (int s = 0; s < 4; ++s)
+                if (s < nseg) tma_load_3d(base + kMTile + s * kSeg, &map_w, n0 + s * 64, c0, u.e, bar);
             }
           } else {
             const int ns = p.swap ? 2 : nseg, x0 = p.swap ? u.m0 : n0;
             const uint32_t dst = base + (p.swap ? 0u : kMTile);
-            for (int s = 0; s < ns; ++s) tma_load_4d(dst + s * kSeg, &map_rows, x0 + s * 64, k, u.e, b, bar);
-            k += kStep;                                  // 64 rows are parts of one batch element or whole ones
-            while (k >= p.K) { k -= p.K; ++b; }
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+              if (s < ns) tma_load_4d(dst + s * kSeg, &map_rows, x0 + s * 64, k, u.e, b, bar);
           }
-          base += stage_bytes;
-          if (++slot == stages) {
-            slot = 0;
-            ++round;
-            base = ring0;
-          }
+        }
+        if (OP == kOpDweight) {
+          k += kStep;                                  // 64 rows are parts of one batch element or whole ones
+          while (k >= p.K) { k -= p.K; ++b; }
+        }
+        base += stage_bytes;
+        if (++slot == stages) {
+          slot = 0;
+          ++round;
+          base = ring0;
         }
       }
     }

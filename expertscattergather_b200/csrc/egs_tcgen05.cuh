@@ -133,6 +133,20 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
   return __shfl_sync(0xffffffffu, ok, 0) != 0u;
 }
 
+// The warps that issue MMAs and box loads run converged: every lane polls and the vote makes the outcome warp-uniform, and the
+// elected lane (the same one each time for a full mask) issues.  Descriptors, coordinates and barrier addresses then live in
+// uniform registers.  The same loops inside `if (lane == 0)` spent 700 clocks a step on four MMAs and a commit, more than the
+// tensor core needs for a 128 x 256 x 64 step (512).
+__device__ __forceinline__ bool mbar_wait_all(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, int32_t* status) {
+  if (__all_sync(0xffffffffu, mbar_try(bar, parity) != 0u)) return true;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status)) != 0;
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t on;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(on)::"memory");
+  return on != 0u;
+}
+
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
 }
@@ -277,6 +291,18 @@ __device__ __forceinline__ void umma2_ss_f16_x4(uint32_t tmem_d, uint64_t adesc,
       "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %5, q;\n\t}" ::"r"(tmem_d),
       "l"(adesc), "l"(bdesc), "r"(a_adv), "r"(b_adv), "r"(idesc), "r"(accumulate_first)
       : "memory");
+}
+// The same four steps, and the commit, for one CTA or a pair.
+template <bool PAIR>
+__device__ __forceinline__ void umma_f16_x4(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t a_adv, uint32_t b_adv,
+                                            uint32_t idesc, uint32_t accumulate_first) {
+  if (PAIR) umma2_ss_f16_x4(tmem_d, adesc, bdesc, a_adv, b_adv, idesc, accumulate_first);
+  else umma_ss_f16_x4(tmem_d, adesc, bdesc, a_adv, b_adv, idesc, accumulate_first);
+}
+template <bool PAIR>
+__device__ __forceinline__ void umma_done(uint32_t bar) {
+  if (PAIR) umma2_commit_both(bar);
+  else umma_commit(bar);
 }
 // Writes 16 consecutive 32-bit columns of this thread's TMEM lane.
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
