@@ -1,7 +1,7 @@
 // Operators G, S and D for 16-bit tensors as one persistent, warp-specialised kernel (sm_100a).
 //
 //   warps 0..7    gather producers: index-driven 16-byte cp.async row copies into the stage ring
-//   warps 8..15   read-out: tensor memory -> stores (G, D) / bulk reductions or red.global.add (S)
+//   warps 8..15   read-out: tensor memory -> stores (G, D) / red.global.add (S)
 //   warp  16      tensor-memory allocation; one lane issues tcgen05.mma, four per stage as straight-line code
 //   warp  17      one lane issues the TMA box loads of everything that is not gathered
 //   warps 18, 19  (D) look up the token rows of the contraction rows to come into a table in shared memory
@@ -40,8 +40,7 @@ constexpr int kBatch = 256;                        // D: contraction rows whose 
 __host__ __device__ constexpr uint32_t table_bytes(bool slots) { return (slots ? 4u : 2u) * kBatch * 4u; }
 constexpr uint32_t kMTile = 16384;                 // bytes of the 128-wide operand: 128 rows x 64 elements, or 64 rows x 128
 constexpr uint32_t kSeg = kStep * 128u;            // one 64-column segment of a 64-row tile
-constexpr uint32_t kEpiPlain = kEpiWarps * 4096u;
-constexpr uint32_t kEpiBulk = (kEpiWarps * 2u * kBulkBufBytes + 1023u) & ~1023u;
+constexpr uint32_t kEpi = kEpiWarps * 4096u;       // transposes of the read-out
 constexpr size_t kSmemMax = 227 * 1024;
 constexpr int kSms = 148;
 
@@ -80,7 +79,6 @@ struct DenseParams {
   int swap;           // D: 1 = the slot rows' features are the accumulator's rows
   int lane_rows;      // D: 1 = the output's rows are the accumulator's rows
   int tma_rows;       // S, D: slot rows come by TMA
-  int bulk;           // S
   int half;           // columns of a tile one CTA stages: BN, or BN / 2 in a pair
 };
 
@@ -140,7 +138,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
   DenseHeader* hdr = reinterpret_cast<DenseHeader*>(smem_raw);
   const uint32_t smem0 = smem_u32(smem_raw);
   const uint32_t epi0 = smem0 + kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : 0u);
-  const uint32_t ring0 = epi0 + ((OP == kOpScatter && p.bulk) ? kEpiBulk : kEpiPlain);
+  const uint32_t ring0 = epi0 + kEpi;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int first = PAIR ? blockIdx.x >> 1 : blockIdx.x, stride = PAIR ? gridDim.x >> 1 : gridDim.x;    // units of this CTA or pair
   const bool leader = !PAIR || (blockIdx.x & 1) == 0;
@@ -351,10 +349,9 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     // =========================== read-out ===========================
     const int ew = warp - kProdWarps;
     const int lg = ew & 3, half = ew >> 2;               // TMEM lane group, share of the column blocks
-    const uint32_t area = epi0 + static_cast<uint32_t>(ew) * ((OP == kOpScatter && p.bulk) ? 2u * kBulkBufBytes : 4096u);
+    const uint32_t area = epi0 + static_cast<uint32_t>(ew) * 4096u;
     const uint32_t lane_base = static_cast<uint32_t>(lg * 32) << 16;
     T* out = static_cast<T*>(p.Out);
-    int q = 0;                                           // bulk groups committed so far by this thread
     bool alive = true;
     pdl_wait();                                          // planning flags, zeros the results are added to
     // G, S: destination of tile row lg * 32 + lane of the next unit - token id, slot, planning flag - loaded a unit ahead
@@ -391,20 +388,18 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
         look_up(un + stride);
       }
       const T* bias_row = (OP != kOpDweight && p.bias) ? static_cast<const T*>(p.bias) + static_cast<long long>(u.e) * p.N + u.n0 : nullptr;
-      const bool bulk = OP == kOpScatter && p.bulk && to_f32 == 0u;
-      if (OP == kOpScatter && p.bulk && !bulk) bulk_wait_all();    // the transposes below reuse the staging buffers
       const int buf = t & 1;
       alive = mbar_wait_warp(smem_u32(&hdr->acc_full[buf]), (t >> 1) & 1, abort_flag, p.status.word, lane);
       if (!alive) break;
       tc_fence_after();
       const uint32_t acc = tmem_base + lane_base + static_cast<uint32_t>(buf) * acc_cols;
-      const bool packed = OP == kOpGather || bulk || (OP == kOpDweight && p.splits == 1 && p.lane_rows);
+      const bool packed = OP == kOpGather || (OP == kOpScatter && to_f32 == 0u) || (OP == kOpDweight && p.splits == 1 && p.lane_rows);
       if (packed) {
-        // 64 columns = 128 bytes of a 16-bit row at a time
-        for (int c = half; c * 64 < bn; c += 2, ++q) {
-          const uint32_t srow = OP == kOpScatter ? area + static_cast<uint32_t>(q & 1) * kBulkBufBytes + static_cast<uint32_t>(lane) * kBulkRowPitch
-                                                 : area + static_cast<uint32_t>(lane) * 128u;
-          if (OP == kOpScatter && q >= 2) bulk_wait_read_1();      // the group that used this buffer two blocks ago has been read
+        // 64 columns = 128 bytes of a 16-bit row at a time, eight lanes to a row: S adds 16 bytes a lane (the memory system takes
+        // 39 KB a microsecond from an SM that way).  Bulk reductions of 128 bytes, one per row and lane, took 85 clocks each to
+        // issue: 9000 clocks a 128 x 256 tile against 3800 of a contraction of 256.
+        for (int c = half; c * 64 < bn; c += 2) {
+          const uint32_t srow = area + static_cast<uint32_t>(lane) * 128u;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             if (c * 64 + h * 32 < bn) {
@@ -416,7 +411,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
               for (int j = 0; j < 4; ++j) {
                 const int ch = h * 4 + j;
                 asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(
-                                 srow + static_cast<uint32_t>(OP == kOpScatter ? ch : ch ^ (lane & 7)) * 16u),
+                                 srow + static_cast<uint32_t>(ch ^ (lane & 7)) * 16u),
                              "r"(pack2(out, v[8 * j], v[8 * j + 1])), "r"(pack2(out, v[8 * j + 2], v[8 * j + 3])),
                              "r"(pack2(out, v[8 * j + 4], v[8 * j + 5])), "r"(pack2(out, v[8 * j + 6], v[8 * j + 7]))
                              : "memory");
@@ -424,36 +419,31 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
             }
           }
           const int col0 = u.n0 + c * 64;
-          if (OP == kOpScatter) {
-            fence_proxy_async_smem();
-            const int ncols = min(64, bn - c * 64);
-            if (my_ro >= 0) bulk_reduce_add(out + static_cast<long long>(my_ro) * p.N + col0, srow, static_cast<uint32_t>(ncols) * 2u);
-            bulk_commit();
-          } else {
-            // eight lanes cover the 128 bytes of one row
-            __syncwarp();
-            const int j = lane & 7, col = col0 + j * 8;
-            uint4 x[8];
+          __syncwarp();
+          const int j = lane & 7, col = col0 + j * 8;
+          uint4 x[8];
 #pragma unroll
-            for (int it = 0; it < 8; ++it) {
-              const int row = it * 4 + (lane >> 3);
-              asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];"
-                           : "=r"(x[it].x), "=r"(x[it].y), "=r"(x[it].z), "=r"(x[it].w)
-                           : "r"(area + row * 128u + (static_cast<uint32_t>(j ^ (row & 7)) << 4))
-                           : "memory");
+          for (int it = 0; it < 8; ++it) {
+            const int row = it * 4 + (lane >> 3);
+            asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];"
+                         : "=r"(x[it].x), "=r"(x[it].y), "=r"(x[it].z), "=r"(x[it].w)
+                         : "r"(area + row * 128u + (static_cast<uint32_t>(j ^ (row & 7)) << 4))
+                         : "memory");
+          }
+          __syncwarp();
+#pragma unroll
+          for (int it = 0; it < 8; ++it) {
+            const int row = it * 4 + (lane >> 3);
+            long long ro;
+            if (OP != kOpDweight) {
+              ro = __shfl_sync(0xffffffffu, my_ro, row);
+            } else {
+              const int f = u.m0 + lg * 32 + row;
+              ro = f < p.C ? static_cast<long long>(u.e) * p.C + f : -1;
             }
-            __syncwarp();
-#pragma unroll
-            for (int it = 0; it < 8; ++it) {
-              const int row = it * 4 + (lane >> 3);
-              long long ro;
-              if (OP == kOpGather) {
-                ro = __shfl_sync(0xffffffffu, my_ro, row);
-              } else {
-                const int f = u.m0 + lg * 32 + row;
-                ro = f < p.C ? static_cast<long long>(u.e) * p.C + f : -1;
-              }
-              if (ro >= 0 && col < n_end) *reinterpret_cast<uint4*>(out + ro * p.N + col) = x[it];
+            if (ro >= 0 && col < n_end) {
+              if (OP == kOpScatter) red8(out + ro * p.N + col, x[it]);
+              else *reinterpret_cast<uint4*>(out + ro * p.N + col) = x[it];
             }
           }
         }
@@ -498,7 +488,6 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
         else mbar_arrive(smem_u32(&hdr->acc_empty[buf]));
       }
     }
-    if (OP == kOpScatter) bulk_wait_all();               // shared memory must outlive the copy engine's reads
   } else if (warp == kMmaWarp) {
     // =========================== MMA issuer ===========================
     if (leader) {
@@ -728,7 +717,7 @@ int ring_stages(int half, bool nc_tile, uint32_t not_ring) {
 template <typename T, int OP, bool PAIR>
 cudaError_t launch(const DenseParams& p, const TensorMap3& mw, const TensorMap3& mr, bool after_own, cudaStream_t st) {
   const size_t n_bytes = (OP != kOpDweight && p.nc) ? static_cast<size_t>(p.half) * 128 : static_cast<size_t>((p.half + 63) / 64) * kSeg;
-  const size_t smem = kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : 0u) + ((OP == kOpScatter && p.bulk) ? kEpiBulk : kEpiPlain) +
+  const size_t smem = kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : 0u) + kEpi +
                       p.stages * (kMTile + n_bytes);
   cudaError_t err = ensure_smem_optin<dense16_kernel<T, OP, PAIR>>(static_cast<int>(kSmemMax));
   if (err != cudaSuccess) return err;
@@ -747,12 +736,11 @@ cudaError_t launch_typed(const DenseParams& p, int dtype, const TensorMap3& mw, 
 void configure_dense16_rowgemm(RowGemmParams& p, bool scatter) {
   const int steps = (p.C + kStep - 1) / kStep;
   const bool cp_rows = !scatter || !rows_fit_boxes(p.K, 128);
-  // (a scatter is bound by its additions: no pairs; bulk reductions go out in blocks of 64 columns)
-  const Tile t = pick_tile(p.N, p.M, p.E, steps, cp_rows ? 340.0 : 0.0, 0.0, scatter ? 28.0 : 16.0, scatter ? 64 : 1, !scatter);
+  const Tile t = pick_tile(p.N, p.M, p.E, steps, cp_rows ? 340.0 : 0.0, 0.0, 16.0, 1, true);
   p.BN = t.bn;
   p.pair = t.pair ? 1 : 0;
   p.bulk_epilogue = scatter ? 1 : 0;
-  p.stages = ring_stages(p.pair ? p.BN / 2 : p.BN, p.w_layout == EGS_W_NC, scatter ? kEpiBulk : kEpiPlain);
+  p.stages = ring_stages(p.pair ? p.BN / 2 : p.BN, p.w_layout == EGS_W_NC, kEpi);
   p.row_tiles = 2;        // two 128-row accumulators per CTA
   p.persistent = (scatter && steps <= 4) ? 1 : 0;        // (for egs_describe_plan) the additions outlast the contraction
 }
@@ -769,7 +757,6 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
   p.tiles_m = (r.M + rows - 1) / rows;
   p.tiles_n = (r.N + r.BN - 1) / r.BN;
   p.order = r.expert_fastest;
-  p.bulk = r.bulk_epilogue;
   const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.E;
   if (units > 2147483647ll - kSms) return cudaErrorInvalidValue;
   p.units = static_cast<int>(units);
@@ -779,7 +766,9 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
   const unsigned box[3] = {64u, p.nc ? static_cast<unsigned>(p.half) : static_cast<unsigned>(kStep), 1u};
   if (!encode_tensor_map_16bit(&mw, r.W, 3, dims, box)) return cudaErrorInvalidValue;
   p.tma_rows = scatter && rows_fit_boxes(r.K, 128) && encode_slot_rows(&mr, r.A, r.B, r.E, r.K, r.C, 128);
-  if (scatter) return launch_typed<kOpScatter, false>(p, dtype, mw, mr, r.after_own != 0, st);
+  if (scatter)
+    return r.pair ? launch_typed<kOpScatter, true>(p, dtype, mw, mr, r.after_own != 0, st)
+                  : launch_typed<kOpScatter, false>(p, dtype, mw, mr, r.after_own != 0, st);
   return r.pair ? launch_typed<kOpGather, true>(p, dtype, mw, mr, false, st) : launch_typed<kOpGather, false>(p, dtype, mw, mr, false, st);
 }
 
@@ -813,7 +802,7 @@ void configure_dense16_dweight(DWeightParams& p) {
       }
     }
   }
-  p.stages = ring_stages(p.pair ? p.BN / 2 : p.BN, false, table_bytes(slot_cp) + kEpiPlain);
+  p.stages = ring_stages(p.pair ? p.BN / 2 : p.BN, false, table_bytes(slot_cp) + kEpi);
   p.row_tiles = 2;        // two 128-row accumulators per CTA
 }
 

@@ -469,6 +469,13 @@ __device__ __forceinline__ void red4(__nv_bfloat16* dst, uint32_t x0, uint32_t x
 __device__ __forceinline__ void red4(__half* dst, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3) {
   asm volatile("red.global.add.noftz.v2.f16x2 [%0], {%1,%2};" ::"l"(dst), "r"(pack2(dst, x0, x1)), "r"(pack2(dst, x2, x3)) : "memory");
 }
+// eight 16-bit elements, packed
+__device__ __forceinline__ void red8(__nv_bfloat16* dst, const uint4& x) {
+  asm volatile("red.global.add.noftz.v4.bf16x2 [%0], {%1,%2,%3,%4};" ::"l"(dst), "r"(x.x), "r"(x.y), "r"(x.z), "r"(x.w) : "memory");
+}
+__device__ __forceinline__ void red8(__half* dst, const uint4& x) {
+  asm volatile("red.global.add.noftz.v4.f16x2 [%0], {%1,%2,%3,%4};" ::"l"(dst), "r"(x.x), "r"(x.y), "r"(x.z), "r"(x.w) : "memory");
+}
 __device__ __forceinline__ void store4(float* dst, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3) {
   *reinterpret_cast<uint4*>(dst) = make_uint4(x0, x1, x2, x3);
 }
