@@ -30,14 +30,15 @@ namespace {
 constexpr int kProdWarps = 8, kProdThreads = kProdWarps * 32;
 constexpr int kEpiWarps = 8;
 constexpr int kMmaWarp = kProdWarps + kEpiWarps, kTmaWarp = kMmaWarp + 1;
-constexpr int kIndexWarp = kTmaWarp + 1, kIndexWarps = 2;      // D only
-template <int OP> constexpr int kDenseThreads = (OP == 2 ? kIndexWarp + kIndexWarps : kTmaWarp + 1) * 32;
+constexpr int kIndexWarp = kTmaWarp + 1, kIndexWarps = 2;
+constexpr int kDenseThreads = (kIndexWarp + kIndexWarps) * 32;
 constexpr int kStep = 64;                          // contraction elements per stage
 constexpr uint32_t kDenseHeader = 1024;
 constexpr int kBatch = 256;                        // D: contraction rows whose ids are looked up at a time (four steps)
 // D: two batches of token rows; without TMA boxes for the slot rows two of those as well.  (Sized so that four stages of a
 // 128 x 256 tile still fit beside it with TMA boxes: three stages cost a quarter of the rate.)
 __host__ __device__ constexpr uint32_t table_bytes(bool slots) { return (slots ? 4u : 2u) * kBatch * 4u; }
+constexpr uint32_t kRowTable = 2u * kTileM * 4u;   // G, S: source rows of two units
 constexpr uint32_t kMTile = 16384;                 // bytes of the 128-wide operand: 128 rows x 64 elements, or 64 rows x 128
 constexpr uint32_t kSeg = kStep * 128u;            // one 64-column segment of a 64-row tile
 constexpr uint32_t kEpi = kEpiWarps * 4096u;       // transposes of the read-out
@@ -49,7 +50,6 @@ enum { kOpGather = 0, kOpScatter = 1, kOpDweight = 2 };
 struct __align__(16) DenseHeader {
   unsigned long long full[kMaxStages];
   unsigned long long empty[kMaxStages];
-  unsigned long long peer_full[kMaxStages];          // pairs: the peer's half of a stage has landed (the leader's copy is used)
   unsigned long long acc_full[2];
   unsigned long long acc_empty[2];
   unsigned long long ids_full[2];
@@ -74,7 +74,8 @@ struct DenseParams {
   int nc;             // G, S: 1 = weights [E, N, C]
   int index_dtype;
   int BN, stages;
-  int tiles_m, tiles_n, units, order;    // order: 1 = experts vary faster than row blocks
+  int tiles_m, tiles_n, units;
+  int r1, r2;                            // radices of the unit number, see Walk
   int splits, rows_per_split;            // D
   int swap;           // D: 1 = the slot rows' features are the accumulator's rows
   int lane_rows;      // D: 1 = the output's rows are the accumulator's rows
@@ -82,47 +83,63 @@ struct DenseParams {
   int half;           // columns of a tile one CTA stages: BN, or BN / 2 in a pair
 };
 
-struct Unit {
-  int e, m0, n0, split;
-};
-template <int OP, bool PAIR>
-__device__ __forceinline__ Unit unit_of(const DenseParams& p, int u) {
-  Unit r;
-  const int nt = u % p.tiles_n;
-  u /= p.tiles_n;
-  int mt;
-  r.split = 0;
-  if (OP == kOpDweight) {
-    mt = u % p.tiles_m;
-    u /= p.tiles_m;
-    r.split = u % p.splits;
-    r.e = u / p.splits;
-  } else if (p.order) {
-    r.e = u % p.E;
-    mt = u / p.E;
-  } else {
-    mt = u % p.tiles_m;
-    r.e = u / p.tiles_m;
+// Position in the stage ring.
+struct Cursor {
+  int slot = 0, round = 0;
+  __device__ __forceinline__ void next(int stages) {
+    if (++slot == stages) {
+      slot = 0;
+      ++round;
+    }
   }
-  r.m0 = PAIR ? mt * 2 * kTileM + static_cast<int>(blockIdx.x & 1) * kTileM : mt * kTileM;     // this CTA's 128 rows
-  r.n0 = nt * p.BN;
-  return r;
-}
-// width of a tile's MMA (the last tile of a row may be narrower), and the first column this CTA stages
-template <bool PAIR>
-__device__ __forceinline__ int mma_width(const DenseParams& p, const Unit& u) {
-  const int left = p.N - u.n0;
-  return min(p.BN, PAIR ? (left + 31) & ~31 : (left + 15) & ~15);
-}
-template <bool PAIR>
-__device__ __forceinline__ int first_column(const DenseParams& p, const Unit& u) {
-  return PAIR && (blockIdx.x & 1) ? u.n0 + mma_width<true>(p, u) / 2 : u.n0;
-}
-template <int OP>
-__device__ __forceinline__ int unit_steps(const DenseParams& p, const Unit& u) {
-  if (OP != kOpDweight) return (p.C + kStep - 1) / kStep;
-  return (min(p.rows_per_split, p.M - u.split * p.rows_per_split) + kStep - 1) / kStep;
-}
+};
+
+// The units of a CTA or pair, `stride` apart.  A unit is a number in a mixed radix - column tile; row block of a group, expert, group
+// (G, S) or row block, row range, expert (D) - and is advanced by adding the stride's digits: three divisions a unit (1000 clocks and
+// more) in the lanes that feed the tensor core were a fifth of the time of a tile with eight steps.
+template <int OP, bool PAIR>
+struct Walk {
+  int left;                    // units to come, this one included
+  int m0, n0, e, split;        // this CTA's 128 rows, the first column of the tile, expert, row range
+  int d0, d1, d2, d3, s0, s1, s2, s3;
+  const DenseParams& p;
+  __device__ __forceinline__ explicit Walk(const DenseParams& q) : p(q) {
+    int u = PAIR ? blockIdx.x >> 1 : blockIdx.x, s = PAIR ? gridDim.x >> 1 : gridDim.x;
+    left = u < p.units ? (p.units - u + s - 1) / s : 0;
+    d0 = u % p.tiles_n; u /= p.tiles_n; s0 = s % p.tiles_n; s /= p.tiles_n;
+    d1 = u % p.r1; u /= p.r1; s1 = s % p.r1; s /= p.r1;
+    d2 = u % p.r2; d3 = u / p.r2; s2 = s % p.r2; s3 = s / p.r2;
+    place();
+  }
+  __device__ __forceinline__ void place() {
+    n0 = d0 * p.BN;
+    const int mt = OP == kOpDweight ? d1 : d3 * p.r1 + d1;
+    e = OP == kOpDweight ? d3 : d2;
+    split = OP == kOpDweight ? d2 : 0;
+    m0 = PAIR ? mt * 2 * kTileM + static_cast<int>(blockIdx.x & 1) * kTileM : mt * kTileM;
+  }
+  __device__ __forceinline__ void next() {
+    --left;
+    d0 += s0;
+    d1 += s1;
+    d2 += s2;
+    d3 += s3;
+    if (d0 >= p.tiles_n) { d0 -= p.tiles_n; ++d1; }
+    if (d1 >= p.r1) { d1 -= p.r1; ++d2; }
+    if (d2 >= p.r2) { d2 -= p.r2; ++d3; }
+    place();
+  }
+  __device__ __forceinline__ int steps() const {
+    if (OP != kOpDweight) return (p.C + kStep - 1) / kStep;
+    return (min(p.rows_per_split, p.M - split * p.rows_per_split) + kStep - 1) / kStep;
+  }
+  // width of the tile's MMA (the last tile of a row may be narrower), and the first column this CTA stages
+  __device__ __forceinline__ int width() const {
+    const int rest = p.N - n0;
+    return min(p.BN, PAIR ? (rest + 31) & ~31 : (rest + 15) & ~15);
+  }
+  __device__ __forceinline__ int first_column() const { return PAIR && (blockIdx.x & 1) ? n0 + width() / 2 : n0; }
+};
 
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* map, int x, int y, int z, int w, uint32_t bar) {
   asm volatile(
@@ -132,15 +149,14 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* map, int x
 }
 
 template <typename T, int OP, bool PAIR>
-__global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThreads<OP>, 1) dense16_kernel(const __grid_constant__ DenseParams p, const __grid_constant__ TensorMap3 map_w,
+__global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThreads, 1) dense16_kernel(const __grid_constant__ DenseParams p, const __grid_constant__ TensorMap3 map_w,
                                                                    const __grid_constant__ TensorMap3 map_rows) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   DenseHeader* hdr = reinterpret_cast<DenseHeader*>(smem_raw);
   const uint32_t smem0 = smem_u32(smem_raw);
-  const uint32_t epi0 = smem0 + kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : 0u);
+  const uint32_t epi0 = smem0 + kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : kRowTable);
   const uint32_t ring0 = epi0 + kEpi;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int first = PAIR ? blockIdx.x >> 1 : blockIdx.x, stride = PAIR ? gridDim.x >> 1 : gridDim.x;    // units of this CTA or pair
   const bool leader = !PAIR || (blockIdx.x & 1) == 0;
   const int nseg = (p.half + 63) >> 6;
   const uint32_t n_bytes = (OP != kOpDweight && p.nc) ? static_cast<uint32_t>(p.half) * 128u : static_cast<uint32_t>(nseg) * kSeg;
@@ -154,9 +170,8 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
 
   if (tid == 0) {
     for (int s = 0; s < kMaxStages; ++s) {
-      mbar_init(smem_u32(&hdr->full[s]), (has_cp ? kProdThreads : 0) + (has_tma ? 1 : 0));
+      mbar_init(smem_u32(&hdr->full[s]), (has_cp ? kProdThreads : 0) + (has_tma ? 1 : 0) + (PAIR && leader ? 1 : 0));      // (+ the peer's stage)
       mbar_init(smem_u32(&hdr->empty[s]), 1);
-      mbar_init(smem_u32(&hdr->peer_full[s]), 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&hdr->acc_full[b]), 1);
@@ -198,34 +213,35 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       const int cc = tid & 7, r0 = tid >> 3;
       const uint32_t rc_dst = static_cast<uint32_t>(r0) * 128u + (static_cast<uint32_t>(cc ^ (r0 & 7)) << 4);
       const long long pitch_c = static_cast<long long>(p.C) * 2;
-      int slot = 0, round = 0;
+      Cursor at;
       bool alive = true;
+      auto wait_free = [&]() {             // for the stage at `at`; moves on
+        if (at.round > 0) alive = mbar_wait_all(smem_u32(&hdr->empty[at.slot]), (at.round - 1) & 1, abort_flag, p.status.word);
+        at.next(stages);
+      };
       if constexpr (OP != kOpDweight) {
-        long long ahead_t[4];              // G: token ids of the next unit's rows, loaded a unit ahead
-        auto fetch_ids = [&](int v) {
-          const Unit w = unit_of<OP, PAIR>(p, v);
+        // The index warps keep the rows of two units in shared memory.  A unit's are read one step ahead, before the copies of the
+        // step before it are issued: a read behind a copy waits for it.
+        const uint32_t table = smem0 + kDenseHeader + static_cast<uint32_t>(r0) * 4u;
+        const int units = Walk<OP, PAIR>(p).left, steps = (p.C + kStep - 1) / kStep;
+        int row[4];
+        auto read_rows = [&](int t) {
+          alive = mbar_wait_all(smem_u32(&hdr->ids_full[t & 1]), (t >> 1) & 1, abort_flag, p.status.word);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int m = min(w.m0 + r0 + 32 * i, p.M - 1), b = m / p.K;
-            ahead_t[i] = load_index(p.Ind, p.index_dtype, static_cast<long long>(b * p.E + w.e) * p.K + (m - b * p.K));
-          }
+          for (int i = 0; i < 4; ++i)
+            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(row[i]) : "r"(table + static_cast<uint32_t>(t & 1) * (kTileM * 4u) + i * 128u) : "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&hdr->ids_empty[t & 1]));
         };
-        if (OP == kOpGather && first < p.units) fetch_ids(first);
-        for (int un = first; un < p.units && alive; un += stride) {
-          const Unit u = unit_of<OP, PAIR>(p, un);
-          const int steps = unit_steps<OP>(p, u);
+        if (units > 0) read_rows(0);
+        for (int t = 0; t < units && alive; ++t) {
           const char* src[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int m = u.m0 + r0 + 32 * i, b = m / p.K;
-            int row = -1;
-            if (OP == kOpScatter) row = m < p.M ? (b * p.E + u.e) * p.K + (m - b * p.K) : -1;
-            else if (m < p.M && ahead_t[i] >= 0 && ahead_t[i] < p.T) row = b * p.T + static_cast<int>(ahead_t[i]);
-            src[i] = row >= 0 ? Rows + static_cast<long long>(row) * pitch_c + cc * 16 : nullptr;
-          }
-          if (OP == kOpGather && un + stride < p.units) fetch_ids(un + stride);
+          for (int i = 0; i < 4; ++i) src[i] = row[i] >= 0 ? Rows + static_cast<long long>(row[i]) * pitch_c + cc * 16 : nullptr;
           for (int k = 0; k < steps; ++k) {
-            if (round > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[slot]), (round - 1) & 1, abort_flag, p.status.word, lane);
+            const int slot = at.slot;
+            wait_free();
+            if (alive && k + 1 == steps && t + 1 < units) read_rows(t + 1);
             if (!alive) break;
             const uint32_t base = ring0 + static_cast<uint32_t>(slot) * stage_bytes + rc_dst;
             const bool kvalid = k * kStep + cc * 8 < p.C;
@@ -236,7 +252,6 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
               if (src[i]) src[i] += 128;
             }
             cp_async_mbar_arrive_noinc(smem_u32(&hdr->full[slot]));
-            if (++slot == stages) { slot = 0; ++round; }
           }
         }
       } else {
@@ -276,20 +291,21 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
             }
           };
           int batch = 0;                                                             // batches begun by this CTA
-          if (first < p.units) {
-            alive = mbar_wait_warp(smem_u32(&hdr->ids_full[0]), 0u, abort_flag, p.status.word, lane);
+          Walk<OP, PAIR> u(p);
+          if (u.left > 0) {
+            alive = mbar_wait_all(smem_u32(&hdr->ids_full[0]), 0u, abort_flag, p.status.word);
             read_ids(table);
           }
-          for (int un = first; un < p.units && alive; un += stride) {
-            const Unit u = unit_of<OP, PAIR>(p, un);
-            const int steps = unit_steps<OP>(p, u);
-            const int nc0 = first_column<PAIR>(p, u);
+          for (; u.left > 0 && alive; u.next()) {
+            const int steps = u.steps();
+            const int nc0 = u.first_column();
             const int f0 = (SWAP ? nc0 : u.m0) + g_c * 8, s0 = (SWAP ? u.m0 : nc0) + s_c * 8;       // first feature of the chunk
             const bool g_in = f0 < (SWAP ? p.N : p.C), s_in = s0 < (SWAP ? p.C : p.N);
             const char* g_col = Rows + (g_in ? static_cast<long long>(f0) * 2 : 0ll);
             const char* s_col = static_cast<const char*>(p.Slot) + (s_in ? static_cast<long long>(s0) * 2 : 0ll);
             for (int k = 0; k < steps; ++k) {
-              if (round > 0) alive = mbar_wait_warp(smem_u32(&hdr->empty[slot]), (round - 1) & 1, abort_flag, p.status.word, lane);
+              const int slot = at.slot;
+              wait_free();
               if (!alive) break;
               int cg[RG], cs[RS];
 #pragma unroll
@@ -305,8 +321,8 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&hdr->ids_empty[batch & 1]));    // this warp has read the batch
                 ++batch;
-                if (!unit_end || un + stride < p.units) {
-                  alive = mbar_wait_warp(smem_u32(&hdr->ids_full[batch & 1]), (batch >> 1) & 1, abort_flag, p.status.word, lane);
+                if (!unit_end || u.left > 1) {
+                  alive = mbar_wait_all(smem_u32(&hdr->ids_full[batch & 1]), (batch >> 1) & 1, abort_flag, p.status.word);
                   if (!alive) break;
                   read_ids(table + static_cast<uint32_t>(batch & 1) * (kBatch * 4u));
                 }
@@ -325,7 +341,6 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
                              (s_in && cs[j] >= 0) ? 16u : 0u);
               }
               cp_async_mbar_arrive_noinc(smem_u32(&hdr->full[slot]));
-              if (++slot == stages) { slot = 0; ++round; }
             }
           }
         };
@@ -357,23 +372,22 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     // G, S: destination of tile row lg * 32 + lane of the next unit - token id, slot, planning flag - loaded a unit ahead
     long long next_t = 0;
     int next_slot = -1, next_b = 0, next_flag = 0;
-    auto look_up = [&](int v) {
-      if (OP == kOpDweight || v >= p.units) return;
-      const Unit w = unit_of<OP, PAIR>(p, v);
-      const int m = w.m0 + lg * 32 + lane;
+    Walk<OP, PAIR> u(p), ahead(p);
+    auto look_up = [&]() {
+      if (OP == kOpDweight || ahead.left <= 0) return;
+      const int m = ahead.m0 + lg * 32 + lane;
       next_slot = -1;
       next_flag = 0;
       if (m < p.M) {
         next_b = m / p.K;
-        next_slot = (next_b * p.E + w.e) * p.K + (m - next_b * p.K);
+        next_slot = (next_b * p.E + ahead.e) * p.K + (m - next_b * p.K);
         next_t = load_index(p.Ind, p.index_dtype, next_slot);
         if (OP == kOpScatter) next_flag = p.plan[next_b];
       }
+      ahead.next();
     };
-    look_up(first);
-    int t = 0;
-    for (int un = first; un < p.units && alive; un += stride, ++t) {
-      const Unit u = unit_of<OP, PAIR>(p, un);
+    look_up();
+    for (int t = 0; u.left > 0 && alive; u.next(), ++t) {
       const int bn = min(p.BN, p.N - u.n0);              // columns of this tile (a multiple of 8)
       const int n_end = u.n0 + bn;
       int my_ro = -1;                                    // G, S: destination row of tile row lg * 32 + lane
@@ -385,11 +399,11 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           my_ro = OP == kOpGather ? next_slot : (ok ? next_b * p.T + static_cast<int>(next_t) : -1);
         }
         if (OP == kOpScatter) to_f32 = __ballot_sync(0xffffffffu, next_flag != 0);
-        look_up(un + stride);
+        look_up();
       }
       const T* bias_row = (OP != kOpDweight && p.bias) ? static_cast<const T*>(p.bias) + static_cast<long long>(u.e) * p.N + u.n0 : nullptr;
       const int buf = t & 1;
-      alive = mbar_wait_warp(smem_u32(&hdr->acc_full[buf]), (t >> 1) & 1, abort_flag, p.status.word, lane);
+      alive = mbar_wait_all(smem_u32(&hdr->acc_full[buf]), (t >> 1) & 1, abort_flag, p.status.word);
       if (!alive) break;
       tc_fence_after();
       const uint32_t acc = tmem_base + lane_base + static_cast<uint32_t>(buf) * acc_cols;
@@ -496,13 +510,12 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       const uint64_t b_desc = (b_mn ? make_smem_desc(0u, kSeg, 1024u) : make_smem_desc(0u, 16u, 1024u)) + (kMTile >> 4);
       const uint32_t a_adv = (a_mn ? 16u * 128u : 32u) >> 4, b_adv = (b_mn ? 16u * 128u : 32u) >> 4;
       bool ok = true;
-      int t = 0, slot = 0, round = 0;
-      uint32_t addr = ring0 >> 4;                        // descriptors: 14 address bits in 16-byte units (shared memory is smaller)
-      for (int un = first; un < p.units && ok; un += stride, ++t) {
-        const Unit u = unit_of<OP, PAIR>(p, un);
-        const int steps = unit_steps<OP>(p, u);
+      int t = 0;
+      Cursor at;
+      for (Walk<OP, PAIR> u(p); u.left > 0 && ok; u.next(), ++t) {
+        const int steps = u.steps();
         const uint32_t idesc =
-            make_idesc(Elem<T>::fmt, a_mn ? 1u : 0u, b_mn ? 1u : 0u, PAIR ? 2 * kTileM : kTileM, static_cast<uint32_t>(mma_width<PAIR>(p, u)));
+            make_idesc(Elem<T>::fmt, a_mn ? 1u : 0u, b_mn ? 1u : 0u, PAIR ? 2 * kTileM : kTileM, static_cast<uint32_t>(u.width()));
         const int buf = t & 1;
         if (t >= 2) {
           ok = mbar_wait_all(smem_u32(&hdr->acc_empty[buf]), ((t >> 1) - 1) & 1, abort_flag, p.status.word);
@@ -510,97 +523,116 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
         }
         const uint32_t d = tmem_base + static_cast<uint32_t>(buf) * acc_cols;
         for (int ks = 0; ks < steps; ++ks) {
-          ok = mbar_wait_all(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status.word);
-          if (PAIR && ok) ok = mbar_wait_all(smem_u32(&hdr->peer_full[slot]), round & 1, abort_flag, p.status.word);
+          ok = mbar_wait_all(smem_u32(&hdr->full[at.slot]), at.round & 1, abort_flag, p.status.word);
           if (!ok) break;
+          const uint32_t empty = smem_u32(&hdr->empty[at.slot]);
+          // (descriptors: 14 address bits in 16-byte units; shared memory is smaller)
+          const uint32_t addr = (ring0 + static_cast<uint32_t>(at.slot) * stage_bytes) >> 4;
+          at.next(stages);
           tc_fence_after();
           if (elect_one()) {
             umma_f16_x4<PAIR>(d, a_desc + addr, b_desc + addr, a_adv, b_adv, idesc, ks > 0 ? 1u : 0u);
-            umma_done<PAIR>(smem_u32(&hdr->empty[slot]));
+            umma_done<PAIR>(empty);
             if (ks + 1 == steps) umma_done<PAIR>(smem_u32(&hdr->acc_full[buf]));
-          }
-          addr += stage_bytes >> 4;
-          if (++slot == stages) {
-            slot = 0;
-            ++round;
-            addr = ring0 >> 4;
           }
         }
       }
     } else if (PAIR) {
       // the peer tells the leader of every stage that has landed here
-      const uint32_t to_leader = map_to_cta(smem_u32(&hdr->peer_full[0]), 0);
+      const uint32_t to_leader = map_to_cta(smem_u32(&hdr->full[0]), 0);
       bool ok = true;
-      int slot = 0, round = 0;
-      for (int un = first; un < p.units && ok; un += stride) {
-        const int steps = unit_steps<OP>(p, unit_of<OP, PAIR>(p, un));
+      Cursor at;
+      for (Walk<OP, PAIR> u(p); u.left > 0 && ok; u.next()) {
+        const int steps = u.steps();
         for (int ks = 0; ks < steps; ++ks) {
-          ok = mbar_wait_all(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status.word);
+          ok = mbar_wait_all(smem_u32(&hdr->full[at.slot]), at.round & 1, abort_flag, p.status.word);
           if (!ok) break;
-          if (elect_one()) mbar_arrive_cluster_relaxed(to_leader + slot * 8u);
-          if (++slot == stages) { slot = 0; ++round; }
+          const uint32_t there = to_leader + at.slot * 8u;
+          at.next(stages);
+          if (elect_one()) mbar_arrive_cluster_relaxed(there);
         }
       }
     }
     __syncwarp();
   } else if (warp >= kIndexWarp) {
-    // =========================== index warps (D) ===========================
+    // =========================== index warps ===========================
     const uint32_t table = smem0 + kDenseHeader;
     const int it = tid - kIndexWarp * 32;
-    constexpr int kPer = kBatch / (kIndexWarps * 32);
     bool alive = true;
-    int batch = 0;
-    for (int un = first; un < p.units && alive; un += stride) {
-      const Unit u = unit_of<OP, PAIR>(p, un);
-      const int m_begin = u.split * p.rows_per_split, m_end = min(p.M, m_begin + p.rows_per_split);
-      const bool report = u.m0 == 0 && u.n0 == 0;
-      for (int m0 = m_begin; m0 < m_end && alive; m0 += kBatch, ++batch) {
-        int tok[kPer], slot_row[kPer];
-        long long t[kPer];
+    if constexpr (OP != kOpDweight) {
+      int t = 0;
+      for (Walk<OP, PAIR> u(p); has_cp && u.left > 0 && alive; u.next(), ++t) {
+        int row[2], b[2];
+        long long id[2];
 #pragma unroll
-        for (int i = 0; i < kPer; ++i) {                 // all loads first
-          const int m = m0 + it + i * kIndexWarps * 32;
-          const bool on = m < m_end;
-          tok[i] = on ? m / p.K : 0;
-          const int s = (tok[i] * p.E + u.e) * p.K + (on ? m - tok[i] * p.K : 0);
-          t[i] = load_index(p.Ind, p.index_dtype, s);
-          slot_row[i] = on ? s : -1;
+        for (int i = 0; i < 2; ++i) {
+          const int m = u.m0 + it + 64 * i;
+          b[i] = m / p.K;
+          row[i] = m < p.M ? (b[i] * p.E + u.e) * p.K + (m - b[i] * p.K) : -1;
+          id[i] = (OP == kOpGather && row[i] >= 0) ? load_index(p.Ind, p.index_dtype, row[i]) : 0;
         }
-#pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-          const bool known = t[i] >= 0 && t[i] < p.T;
-          if (slot_row[i] >= 0 && !known && report) p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
-          tok[i] = (slot_row[i] >= 0 && known) ? tok[i] * p.T + static_cast<int>(t[i]) : -1;
-        }
-        if (batch >= 2) alive = mbar_wait_warp(smem_u32(&hdr->ids_empty[batch & 1]), ((batch >> 1) - 1) & 1, abort_flag, p.status.word, lane);
+        if (t >= 2) alive = mbar_wait_all(smem_u32(&hdr->ids_empty[t & 1]), ((t >> 1) - 1) & 1, abort_flag, p.status.word);
         if (!alive) break;
-        const uint32_t dst = table + static_cast<uint32_t>(batch & 1) * (kBatch * 4u) + static_cast<uint32_t>(it) * 4u;
 #pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-          asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + i * kIndexWarps * 128u), "r"(tok[i]) : "memory");
-          if (!p.tma_rows) asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + 2u * kBatch * 4u + i * kIndexWarps * 128u), "r"(slot_row[i]) : "memory");
+        for (int i = 0; i < 2; ++i) {
+          if (OP == kOpGather) row[i] = (row[i] >= 0 && id[i] >= 0 && id[i] < p.T) ? b[i] * p.T + static_cast<int>(id[i]) : -1;
+          asm volatile("st.shared.b32 [%0], %1;" ::"r"(table + static_cast<uint32_t>(t & 1) * (kTileM * 4u) + static_cast<uint32_t>(it + 64 * i) * 4u), "r"(row[i]) : "memory");
         }
-        mbar_arrive(smem_u32(&hdr->ids_full[batch & 1]));
+        mbar_arrive(smem_u32(&hdr->ids_full[t & 1]));
+      }
+    } else {
+      constexpr int kPer = kBatch / (kIndexWarps * 32);
+      int batch = 0;
+      for (Walk<OP, PAIR> u(p); u.left > 0 && alive; u.next()) {
+        const int m_begin = u.split * p.rows_per_split, m_end = min(p.M, m_begin + p.rows_per_split);
+        const bool report = u.m0 == 0 && u.n0 == 0;
+        for (int m0 = m_begin; m0 < m_end && alive; m0 += kBatch, ++batch) {
+          int tok[kPer], slot_row[kPer];
+          long long t[kPer];
+#pragma unroll
+          for (int i = 0; i < kPer; ++i) {                 // all loads first
+            const int m = m0 + it + i * kIndexWarps * 32;
+            const bool on = m < m_end;
+            tok[i] = on ? m / p.K : 0;
+            const int s = (tok[i] * p.E + u.e) * p.K + (on ? m - tok[i] * p.K : 0);
+            t[i] = load_index(p.Ind, p.index_dtype, s);
+            slot_row[i] = on ? s : -1;
+          }
+#pragma unroll
+          for (int i = 0; i < kPer; ++i) {
+            const bool known = t[i] >= 0 && t[i] < p.T;
+            if (slot_row[i] >= 0 && !known && report) p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
+            tok[i] = (slot_row[i] >= 0 && known) ? tok[i] * p.T + static_cast<int>(t[i]) : -1;
+          }
+          if (batch >= 2) alive = mbar_wait_all(smem_u32(&hdr->ids_empty[batch & 1]), ((batch >> 1) - 1) & 1, abort_flag, p.status.word);
+          if (!alive) break;
+          const uint32_t dst = table + static_cast<uint32_t>(batch & 1) * (kBatch * 4u) + static_cast<uint32_t>(it) * 4u;
+#pragma unroll
+          for (int i = 0; i < kPer; ++i) {
+            asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + i * kIndexWarps * 128u), "r"(tok[i]) : "memory");
+            if (!p.tma_rows) asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + 2u * kBatch * 4u + i * kIndexWarps * 128u), "r"(slot_row[i]) : "memory");
+          }
+          mbar_arrive(smem_u32(&hdr->ids_full[batch & 1]));
+        }
       }
     }
   } else if (has_tma) {
     // =========================== TMA issuer ===========================
     const uint32_t bytes = (OP != kOpDweight ? n_bytes : (p.swap ? kMTile : n_bytes)) + ((OP == kOpScatter && p.tma_rows) ? kMTile : 0u);
     bool ok = true;
-    int slot = 0, round = 0;
-    uint32_t base = ring0;
-    for (int un = first; un < p.units && ok; un += stride) {
-      const Unit u = unit_of<OP, PAIR>(p, un);
-      const int steps = unit_steps<OP>(p, u);
-      const int n0 = first_column<PAIR>(p, u);
+    Cursor at;
+    for (Walk<OP, PAIR> u(p); u.left > 0 && ok; u.next()) {
+      const int steps = u.steps();
+      const int n0 = u.first_column();
       int m = OP == kOpDweight ? u.split * p.rows_per_split : u.m0;
       int b = m / p.K, k = m - b * p.K;                // first slot row of the step
       for (int ks = 0, c0 = 0; ks < steps; ++ks, c0 += kStep) {
-        if (round > 0) {
-          ok = mbar_wait_all(smem_u32(&hdr->empty[slot]), (round - 1) & 1, abort_flag, p.status.word);
+        if (at.round > 0) {
+          ok = mbar_wait_all(smem_u32(&hdr->empty[at.slot]), (at.round - 1) & 1, abort_flag, p.status.word);
           if (!ok) break;
         }
-        const uint32_t bar = smem_u32(&hdr->full[slot]);
+        const uint32_t bar = smem_u32(&hdr->full[at.slot]), base = ring0 + static_cast<uint32_t>(at.slot) * stage_bytes;
+        at.next(stages);
         if (elect_one()) {
           mbar_arrive_expect_tx(bar, bytes);
           if (OP != kOpDweight) {
@@ -623,12 +655,6 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
         if (OP == kOpDweight) {
           k += kStep;                                  // 64 rows are parts of one batch element or whole ones
           while (k >= p.K) { k -= p.K; ++b; }
-        }
-        base += stage_bytes;
-        if (++slot == stages) {
-          slot = 0;
-          ++round;
-          base = ring0;
         }
       }
     }
@@ -717,12 +743,12 @@ int ring_stages(int half, bool nc_tile, uint32_t not_ring) {
 template <typename T, int OP, bool PAIR>
 cudaError_t launch(const DenseParams& p, const TensorMap3& mw, const TensorMap3& mr, bool after_own, cudaStream_t st) {
   const size_t n_bytes = (OP != kOpDweight && p.nc) ? static_cast<size_t>(p.half) * 128 : static_cast<size_t>((p.half + 63) / 64) * kSeg;
-  const size_t smem = kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : 0u) + kEpi +
+  const size_t smem = kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : kRowTable) + kEpi +
                       p.stages * (kMTile + n_bytes);
   cudaError_t err = ensure_smem_optin<dense16_kernel<T, OP, PAIR>>(static_cast<int>(kSmemMax));
   if (err != cudaSuccess) return err;
   const int grid = PAIR ? 2 * (p.units < kSms / 2 ? p.units : kSms / 2) : (p.units < kSms ? p.units : kSms);
-  err = launch_kernel(dense16_kernel<T, OP, PAIR>, grid, kDenseThreads<OP>, smem, st, after_own, p, mw, mr);
+  err = launch_kernel(dense16_kernel<T, OP, PAIR>, grid, kDenseThreads, smem, st, after_own, p, mw, mr);
   count_launch();
   return err;
 }
@@ -740,7 +766,7 @@ void configure_dense16_rowgemm(RowGemmParams& p, bool scatter) {
   p.BN = t.bn;
   p.pair = t.pair ? 1 : 0;
   p.bulk_epilogue = scatter ? 1 : 0;
-  p.stages = ring_stages(p.pair ? p.BN / 2 : p.BN, p.w_layout == EGS_W_NC, kEpi);
+  p.stages = ring_stages(p.pair ? p.BN / 2 : p.BN, p.w_layout == EGS_W_NC, kRowTable + kEpi);
   p.row_tiles = 2;        // two 128-row accumulators per CTA
   p.persistent = (scatter && steps <= 4) ? 1 : 0;        // (for egs_describe_plan) the additions outlast the contraction
 }
@@ -756,7 +782,11 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
   const int rows = r.pair ? 2 * kTileM : kTileM;
   p.tiles_m = (r.M + rows - 1) / rows;
   p.tiles_n = (r.N + r.BN - 1) / r.BN;
-  p.order = r.expert_fastest;
+  p.r1 = p.tiles_m;
+  p.r2 = r.E;
+  if (r.expert_fastest) {
+    p.r1 = 1;
+  }
   const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.E;
   if (units > 2147483647ll - kSms) return cudaErrorInvalidValue;
   p.units = static_cast<int>(units);
@@ -820,6 +850,8 @@ cudaError_t launch_dense16_dweight(const DWeightParams& r, int dtype, cudaStream
   const int rows = r.pair ? 2 * kTileM : kTileM;
   p.tiles_m = (p.C + rows - 1) / rows;
   p.tiles_n = (p.N + r.BN - 1) / r.BN;
+  p.r1 = p.tiles_m;
+  p.r2 = p.splits;
   const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.E * p.splits;
   if (units > 2147483647ll - kSms) return cudaErrorInvalidValue;
   p.units = static_cast<int>(units);
