@@ -38,10 +38,12 @@ constexpr int kBatch = 256;                        // D: contraction rows whose 
 // D: two batches of token rows; without TMA boxes for the slot rows two of those as well.  (Sized so that four stages of a
 // 128 x 256 tile still fit beside it with TMA boxes: three stages cost a quarter of the rate.)
 __host__ __device__ constexpr uint32_t table_bytes(bool slots) { return (slots ? 4u : 2u) * kBatch * 4u; }
-constexpr uint32_t kRowTable = 2u * kTileM * 4u;   // G, S: source rows of two units
+// G, S: source rows of two units, then destination rows of two units (kNoRow: none; top bit: added to the float32 rows)
+constexpr uint32_t kRowTable = 4u * kTileM * 4u;
+constexpr int kNoRow = 0x7fffffff;
 constexpr uint32_t kMTile = 16384;                 // bytes of the 128-wide operand: 128 rows x 64 elements, or 64 rows x 128
 constexpr uint32_t kSeg = kStep * 128u;            // one 64-column segment of a 64-row tile
-constexpr uint32_t kEpi = kEpiWarps * 4096u;       // transposes of the read-out
+__host__ __device__ constexpr uint32_t epi_bytes(bool wide) { return (wide ? kProdWarps + kEpiWarps : kEpiWarps) * 4096u; }       // transposes of the read-out
 constexpr size_t kSmemMax = 227 * 1024;
 constexpr int kSms = 148;
 
@@ -54,6 +56,8 @@ struct __align__(16) DenseHeader {
   unsigned long long acc_empty[2];
   unsigned long long ids_full[2];
   unsigned long long ids_empty[2];
+  unsigned long long dst_full[2];
+  unsigned long long dst_empty[2];
   unsigned long long drain;
   uint32_t tmem_base;
   uint32_t abort_flag;
@@ -155,7 +159,10 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
   DenseHeader* hdr = reinterpret_cast<DenseHeader*>(smem_raw);
   const uint32_t smem0 = smem_u32(smem_raw);
   const uint32_t epi0 = smem0 + kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : kRowTable);
-  const uint32_t ring0 = epi0 + kEpi;
+  const bool has_cp = OP != kOpScatter || !p.tma_rows;
+  const bool has_tma = OP != kOpDweight || p.tma_rows;
+  const int readers = has_cp ? kEpiWarps : kProdWarps + kEpiWarps;      // read-out warps: producers with nothing to gather join
+  const uint32_t ring0 = epi0 + epi_bytes(!has_cp);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool leader = !PAIR || (blockIdx.x & 1) == 0;
   const int nseg = (p.half + 63) >> 6;
@@ -165,8 +172,6 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
   const uint32_t acc_cols = tmem_cols_for(p.BN);
   const uint32_t tmem_cols = 2u * acc_cols;
   volatile uint32_t* abort_flag = &hdr->abort_flag;
-  const bool has_cp = OP != kOpScatter || !p.tma_rows;
-  const bool has_tma = OP != kOpDweight || p.tma_rows;
 
   if (tid == 0) {
     for (int s = 0; s < kMaxStages; ++s) {
@@ -175,8 +180,10 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&hdr->acc_full[b]), 1);
-      mbar_init(smem_u32(&hdr->acc_empty[b]), PAIR ? 2 * kEpiWarps : kEpiWarps);       // (a pair's: the leader's copy is used)
-      mbar_init(smem_u32(&hdr->ids_full[b]), kIndexWarps * 32);
+      mbar_init(smem_u32(&hdr->acc_empty[b]), PAIR ? 2 * readers : readers);       // (a pair's: the leader's copy is used)
+      mbar_init(smem_u32(&hdr->ids_full[b]), OP == kOpDweight ? kIndexWarps * 32 : 32);
+      mbar_init(smem_u32(&hdr->dst_full[b]), 32);
+      mbar_init(smem_u32(&hdr->dst_empty[b]), readers);
       mbar_init(smem_u32(&hdr->ids_empty[b]), kProdWarps);
     }
     mbar_init(smem_u32(&hdr->drain), 1);
@@ -206,200 +213,185 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
 
   if (hdr->abort_flag != 0u) {
     // fall through to the common exit
-  } else if (warp < kProdWarps) {
+  } else if (warp < kProdWarps && has_cp) {
     // =========================== gather producers ===========================
-    if (has_cp) {
-      const char* Rows = static_cast<const char*>(p.Rows);
-      const int cc = tid & 7, r0 = tid >> 3;
-      const uint32_t rc_dst = static_cast<uint32_t>(r0) * 128u + (static_cast<uint32_t>(cc ^ (r0 & 7)) << 4);
-      const long long pitch_c = static_cast<long long>(p.C) * 2;
-      Cursor at;
-      bool alive = true;
-      auto wait_free = [&]() {             // for the stage at `at`; moves on
-        if (at.round > 0) alive = mbar_wait_all(smem_u32(&hdr->empty[at.slot]), (at.round - 1) & 1, abort_flag, p.status.word);
-        at.next(stages);
+    const char* Rows = static_cast<const char*>(p.Rows);
+    const int cc = tid & 7, r0 = tid >> 3;
+    const uint32_t rc_dst = static_cast<uint32_t>(r0) * 128u + (static_cast<uint32_t>(cc ^ (r0 & 7)) << 4);
+    const long long pitch_c = static_cast<long long>(p.C) * 2;
+    Cursor at;
+    bool alive = true;
+    auto wait_free = [&]() {             // for the stage at `at`; moves on
+      if (at.round > 0) alive = mbar_wait_all(smem_u32(&hdr->empty[at.slot]), (at.round - 1) & 1, abort_flag, p.status.word);
+      at.next(stages);
+    };
+    if constexpr (OP != kOpDweight) {
+      // The index warps keep the rows of two units in shared memory.  A unit's are read one step ahead, before the copies of the
+      // step before it are issued: a read behind a copy waits for it.
+      const uint32_t table = smem0 + kDenseHeader + static_cast<uint32_t>(r0) * 4u;
+      const int units = Walk<OP, PAIR>(p).left, steps = (p.C + kStep - 1) / kStep;
+      int row[4];
+      auto read_rows = [&](int t) {
+        alive = mbar_wait_all(smem_u32(&hdr->ids_full[t & 1]), (t >> 1) & 1, abort_flag, p.status.word);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          asm volatile("ld.shared.b32 %0, [%1];" : "=r"(row[i]) : "r"(table + static_cast<uint32_t>(t & 1) * (kTileM * 4u) + i * 128u) : "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&hdr->ids_empty[t & 1]));
       };
-      if constexpr (OP != kOpDweight) {
-        // The index warps keep the rows of two units in shared memory.  A unit's are read one step ahead, before the copies of the
-        // step before it are issued: a read behind a copy waits for it.
-        const uint32_t table = smem0 + kDenseHeader + static_cast<uint32_t>(r0) * 4u;
-        const int units = Walk<OP, PAIR>(p).left, steps = (p.C + kStep - 1) / kStep;
-        int row[4];
-        auto read_rows = [&](int t) {
-          alive = mbar_wait_all(smem_u32(&hdr->ids_full[t & 1]), (t >> 1) & 1, abort_flag, p.status.word);
+      if (units > 0) read_rows(0);
+      for (int t = 0; t < units && alive; ++t) {
+        const char* src[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(row[i]) : "r"(table + static_cast<uint32_t>(t & 1) * (kTileM * 4u) + i * 128u) : "memory");
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&hdr->ids_empty[t & 1]));
+        for (int i = 0; i < 4; ++i) src[i] = row[i] >= 0 ? Rows + static_cast<long long>(row[i]) * pitch_c + cc * 16 : nullptr;
+        for (int k = 0; k < steps; ++k) {
+          const int slot = at.slot;
+          wait_free();
+          if (alive && k + 1 == steps && t + 1 < units) read_rows(t + 1);
+          if (!alive) break;
+          const uint32_t base = ring0 + static_cast<uint32_t>(slot) * stage_bytes + rc_dst;
+          const bool kvalid = k * kStep + cc * 8 < p.C;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const bool v = kvalid && src[i];
+            cp_async16(base + i * 4096u, v ? src[i] : Rows, v ? 16u : 0u);
+            if (src[i]) src[i] += 128;
+          }
+          cp_async_mbar_arrive_noinc(smem_u32(&hdr->full[slot]));
+        }
+      }
+    } else {
+      // A 64-row tile is walked with a fixed 16-byte chunk per thread: 16 threads per row of the 128-wide operand (4 rows per
+      // thread, 16 apart), 4 * RN threads per row of the BN-wide one (RN rows per thread).  Rows are whole multiples of eight
+      // apart, so the swizzle of a thread's chunk is the same in all of them.  A warp must not spend more than some 60
+      // instructions on a step (two producer warps share a scheduler, and a step is 500-1000 clocks): the counts are template
+      // parameters, the products 32-bit.  Generic loops took 390 instructions and twice the kernel's time.
+      // The index warps keep the token (and slot) rows of two batches of kBatch contraction rows in shared memory.  A step's ids
+      // are read one step ahead, before the copies of the step before it are issued: a read behind a copy waits for it.
+      auto run = [&](auto rn_tag, auto swap_tag, auto tma_tag) {
+        constexpr int RN = decltype(rn_tag)::value, kBatchSteps = kBatch / kStep;
+        constexpr bool SWAP = decltype(swap_tag)::value, TMA = decltype(tma_tag)::value;
+        constexpr int RG = SWAP ? RN : 4, RS = SWAP ? 4 : RN;                      // rows per thread: gathered, slot operand
+        constexpr int TN = 4 * RN;                                                 // threads per row of the BN-wide operand
+        const int m_c = tid & 15, m_r = tid >> 4, n_c = tid & (TN - 1), n_r = tid / TN;
+        const bool n_on = n_c * 8 < p.half;
+        const int g_c = SWAP ? n_c : m_c, g_r = SWAP ? n_r : m_r, s_c = SWAP ? m_c : n_c, s_r = SWAP ? m_r : n_r;
+        const bool g_on = !SWAP || n_on, s_on = !TMA && (SWAP || n_on);
+        constexpr uint32_t GSTEP = kStep / RG, SSTEP = kStep / RS;                 // rows from one of a thread's copies to the next
+        const uint32_t g_dst = ring0 + (SWAP ? kMTile : 0u) + static_cast<uint32_t>(g_c >> 3) * kSeg + g_r * 128u + (((g_c & 7) ^ (g_r & 7)) << 4);
+        const uint32_t s_dst = ring0 + (SWAP ? 0u : kMTile) + static_cast<uint32_t>(s_c >> 3) * kSeg + s_r * 128u + (((s_c & 7) ^ (s_r & 7)) << 4);
+        const unsigned g_pitch = static_cast<unsigned>(SWAP ? p.N : p.C) * 2u, s_pitch = static_cast<unsigned>(SWAP ? p.C : p.N) * 2u;
+        const uint32_t table = smem0 + kDenseHeader;                               // [2][token][kBatch], then [2][slot][kBatch]
+        auto get = [](uint32_t a) -> int {
+          int v;
+          asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+          return v;
         };
-        if (units > 0) read_rows(0);
-        for (int t = 0; t < units && alive; ++t) {
-          const char* src[4];
+        int tg[RG], ts[RS];
+        auto read_ids = [&](uint32_t at) {             // the ids of one step: its first entry in the token table
 #pragma unroll
-          for (int i = 0; i < 4; ++i) src[i] = row[i] >= 0 ? Rows + static_cast<long long>(row[i]) * pitch_c + cc * 16 : nullptr;
+          for (int j = 0; j < RG; ++j) tg[j] = get(at + (g_r + j * GSTEP) * 4u);
+          if (!TMA) {
+#pragma unroll
+            for (int j = 0; j < RS; ++j) ts[j] = get(at + 2u * kBatch * 4u + (s_r + j * SSTEP) * 4u);
+          }
+        };
+        int batch = 0;                                                             // batches begun by this CTA
+        Walk<OP, PAIR> u(p);
+        if (u.left > 0) {
+          alive = mbar_wait_all(smem_u32(&hdr->ids_full[0]), 0u, abort_flag, p.status.word);
+          read_ids(table);
+        }
+        for (; u.left > 0 && alive; u.next()) {
+          const int steps = u.steps();
+          const int nc0 = u.first_column();
+          const int f0 = (SWAP ? nc0 : u.m0) + g_c * 8, s0 = (SWAP ? u.m0 : nc0) + s_c * 8;       // first feature of the chunk
+          const bool g_in = f0 < (SWAP ? p.N : p.C), s_in = s0 < (SWAP ? p.C : p.N);
+          const char* g_col = Rows + (g_in ? static_cast<long long>(f0) * 2 : 0ll);
+          const char* s_col = static_cast<const char*>(p.Slot) + (s_in ? static_cast<long long>(s0) * 2 : 0ll);
           for (int k = 0; k < steps; ++k) {
             const int slot = at.slot;
             wait_free();
-            if (alive && k + 1 == steps && t + 1 < units) read_rows(t + 1);
             if (!alive) break;
-            const uint32_t base = ring0 + static_cast<uint32_t>(slot) * stage_bytes + rc_dst;
-            const bool kvalid = k * kStep + cc * 8 < p.C;
+            int cg[RG], cs[RS];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const bool v = kvalid && src[i];
-              cp_async16(base + i * 4096u, v ? src[i] : Rows, v ? 16u : 0u);
-              if (src[i]) src[i] += 128;
+            for (int j = 0; j < RG; ++j) cg[j] = tg[j];
+            if (!TMA) {
+#pragma unroll
+              for (int j = 0; j < RS; ++j) cs[j] = ts[j];
+            }
+            const bool unit_end = k + 1 == steps;
+            if (!unit_end && (k + 1) % kBatchSteps != 0) {
+              read_ids(table + static_cast<uint32_t>(batch & 1) * (kBatch * 4u) + static_cast<uint32_t>((k + 1) % kBatchSteps) * (kStep * 4u));
+            } else {                                   // the next batch: of this unit or of the next one
+              __syncwarp();
+              if (lane == 0) mbar_arrive(smem_u32(&hdr->ids_empty[batch & 1]));    // this warp has read the batch
+              ++batch;
+              if (!unit_end || u.left > 1) {
+                alive = mbar_wait_all(smem_u32(&hdr->ids_full[batch & 1]), (batch >> 1) & 1, abort_flag, p.status.word);
+                if (!alive) break;
+                read_ids(table + static_cast<uint32_t>(batch & 1) * (kBatch * 4u));
+              }
+            }
+            const uint32_t base = static_cast<uint32_t>(slot) * stage_bytes;
+            if (g_on && (RG > 1 || g_r < kStep)) {
+#pragma unroll
+              for (int j = 0; j < RG; ++j)
+                cp_async16(base + g_dst + j * GSTEP * 128u, g_col + static_cast<unsigned long long>(static_cast<unsigned>(max(cg[j], 0))) * g_pitch,
+                           (g_in && cg[j] >= 0) ? 16u : 0u);
+            }
+            if (s_on && (RS > 1 || s_r < kStep)) {
+#pragma unroll
+              for (int j = 0; j < RS; ++j)
+                cp_async16(base + s_dst + j * SSTEP * 128u, s_col + static_cast<unsigned long long>(static_cast<unsigned>(max(cs[j], 0))) * s_pitch,
+                           (s_in && cs[j] >= 0) ? 16u : 0u);
             }
             cp_async_mbar_arrive_noinc(smem_u32(&hdr->full[slot]));
           }
         }
+      };
+      auto pick_rn = [&](auto swap_tag, auto tma_tag) {
+        if (p.half > 128) run(std::integral_constant<int, 8>{}, swap_tag, tma_tag);
+        else if (p.half > 64) run(std::integral_constant<int, 4>{}, swap_tag, tma_tag);
+        else if (p.half > 32) run(std::integral_constant<int, 2>{}, swap_tag, tma_tag);
+        else run(std::integral_constant<int, 1>{}, swap_tag, tma_tag);
+      };
+      if (p.swap) {
+        if (p.tma_rows) pick_rn(std::true_type{}, std::true_type{});
+        else pick_rn(std::true_type{}, std::false_type{});
       } else {
-        // A 64-row tile is walked with a fixed 16-byte chunk per thread: 16 threads per row of the 128-wide operand (4 rows per
-        // thread, 16 apart), 4 * RN threads per row of the BN-wide one (RN rows per thread).  Rows are whole multiples of eight
-        // apart, so the swizzle of a thread's chunk is the same in all of them.  A warp must not spend more than some 60
-        // instructions on a step (two producer warps share a scheduler, and a step is 500-1000 clocks): the counts are template
-        // parameters, the products 32-bit.  Generic loops took 390 instructions and twice the kernel's time.
-        // The index warps keep the token (and slot) rows of two batches of kBatch contraction rows in shared memory.  A step's ids
-        // are read one step ahead, before the copies of the step before it are issued: a read behind a copy waits for it.
-        auto run = [&](auto rn_tag, auto swap_tag, auto tma_tag) {
-          constexpr int RN = decltype(rn_tag)::value, kBatchSteps = kBatch / kStep;
-          constexpr bool SWAP = decltype(swap_tag)::value, TMA = decltype(tma_tag)::value;
-          constexpr int RG = SWAP ? RN : 4, RS = SWAP ? 4 : RN;                      // rows per thread: gathered, slot operand
-          constexpr int TN = 4 * RN;                                                 // threads per row of the BN-wide operand
-          const int m_c = tid & 15, m_r = tid >> 4, n_c = tid & (TN - 1), n_r = tid / TN;
-          const bool n_on = n_c * 8 < p.half;
-          const int g_c = SWAP ? n_c : m_c, g_r = SWAP ? n_r : m_r, s_c = SWAP ? m_c : n_c, s_r = SWAP ? m_r : n_r;
-          const bool g_on = !SWAP || n_on, s_on = !TMA && (SWAP || n_on);
-          constexpr uint32_t GSTEP = kStep / RG, SSTEP = kStep / RS;                 // rows from one of a thread's copies to the next
-          const uint32_t g_dst = ring0 + (SWAP ? kMTile : 0u) + static_cast<uint32_t>(g_c >> 3) * kSeg + g_r * 128u + (((g_c & 7) ^ (g_r & 7)) << 4);
-          const uint32_t s_dst = ring0 + (SWAP ? 0u : kMTile) + static_cast<uint32_t>(s_c >> 3) * kSeg + s_r * 128u + (((s_c & 7) ^ (s_r & 7)) << 4);
-          const unsigned g_pitch = static_cast<unsigned>(SWAP ? p.N : p.C) * 2u, s_pitch = static_cast<unsigned>(SWAP ? p.C : p.N) * 2u;
-          const uint32_t table = smem0 + kDenseHeader;                               // [2][token][kBatch], then [2][slot][kBatch]
-          auto get = [](uint32_t a) -> int {
-            int v;
-            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-            return v;
-          };
-          int tg[RG], ts[RS];
-          auto read_ids = [&](uint32_t at) {             // the ids of one step: its first entry in the token table
-#pragma unroll
-            for (int j = 0; j < RG; ++j) tg[j] = get(at + (g_r + j * GSTEP) * 4u);
-            if (!TMA) {
-#pragma unroll
-              for (int j = 0; j < RS; ++j) ts[j] = get(at + 2u * kBatch * 4u + (s_r + j * SSTEP) * 4u);
-            }
-          };
-          int batch = 0;                                                             // batches begun by this CTA
-          Walk<OP, PAIR> u(p);
-          if (u.left > 0) {
-            alive = mbar_wait_all(smem_u32(&hdr->ids_full[0]), 0u, abort_flag, p.status.word);
-            read_ids(table);
-          }
-          for (; u.left > 0 && alive; u.next()) {
-            const int steps = u.steps();
-            const int nc0 = u.first_column();
-            const int f0 = (SWAP ? nc0 : u.m0) + g_c * 8, s0 = (SWAP ? u.m0 : nc0) + s_c * 8;       // first feature of the chunk
-            const bool g_in = f0 < (SWAP ? p.N : p.C), s_in = s0 < (SWAP ? p.C : p.N);
-            const char* g_col = Rows + (g_in ? static_cast<long long>(f0) * 2 : 0ll);
-            const char* s_col = static_cast<const char*>(p.Slot) + (s_in ? static_cast<long long>(s0) * 2 : 0ll);
-            for (int k = 0; k < steps; ++k) {
-              const int slot = at.slot;
-              wait_free();
-              if (!alive) break;
-              int cg[RG], cs[RS];
-#pragma unroll
-              for (int j = 0; j < RG; ++j) cg[j] = tg[j];
-              if (!TMA) {
-#pragma unroll
-                for (int j = 0; j < RS; ++j) cs[j] = ts[j];
-              }
-              const bool unit_end = k + 1 == steps;
-              if (!unit_end && (k + 1) % kBatchSteps != 0) {
-                read_ids(table + static_cast<uint32_t>(batch & 1) * (kBatch * 4u) + static_cast<uint32_t>((k + 1) % kBatchSteps) * (kStep * 4u));
-              } else {                                   // the next batch: of this unit or of the next one
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&hdr->ids_empty[batch & 1]));    // this warp has read the batch
-                ++batch;
-                if (!unit_end || u.left > 1) {
-                  alive = mbar_wait_all(smem_u32(&hdr->ids_full[batch & 1]), (batch >> 1) & 1, abort_flag, p.status.word);
-                  if (!alive) break;
-                  read_ids(table + static_cast<uint32_t>(batch & 1) * (kBatch * 4u));
-                }
-              }
-              const uint32_t base = static_cast<uint32_t>(slot) * stage_bytes;
-              if (g_on && (RG > 1 || g_r < kStep)) {
-#pragma unroll
-                for (int j = 0; j < RG; ++j)
-                  cp_async16(base + g_dst + j * GSTEP * 128u, g_col + static_cast<unsigned long long>(static_cast<unsigned>(max(cg[j], 0))) * g_pitch,
-                             (g_in && cg[j] >= 0) ? 16u : 0u);
-              }
-              if (s_on && (RS > 1 || s_r < kStep)) {
-#pragma unroll
-                for (int j = 0; j < RS; ++j)
-                  cp_async16(base + s_dst + j * SSTEP * 128u, s_col + static_cast<unsigned long long>(static_cast<unsigned>(max(cs[j], 0))) * s_pitch,
-                             (s_in && cs[j] >= 0) ? 16u : 0u);
-              }
-              cp_async_mbar_arrive_noinc(smem_u32(&hdr->full[slot]));
-            }
-          }
-        };
-        auto pick_rn = [&](auto swap_tag, auto tma_tag) {
-          if (p.half > 128) run(std::integral_constant<int, 8>{}, swap_tag, tma_tag);
-          else if (p.half > 64) run(std::integral_constant<int, 4>{}, swap_tag, tma_tag);
-          else if (p.half > 32) run(std::integral_constant<int, 2>{}, swap_tag, tma_tag);
-          else run(std::integral_constant<int, 1>{}, swap_tag, tma_tag);
-        };
-        if (p.swap) {
-          if (p.tma_rows) pick_rn(std::true_type{}, std::true_type{});
-          else pick_rn(std::true_type{}, std::false_type{});
-        } else {
-          if (p.tma_rows) pick_rn(std::false_type{}, std::true_type{});
-          else pick_rn(std::false_type{}, std::false_type{});
-        }
+        if (p.tma_rows) pick_rn(std::false_type{}, std::true_type{});
+        else pick_rn(std::false_type{}, std::false_type{});
       }
-      cp_async_wait_all();
     }
+    cp_async_wait_all();
   } else if (warp < kMmaWarp) {
     // =========================== read-out ===========================
-    const int ew = warp - kProdWarps;
-    const int lg = ew & 3, half = ew >> 2;               // TMEM lane group, share of the column blocks
+    const int ew = warp >= kProdWarps ? warp - kProdWarps : warp + kEpiWarps;
+    const int lg = ew & 3, share = ew >> 2, shares = readers >> 2;       // TMEM lane group (warp number mod 4), share of the column blocks
     const uint32_t area = epi0 + static_cast<uint32_t>(ew) * 4096u;
     const uint32_t lane_base = static_cast<uint32_t>(lg * 32) << 16;
     T* out = static_cast<T*>(p.Out);
     bool alive = true;
-    pdl_wait();                                          // planning flags, zeros the results are added to
-    // G, S: destination of tile row lg * 32 + lane of the next unit - token id, slot, planning flag - loaded a unit ahead
-    long long next_t = 0;
-    int next_slot = -1, next_b = 0, next_flag = 0;
-    Walk<OP, PAIR> u(p), ahead(p);
-    auto look_up = [&]() {
-      if (OP == kOpDweight || ahead.left <= 0) return;
-      const int m = ahead.m0 + lg * 32 + lane;
-      next_slot = -1;
-      next_flag = 0;
-      if (m < p.M) {
-        next_b = m / p.K;
-        next_slot = (next_b * p.E + ahead.e) * p.K + (m - next_b * p.K);
-        next_t = load_index(p.Ind, p.index_dtype, next_slot);
-        if (OP == kOpScatter) next_flag = p.plan[next_b];
-      }
-      ahead.next();
-    };
-    look_up();
-    for (int t = 0; u.left > 0 && alive; u.next(), ++t) {
+    pdl_wait();                                          // zeros the results are added to
+    int t = 0;
+    for (Walk<OP, PAIR> u(p); u.left > 0 && alive; u.next(), ++t) {
       const int bn = min(p.BN, p.N - u.n0);              // columns of this tile (a multiple of 8)
       const int n_end = u.n0 + bn;
       int my_ro = -1;                                    // G, S: destination row of tile row lg * 32 + lane
       uint32_t to_f32 = 0u;
       if (OP != kOpDweight) {
-        if (next_slot >= 0) {
-          const bool ok = next_t >= 0 && next_t < p.T;
-          if (!ok && half == 0 && u.n0 == 0) p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
-          my_ro = OP == kOpGather ? next_slot : (ok ? next_b * p.T + static_cast<int>(next_t) : -1);
+        alive = mbar_wait_all(smem_u32(&hdr->dst_full[t & 1]), (t >> 1) & 1, abort_flag, p.status.word);
+        if (!alive) break;
+        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(my_ro)
+                     : "r"(smem0 + kDenseHeader + static_cast<uint32_t>((2 + (t & 1)) * kTileM + lg * 32 + lane) * 4u) : "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&hdr->dst_empty[t & 1]));
+        if (OP == kOpScatter) {
+          to_f32 = __ballot_sync(0xffffffffu, my_ro < 0);
+          my_ro &= 0x7fffffff;
         }
-        if (OP == kOpScatter) to_f32 = __ballot_sync(0xffffffffu, next_flag != 0);
-        look_up();
+        if (my_ro == kNoRow) my_ro = -1;
       }
       const T* bias_row = (OP != kOpDweight && p.bias) ? static_cast<const T*>(p.bias) + static_cast<long long>(u.e) * p.N + u.n0 : nullptr;
       const int buf = t & 1;
@@ -412,7 +404,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
         // 64 columns = 128 bytes of a 16-bit row at a time, eight lanes to a row: S adds 16 bytes a lane (the memory system takes
         // 39 KB a microsecond from an SM that way).  Bulk reductions of 128 bytes, one per row and lane, took 85 clocks each to
         // issue: 9000 clocks a 128 x 256 tile against 3800 of a contraction of 256.
-        for (int c = half; c * 64 < bn; c += 2) {
+        for (int c = share; c * 64 < bn; c += shares) {
           const uint32_t srow = area + static_cast<uint32_t>(lane) * 128u;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
@@ -462,7 +454,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           }
         }
       } else {
-        for (int c = half; c * 32 < bn; c += 2) {
+        for (int c = share; c * 32 < bn; c += shares) {
           const int col0 = u.n0 + c * 32;
           uint32_t v[32];
           tmem_ld32(acc + static_cast<uint32_t>(c * 32), v);
@@ -560,25 +552,40 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     const int it = tid - kIndexWarp * 32;
     bool alive = true;
     if constexpr (OP != kOpDweight) {
+      // the first warp: where the producers find the rows; the second: where the read-out puts them
+      const bool dst = warp != kIndexWarp;
+      unsigned long long* full = dst ? hdr->dst_full : hdr->ids_full;
+      unsigned long long* empty = dst ? hdr->dst_empty : hdr->ids_empty;
+      if (dst && OP == kOpScatter) pdl_wait();           // planning flags
       int t = 0;
-      for (Walk<OP, PAIR> u(p); has_cp && u.left > 0 && alive; u.next(), ++t) {
-        int row[2], b[2];
-        long long id[2];
+      for (Walk<OP, PAIR> u(p); (dst || has_cp) && u.left > 0 && alive; u.next(), ++t) {
+        int row[4], b[4], f32[4];
+        long long id[4];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const int m = u.m0 + it + 64 * i;
+        for (int i = 0; i < 4; ++i) {
+          const int m = u.m0 + lane + 32 * i;
           b[i] = m / p.K;
           row[i] = m < p.M ? (b[i] * p.E + u.e) * p.K + (m - b[i] * p.K) : -1;
-          id[i] = (OP == kOpGather && row[i] >= 0) ? load_index(p.Ind, p.index_dtype, row[i]) : 0;
+          id[i] = (row[i] >= 0 && (dst || OP == kOpGather)) ? load_index(p.Ind, p.index_dtype, row[i]) : 0;
+          f32[i] = (OP == kOpScatter && dst && row[i] >= 0) ? p.plan[b[i]] : 0;
         }
-        if (t >= 2) alive = mbar_wait_all(smem_u32(&hdr->ids_empty[t & 1]), ((t >> 1) - 1) & 1, abort_flag, p.status.word);
+        if (t >= 2) alive = mbar_wait_all(smem_u32(&empty[t & 1]), ((t >> 1) - 1) & 1, abort_flag, p.status.word);
         if (!alive) break;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          if (OP == kOpGather) row[i] = (row[i] >= 0 && id[i] >= 0 && id[i] < p.T) ? b[i] * p.T + static_cast<int>(id[i]) : -1;
-          asm volatile("st.shared.b32 [%0], %1;" ::"r"(table + static_cast<uint32_t>(t & 1) * (kTileM * 4u) + static_cast<uint32_t>(it + 64 * i) * 4u), "r"(row[i]) : "memory");
+        for (int i = 0; i < 4; ++i) {
+          const bool known = row[i] >= 0 && id[i] >= 0 && id[i] < p.T;
+          const int token_row = b[i] * p.T + static_cast<int>(id[i]);
+          int v;
+          if (!dst) {
+            v = OP == kOpScatter ? row[i] : (known ? token_row : -1);
+          } else {
+            if (row[i] >= 0 && !known && u.n0 == 0) p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
+            if (OP == kOpGather) v = row[i] >= 0 ? row[i] : kNoRow;
+            else v = known ? (f32[i] ? static_cast<int>(static_cast<unsigned>(token_row) | 0x80000000u) : token_row) : kNoRow;
+          }
+          asm volatile("st.shared.b32 [%0], %1;" ::"r"(table + static_cast<uint32_t>(((dst ? 2 : 0) + (t & 1)) * kTileM + lane + 32 * i) * 4u), "r"(v) : "memory");
         }
-        mbar_arrive(smem_u32(&hdr->ids_full[t & 1]));
+        mbar_arrive(smem_u32(&full[t & 1]));
       }
     } else {
       constexpr int kPer = kBatch / (kIndexWarps * 32);
@@ -743,7 +750,7 @@ int ring_stages(int half, bool nc_tile, uint32_t not_ring) {
 template <typename T, int OP, bool PAIR>
 cudaError_t launch(const DenseParams& p, const TensorMap3& mw, const TensorMap3& mr, bool after_own, cudaStream_t st) {
   const size_t n_bytes = (OP != kOpDweight && p.nc) ? static_cast<size_t>(p.half) * 128 : static_cast<size_t>((p.half + 63) / 64) * kSeg;
-  const size_t smem = kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : kRowTable) + kEpi +
+  const size_t smem = kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : kRowTable) + epi_bytes(OP == kOpScatter && p.tma_rows) +
                       p.stages * (kMTile + n_bytes);
   cudaError_t err = ensure_smem_optin<dense16_kernel<T, OP, PAIR>>(static_cast<int>(kSmemMax));
   if (err != cudaSuccess) return err;
@@ -766,7 +773,7 @@ void configure_dense16_rowgemm(RowGemmParams& p, bool scatter) {
   p.BN = t.bn;
   p.pair = t.pair ? 1 : 0;
   p.bulk_epilogue = scatter ? 1 : 0;
-  p.stages = ring_stages(p.pair ? p.BN / 2 : p.BN, p.w_layout == EGS_W_NC, kRowTable + kEpi);
+  p.stages = ring_stages(p.pair ? p.BN / 2 : p.BN, p.w_layout == EGS_W_NC, kRowTable + epi_bytes(!cp_rows));
   p.row_tiles = 2;        // two 128-row accumulators per CTA
   p.persistent = (scatter && steps <= 4) ? 1 : 0;        // (for egs_describe_plan) the additions outlast the contraction
 }
@@ -832,7 +839,7 @@ void configure_dense16_dweight(DWeightParams& p) {
       }
     }
   }
-  p.stages = ring_stages(p.pair ? p.BN / 2 : p.BN, false, table_bytes(slot_cp) + kEpi);
+  p.stages = ring_stages(p.pair ? p.BN / 2 : p.BN, false, table_bytes(slot_cp) + epi_bytes(false));
   p.row_tiles = 2;        // two 128-row accumulators per CTA
 }
 
