@@ -399,6 +399,16 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       if (!alive) break;
       tc_fence_after();
       const uint32_t acc = tmem_base + lane_base + static_cast<uint32_t>(buf) * acc_cols;
+      bool released = false;
+      auto release = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (PAIR) mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(&hdr->acc_empty[buf]), 0));
+          else mbar_arrive(smem_u32(&hdr->acc_empty[buf]));
+        }
+        released = true;
+      };
       const bool packed = OP == kOpGather || (OP == kOpScatter && to_f32 == 0u) || (OP == kOpDweight && p.splits == 1 && p.lane_rows);
       if (packed) {
         // 64 columns = 128 bytes of a 16-bit row at a time, eight lanes to a row: S adds 16 bytes a lane (the memory system takes
@@ -424,6 +434,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
               }
             }
           }
+          if ((c + shares) * 64 >= bn) release();        // the accumulator has been read: the next tile but one may begin
           const int col0 = u.n0 + c * 64;
           __syncwarp();
           const int j = lane & 7, col = col0 + j * 8;
@@ -487,12 +498,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           }
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        if (PAIR) mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(&hdr->acc_empty[buf]), 0));
-        else mbar_arrive(smem_u32(&hdr->acc_empty[buf]));
-      }
+      if (!released) release();
     }
   } else if (warp == kMmaWarp) {
     // =========================== MMA issuer ===========================
@@ -705,33 +711,36 @@ bool encode_slot_rows(TensorMap3* map, const void* base, int B, int E, int K, in
   return encode_tensor_map_16bit(map, base, 4, dims, box);
 }
 
-// One CTA per tile of 128 x BN or a pair of CTAs per tile of 256 x BN, and BN.  Per step a CTA's shared memory moves
-// 2 * (128 + columns it stages) * 128 bytes at 128 bytes per clock and the tensor core multiplies BN columns in 2 * BN clocks; the
-// load/store unit needs lsu0 + lsu1 * (columns staged) clocks for its share of the copies; read-out takes epi clocks per column
-// (counted in blocks of `block` columns) beside the next tile's main loop; units go out in waves of one per SM or pair of SMs.
+// One CTA per tile of 128 x BN or a pair of CTAs per tile of 256 x BN, and BN, by clocks.  A step writes and reads 128 + `staged`
+// rows of 128 bytes of a CTA's shared memory, 2 clocks a row at 128 bytes a clock (measured: 2.0 in pairs, 2.4 on single CTAs, 2.6 for
+// their scatters), the tensor core multiplies BN columns in 2 * BN clocks, the load/store unit needs lsu0 + lsu1 * staged for its
+// share of the copies, and the barriers of a step take 600 (800 in a scatter that gathers its rows).  Read-out takes epi clocks a
+// column beside the next tile's main loop; the additions of a scatter share the way to the L2 with the loads, and half of the shorter
+// one shows.  Units go out in waves of one per SM or pair of SMs; a pair starts and ends 2500 clocks slower.
 struct Tile {
   int bn = 256;
   bool pair = false;
   double cost = 1e30;
 };
-Tile pick_tile(int n, int m, long long groups, int steps, double lsu0, double lsu1, double epi, int block, bool may_pair) {
+Tile pick_tile(int n, int m, long long groups, int steps, double lsu0, double lsu1, double epi, bool scatter) {
   Tile best;
-  for (int pair = 0; pair <= (may_pair ? 1 : 0); ++pair) {
+  for (int pair = 0; pair < 2; ++pair) {
     const int rows = pair ? 2 * kTileM : kTileM, sms = pair ? kSms / 2 : kSms, unit16 = pair ? 32 : 16;
+    const double per_row = pair ? 2.0 : scatter ? 2.6 : 2.4, least = scatter && lsu0 > 0.0 ? 800.0 : 600.0;
     const long long row_units = (m + rows - 1) / rows * groups;
     const int top = n < 256 ? (n + unit16 - 1) / unit16 * unit16 : 256;
     for (int bn = top; bn >= unit16; bn -= unit16) {
       const long long tiles = (n + bn - 1) / bn;
       const long long units = row_units * tiles, waves = (units + sms - 1) / sms;
       const int staged = pair ? bn / 2 : bn;
-      double step = 2.0 * (128 + staged);
+      double step = per_row * (128 + staged);
       if (2.0 * bn > step) step = 2.0 * bn;
       if (lsu0 + lsu1 * staged > step) step = lsu0 + lsu1 * staged;
-      double unit = steps * step;
-      const double out = epi * ((bn + block - 1) / block * block);
-      if (out > unit) unit = out;
-      const double cost = waves * (unit + 1000) + out;
-      if (cost < best.cost * (pair && !best.pair ? 0.95 : 0.98)) {
+      if (step < least) step = least;
+      const double loop = steps * step, out = epi * bn;
+      const double unit = (loop > out ? loop : out) + (scatter ? 0.5 * (loop > out ? out : loop) : 0.0);
+      const double cost = waves * (unit + 1000) + out + (pair ? 2500 : 0);
+      if (cost < best.cost * (pair && !best.pair ? 0.97 : 0.98)) {
         best.bn = bn;
         best.pair = pair != 0;
         best.cost = cost;
@@ -769,7 +778,7 @@ cudaError_t launch_typed(const DenseParams& p, int dtype, const TensorMap3& mw, 
 void configure_dense16_rowgemm(RowGemmParams& p, bool scatter) {
   const int steps = (p.C + kStep - 1) / kStep;
   const bool cp_rows = !scatter || !rows_fit_boxes(p.K, 128);
-  const Tile t = pick_tile(p.N, p.M, p.E, steps, cp_rows ? 340.0 : 0.0, 0.0, 16.0, 1, true);
+  const Tile t = pick_tile(p.N, p.M, p.E, steps, cp_rows ? 340.0 : 0.0, 0.0, 16.0, scatter);
   p.BN = t.bn;
   p.pair = t.pair ? 1 : 0;
   p.bulk_epilogue = scatter ? 1 : 0;
@@ -825,7 +834,7 @@ void configure_dense16_dweight(DWeightParams& p) {
       const long long sp_steps = (steps_all + s - 1) / s;
       const long long real = (steps_all + sp_steps - 1) / sp_steps;      // ranges of whole steps
       const double epi = real > 1 ? 32.0 : o == 0 ? 16.0 : 20.0;         // (partial tiles are added atomically)
-      const Tile t = pick_tile(nf, mf, p.E * real, static_cast<int>(sp_steps), lsu0, lsu1, epi, 1, true);
+      const Tile t = pick_tile(nf, mf, p.E * real, static_cast<int>(sp_steps), lsu0, lsu1, epi, false);
       double cost = t.cost;
       // more than one range: zero fill and rounding of the float32 sums, two launches and 10 bytes an element
       if (real > 1) cost += 9000 + static_cast<double>(p.E) * p.FG * p.FD * 10 / (148 * 20.0);
