@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(StrictParams 
     for (int g = 0; g < total && alive; ++g) {
       cp_async_wait_pending(dist - 1);
       if (g >= kLoStages) {
-        alive = mbar_wait_warp(smem_u32(&hdr->empty[eslot]), eround & 1, abort_flag, p.status.word, lane);
+        alive = mbar_wait_all(smem_u32(&hdr->empty[eslot]), eround & 1, abort_flag, p.status.word);
         if (!alive) break;
         if (++eslot == raw) { eslot = 0; ++eround; }
       }
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(StrictParams 
       const int nblk = (bn + 31) >> 5;
       for (int ch = 0; ch < chunks && alive; ++ch, ++t) {
         const int buf = t & 1;
-        alive = mbar_wait_warp(smem_u32(&hdr->acc_full[buf]), (t >> 1) & 1, abort_flag, p.status.word, lane);
+        alive = mbar_wait_all(smem_u32(&hdr->acc_full[buf]), (t >> 1) & 1, abort_flag, p.status.word);
         if (!alive) break;
         tc_fence_after();
         const uint32_t acc = tmem_base + lane_base + static_cast<uint32_t>(buf) * acc_cols;
@@ -436,56 +436,54 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(StrictParams 
     }
   } else {
     // =========================== MMA issuer ===========================
-    if (lane == 0) {
-      // A: K-major rows (G, S) or rows = contraction (D); B: rows = n (weights [n][contraction]) or rows = contraction
-      const bool a_mn = OP == kOpDweight, b_mn = OP == kOpDweight || !p.nc;
-      const uint32_t a_lbo = a_mn ? kStepElems * 128u : 16u, a_sbo = a_mn ? 512u : 1024u, a_lay = a_mn ? kSwizzle128Base32 : kSwizzle128;
-      const uint32_t b_lbo = b_mn ? kStepElems * 128u : 16u, b_sbo = b_mn ? 512u : 1024u, b_lay = b_mn ? kSwizzle128Base32 : kSwizzle128;
-      const uint64_t a_adv = (a_mn ? 8u * 128u : 32u) >> 4, b_adv = (b_mn ? 8u * 128u : 32u) >> 4;
-      bool ok = true;
-      int t = 0, slot = 0, round = 0, lo = 0;
-      for (int un = blockIdx.x; un < p.units && ok; un += gridDim.x) {
-        const Unit u = unit_of<OP>(p, un);
-        const int steps = unit_steps<OP>(p, u);
-        const int bn = min(p.BN, ((p.N - u.n0) + 15) & ~15);
-        const uint32_t idesc = make_idesc(2u, a_mn ? 1u : 0u, b_mn ? 1u : 0u, kTileM, static_cast<uint32_t>(bn));
-        int len = steps;                                  // contraction elements of the unit (rows for D)
-        if (OP == kOpDweight) len = min(p.rows_per_split, p.M - u.split * p.rows_per_split);
-        else len = p.C;
-        for (int ks = 0; ks < steps && ok; ++ks) {
-          const bool first = OP == kOpDweight ? ks == 0 : ks % kChunkSteps == 0;
-          const bool last = ks == steps - 1 || (OP != kOpDweight && ks % kChunkSteps == kChunkSteps - 1);
-          const int buf = t & 1;
-          if (first && t >= 2) {
-            ok = mbar_wait(smem_u32(&hdr->acc_empty[buf]), ((t >> 1) - 1) & 1, abort_flag, p.status.word);
-            if (!ok) break;
-            tc_fence_after();
-          }
-          ok = mbar_wait(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status.word);
+    // (the warp runs converged and an elected lane issues, see mbar_wait_all: twelve MMAs from a lane on its own took 1000 clocks)
+    // A: K-major rows (G, S) or rows = contraction (D); B: rows = n (weights [n][contraction]) or rows = contraction
+    const bool a_mn = OP == kOpDweight, b_mn = OP == kOpDweight || !p.nc;
+    const uint32_t a_lbo = a_mn ? kStepElems * 128u : 16u, a_sbo = a_mn ? 512u : 1024u, a_lay = a_mn ? kSwizzle128Base32 : kSwizzle128;
+    const uint32_t b_lbo = b_mn ? kStepElems * 128u : 16u, b_sbo = b_mn ? 512u : 1024u, b_lay = b_mn ? kSwizzle128Base32 : kSwizzle128;
+    const uint32_t a_adv = (a_mn ? 8u * 128u : 32u) >> 4, b_adv = (b_mn ? 8u * 128u : 32u) >> 4;
+    const uint64_t a_desc = make_smem_desc(0u, a_lbo, a_sbo, a_lay), b_desc = make_smem_desc(0u, b_lbo, b_sbo, b_lay) + (kATile >> 4);
+    bool ok = true;
+    int t = 0, slot = 0, round = 0, lo = 0;
+    for (int un = blockIdx.x; un < p.units && ok; un += gridDim.x) {
+      const Unit u = unit_of<OP>(p, un);
+      const int steps = unit_steps<OP>(p, u);
+      const int bn = min(p.BN, ((p.N - u.n0) + 15) & ~15);
+      const uint32_t idesc = make_idesc(2u, a_mn ? 1u : 0u, b_mn ? 1u : 0u, kTileM, static_cast<uint32_t>(bn));
+      // contraction elements of the unit (rows for D)
+      const int len = OP == kOpDweight ? min(p.rows_per_split, p.M - u.split * p.rows_per_split) : p.C;
+      for (int ks = 0; ks < steps && ok; ++ks) {
+        const bool first = OP == kOpDweight ? ks == 0 : ks % kChunkSteps == 0;
+        const bool last = ks == steps - 1 || (OP != kOpDweight && ks % kChunkSteps == kChunkSteps - 1);
+        const int buf = t & 1;
+        if (first && t >= 2) {
+          ok = mbar_wait_all(smem_u32(&hdr->acc_empty[buf]), ((t >> 1) - 1) & 1, abort_flag, p.status.word);
           if (!ok) break;
-          tc_fence_after();
-          const uint32_t d = tmem_base + static_cast<uint32_t>(buf) * acc_cols;
-          const uint32_t a_hi = raw0 + static_cast<uint32_t>(slot) * stage_bytes, a_lo = lo0 + static_cast<uint32_t>(lo) * stage_bytes;
-          uint64_t ad = make_smem_desc(a_hi, a_lbo, a_sbo, a_lay), adl = make_smem_desc(a_lo, a_lbo, a_sbo, a_lay);
-          uint64_t bd = make_smem_desc(a_hi + kATile, b_lbo, b_sbo, b_lay), bdl = make_smem_desc(a_lo + kATile, b_lbo, b_sbo, b_lay);
-          const int nkq = min(4, (len - ks * kStepElems + 7) / 8);
-          for (int kq = 0; kq < nkq; ++kq) {
-            umma<true>(d, adl, bd, idesc, (first && kq == 0) ? 0u : 1u);
-            umma<true>(d, ad, bdl, idesc, 1u);
-            umma<true>(d, ad, bd, idesc, 1u);
-            ad += a_adv;
-            adl += a_adv;
-            bd += b_adv;
-            bdl += b_adv;
+        }
+        ok = mbar_wait_all(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status.word);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t d = tmem_base + static_cast<uint32_t>(buf) * acc_cols;
+        // (descriptors: 14 address bits in 16-byte units; shared memory is smaller)
+        const uint32_t hi16 = (raw0 + static_cast<uint32_t>(slot) * stage_bytes) >> 4, lo16 = (lo0 + static_cast<uint32_t>(lo) * stage_bytes) >> 4;
+        const int nkq = min(4, (len - ks * kStepElems + 7) / 8);
+        if (elect_one()) {
+#pragma unroll
+          for (int kq = 0; kq < 4; ++kq) {
+            if (kq < nkq) {
+              const uint64_t ad = a_desc + (hi16 + kq * a_adv), adl = a_desc + (lo16 + kq * a_adv);
+              const uint64_t bd = b_desc + (hi16 + kq * b_adv), bdl = b_desc + (lo16 + kq * b_adv);
+              umma<true>(d, adl, bd, idesc, (first && kq == 0) ? 0u : 1u);
+              umma<true>(d, ad, bdl, idesc, 1u);
+              umma<true>(d, ad, bd, idesc, 1u);
+            }
           }
           umma_commit(smem_u32(&hdr->empty[slot]));
-          if (last) {
-            umma_commit(smem_u32(&hdr->acc_full[buf]));
-            ++t;
-          }
-          lo ^= 1;
-          if (++slot == raw) { slot = 0; ++round; }
+          if (last) umma_commit(smem_u32(&hdr->acc_full[buf]));
         }
+        if (last) ++t;
+        lo ^= 1;
+        if (++slot == raw) { slot = 0; ++round; }
       }
     }
     __syncwarp();
