@@ -212,8 +212,8 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
       configure_dense16_rowgemm(p, scatter);
       err = launch_dense16_rowgemm(p, scatter, dtype, st);
     } else {
-      const size_t smem = configure_tensor_rowgemm(p, scatter, dtype);
-      err = launch_tensor_rowgemm(p, scatter, dtype, smem, st);
+      const size_t smem = configure_tensor_rowgemm(p, scatter);
+      err = launch_tensor_rowgemm(p, scatter, smem, st);
     }
   } else {
     err = launch_generic_rowgemm(p, scatter, dtype, st);
@@ -499,7 +499,7 @@ static int dweight_impl(const void* Xsrc, const void* Ysrc, const void* Ind, voi
   } else if (dense16) {
     configure_dense16_dweight(p);
   } else if (tensor) {
-    smem = configure_tensor_dweight(p, dtype);
+    smem = configure_tensor_dweight(p);
   } else {
     configure_generic_dweight(p);
   }
@@ -519,7 +519,7 @@ static int dweight_impl(const void* Xsrc, const void* Ysrc, const void* Ind, voi
       p.after_own = 1;
     }
   }
-  err = strict ? launch_strict_dweight(p, st) : dense16 ? launch_dense16_dweight(p, dtype, st) : tensor ? launch_tensor_dweight(p, dtype, smem, st) : launch_generic_dweight(p, dtype, st);
+  err = strict ? launch_strict_dweight(p, st) : dense16 ? launch_dense16_dweight(p, dtype, st) : tensor ? launch_tensor_dweight(p, smem, st) : launch_generic_dweight(p, dtype, st);
   if (err != cudaSuccess) return fail_cuda(err, "dweight launch");
   if (p.splits > 1 && dtype != EGS_F32) {
     err = launch_convert_from_f32(p.acc, out, n_out, dtype, st, tensor);   // (the tensor-core kernel triggers its dependents)
@@ -602,7 +602,7 @@ int egs_describe_plan(int op, const egs_dims* dims, int w_layout, int dtype, int
     p.FG = static_cast<int>(d.C); p.FD = static_cast<int>(d.N); p.M = static_cast<int>(d.B * d.K);
     if (dtype != EGS_F32) configure_dense16_dweight(p);
     else if (precision == EGS_PREC_STRICT) configure_strict_dweight(p);
-    else configure_tensor_dweight(p, dtype);
+    else configure_tensor_dweight(p);
     out->tile_n = p.BN; out->stages = p.stages; out->row_tiles = p.row_tiles; out->splits = p.splits;
     out->rows_per_split = p.rows_per_split;
     return EGS_OK;
@@ -614,7 +614,7 @@ int egs_describe_plan(int op, const egs_dims* dims, int w_layout, int dtype, int
   p.expert_fastest = pick_expert_fastest(d, op == 1, dtype);
   if (dtype != EGS_F32) configure_dense16_rowgemm(p, op == 1);
   else if (precision == EGS_PREC_STRICT) configure_strict_rowgemm(p);
-  else configure_tensor_rowgemm(p, op == 1, dtype);
+  else configure_tensor_rowgemm(p, op == 1);
   out->tile_n = p.BN; out->stages = p.stages; out->row_tiles = p.row_tiles; out->persistent = p.persistent;
   out->bulk_epilogue = (p.persistent || op == 1) ? p.bulk_epilogue : 0; out->expert_fastest = p.expert_fastest;
   return EGS_OK;

@@ -473,7 +473,8 @@ Tensor expert_row_sum(const Tensor& Src, const OptTensor& Ind, int64_t B, int64_
 // ---- backward passes of the two operators ------------------------------------------------------------------------------------
 // The weight gradient runs on the helper stream next to the dX / dY kernel: the two are independent and share the SMs.  Below
 // kSmallWork multiply-adds (kernels of under 10 us) a backward pass is bound by the host, and the fork and join are left out.
-constexpr double kSmallWork = 1 << 27;
+// (At 2^27 the FFMA kernels of odd float32 sizes take 30 us and want the overlap: 117 against 131 us a pass at 132M.)
+constexpr double kSmallWork = 1 << 25;
 bool worth_a_side_stream(const Tensor& slot_rows, const Tensor& W) {      // [B,E,K,J] and a weight tensor of E * I * J elements
   const double slots = static_cast<double>(slot_rows.size(0)) * slot_rows.size(2);
   return slots * W.numel() > kSmallWork;

@@ -79,9 +79,9 @@ struct RowGemmParams {
   int expert_fastest; // tensor path: grid order (1: experts vary fastest, row tiles slowest)
   int row_tiles;      // tensor path: 128-row accumulator tiles per CTA (1 or 2)
   int persistent;     // tensor path: 1 = persistent warp-specialised variant
-  int pair;           // 16-bit G: tiles of 256 rows on pairs of SMs
+  int pair;           // 16-bit G, S: tiles of 256 rows on pairs of SMs
   int after_own;      // launched behind a kernel of the same call (fill, preparation): see launch_kernel
-  int bulk_epilogue;  // persistent scatter: rows staged in shared memory and added with bulk asynchronous reductions
+  int bulk_epilogue;  // 16-bit S: additions go out as whole 128-byte row segments (for egs_describe_plan)
 };
 
 struct DWeightParams {
@@ -148,10 +148,10 @@ cudaError_t launch_scatter_prepare(const void* Ind, int index_dtype, int B, int 
 cudaError_t launch_scatter_finish(const int* plan, const float* acc, void* out16, int B, size_t per_batch, int dtype, cudaStream_t st);
 
 // Tensor-core (tcgen05) family.  `configure_*` fills BN/stages and returns the dynamic shared memory size.
-size_t configure_tensor_rowgemm(RowGemmParams& p, bool scatter, int dtype);
-size_t configure_tensor_dweight(DWeightParams& p, int dtype);
-cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, int dtype, size_t smem_bytes, cudaStream_t st);
-cudaError_t launch_tensor_dweight(const DWeightParams& p, int dtype, size_t smem_bytes, cudaStream_t st);
+size_t configure_tensor_rowgemm(RowGemmParams& p, bool scatter);
+size_t configure_tensor_dweight(DWeightParams& p);
+cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, size_t smem_bytes, cudaStream_t st);
+cudaError_t launch_tensor_dweight(const DWeightParams& p, size_t smem_bytes, cudaStream_t st);
 
 // 16-bit tensors (egs_dense16.cu): persistent kernels for G, S and D.
 void configure_dense16_rowgemm(RowGemmParams& p, bool scatter);

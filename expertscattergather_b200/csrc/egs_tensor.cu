@@ -1,4 +1,4 @@
-// tcgen05 / TMEM kernels for the three operators (sm_100a only).
+// tcgen05 / TMEM kernels for float32 tensors in TF32 arithmetic: the three operators and the fused pair (sm_100a only).
 //
 // Common structure of both kernels (one CTA = one 128-row accumulator tile in tensor memory):
 //   warps 0..7  producers: index-driven 16-byte cp.async row gathers from global memory into shared
@@ -26,13 +26,15 @@
 // whose XOR acts on 32-byte pairs with the row index modulo 4 (atoms of 4 rows; SBO = 512); float32 tiles
 // that are consumed MN-major are written in that variant.
 //
-// float32 tensors: kind::tf32, one TF32 product per element.  Strict float32 (three products) has its own kernels in
-// egs_strict.cu, except for the fused pair below.  16-bit tensors: kind::f16 with fp32 accumulation.
+// kind::tf32, one TF32 product per element.  Strict float32 (three products) has its own kernels in egs_strict.cu, except for the
+// fused pair below; 16-bit tensors have theirs in egs_dense16.cu.
 #include "egs_tcgen05.cuh"
 
 namespace egs {
 
 namespace {
+
+using T = float;                    // element type of every tensor here
 
 // ------------------------------------------------------------------------------------------------
 // Pipeline pieces shared by the two kernels
@@ -159,7 +161,7 @@ __device__ __forceinline__ void run_mma_lane(const Pipe& pp, Mma&& mma) {
 // MT = number of 128-row accumulator tiles per CTA (1 or 2).  With MT = 2 the CTA owns 256 expert rows: both
 // accumulators are fed from the same W tile, which cuts the bytes loaded per flop by a third and lets a
 // three-stage ring of one CTA per SM cover the load latency that two 2-stage CTAs cannot.
-template <typename T, bool SCATTER, int MT>
+template <bool SCATTER, int MT>
 __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_rowgemm_kernel(RowGemmParams p) {
   constexpr int kRows = kTileM * MT;        // expert rows per CTA
   constexpr int ES = sizeof(T);
@@ -326,65 +328,14 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_rowgemm_kern
     const bool alive = run_producer(pp, lane, issue_stage);
 
     // =========================== epilogue ===========================
-    // The stage ring is idle once `done` has completed: it holds, per warp, a 4 KB transpose tile or, where the ring has room, the
-    // two staging buffers of the bulk reductions (the tile fits in them; warps of one CTA may differ in which they use).
+    // The stage ring is idle once `done` has completed: it holds a 4 KB transpose tile per warp.
     if (alive) {
       const int lg = warp & 3, half = warp >> 2;
-      const bool bulk_room = SCATTER && ES == 2 && p.bulk_epilogue && (pp.stages * pp.stage_bytes >= 8u * 2u * kBulkBufBytes);
-      const uint32_t area = pp.tiles0 + static_cast<uint32_t>(warp) * (bulk_room ? 2u * kBulkBufBytes : 4096u);
+      const uint32_t area = pp.tiles0 + static_cast<uint32_t>(warp) * 4096u;
       T* out = static_cast<T*>(p.Out);
-      float* acc_rows = (ES == 2) ? p.acc : reinterpret_cast<float*>(p.Out);   // S: float32 rows being added to
-      // 16-bit S: the planning flags say, per batch element, whether to add into the float32 rows or straight into the output.
-      // f32_rows(mt): which of this warp's 32 rows of accumulator mt go to the float32 rows.
-      auto f32_rows = [&](int mt) -> uint32_t {
-        const int m = m0 + mt * kTileM + lg * 32 + lane;
-        return __ballot_sync(0xffffffffu, p.plan == nullptr || (m < p.M && p.plan[m / p.K] != 0));
-      };
-      // direct 16-bit adds go out as bulk reductions: every lane stages 128 bytes (64 columns) of its own row and hands them to the
-      // copy engine (see the persistent variant)
-      bool bulk16 = bulk_room;
-      if (bulk_room)
-        for (int mt = 0; mt < MT; ++mt) bulk16 = bulk16 && f32_rows(mt) == 0u;
       const int nblk = (bn + 31) >> 5;
       const T* bias_row = p.bias ? static_cast<const T*>(p.bias) + static_cast<long long>(e) * p.N : nullptr;
-      if (bulk16) {
-        if constexpr (ES == 2 && SCATTER) {
-          const uint32_t my_stage = area + static_cast<uint32_t>(lane) * kBulkRowPitch;
-          int q = 0;
-          for (int mt = 0; mt < MT; ++mt) {
-            const int ro = hdr->row_o[mt * kTileM + lg * 32 + lane];
-            const uint32_t acc0 = tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + mt * acc_cols;
-            for (int c = half; c * 64 < bn; c += 2, ++q) {
-              const uint32_t srow = my_stage + static_cast<uint32_t>(q & 1) * kBulkBufBytes;
-              if (q >= 2) bulk_wait_read_1();
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                if (c * 64 + h * 32 < bn) {
-                  uint32_t v[32];
-                  tmem_ld32(acc0 + static_cast<uint32_t>(c * 64 + h * 32), v);
-                  tmem_ld_wait();
-                  if (bias_row) add_bias32<T>(bias_row + n0 + c * 64 + h * 32, p.N - (n0 + c * 64 + h * 32), v);
-#pragma unroll
-                  for (int j = 0; j < 4; ++j)
-                    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(srow + h * 64u + j * 16u),
-                                 "r"(pack2(out, v[8 * j], v[8 * j + 1])), "r"(pack2(out, v[8 * j + 2], v[8 * j + 3])),
-                                 "r"(pack2(out, v[8 * j + 4], v[8 * j + 5])), "r"(pack2(out, v[8 * j + 6], v[8 * j + 7]))
-                                 : "memory");
-                }
-              }
-              fence_proxy_async_smem();
-              const int col0 = n0 + c * 64;
-              const int ncols = min(64, p.N - col0);
-              if (ro >= 0 && ncols > 0)
-                bulk_reduce_add(out + static_cast<long long>(ro) * p.N + col0, srow, static_cast<uint32_t>(ncols) * 2u);
-              bulk_commit();
-            }
-          }
-          bulk_wait_all();                               // shared memory must outlive the copy engine's reads
-        }
-      } else
       for (int mt = 0; mt < MT; ++mt) {
-        const uint32_t to_f32 = (SCATTER && ES == 2) ? f32_rows(mt) : 0xffffffffu;
         for (int c = half; c < nblk; c += 2) {
           const int col0 = n0 + c * 32;
           warp_block_emit(tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + mt * acc_cols + static_cast<uint32_t>(c * 32), area,
@@ -394,12 +345,8 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_rowgemm_kern
                             if (ro >= 0 && col < p.N) {
                               const long long off = static_cast<long long>(ro) * p.N + col;
                               if (bias_row) add_bias4<T>(bias_row + col, x0, x1, x2, x3);
-                              if (SCATTER) {
-                                if ((to_f32 >> row) & 1u) red4(acc_rows + off, x0, x1, x2, x3);
-                                else red4(out + off, x0, x1, x2, x3);
-                              } else {
-                                store4(out + off, x0, x1, x2, x3);   // masked source rows were zero-filled: zeros
-                              }
+                              if (SCATTER) red4(out + off, x0, x1, x2, x3);
+                              else store4(out + off, x0, x1, x2, x3);   // masked source rows were zero-filled: zeros
                             }
                           });
         }
@@ -509,7 +456,7 @@ __device__ __forceinline__ void lookup_rows(const RowGemmParams& p, int e, int m
   }
 }
 
-template <typename T, bool SCATTER>
+template <bool SCATTER>
 __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_rowgemm_persistent_kernel(RowGemmParams p) {
   constexpr int kPersistProducerWarps = PersistShape<SCATTER>::kProducerWarps;
   constexpr int kPersistEpilogueWarps = PersistShape<SCATTER>::kEpilogueWarps;
@@ -525,9 +472,7 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
   PersistHeader* hdr = reinterpret_cast<PersistHeader*>(smem_raw);
   const uint32_t smem0 = smem_u32(smem_raw);
   const uint32_t xpose0 = smem0 + kPersistHeaderBytes;                             // 8 transpose tiles of 4 KB
-  // per epilogue warp: a 4 KB transpose tile, or the two staging buffers of the bulk adds (the tile fits in them)
-  const uint32_t xpose_tile = p.bulk_epilogue ? 2u * kBulkBufBytes : 4096u;
-  const uint32_t tiles0 = xpose0 + ((kPersistMaxEpilogueWarps * xpose_tile + 1023u) & ~1023u);   // stage ring
+  const uint32_t tiles0 = xpose0 + kPersistMaxEpilogueWarps * 4096u;               // stage ring
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool w_nc = (p.w_layout == EGS_W_NC);
@@ -704,27 +649,16 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
     const int ew = warp - kPersistProducerWarps;
     constexpr int kColGroups = kPersistEpilogueWarps / 4;
     const int lg = ew & 3, half = ew >> 2;               // TMEM lane group of this warp, which share of the column blocks
-    const uint32_t tile = xpose0 + static_cast<uint32_t>(ew) * xpose_tile;
+    const uint32_t tile = xpose0 + static_cast<uint32_t>(ew) * 4096u;
     T* out = static_cast<T*>(p.Out);
-    float* acc_rows = (ES == 2) ? p.acc : reinterpret_cast<float*>(p.Out);   // S: float32 rows being added to
-    // bulk adds (direct 16-bit scatter): every lane stages 128 bytes of its own row and hands them to the copy
-    // engine - no transpose, no shuffles, and the warp does not wait on the load/store unit.  (For float32 rows
-    // the same scheme needs twice the operations per column and measured slower than the transposed reds.)
-    const uint32_t my_stage = tile + static_cast<uint32_t>(lane) * kBulkRowPitch;
-    int q = 0;                                           // bulk groups committed so far by this thread
     bool alive = true;
-    if (SCATTER) pdl_wait();                             // the planning flags and the zeros the rows are added to
+    if (SCATTER) pdl_wait();                             // the zeros the rows are added to
     int t = 0;                                           // tiles finished so far by this CTA
     for (int rb = blockIdx.x; rb < row_blocks && alive; rb += gridDim.x) {
       const RowBlock blk = row_block_of(p, rb, m_tiles);
       int src_row, my_ro;                                // destination row of tile row lg*32 + lane
       const int my_m = blk.m0 + lg * 32 + lane;
       lookup_rows<SCATTER>(p, blk.e, my_m, src_row, my_ro, half == 0);
-      // rows of this warp whose batch element sums in float32 rows (bits), see RowGemmParams::plan
-      const uint32_t to_f32 = (SCATTER && ES == 2) ? __ballot_sync(0xffffffffu, p.plan == nullptr || (my_m < p.M && p.plan[my_m / p.K] != 0))
-                                                   : 0xffffffffu;
-      const bool bulk = SCATTER && ES == 2 && p.bulk_epilogue && to_f32 == 0u;
-      if (SCATTER && ES == 2 && !bulk) bulk_wait_all();  // the transposes below reuse the staging buffers
       for (int nt = 0; nt < n_tiles && alive; ++nt, ++t) {
         const int n0 = nt * p.BN;
         const int bn = min(p.BN, ((p.N - n0) + 15) & ~15);
@@ -733,39 +667,6 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
         if (!alive) break;
         tc_fence_after();
         const int nblk = (bn + 31) >> 5;
-        if (bulk) {
-          const uint32_t acc0 = tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + buf * acc_cols;
-          if constexpr (ES == 2) {
-            // 64 columns = 128 bytes of a 16-bit row per block
-            for (int c = half; c * 64 < bn; c += kColGroups, ++q) {
-              const uint32_t srow = my_stage + static_cast<uint32_t>(q & 1) * kBulkBufBytes;
-              if (q >= 2) bulk_wait_read_1();            // the group that used this buffer two blocks ago has been read
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                if (c * 64 + h * 32 < bn) {
-                  uint32_t v[32];
-                  tmem_ld32(acc0 + static_cast<uint32_t>(c * 64 + h * 32), v);
-                  tmem_ld_wait();
-                  if (p.bias)
-                    add_bias32<T>(static_cast<const T*>(p.bias) + static_cast<long long>(blk.e) * p.N + n0 + c * 64 + h * 32,
-                                  p.N - (n0 + c * 64 + h * 32), v);
-#pragma unroll
-                  for (int j = 0; j < 4; ++j)
-                    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(srow + h * 64u + j * 16u),
-                                 "r"(pack2(out, v[8 * j], v[8 * j + 1])), "r"(pack2(out, v[8 * j + 2], v[8 * j + 3])),
-                                 "r"(pack2(out, v[8 * j + 4], v[8 * j + 5])), "r"(pack2(out, v[8 * j + 6], v[8 * j + 7]))
-                                 : "memory");
-                }
-              }
-              fence_proxy_async_smem();
-              const int col0 = n0 + c * 64;
-              const int ncols = min(64, p.N - col0);
-              if (my_ro >= 0 && ncols > 0)
-                bulk_reduce_add(out + static_cast<long long>(my_ro) * p.N + col0, srow, static_cast<uint32_t>(ncols) * 2u);
-              bulk_commit();
-            }
-          }
-        } else
         for (int c = half; c < nblk; c += kColGroups) {
           const int col0 = n0 + c * 32;
           warp_block_emit(tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + buf * acc_cols + static_cast<uint32_t>(c * 32), tile, lane,
@@ -775,12 +676,8 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
                             if (ro >= 0 && col < p.N) {
                               const long long off = static_cast<long long>(ro) * p.N + col;
                               if (p.bias) add_bias4<T>(static_cast<const T*>(p.bias) + static_cast<long long>(blk.e) * p.N + col, x0, x1, x2, x3);
-                              if (SCATTER) {
-                                if ((to_f32 >> row) & 1u) red4(acc_rows + off, x0, x1, x2, x3);
-                                else red4(out + off, x0, x1, x2, x3);
-                              } else {
-                                store4(out + off, x0, x1, x2, x3);
-                              }
+                              if (SCATTER) red4(out + off, x0, x1, x2, x3);
+                              else store4(out + off, x0, x1, x2, x3);
                             }
                           });
         }
@@ -790,7 +687,6 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
         if (lane == 0) mbar_arrive(smem_u32(&hdr->acc_empty[buf]));
       }
     }
-    if (SCATTER && ES == 2) bulk_wait_all();             // shared memory must outlive the copy engine's reads
   } else {
     // =========================== MMA issuer ===========================
     if (lane == 0) {
@@ -852,7 +748,7 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
 //   the same B tile: a third fewer bytes loaded per flop, which is what bounds this kernel once the contraction
 //   is long (the loads of two 128 x 256 CTAs per SM top out well below the tensor rate).
 // ------------------------------------------------------------------------------------------------
-template <typename T, int MT>
+template <int MT>
 __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_dweight_kernel(DWeightParams p) {
   constexpr int ES = sizeof(T);
   constexpr int KR = 128 / ES;          // contraction rows per stage (4 MMAs of UK rows)
@@ -1486,9 +1382,8 @@ int pick_stages(size_t fixed_bytes, size_t stage_bytes, long long ctas, bool all
 
 }  // namespace
 
-size_t configure_tensor_rowgemm(RowGemmParams& p, bool scatter, int dtype) {
-  const int es = (dtype == EGS_F32) ? 4 : 2;
-  const int ke = 128 / es;
+size_t configure_tensor_rowgemm(RowGemmParams& p, bool scatter) {
+  constexpr int es = 4, ke = 128 / es;
   int bn = (p.N + 15) & ~15;
   if (bn > 256) bn = 256;
   p.BN = bn;
@@ -1508,23 +1403,17 @@ size_t configure_tensor_rowgemm(RowGemmParams& p, bool scatter, int dtype) {
   // persistent variant (see its kernel): scatter problems with many tiles, non-strict arithmetic
   const long long tiles1 = static_cast<long long>((p.M + kTileM - 1) / kTileM) * n_tiles * p.E;
   p.persistent = 0;
-  // direct 16-bit scatter adds go out as bulk reductions
-  p.bulk_epilogue = (scatter && es == 2) ? 1 : 0;
+  p.bulk_epilogue = 0;
   // (measured: it wins for contractions of up to four stages - the scatter of cfg4 and cfg2 - and loses for longer ones)
   if (scatter && p.C * es <= 512 && tiles1 >= 2 * kSmCount) {
     const size_t st1 = static_cast<size_t>(kTileM) * 128 + b_bytes;
-    size_t fixed_p = kPersistHeaderBytes + kPersistMaxEpilogueWarps * 4096;
-    // 16-bit scatter: staging buffers for the bulk adds when the ring keeps three stages
-    const size_t bulk_bytes = (kPersistMaxEpilogueWarps * 2 * kBulkBufBytes + 1023) & ~static_cast<size_t>(1023);
-    const bool bulk_fits = (kSmemMaxPerCta - kPersistHeaderBytes - bulk_bytes) / st1 >= 3;
-    if (p.bulk_epilogue && bulk_fits) fixed_p = kPersistHeaderBytes + bulk_bytes;
+    const size_t fixed_p = kPersistHeaderBytes + kPersistMaxEpilogueWarps * 4096;
     size_t ns = (kSmemMaxPerCta - fixed_p) / st1;
     if (ns > static_cast<size_t>(kMaxStages)) ns = kMaxStages;
     if (ns >= 3) {
       p.persistent = 1;
       p.row_tiles = 1;
       p.stages = static_cast<int>(ns);
-      if (!bulk_fits) p.bulk_epilogue = 0;
       return fixed_p + ns * st1;
     }
   }
@@ -1532,9 +1421,8 @@ size_t configure_tensor_rowgemm(RowGemmParams& p, bool scatter, int dtype) {
   return fixed + p.stages * stage_bytes;
 }
 
-size_t configure_tensor_dweight(DWeightParams& p, int dtype) {
-  const int es = (dtype == EGS_F32) ? 4 : 2;
-  const int kr = 128 / es;
+size_t configure_tensor_dweight(DWeightParams& p) {
+  constexpr int es = 4, kr = 128 / es;
   int bn = (p.FD + 15) & ~15;
   if (bn > 256) bn = 256;
   p.BN = bn;
@@ -1598,26 +1486,19 @@ size_t configure_tensor_fused_pair(FusedParams& p, int precision) {
   return fixed + ns * stage_bytes;
 }
 
-cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, int dtype, size_t smem_bytes, cudaStream_t st) {
+cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, size_t smem_bytes, cudaStream_t st) {
   if (p.persistent) {
     const int row_blocks = p.E * ((p.M + kTileM - 1) / kTileM);
     dim3 pgrid(row_blocks < kSmCount ? row_blocks : kSmCount);
     dim3 pblock(scatter ? PersistShape<true>::kThreads : PersistShape<false>::kThreads);
     cudaError_t perr = cudaSuccess;
-#define EGS_LAUNCH_P(TY)                                                                                     \
-  do {                                                                                                       \
-    if (scatter) {                                                                                           \
-      perr = (ensure_smem_optin<tensor_rowgemm_persistent_kernel<TY, true>>(static_cast<int>(kSmemMaxPerCta)));                              \
-      if (perr == cudaSuccess) perr = launch_kernel(tensor_rowgemm_persistent_kernel<TY, true>, pgrid, pblock, smem_bytes, st, p.after_own != 0, p);  \
-    } else {                                                                                                 \
-      perr = (ensure_smem_optin<tensor_rowgemm_persistent_kernel<TY, false>>(static_cast<int>(kSmemMaxPerCta)));                             \
-      if (perr == cudaSuccess) perr = launch_kernel(tensor_rowgemm_persistent_kernel<TY, false>, pgrid, pblock, smem_bytes, st, false, p); \
-    }                                                                                                        \
-  } while (0)
-    if (dtype == EGS_F32) EGS_LAUNCH_P(float);
-    else if (dtype == EGS_F16) EGS_LAUNCH_P(__half);
-    else EGS_LAUNCH_P(__nv_bfloat16);
-#undef EGS_LAUNCH_P
+    if (scatter) {
+      perr = ensure_smem_optin<tensor_rowgemm_persistent_kernel<true>>(static_cast<int>(kSmemMaxPerCta));
+      if (perr == cudaSuccess) perr = launch_kernel(tensor_rowgemm_persistent_kernel<true>, pgrid, pblock, smem_bytes, st, p.after_own != 0, p);
+    } else {
+      perr = ensure_smem_optin<tensor_rowgemm_persistent_kernel<false>>(static_cast<int>(kSmemMaxPerCta));
+      if (perr == cudaSuccess) perr = launch_kernel(tensor_rowgemm_persistent_kernel<false>, pgrid, pblock, smem_bytes, st, false, p);
+    }
     if (perr != cudaSuccess) return perr;
     count_launch();
     return cudaGetLastError();
@@ -1627,50 +1508,36 @@ cudaError_t launch_tensor_rowgemm(const RowGemmParams& p, bool scatter, int dtyp
   dim3 grid(p.expert_fastest ? p.E : row_tiles, (p.N + p.BN - 1) / p.BN, p.expert_fastest ? row_tiles : p.E);
   dim3 block(kThreads);
   cudaError_t err = cudaSuccess;
-#define EGS_LAUNCH2(TY, SC, MTV)                                                                                \
-  do {                                                                                                          \
-    err = (ensure_smem_optin<tensor_rowgemm_kernel<TY, SC, MTV>>(static_cast<int>(kSmemMaxPerCta)));            \
-    if (err == cudaSuccess) err = launch_kernel(tensor_rowgemm_kernel<TY, SC, MTV>, grid, block, smem_bytes, st, p.after_own != 0, p); \
+#define EGS_LAUNCH2(SC, MTV)                                                                                \
+  do {                                                                                                      \
+    err = ensure_smem_optin<tensor_rowgemm_kernel<SC, MTV>>(static_cast<int>(kSmemMaxPerCta));              \
+    if (err == cudaSuccess) err = launch_kernel(tensor_rowgemm_kernel<SC, MTV>, grid, block, smem_bytes, st, p.after_own != 0, p); \
   } while (0)
-#define EGS_LAUNCH(TY)                                  \
-  do {                                                  \
-    if (scatter) {                                      \
-      if (p.row_tiles == 2) EGS_LAUNCH2(TY, true, 2);   \
-      else EGS_LAUNCH2(TY, true, 1);                    \
-    } else {                                            \
-      if (p.row_tiles == 2) EGS_LAUNCH2(TY, false, 2);  \
-      else EGS_LAUNCH2(TY, false, 1);                   \
-    }                                                   \
-  } while (0)
-  if (dtype == EGS_F32) EGS_LAUNCH(float);
-  else if (dtype == EGS_F16) EGS_LAUNCH(__half);
-  else EGS_LAUNCH(__nv_bfloat16);
-#undef EGS_LAUNCH
+  if (scatter) {
+    if (p.row_tiles == 2) EGS_LAUNCH2(true, 2);
+    else EGS_LAUNCH2(true, 1);
+  } else {
+    if (p.row_tiles == 2) EGS_LAUNCH2(false, 2);
+    else EGS_LAUNCH2(false, 1);
+  }
 #undef EGS_LAUNCH2
   if (err != cudaSuccess) return err;
   count_launch();
   return cudaGetLastError();
 }
 
-cudaError_t launch_tensor_dweight(const DWeightParams& p, int dtype, size_t smem_bytes, cudaStream_t st) {
+cudaError_t launch_tensor_dweight(const DWeightParams& p, size_t smem_bytes, cudaStream_t st) {
   const int f_tile = kTileM * p.row_tiles;
   dim3 grid((p.FG + f_tile - 1) / f_tile, (p.FD + p.BN - 1) / p.BN, p.E * p.splits);
   dim3 block(kThreads);
   cudaError_t err = cudaSuccess;
-#define EGS_LAUNCH_D(TY, MTV)                                                                                   \
-  do {                                                                                                          \
-    err = (ensure_smem_optin<tensor_dweight_kernel<TY, MTV>>(static_cast<int>(kSmemMaxPerCta)));                \
-    if (err == cudaSuccess) err = launch_kernel(tensor_dweight_kernel<TY, MTV>, grid, block, smem_bytes, st, p.after_own != 0, p); \
+#define EGS_LAUNCH_D(MTV)                                                                                   \
+  do {                                                                                                      \
+    err = ensure_smem_optin<tensor_dweight_kernel<MTV>>(static_cast<int>(kSmemMaxPerCta));                  \
+    if (err == cudaSuccess) err = launch_kernel(tensor_dweight_kernel<MTV>, grid, block, smem_bytes, st, p.after_own != 0, p); \
   } while (0)
-#define EGS_LAUNCH(TY)                          \
-  do {                                          \
-    if (p.row_tiles == 2) EGS_LAUNCH_D(TY, 2);  \
-    else EGS_LAUNCH_D(TY, 1);                   \
-  } while (0)
-  if (dtype == EGS_F32) EGS_LAUNCH(float);
-  else if (dtype == EGS_F16) EGS_LAUNCH(__half);
-  else EGS_LAUNCH(__nv_bfloat16);
-#undef EGS_LAUNCH
+  if (p.row_tiles == 2) EGS_LAUNCH_D(2);
+  else EGS_LAUNCH_D(1);
 #undef EGS_LAUNCH_D
   if (err != cudaSuccess) return err;
   count_launch();

@@ -274,7 +274,7 @@ typedef struct egs_plan_info {
   int row_tiles;      /* 128-row accumulators a CTA holds: 1 or 2 */
   int persistent;     /* float32 S: 1 = the persistent kernel.  16-bit tensors (all kernels are persistent): 1 = a scatter whose
                        * tiles are bound by their additions, not by their contraction */
-  int bulk_epilogue;  /* S with 16-bit tensors: direct additions go out as bulk reductions */
+  int bulk_epilogue;  /* S with 16-bit tensors: direct additions go out as whole 128-byte row segments */
   int expert_fastest; /* G / S: grid order, 1 = experts vary fastest */
   int splits;         /* D: row ranges the contraction is split into */
   int rows_per_split; /* D: contraction rows per range */

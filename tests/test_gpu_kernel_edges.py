@@ -112,6 +112,38 @@ def test_strict_float32_edges(cuda_device, B, T, E, K, I, J):
         assert orc.rel_err(got[k], truth[k]) <= 1e-5, k
 
 
+# 16-bit kernels: one CTA or a pair per tile (the last two shapes are large enough for pairs), slot rows as boxes (K = 1, 16, 64, 128)
+# or gathered (K = 43, 101), one row or one column block in the last tile, row ranges of D that are split and that are not
+@pytest.mark.parametrize("B,T,E,K,I,J", [(1, 8, 1, 1, 8, 8), (3, 60, 2, 43, 72, 40), (5, 90, 3, 64, 264, 136), (33, 70, 5, 16, 520, 264),
+                                         (5, 300, 2, 128, 1000, 200), (9, 777, 24, 101, 1000, 200), (16, 300, 16, 64, 264, 512)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_dense16_edges(cuda_device, B, T, E, K, I, J, bias):
+    g = torch.Generator().manual_seed(I + J)
+    dt = torch.float16                                              # integers to 2048 are exact, and no sum here comes near that
+    small = lambda *shape: torch.randint(-1, 2, shape, generator=g).to(dt)
+    X, G, Y, dY = small(B, T, I), small(B, T, I), small(B, E, K, J), small(B, E, K, J)
+    Wg, Ws, bg, bs = small(E, I, J), small(E, J, I), small(E, 1, J), small(E, 1, I)
+    # one slot after another through all the tokens: every row meets about E * K / T contributions
+    Ind = (torch.arange(B * E * K).view(B, E, K) * 7 + torch.arange(B).view(B, 1, 1)) % T
+    d = {k: v.to(cuda_device) for k, v in dict(X=X, G=G, Y=Y, dY=dY, Wg=Wg, Ws=Ws, bg=bg, bs=bs, Ind=Ind).items()}
+
+    def same(got, want):
+        assert np.abs(want).max() <= 2048 and np.array_equal(got.cpu().double().numpy(), want)
+
+    rows = orc.np_gather(X, Wg, Ind) + (bg[:, 0].double().numpy()[None, :, None, :] if bias else 0)
+    same(ops.gather_gemm(d["X"], d["Wg"], d["Ind"], bias=d["bg"] if bias else None, path="tensor"), rows)
+    same(ops.gather_gemm(d["G"], d["Ws"], d["Ind"], w_layout="nc", path="tensor"), orc.np_gather(G, Ws.transpose(1, 2).contiguous(), Ind))
+    sums = orc.np_scatter(Y, Ws, Ind, T)
+    if bias:
+        for e in range(E):
+            for b in range(B):
+                np.add.at(sums[b], Ind[b, e].numpy(), bs[e, 0].double().numpy())
+    same(ops.gemm_scatter(d["Y"], d["Ws"], d["Ind"], T, bias=d["bs"] if bias else None, path="tensor"), sums)
+    same(ops.gemm_scatter(d["dY"], d["Wg"], d["Ind"], T, w_layout="nc", path="tensor"), orc.np_scatter(dY, Wg.transpose(1, 2).contiguous(), Ind, T))
+    same(ops.dweight(d["X"], d["dY"], d["Ind"], path="tensor"), orc.np_dweight(X, dY, Ind))
+    same(ops.dweight(d["G"], d["Y"], d["Ind"], out_layout="direct_rows", path="tensor"), orc.np_dweight(G, Y, Ind).transpose(0, 2, 1))
+
+
 # 16-bit scatter: the choice between direct additions and float32 rows is made per batch element; tiles of 128 expert rows here
 # span batch elements of both kinds (K = 48), the persistent kernel (N = 1032) and the one-tile kernel (long contraction)
 @pytest.mark.parametrize("C,N", [(40, 72), (256, 1032), (520, 64)])
