@@ -115,7 +115,7 @@ def test_strict_float32_edges(cuda_device, B, T, E, K, I, J):
 # 16-bit kernels: one CTA or a pair per tile (the last two shapes are large enough for pairs), slot rows as boxes (K = 1, 16, 64, 128)
 # or gathered (K = 43, 101), one row or one column block in the last tile, row ranges of D that are split and that are not
 @pytest.mark.parametrize("B,T,E,K,I,J", [(1, 8, 1, 1, 8, 8), (3, 60, 2, 43, 72, 40), (5, 90, 3, 64, 264, 136), (33, 70, 5, 16, 520, 264),
-                                         (5, 300, 2, 128, 1000, 200), (9, 777, 24, 101, 1000, 200), (16, 300, 16, 64, 264, 512)])
+                                         (5, 300, 2, 128, 1000, 200), (9, 777, 24, 101, 1000, 200), (20, 200, 24, 64, 520, 512)])
 @pytest.mark.parametrize("bias", [False, True])
 def test_dense16_edges(cuda_device, B, T, E, K, I, J, bias):
     g = torch.Generator().manual_seed(I + J)
