@@ -1,24 +1,28 @@
-// Operators G, S and D for 16-bit tensors as one persistent, warp-specialised kernel (sm_100a).
+// Operators G, S and D for 16-bit tensors as one persistent, warp-specialised kernel (sm_100a), on one CTA or a pair of CTAs per tile.
 //
-//   warps 0..7    gather producers: index-driven 16-byte cp.async row copies into the stage ring
+//   warps 0..7    gather producers: index-driven 16-byte cp.async row copies into the stage ring; in a scatter whose slot rows come
+//                 as boxes they have nothing to gather and join the read-out
 //   warps 8..15   read-out: tensor memory -> stores (G, D) / red.global.add (S)
-//   warp  16      tensor-memory allocation; one lane issues tcgen05.mma, four per stage as straight-line code
-//   warp  17      one lane issues the TMA box loads of everything that is not gathered
-//   warps 18, 19  (D) look up the token rows of the contraction rows to come into a table in shared memory
+//   warp  16      tensor-memory allocation; four tcgen05.mma per stage.  In a pair the leader's warp issues for both (cta_group::2)
+//                 and the peer's tells the leader of every stage that has landed there
+//   warp  17      the TMA box loads of everything that is not gathered
+//   warps 18, 19  look up the rows of the tiles to come: G, S source rows (18) and destination rows (19); D the contraction rows
 //
-// A unit of work is one 128 x BN accumulator tile; CTAs (one per SM) walk the units, the stage ring runs on across them and the
-// accumulator is double-buffered in tensor memory, so neither set-up nor read-out stands between two tiles.
+// A unit of work is one accumulator tile of 128 x BN per CTA (256 x BN per pair); CTAs (one per SM) walk the units, the stage ring
+// runs on across them and the accumulator is double-buffered in tensor memory, so neither set-up nor read-out stands between two tiles.
 //   G  rows = expert rows, token rows through Ind (cp.async);     columns = W[e] (TMA)
 //   S  rows = expert rows, slot rows (TMA where 128 rows are whole batch elements or parts of one, else cp.async);  columns = W[e]
 //   D  contraction = expert rows; one operand the gathered token rows (cp.async), the other the slot rows (TMA under the same
 //      condition for 64 rows, else cp.async).  Either may be the one whose features are the accumulator's rows.
 //
-// What bounds the main loop is shared-memory bandwidth: a stage (64 contraction elements) of a 128 x 256 tile is 48 KB written
-// and 48 KB read by its four MMAs, 750 clocks at 128 bytes per clock against 512 clocks of tensor work.  The two copy paths have
-// to stay below that, and neither does alone: 16-byte cp.async costs about 10 clocks per warp instruction (960 for such a stage),
-// a TMA box about 2 clocks per 128-byte row.  Split between them, a stage of G costs the load/store unit 320 and the TMA unit
-// 550 clocks, side by side.  A lone issuing lane needs 7-10 clocks per instruction: nothing on the per-stage paths of the TMA and
-// MMA lanes divides or multiplies.
+// What bounds the main loop is shared-memory bandwidth and the tensor core together: a stage (64 contraction elements) of a 128 x 256
+// tile is 48 KB written and 48 KB read by its four MMAs, 750 clocks at 128 bytes per clock against 512 clocks of tensor work; a pair
+// stages half the columns per CTA and moves 64 KB, 512 clocks.  16-byte cp.async costs the load/store unit about 10 clocks per warp
+// instruction (320 a stage of G), side by side with the TMA unit.  Everything else has to stay out of the way: a satisfied barrier
+// wait takes 150 clocks and every dependent instruction of a lone warp 5-10, so nothing on a per-stage or per-tile path divides, the
+// issuing warps run converged (see mbar_wait_all) and ids are looked up elsewhere.
+// B=64, T=1024, E=64, K=64, I=1024, J=256, bf16: G 151 -> 110 us, S 243 -> 153, D 171 -> 123 (kernels of one CTA per tile, a 256-row
+// ring and 128-byte bulk reductions before); B=512: G 1160 -> 880 us = 1.25 PFLOP/s, under the power cap.
 #include <type_traits>
 
 #include "egs_tcgen05.cuh"

@@ -34,7 +34,7 @@ __device__ __forceinline__ uint32_t float_key(float f) {
 // by bit - R compares and a reduction per bit - and the search stops as soon as exactly K keys lie at or above the candidate,
 // after about 20 of 32 bits for scores without ties.  What bounds it is that chain of reductions and, before it, of chunks read one
 // after the other, not the bytes: few (batch, expert) pairs get more warps each (see launch_route_topk).
-// B=32, T=2048, E=64, K=128: 127 us with one CTA per expert column and shared-memory histograms.
+// B=32, T=2048, E=64, K=128: 28 us; 127 us with one CTA per expert column and shared-memory histograms.
 constexpr int kSelChunk = 8;          // keys per thread and chunk of the turn through shared memory
 constexpr int kSelMaxKeys = 64;       // keys per thread
 
