@@ -300,9 +300,9 @@ __global__ void __launch_bounds__(NTHREADS, FI * GJ > 4 ? 3 : 4) generic_dweight
 // Row sums per expert (the bias gradients):  out[e, n] = sum over the slots of expert e of row[n] of a token row (through Ind)
 // or of the slot row itself (Ind == NULL).  Eight lanes cover 128 bytes of a row; a cluster of CTAs shares the rows of one
 // (expert, 128-byte column block) and adds its partial sums through distributed shared memory, so that there is neither a
-// scratch buffer nor a second pass and the order of the additions is fixed.  Memory-bound: four rows in flight per thread.
-// 65536 routed rows of 768 bf16 features: 40 us as the weight-gradient contraction against ones, 26 us as a library reduction
-// of 192 features.
+// scratch buffer nor a second pass and the order of the additions is fixed.
+// 65536 routed rows of 768 bf16 features: 16 us = 6.3 TB/s from L2 and HBM (32 us while all eight lanes of a row looked it up, 40 us
+// as the weight-gradient contraction against ones).
 // ------------------------------------------------------------------------------------------------
 constexpr int kSumThreads = 256;
 template <typename T, bool VEC>
@@ -322,28 +322,28 @@ __global__ void __launch_bounds__(kSumThreads) expert_row_sum_kernel(const T* __
   float acc[PER];
 #pragma unroll
   for (int i = 0; i < PER; ++i) acc[i] = 0.f;
+  // eight rows in flight; each of a row's eight lanes looks one of them up (a division and a load) and the others get it by a shuffle
   constexpr int U = 8;
-  for (int m0 = rank * per + rl; m0 < m_end; m0 += U * ROWS) {
-    long long row[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int m = m0 + u * ROWS;
-      row[u] = -1;
-      if (m < m_end) {
-        const int b = m / K, k = m - b * K;
-        const long long slot = (static_cast<long long>(b) * E + e) * K + k;
-        row[u] = slot;
-        if (Ind) {
-          const long long t = load_index(Ind, index_dtype, slot);
-          if (t >= 0 && t < T_) {
-            row[u] = static_cast<long long>(b) * T_ + t;
-          } else {
-            row[u] = -1;
-            status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
-          }
+  for (unsigned base = static_cast<unsigned>(rank) * per; base < static_cast<unsigned>(m_end); base += U * ROWS) {
+    int found = -1;
+    const unsigned at = base + rl + cl * ROWS;
+    if (at < static_cast<unsigned>(m_end)) {
+      const int m = static_cast<int>(at), b = m / K, k = m - b * K;
+      const int slot = (b * E + e) * K + k;              // (B*E*K and B*T fit in 31 bits)
+      found = slot;
+      if (Ind) {
+        const long long t = load_index(Ind, index_dtype, slot);
+        if (t >= 0 && t < T_) {
+          found = b * T_ + static_cast<int>(t);
+        } else {
+          found = -1;
+          status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
         }
       }
     }
+    long long row[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) row[u] = __shfl_sync(0xffffffffu, found, (tid & 24) | u);
     if (VEC) {
       uint4 x[U];
 #pragma unroll
