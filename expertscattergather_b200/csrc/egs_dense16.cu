@@ -1,28 +1,35 @@
 // Operators G, S and D for 16-bit tensors as one persistent, warp-specialised kernel (sm_100a), on one CTA or a pair of CTAs per tile.
 //
-//   warps 0..7    gather producers: index-driven 16-byte cp.async row copies into the stage ring; in a scatter whose slot rows come
-//                 as boxes they have nothing to gather and join the read-out
+//   warps 0..7    gather producers: index-driven row copies into the stage ring, 16-byte cp.async on a CTA of its own, four rows by
+//                 TMA (tile::gather4) in a pair; in a scatter whose slot rows come as boxes they have nothing to gather and join the
+//                 read-out
 //   warps 8..15   read-out: tensor memory -> stores (G, D) / red.global.add (S)
-//   warp  16      tensor-memory allocation; four tcgen05.mma per stage.  In a pair the leader's warp issues for both (cta_group::2)
-//                 and the peer's tells the leader of every stage that has landed there
-//   warp  17      the TMA box loads of everything that is not gathered
+//   warp  16      tensor-memory allocation; four tcgen05.mma per stage, issued by the leader of a pair for both (cta_group::2)
+//   warp  17      the TMA box loads of everything that is not gathered; announces the bytes of a stage
 //   warps 18, 19  look up the rows of the tiles to come: G, S source rows (18) and destination rows (19); D the contraction rows
 //
 // A unit of work is one accumulator tile of 128 x BN per CTA (256 x BN per pair); CTAs (one per SM) walk the units, the stage ring
 // runs on across them and the accumulator is double-buffered in tensor memory, so neither set-up nor read-out stands between two tiles.
-//   G  rows = expert rows, token rows through Ind (cp.async);     columns = W[e] (TMA)
-//   S  rows = expert rows, slot rows (TMA where 128 rows are whole batch elements or parts of one, else cp.async);  columns = W[e]
-//   D  contraction = expert rows; one operand the gathered token rows (cp.async), the other the slot rows (TMA under the same
-//      condition for 64 rows, else cp.async).  Either may be the one whose features are the accumulator's rows.
+//   G  rows = expert rows, token rows through Ind (gathered);     columns = W[e] (boxes)
+//   S  rows = expert rows, slot rows (boxes where 128 rows are whole batch elements or parts of one, else gathered);  columns = W[e]
+//   D  contraction = expert rows; one operand the gathered token rows, the other the slot rows (boxes under the same condition for
+//      64 rows, else gathered).  Either may be the one whose features are the accumulator's rows.
+//
+// Everything a pair stages comes through the TMA units, and both CTAs' bytes are counted by the leader's barrier
+// (cp.async.bulk.tensor with cta_group::2): the leader's MMAs read the peer's shared memory behind nothing but that count.  Rows
+// copied there by cp.async would have to be handed over by a thread of the peer, with a proxy fence and an arrival that releases at
+// cluster scope: 1400 clocks a stage (B=512 as below: 10.4 ms a pass against 8.0; with three threads handing over in turn 8.5).
+// Accumulators go back to the leader by relaxed arrivals: nothing written is handed over, and tcgen05.wait::ld has returned, so
+// the loads have their values before the arrival is made.
 //
 // What bounds the main loop is shared-memory bandwidth and the tensor core together: a stage (64 contraction elements) of a 128 x 256
 // tile is 48 KB written and 48 KB read by its four MMAs, 750 clocks at 128 bytes per clock against 512 clocks of tensor work; a pair
 // stages half the columns per CTA and moves 64 KB, 512 clocks.  16-byte cp.async costs the load/store unit about 10 clocks per warp
-// instruction (320 a stage of G), side by side with the TMA unit.  Everything else has to stay out of the way: a satisfied barrier
+// instruction (320 a stage of G), side by side with the TMA unit; a pair's gathers take the TMA units about as long.  Everything else has to stay out of the way: a satisfied barrier
 // wait takes 150 clocks and every dependent instruction of a lone warp 5-10, so nothing on a per-stage or per-tile path divides, the
 // issuing warps run converged (see mbar_wait_all) and ids are looked up elsewhere.
-// B=64, T=1024, E=64, K=64, I=1024, J=256, bf16: G 151 -> 110 us, S 243 -> 153, D 171 -> 123 (kernels of one CTA per tile, a 256-row
-// ring and 128-byte bulk reductions before); B=512: G 1160 -> 880 us = 1.25 PFLOP/s, under the power cap.
+// T=1024, E=64, K=64, I=1024, J=256, bf16: B=64 G 126-138 us, S 215, D 148-165; B=512 G 950 us, dY (weights [E, N, C]) 895 = 1.23
+// PFLOP/s, S 1450, D 1050, under the power cap.
 #include <type_traits>
 
 #include "egs_tcgen05.cuh"
@@ -163,10 +170,11 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
   DenseHeader* hdr = reinterpret_cast<DenseHeader*>(smem_raw);
   const uint32_t smem0 = smem_u32(smem_raw);
   const uint32_t epi0 = smem0 + kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : kRowTable);
-  const bool has_cp = OP != kOpScatter || !p.tma_rows;
-  const bool has_tma = OP != kOpDweight || p.tma_rows;
-  const int readers = has_cp ? kEpiWarps : kProdWarps + kEpiWarps;      // read-out warps: producers with nothing to gather join
-  const uint32_t ring0 = epi0 + epi_bytes(!has_cp);
+  const bool gathers = OP != kOpScatter || !p.tma_rows;
+  const bool has_cp = !PAIR && gathers;
+  const bool has_tma = PAIR || OP != kOpDweight || p.tma_rows;          // (in a pair it also announces what the producers gather)
+  const int readers = gathers ? kEpiWarps : kProdWarps + kEpiWarps;     // read-out warps: producers with nothing to gather join
+  const uint32_t ring0 = epi0 + epi_bytes(!gathers);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool leader = !PAIR || (blockIdx.x & 1) == 0;
   const int nseg = (p.half + 63) >> 6;
@@ -179,7 +187,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
 
   if (tid == 0) {
     for (int s = 0; s < kMaxStages; ++s) {
-      mbar_init(smem_u32(&hdr->full[s]), (has_cp ? kProdThreads : 0) + (has_tma ? 1 : 0) + (PAIR && leader ? 1 : 0));      // (+ the peer's stage)
+      mbar_init(smem_u32(&hdr->full[s]), (has_cp ? kProdThreads : 0) + (has_tma ? 1 : 0));      // (a pair's: the leader's copy is used)
       mbar_init(smem_u32(&hdr->empty[s]), 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -217,6 +225,91 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
 
   if (hdr->abort_flag != 0u) {
     // fall through to the common exit
+  } else if (PAIR && warp < kProdWarps && gathers) {
+    // =========================== gather producers of a pair ===========================
+    // Every warp gathers the same rows of each stage, four at a time (tile::gather4).
+    const uint32_t table = smem0 + kDenseHeader;
+    auto get4 = [](uint32_t a, int (&r)[4]) {
+      asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+    };
+    Cursor at;
+    bool alive = true;
+    auto wait_free = [&]() {             // for the stage at `at`; its barrier (the leader's) and its first byte here; moves on
+      if (at.round > 0) alive = mbar_wait_all(smem_u32(&hdr->empty[at.slot]), (at.round - 1) & 1, abort_flag, p.status.word);
+    };
+    const uint32_t full0 = map_to_cta(smem_u32(&hdr->full[0]), 0);
+    if constexpr (OP != kOpDweight) {
+      constexpr int kQuads = kTileM / kProdWarps / 4;    // G, S: 16 rows a warp
+      const int steps = (p.C + kStep - 1) / kStep;
+      int t = 0;
+      for (Walk<OP, PAIR> u(p); u.left > 0 && alive; u.next(), ++t) {
+        alive = mbar_wait_all(smem_u32(&hdr->ids_full[t & 1]), (t >> 1) & 1, abort_flag, p.status.word);
+        if (!alive) break;
+        int row[kQuads][4];
+#pragma unroll
+        for (int q = 0; q < kQuads; ++q) get4(table + static_cast<uint32_t>((t & 1) * kTileM + (warp * kQuads + q) * 4) * 4u, row[q]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&hdr->ids_empty[t & 1]));
+        for (int k = 0; k < steps; ++k) {
+          wait_free();
+          if (!alive) break;
+          const uint32_t bar = full0 + at.slot * 8u;
+          const uint32_t dst = ring0 + static_cast<uint32_t>(at.slot) * stage_bytes + static_cast<uint32_t>(warp * kQuads) * 512u;
+          at.next(stages);
+          if (elect_one()) {
+#pragma unroll
+            for (int q = 0; q < kQuads; ++q) tma_gather4_pair(dst + q * 512u, &map_rows, k * kStep, row[q][0], row[q][1], row[q][2], row[q][3], bar);
+          }
+        }
+      }
+    } else {
+      constexpr int kQuads = kStep / kProdWarps / 4;     // 8 rows a warp
+      const uint32_t g_dst = p.swap ? kMTile : 0u, s_dst = p.swap ? 0u : kMTile;
+      const int g_seg = p.swap ? nseg : 2, s_seg = p.swap ? 2 : nseg;
+      int batch = 0;
+      for (Walk<OP, PAIR> u(p); u.left > 0 && alive; u.next()) {
+        const int steps = u.steps(), n0 = u.first_column();
+        const int gx = p.swap ? n0 : u.m0, sx = p.swap ? u.m0 : n0;
+        for (int k = 0; k < steps; ++k) {
+          constexpr int kBatchSteps = kBatch / kStep;
+          const int in_batch = k % kBatchSteps;
+          if (in_batch == 0) alive = mbar_wait_all(smem_u32(&hdr->ids_full[batch & 1]), (batch >> 1) & 1, abort_flag, p.status.word);
+          if (!alive) break;
+          int tok[kQuads][4], slot_row[kQuads][4];
+          const uint32_t ids = table + static_cast<uint32_t>((batch & 1) * kBatch + in_batch * kStep + warp * kQuads * 4) * 4u;
+#pragma unroll
+          for (int q = 0; q < kQuads; ++q) {
+            get4(ids + q * 16u, tok[q]);
+            if (!p.tma_rows) get4(ids + 2u * kBatch * 4u + q * 16u, slot_row[q]);
+          }
+          if (in_batch == kBatchSteps - 1 || k + 1 == steps) {                     // this warp has read the batch
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&hdr->ids_empty[batch & 1]));
+            ++batch;
+          }
+          wait_free();
+          if (!alive) break;
+          const uint32_t bar = full0 + at.slot * 8u;
+          const uint32_t dst = ring0 + static_cast<uint32_t>(at.slot) * stage_bytes + static_cast<uint32_t>(warp * kQuads) * 512u;
+          at.next(stages);
+          if (elect_one()) {
+#pragma unroll
+            for (int q = 0; q < kQuads; ++q) {
+#pragma unroll
+              for (int s = 0; s < 2; ++s)
+                if (s < g_seg) tma_gather4_pair(dst + g_dst + s * kSeg + q * 512u, &map_w, gx + s * 64, tok[q][0], tok[q][1], tok[q][2], tok[q][3], bar);
+              if (!p.tma_rows) {
+#pragma unroll
+                for (int s = 0; s < 2; ++s)
+                  if (s < s_seg)
+                    tma_gather4_pair(dst + s_dst + s * kSeg + q * 512u, &map_rows, sx + s * 64, slot_row[q][0], slot_row[q][1], slot_row[q][2], slot_row[q][3], bar);
+              }
+            }
+          }
+        }
+      }
+    }
+    __syncwarp();
   } else if (warp < kProdWarps && has_cp) {
     // =========================== gather producers ===========================
     const char* Rows = static_cast<const char*>(p.Rows);
@@ -520,12 +613,12 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
             make_idesc(Elem<T>::fmt, a_mn ? 1u : 0u, b_mn ? 1u : 0u, PAIR ? 2 * kTileM : kTileM, static_cast<uint32_t>(u.width()));
         const int buf = t & 1;
         if (t >= 2) {
-          ok = mbar_wait_all(smem_u32(&hdr->acc_empty[buf]), ((t >> 1) - 1) & 1, abort_flag, p.status.word);
+          ok = mbar_wait_all<PAIR>(smem_u32(&hdr->acc_empty[buf]), ((t >> 1) - 1) & 1, abort_flag, p.status.word);
           if (!ok) break;
         }
         const uint32_t d = tmem_base + static_cast<uint32_t>(buf) * acc_cols;
         for (int ks = 0; ks < steps; ++ks) {
-          ok = mbar_wait_all(smem_u32(&hdr->full[at.slot]), at.round & 1, abort_flag, p.status.word);
+          ok = mbar_wait_all<PAIR>(smem_u32(&hdr->full[at.slot]), at.round & 1, abort_flag, p.status.word);
           if (!ok) break;
           const uint32_t empty = smem_u32(&hdr->empty[at.slot]);
           // (descriptors: 14 address bits in 16-byte units; shared memory is smaller)
@@ -537,21 +630,6 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
             umma_done<PAIR>(empty);
             if (ks + 1 == steps) umma_done<PAIR>(smem_u32(&hdr->acc_full[buf]));
           }
-        }
-      }
-    } else if (PAIR) {
-      // the peer tells the leader of every stage that has landed here
-      const uint32_t to_leader = map_to_cta(smem_u32(&hdr->full[0]), 0);
-      bool ok = true;
-      Cursor at;
-      for (Walk<OP, PAIR> u(p); u.left > 0 && ok; u.next()) {
-        const int steps = u.steps();
-        for (int ks = 0; ks < steps; ++ks) {
-          ok = mbar_wait_all(smem_u32(&hdr->full[at.slot]), at.round & 1, abort_flag, p.status.word);
-          if (!ok) break;
-          const uint32_t there = to_leader + at.slot * 8u;
-          at.next(stages);
-          if (elect_one()) mbar_arrive_cluster_relaxed(there);
         }
       }
     }
@@ -568,7 +646,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       unsigned long long* empty = dst ? hdr->dst_empty : hdr->ids_empty;
       if (dst && OP == kOpScatter) pdl_wait();           // planning flags
       int t = 0;
-      for (Walk<OP, PAIR> u(p); (dst || has_cp) && u.left > 0 && alive; u.next(), ++t) {
+      for (Walk<OP, PAIR> u(p); (dst || gathers) && u.left > 0 && alive; u.next(), ++t) {
         int row[4], b[4], f32[4];
         long long id[4];
 #pragma unroll
@@ -635,7 +713,8 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     }
   } else if (has_tma) {
     // =========================== TMA issuer ===========================
-    const uint32_t bytes = (OP != kOpDweight ? n_bytes : (p.swap ? kMTile : n_bytes)) + ((OP == kOpScatter && p.tma_rows) ? kMTile : 0u);
+    // a pair's stage is announced by the leader, for both CTAs and for what the producers gather
+    const uint32_t bytes = PAIR ? 2u * stage_bytes : (OP != kOpDweight ? n_bytes : (p.swap ? kMTile : n_bytes)) + ((OP == kOpScatter && p.tma_rows) ? kMTile : 0u);
     bool ok = true;
     Cursor at;
     for (Walk<OP, PAIR> u(p); u.left > 0 && ok; u.next()) {
@@ -648,25 +727,34 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           ok = mbar_wait_all(smem_u32(&hdr->empty[at.slot]), (at.round - 1) & 1, abort_flag, p.status.word);
           if (!ok) break;
         }
-        const uint32_t bar = smem_u32(&hdr->full[at.slot]), base = ring0 + static_cast<uint32_t>(at.slot) * stage_bytes;
+        const uint32_t own = smem_u32(&hdr->full[at.slot]), base = ring0 + static_cast<uint32_t>(at.slot) * stage_bytes;
+        const uint32_t bar = PAIR ? map_to_cta(own, 0) : own;
         at.next(stages);
+        auto box3 = [&](uint32_t dst, int x, int y) {
+          if (PAIR) tma_load_3d_pair(dst, &map_w, x, y, u.e, bar);
+          else tma_load_3d(dst, &map_w, x, y, u.e, bar);
+        };
+        auto box4 = [&](uint32_t dst, int x) {
+          if (PAIR) tma_load_4d_pair(dst, &map_rows, x, k, u.e, b, bar);
+          else tma_load_4d(dst, &map_rows, x, k, u.e, b, bar);
+        };
         if (elect_one()) {
-          mbar_arrive_expect_tx(bar, bytes);
+          if (leader) mbar_arrive_expect_tx(own, bytes);
           if (OP != kOpDweight) {
-            if (OP == kOpScatter && p.tma_rows) tma_load_4d(base, &map_rows, c0, k, u.e, b, bar);
+            if (OP == kOpScatter && p.tma_rows) box4(base, c0);
             if (p.nc) {
-              tma_load_3d(base + kMTile, &map_w, c0, n0, u.e, bar);
+              box3(base + kMTile, c0, n0);
             } else {
 #pragma unroll
               for (int s = 0; s < 4; ++s)
-                if (s < nseg) tma_load_3d(base + kMTile + s * kSeg, &map_w, n0 + s * 64, c0, u.e, bar);
+                if (s < nseg) box3(base + kMTile + s * kSeg, n0 + s * 64, c0);
             }
-          } else {
+          } else if (p.tma_rows) {
             const int ns = p.swap ? 2 : nseg, x0 = p.swap ? u.m0 : n0;
             const uint32_t dst = base + (p.swap ? 0u : kMTile);
 #pragma unroll
             for (int s = 0; s < 4; ++s)
-              if (s < ns) tma_load_4d(dst + s * kSeg, &map_rows, x0 + s * 64, k, u.e, b, bar);
+              if (s < ns) box4(dst + s * kSeg, x0 + s * 64);
           }
         }
         if (OP == kOpDweight) {
@@ -707,6 +795,12 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
 // Slot rows can come as one TMA box per 64-element column segment when `rows` consecutive expert rows starting at a multiple of
 // `rows` are whole batch elements or lie inside one.
 bool rows_fit_boxes(int K, int rows) { return K % rows == 0 || rows % K == 0; }
+// The same rows one by one, for tile::gather4: rows of 64 elements of a [rows, width] matrix.
+bool encode_gather(TensorMap3* map, const void* base, long long rows, int width) {
+  const unsigned long long dims[2] = {static_cast<unsigned long long>(width), static_cast<unsigned long long>(rows)};
+  const unsigned box[2] = {64u, 1u};
+  return encode_tensor_map_16bit(map, base, 2, dims, box);
+}
 bool encode_slot_rows(TensorMap3* map, const void* base, int B, int E, int K, int width, int rows) {
   const unsigned kk = static_cast<unsigned>(K < rows ? K : rows);
   const unsigned long long dims[4] = {static_cast<unsigned long long>(width), static_cast<unsigned long long>(K),
@@ -816,6 +910,9 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
   const unsigned box[3] = {64u, p.nc ? static_cast<unsigned>(p.half) : static_cast<unsigned>(kStep), 1u};
   if (!encode_tensor_map_16bit(&mw, r.W, 3, dims, box)) return cudaErrorInvalidValue;
   p.tma_rows = scatter && rows_fit_boxes(r.K, 128) && encode_slot_rows(&mr, r.A, r.B, r.E, r.K, r.C, 128);
+  if (r.pair && !p.tma_rows &&
+      !encode_gather(&mr, r.A, scatter ? static_cast<long long>(r.M) * r.E : static_cast<long long>(r.B) * r.T, r.C))
+    return cudaErrorInvalidValue;
   if (scatter)
     return r.pair ? launch_typed<kOpScatter, true>(p, dtype, mw, mr, r.after_own != 0, st)
                   : launch_typed<kOpScatter, false>(p, dtype, mw, mr, r.after_own != 0, st);
@@ -877,6 +974,9 @@ cudaError_t launch_dense16_dweight(const DWeightParams& r, int dtype, cudaStream
   p.units = static_cast<int>(units);
   TensorMap3 mw{}, mr{};
   p.tma_rows = rows_fit_boxes(r.K, kStep) && encode_slot_rows(&mr, r.Ysrc, r.B, r.E, r.K, r.FD, kStep);
+  if (r.pair && (!encode_gather(&mw, r.Xsrc, static_cast<long long>(r.B) * r.T, r.FG) ||
+                 (!p.tma_rows && !encode_gather(&mr, r.Ysrc, static_cast<long long>(r.M) * r.E, r.FD))))
+    return cudaErrorInvalidValue;
   return r.pair ? launch_typed<kOpDweight, true>(p, dtype, mw, mr, r.after_own != 0, st)
                 : launch_typed<kOpDweight, false>(p, dtype, mw, mr, r.after_own != 0, st);
 }

@@ -106,14 +106,29 @@ __device__ __forceinline__ uint32_t mbar_try(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok;
 }
+// The same for a barrier that the other CTA of a pair arrives on: what was released there is visible here.
+__device__ __forceinline__ uint32_t mbar_try_pair(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(kTryWaitSuspendNs)
+      : "memory");
+  return ok;
+}
+
 // Bounded wait.  Returns false when the CTA is aborting (this or another thread ran out of time).
+template <bool FROM_PAIR = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag,
                                           int32_t* status, long long limit_cycles = kWaitLimitCycles) {
-  if (mbar_try(bar, parity)) return true;
+  auto arrived = [&]() { return (FROM_PAIR ? mbar_try_pair(bar, parity) : mbar_try(bar, parity)) != 0u; };
+  if (arrived()) return true;
   const long long t0 = clock64();
   uint32_t spins = 0;
   for (;;) {
-    if (mbar_try(bar, parity)) return true;
+    if (arrived()) return true;
     if (((++spins) & 63u) == 0u) {
       if (*abort_flag) return false;
       if (clock64() - t0 > limit_cycles) {
@@ -137,9 +152,10 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
 // elected lane (the same one each time for a full mask) issues.  Descriptors, coordinates and barrier addresses then live in
 // uniform registers.  The same loops inside `if (lane == 0)` spent 700 clocks a step on four MMAs and a commit, more than the
 // tensor core needs for a 128 x 256 x 64 step (512).
+template <bool FROM_PAIR = false>
 __device__ __forceinline__ bool mbar_wait_all(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, int32_t* status) {
-  if (__all_sync(0xffffffffu, mbar_try(bar, parity) != 0u)) return true;
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status)) != 0;
+  if (__all_sync(0xffffffffu, (FROM_PAIR ? mbar_try_pair(bar, parity) : mbar_try(bar, parity)) != 0u)) return true;
+  return __all_sync(0xffffffffu, mbar_wait<FROM_PAIR>(bar, parity, abort_flag, status)) != 0;
 }
 __device__ __forceinline__ bool elect_one() {
   uint32_t on;
@@ -248,13 +264,34 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t ran
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
   return r;
 }
-// Arrival on another CTA's barrier without a release: nothing this thread has written is handed over.  (With release semantics the
-// thread waits behind a cluster-wide memory barrier on every arrival, 1400 clocks under load.)
+// Arrivals on another CTA's barrier.  The releasing one hands over what this thread has written, or has observed to be written, to a
+// waiter that acquires at cluster scope, and waits behind a cluster-wide memory barrier for it (1400 clocks under load); the relaxed
+// one orders nothing: only for what is complete by other means.
 __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// TMA tile loads of a CTA of a pair into its own shared memory, the bytes counted on a barrier of either CTA (shared::cluster address)
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst_smem, const void* tensor_map, int x, int y, int z, uint32_t cluster_bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst_smem),
+      "l"(tensor_map), "r"(x), "r"(y), "r"(z), "r"(cluster_bar)
+      : "memory");
+}
+// ... four rows of 128 bytes of a 2-D map (box of one row), one below the other; rows outside the tensor read as zeros
+__device__ __forceinline__ void tma_gather4_pair(uint32_t dst_smem, const void* tensor_map, int x, int r0, int r1, int r2, int r3, uint32_t cluster_bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst_smem),
+      "l"(tensor_map), "r"(x), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(cluster_bar)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst_smem, const void* tensor_map, int x, int y, int z, int w, uint32_t cluster_bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst_smem),
+      "l"(tensor_map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(cluster_bar)
+      : "memory");
 }
 __device__ __forceinline__ void tmem_alloc2(uint32_t smem_dst, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");

@@ -144,6 +144,37 @@ def test_dense16_edges(cuda_device, B, T, E, K, I, J, bias):
     same(ops.dweight(d["G"], d["Y"], d["Ind"], out_layout="direct_rows", path="tensor"), orc.np_dweight(G, Y, Ind).transpose(0, 2, 1))
 
 
+# pairs of SMs: the leader multiplies what both CTAs have staged.  The same launches over and over, under copies on another stream
+# that disturb their timing, give the same bits (integer values: every sum is exact in any order), with slot rows that come as boxes
+# (K = 64) and that are gathered (K = 72)
+@pytest.mark.parametrize("B,T,E,K,I,J", [(20, 200, 24, 64, 520, 512), (24, 600, 40, 72, 1280, 320)])
+def test_dense16_pairs_repeat_their_bits(cuda_device, B, T, E, K, I, J):
+    g = torch.Generator(device=cuda_device).manual_seed(J)
+    dt = torch.float16
+    small = lambda *shape: torch.randint(-1, 2, shape, generator=g, device=cuda_device).to(dt)
+    X, Y, Wg, Ws = small(B, T, I), small(B, E, K, J), small(E, I, J), small(E, J, I)
+    Ind = (torch.arange(B * E * K, device=cuda_device).view(B, E, K) * 7) % T
+    runs = {"G": lambda: ops.gather_gemm(X, Wg, Ind), "dY": lambda: ops.gather_gemm(X, Ws, Ind, w_layout="nc"),
+            "S": lambda: ops.gemm_scatter(Y, Ws, Ind, T), "dX": lambda: ops.gemm_scatter(Y, Wg, Ind, T, w_layout="nc"),
+            "D": lambda: ops.dweight(X, Y, Ind), "D direct": lambda: ops.dweight(X, Y, Ind, out_layout="direct_rows")}
+    rows = torch.gather(X.float(), 1, Ind.reshape(B, -1, 1).expand(-1, -1, I)).reshape(B, E, K, I)
+    outs = torch.einsum("bekj,eji->beki", Y.float(), Ws.float())
+    want = {"G": torch.einsum("beki,eij->bekj", rows, Wg.float()), "D": torch.einsum("beki,bekj->eij", rows, Y.float()),
+            "S": torch.zeros(B, T, I, device=cuda_device).scatter_add_(1, Ind.reshape(B, -1, 1).expand(-1, -1, I), outs.reshape(B, -1, I))}
+    first = {k: f() for k, f in runs.items()}
+    for k, w in want.items():
+        assert w.abs().max() <= 2048 and torch.equal(first[k].float(), w), k
+    assert torch.equal(first["D direct"], first["D"].transpose(1, 2))
+    other, noise = torch.cuda.Stream(), torch.empty(1 << 25, device=cuda_device)
+    for i in range(40):
+        with torch.cuda.stream(other):
+            noise[: 1 << (16 + i % 10)].add_(1.0)
+        for k, f in runs.items():
+            assert torch.equal(f(), first[k]), (k, i)
+    torch.cuda.synchronize()
+    ops.check_status()
+
+
 # 16-bit scatter: the choice between direct additions and float32 rows is made per batch element; tiles of 128 expert rows here
 # span batch elements of both kinds (K = 48), the persistent kernel (N = 1032) and the one-tile kernel (long contraction)
 @pytest.mark.parametrize("C,N", [(40, 72), (256, 1032), (520, 64)])
