@@ -620,6 +620,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
         for (int ks = 0; ks < steps; ++ks) {
           ok = mbar_wait_all<PAIR>(smem_u32(&hdr->full[at.slot]), at.round & 1, abort_flag, p.status.word);
           if (!ok) break;
+          if (has_cp) fence_proxy_async_smem();
           const uint32_t empty = smem_u32(&hdr->empty[at.slot]);
           // (descriptors: 14 address bits in 16-byte units; shared memory is smaller)
           const uint32_t addr = (ring0 + static_cast<uint32_t>(at.slot) * stage_bytes) >> 4;

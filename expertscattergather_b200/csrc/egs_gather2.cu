@@ -239,8 +239,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kG2Threads, 1) tenso
         tc_fence_after();
         for (int ks = 0; ks < nk && ok; ++ks) {
           ok = mbar_wait(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status.word);
-          if (ok) ok = mbar_wait(smem_u32(&hdr->peer_full[slot]), round & 1, abort_flag, p.status.word);
+          if (ok) ok = mbar_wait<true>(smem_u32(&hdr->peer_full[slot]), round & 1, abort_flag, p.status.word);
           if (!ok) break;
+          fence_proxy_async_smem();
           tc_fence_after();
           const uint32_t base = (ring0 + static_cast<uint32_t>(slot) * stage_bytes) & 0x3FFFFu;   // offset inside the CTA
           const uint64_t bd = b_desc0 + ((base + a_bytes) >> 4);

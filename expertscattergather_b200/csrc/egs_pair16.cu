@@ -404,6 +404,7 @@ __global__ void __launch_bounds__(kP16Threads, 1) tensor_pair16_persistent_kerne
       auto mma_g = [&](int ks) {                 // one G stage into acc1
         ok = mbar_wait(smem_u32(&hdr->full[ring.slot]), ring.round & 1, abort_flag, p.status.word);
         if (!ok) return;
+        fence_proxy_async_smem();
         const uint32_t base = ring0 + static_cast<uint32_t>(ring.slot) * slot_bytes;
         const uint64_t ad = a_desc0 + (base >> 4);
         const uint64_t bd = b1_desc0 + ((base + a_bytes) >> 4);

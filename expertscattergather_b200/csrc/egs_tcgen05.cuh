@@ -75,6 +75,8 @@ __device__ __forceinline__ void cp_async_wait_pending(int n) {
     default: asm volatile("cp.async.wait_group 6;" ::: "memory"); break;
   }
 }
+// Shared memory written through the generic proxy (st.shared, cp.async) is read by the tensor core through the async proxy: the
+// fence stands between, in the writing thread before it arrives or in the waiting one after it has seen the arrival.
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");

@@ -142,6 +142,7 @@ __device__ __forceinline__ void run_mma_lane(const Pipe& pp, Mma&& mma) {
     const int slot = ks % pp.stages;
     ok = mbar_wait(smem_u32(&hdr->full[slot]), (ks / pp.stages) & 1, pp.abort_flag, pp.status.word);
     if (!ok) break;
+    fence_proxy_async_smem();
     tc_fence_after();
     mma(ks, pp.tiles0 + slot * pp.stage_bytes);
     umma_commit(smem_u32(&hdr->empty[slot]));
@@ -712,6 +713,7 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
             const int slot = g % stages;
             ok = mbar_wait(smem_u32(&hdr->full[slot]), (g / stages) & 1, abort_flag, p.status.word);
             if (!ok) break;
+            fence_proxy_async_smem();
             tc_fence_after();
             const uint32_t a_hi = tiles0 + slot * stage_bytes;
             uint64_t ad = make_smem_desc(a_hi, 16u, 1024u);
