@@ -30,6 +30,7 @@
 // issuing warps run converged (see mbar_wait_all) and ids are looked up elsewhere.
 // T=1024, E=64, K=64, I=1024, J=256, bf16: B=64 G 126-138 us, S 215, D 148-165; B=512 G 950 us, dY (weights [E, N, C]) 895 = 1.23
 // PFLOP/s, S 1450, D 1050, under the power cap.
+#include <algorithm>
 #include <type_traits>
 
 #include "egs_tcgen05.cuh"
@@ -920,11 +921,16 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
   return r.pair ? launch_typed<kOpGather, true>(p, dtype, mw, mr, false, st) : launch_typed<kOpGather, false>(p, dtype, mw, mr, false, st);
 }
 
+// Rows one accumulator of D sums: the tensor core truncates as it adds, and the error grows with the number of additions, 1.5e-5 of
+// the largest sum after 8192 rows. The ranges of a longer contraction are added by float32 atomics, which round.
+constexpr int kMaxRangeRows = 8192;
+
 // D: which operand's features are the accumulator's rows, the tile, and the row ranges.
 void configure_dense16_dweight(DWeightParams& p) {
   const bool slot_cp = !rows_fit_boxes(p.K, kStep);
   double best = 1e30;
   const long long steps_all = (p.M + kStep - 1) / kStep;
+  const long long least = (p.M + kMaxRangeRows - 1) / kMaxRangeRows, most = std::min(std::max(64ll, least), steps_all);
   // the orientation whose accumulator rows are the output's rows first: its read-out stores whole row segments
   const bool pref = p.out_layout == EGS_DW_DIRECT_ROWS;
   for (int o = 0; o < 2; ++o) {
@@ -932,7 +938,7 @@ void configure_dense16_dweight(DWeightParams& p) {
     const int mf = sw ? p.FD : p.FG, nf = sw ? p.FG : p.FD;
     // load/store clocks per step: 10 per 512 bytes; the gathered operand always, the slot operand where it has no boxes
     const double lsu0 = (!sw ? 320.0 : 0.0) + (sw && slot_cp ? 320.0 : 0.0), lsu1 = (sw ? 2.5 : 0.0) + (!sw && slot_cp ? 2.5 : 0.0);
-    for (int s = 1; s <= 64 && s <= steps_all; s = s < 4 ? s + 1 : s + s / 2) {
+    for (long long s = least; s <= most; s = s < 4 ? s + 1 : s + s / 2) {
       const long long sp_steps = (steps_all + s - 1) / s;
       const long long real = (steps_all + sp_steps - 1) / sp_steps;      // ranges of whole steps
       const double epi = real > 1 ? 32.0 : o == 0 ? 16.0 : 20.0;         // (partial tiles are added atomically)

@@ -144,6 +144,23 @@ def test_dense16_edges(cuda_device, B, T, E, K, I, J, bias):
     same(ops.dweight(d["G"], d["Y"], d["Ind"], out_layout="direct_rows", path="tensor"), orc.np_dweight(G, Y, Ind).transpose(0, 2, 1))
 
 
+# 16-bit weight gradients: one accumulator sums at most 8192 rows.  Values of one sign: its truncating additions (16 products each)
+# all err the same way, by at most a unit in the last place of the result, and fp16 rounding has no bias over 10^7 elements
+@pytest.mark.parametrize("B,T,E,K,I,J", [(200, 64, 18, 177, 1984, 288)])
+def test_dense16_dweight_sums_long_contractions_in_ranges(cuda_device, B, T, E, K, I, J):
+    assert ops.describe_plan("D", B, T, E, K, I, J, torch.float16)["rows_per_split"] <= 8192
+    g = torch.Generator(device=cuda_device).manual_seed(5)
+    X, Y = (torch.rand(s, generator=g, device=cuda_device).mul_(0.05).half() for s in ((B, T, I), (B, E, K, J)))
+    Ind = torch.randint(0, T, (B, E, K), generator=g, device=cuda_device)
+    got = ops.dweight(X, Y, Ind).double()
+    bias = []
+    for e in range(E):
+        rows = X[torch.arange(B, device=cuda_device)[:, None], Ind[:, e]].reshape(B * K, I).double()
+        ref = rows.T @ Y[:, e].reshape(B * K, J).double()
+        bias.append(((got[e] - ref) / ref).mean())
+    assert torch.stack(bias).mean().abs().item() <= 8192 / 16 * 2.0 ** -23
+
+
 # pairs of SMs: the leader multiplies what both CTAs have staged.  The same launches over and over, under copies on another stream
 # that disturb their timing, give the same bits (integer values: every sum is exact in any order), with slot rows that come as boxes
 # (K = 64) and that are gathered (K = 72)
