@@ -136,9 +136,9 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
   const bool no_work = (d.B * d.E * d.K == 0);
   if (!no_work && (!A || !W || !Ind) && d.C > 0) return EGS_ERR_INVALID_ARGUMENT;
 
-  // 16-bit scatter.  Workspace layout: [256 B unused][planning flags, B ints in room for B*T][float32 rows, B*T*N].  Generic
-  // kernels always sum in the float32 rows; the tensor-core path decides per batch element between those and direct 16-bit
-  // additions (see egs_generic.cu).
+  // 16-bit scatter.  Workspace layout: [plan flag, 256 B][counting flags, room for B*T ints][float32 rows, B*T*N].  Generic
+  // kernels always sum in the float32 rows; the tensor-core path decides between those and direct 16-bit additions (see
+  // egs_generic.cu).
   const bool f32_rows = scatter && dtype != EGS_F32;
   const size_t n_out = static_cast<size_t>(out_rows) * d.N;
   float* acc = nullptr;
@@ -161,9 +161,9 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
     acc = reinterpret_cast<float*>(ws + 256 + counter_bytes);
     cudaError_t err;
     if (tensor && !no_work && d.C > 0) {
-      plan = reinterpret_cast<int*>(ws + 256);
+      plan = reinterpret_cast<int*>(ws);
       err = launch_scatter_prepare(Ind, index_dtype, static_cast<int>(d.B), static_cast<int>(d.T), static_cast<int>(d.E),
-                                   static_cast<int>(d.K), csr_info, kDirect16Limit, plan, acc, Out, static_cast<int>(d.N),
+                                   static_cast<int>(d.K), csr_info, kDirect16Limit, plan + 64, plan, acc, Out, static_cast<int>(d.N),
                                    zero_output, dtype, status_ref(status), st);
       own = true;
     } else {
@@ -177,7 +177,7 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
   }
   auto finish_rows = [&]() -> int {
     if (!f32_rows) return EGS_OK;
-    cudaError_t err = plan ? launch_scatter_finish(plan, acc, Out, static_cast<int>(d.B), static_cast<size_t>(d.T) * d.N, dtype, st)
+    cudaError_t err = plan ? launch_scatter_finish(plan, acc, Out, n_out, dtype, st)
                            : launch_convert_from_f32(acc, Out, n_out, dtype, st);
     return err == cudaSuccess ? EGS_OK : fail_cuda(err, "scatter scratch convert");
   };
@@ -422,9 +422,9 @@ int egs_gather_scatter_pair(const void* Src, const void* W1, const void* W2, con
   if (!workspace || workspace_bytes < need || !aligned16(workspace)) return EGS_ERR_WORKSPACE;
   char* ws = static_cast<char*>(workspace);
   const size_t counter_bytes = (static_cast<size_t>(B) * T * sizeof(int) + 255) & ~static_cast<size_t>(255);
-  int* plan = reinterpret_cast<int*>(ws + 256);
+  int* plan = reinterpret_cast<int*>(ws);
   float* acc = reinterpret_cast<float*>(ws + 256 + counter_bytes);
-  cudaError_t err = launch_scatter_prepare(Ind, index_dtype, p.B, p.T, p.E, p.K, nullptr, kDirect16Limit, plan, acc, Dst, p.N2, zero_output,
+  cudaError_t err = launch_scatter_prepare(Ind, index_dtype, p.B, p.T, p.E, p.K, nullptr, kDirect16Limit, plan + 64, plan, acc, Dst, p.N2, zero_output,
                                            dtype, status_ref(status_word), st);
   if (err != cudaSuccess) return fail_cuda(err, "scatter preparation");
   p.after_own = 1;
@@ -439,7 +439,7 @@ int egs_gather_scatter_pair(const void* Src, const void* W1, const void* W2, con
   if (smem == 0) return EGS_ERR_UNSUPPORTED;
   err = launch_tensor_pair16(p, dtype, smem, st);
   if (err != cudaSuccess) return fail_cuda(err, "gather_scatter_pair launch");
-  err = launch_scatter_finish(plan, acc, Dst, p.B, static_cast<size_t>(p.T) * p.N2, dtype, st);
+  err = launch_scatter_finish(plan, acc, Dst, n_dst, dtype, st);
   return err == cudaSuccess ? EGS_OK : fail_cuda(err, "scatter scratch convert");
 }
 

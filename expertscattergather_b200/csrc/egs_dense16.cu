@@ -50,9 +50,8 @@ constexpr int kBatch = 256;                        // D: contraction rows whose 
 // D: two batches of token rows; without TMA boxes for the slot rows two of those as well.  (Sized so that four stages of a
 // 128 x 256 tile still fit beside it with TMA boxes: three stages cost a quarter of the rate.)
 __host__ __device__ constexpr uint32_t table_bytes(bool slots) { return (slots ? 4u : 2u) * kBatch * 4u; }
-// G, S: source rows of two units, then destination rows of two units (kNoRow: none; top bit: added to the float32 rows)
+// G, S: source rows of two units, then destination rows of two units (-1: none)
 constexpr uint32_t kRowTable = 4u * kTileM * 4u;
-constexpr int kNoRow = 0x7fffffff;
 constexpr uint32_t kMTile = 16384;                 // bytes of the 128-wide operand: 128 rows x 64 elements, or 64 rows x 128
 constexpr uint32_t kSeg = kStep * 128u;            // one 64-column segment of a 64-row tile
 __host__ __device__ constexpr uint32_t epi_bytes(bool wide) { return (wide ? kProdWarps + kEpiWarps : kEpiWarps) * 4096u; }       // transposes of the read-out
@@ -471,13 +470,13 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     const uint32_t lane_base = static_cast<uint32_t>(lg * 32) << 16;
     T* out = static_cast<T*>(p.Out);
     bool alive = true;
-    pdl_wait();                                          // zeros the results are added to
+    pdl_wait();                                          // zeros the results are added to, the scatter's plan
+    const bool f32_rows = OP == kOpScatter && *p.plan != 0;
     int t = 0;
     for (Walk<OP, PAIR> u(p); u.left > 0 && alive; u.next(), ++t) {
       const int bn = min(p.BN, p.N - u.n0);              // columns of this tile (a multiple of 8)
       const int n_end = u.n0 + bn;
       int my_ro = -1;                                    // G, S: destination row of tile row lg * 32 + lane
-      uint32_t to_f32 = 0u;
       if (OP != kOpDweight) {
         alive = mbar_wait_all(smem_u32(&hdr->dst_full[t & 1]), (t >> 1) & 1, abort_flag, p.status.word);
         if (!alive) break;
@@ -485,11 +484,6 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
                      : "r"(smem0 + kDenseHeader + static_cast<uint32_t>((2 + (t & 1)) * kTileM + lg * 32 + lane) * 4u) : "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&hdr->dst_empty[t & 1]));
-        if (OP == kOpScatter) {
-          to_f32 = __ballot_sync(0xffffffffu, my_ro < 0);
-          my_ro &= 0x7fffffff;
-        }
-        if (my_ro == kNoRow) my_ro = -1;
       }
       const T* bias_row = (OP != kOpDweight && p.bias) ? static_cast<const T*>(p.bias) + static_cast<long long>(u.e) * p.N + u.n0 : nullptr;
       const int buf = t & 1;
@@ -507,7 +501,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
         }
         released = true;
       };
-      const bool packed = OP == kOpGather || (OP == kOpScatter && to_f32 == 0u) || (OP == kOpDweight && p.splits == 1 && p.lane_rows);
+      const bool packed = OP == kOpGather || (OP == kOpScatter && !f32_rows) || (OP == kOpDweight && p.splits == 1 && p.lane_rows);
       if (packed) {
         // 64 columns = 128 bytes of a 16-bit row at a time, eight lanes to a row: S adds 16 bytes a lane (the memory system takes
         // 39 KB a microsecond from an SM that way).  Bulk reductions of 128 bytes, one per row and lane, took 85 clocks each to
@@ -575,8 +569,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
               if (ro >= 0 && col < n_end) {
                 const long long off = static_cast<long long>(ro) * p.N + col;
                 if (bias_row) add_bias4<T>(bias_row + c * 32 + cj, x0, x1, x2, x3);
-                if ((to_f32 >> row) & 1u) red4(p.acc + off, x0, x1, x2, x3);
-                else red4(out + off, x0, x1, x2, x3);
+                red4(p.acc + off, x0, x1, x2, x3);
               }
             });
           } else if (OP == kOpDweight && p.lane_rows) {  // partial sums, output rows = accumulator rows
@@ -646,10 +639,9 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       const bool dst = warp != kIndexWarp;
       unsigned long long* full = dst ? hdr->dst_full : hdr->ids_full;
       unsigned long long* empty = dst ? hdr->dst_empty : hdr->ids_empty;
-      if (dst && OP == kOpScatter) pdl_wait();           // planning flags
       int t = 0;
       for (Walk<OP, PAIR> u(p); (dst || gathers) && u.left > 0 && alive; u.next(), ++t) {
-        int row[4], b[4], f32[4];
+        int row[4], b[4];
         long long id[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -657,7 +649,6 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           b[i] = m / p.K;
           row[i] = m < p.M ? (b[i] * p.E + u.e) * p.K + (m - b[i] * p.K) : -1;
           id[i] = (row[i] >= 0 && (dst || OP == kOpGather)) ? load_index(p.Ind, p.index_dtype, row[i]) : 0;
-          f32[i] = (OP == kOpScatter && dst && row[i] >= 0) ? p.plan[b[i]] : 0;
         }
         if (t >= 2) alive = mbar_wait_all(smem_u32(&empty[t & 1]), ((t >> 1) - 1) & 1, abort_flag, p.status.word);
         if (!alive) break;
@@ -670,8 +661,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
             v = OP == kOpScatter ? row[i] : (known ? token_row : -1);
           } else {
             if (row[i] >= 0 && !known && u.n0 == 0) p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
-            if (OP == kOpGather) v = row[i] >= 0 ? row[i] : kNoRow;
-            else v = known ? (f32[i] ? static_cast<int>(static_cast<unsigned>(token_row) | 0x80000000u) : token_row) : kNoRow;
+            v = OP == kOpGather ? row[i] : known ? token_row : -1;
           }
           asm volatile("st.shared.b32 [%0], %1;" ::"r"(table + static_cast<uint32_t>(((dst ? 2 : 0) + (t & 1)) * kTileM + lane + 32 * i) * 4u), "r"(v) : "memory");
         }

@@ -429,53 +429,72 @@ __global__ void __launch_bounds__(256) convert_to_f32_kernel(const T* __restrict
 // Adding straight into a bf16/fp16 output rounds at every addition, which is accurate enough only while few
 // contributions meet in one token row; summing in float32 rows and rounding once is always accurate but costs
 // a float32 fill, float32 atomics on a buffer twice the size and a conversion pass.  The choice is made on the
-// device, per call and batch element, from the actual indices: plan[b] != 0 selects the float32 rows.
-// One kernel counts and zeroes: every CTA counts the slots of its batch element in shared memory (4096 ids: about 2 us, under
-// the stores of the other CTAs) and zeroes its share of the buffer the additions of that batch element go to.  A chain of a
-// counter fill, a counting pass over global atomics and an init pass took three launches and 10-14 us of gaps and kernels
-// (with the dependent launches, a serving pass of one 64-token prompt went from 37 to 27 us).
+// device, per call, from the actual indices: *plan != 0 selects the float32 rows.  One hot row anywhere selects them for every row
+// of the call, so that what a row is summed in does not depend on its own luck alone.
+// The ids of a batch element are counted in shared memory by one CTA (4096 ids: about 2 us) of a kernel of their own, with a flag
+// per CTA; the kernel that zeroes what the additions go to starts under it (dependent launch) and collects the flags: 2 us of the
+// chain.  With a single batch element, or few ids in all (kPrepOwnIds: as long to count as the second launch takes), the CTAs of the
+// zeroing kernel count everything themselves: a serving pass of one 64-token prompt has 25 us in all.
 // Sequences beyond kPrepCounters tokens share counters (token id modulo kPrepCounters): that can choose the float32 rows where
 // they are not needed, never the reverse.
 constexpr int kPrepThreads = 512;
 constexpr int kPrepCounters = 50 * 1024;
+constexpr int kPrepCountCtas = 4 * 148;
+constexpr int kPrepOwnIds = 8192;
+
+// whether a token row of batch elements b0 .. b0 + nb - 1 gets more than `limit` contributions, counted by the whole CTA;
+// cnt: [min(nb * T_, kPrepCounters)]
+__device__ __forceinline__ int has_hot_row(const void* __restrict__ ind, int index_dtype, int b0, int nb, int T_, int EK, int limit, int* cnt) {
+  const int tid = threadIdx.x, nc = static_cast<int>(min(static_cast<long long>(nb) * T_, static_cast<long long>(kPrepCounters)));
+  for (int t = tid; t < nc; t += kPrepThreads) cnt[t] = 0;
+  __syncthreads();
+  int over = 0;
+  for (int s = tid; s < nb * EK; s += kPrepThreads) {
+    const long long t = load_index(ind, index_dtype, static_cast<long long>(b0) * EK + s);
+    if (t >= 0 && t < T_) over |= atomicAdd(&cnt[(s / EK * T_ + static_cast<int>(t)) % nc], 1) >= limit;
+  }
+  return __syncthreads_or(over);         // (and the counters may be used again)
+}
+
+__global__ void __launch_bounds__(kPrepThreads) scatter_count_kernel(const void* __restrict__ ind, int index_dtype, int B, int T_, int EK,
+                                                                     int limit, int* __restrict__ flags) {
+  extern __shared__ int prep_cnt[];
+  pdl_trigger();
+  int flag = 0;
+  for (int b = blockIdx.x; b < B && !flag; b += gridDim.x) flag = has_hot_row(ind, index_dtype, b, 1, T_, EK, limit, prep_cnt);
+  if (threadIdx.x == 0) flags[blockIdx.x] = flag;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kPrepThreads) scatter_prepare_kernel(const void* __restrict__ ind, int index_dtype, int B, int T_, int EK,
-                                                                       const int* __restrict__ info, int limit,
-                                                                       int* __restrict__ plan, float* __restrict__ acc, T* __restrict__ out,
-                                                                       size_t per_batch, int zero_output, StatusRef status) {
-  extern __shared__ int prep_cnt[];      // [min(T_, kPrepCounters)] without `info`
+                                                                       const int* __restrict__ info, const int* __restrict__ flags, int nflags,
+                                                                       int limit, int* __restrict__ plan, float* __restrict__ acc,
+                                                                       T* __restrict__ out, size_t n, int zero_output, StatusRef status) {
+  extern __shared__ int prep_cnt[];      // without `info` and `flags`
   pdl_trigger();
   const int tid = threadIdx.x;
-  for (int b = blockIdx.y; b < B; b += gridDim.y) {
-    int flag = 0;
-    if (info) {
-      flag = info[0] > limit;
-      if (info[2] && blockIdx.x == 0 && b == 0 && tid == 0) status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
-    } else if (EK > limit) {
-      const int nc = min(T_, kPrepCounters);
-      for (int t = tid; t < nc; t += kPrepThreads) prep_cnt[t] = 0;
-      __syncthreads();
-      int over = 0;
-      for (int s = tid; s < EK; s += kPrepThreads) {
-        const long long t = load_index(ind, index_dtype, static_cast<long long>(b) * EK + s);
-        if (t >= 0 && t < T_) over |= atomicAdd(&prep_cnt[static_cast<int>(t) % nc], 1) >= limit;
-      }
-      flag = __syncthreads_or(over);
-    }
-    if (blockIdx.x == 0 && tid == 0) plan[b] = flag;
-    const size_t base = static_cast<size_t>(b) * per_batch;
-    const size_t stride = static_cast<size_t>(gridDim.x) * kPrepThreads, i0 = static_cast<size_t>(blockIdx.x) * kPrepThreads + tid;
-    // (per_batch is a multiple of 8 elements and both buffers are 16-byte aligned: tensor-core path only)
-    if (flag && zero_output) {
-      float4* a4 = reinterpret_cast<float4*>(acc + base);
-      for (size_t i = i0; i < per_batch / 4; i += stride) a4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    } else if (flag) {                   // seed the float32 rows with what the output holds
-      for (size_t i = i0; i < per_batch; i += stride) acc[base + i] = to_f32<T>(out[base + i]);
-    } else if (zero_output) {
-      uint4* o16 = reinterpret_cast<uint4*>(out + base);
-      for (size_t i = i0; i < per_batch / 8; i += stride) o16[i] = make_uint4(0, 0, 0, 0);
-    }
-    __syncthreads();                     // the counters of this batch element have been used
+  int flag = 0;
+  if (info) {
+    flag = info[0] > limit;
+    if (info[2] && blockIdx.x == 0 && tid == 0) status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
+  } else if (nflags > 0) {
+    pdl_wait();
+    for (int i = tid; i < nflags; i += kPrepThreads) flag |= flags[i];
+    flag = __syncthreads_or(flag);
+  } else if (EK > limit) {
+    flag = has_hot_row(ind, index_dtype, 0, B, T_, EK, limit, prep_cnt);
+  }
+  if (blockIdx.x == 0 && tid == 0) *plan = flag;
+  const size_t stride = static_cast<size_t>(gridDim.x) * kPrepThreads, i0 = static_cast<size_t>(blockIdx.x) * kPrepThreads + tid;
+  // (n is a multiple of 8 elements and both buffers are 16-byte aligned: tensor-core path only)
+  if (flag && zero_output) {
+    float4* a4 = reinterpret_cast<float4*>(acc);
+    for (size_t i = i0; i < n / 4; i += stride) a4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  } else if (flag) {                     // seed the float32 rows with what the output holds
+    for (size_t i = i0; i < n; i += stride) acc[i] = to_f32<T>(out[i]);
+  } else if (zero_output) {
+    uint4* o16 = reinterpret_cast<uint4*>(out);
+    for (size_t i = i0; i < n / 8; i += stride) o16[i] = make_uint4(0, 0, 0, 0);
   }
 }
 
@@ -490,15 +509,11 @@ __device__ __forceinline__ void convert8(const float* __restrict__ src, T* __res
 
 template <typename T>
 __global__ void __launch_bounds__(256) scatter_finish_kernel(const int* __restrict__ plan, const float* __restrict__ acc,
-                                                            T* __restrict__ out, int B, size_t per_batch) {
+                                                            T* __restrict__ out, size_t n) {
   pdl_wait();
+  if (!*plan) return;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-  for (int b = blockIdx.y; b < B; b += gridDim.y) {
-    if (!plan[b]) continue;
-    const size_t base = static_cast<size_t>(b) * per_batch;
-    for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < per_batch / 8; i += stride)
-      convert8<T>(acc + base + 8 * i, out + base + 8 * i);
-  }
+  for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n / 8; i += stride) convert8<T>(acc + 8 * i, out + 8 * i);
 }
 
 int grid_for(size_t work_items, int per_block) {
@@ -652,49 +667,56 @@ cudaError_t launch_convert_from_f32(const float* src, void* dst, size_t n, int d
 }
 
 template <typename T>
-static cudaError_t prepare(const void* Ind, int index_dtype, int B, int T_, int EK, const int* info, int limit, int* plan, float* acc,
-                           void* out16, size_t per_batch, int zero_output, StatusRef status, cudaStream_t st) {
-  // CTAs per batch element: four per SM in all, each with at least 4 KB to zero and no more ids to count than half the elements
-  // it zeroes
+static cudaError_t prepare(const void* Ind, int index_dtype, int B, int T_, int EK, const int* info, int limit, int* flags, int* plan,
+                           float* acc, void* out16, size_t n, int zero_output, StatusRef status, cudaStream_t st) {
   const bool count = info == nullptr && EK > limit;
-  size_t per = (4 * 148 + B - 1) / B;
-  const size_t by_bytes = per_batch * sizeof(T) / 4096, by_count = count ? per_batch / (2 * static_cast<size_t>(EK)) : per;
-  if (per > by_bytes) per = by_bytes;
-  if (per > by_count) per = by_count;
-  if (per < 1) per = 1;
-  const size_t smem = count ? static_cast<size_t>(T_ < kPrepCounters ? T_ : kPrepCounters) * sizeof(int) : 0;
-  if (smem > 48 * 1024) {
-    cudaError_t err = ensure_smem_optin<scatter_prepare_kernel<T>>(kPrepCounters * static_cast<int>(sizeof(int)));
+  const long long ids = static_cast<long long>(B) * EK, rows = static_cast<long long>(B) * T_;
+  const bool own_count = count && (B == 1 || (ids <= kPrepOwnIds && rows <= kPrepCounters));
+  const long long counters = own_count ? rows : T_;
+  const size_t smem = count ? static_cast<size_t>(counters < kPrepCounters ? counters : kPrepCounters) * sizeof(int) : 0;
+  cudaError_t err = cudaSuccess;
+  int nflags = 0;
+  if (count && !own_count) {
+    nflags = B < kPrepCountCtas ? B : kPrepCountCtas;
+    if (smem > 48 * 1024) err = ensure_smem_optin<scatter_count_kernel>(kPrepCounters * static_cast<int>(sizeof(int)));
+    if (err != cudaSuccess) return err;
+    scatter_count_kernel<<<nflags, kPrepThreads, smem, st>>>(Ind, index_dtype, B, T_, EK, limit, flags);
+    count_launch();
+    err = cudaGetLastError();
     if (err != cudaSuccess) return err;
   }
-  scatter_prepare_kernel<T><<<dim3(static_cast<unsigned>(per), B < 65535 ? B : 65535), kPrepThreads, smem, st>>>(
-      Ind, index_dtype, B, T_, EK, info, limit, plan, acc, static_cast<T*>(out16), per_batch, zero_output, status);
+  // four CTAs per SM, each with at least 4 KB to zero and, where it counts, no more ids than half the elements it zeroes
+  size_t grid = 4 * 148;
+  const size_t by_bytes = n * sizeof(T) / 4096, by_count = own_count ? n / (2 * static_cast<size_t>(ids)) : grid;
+  if (grid > by_bytes) grid = by_bytes;
+  if (grid > by_count) grid = by_count;
+  if (grid < 1) grid = 1;
+  if (own_count && smem > 48 * 1024) err = ensure_smem_optin<scatter_prepare_kernel<T>>(kPrepCounters * static_cast<int>(sizeof(int)));
+  if (err != cudaSuccess) return err;
+  err = launch_kernel(scatter_prepare_kernel<T>, static_cast<unsigned>(grid), kPrepThreads, own_count ? smem : 0, st, nflags > 0, Ind, index_dtype,
+                      B, T_, EK, info, flags, nflags, limit, plan, acc, static_cast<T*>(out16), n, zero_output, status);
   count_launch();
-  return cudaGetLastError();
+  return err;
 }
 
-cudaError_t launch_scatter_prepare(const void* Ind, int index_dtype, int B, int T, int E, int K, const int* csr_info, int limit, int* plan,
-                                   float* acc, void* out16, int N, int zero_output, int dtype, StatusRef status, cudaStream_t st) {
-  const size_t per_batch = static_cast<size_t>(T) * N;
-  if (B == 0 || per_batch == 0) return cudaSuccess;
+cudaError_t launch_scatter_prepare(const void* Ind, int index_dtype, int B, int T, int E, int K, const int* csr_info, int limit, int* flags,
+                                   int* plan, float* acc, void* out16, int N, int zero_output, int dtype, StatusRef status, cudaStream_t st) {
+  const size_t n = static_cast<size_t>(B) * T * N;
+  if (n == 0) return cudaSuccess;
   const int ek = E * K;      // B*E*K fits in 32 bits
-  if (dtype == EGS_F16) return prepare<__half>(Ind, index_dtype, B, T, ek, csr_info, limit, plan, acc, out16, per_batch, zero_output, status, st);
+  if (dtype == EGS_F16) return prepare<__half>(Ind, index_dtype, B, T, ek, csr_info, limit, flags, plan, acc, out16, n, zero_output, status, st);
   if (dtype == EGS_BF16)
-    return prepare<__nv_bfloat16>(Ind, index_dtype, B, T, ek, csr_info, limit, plan, acc, out16, per_batch, zero_output, status, st);
+    return prepare<__nv_bfloat16>(Ind, index_dtype, B, T, ek, csr_info, limit, flags, plan, acc, out16, n, zero_output, status, st);
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_scatter_finish(const int* plan, const float* acc, void* out16, int B, size_t per_batch, int dtype, cudaStream_t st) {
-  if (B == 0 || per_batch == 0) return cudaSuccess;
-  size_t per = per_batch / (256 * 8 * 4);                // four vectors per thread, a few waves of CTAs at most
-  const size_t most = (148 * 8 + B - 1) / B;
-  if (per > most) per = most;
-  if (per < 1) per = 1;
-  const dim3 grid(static_cast<unsigned>(per), B < 65535 ? B : 65535);
+cudaError_t launch_scatter_finish(const int* plan, const float* acc, void* out16, size_t n, int dtype, cudaStream_t st) {
+  if (n == 0) return cudaSuccess;
+  const int grid = grid_for(n, 256 * 8 * 4);             // four vectors per thread, a few waves of CTAs at most
   cudaError_t err;
-  if (dtype == EGS_F16) err = launch_kernel(scatter_finish_kernel<__half>, grid, 256, 0, st, true, plan, acc, static_cast<__half*>(out16), B, per_batch);
+  if (dtype == EGS_F16) err = launch_kernel(scatter_finish_kernel<__half>, grid, 256, 0, st, true, plan, acc, static_cast<__half*>(out16), n);
   else if (dtype == EGS_BF16)
-    err = launch_kernel(scatter_finish_kernel<__nv_bfloat16>, grid, 256, 0, st, true, plan, acc, static_cast<__nv_bfloat16*>(out16), B, per_batch);
+    err = launch_kernel(scatter_finish_kernel<__nv_bfloat16>, grid, 256, 0, st, true, plan, acc, static_cast<__nv_bfloat16*>(out16), n);
   else return cudaErrorInvalidValue;
   count_launch();
   return err;

@@ -20,7 +20,7 @@
 //   warps 8..11   converters: acc1 -> Y (tensor memory + global store)
 //   warps 12..19  scatter epilogue, two groups of four warps (one per TMEM lane group) taking pairs of S tiles in turn:
 //                 acc2 -> 16 bits -> staged in shared memory -> one bulk reduction per row and tile pair into the output
-//                 rows; or (heavy collisions, decided by the planning flags) float32 red.global.add into the rows of the scratch
+//                 rows; or (heavy collisions, decided by the planning flag) float32 red.global.add into the rows of the scratch
 //   warp  20      TMEM allocation; one lane issues the tcgen05.mma of the G stages
 //   warp  21      one lane issues the tcgen05.mma of the S tiles
 // Tensor memory (512 columns): Y [0,128), acc1 [128,384), acc2[0] [384,448), acc2[1] [448,512).
@@ -310,17 +310,13 @@ __global__ void __launch_bounds__(kP16Threads, 1) tensor_pair16_persistent_kerne
     const uint32_t srow = my_area + static_cast<uint32_t>(lane) * kP16RowPitch;
     T* out16 = static_cast<T*>(p.Out16);
     bool alive = true;
-    pdl_wait();                                          // the planning flags and the zeros the rows are added to
+    pdl_wait();                                          // the planning flag and the zeros the rows are added to
+    const bool direct16 = *p.plan == 0;
     uint32_t seen = 0;                                   // bit b: parity of the tiles this group has taken from acc2[b]
     for (int rb = blockIdx.x; rb < row_blocks && alive; rb += gridDim.x) {
       const P16Block blk = p16_block(p, rb, m_tiles);
       int tok, slot;
-      const int my_m = blk.m0 + q * 32 + lane;
-      p16_rows(p, blk.e, my_m, tok, slot, false);
-      // rows of this warp whose batch element sums in float32 rows (bits)
-      const uint32_t to_f32 = __ballot_sync(0xffffffffu, my_m < p.M && p.plan[my_m / p.K] != 0);
-      const bool direct16 = to_f32 == 0u;
-      if (!direct16) bulk_wait_all();                    // the transposes below reuse the staging buffer
+      p16_rows(p, blk.e, blk.m0 + q * 32 + lane, tok, slot, false);
       for (int nt = 0; nt < n2 && alive; ++nt) {
         if (((nt >> 1) & 1) != grp) continue;
         const int buf = nt & 1;                          // tile nt of every row block goes through acc2[nt & 1]
@@ -373,11 +369,7 @@ __global__ void __launch_bounds__(kP16Threads, 1) tensor_pair16_persistent_kerne
                             [&](int row, int cj, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3) {
                               const int ro = __shfl_sync(0xffffffffu, tok, row);
                               const int col = col0 + cj;
-                              if (ro >= 0 && col < p.N2) {
-                                const long long off = static_cast<long long>(ro) * p.N2 + col;
-                                if ((to_f32 >> row) & 1u) red4(p.Dst + off, x0, x1, x2, x3);
-                                else red4(out16 + off, x0, x1, x2, x3);
-                              }
+                              if (ro >= 0 && col < p.N2) red4(p.Dst + static_cast<long long>(ro) * p.N2 + col, x0, x1, x2, x3);
                             });
           }
           tc_fence_before();
@@ -386,7 +378,7 @@ __global__ void __launch_bounds__(kP16Threads, 1) tensor_pair16_persistent_kerne
         }
       }
     }
-    bulk_wait_all();                                     // shared memory must outlive the copy engine's reads
+    if (direct16) bulk_wait_all();                       // shared memory must outlive the copy engine's reads
   } else if (warp == kP16WarpG) {
     // =========================== MMA issuer of the G stages ===========================
     if (lane == 0) {

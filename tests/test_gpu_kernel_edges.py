@@ -192,8 +192,7 @@ def test_dense16_pairs_repeat_their_bits(cuda_device, B, T, E, K, I, J):
     ops.check_status()
 
 
-# 16-bit scatter: the choice between direct additions and float32 rows is made per batch element; tiles of 128 expert rows here
-# span batch elements of both kinds (K = 48), the persistent kernel (N = 1032) and the one-tile kernel (long contraction)
+# 16-bit scatter with hot token rows in some batch elements only; tiles of 128 expert rows here span elements with and without (K = 48)
 @pytest.mark.parametrize("C,N", [(40, 72), (256, 1032), (520, 64)])
 @pytest.mark.parametrize("pair", [False, True])
 def test_scatter16_mixes_both_kinds_of_batch_elements(cuda_device, C, N, pair):
@@ -222,3 +221,24 @@ def test_scatter16_mixes_both_kinds_of_batch_elements(cuda_device, C, N, pair):
     for b in (2, 5):
         exact = torch.from_numpy(ref[b]).to(torch.bfloat16).double().numpy()
         assert np.abs(Out[b].cpu().double().numpy() - exact).max() <= 2.0 ** -8 * np.abs(ref[b]).max()
+
+
+# ... and one hot token row anywhere makes every row of the call a float32 sum that is rounded once: bf16 has eight significant bits,
+# so half a unit in the last place is at most 2^-8 of the value (the float32 sums themselves are good to 1e-5 of the largest)
+@pytest.mark.parametrize("B", [1, 2, 30, 700])        # counted by the zeroing kernel itself (1, 2), by a CTA an element, by fewer CTAs
+@pytest.mark.parametrize("pair", [False, True])
+def test_scatter16_one_hot_row_rounds_all_rows_once(cuda_device, B, pair):
+    T, E, K, C, N = 40, 12, 24, 32, 64
+    g = torch.Generator().manual_seed(B)
+    Ind = (torch.arange(B * E * K).view(B, E, K) * 7) % T          # 7 or 8 per row
+    Ind[B - 1, :, :4] = 3                                          # 40 more on one row of the last batch element
+    Y, W = torch.randn(B, E, K, C, generator=g).bfloat16(), torch.randn(E, C, N, generator=g).bfloat16()
+    d_ind = Ind.to(cuda_device)
+    if pair:
+        X, W1 = torch.randn(B, T, 32, generator=g).bfloat16(), torch.randn(E, 32, C, generator=g).bfloat16()
+        Mid, Out = ops.gather_scatter_pair(X.to(cuda_device), W1.to(cuda_device), W.to(cuda_device), d_ind)
+        Y = Mid.cpu()
+    else:
+        Out = ops.gemm_scatter(Y.to(cuda_device), W.to(cuda_device), d_ind, T)
+    ref = orc.np_scatter(Y, W, Ind, T)
+    assert (np.abs(Out.cpu().double().numpy() - ref) <= 2.0 ** -8 * np.abs(ref) + 1e-5 * np.abs(ref).max()).all()
