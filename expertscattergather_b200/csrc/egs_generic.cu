@@ -526,12 +526,13 @@ int grid_for(size_t work_items, int per_block) {
 
 }  // namespace
 
-// Tile width over n features in units of 32, at most `most`: the least padding, the widest of equals.
+// Tile width over n features in units of 32, at most `most`: the least padding, the widest of equals.  The widest of all where a
+// narrower tile's columns would not fit in a grid's y (65535 blocks).
 static int width_in_32s(int n, int most) {
-  int best = 1, best_pad = 1 << 30;
+  int best = most, best_pad = 1 << 30;
   for (int w = 1; w <= most; ++w) {
-    const int tile = 32 * w, pad = (n + tile - 1) / tile * tile - n;
-    if (pad <= best_pad) {
+    const int tile = 32 * w, tiles = (n + tile - 1) / tile, pad = tiles * tile - n;
+    if (pad <= best_pad && tiles <= 65535) {
       best = w;
       best_pad = pad;
     }

@@ -61,6 +61,16 @@ def test_generic_kernels_edges(cuda_device, B, T, E, K, I, J, dtype):
             assert torch.equal(got[k], torch.from_numpy(ref[k]).to(dtype)), k
 
 
+# generic kernels at widths whose narrowest tiles would exceed a grid's y
+@pytest.mark.parametrize("N", [32 * 65535, 32 * 65536 + 32])
+def test_generic_kernels_take_wide_outputs(cuda_device, N):
+    x, W, Ind = torch.tensor([[[3.0], [2.0]]]), torch.arange(N).view(1, 1, N).float() % 7, torch.ones(1, 1, 1, dtype=torch.int64)
+    x, W, Ind = x.to(cuda_device), W.to(cuda_device), Ind.to(cuda_device)
+    assert torch.equal(ops.gather_gemm(x, W, Ind, path="generic"), 2 * W.view(1, 1, 1, N))
+    assert torch.equal(ops.gemm_scatter(x[:, :1].view(1, 1, 1, 1), W, Ind, 2, path="generic")[0], torch.cat([0 * W[0], 3 * W[0]]))
+    assert torch.equal(ops.dweight(x, W.view(1, 1, 1, N), Ind, path="generic"), 2 * W)
+
+
 @pytest.mark.parametrize("B,T,E,K,N", [(1, 5, 1, 1, 1), (3, 40, 4, 50, 24), (16, 64, 2, 100, 72), (70, 33, 3, 30, 33)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
 @pytest.mark.parametrize("gathered", [False, True])
