@@ -308,14 +308,14 @@ constexpr int kSumThreads = 256;
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(kSumThreads) expert_row_sum_kernel(const T* __restrict__ Src, const void* __restrict__ Ind,
                                                                      int index_dtype, T* __restrict__ out, int T_, int E, int K, int N,
-                                                                     int M, StatusRef status) {
+                                                                     int M, int nranks, StatusRef status) {
   constexpr int PER = VEC ? 16 / static_cast<int>(sizeof(T)) : 1;   // columns per lane
   constexpr int COLS = 8 * PER;                                     // columns per CTA
   constexpr int ROWS = kSumThreads / 8;                             // rows a CTA reads at a time
   __shared__ float part[ROWS][COLS + 1];
   __shared__ float total[COLS];
-  const int rank = blockIdx.x, nranks = gridDim.x;                  // the cluster spans gridDim.x
-  const int e = blockIdx.z, c0 = blockIdx.y * COLS;
+  const int rank = blockIdx.x % nranks;                             // a cluster is `nranks` CTAs along x
+  const int e = blockIdx.y, c0 = blockIdx.x / nranks * COLS;
   const int tid = threadIdx.x, cl = tid & 7, rl = tid >> 3;
   const int col = c0 + cl * PER;
   const int per = (M + nranks - 1) / nranks, m_end = min(M, (rank + 1) * per);
@@ -613,7 +613,7 @@ static cudaError_t launch_row_sum(const void* Src, const void* Ind, int index_dt
   int ranks = 1;
   while (ranks < 8 && static_cast<long long>(blocks) * E * ranks < 8 * 148 && M >= 128 * 2 * ranks) ranks *= 2;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(ranks, blocks, E);
+  cfg.gridDim = dim3(ranks * blocks, E);
   cfg.blockDim = dim3(kSumThreads);
   cfg.stream = st;
   cudaLaunchAttribute attr{};
@@ -624,7 +624,7 @@ static cudaError_t launch_row_sum(const void* Src, const void* Ind, int index_dt
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, expert_row_sum_kernel<T, VEC>, static_cast<const T*>(Src), Ind, index_dtype, static_cast<T*>(out), T_, E, K,
-                            N, M, status);
+                            N, M, ranks, status);
 }
 
 cudaError_t launch_expert_row_sum(const void* Src, const void* Ind, int index_dtype, void* out, int B, int T, int E, int K, int N,

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 import torch
 
+import expertscattergather_b200 as egs
 from expertscattergather_b200 import _lib, ops, workloads
 from expertscattergather_b200.workloads import Workload
 from gpu_util import STEP_KEYS, gpu_step
@@ -85,6 +86,13 @@ def test_expert_row_sum(cuda_device, B, T, E, K, N, dtype, gathered):
     assert rc == _lib.OK
     rows = torch.gather(src.double(), 1, Ind.reshape(B, -1, 1).expand(-1, -1, N)).reshape(B, E, K, N) if gathered else src.double()
     assert torch.equal(out.cpu(), rows.sum((0, 2)).to(dtype))       # integers: exact in float32, rounded once
+
+
+def test_expert_row_sum_takes_wide_rows(cuda_device):
+    N = 8 * 65536 + 9                                              # more blocks of columns than a grid's y holds
+    m = egs.ExpertGather(1, 1, N, bias=True).to(cuda_device)
+    m(torch.ones(1, 2, 1, device=cuda_device), torch.zeros(1, 1, 3, dtype=torch.int64, device=cuda_device)).sum().backward()
+    assert torch.equal(m.bias.grad, torch.full_like(m.bias, 3.0))
 
 
 # strict float32 kernels: tile widths 32 / 64 / 96 / 128 with partial last tiles, contractions around one step (32), one chunk
