@@ -88,6 +88,24 @@ def test_expert_row_sum(cuda_device, B, T, E, K, N, dtype, gathered):
     assert torch.equal(out.cpu(), rows.sum((0, 2)).to(dtype))       # integers: exact in float32, rounded once
 
 
+# long sums: no worse than 64-bit truth rounded a few times (2^-24 each), with rows read 16 bytes a lane (N = 8) and one column a lane
+@pytest.mark.parametrize("N", [8, 5])
+def test_expert_row_sum_of_many_rows(cuda_device, N):
+    B, E, K = 512, 1, 4096
+    m = egs.ExpertGather(E, 1, N, bias=True).to(cuda_device)
+    dY = torch.randn(B, E, K, N, generator=torch.Generator(device=cuda_device).manual_seed(2), device=cuda_device)
+    Y = m(torch.zeros(B, 1, 1, device=cuda_device), torch.zeros(B, E, K, dtype=torch.int64, device=cuda_device))
+    Y.backward(dY)
+    ref = dY.double().sum((0, 2)).view(-1)
+    # eight-row trees lose 2^-24 of partial sums of a few units, 2^18 of them at random: 2^-24 * 3 * 2^9; the sums themselves are ~2^10.5
+    assert ((m.bias.grad.double().view(-1) - ref).abs().max() <= 2.0 ** -24 * (3 * 2 ** 9 + 4 * ref.abs().max())).item()
+    dY[0, 0, 7, 1], dY[3, 0, 9, 2], dY[4, 0, 2, 2] = float("inf"), float("inf"), float("-inf")
+    m.bias.grad = None
+    m(torch.zeros(B, 1, 1, device=cuda_device), torch.zeros(B, E, K, dtype=torch.int64, device=cuda_device)).backward(dY)
+    got = m.bias.grad.view(-1)
+    assert got[1] == float("inf") and got[2].isnan() and got[0].isfinite()
+
+
 def test_expert_row_sum_takes_wide_rows(cuda_device):
     N = 8 * 65536 + 9                                              # more blocks of columns than a grid's y holds
     m = egs.ExpertGather(1, 1, N, bias=True).to(cuda_device)
