@@ -76,8 +76,8 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 constexpr long long kInt32Max = 2147483647LL;
 // 16-bit scatter adds directly into the output while no token row receives more contributions than this.
 constexpr int kDirect16Limit = 32;
-// Longest contraction strict float32 runs on the tensor cores under EGS_PATH_AUTO (see run_rowgemm), and longest that one
-// accumulator of the fused pair kernel sees.
+// Longest contraction strict float32 runs on the tensor cores under EGS_PATH_AUTO (measured against float64 up to there, see
+// egs_strict.cu), and longest that one accumulator of the fused pair kernel sees.
 constexpr long long kStrictMaxContraction = 2048;
 constexpr long long kStrictMaxFusedContraction = 512;
 
@@ -147,8 +147,8 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
   const bool eligible = device_is_sm100() && rowgemm_tensor_ok(d, dtype, A, W, Out);
   if ((path == EGS_PATH_TENSOR || path == EGS_PATH_PAIRED) && !eligible) return EGS_ERR_UNSUPPORTED;
   // Strict float32 on long contractions: the tensor core's accumulator additions truncate, and the error grows with the
-  // contraction length (3.3e-5 of max|ref| at C = 4096 against the 1e-5 bar).  The strict kernels sum chunks of 512 elements with
-  // correct rounding; EGS_PATH_AUTO takes them up to kStrictMaxContraction and the FFMA kernels beyond.
+  // contraction length (3.3e-5 of max|ref| at C = 4096 against the 1e-5 bar).  Beyond 512 elements the strict kernels therefore sum
+  // step by step with correct rounding; EGS_PATH_AUTO takes them up to kStrictMaxContraction and the FFMA kernels beyond.
   const bool strict_long = (dtype == EGS_F32 && precision == EGS_PREC_STRICT && d.C > kStrictMaxContraction);
   const bool tensor = ((path == EGS_PATH_TENSOR || path == EGS_PATH_PAIRED) || (path == EGS_PATH_AUTO && eligible && !strict_long)) && !(d.C == 0) &&
                       (bias == nullptr || aligned16(bias));

@@ -10,15 +10,16 @@
 // therefore pay (at BN = 64 the same bytes serve half the products), and the rest is keeping those clocks busy:
 //   * two rings.  Raw tiles are prefetched `raw - lo` steps ahead (each thread splits exactly the chunks it has copied itself, so
 //     its own copy group is all it waits for); lo tiles need two buffers, the one the tensor core reads and the one being
-//     written.  One ring of hi+lo stages, as before, left room for two stages and therefore no prefetch at all: a step cost
-//     1.9 us, most of it load latency.
+//     written.  (One ring of hi+lo stages has room for two stages and therefore no prefetch: 1.9 us a step, most of it load latency.)
 //   * persistent CTAs, the rings run on across tiles, the accumulator is double-buffered in tensor memory, and dedicated warps
 //     read it out while the next tile is multiplied.
 // The tensor core adds product groups into its accumulator with truncation, an error that grows with the number of steps
-// (3.3e-5 of max|ref| at a contraction of 4096).  An accumulator therefore sees at most 512 elements of a G / S contraction;
-// the chunks of a longer one are summed, with correct rounding, by the read-out warps in spare tensor-memory columns.  D keeps
-// its ranges of at most 1024 rows.
-// 32768 routed rows, I = 1024, J = 256: S 266 us, D 236 us, G (with FFMA kernels) 978 us before.
+// (3.3e-5 of max|ref| at a contraction of 4096).  G and S up to a contraction of 512 and D, in ranges of at most 1024 rows, stay
+// below 1.2e-5.  A longer contraction of G and S (LONG) takes an accumulator per step, the small products first, and sums the steps in
+// registers of the read-out warps with correct rounding: 2.0e-7 to 2.6e-7 against float64 (2-norm, normal and positive values,
+// 516 to 2048 elements), where FFMA sums have 3.5e-7 to 8.1e-7 and accumulators of 16, 4 and 2 steps 1.1e-5, 2.1e-6 and 8.2e-7.
+// (Operands below 2^-110 lose their lo parts to the smallest exponent: 2e-5.)  The registers come from the producers (setmaxnreg).
+// 32768 routed rows, I = 1024, J = 256: S 138 us, D 171, G 154 (FFMA 474).
 #include "egs_tcgen05.cuh"
 
 namespace egs {
@@ -28,14 +29,18 @@ namespace {
 // Sixteen producer warps: a step costs a producer thread about 120 instructions for its (up to) four chunks, and with eight warps
 // (two per scheduler) their latencies, not the shared-memory clocks, set the pace: 1.4 us per step instead of 1.1.
 constexpr int kProdWarps = 16, kProdThreads = kProdWarps * 32;
-constexpr int kEpiWarps = 4;
-constexpr int kMmaWarp = kProdWarps + kEpiWarps;
-constexpr int kStrictThreads = (kMmaWarp + 1) * 32;
+// Read-out warps; twice as many, each with half of the columns, where they also add up a long contraction.
+__host__ __device__ constexpr int epi_warps(bool long_c) { return long_c ? 8 : 4; }
+// (long contractions: the register split is by warpgroups, see kLongProdRegs)
+__host__ __device__ constexpr int strict_threads(bool long_c) { return (kProdWarps + epi_warps(long_c) + (long_c ? 4 : 1)) * 32; }
 constexpr int kLoStages = 2;
 constexpr uint32_t kStrictHeader = 1024;
-constexpr uint32_t kXposeBytes = kEpiWarps * 4096;
+__host__ __device__ constexpr uint32_t xpose_bytes(bool long_c) { return epi_warps(long_c) * 4096u; }
 constexpr int kStepElems = 32;                     // contraction elements per step: one 128-byte segment of float32
-constexpr int kChunkSteps = 16;                    // G / S: steps one accumulator sees
+constexpr int kWholeSteps = 16;                    // G / S: steps of a contraction that one accumulator sees whole (512 elements)
+// Longer ones: registers a thread of the producers, the read-out and the MMA warp's group; 28 warps of 72 at launch.
+constexpr int kLongProdRegs = 48, kLongEpiRegs = 144, kLongMmaRegs = 24;
+static_assert(kProdWarps * kLongProdRegs + epi_warps(true) * kLongEpiRegs + 4 * kLongMmaRegs <= 28 * 72, "more registers than the block has");
 constexpr uint32_t kATile = kTileM * 128u;         // bytes of a raw A tile; D: 32 rows of 128 features, the same
 constexpr size_t kSmemMax = 227 * 1024;
 constexpr int kSms = 148;
@@ -45,8 +50,8 @@ enum { kOpGather = 0, kOpScatter = 1, kOpDweight = 2 };
 struct __align__(16) StrictHeader {
   unsigned long long full[kMaxStages];
   unsigned long long empty[kMaxStages];
-  unsigned long long acc_full[2];
-  unsigned long long acc_empty[2];
+  unsigned long long acc_full[4];
+  unsigned long long acc_empty[4];
   unsigned long long drain;
   uint32_t tmem_base;
   uint32_t abort_flag;
@@ -122,19 +127,27 @@ __device__ __forceinline__ uint32_t swz32(int c, int r) {
   return (static_cast<uint32_t>(((c & 7) >> 1) ^ (r & 3)) << 5) + (static_cast<uint32_t>(c & 1) << 4);
 }
 
-template <int OP>
-__global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(StrictParams p) {
+__device__ __forceinline__ void add2(uint32_t& a0, uint32_t& a1, uint32_t b0, uint32_t b1) {
+  asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\tadd.rn.f32x2 a, a, b;\n\tmov.b64 {%0, %1}, a;\n\t}"
+      : "+r"(a0), "+r"(a1)
+      : "r"(b0), "r"(b1));
+}
+
+template <int OP, bool LONG>
+__global__ void __launch_bounds__(strict_threads(LONG), 1) strict_kernel(StrictParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   StrictHeader* hdr = reinterpret_cast<StrictHeader*>(smem_raw);
   const uint32_t smem0 = smem_u32(smem_raw);
   const uint32_t xpose0 = smem0 + kStrictHeader;
-  const uint32_t raw0 = xpose0 + kXposeBytes;
+  constexpr int kEpiWarps = epi_warps(LONG), kMmaWarp = kProdWarps + kEpiWarps;
+  constexpr int kAccs = LONG ? 4 : 2;                 // accumulators in tensor memory
+  const uint32_t raw0 = xpose0 + xpose_bytes(LONG);
   const uint32_t stage_bytes = kATile + static_cast<uint32_t>(p.BN) * 128u;      // A then B, the same in the lo ring
   const uint32_t lo0 = raw0 + static_cast<uint32_t>(p.raw) * stage_bytes;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int raw = p.raw;
   const uint32_t acc_cols = tmem_cols_for(p.BN);
-  const uint32_t tmem_cols = 4u * acc_cols;           // two accumulators and the running sums of long contractions
+  const uint32_t tmem_cols = kAccs * acc_cols;
   volatile uint32_t* abort_flag = &hdr->abort_flag;
 
   if (tid == 0) {
@@ -142,7 +155,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(StrictParams 
       mbar_init(smem_u32(&hdr->full[s]), kProdWarps);
       mbar_init(smem_u32(&hdr->empty[s]), 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < kAccs; ++b) {
       mbar_init(smem_u32(&hdr->acc_full[b]), 1);
       mbar_init(smem_u32(&hdr->acc_empty[b]), kEpiWarps);
     }
@@ -168,6 +181,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(StrictParams 
     // fall through to the common exit
   } else if (warp < kProdWarps) {
     // =========================== producers ===========================
+    if (LONG) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kLongProdRegs));
     const char* A = static_cast<const char*>(p.A);
     const char* Bs = static_cast<const char*>(p.Bsrc);
     const long long pitch_c = static_cast<long long>(p.C) * 4, pitch_n = static_cast<long long>(p.N) * 4;
@@ -336,18 +350,18 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(StrictParams 
     cp_async_wait_all();
   } else if (warp < kMmaWarp) {
     // =========================== read-out ===========================
+    if (LONG) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kLongEpiRegs));
+    constexpr int kShares = kEpiWarps / 4, kBlocks = 4 / kShares;      // (the widest tile has four blocks of 32 columns)
     const int ew = warp - kProdWarps;
-    const int lg = ew & 3;                               // TMEM lane group
+    const int lg = ew & 3, share = ew >> 2;              // TMEM lane group, share of the blocks
     const uint32_t tile = xpose0 + static_cast<uint32_t>(ew) * 4096u;
     const uint32_t lane_base = static_cast<uint32_t>(lg * 32) << 16;
-    const uint32_t sums = tmem_base + lane_base + 2u * acc_cols;
     bool alive = true;
     pdl_wait();                                          // the zeros the results are added to
-    int t = 0;                                           // accumulators taken so far
+    int buf = 0, around = 0;                             // next accumulator, times through all of them
     for (int un = blockIdx.x; un < p.units && alive; un += gridDim.x) {
       const Unit u = unit_of<OP>(p, un);
       const int steps = unit_steps<OP>(p, u);
-      const int chunks = OP == kOpDweight ? 1 : (steps + kChunkSteps - 1) / kChunkSteps;
       int my_ro = -1;                                    // G, S: destination row of tile row lg * 32 + lane
       if (OP != kOpDweight) {
         const int m = u.m0 + lg * 32 + lane;
@@ -362,41 +376,21 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(StrictParams 
       }
       const int bn = min(p.BN, p.N - u.n0);
       const int nblk = (bn + 31) >> 5;
-      for (int ch = 0; ch < chunks && alive; ++ch, ++t) {
-        const int buf = t & 1;
-        alive = mbar_wait_all(smem_u32(&hdr->acc_full[buf]), (t >> 1) & 1, abort_flag, p.status.word);
-        if (!alive) break;
-        tc_fence_after();
-        const uint32_t acc = tmem_base + lane_base + static_cast<uint32_t>(buf) * acc_cols;
-        const bool last = ch == chunks - 1;
-        for (int c = 0; c < nblk; ++c) {
-          uint32_t v[32];
-          tmem_ld32(acc + static_cast<uint32_t>(c * 32), v);
-          tmem_ld_wait();
-          if (ch > 0) {                                  // add the chunks before this one
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              uint32_t s[16];
-              tmem_ld16(sums + static_cast<uint32_t>(c * 32 + h * 16), s);
-              tmem_ld_wait();
-#pragma unroll
-              for (int i = 0; i < 16; ++i) v[h * 16 + i] = __float_as_uint(__uint_as_float(v[h * 16 + i]) + __uint_as_float(s[i]));
-            }
-          }
-          if (!last) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              uint32_t s[16];
-#pragma unroll
-              for (int i = 0; i < 16; ++i) s[i] = v[h * 16 + i];
-              tmem_st16(sums + static_cast<uint32_t>(c * 32 + h * 16), s);
-            }
-            tmem_st_wait();
-            continue;
-          }
+      auto wait_full = [&]() {
+        alive = mbar_wait_all(smem_u32(&hdr->acc_full[buf]), around & 1, abort_flag, p.status.word);
+        if (alive) tc_fence_after();
+        return tmem_base + lane_base + static_cast<uint32_t>(buf) * acc_cols;
+      };
+      auto release = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&hdr->acc_empty[buf]));
+        if (++buf == kAccs) { buf = 0; ++around; }
+      };
+      auto emit = [&](int c, const uint32_t (&w)[32]) {
           const int col0 = u.n0 + c * 32;
           if (OP != kOpDweight) {
-            warp_regs_emit(v, tile, lane, [&](int row, int cj, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3) {
+            warp_regs_emit(w, tile, lane, [&](int row, int cj, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3) {
               const int ro = __shfl_sync(0xffffffffu, my_ro, row);
               const int col = col0 + cj;
               if (ro >= 0 && col < p.N) {
@@ -407,7 +401,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(StrictParams 
               }
             });
           } else if (p.out_layout == EGS_DW_GATHERED_ROWS) {     // out[e, f, g]: rows f are contiguous over g
-            warp_regs_emit(v, tile, lane, [&](int row, int cj, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3) {
+            warp_regs_emit(w, tile, lane, [&](int row, int cj, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3) {
               const int f = u.m0 + lg * 32 + row, g = col0 + cj;
               if (f < p.C && g < p.N) {
                 float* out = p.Out + (static_cast<long long>(u.e) * p.C + f) * p.N + g;
@@ -422,20 +416,94 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(StrictParams 
               for (int i = 0; i < 32; ++i) {
                 if (col0 + i < p.N) {
                   float* out = p.Out + (static_cast<long long>(u.e) * p.N + col0 + i) * p.C + f;
-                  if (p.splits > 1) atomicAdd(out, __uint_as_float(v[i]));
-                  else *out = __uint_as_float(v[i]);
+                  if (p.splits > 1) atomicAdd(out, __uint_as_float(w[i]));
+                  else *out = __uint_as_float(w[i]);
                 }
               }
             }
           }
+      };
+      // An infinite operand times a zero lo part is NaN where the float32 product is infinite: sums that came out as NaN are formed
+      // again, one product after the other as the generic kernel does.
+      auto again_if_nan = [&](int c, uint32_t (&w)[32]) {
+        bool nan = false;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) nan |= isnan(__uint_as_float(w[i]));
+        if (!__any_sync(0xffffffffu, nan)) return;
+        const int m = u.m0 + lg * 32 + lane, b = m / p.K, slot = (b * p.E + u.e) * p.K + (m - b * p.K);
+        int row = m < p.M ? slot : -1;
+        if (OP == kOpGather && row >= 0) {
+          const long long tk = load_index(p.Ind, p.index_dtype, slot);
+          row = tk >= 0 && tk < p.T ? b * p.T + static_cast<int>(tk) : -1;
         }
-        tc_fence_before();
+        const float* a = static_cast<const float*>(p.A) + static_cast<long long>(row) * p.C;
+        const float* wt = static_cast<const float*>(p.Bsrc) + static_cast<long long>(u.e) * p.C * p.N;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + i * 128u + lane * 4u), "r"(w[i]) : "memory");
+#pragma unroll 1
+        for (int i = 0; i < 32; ++i) {
+          float x;
+          const int n = u.n0 + c * 32 + i;
+          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(tile + i * 128u + lane * 4u) : "memory");
+          if (m < p.M && n < p.N && isnan(x)) {
+            x = 0.f;
+#pragma unroll 1
+            for (int k = 0; k < p.C; ++k)
+              x = fmaf(row >= 0 ? a[k] : 0.f, wt[p.nc ? static_cast<long long>(n) * p.C + k : static_cast<long long>(k) * p.N + n], x);
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(tile + i * 128u + lane * 4u), "f"(x) : "memory");
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 32; ++i) asm volatile("ld.shared.b32 %0, [%1];" : "=r"(w[i]) : "r"(tile + i * 128u + lane * 4u) : "memory");
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&hdr->acc_empty[buf]));
+      };
+      if (LONG) {
+        uint32_t v[kBlocks][32];                         // the sums of this thread's row
+        for (int ch = 0; ch < steps; ++ch) {
+          const uint32_t acc = wait_full();
+          if (!alive) break;
+#pragma unroll
+          for (int c = 0; c < kBlocks; ++c) {
+            if (c * kShares + share < nblk) {
+              uint32_t x[32];
+              tmem_ld32(acc + static_cast<uint32_t>((c * kShares + share) * 32), x);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 32; i += 2) {
+                if (ch == 0) {
+                  v[c][i] = x[i];
+                  v[c][i + 1] = x[i + 1];
+                } else {
+                  add2(v[c][i], v[c][i + 1], x[i], x[i + 1]);
+                }
+              }
+            }
+          }
+          release();
+        }
+        if (!alive) break;
+#pragma unroll
+        for (int c = 0; c < kBlocks; ++c) {
+          if (c * kShares + share < nblk) {
+            again_if_nan(c * kShares + share, v[c]);
+            emit(c * kShares + share, v[c]);
+          }
+        }
+      } else {
+        const uint32_t acc = wait_full();
+        if (!alive) break;
+        for (int c = 0; c < nblk; ++c) {
+          uint32_t v[32];
+          tmem_ld32(acc + static_cast<uint32_t>(c * 32), v);
+          tmem_ld_wait();
+          emit(c, v);
+        }
+        release();
       }
     }
   } else {
     // =========================== MMA issuer ===========================
+    if (LONG) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kLongMmaRegs));
     // (the warp runs converged and an elected lane issues, see mbar_wait_all: twelve MMAs from a lane on its own took 1000 clocks)
     // A: K-major rows (G, S) or rows = contraction (D); B: rows = n (weights [n][contraction]) or rows = contraction
     const bool a_mn = OP == kOpDweight, b_mn = OP == kOpDweight || !p.nc;
@@ -444,8 +512,8 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(StrictParams 
     const uint32_t a_adv = (a_mn ? 8u * 128u : 32u) >> 4, b_adv = (b_mn ? 8u * 128u : 32u) >> 4;
     const uint64_t a_desc = make_smem_desc(0u, a_lbo, a_sbo, a_lay), b_desc = make_smem_desc(0u, b_lbo, b_sbo, b_lay) + (kATile >> 4);
     bool ok = true;
-    int t = 0, slot = 0, round = 0, lo = 0;
-    for (int un = blockIdx.x; un < p.units && ok; un += gridDim.x) {
+    int buf = 0, around = 0, slot = 0, round = 0, lo = 0;
+    for (int un = blockIdx.x; un < p.units && ok && warp == kMmaWarp; un += gridDim.x) {
       const Unit u = unit_of<OP>(p, un);
       const int steps = unit_steps<OP>(p, u);
       const int bn = min(p.BN, ((p.N - u.n0) + 15) & ~15);
@@ -453,11 +521,9 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(StrictParams 
       // contraction elements of the unit (rows for D)
       const int len = OP == kOpDweight ? min(p.rows_per_split, p.M - u.split * p.rows_per_split) : p.C;
       for (int ks = 0; ks < steps && ok; ++ks) {
-        const bool first = OP == kOpDweight ? ks == 0 : ks % kChunkSteps == 0;
-        const bool last = ks == steps - 1 || (OP != kOpDweight && ks % kChunkSteps == kChunkSteps - 1);
-        const int buf = t & 1;
-        if (first && t >= 2) {
-          ok = mbar_wait_all(smem_u32(&hdr->acc_empty[buf]), ((t >> 1) - 1) & 1, abort_flag, p.status.word);
+        const bool first = LONG || ks == 0, last = LONG || ks == steps - 1;
+        if (first && around > 0) {
+          ok = mbar_wait_all(smem_u32(&hdr->acc_empty[buf]), (around - 1) & 1, abort_flag, p.status.word);
           if (!ok) break;
         }
         ok = mbar_wait_all(smem_u32(&hdr->full[slot]), round & 1, abort_flag, p.status.word);
@@ -468,20 +534,24 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(StrictParams 
         const uint32_t hi16 = (raw0 + static_cast<uint32_t>(slot) * stage_bytes) >> 4, lo16 = (lo0 + static_cast<uint32_t>(lo) * stage_bytes) >> 4;
         const int nkq = min(4, (len - ks * kStepElems + 7) / 8);
         if (elect_one()) {
+          auto hi_hi = [&](int kq) { umma<true>(d, a_desc + (hi16 + kq * a_adv), b_desc + (hi16 + kq * b_adv), idesc, 1u); };
 #pragma unroll
           for (int kq = 0; kq < 4; ++kq) {
             if (kq < nkq) {
-              const uint64_t ad = a_desc + (hi16 + kq * a_adv), adl = a_desc + (lo16 + kq * a_adv);
-              const uint64_t bd = b_desc + (hi16 + kq * b_adv), bdl = b_desc + (lo16 + kq * b_adv);
-              umma<true>(d, adl, bd, idesc, (first && kq == 0) ? 0u : 1u);
-              umma<true>(d, ad, bdl, idesc, 1u);
-              umma<true>(d, ad, bd, idesc, 1u);
+              umma<true>(d, a_desc + (lo16 + kq * a_adv), b_desc + (hi16 + kq * b_adv), idesc, (first && kq == 0) ? 0u : 1u);
+              umma<true>(d, a_desc + (hi16 + kq * a_adv), b_desc + (lo16 + kq * b_adv), idesc, 1u);
+              if (!LONG) hi_hi(kq);
             }
+          }
+          if (LONG) {                                    // the small products first: additions truncate, and to a small sum that is little
+#pragma unroll
+            for (int kq = 0; kq < 4; ++kq)
+              if (kq < nkq) hi_hi(kq);
           }
           umma_commit(smem_u32(&hdr->empty[slot]));
           if (last) umma_commit(smem_u32(&hdr->acc_full[buf]));
         }
-        if (last) ++t;
+        if (last && ++buf == kAccs) { buf = 0; ++around; }
         lo ^= 1;
         if (++slot == raw) { slot = 0; ++round; }
       }
@@ -507,19 +577,27 @@ int strict_bn(int n) {
   }
   return best;
 }
-int strict_raw_stages(int bn) {
+bool long_contraction(int c) { return c > kWholeSteps * kStepElems; }
+int strict_raw_stages(int bn, bool long_c) {
   const size_t stage = kATile + static_cast<size_t>(bn) * 128;
-  size_t raw = (kSmemMax - kStrictHeader - kXposeBytes) / stage - kLoStages;
+  size_t raw = (kSmemMax - kStrictHeader - xpose_bytes(long_c)) / stage - kLoStages;
   return static_cast<int>(raw > kMaxStages ? kMaxStages : raw);
 }
 
-template <int OP>
+template <int OP, bool LONG = false>
 cudaError_t launch(const StrictParams& p, bool after_own, cudaStream_t st) {
   const size_t stage = kATile + static_cast<size_t>(p.BN) * 128;
-  const size_t smem = kStrictHeader + kXposeBytes + (p.raw + kLoStages) * stage;
-  cudaError_t err = ensure_smem_optin<strict_kernel<OP>>(static_cast<int>(kSmemMax));
+  const size_t smem = kStrictHeader + xpose_bytes(LONG) + (p.raw + kLoStages) * stage;
+  cudaError_t err = ensure_smem_optin<strict_kernel<OP, LONG>>(static_cast<int>(kSmemMax));
   if (err != cudaSuccess) return err;
-  err = launch_kernel(strict_kernel<OP>, p.units < kSms ? p.units : kSms, kStrictThreads, smem, st, after_own, p);
+  if (LONG) {                                            // setmaxnreg can only share out what the block is launched with
+    static const int regs = [] {
+      cudaFuncAttributes a{};
+      return cudaFuncGetAttributes(&a, strict_kernel<OP, LONG>) == cudaSuccess ? a.numRegs : 0;
+    }();
+    if (regs * strict_threads(true) < (kProdWarps * kLongProdRegs + epi_warps(true) * kLongEpiRegs + 4 * kLongMmaRegs) * 32) return cudaErrorInvalidConfiguration;
+  }
+  err = launch_kernel(strict_kernel<OP, LONG>, p.units < kSms ? p.units : kSms, strict_threads(LONG), smem, st, after_own, p);
   count_launch();
   return err;
 }
@@ -528,7 +606,7 @@ cudaError_t launch(const StrictParams& p, bool after_own, cudaStream_t st) {
 
 void configure_strict_rowgemm(RowGemmParams& p) {
   p.BN = strict_bn(p.N);
-  p.stages = strict_raw_stages(p.BN);
+  p.stages = strict_raw_stages(p.BN, long_contraction(p.C));
   p.row_tiles = 1;
   p.persistent = 1;
   p.bulk_epilogue = 0;
@@ -546,12 +624,14 @@ cudaError_t launch_strict_rowgemm(const RowGemmParams& r, bool scatter, cudaStre
   const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.E;
   if (units > 2147483647ll) return cudaErrorInvalidValue;
   p.units = static_cast<int>(units);
+  if (long_contraction(r.C))
+    return scatter ? launch<kOpScatter, true>(p, r.after_own != 0, st) : launch<kOpGather, true>(p, r.after_own != 0, st);
   return scatter ? launch<kOpScatter>(p, r.after_own != 0, st) : launch<kOpGather>(p, r.after_own != 0, st);
 }
 
 void configure_strict_dweight(DWeightParams& p) {
   p.BN = strict_bn(p.FD);
-  p.stages = strict_raw_stages(p.BN);
+  p.stages = strict_raw_stages(p.BN, false);
   p.row_tiles = 1;
   // row ranges: as many as still leave one unit per SM, at most 1024 rows each (see the top of the file)
   const long long tiles = static_cast<long long>((p.FG + kTileM - 1) / kTileM) * ((p.FD + p.BN - 1) / p.BN) * p.E;

@@ -148,6 +148,52 @@ def test_strict_float32_edges(cuda_device, B, T, E, K, I, J):
         assert orc.rel_err(got[k], truth[k]) <= 1e-5, k
 
 
+# contractions beyond 512 on the tensor cores: no further from float64 than the float32 sums of the generic kernels
+@pytest.mark.parametrize("C", [516, 1024, 2048])
+@pytest.mark.parametrize("positive", [False, True])
+@pytest.mark.parametrize("op", ["G", "S"])
+def test_strict_float32_long_contractions_are_as_good_as_ffma(cuda_device, C, positive, op):
+    B, T, E, K, N = 3, 400, 2, 100, 136
+    g = torch.Generator(device=cuda_device).manual_seed(C)
+    normal = lambda *s: torch.randn(s, generator=g, device=cuda_device).abs_() if positive else torch.randn(s, generator=g, device=cuda_device)
+    W, Ind = normal(E, C, N), torch.randperm(T, generator=g, device=cuda_device)[: E * K].view(1, E, K).expand(B, E, K).contiguous()
+    A = normal(B, T, C) if op == "G" else normal(B, E, K, C)
+    rows = torch.gather(A, 1, Ind.reshape(B, -1, 1).expand(-1, -1, C)).view(B, E, K, C) if op == "G" else A
+    ref = torch.einsum("bekc,ecn->bekn", rows.double(), W.double())
+
+    def err(path):
+        if op == "G":
+            got = ops.gather_gemm(A, W, Ind, path=path)
+        else:                                     # distinct tokens: one contribution a row
+            got = torch.gather(ops.gemm_scatter(A, W, Ind, T, path=path), 1, Ind.reshape(B, -1, 1).expand(-1, -1, N)).view(B, E, K, N)
+        return ((got.double() - ref).norm() / ref.norm()).item()
+
+    assert ops.describe_plan(op, B, T, E, K, C, N, torch.float32)["tensor_path"] == 1
+    assert err("auto") <= err("generic")
+
+
+# ... and the same infinities and NaNs
+@pytest.mark.parametrize("w_layout", ["cn", "nc"])
+def test_strict_float32_long_contractions_keep_infinities(cuda_device, w_layout):
+    B, T, E, K, C, N = 2, 60, 3, 50, 520, 140
+    g = torch.Generator().manual_seed(6)
+    X, W = torch.randint(-3, 4, (B, T, C), generator=g).float(), torch.randint(1, 4, (E, C, N), generator=g).float()
+    Y = torch.randint(-3, 4, (B, E, K, C), generator=g).float()
+    Ind = torch.randint(0, T, (B, E, K), generator=g)
+    Ind[0, 1, 3] = T                              # out of range: a row of zeros
+    for A in (X.view(-1, C), Y.view(-1, C)):
+        A[3, 7], A[9, 519], A[9, 2], A[17, 300] = float("inf"), float("inf"), float("-inf"), float("nan")
+    W[2, 33, 5], W[1, 0, 139], W[0, 4, 64] = float("-inf"), float("nan"), 0.0
+    Wd = (W if w_layout == "cn" else W.transpose(1, 2)).contiguous().to(cuda_device)
+    Xd, Yd, Id = X.to(cuda_device), Y.to(cuda_device), Ind.to(cuda_device)
+    for f in (lambda path: ops.gather_gemm(Xd, Wd, Id, w_layout=w_layout, path=path),
+              lambda path: ops.gemm_scatter(Yd, Wd, Id, T, w_layout=w_layout, path=path)):
+        got, want = f("tensor"), f("generic")
+        assert got.isinf().any() and got.isnan().any() and torch.equal(got.nan_to_num(nan=12345.0), want.nan_to_num(nan=12345.0))
+        assert torch.equal(got.isnan(), want.isnan())
+    ops.reset_status()
+
+
 # 16-bit kernels: one CTA or a pair per tile (the last two shapes are large enough for pairs), slot rows as boxes (K = 1, 16, 64, 128)
 # or gathered (K = 43, 101), one row or one column block in the last tile, row ranges of D that are split and that are not
 @pytest.mark.parametrize("B,T,E,K,I,J", [(1, 8, 1, 1, 8, 8), (3, 60, 2, 43, 72, 40), (5, 90, 3, 64, 264, 136), (33, 70, 5, 16, 520, 264),
