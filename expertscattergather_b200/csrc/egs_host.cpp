@@ -12,6 +12,7 @@
 //   * nothing synchronises with the device;
 //   * one status word per device (see egs_b200.h) with a mapped host mirror that kernels write when they report invalid
 //     results: every operator call looks at the mirror first and raises.
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include <ATen/cuda/EmptyTensor.h>
@@ -253,6 +254,8 @@ int index_type(at::ScalarType t) {
   }
 }
 Tensor empty(at::IntArrayRef sizes, at::ScalarType dtype, int idx) {
+  if (torch::jit::tracer::isTracing())     // a trace has to know its outputs
+    return at::empty(sizes, at::TensorOptions().dtype(dtype).device(at::kCUDA, static_cast<c10::DeviceIndex>(idx)));
   return at::detail::empty_cuda(sizes, dtype, c10::Device(c10::kCUDA, static_cast<c10::DeviceIndex>(idx)), std::nullopt);
 }
 // device scratch of `bytes` (undefined tensor for none)
@@ -638,15 +641,16 @@ bool plain(const Tensor& t) {
 }
 template <class... Ts>
 bool native_ok(const Ts&... ts) {
-  return !c10::impl::dispatch_mode_enabled() && (plain(ts) && ...);
+  return !c10::impl::dispatch_mode_enabled() && !torch::jit::tracer::isTracing() && (plain(ts) && ...);
 }
+bool native_ok_bias(const OptTensor& bias) { return !bias || plain(*bias); }
 
 OptTensor gather_autograd(const Tensor& X, const Tensor& W, const OptTensor& bias, const Tensor& Ind) {
-  if (!native_ok(X, W, Ind)) return std::nullopt;
+  if (!native_ok(X, W, Ind) || !native_ok_bias(bias)) return std::nullopt;
   return bias ? GatherBiasFunction::apply(X, W, *bias, Ind) : GatherFunction::apply(X, W, Ind);
 }
 OptTensor scatter_autograd(const Tensor& Y, const Tensor& W, const OptTensor& bias, const Tensor& Ind, int64_t T) {
-  if (!native_ok(Y, W, Ind)) return std::nullopt;
+  if (!native_ok(Y, W, Ind) || !native_ok_bias(bias)) return std::nullopt;
   return bias ? ScatterBiasFunction::apply(Y, W, *bias, Ind, T) : ScatterFunction::apply(Y, W, Ind, T);
 }
 OptTensor gather_scatter_autograd(const Tensor& X, const Tensor& Wg, const Tensor& Ws, const Tensor& Ind) {

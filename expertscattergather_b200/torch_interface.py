@@ -21,8 +21,13 @@ from .kernels import (ExpertGatherBiasFunction, ExpertGatherFunction, ExpertGath
 __all__ = ["ExpertGather", "ExpertScatter", "ExpertGatherScatter"]
 
 # Eager calls go to the native autograd functions of csrc/egs_host.cpp.  They return None for tensors they do not take (fake
-# tensors, tensor subclasses, functorch wrappers); those, and traced calls, run the Python functions of kernels.py.
-_tracing = torch.compiler.is_compiling
+# tensors, tensor subclasses, functorch wrappers) and under torch.jit.trace, which records the dispatcher ops; those, and calls
+# that are compiled or traced symbolically, run the Python functions of kernels.py.
+_Tensor, _compiling = torch.Tensor, torch.compiler.is_compiling
+
+
+def _eager(a, b) -> bool:
+    return isinstance(a, _Tensor) and isinstance(b, _Tensor) and not _compiling()
 
 
 class ExpertGather(nn.Module):
@@ -49,7 +54,7 @@ class ExpertGather(nn.Module):
             nn.init.uniform_(self.bias, -bound, bound)
 
     def forward(self, x: torch.Tensor, Ind: torch.Tensor) -> torch.Tensor:
-        if not _tracing():
+        if _eager(x, Ind):
             y = ops._host().gather_autograd(x, self.W, self.bias, Ind)
             if y is not None:
                 return y
@@ -93,7 +98,7 @@ class ExpertScatter(nn.Module):
             nn.init.uniform_(self.bias, -bound, bound)
 
     def forward(self, Y: torch.Tensor, Ind: torch.Tensor, T: int) -> torch.Tensor:
-        if not _tracing():
+        if _eager(Y, Ind):
             per_slot = self.bias if self.bias_mode == "per_slot" else None
             out = ops._host().scatter_autograd(Y, self.W, per_slot, Ind, int(T))
             if out is not None:
@@ -125,7 +130,7 @@ class ExpertGatherScatter(nn.Module):
     def forward(self, x: torch.Tensor, Ind: torch.Tensor) -> torch.Tensor:
         if self.gather.bias is not None or self.scatter.bias is not None:
             return self.scatter(self.gather(x, Ind), Ind, x.shape[1])
-        if not _tracing():
+        if _eager(x, Ind):
             out = ops._host().gather_scatter_autograd(x, self.gather.W, self.scatter.W, Ind)
             if out is not None:
                 return out

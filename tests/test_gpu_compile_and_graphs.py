@@ -49,6 +49,27 @@ def test_modules_compile_with_fullgraph(cuda_device, dtype):
     assert abs(float(loss.detach()) - ref_loss) <= tol * max(1.0, float((ref["Out"].double() * ins["G"].double()).abs().sum()))
 
 
+@pytest.mark.parametrize("bias", [False, True])
+@pytest.mark.parametrize("block", [False, True])
+def test_jit_traces_run_on_new_inputs(cuda_device, bias, block):
+    if block:
+        m = egs.ExpertGatherScatter(4, 64, 32, bias=bias).to(cuda_device)
+    else:
+        class Pair(torch.nn.Module):
+            def __init__(self):
+                super().__init__()
+                self.g, self.s = egs.ExpertGather(4, 64, 32, bias=bias), egs.ExpertScatter(4, 32, 64, bias=bias)
+
+            def forward(self, x, ind):
+                return self.s(self.g(x, ind), ind, 40)
+        m = Pair().to(cuda_device)
+    g = torch.Generator(device=cuda_device).manual_seed(1)
+    new = lambda: (torch.randn(2, 40, 64, generator=g, device=cuda_device), torch.randint(0, 40, (2, 4, 8), generator=g, device=cuda_device))
+    traced = torch.jit.trace(m, new(), check_trace=False)
+    x, ind = new()
+    assert orc.rel_err(traced(x, ind).detach().cpu(), m(x, ind).detach().cpu()) <= 1e-5
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_modules_forward_and_backward_in_a_cuda_graph(cuda_device, dtype):
     """Forward + backward of the modules captured once and replayed on new input values: the helper streams the backward

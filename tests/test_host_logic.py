@@ -59,6 +59,28 @@ def test_cpu_tensors_are_refused():
         ops.gather_gemm(torch.randn(3, 4), torch.randn(2, 4, 4), torch.zeros(1, 2, 2, dtype=torch.int64))
 
 
+def test_traced_calls_do_not_take_the_native_functions():
+    """torch.jit.trace and torch.fx record what runs: both must see the dispatcher ops, or a trace would hold this call's results."""
+    g, s = egs.ExpertGather(2, 4, 4, bias=True), egs.ExpertScatter(2, 4, 4)
+    x, ind = torch.randn(1, 3, 4), torch.zeros(1, 2, 2, dtype=torch.int64)
+    taken = []
+
+    def f(x):
+        taken.append(ops._host().gather_autograd(x, g.W, None, ind))
+        taken.append(ops._host().scatter_autograd(x.view(1, 1, 3, 4), s.W, None, ind, 3))
+        taken.append(ops._host().gather_scatter_autograd(x, g.W, s.W, ind))
+        return x + 0
+
+    torch.jit.trace(f, (x,), check_trace=False)
+    assert taken == [None, None, None]
+    gather = egs.ExpertGather(2, 4, 4)
+    targets = [str(n.target) for n in torch.fx.symbolic_trace(gather).graph.nodes]
+    assert any("expert_gather_forward_call_fn" in t for t in targets), targets
+    with torch._subclasses.FakeTensorMode():
+        fake = torch.empty(2, 1, 4)
+    assert ops._host().gather_autograd(x, g.W, fake, ind) is None
+
+
 def test_install_as_egs_aliases():
     saved = {k: sys.modules.pop(k) for k in list(sys.modules) if k == "egs" or k.startswith("egs.")}
     try:
