@@ -9,7 +9,7 @@
 //   * buffers (outputs, workspaces, gradients) come from torch's caching allocator on the CURRENT stream; work that runs on
 //     the helper stream is forked from it and joined to it before the call returns, so stream order on the current stream
 //     covers every buffer;
-//   * nothing synchronises with the device;
+//   * nothing synchronises with the device (the first call on a device waits for a 4-byte fill on a stream of its own);
 //   * one status word per device (see egs_b200.h) with a mapped host mirror that kernels write when they report invalid
 //     results: every operator call looks at the mirror first and raises.
 #include <torch/csrc/jit/frontend/tracer.h>
@@ -17,6 +17,7 @@
 
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
@@ -98,12 +99,23 @@ DeviceState& device_state(int idx) {
   std::lock_guard<std::mutex> lock(g_devices_mutex);
   if (DeviceState* s = g_devices[idx].load(std::memory_order_acquire)) return *s;
   c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(idx));
-  auto* s = new DeviceState;                    // lives as long as the process, like the device's context
-  s->word = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, idx));
-  void* host = nullptr;
-  const cudaError_t err = cudaHostAlloc(&host, sizeof(int32_t), cudaHostAllocMapped | cudaHostAllocPortable);
-  if (err != cudaSuccess) throw std::runtime_error(std::string("cudaHostAlloc: ") + cudaGetErrorString(err));
+  // The first call on a device may come while this or another thread captures a graph: the allocations are allowed then, and the
+  // word is neither the graph's memory nor zeroed by a node of it.
+  c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+  auto ok = [](cudaError_t e, const char* what) {
+    if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
+  };
+  void *host = nullptr, *word = nullptr;
+  cudaStream_t once = nullptr;
+  ok(cudaHostAlloc(&host, sizeof(int32_t), cudaHostAllocMapped | cudaHostAllocPortable), "cudaHostAlloc");
+  ok(cudaMalloc(&word, sizeof(int32_t)), "cudaMalloc");
+  ok(cudaStreamCreateWithFlags(&once, cudaStreamNonBlocking), "cudaStreamCreate");
+  ok(cudaMemsetAsync(word, 0, sizeof(int32_t), once), "cudaMemsetAsync");
+  ok(cudaStreamSynchronize(once), "cudaStreamSynchronize");
+  cudaStreamDestroy(once);
   *static_cast<volatile int32_t*>(host) = 0;
+  auto* s = new DeviceState;                    // lives as long as the process, like the device's context
+  s->word = at::from_blob(word, {1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, idx));
   s->mirror = static_cast<volatile int32_t*>(host);
   check(api.egs_set_status_mirror(s->word.data_ptr<int32_t>(), static_cast<int32_t*>(host)), "egs_set_status_mirror");
   s->side = c10::cuda::getStreamFromPool(/*isHighPriority=*/false, static_cast<c10::DeviceIndex>(idx));

@@ -1,6 +1,9 @@
 """The modules under torch.compile (the dispatcher ops carry fake implementations so that a compiled graph can trace through
 them, as the reference's do, egs/triton_kernels.py:527-567) and under CUDA-graph capture (forward + backward, helper
 streams included), both against the CPU oracle."""
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -47,6 +50,26 @@ def test_modules_compile_with_fullgraph(cuda_device, dtype):
     assert orc.rel_err(s.W.grad.cpu(), ref["dWs"]) <= tol
     ref_loss = float((ref["Out"].double() * ins["G"].double()).sum())
     assert abs(float(loss.detach()) - ref_loss) <= tol * max(1.0, float((ref["Out"].double() * ins["G"].double()).abs().sum()))
+
+
+def test_the_first_call_of_a_process_may_be_captured(cuda_device):
+    code = """
+import torch
+from expertscattergather_b200 import ops
+X, W = torch.ones(2, 8, 32, device="cuda"), torch.ones(2, 32, 16, device="cuda")
+Ind = torch.zeros(2, 2, 4, dtype=torch.int64, device="cuda")
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    Y = ops.gather_gemm(X, W, Ind)
+for _ in range(2):
+    X.add_(1.0)
+    graph.replay()
+    assert (Y == 32 * X[0, 0, 0]).all().item()
+ops.check_status()
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
 
 
 @pytest.mark.parametrize("bias", [False, True])
