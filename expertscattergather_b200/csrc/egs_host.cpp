@@ -191,7 +191,7 @@ struct Call {
 // Runs independent work of one call on the device's helper stream: forks at construction, joins when it goes out of scope.
 class SideStream {
  public:
-  explicit SideStream(const Call& c) : main_(c.stream), side_(c.st->side->stream()) {
+  explicit SideStream(const Call& c) : idx_(static_cast<c10::DeviceIndex>(c.idx)), main_(c.stream), side_(c.st->side->stream()) {
     events_ = &events_for(c.idx);
     sync_from_main();
   }
@@ -200,12 +200,14 @@ class SideStream {
   cudaStream_t stream() const { return side_; }
   // later work on the side stream starts after what the main stream holds now
   void sync_from_main() {
+    c10::cuda::CUDAGuard guard(idx_);                  // (the default stream's handle means the current device's)
     ok(cudaEventRecord(events_->fork, main_));
     ok(cudaStreamWaitEvent(side_, events_->fork, 0));
   }
   void join() {
     if (joined_) return;
     joined_ = true;
+    c10::cuda::CUDAGuard guard(idx_);
     if (cudaEventRecord(events_->join, side_) == cudaSuccess) cudaStreamWaitEvent(main_, events_->join, 0);
   }
 
@@ -229,6 +231,7 @@ class SideStream {
     }
     return e;
   }
+  c10::DeviceIndex idx_;
   cudaStream_t main_, side_;
   Events* events_;
   bool joined_ = false;

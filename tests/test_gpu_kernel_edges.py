@@ -194,6 +194,17 @@ def test_strict_float32_long_contractions_keep_infinities(cuda_device, w_layout)
     ops.reset_status()
 
 
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs a device that is not the current one")
+def test_train_step_on_another_device_than_the_current():
+    w = Workload("other", 4, 64, 4, 16, 64, 32, torch.float32, "distinct", 9)
+    ins = workloads.make_inputs(w, integer_valued=True)
+    ref = orc.np_step(ins["X"], ins["Wg"], ins["Ws"], ins["Ind"], ins["G"])
+    with torch.cuda.device(0):
+        got = gpu_step(ins, torch.device("cuda", 1))
+    for k in STEP_KEYS:
+        assert np.array_equal(got[k].double().numpy(), ref[k]), k
+
+
 # 16-bit kernels: one CTA or a pair per tile (the last two shapes are large enough for pairs), slot rows as boxes (K = 1, 16, 64, 128)
 # or gathered (K = 43, 101), one row or one column block in the last tile, row ranges of D that are split and that are not
 @pytest.mark.parametrize("B,T,E,K,I,J", [(1, 8, 1, 1, 8, 8), (3, 60, 2, 43, 72, 40), (5, 90, 3, 64, 264, 136), (33, 70, 5, 16, 520, 264),
