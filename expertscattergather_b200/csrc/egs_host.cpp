@@ -494,6 +494,7 @@ Tensor expert_row_sum(const Tensor& Src, const OptTensor& Ind, int64_t B, int64_
 // (At 2^27 the FFMA kernels of odd float32 sizes take 30 us and want the overlap: 117 against 131 us a pass at 132M.)
 constexpr double kSmallWork = 1 << 25;
 bool worth_a_side_stream(const Tensor& slot_rows, const Tensor& W) {      // [B,E,K,J] and a weight tensor of E * I * J elements
+  if (g_debug.load(std::memory_order_relaxed)) return false;             // every operator is checked behind its own kernels
   const double slots = static_cast<double>(slot_rows.size(0)) * slot_rows.size(2);
   return slots * W.numel() > kSmallWork;
 }
@@ -690,7 +691,7 @@ Step train_step(const Tensor& X_, const Tensor& Wg, const Tensor& Ws, const Tens
   const int64_t T = X.size(1);
   const auto none = std::nullopt;
   Tensor Y, Out, dY, dX, dWg, dWs;
-  if (!overlap) {
+  if (!overlap || g_debug.load(std::memory_order_relaxed)) {
     Y = gather_gemm(X, Wg, Ind, EGS_W_CN, -1, -1, none);
     Out = gemm_scatter(Y, Ws, Ind, T, EGS_W_CN, none, -1, -1, none, none);
     dY = gather_gemm(G, Ws, Ind, EGS_W_NC, -1, -1, none);
