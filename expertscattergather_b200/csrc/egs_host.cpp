@@ -15,6 +15,7 @@
 #include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
+#include <ATen/core/dispatch/Dispatcher.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
@@ -542,6 +543,17 @@ Grads scatter_backward(const Tensor& Y_, const Tensor& W, const Tensor& Ind_, co
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
+// Under create_graph a backward pass runs as the dispatcher op, as it does behind the Python functions, so that torch's fallback for
+// ops without a derivative of their own (a warning, zero second derivatives) is what a caller meets either way.
+std::string g_namespace;               // of the dispatcher ops
+variable_list through_dispatcher(const char* op, const Tensor& A, const Tensor& W, const Tensor& Ind, const Tensor& grad) {
+  using Fn = std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, const Tensor&, const Tensor&, at::ScalarType);
+  const std::string name = g_namespace + "::" + op;
+  auto r = c10::Dispatcher::singleton().findSchemaOrThrow(name.c_str(), "").typed<Fn>().call(A, W, Ind, grad, at::kFloat);
+  return {std::get<0>(r), std::get<1>(r)};
+}
+bool wants_graph(const Tensor& A, const Tensor& W) { return at::GradMode::is_enabled() && A.requires_grad() && W.requires_grad(); }
+
 struct GatherFunction : torch::autograd::Function<GatherFunction> {
   static Tensor forward(AutogradContext* ctx, const Tensor& X, const Tensor& W, const Tensor& Ind) {
     Tensor Y = gather_gemm(X, W, Ind, EGS_W_CN, -1, -1, std::nullopt);
@@ -550,6 +562,10 @@ struct GatherFunction : torch::autograd::Function<GatherFunction> {
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& g) {
     const auto s = ctx->get_saved_variables();
+    if (wants_graph(s[0], s[1])) {
+      variable_list d = through_dispatcher("expert_gather_backward_call_fn", s[0], s[1], s[2], g[0]);
+      return {d[0], d[1], Tensor()};
+    }
     Grads r = gather_backward(s[0], s[1], s[2], g[0], ctx->needs_input_grad(0), ctx->needs_input_grad(1), false);
     return {r.in, r.w, Tensor()};
   }
@@ -563,6 +579,10 @@ struct ScatterFunction : torch::autograd::Function<ScatterFunction> {
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& g) {
     const auto s = ctx->get_saved_variables();
+    if (wants_graph(s[0], s[1])) {
+      variable_list d = through_dispatcher("expert_scatter_backward_call_fn", s[0], s[1], s[2], g[0]);
+      return {d[0], d[1], Tensor(), Tensor()};
+    }
     Grads r = scatter_backward(s[0], s[1], s[2], g[0], ctx->needs_input_grad(0), ctx->needs_input_grad(1), false);
     return {r.in, r.w, Tensor(), Tensor()};
   }
@@ -725,6 +745,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   using nogil = py::call_guard<py::gil_scoped_release>;
   m.def("init", &init);
   m.def("configure", &configure);
+  m.def("set_namespace", [](const std::string& ns) { g_namespace = ns; });
   m.def("status_word", [](int idx) { return device_state(idx).word; });
   m.def("reset_status", &reset_status);
   m.def("check_status", &check_status, nogil());

@@ -38,7 +38,11 @@ def _push_state() -> None:
 def _host():
     global _native
     if _native is None:
-        _native = _lib.host()
+        host = _lib.host()
+        from . import kernels
+        kernels.create_kernels()
+        host.set_namespace(kernels.OP_NAMESPACE)
+        _native = host
         _push_state()
     return _native
 

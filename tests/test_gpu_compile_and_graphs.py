@@ -52,6 +52,17 @@ def test_modules_compile_with_fullgraph(cuda_device, dtype):
     assert abs(float(loss.detach()) - ref_loss) <= tol * max(1.0, float((ref["Out"].double() * ins["G"].double()).abs().sum()))
 
 
+@pytest.mark.filterwarnings("ignore:.*an autograd kernel was not registered")
+def test_backward_with_create_graph_returns_a_graph(cuda_device):
+    """The dispatcher ops have no second derivative of their own: torch warns and goes on, for the modules as for the Functions."""
+    g, s = egs.ExpertGather(4, 64, 32).to(cuda_device), egs.ExpertScatter(4, 32, 64).to(cuda_device)
+    x = torch.randn(2, 40, 64, device=cuda_device, requires_grad=True)
+    ind = torch.randint(0, 40, (2, 4, 8), device=cuda_device)
+    gx, = torch.autograd.grad(s(g(x, ind), ind, 40).pow(2).sum(), x, create_graph=True)
+    assert gx.requires_grad
+    gx.pow(2).sum().backward()
+
+
 def test_the_first_call_of_a_process_may_be_captured(cuda_device):
     code = """
 import torch
