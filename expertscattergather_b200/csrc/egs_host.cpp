@@ -618,53 +618,64 @@ struct ScatterBiasFunction : torch::autograd::Function<ScatterBiasFunction> {
   }
 };
 
+// The block: Y, Out and whether the fused kernel ran.
+std::tuple<Tensor, Tensor, bool> gather_scatter_forward(const Tensor& X, const Tensor& Wg, const Tensor& Ws, const Tensor& Ind) {
+  const bool fused = fused_pair_preferred(X, Wg, Ind);
+  Tensor Y, out;
+  if (fused) {
+    std::tie(Y, out) = gather_scatter_pair(X, Wg, Ws, Ind, EGS_W_CN, std::nullopt, -1);
+  } else {
+    Y = gather_gemm(X, Wg, Ind, EGS_W_CN, -1, -1, std::nullopt);
+    out = gemm_scatter(Y, Ws, Ind, X.size(1), EGS_W_CN, std::nullopt, -1, -1, std::nullopt, std::nullopt);
+  }
+  return {Y, out, fused};
+}
+
+// dX, dWg, dWs; those not needed stay undefined
+std::array<Tensor, 3> gather_scatter_backward(const Tensor& X_, const Tensor& Wg, const Tensor& Ws, const Tensor& Ind_, const Tensor& Y,
+                                              const Tensor& dOut_, bool fused, bool need_x, bool need_wg, bool need_ws) {
+  const Tensor X = X_.contiguous(), dOut = dOut_.contiguous(), Ind = index_tensor(Ind_).t;
+  Tensor dX, dWg, dWs, dY, ws;
+  std::optional<SideStream> side;
+  const bool fork = worth_a_side_stream(Y, Wg);
+  std::optional<cudaStream_t> on;
+  if (need_ws) {                                     // needs only dOut and Y
+    if (fork) {
+      side.emplace(Call(X, dOut));
+      on = side->stream();
+    }
+    dWs = dweight_on(dOut, Y, Ind, EGS_DW_DIRECT_ROWS, -1, -1, std::nullopt, on, &ws);
+  }
+  if (need_x && fused)
+    std::tie(dY, dX) = gather_scatter_pair(dOut, Ws, Wg, Ind, EGS_W_NC, std::nullopt, -1);
+  else if (need_x || need_wg)
+    dY = gather_gemm(dOut, Ws, Ind, EGS_W_NC, -1, -1, std::nullopt);
+  if (need_wg) {
+    if (side) {
+      side->sync_from_main();
+    } else if (fork) {
+      side.emplace(Call(X, dOut));
+      on = side->stream();
+    }
+    dWg = dweight_on(X, dY, Ind, EGS_DW_GATHERED_ROWS, -1, -1, std::nullopt, on, &ws);
+  }
+  if (need_x && !dX.defined()) dX = gemm_scatter(dY, Wg, Ind, X.size(1), EGS_W_NC, std::nullopt, -1, -1, std::nullopt, std::nullopt);
+  return {dX, dWg, dWs};
+}
+
 struct GatherScatterFunction : torch::autograd::Function<GatherScatterFunction> {
   static Tensor forward(AutogradContext* ctx, const Tensor& X_, const Tensor& Wg_, const Tensor& Ws_, const Tensor& Ind) {
     const Tensor X = X_.contiguous(), Wg = Wg_.contiguous(), Ws = Ws_.contiguous();
-    const bool fused = fused_pair_preferred(X, Wg, Ind);
-    Tensor Y, out;
-    if (fused) {
-      std::tie(Y, out) = gather_scatter_pair(X, Wg, Ws, Ind, EGS_W_CN, std::nullopt, -1);
-    } else {
-      Y = gather_gemm(X, Wg, Ind, EGS_W_CN, -1, -1, std::nullopt);
-      out = gemm_scatter(Y, Ws, Ind, X.size(1), EGS_W_CN, std::nullopt, -1, -1, std::nullopt, std::nullopt);
-    }
+    auto [Y, out, fused] = gather_scatter_forward(X, Wg, Ws, Ind);
     ctx->saved_data["fused"] = fused;
     ctx->save_for_backward({X, Wg, Ws, Ind, Y});
     return out;
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
     const auto s = ctx->get_saved_variables();
-    const Tensor &X = s[0], &Wg = s[1], &Ws = s[2], &Y = s[4];
-    const Tensor Ind = index_tensor(s[3]).t;
-    const bool need_x = ctx->needs_input_grad(0), need_wg = ctx->needs_input_grad(1), need_ws = ctx->needs_input_grad(2);
-    const Tensor dOut = grads[0].contiguous();
-    Tensor dX, dWg, dWs, dY, ws;
-    std::optional<SideStream> side;
-    const bool fork = worth_a_side_stream(Y, Wg);
-    std::optional<cudaStream_t> on;
-    if (need_ws) {                                     // needs only dOut and Y
-      if (fork) {
-        side.emplace(Call(X, dOut));
-        on = side->stream();
-      }
-      dWs = dweight_on(dOut, Y, Ind, EGS_DW_DIRECT_ROWS, -1, -1, std::nullopt, on, &ws);
-    }
-    if (need_x && ctx->saved_data["fused"].toBool())
-      std::tie(dY, dX) = gather_scatter_pair(dOut, Ws, Wg, Ind, EGS_W_NC, std::nullopt, -1);
-    else if (need_x || need_wg)
-      dY = gather_gemm(dOut, Ws, Ind, EGS_W_NC, -1, -1, std::nullopt);
-    if (need_wg) {
-      if (side) {
-        side->sync_from_main();
-      } else if (fork) {
-        side.emplace(Call(X, dOut));
-        on = side->stream();
-      }
-      dWg = dweight_on(X, dY, Ind, EGS_DW_GATHERED_ROWS, -1, -1, std::nullopt, on, &ws);
-    }
-    if (need_x && !dX.defined()) dX = gemm_scatter(dY, Wg, Ind, X.size(1), EGS_W_NC, std::nullopt, -1, -1, std::nullopt, std::nullopt);
-    return {dX, dWg, dWs, Tensor()};
+    auto d = gather_scatter_backward(s[0], s[1], s[2], s[3], s[4], grads[0], ctx->saved_data["fused"].toBool(), ctx->needs_input_grad(0),
+                                     ctx->needs_input_grad(1), ctx->needs_input_grad(2));
+    return {d[0], d[1], d[2], Tensor()};
   }
 };
 
@@ -694,13 +705,21 @@ OptTensor gather_scatter_autograd(const Tensor& X, const Tensor& Wg, const Tenso
   return GatherScatterFunction::apply(X, Wg, Ws, Ind);
 }
 
-std::tuple<Tensor, Tensor> gather_backward_op(const Tensor& X, const Tensor& W, const Tensor& Ind, const Tensor& dY) {
-  Grads g = gather_backward(X, W, Ind, dY, true, true, false);
-  return {g.in, g.w};
+// The backward passes for the Python functions: gradients that are not needed come back as None.
+OptTensor opt(const Tensor& t) { return t.defined() ? OptTensor(t) : std::nullopt; }
+using OptGrads = std::tuple<OptTensor, OptTensor, OptTensor>;
+OptGrads gather_backward_op(const Tensor& X, const Tensor& W, const Tensor& Ind, const Tensor& dY, bool need_x, bool need_w, bool need_b) {
+  Grads g = gather_backward(X, W, Ind, dY, need_x, need_w, need_b);
+  return {opt(g.in), opt(g.w), opt(g.b)};
 }
-std::tuple<Tensor, Tensor> scatter_backward_op(const Tensor& Y, const Tensor& W, const Tensor& Ind, const Tensor& dOut) {
-  Grads g = scatter_backward(Y, W, Ind, dOut, true, true, false);
-  return {g.in, g.w};
+OptGrads scatter_backward_op(const Tensor& Y, const Tensor& W, const Tensor& Ind, const Tensor& dOut, bool need_y, bool need_w, bool need_b) {
+  Grads g = scatter_backward(Y, W, Ind, dOut, need_y, need_w, need_b);
+  return {opt(g.in), opt(g.w), opt(g.b)};
+}
+OptGrads gather_scatter_backward_op(const Tensor& X, const Tensor& Wg, const Tensor& Ws, const Tensor& Ind, const Tensor& Y, const Tensor& dOut,
+                                    bool fused, bool need_x, bool need_wg, bool need_ws) {
+  auto d = gather_scatter_backward(X, Wg, Ws, Ind, Y, dOut, fused, need_x, need_wg, need_ws);
+  return {opt(d[0]), opt(d[1]), opt(d[2])};
 }
 
 // ---- the explicit step ---------------------------------------------------------------------------------------------------------
@@ -763,5 +782,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gather_scatter_autograd", &gather_scatter_autograd, nogil());
   m.def("gather_backward", &gather_backward_op, nogil());
   m.def("scatter_backward", &scatter_backward_op, nogil());
+  m.def("gather_scatter_forward", &gather_scatter_forward, nogil());
+  m.def("gather_scatter_backward", &gather_scatter_backward_op, nogil());
   m.def("train_step", &train_step, nogil());
 }

@@ -46,7 +46,7 @@ def _gather_forward(X, W, Ind, out_dtype):
 
 def _gather_backward(X, W, Ind, grad_output, out_dtype):
     # dX = scatter(dY @ W_g^T), dW_g = gather(X)^T @ dY        (reference: egs/triton_kernels.py:400-441)
-    return ops._host().gather_backward(X, W, Ind, grad_output)
+    return ops._host().gather_backward(X, W, Ind, grad_output, True, True, False)[:2]
 
 
 def _scatter_forward(Y, W, Ind, T, out_dtype):
@@ -56,7 +56,7 @@ def _scatter_forward(Y, W, Ind, T, out_dtype):
 
 def _scatter_backward(Y, W, Ind, grad_X, out_dtype):
     # dY = gather(dOut) @ W_s^T, dW_s = Y^T @ gather(dOut)     (reference: egs/triton_kernels.py:483-525)
-    return ops._host().scatter_backward(Y, W, Ind, grad_X)
+    return ops._host().scatter_backward(Y, W, Ind, grad_X, True, True, False)[:2]
 
 
 # ---- fake (meta) implementations: shapes and dtypes only --------------------------------------------
@@ -145,9 +145,7 @@ class ExpertGatherFunction(torch.autograd.Function):
         if need_x and need_w:
             grad_X, grad_W = expert_gather_backward_call(X, W, Ind, grad_output, ctx.dtype)
             return grad_X, grad_W, None, None
-        grad_output = grad_output.contiguous()
-        grad_X = ops.gemm_scatter(grad_output, W, Ind, X.shape[1], w_layout="nc") if need_x else None
-        grad_W = ops.dweight(X, grad_output, Ind, out_layout="gathered_rows") if need_w else None
+        grad_X, grad_W, _ = ops._host().gather_backward(X, W, Ind, grad_output, need_x, need_w, False)
         return grad_X, grad_W, None, None
 
 
@@ -173,9 +171,7 @@ class ExpertScatterFunction(torch.autograd.Function):
         if need_y and need_w:
             grad_Y, grad_W = expert_scatter_backward_call(Y, W, Ind, grad_X, ctx.dtype)
             return grad_Y, grad_W, None, None, None
-        grad_X = grad_X.contiguous()
-        grad_Y = ops.gather_gemm(grad_X, W, Ind, w_layout="nc") if need_y else None
-        grad_W = ops.dweight(grad_X, Y, Ind, out_layout="direct_rows") if need_w else None
+        grad_Y, grad_W, _ = ops._host().scatter_backward(Y, W, Ind, grad_X, need_y, need_w, False)
         return grad_Y, grad_W, None, None, None
 
 
@@ -195,19 +191,16 @@ class ExpertGatherBiasFunction(torch.autograd.Function):
     def backward(ctx, grad_output):
         X, W, Ind = ctx.saved_tensors
         need_x, need_w, need_b = ctx.needs_input_grad[:3]
-        grad_output = grad_output.contiguous()
-        grad_W = ops.dweight(X, grad_output, Ind, out_layout="gathered_rows") if need_w else None
-        grad_X = ops.gemm_scatter(grad_output, W, Ind, X.shape[1], w_layout="nc") if need_x else None
-        grad_b = grad_output.sum(dim=(0, 2)).reshape(ctx.bias_shape) if need_b else None
-        return grad_X, grad_W, grad_b, None
+        grad_X, grad_W, grad_b = ops._host().gather_backward(X, W, Ind, grad_output, need_x, need_w, need_b)
+        return grad_X, grad_W, grad_b.reshape(ctx.bias_shape) if need_b else None, None
 
 
 class ExpertScatterBiasFunction(torch.autograd.Function):
     """``ExpertScatterFunction`` with a per-expert bias added to every routed slot's product before it is scattered:
     ``Out[b,t,:] = sum over slots (e,k) routed to t of (Y[b,e,k,:] @ W[e] + bias[e])`` with bias [E,1,I], fused into the
     scatter's epilogue.  ``apply(Y, W, bias, Ind, T)``; backward returns ``(grad_Y, grad_W, grad_bias, None, None)``.
-    grad_bias[e] is the sum over the slots of expert e of the gathered rows of grad_Out - operator D against a tensor of
-    ones, so no [B,E,K,I] gather is materialised."""
+    grad_bias[e] is the sum over the slots of expert e of the gathered rows of grad_Out (no [B,E,K,I] gather is
+    materialised)."""
 
     @staticmethod
     def forward(ctx, Y, W, bias, Ind, T):
@@ -219,14 +212,8 @@ class ExpertScatterBiasFunction(torch.autograd.Function):
     def backward(ctx, grad_X):
         Y, W, Ind = ctx.saved_tensors
         need_y, need_w, need_b = ctx.needs_input_grad[:3]
-        grad_X = grad_X.contiguous()
-        grad_W = ops.dweight(grad_X, Y, Ind, out_layout="direct_rows") if need_w else None
-        grad_Y = ops.gather_gemm(grad_X, W, Ind, w_layout="nc") if need_y else None
-        grad_b = None
-        if need_b:
-            ones = torch.ones(Y.shape[0], Y.shape[1], Y.shape[2], 8, device=Y.device, dtype=Y.dtype)
-            grad_b = ops.dweight(grad_X, ones, Ind, out_layout="gathered_rows")[:, :, 0].reshape(ctx.bias_shape)
-        return grad_Y, grad_W, grad_b, None, None
+        grad_Y, grad_W, grad_b = ops._host().scatter_backward(Y, W, Ind, grad_X, need_y, need_w, need_b)
+        return grad_Y, grad_W, grad_b.reshape(ctx.bias_shape) if need_b else None, None, None
 
 
 class ExpertGatherScatterFunction(torch.autograd.Function):
@@ -237,18 +224,14 @@ class ExpertGatherScatterFunction(torch.autograd.Function):
     Where the fused kernel pays (float32, single-wave grids: ``ops.fused_pair_preferred``) the forward pass is one
     kernel (Y is written once, for the backward pass, and consumed from shared memory) and so is dY -> dX of the
     backward pass; otherwise each pass runs the two separate operators.  The weight gradients are the same two
-    contractions as in ``ExpertGatherFunction`` / ``ExpertScatterFunction``.  backward returns ``(grad_X, grad_W_g, grad_W_s, None)``; gradients autograd does not ask for are skipped.
+    contractions as in ``ExpertGatherFunction`` / ``ExpertScatterFunction`` and run next to dY -> dX on the helper
+    stream.  backward returns ``(grad_X, grad_W_g, grad_W_s, None)``; gradients autograd does not ask for are skipped.
     """
 
     @staticmethod
     def forward(ctx, X, Wg, Ws, Ind):
         X, Wg, Ws = X.contiguous(), Wg.contiguous(), Ws.contiguous()
-        ctx.fused = ops.fused_pair_preferred(X, Wg, Ind)
-        if ctx.fused:
-            Y, Out = ops.gather_scatter_pair(X, Wg, Ws, Ind, w_layout="cn")
-        else:
-            Y = ops.gather_gemm(X, Wg, Ind, w_layout="cn")
-            Out = ops.gemm_scatter(Y, Ws, Ind, X.shape[1], w_layout="cn")
+        Y, Out, ctx.fused = ops._host().gather_scatter_forward(X, Wg, Ws, Ind)
         ctx.save_for_backward(X, Wg, Ws, Ind, Y)
         return Out
 
@@ -256,16 +239,4 @@ class ExpertGatherScatterFunction(torch.autograd.Function):
     def backward(ctx, grad_out):
         X, Wg, Ws, Ind, Y = ctx.saved_tensors
         need_x, need_wg, need_ws = ctx.needs_input_grad[:3]
-        grad_out = grad_out.contiguous()
-        grad_X = grad_Wg = grad_Ws = dY = None
-        if need_ws:
-            grad_Ws = ops.dweight(grad_out, Y, Ind, out_layout="direct_rows")
-        if need_x and ctx.fused:
-            dY, grad_X = ops.gather_scatter_pair(grad_out, Ws, Wg, Ind, w_layout="nc")
-        elif need_x or need_wg:
-            dY = ops.gather_gemm(grad_out, Ws, Ind, w_layout="nc")
-        if need_wg:
-            grad_Wg = ops.dweight(X, dY, Ind, out_layout="gathered_rows")
-        if need_x and grad_X is None:
-            grad_X = ops.gemm_scatter(dY, Wg, Ind, X.shape[1], w_layout="nc")
-        return grad_X, grad_Wg, grad_Ws, None
+        return (*ops._host().gather_scatter_backward(X, Wg, Ws, Ind, Y, grad_out, ctx.fused, need_x, need_wg, need_ws), None)

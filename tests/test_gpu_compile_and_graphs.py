@@ -52,6 +52,51 @@ def test_modules_compile_with_fullgraph(cuda_device, dtype):
     assert abs(float(loss.detach()) - ref_loss) <= tol * max(1.0, float((ref["Out"].double() * ins["G"].double()).abs().sum()))
 
 
+@pytest.mark.parametrize("bias", [False, True])
+@pytest.mark.parametrize("block", [False, True])
+def test_bias_modules_and_the_block_compile(cuda_device, bias, block):
+    """Compiled calls run the Python functions (with graph breaks): the same gradients as the eager calls."""
+    w = Workload("cb", 4, 64, 6, 16, 64, 32, torch.float32, "distinct", 52)
+    ins = {k: v.to(cuda_device) for k, v in workloads.make_inputs(w).items()}
+    torch.manual_seed(3)
+    m = egs.ExpertGatherScatter(w.E, w.I, w.J, bias=bias).to(cuda_device)
+    f = m if block else lambda x, ind: m.scatter(m.gather(x, ind), ind, w.T)
+
+    def grads(f):
+        m.zero_grad()
+        x = ins["X"].clone().requires_grad_(True)
+        out = f(x, ins["Ind"])
+        out.backward(ins["G"])
+        return [out.detach(), x.grad] + [p.grad for p in m.parameters()]
+
+    for a, b in zip(grads(torch.compile(f, backend="aot_eager")), grads(f)):
+        assert orc.rel_err(a.cpu(), b.cpu()) <= 1e-5
+
+
+def test_the_functions_overlap_weight_gradients_like_the_modules(cuda_device):
+    """A direct caller of the Functions launches what the modules launch: no ones-contraction, no torch reduction."""
+    w = Workload("direct", 8, 256, 8, 64, 256, 128, torch.bfloat16, "distinct", 54)
+    ins = {k: v.to(cuda_device) for k, v in workloads.make_inputs(w).items()}
+    bg = torch.zeros(w.E, 1, w.J, device=cuda_device, dtype=w.dtype, requires_grad=True)
+    bs = torch.zeros(w.E, 1, w.I, device=cuda_device, dtype=w.dtype, requires_grad=True)
+    Wg, Ws, X = (ins[k].clone().requires_grad_(True) for k in ("Wg", "Ws", "X"))
+    host = ops._host()
+
+    def run(gather, scatter):
+        out = scatter(gather())
+        n = ops.launch_count()
+        got = torch.autograd.grad(out, (X, Wg, bg, Ws, bs), ins["G"])
+        torch.cuda.synchronize()
+        return ops.launch_count() - n, got
+
+    n_fn, fn = run(lambda: egs.kernels.ExpertGatherBiasFunction.apply(X, Wg, bg, ins["Ind"]),
+                   lambda Y: egs.kernels.ExpertScatterBiasFunction.apply(Y, Ws, bs, ins["Ind"], w.T))
+    n_native, native = run(lambda: host.gather_autograd(X, Wg, bg, ins["Ind"]), lambda Y: host.scatter_autograd(Y, Ws, bs, ins["Ind"], w.T))
+    assert n_fn == n_native
+    for a, b in zip(fn, native):
+        assert a.shape == b.shape and orc.rel_err(a.cpu(), b.cpu()) <= 1e-2
+
+
 @pytest.mark.filterwarnings("ignore:.*an autograd kernel was not registered")
 def test_backward_with_create_graph_returns_a_graph(cuda_device):
     """The dispatcher ops have no second derivative of their own: torch warns and goes on, for the modules as for the Functions."""
