@@ -40,7 +40,7 @@ class Dims(ctypes.Structure):
 
 class PlanInfo(ctypes.Structure):
     _fields_ = [(n, ctypes.c_int) for n in ("tensor_path", "tile_n", "stages", "row_tiles", "persistent", "bulk_epilogue",
-                                            "expert_fastest", "splits", "rows_per_split")]
+                                            "expert_fastest", "splits", "rows_per_split", "pair", "slot_boxes", "swap")]
 
 
 _lock = threading.RLock()

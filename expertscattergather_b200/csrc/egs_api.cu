@@ -605,6 +605,8 @@ int egs_describe_plan(int op, const egs_dims* dims, int w_layout, int dtype, int
     else configure_tensor_dweight(p);
     out->tile_n = p.BN; out->stages = p.stages; out->row_tiles = p.row_tiles; out->splits = p.splits;
     out->rows_per_split = p.rows_per_split;
+    out->persistent = dtype != EGS_F32 || precision == EGS_PREC_STRICT;
+    out->pair = p.pair; out->slot_boxes = p.slot_boxes; out->swap = p.swap;
     return EGS_OK;
   }
   RowGemmParams p{};
@@ -616,7 +618,7 @@ int egs_describe_plan(int op, const egs_dims* dims, int w_layout, int dtype, int
   else if (precision == EGS_PREC_STRICT) configure_strict_rowgemm(p);
   else configure_tensor_rowgemm(p, op == 1);
   out->tile_n = p.BN; out->stages = p.stages; out->row_tiles = p.row_tiles; out->persistent = p.persistent;
-  out->bulk_epilogue = (p.persistent || op == 1) ? p.bulk_epilogue : 0; out->expert_fastest = p.expert_fastest;
+  out->expert_fastest = p.expert_fastest; out->pair = p.pair; out->slot_boxes = p.slot_boxes;
   return EGS_OK;
 }
 

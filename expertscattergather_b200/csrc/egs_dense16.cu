@@ -871,10 +871,10 @@ void configure_dense16_rowgemm(RowGemmParams& p, bool scatter) {
   const Tile t = pick_tile(p.N, p.M, p.E, steps, cp_rows ? 340.0 : 0.0, 0.0, 16.0, scatter);
   p.BN = t.bn;
   p.pair = t.pair ? 1 : 0;
-  p.bulk_epilogue = scatter ? 1 : 0;
+  p.slot_boxes = scatter && !cp_rows ? 1 : 0;
   p.stages = ring_stages(p.pair ? p.BN / 2 : p.BN, p.w_layout == EGS_W_NC, kRowTable + epi_bytes(!cp_rows));
-  p.row_tiles = 2;        // two 128-row accumulators per CTA
-  p.persistent = (scatter && steps <= 4) ? 1 : 0;        // (for egs_describe_plan) the additions outlast the contraction
+  p.row_tiles = 1;
+  p.persistent = 1;
 }
 
 cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dtype, cudaStream_t st) {
@@ -901,7 +901,7 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
   const unsigned long long dims[3] = {inner, outer, static_cast<unsigned long long>(r.E)};
   const unsigned box[3] = {64u, p.nc ? static_cast<unsigned>(p.half) : static_cast<unsigned>(kStep), 1u};
   if (!encode_tensor_map_16bit(&mw, r.W, 3, dims, box)) return cudaErrorInvalidValue;
-  p.tma_rows = scatter && rows_fit_boxes(r.K, 128) && encode_slot_rows(&mr, r.A, r.B, r.E, r.K, r.C, 128);
+  p.tma_rows = r.slot_boxes && encode_slot_rows(&mr, r.A, r.B, r.E, r.K, r.C, 128);
   if (r.pair && !p.tma_rows &&
       !encode_gather(&mr, r.A, scatter ? static_cast<long long>(r.M) * r.E : static_cast<long long>(r.B) * r.T, r.C))
     return cudaErrorInvalidValue;
@@ -947,7 +947,8 @@ void configure_dense16_dweight(DWeightParams& p) {
     }
   }
   p.stages = ring_stages(p.pair ? p.BN / 2 : p.BN, false, table_bytes(slot_cp) + epi_bytes(false));
-  p.row_tiles = 2;        // two 128-row accumulators per CTA
+  p.row_tiles = 1;
+  p.slot_boxes = slot_cp ? 0 : 1;
 }
 
 cudaError_t launch_dense16_dweight(const DWeightParams& r, int dtype, cudaStream_t st) {
@@ -970,7 +971,7 @@ cudaError_t launch_dense16_dweight(const DWeightParams& r, int dtype, cudaStream
   if (units > 2147483647ll - kSms) return cudaErrorInvalidValue;
   p.units = static_cast<int>(units);
   TensorMap3 mw{}, mr{};
-  p.tma_rows = rows_fit_boxes(r.K, kStep) && encode_slot_rows(&mr, r.Ysrc, r.B, r.E, r.K, r.FD, kStep);
+  p.tma_rows = r.slot_boxes && encode_slot_rows(&mr, r.Ysrc, r.B, r.E, r.K, r.FD, kStep);
   if (r.pair && (!encode_gather(&mw, r.Xsrc, static_cast<long long>(r.B) * r.T, r.FG) ||
                  (!p.tma_rows && !encode_gather(&mr, r.Ysrc, static_cast<long long>(r.M) * r.E, r.FD))))
     return cudaErrorInvalidValue;

@@ -80,8 +80,8 @@ struct RowGemmParams {
   int row_tiles;      // tensor path: 128-row accumulator tiles per CTA (1 or 2)
   int persistent;     // tensor path: 1 = persistent warp-specialised variant
   int pair;           // 16-bit G, S: tiles of 256 rows on pairs of SMs
+  int slot_boxes;     // 16-bit S: slot rows come as TMA boxes
   int after_own;      // launched behind a kernel of the same call (fill, preparation): see launch_kernel
-  int bulk_epilogue;  // 16-bit S: additions go out as whole 128-byte row segments (for egs_describe_plan)
 };
 
 struct DWeightParams {
@@ -103,6 +103,7 @@ struct DWeightParams {
   int after_own;      // launched behind the fill of `acc`: see launch_kernel
   int swap;           // 16-bit: the slot rows' features run along the accumulator's rows
   int pair;           // 16-bit: tiles of 256 rows on pairs of SMs
+  int slot_boxes;     // 16-bit: slot rows come as TMA boxes
 };
 
 // Fused pair G -> S (tensor path only):  Mid = gather(Src) x W1[e] is stored as slot rows AND fed, without leaving the

@@ -609,7 +609,6 @@ void configure_strict_rowgemm(RowGemmParams& p) {
   p.stages = strict_raw_stages(p.BN, long_contraction(p.C));
   p.row_tiles = 1;
   p.persistent = 1;
-  p.bulk_epilogue = 0;
 }
 
 cudaError_t launch_strict_rowgemm(const RowGemmParams& r, bool scatter, cudaStream_t st) {

@@ -1405,7 +1405,6 @@ size_t configure_tensor_rowgemm(RowGemmParams& p, bool scatter) {
   // persistent variant (see its kernel): scatter problems with many tiles, non-strict arithmetic
   const long long tiles1 = static_cast<long long>((p.M + kTileM - 1) / kTileM) * n_tiles * p.E;
   p.persistent = 0;
-  p.bulk_epilogue = 0;
   // (measured: it wins for contractions of up to four stages - the scatter of cfg4 and cfg2 - and loses for longer ones)
   if (scatter && p.C * es <= 512 && tiles1 >= 2 * kSmCount) {
     const size_t st1 = static_cast<size_t>(kTileM) * 128 + b_bytes;

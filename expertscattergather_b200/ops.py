@@ -295,7 +295,8 @@ def dweight(Xsrc, Ysrc, Ind, *, out_layout="gathered_rows", precision=None, path
 
 def describe_plan(op: str, B, T, E, K, C, N, dtype, *, w_layout="cn", precision=None) -> dict:
     """The kernel variant 'auto' runs for operator op ('G', 'S' or 'D'; for D pass C = FG, N = FD) at these sizes:
-    dict with tensor_path, tile_n, stages, row_tiles, persistent, bulk_epilogue, expert_fastest, splits, rows_per_split."""
+    dict with tensor_path, tile_n, stages, row_tiles, persistent, bulk_epilogue, expert_fastest, splits, rows_per_split,
+    pair, slot_boxes, swap (see ``egs_plan_info``)."""
     lib = _lib.load()
     dims = _lib.Dims(B, T, E, K, C, N)
     info = _lib.PlanInfo()

@@ -271,13 +271,15 @@ typedef struct egs_plan_info {
   int tensor_path;    /* 1: tcgen05 tensor-core kernels, 0: generic CUDA-core kernels (the fields below are then 0) */
   int tile_n;         /* tile width over the produced features */
   int stages;         /* depth of the shared-memory stage ring */
-  int row_tiles;      /* 128-row accumulators a CTA holds: 1 or 2 */
-  int persistent;     /* float32 S: 1 = the persistent kernel.  16-bit tensors (all kernels are persistent): 1 = a scatter whose
-                       * tiles are bound by their additions, not by their contraction */
-  int bulk_epilogue;  /* S with 16-bit tensors: direct additions go out as whole 128-byte row segments */
+  int row_tiles;      /* 128-row blocks a CTA multiplies with one weight tile: 1 or 2 */
+  int persistent;     /* 1: CTAs walk the tiles (all 16-bit and strict float32 kernels, some TF32 scatters), 0: one tile a CTA */
+  int bulk_epilogue;  /* always 0: no kernel of the automatic path adds whole rows by the copy engine */
   int expert_fastest; /* G / S: grid order, 1 = experts vary fastest */
   int splits;         /* D: row ranges the contraction is split into */
   int rows_per_split; /* D: contraction rows per range */
+  int pair;           /* 16-bit tensors: 1 = tiles of 256 rows on pairs of SMs (cta_group::2) */
+  int slot_boxes;     /* 16-bit S and D: 1 = slot rows come as TMA boxes, 0 = row by row */
+  int swap;           /* 16-bit D: 1 = the slot rows' features are the accumulator's rows */
 } egs_plan_info;
 int egs_describe_plan(int op, const egs_dims* dims, int w_layout, int dtype, int precision, egs_plan_info* out);
 

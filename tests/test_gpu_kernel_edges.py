@@ -205,10 +205,31 @@ def test_train_step_on_another_device_than_the_current():
         assert np.array_equal(got[k].double().numpy(), ref[k]), k
 
 
-# 16-bit kernels: one CTA or a pair per tile (the last two shapes are large enough for pairs), slot rows as boxes (K = 1, 16, 64, 128)
-# or gathered (K = 43, 101), one row or one column block in the last tile, row ranges of D that are split and that are not
-@pytest.mark.parametrize("B,T,E,K,I,J", [(1, 8, 1, 1, 8, 8), (3, 60, 2, 43, 72, 40), (5, 90, 3, 64, 264, 136), (33, 70, 5, 16, 520, 264),
-                                         (5, 300, 2, 128, 1000, 200), (9, 777, 24, 101, 1000, 200), (20, 200, 24, 64, 520, 512)])
+# 16-bit kernels: one CTA or a pair per tile, slot rows as boxes (K = 1, 16, 64, 128) or gathered (K = 43, 101), one row or one column
+# block in the last tile, row ranges of D that are split and that are not
+DENSE16_EDGES = [(1, 8, 1, 1, 8, 8), (3, 60, 2, 43, 72, 40), (5, 90, 3, 64, 264, 136), (33, 70, 5, 16, 520, 264),
+                 (5, 300, 2, 128, 1000, 200), (9, 777, 24, 101, 1000, 200), (20, 200, 24, 64, 520, 512), (40, 64, 2, 128, 72, 40),
+                 (8, 100, 40, 50, 40, 256)]
+
+PAIR_SHAPES = [(20, 200, 24, 64, 520, 512), (24, 600, 40, 72, 1280, 320)]          # compared on the device: see the repeated launches
+
+
+def _dense16_plans(B, T, E, K, I, J):
+    plan = lambda op, c, n, **kw: ops.describe_plan(op, B, T, E, K, c, n, torch.float16, **kw)
+    return {"G": plan("G", I, J), "dY": plan("G", I, J, w_layout="nc"), "S": plan("S", J, I), "dX": plan("S", J, I, w_layout="nc"),
+            "D": plan("D", I, J)}
+
+
+def test_dense16_edges_reach_every_form(cuda_device):
+    plans = [_dense16_plans(*shape) for shape in DENSE16_EDGES + PAIR_SHAPES]
+    for op in ("G", "dY", "S", "dX", "D"):
+        assert {p[op]["pair"] for p in plans} == {0, 1}, op
+    assert {(p["D"]["splits"] > 1) for p in plans} == {False, True} and {p["D"]["swap"] for p in plans} == {0, 1}
+    for op in ("S", "D"):         # slot rows as boxes and gathered, on one CTA and in a pair
+        assert {(p[op]["pair"], p[op]["slot_boxes"]) for p in plans} == {(0, 0), (0, 1), (1, 0), (1, 1)}, op
+
+
+@pytest.mark.parametrize("B,T,E,K,I,J", DENSE16_EDGES)
 @pytest.mark.parametrize("bias", [False, True])
 def test_dense16_edges(cuda_device, B, T, E, K, I, J, bias):
     g = torch.Generator().manual_seed(I + J)
@@ -257,8 +278,10 @@ def test_dense16_dweight_sums_long_contractions_in_ranges(cuda_device, B, T, E, 
 # pairs of SMs: the leader multiplies what both CTAs have staged.  The same launches over and over, under copies on another stream
 # that disturb their timing, give the same bits (integer values: every sum is exact in any order), with slot rows that come as boxes
 # (K = 64) and that are gathered (K = 72)
-@pytest.mark.parametrize("B,T,E,K,I,J", [(20, 200, 24, 64, 520, 512), (24, 600, 40, 72, 1280, 320)])
+@pytest.mark.parametrize("B,T,E,K,I,J", PAIR_SHAPES)
 def test_dense16_pairs_repeat_their_bits(cuda_device, B, T, E, K, I, J):
+    for plan in _dense16_plans(B, T, E, K, I, J).values():
+        assert plan["pair"] and plan["slot_boxes"] in (0, int(K == 64)), plan
     g = torch.Generator(device=cuda_device).manual_seed(J)
     dt = torch.float16
     small = lambda *shape: torch.randint(-1, 2, shape, generator=g, device=cuda_device).to(dt)

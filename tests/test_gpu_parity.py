@@ -443,17 +443,14 @@ def _rel_err_on_device(a, ref):
 def test_full_size_parity_of_the_tensor_bound_configurations(cuda_device, name, B, chunk):
     """cfg4 at its per-GPU batch (64) and cfg3 at full size through the explicit step: every element of Y, Out, dY, dX, dW_g
     and dW_s against the checker, and the kernel variants the benchmark times at these sizes must be the ones that ran
-    (256-row gather CTAs, the persistent scatter with bulk reductions, two-accumulator weight-gradient CTAs)."""
+    (tiles of 256 rows on pairs of SMs for all three operators, slot rows as boxes)."""
     w = workloads.WORKLOADS[name].with_batch(B)
     plan_g = ops.describe_plan("G", B, w.T, w.E, w.K, w.I, w.J, w.dtype)
     plan_s = ops.describe_plan("S", B, w.T, w.E, w.K, w.J, w.I, w.dtype)
     plan_d = ops.describe_plan("D", B, w.T, w.E, w.K, w.I, w.J, w.dtype)
-    assert plan_g["tensor_path"] and plan_g["row_tiles"] == 2, plan_g
-    assert plan_d["tensor_path"] and plan_d["row_tiles"] == 2, plan_d
-    if name == "cfg4":
-        assert plan_s["persistent"] == 1 and plan_s["bulk_epilogue"] == 1 and plan_s["expert_fastest"] == 1, plan_s
-    else:
-        assert plan_s["tensor_path"] == 1 and plan_s["persistent"] == 0, plan_s
+    for plan in (plan_g, plan_s, plan_d):
+        assert plan["tensor_path"] and plan["persistent"] and plan["pair"] and plan["tile_n"] == 256, plan
+    assert plan_s["slot_boxes"] and plan_d["slot_boxes"] and plan_s["expert_fastest"] == (name == "cfg4"), (plan_s, plan_d)
     d = to_dev(workloads.make_inputs(w), cuda_device)
     ops.reset_status()
     got = train_step(d["X"], d["Wg"], d["Ws"], d["Ind"], d["G"])
@@ -477,8 +474,9 @@ def test_strict_float32_on_long_contractions(cuda_device):
     """Strict float32 is three TF32 products per element (hi*hi + hi*lo + lo*hi) summed in the tensor core's float32
     accumulator, whose additions truncate: the error grows with the number of accumulation steps (3.3e-5 at a contraction
     of 4096, 1.5e-5 after 8192 rows of D were measured with everything on the tensor cores).  The library therefore
-    bounds what one accumulator sees: G / S beyond a contraction of 512 take the FFMA kernels, D splits its rows into
-    ranges of at most 1024 whose partial tiles are summed by float32 atomics.  Checked against float64 truth."""
+    bounds what one accumulator sees: 512 elements of G / S, single steps of longer contractions up to 2048 (summed with
+    correct rounding; the FFMA kernels run beyond), 1024 rows of D, whose partial tiles are summed by float32 atomics.
+    Checked against float64 truth."""
     w = Workload("long", 64, 512, 2, 128, 4096, 64, torch.float32, "distinct", 99)
     ins = workloads.make_inputs(w)
     d = to_dev(ins, cuda_device)
@@ -492,7 +490,7 @@ def test_strict_float32_on_long_contractions(cuda_device):
     ops.check_status()
     e_g = orc.rel_err(Y.cpu(), orc.np_gather(ins["X"], ins["Wg"], ins["Ind"]))
     e_d = orc.rel_err(dWg.cpu(), orc.np_dweight(ins["X"], Y.cpu(), ins["Ind"]))
-    # the longest contraction that stays on the tensor cores in strict mode
+    # the longest contraction that one accumulator sums
     w2 = Workload("long512", 16, 256, 4, 64, 512, 64, torch.float32, "distinct", 98)
     ins2 = workloads.make_inputs(w2)
     d2 = to_dev(ins2, cuda_device)
