@@ -47,3 +47,28 @@ def test_a_wait_that_cannot_be_satisfied_runs_out_and_is_reported(cuda_device):
     torch.cuda.synchronize()
     ops.check_status()
     assert torch.equal(again, good)
+
+
+@pytest.mark.parametrize("dtype,precision,path", [(torch.bfloat16, "strict", "tensor"), (torch.float32, "strict", "tensor"),
+                                                  (torch.float32, "tf32", "tensor"), (torch.bfloat16, "strict", "paired")])
+def test_the_next_call_raises_without_a_check(cuda_device, dtype, precision, path):
+    """A kernel that gives up stores the reason in the host's mirror of the status word as well, and the next operator call
+    raises: nobody has to ask.  (The kernel here finds the bit of a wait that ran out before it.)"""
+    lib = _lib.load()
+    ops.reset_status()
+    w = Workload("mirror", 4, 64, 2, 40, 64, 32, dtype, "distinct", 4)
+    d = {k: v.to(cuda_device) for k, v in workloads.make_inputs(w, integer_valued=True).items()}
+    call = lambda: ops.gather_gemm(d["X"], d["Wg"], d["Ind"], path=path, precision=precision)
+    good = call()
+    out2 = torch.zeros(2, dtype=torch.int32, device=cuda_device)
+    rc = lib.egs_selftest_wait_timeout(ops._status_word(cuda_device).data_ptr(), out2.data_ptr(), ctypes.c_int64(1_000_000),
+                                       torch.cuda.current_stream(cuda_device).cuda_stream)
+    _lib.check(rc, "egs_selftest_wait_timeout")
+    call()                                   # finds the bit, does no work and tells the host
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="bounded wait"):
+        call()
+    again = call()                           # cleared on both sides: usable and right again
+    torch.cuda.synchronize()
+    ops.check_status()
+    assert torch.equal(again, good)
