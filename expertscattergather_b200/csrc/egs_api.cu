@@ -24,6 +24,14 @@ bool encode_tensor_map_16bit(TensorMap3* out, const void* base, int rank, const 
     return reinterpret_cast<EncodeFn>(fn);
   }();
   static_assert(sizeof(TensorMap3) == sizeof(CUtensorMap), "tensor map size");
+  // The encoder is a driver call and wants a current context, which a thread has from its first runtime call that needs one.  The
+  // encoding may come before that: in autograd's thread, for instance, at the first backward pass of a process.
+  static thread_local bool has_context = false;
+  if (!has_context) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return false;
+    has_context = true;
+  }
   if (!encode || !out || !base || rank < 2 || rank > 4) return false;
   cuuint64_t gdim[4], gstride[3];
   cuuint32_t bdim[4], estride[4] = {1u, 1u, 1u, 1u};

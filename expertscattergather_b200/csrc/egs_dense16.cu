@@ -901,7 +901,8 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
   const unsigned long long dims[3] = {inner, outer, static_cast<unsigned long long>(r.E)};
   const unsigned box[3] = {64u, p.nc ? static_cast<unsigned>(p.half) : static_cast<unsigned>(kStep), 1u};
   if (!encode_tensor_map_16bit(&mw, r.W, 3, dims, box)) return cudaErrorInvalidValue;
-  p.tma_rows = r.slot_boxes && encode_slot_rows(&mr, r.A, r.B, r.E, r.K, r.C, 128);
+  p.tma_rows = r.slot_boxes;
+  if (p.tma_rows && !encode_slot_rows(&mr, r.A, r.B, r.E, r.K, r.C, 128)) return cudaErrorInvalidValue;
   if (r.pair && !p.tma_rows &&
       !encode_gather(&mr, r.A, scatter ? static_cast<long long>(r.M) * r.E : static_cast<long long>(r.B) * r.T, r.C))
     return cudaErrorInvalidValue;
@@ -971,7 +972,8 @@ cudaError_t launch_dense16_dweight(const DWeightParams& r, int dtype, cudaStream
   if (units > 2147483647ll - kSms) return cudaErrorInvalidValue;
   p.units = static_cast<int>(units);
   TensorMap3 mw{}, mr{};
-  p.tma_rows = r.slot_boxes && encode_slot_rows(&mr, r.Ysrc, r.B, r.E, r.K, r.FD, kStep);
+  p.tma_rows = r.slot_boxes;
+  if (p.tma_rows && !encode_slot_rows(&mr, r.Ysrc, r.B, r.E, r.K, r.FD, kStep)) return cudaErrorInvalidValue;
   if (r.pair && (!encode_gather(&mw, r.Xsrc, static_cast<long long>(r.B) * r.T, r.FG) ||
                  (!p.tma_rows && !encode_gather(&mr, r.Ysrc, static_cast<long long>(r.M) * r.E, r.FD))))
     return cudaErrorInvalidValue;

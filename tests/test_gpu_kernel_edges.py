@@ -1,5 +1,7 @@
 """Kernel variants at the sizes where their dispatch or their tiles change over: remainders, the smallest and largest of each
 range, ties.  Integer-valued or index results are compared bit for bit, sums against float64."""
+import concurrent.futures
+
 import numpy as np
 import pytest
 import torch
@@ -273,6 +275,20 @@ def test_dense16_dweight_sums_long_contractions_in_ranges(cuda_device, B, T, E, 
         ref = rows.T @ Y[:, e].reshape(B * K, J).double()
         bias.append(((got[e] - ref) / ref).mean())
     assert torch.stack(bias).mean().abs().item() <= 8192 / 16 * 2.0 ** -23
+
+
+# the first CUDA call of a thread: boxes are described to the driver before anything else has made a context current there
+@pytest.mark.parametrize("op", ["G", "S", "D"])
+def test_dense16_first_call_of_a_thread(cuda_device, op):
+    B, T, E, K, I, J = 8, 128, 8, 16, 256, 64
+    X, Y = torch.ones(B, T, I, device=cuda_device).half(), torch.ones(B, E, K, J, device=cuda_device).half()
+    Wg, Ws = torch.ones(E, I, J, device=cuda_device).half(), torch.ones(E, J, I, device=cuda_device).half()
+    Ind = (torch.arange(B * E * K, device=cuda_device) % T).view(B, E, K)
+    run = {"G": lambda: ops.gather_gemm(X, Wg, Ind), "S": lambda: ops.gemm_scatter(Y, Ws, Ind, T), "D": lambda: ops.dweight(X, Y, Ind)}[op]
+    torch.cuda.synchronize()
+    with concurrent.futures.ThreadPoolExecutor(max_workers=1) as pool:
+        got = pool.submit(run).result(timeout=120)
+    assert (got == {"G": I, "S": J * E * K // T, "D": B * K}[op]).all().item()
 
 
 # pairs of SMs: the leader multiplies what both CTAs have staged.  The same launches over and over, under copies on another stream
