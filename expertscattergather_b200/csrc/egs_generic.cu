@@ -440,8 +440,8 @@ __global__ void __launch_bounds__(256) convert_to_f32_kernel(const T* __restrict
 // of the call, so that what a row is summed in does not depend on its own luck alone.
 // The ids of a batch element are counted in shared memory by one CTA (4096 ids: about 2 us) of a kernel of their own, with a flag
 // per CTA; the kernel that zeroes what the additions go to starts under it (dependent launch) and collects the flags: 2 us of the
-// chain.  With a single batch element, or few ids in all (kPrepOwnIds: as long to count as the second launch takes), the CTAs of the
-// zeroing kernel count everything themselves: a serving pass of one 64-token prompt has 25 us in all.
+// chain.  With a single batch element, or few ids and token rows in all (kPrepOwnIds of each: as long to count as the second launch
+// takes; 32712 counters a CTA took a pass with 133 MB of rows from 172 to 218 us), the CTAs of the zeroing kernel count everything themselves: a serving pass of one 64-token prompt has 25 us in all.
 // Sequences beyond kPrepCounters tokens share counters (token id modulo kPrepCounters): that can choose the float32 rows where
 // they are not needed, never the reverse.
 constexpr int kPrepThreads = 512;
@@ -679,7 +679,7 @@ static cudaError_t prepare(const void* Ind, int index_dtype, int B, int T_, int 
                            float* acc, void* out16, size_t n, int zero_output, StatusRef status, cudaStream_t st) {
   const bool count = info == nullptr && EK > limit;
   const long long ids = static_cast<long long>(B) * EK, rows = static_cast<long long>(B) * T_;
-  const bool own_count = count && (B == 1 || (ids <= kPrepOwnIds && rows <= kPrepCounters));
+  const bool own_count = count && (B == 1 || (ids <= kPrepOwnIds && rows <= kPrepOwnIds));
   const long long counters = own_count ? rows : T_;
   const size_t smem = count ? static_cast<size_t>(counters < kPrepCounters ? counters : kPrepCounters) * sizeof(int) : 0;
   cudaError_t err = cudaSuccess;
