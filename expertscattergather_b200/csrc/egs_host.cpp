@@ -1,9 +1,9 @@
 // Native host path of the package: tensor-level operators, autograd functions and the explicit training step over the C ABI
 // of libegs_b200.so.  Python (ops.py, kernels.py, torch_interface.py, step.py) only parses arguments and calls in here.
 //
-// Why it is native: a training step of a small block is eight to ten kernels of 5-30 us, and issuing them from Python cost
+// Why it is native: a training step of a small block is eight to ten kernels of 5-30 us, and issuing them from Python costs
 // 400-570 us per step (argument handling, ctypes marshalling, Python autograd functions, stream contexts), several times the
-// device time.  Issued from here a step of a tiny float32 block takes 110 us instead of 420 us, device time included.
+// device time.  Issued from here a step of a tiny float32 block takes 105 us, device time included, against 420 us from Python.
 //
 // Conventions, shared by everything in this file:
 //   * buffers (outputs, workspaces, gradients) come from torch's caching allocator on the CURRENT stream; work that runs on
@@ -490,14 +490,18 @@ Tensor expert_row_sum(const Tensor& Src, const OptTensor& Ind, int64_t B, int64_
 }
 
 // ---- backward passes of the two operators ------------------------------------------------------------------------------------
-// The weight gradient runs on the helper stream next to the dX / dY kernel: the two are independent and share the SMs.  Below
-// kSmallWork multiply-adds (kernels of under 10 us) a backward pass is bound by the host, and the fork and join are left out.
-// (At 2^27 the FFMA kernels of odd float32 sizes take 30 us and want the overlap: 117 against 131 us a pass at 132M.)
-constexpr double kSmallWork = 1 << 25;
+// The weight gradient runs on the helper stream next to the dX / dY kernel: the two are independent and share the SMs.  The fork and
+// the join cost the host 3 us, which small passes, bound by the host, would only pay for.  Where the line lies depends on the kernels:
+// forward and backward of two modules take 110 us with and 107 without the fork at 2^26 multiply-adds on the tensor cores (float32: 105
+// and 101), at 2^27 the fills of long sequences turn it (T=16384: 101 and 104 us); on the generic kernels 141 and 158 us at 2^26, and
+// at 2^25 the same.
+constexpr double kSmallTensorWork = 1 << 26, kSmallGenericWork = 1 << 25;
 bool worth_a_side_stream(const Tensor& slot_rows, const Tensor& W) {      // [B,E,K,J] and a weight tensor of E * I * J elements
   if (g_debug.load(std::memory_order_relaxed)) return false;             // every operator is checked behind its own kernels
   const double slots = static_cast<double>(slot_rows.size(0)) * slot_rows.size(2);
-  return slots * W.numel() > kSmallWork;
+  const int64_t per16 = 16 / W.element_size();                           // whole 16-byte chunks in both widths: see rowgemm_tensor_ok
+  const bool tensor = W.size(1) % per16 == 0 && W.size(2) % per16 == 0 && g_path.load(std::memory_order_relaxed) != EGS_PATH_GENERIC;
+  return slots * W.numel() > (tensor ? kSmallTensorWork : kSmallGenericWork);
 }
 struct Grads {
   Tensor in, w, b;
