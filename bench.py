@@ -701,7 +701,7 @@ def main():
             "config": cfg,
             "run": {"l2": l2_mode,
                     "cuda_graph": used_graph, "precision": ops.get_precision(),
-                    "streams": "weight gradients on a side stream next to the main chain; float32 outputs zero-filled on a fill stream",
+                    "streams": "weight gradients on a side stream next to the main chain",
                     "ms_per_step_quantiles_this_rank": {k: round(v, 5) for k, v in step_q.items()}},
             "gpu_launches": int(launches_per_step * args.steps),
             "clocks": clocks,

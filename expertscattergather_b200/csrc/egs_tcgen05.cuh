@@ -493,10 +493,7 @@ __device__ __forceinline__ void bulk_reduce_add(__half* dst, uint32_t src_smem, 
                : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read_1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-constexpr uint32_t kBulkRowPitch = 144;                  // 128 staged bytes per row + 16: conflict-free 16-byte stores
-constexpr uint32_t kBulkBufBytes = 32 * kBulkRowPitch;   // one 32-row staging buffer
 __device__ __forceinline__ void red4(float* dst, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3) {
   asm volatile("red.global.add.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(dst), "f"(__uint_as_float(x0)), "f"(__uint_as_float(x1)),
                "f"(__uint_as_float(x2)), "f"(__uint_as_float(x3))

@@ -128,8 +128,8 @@ _fill_streams: dict[int, "torch.cuda.Stream"] = {}
 
 
 def side_stream(device) -> "torch.cuda.Stream":
-    """A per-device helper stream on which independent work of one step (zero fills, weight gradients) is
-    enqueued next to the main chain.  Users fork with ``side.wait_stream(current)`` and join with
+    """A per-device helper stream for callers that enqueue independent work of their own next to the main chain (the
+    weight gradients run on one that the native host module owns).  Users fork with ``side.wait_stream(current)`` and join with
     ``current.wait_stream(side)``."""
     dev = torch.device(device)
     idx = dev.index if dev.index is not None else torch.cuda.current_device()
@@ -142,8 +142,7 @@ def side_stream(device) -> "torch.cuda.Stream":
 
 def fill_stream(device) -> "torch.cuda.Stream":
     """A second per-device helper stream, for the zero fills of a step's outputs alone: kept apart from
-    :func:`side_stream` so that the fills of the next step are not ordered behind the weight-gradient kernels of the
-    current one."""
+    :func:`side_stream` so that the fills of the next step are not ordered behind other work on it."""
     dev = torch.device(device)
     idx = dev.index if dev.index is not None else torch.cuda.current_device()
     st = _fill_streams.get(idx)
