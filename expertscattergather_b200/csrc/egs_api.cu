@@ -530,7 +530,7 @@ static int dweight_impl(const void* Xsrc, const void* Ysrc, const void* Ind, voi
   err = strict ? launch_strict_dweight(p, st) : dense16 ? launch_dense16_dweight(p, dtype, st) : tensor ? launch_tensor_dweight(p, smem, st) : launch_generic_dweight(p, dtype, st);
   if (err != cudaSuccess) return fail_cuda(err, "dweight launch");
   if (p.splits > 1 && dtype != EGS_F32) {
-    err = launch_convert_from_f32(p.acc, out, n_out, dtype, st, tensor);   // (the tensor-core kernel triggers its dependents)
+    err = launch_convert_from_f32(p.acc, out, n_out, dtype, st);
     if (err != cudaSuccess) return fail_cuda(err, "convert launch");
   }
   return EGS_OK;

@@ -96,6 +96,7 @@ struct DenseParams {
   int lane_rows;      // D: 1 = the output's rows are the accumulator's rows
   int tma_rows;       // S, D: slot rows come by TMA
   int half;           // columns of a tile one CTA stages: BN, or BN / 2 in a pair
+  int after_own;      // see launch_kernel
 };
 
 // Position in the stage ring.
@@ -200,6 +201,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     }
     mbar_init(smem_u32(&hdr->drain), 1);
     fence_mbar_init();
+    if (!p.after_own) pdl_wait();
     hdr->abort_flag = p.status.timed_out() ? 1u : 0u;
     if (smem_misaligned(smem_raw)) {
       hdr->abort_flag = 1u;
@@ -221,10 +223,10 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
   if (PAIR) cluster_sync_all();          // both CTAs' barriers are initialised before anything crosses the pair
   tc_fence_after();
   const uint32_t tmem_base = hdr->tmem_base;
-  pdl_trigger();
+  if (!p.after_own) pdl_wait();
 
   if (hdr->abort_flag != 0u) {
-    // fall through to the common exit
+    pdl_wait();                          // (and fall through to the common exit)
   } else if (PAIR && warp < kProdWarps && gathers) {
     // =========================== gather producers of a pair ===========================
     // Every warp gathers the same rows of each stage, four at a time (tile::gather4).
@@ -628,6 +630,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
         }
       }
     }
+    pdl_trigger();                       // (not before: a dependent's waiting CTAs would keep a kernel of another stream off this SM)
     __syncwarp();
   } else if (warp >= kIndexWarp) {
     // =========================== index warps ===========================
@@ -847,20 +850,20 @@ int ring_stages(int half, bool nc_tile, uint32_t not_ring) {
 }
 
 template <typename T, int OP, bool PAIR>
-cudaError_t launch(const DenseParams& p, const TensorMap3& mw, const TensorMap3& mr, bool after_own, cudaStream_t st) {
+cudaError_t launch(const DenseParams& p, const TensorMap3& mw, const TensorMap3& mr, cudaStream_t st) {
   const size_t n_bytes = (OP != kOpDweight && p.nc) ? static_cast<size_t>(p.half) * 128 : static_cast<size_t>((p.half + 63) / 64) * kSeg;
   const size_t smem = kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : kRowTable) + epi_bytes(OP == kOpScatter && p.tma_rows) +
                       p.stages * (kMTile + n_bytes);
   cudaError_t err = ensure_smem_optin<dense16_kernel<T, OP, PAIR>>(static_cast<int>(kSmemMax));
   if (err != cudaSuccess) return err;
   const int grid = PAIR ? 2 * (p.units < kSms / 2 ? p.units : kSms / 2) : (p.units < kSms ? p.units : kSms);
-  err = launch_kernel(dense16_kernel<T, OP, PAIR>, grid, kDenseThreads, smem, st, after_own, p, mw, mr);
+  err = launch_kernel(dense16_kernel<T, OP, PAIR>, grid, kDenseThreads, smem, st, true, p, mw, mr);
   count_launch();
   return err;
 }
 template <int OP, bool PAIR>
-cudaError_t launch_typed(const DenseParams& p, int dtype, const TensorMap3& mw, const TensorMap3& mr, bool after_own, cudaStream_t st) {
-  return dtype == EGS_F16 ? launch<__half, OP, PAIR>(p, mw, mr, after_own, st) : launch<__nv_bfloat16, OP, PAIR>(p, mw, mr, after_own, st);
+cudaError_t launch_typed(const DenseParams& p, int dtype, const TensorMap3& mw, const TensorMap3& mr, cudaStream_t st) {
+  return dtype == EGS_F16 ? launch<__half, OP, PAIR>(p, mw, mr, st) : launch<__nv_bfloat16, OP, PAIR>(p, mw, mr, st);
 }
 
 }  // namespace
@@ -885,6 +888,7 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
   p.index_dtype = r.index_dtype;
   p.BN = r.BN; p.stages = r.stages;
   p.half = r.pair ? r.BN / 2 : r.BN;
+  p.after_own = r.after_own;
   const int rows = r.pair ? 2 * kTileM : kTileM;
   p.tiles_m = (r.M + rows - 1) / rows;
   p.tiles_n = (r.N + r.BN - 1) / r.BN;
@@ -907,9 +911,9 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
       !encode_gather(&mr, r.A, scatter ? static_cast<long long>(r.M) * r.E : static_cast<long long>(r.B) * r.T, r.C))
     return cudaErrorInvalidValue;
   if (scatter)
-    return r.pair ? launch_typed<kOpScatter, true>(p, dtype, mw, mr, r.after_own != 0, st)
-                  : launch_typed<kOpScatter, false>(p, dtype, mw, mr, r.after_own != 0, st);
-  return r.pair ? launch_typed<kOpGather, true>(p, dtype, mw, mr, false, st) : launch_typed<kOpGather, false>(p, dtype, mw, mr, false, st);
+    return r.pair ? launch_typed<kOpScatter, true>(p, dtype, mw, mr, st)
+                  : launch_typed<kOpScatter, false>(p, dtype, mw, mr, st);
+  return r.pair ? launch_typed<kOpGather, true>(p, dtype, mw, mr, st) : launch_typed<kOpGather, false>(p, dtype, mw, mr, st);
 }
 
 // Rows one accumulator of D sums: the tensor core truncates as it adds, and the error grows with the number of additions, 1.5e-5 of
@@ -963,6 +967,7 @@ cudaError_t launch_dense16_dweight(const DWeightParams& r, int dtype, cudaStream
   p.index_dtype = r.index_dtype;
   p.BN = r.BN; p.stages = r.stages; p.splits = r.splits; p.rows_per_split = r.rows_per_split;
   p.half = r.pair ? r.BN / 2 : r.BN;
+  p.after_own = r.after_own;
   const int rows = r.pair ? 2 * kTileM : kTileM;
   p.tiles_m = (p.C + rows - 1) / rows;
   p.tiles_n = (p.N + r.BN - 1) / r.BN;
@@ -977,8 +982,8 @@ cudaError_t launch_dense16_dweight(const DWeightParams& r, int dtype, cudaStream
   if (r.pair && (!encode_gather(&mw, r.Xsrc, static_cast<long long>(r.B) * r.T, r.FG) ||
                  (!p.tma_rows && !encode_gather(&mr, r.Ysrc, static_cast<long long>(r.M) * r.E, r.FD))))
     return cudaErrorInvalidValue;
-  return r.pair ? launch_typed<kOpDweight, true>(p, dtype, mw, mr, r.after_own != 0, st)
-                : launch_typed<kOpDweight, false>(p, dtype, mw, mr, r.after_own != 0, st);
+  return r.pair ? launch_typed<kOpDweight, true>(p, dtype, mw, mr, st)
+                : launch_typed<kOpDweight, false>(p, dtype, mw, mr, st);
 }
 
 }  // namespace egs

@@ -39,6 +39,8 @@ __global__ void __launch_bounds__(NTHREADS, NJ == 4 ? 3 : 4) generic_rowgemm_ker
   const int n0 = blockIdx.y * BN;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tx = tid & 7, ty = tid >> 3;
+  pdl_wait();
+  pdl_trigger();
   const T* __restrict__ A = static_cast<const T*>(p.A);
   const T* __restrict__ W = static_cast<const T*>(p.W) + static_cast<long long>(e) * p.C * p.N;
   T* __restrict__ Out = static_cast<T*>(p.Out);
@@ -187,6 +189,8 @@ __global__ void __launch_bounds__(NTHREADS, FI * GJ > 4 ? 3 : 4) generic_dweight
   const int g0 = blockIdx.y * 32 * GJ;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tx = tid & 7, ty = tid >> 3;
+  pdl_wait();
+  pdl_trigger();
   const T* __restrict__ Xs = static_cast<const T*>(p.Xsrc);
   const T* __restrict__ Ys = static_cast<const T*>(p.Ysrc);
 
@@ -324,6 +328,7 @@ __global__ void __launch_bounds__(kSumThreads) expert_row_sum_kernel(const T* __
   float acc[PER], low[PER];                                         // running sums, and what rounding took from them
 #pragma unroll
   for (int i = 0; i < PER; ++i) acc[i] = low[i] = 0.f;
+  pdl_trigger();
   auto add = [&](int i, float t) {
     const float s = acc[i] + t, b = s - acc[i];
     low[i] += (acc[i] - (s - b)) + (t - b);
@@ -397,6 +402,7 @@ __global__ void __launch_bounds__(kSumThreads) expert_row_sum_kernel(const T* __
 // ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) fill_zero_kernel(uint4* __restrict__ p16, size_t n16, unsigned char* tail,
                                                        size_t ntail) {
+  pdl_wait();
   pdl_trigger();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   const uint4 z = make_uint4(0, 0, 0, 0);
@@ -405,6 +411,7 @@ __global__ void __launch_bounds__(256) fill_zero_kernel(uint4* __restrict__ p16,
 }
 
 __global__ void __launch_bounds__(256) fill_zero_bytes_kernel(unsigned char* p, size_t n) {
+  pdl_wait();
   pdl_trigger();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) p[i] = 0;
@@ -416,6 +423,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) convert_from_f32_kernel(const float* __restrict__ src, T* __restrict__ dst,
                                                               size_t n) {
   pdl_wait();
+  pdl_trigger();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   const size_t i0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const bool vec = sizeof(T) == 2 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0;
@@ -427,6 +435,8 @@ __global__ void __launch_bounds__(256) convert_from_f32_kernel(const float* __re
 template <typename T>
 __global__ void __launch_bounds__(256) convert_to_f32_kernel(const T* __restrict__ src, float* __restrict__ dst,
                                                             size_t n) {
+  pdl_wait();
+  pdl_trigger();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
     dst[i] = to_f32<T>(src[i]);
@@ -466,6 +476,7 @@ __device__ __forceinline__ int has_hot_row(const void* __restrict__ ind, int ind
 __global__ void __launch_bounds__(kPrepThreads) scatter_count_kernel(const void* __restrict__ ind, int index_dtype, int B, int T_, int EK,
                                                                      int limit, int* __restrict__ flags) {
   extern __shared__ int prep_cnt[];
+  pdl_wait();
   pdl_trigger();
   int flag = 0;
   for (int b = blockIdx.x; b < B && !flag; b += gridDim.x) flag = has_hot_row(ind, index_dtype, b, 1, T_, EK, limit, prep_cnt);
@@ -478,6 +489,7 @@ __global__ void __launch_bounds__(kPrepThreads) scatter_prepare_kernel(const voi
                                                                        int limit, int* __restrict__ plan, float* __restrict__ acc,
                                                                        T* __restrict__ out, size_t n, int zero_output, StatusRef status) {
   extern __shared__ int prep_cnt[];      // without `info` and `flags`
+  pdl_wait();
   pdl_trigger();
   const int tid = threadIdx.x;
   int flag = 0;
@@ -485,7 +497,6 @@ __global__ void __launch_bounds__(kPrepThreads) scatter_prepare_kernel(const voi
     flag = info[0] > limit;
     if (info[2] && blockIdx.x == 0 && tid == 0) status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
   } else if (nflags > 0) {
-    pdl_wait();
     for (int i = tid; i < nflags; i += kPrepThreads) flag |= flags[i];
     flag = __syncthreads_or(flag);
   } else if (EK > limit) {
@@ -518,6 +529,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) scatter_finish_kernel(const int* __restrict__ plan, const float* __restrict__ acc,
                                                             T* __restrict__ out, size_t n) {
   pdl_wait();
+  pdl_trigger();
   if (!*plan) return;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n / 8; i += stride) convert8<T>(acc + 8 * i, out + 8 * i);
@@ -550,10 +562,11 @@ static int width_in_32s(int n, int most) {
 cudaError_t launch_generic_rowgemm(const RowGemmParams& p, bool scatter, int dtype, cudaStream_t st) {
   const int nj = width_in_32s(p.N, 4);
   dim3 grid((p.M + TM - 1) / TM, (p.N + 32 * nj - 1) / (32 * nj), p.E);
+  cudaError_t err;
 #define EGS_LAUNCH_NJ(TY, NJV)                                                             \
   do {                                                                                     \
-    if (scatter) generic_rowgemm_kernel<TY, true, NJV><<<grid, NTHREADS, 0, st>>>(p);      \
-    else generic_rowgemm_kernel<TY, false, NJV><<<grid, NTHREADS, 0, st>>>(p);             \
+    if (scatter) err = launch_kernel(generic_rowgemm_kernel<TY, true, NJV>, grid, NTHREADS, 0, st, true, p);      \
+    else err = launch_kernel(generic_rowgemm_kernel<TY, false, NJV>, grid, NTHREADS, 0, st, true, p);             \
   } while (0)
 #define EGS_LAUNCH(TY)                       \
   do {                                       \
@@ -568,7 +581,7 @@ cudaError_t launch_generic_rowgemm(const RowGemmParams& p, bool scatter, int dty
 #undef EGS_LAUNCH
 #undef EGS_LAUNCH_NJ
   count_launch();
-  return cudaGetLastError();
+  return err;
 }
 
 // Tile over FG x FD and the split of the contraction: about four CTAs per SM, and no fewer than 64 rows in a range, below which
@@ -590,10 +603,11 @@ void configure_generic_dweight(DWeightParams& p) {
 cudaError_t launch_generic_dweight(const DWeightParams& p, int dtype, cudaStream_t st) {
   const int fi = p.row_tiles, gj = p.BN / 32;
   dim3 grid((p.FG + 32 * fi - 1) / (32 * fi), (p.FD + p.BN - 1) / p.BN, p.E * p.splits);
+  cudaError_t err;
 #define EGS_LAUNCH_FI(TY, FIV)                                                           \
   do {                                                                                   \
-    if (gj == 1) generic_dweight_kernel<TY, FIV, 1><<<grid, NTHREADS, 0, st>>>(p);       \
-    else generic_dweight_kernel<TY, FIV, 2><<<grid, NTHREADS, 0, st>>>(p);               \
+    if (gj == 1) err = launch_kernel(generic_dweight_kernel<TY, FIV, 1>, grid, NTHREADS, 0, st, true, p);       \
+    else err = launch_kernel(generic_dweight_kernel<TY, FIV, 2>, grid, NTHREADS, 0, st, true, p);               \
   } while (0)
 #define EGS_LAUNCH(TY)                       \
   do {                                       \
@@ -608,7 +622,7 @@ cudaError_t launch_generic_dweight(const DWeightParams& p, int dtype, cudaStream
 #undef EGS_LAUNCH
 #undef EGS_LAUNCH_FI
   count_launch();
-  return cudaGetLastError();
+  return err;
 }
 
 template <typename T, bool VEC>
@@ -623,6 +637,8 @@ static cudaError_t launch_row_sum(const void* Src, const void* Ind, int index_dt
   cfg.gridDim = dim3(ranks * blocks, E);
   cfg.blockDim = dim3(kSumThreads);
   cfg.stream = st;
+  // (not a dependent launch: its CTAs, several to an SM, would gather on the SMs that the kernel before it leaves first and stay there:
+  // 33 us of row sums then took 48)
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = ranks;
@@ -651,24 +667,25 @@ cudaError_t launch_expert_row_sum(const void* Src, const void* Ind, int index_dt
 cudaError_t launch_fill_zero(void* ptr, size_t bytes, cudaStream_t st) {
   if (bytes == 0) return cudaSuccess;
   const uintptr_t a = reinterpret_cast<uintptr_t>(ptr);
+  cudaError_t err;
   if (a % 16 != 0) {
-    fill_zero_bytes_kernel<<<grid_for(bytes, 256), 256, 0, st>>>(static_cast<unsigned char*>(ptr), bytes);
+    err = launch_kernel(fill_zero_bytes_kernel, grid_for(bytes, 256), 256, 0, st, true, static_cast<unsigned char*>(ptr), bytes);
   } else {
     const size_t n16 = bytes / 16, ntail = bytes % 16;
-    fill_zero_kernel<<<grid_for(n16, 256 * 4), 256, 0, st>>>(static_cast<uint4*>(ptr), n16,
-                                                            static_cast<unsigned char*>(ptr) + n16 * 16, ntail);
+    err = launch_kernel(fill_zero_kernel, grid_for(n16, 256 * 4), 256, 0, st, true, static_cast<uint4*>(ptr), n16,
+                        static_cast<unsigned char*>(ptr) + n16 * 16, ntail);
   }
   count_launch();
-  return cudaGetLastError();
+  return err;
 }
 
-cudaError_t launch_convert_from_f32(const float* src, void* dst, size_t n, int dtype, cudaStream_t st, bool after_own) {
+cudaError_t launch_convert_from_f32(const float* src, void* dst, size_t n, int dtype, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   const int grid = grid_for(n, 256 * 4);
   cudaError_t err;
-  if (dtype == EGS_F16) err = launch_kernel(convert_from_f32_kernel<__half>, grid, 256, 0, st, after_own, src, static_cast<__half*>(dst), n);
+  if (dtype == EGS_F16) err = launch_kernel(convert_from_f32_kernel<__half>, grid, 256, 0, st, true, src, static_cast<__half*>(dst), n);
   else if (dtype == EGS_BF16)
-    err = launch_kernel(convert_from_f32_kernel<__nv_bfloat16>, grid, 256, 0, st, after_own, src, static_cast<__nv_bfloat16*>(dst), n);
+    err = launch_kernel(convert_from_f32_kernel<__nv_bfloat16>, grid, 256, 0, st, true, src, static_cast<__nv_bfloat16*>(dst), n);
   else return cudaErrorInvalidValue;
   count_launch();
   return err;
@@ -688,9 +705,8 @@ static cudaError_t prepare(const void* Ind, int index_dtype, int B, int T_, int 
     nflags = B < kPrepCountCtas ? B : kPrepCountCtas;
     if (smem > 48 * 1024) err = ensure_smem_optin<scatter_count_kernel>(kPrepCounters * static_cast<int>(sizeof(int)));
     if (err != cudaSuccess) return err;
-    scatter_count_kernel<<<nflags, kPrepThreads, smem, st>>>(Ind, index_dtype, B, T_, EK, limit, flags);
+    err = launch_kernel(scatter_count_kernel, nflags, kPrepThreads, smem, st, true, Ind, index_dtype, B, T_, EK, limit, flags);
     count_launch();
-    err = cudaGetLastError();
     if (err != cudaSuccess) return err;
   }
   // four CTAs per SM, each with at least 4 KB to zero and, where it counts, no more ids than half the elements it zeroes
@@ -701,7 +717,7 @@ static cudaError_t prepare(const void* Ind, int index_dtype, int B, int T_, int 
   if (grid < 1) grid = 1;
   if (own_count && smem > 48 * 1024) err = ensure_smem_optin<scatter_prepare_kernel<T>>(kPrepCounters * static_cast<int>(sizeof(int)));
   if (err != cudaSuccess) return err;
-  err = launch_kernel(scatter_prepare_kernel<T>, static_cast<unsigned>(grid), kPrepThreads, own_count ? smem : 0, st, nflags > 0, Ind, index_dtype,
+  err = launch_kernel(scatter_prepare_kernel<T>, static_cast<unsigned>(grid), kPrepThreads, own_count ? smem : 0, st, true, Ind, index_dtype,
                       B, T_, EK, info, flags, nflags, limit, plan, acc, static_cast<T*>(out16), n, zero_output, status);
   count_launch();
   return err;
@@ -733,12 +749,13 @@ cudaError_t launch_scatter_finish(const int* plan, const float* acc, void* out16
 cudaError_t launch_convert_to_f32(const void* src, float* dst, size_t n, int dtype, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   const int grid = grid_for(n, 256 * 4);
-  if (dtype == EGS_F16) convert_to_f32_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(src), dst, n);
+  cudaError_t err;
+  if (dtype == EGS_F16) err = launch_kernel(convert_to_f32_kernel<__half>, grid, 256, 0, st, true, static_cast<const __half*>(src), dst, n);
   else if (dtype == EGS_BF16)
-    convert_to_f32_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(src), dst, n);
+    err = launch_kernel(convert_to_f32_kernel<__nv_bfloat16>, grid, 256, 0, st, true, static_cast<const __nv_bfloat16*>(src), dst, n);
   else return cudaErrorInvalidValue;
   count_launch();
-  return cudaGetLastError();
+  return err;
 }
 
 }  // namespace egs

@@ -74,6 +74,8 @@ __global__ void __launch_bounds__(512) route_topk_regs_kernel(const float* __res
   const float* base = scores + static_cast<long long>(b) * T * E + e0;
   const int nthreads = EG * WPE * 32;
 
+  pdl_wait();
+  pdl_trigger();
   uint32_t key[R];
   float v[kSelChunk];
   auto fetch = [&](int t0) {
@@ -322,6 +324,8 @@ __global__ void __launch_bounds__(kCsrBatchThreads) csr_batch_count_kernel(const
   const int b = blockIdx.x, tid = threadIdx.x;
   for (int t = tid; t < T; t += kCsrBatchThreads) cnt[t] = 0;
   __syncthreads();
+  pdl_wait();
+  pdl_trigger();
   int valid = 0, bad = 0;
   for (int s = tid; s < EK; s += kCsrBatchThreads) {
     const long long t = load_index(ind, index_dtype, static_cast<long long>(b) * EK + s);
@@ -363,6 +367,8 @@ __global__ void __launch_bounds__(kCsrBatchThreads) csr_batch_place_kernel(const
   int* list = cursor + T;               // [EK] slots grouped by row, unordered inside a row
   const int b = blockIdx.x, nb = gridDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
+  pdl_wait();
+  pdl_trigger();
   int before = 0;
   for (int i = tid; i < b; i += kCsrBatchThreads) before += partial[i].w;
   before = cta_sum(before, red);
@@ -647,8 +653,7 @@ static cudaError_t launch_topk_regs(const float* scores, void* ind, int index_dt
     cudaError_t err = ensure_smem_optin<route_topk_regs_kernel<WPE, R>>(8 * kTopkMaxK * 8);
     if (err != cudaSuccess) return err;
   }
-  route_topk_regs_kernel<WPE, R><<<B * ((E + eg - 1) / eg), eg * WPE * 32, smem, st>>>(scores, ind, index_dtype, T, E, K, eg_log2, P);
-  return cudaGetLastError();
+  return launch_kernel(route_topk_regs_kernel<WPE, R>, B * ((E + eg - 1) / eg), eg * WPE * 32, smem, st, true, scores, ind, index_dtype, T, E, K, eg_log2, P);
 }
 
 cudaError_t launch_route_topk(const float* scores, void* ind, int index_dtype, int B, int T, int E, int K, cudaStream_t st) {
@@ -699,10 +704,11 @@ cudaError_t launch_index_csr(const void* ind, int index_dtype, int B, int T, int
     cudaError_t err = ensure_smem_optin<csr_batch_place_kernel>(200 * 1024);
     if (err == cudaSuccess) err = ensure_smem_optin<csr_batch_count_kernel>(200 * 1024);
     if (err != cudaSuccess) return err;
-    csr_batch_count_kernel<<<B, kCsrBatchThreads, static_cast<size_t>(T) * sizeof(int), st>>>(ind, index_dtype, T, static_cast<int>(ek), counts, partial);
-    csr_batch_place_kernel<<<B, kCsrBatchThreads, place_smem, st>>>(ind, index_dtype, T, static_cast<int>(ek), counts, partial, offsets, entries, info);
+    err = launch_kernel(csr_batch_count_kernel, B, kCsrBatchThreads, static_cast<size_t>(T) * sizeof(int), st, true, ind, index_dtype, T, static_cast<int>(ek), counts, partial);
+    if (err == cudaSuccess)
+      err = launch_kernel(csr_batch_place_kernel, B, kCsrBatchThreads, place_smem, st, true, ind, index_dtype, T, static_cast<int>(ek), counts, partial, offsets, entries, info);
     count_launch(2);
-    return cudaGetLastError();
+    return err;
   }
   cudaError_t err = launch_fill_zero(counts, static_cast<size_t>(rows) * sizeof(int), st);
   if (err == cudaSuccess) err = launch_fill_zero(info, 4 * sizeof(int), st);

@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kP16Threads, 1) tensor_pair16_persistent_kerne
   const bool run = (hdr->abort_flag == 0u);
 
   if (!run) {
-    // fall through to the common exit
+    pdl_wait();                          // (and fall through to the common exit)
   } else if (warp < kP16ProducerWarps) {
     // =========================== producers ===========================
     // The dense weight tiles come by TMA (one thread, a few box loads per stage, written in the 128-byte swizzle the

@@ -74,6 +74,7 @@ struct StrictParams {
   int splits, rows_per_split;     // D
   int tiles_m, tiles_n;           // G, S: 128-row blocks per expert; D: 128-feature blocks; columns in BN
   int units;
+  int after_own;      // see launch_kernel
 };
 
 struct Unit {
@@ -161,6 +162,7 @@ __global__ void __launch_bounds__(strict_threads(LONG), 1) strict_kernel(StrictP
     }
     mbar_init(smem_u32(&hdr->drain), 1);
     fence_mbar_init();
+    if (!p.after_own) pdl_wait();
     hdr->abort_flag = p.status.timed_out() ? 1u : 0u;
     if (smem_misaligned(smem_raw)) {
       hdr->abort_flag = 1u;
@@ -176,9 +178,9 @@ __global__ void __launch_bounds__(strict_threads(LONG), 1) strict_kernel(StrictP
   tc_fence_after();
   const uint32_t tmem_base = hdr->tmem_base;
 
-  pdl_trigger();
+  if (!p.after_own) pdl_wait();
   if (hdr->abort_flag != 0u) {
-    // fall through to the common exit
+    pdl_wait();                                          // (and fall through to the common exit)
   } else if (warp < kProdWarps) {
     // =========================== producers ===========================
     if (LONG) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kLongProdRegs));
@@ -556,6 +558,7 @@ __global__ void __launch_bounds__(strict_threads(LONG), 1) strict_kernel(StrictP
         if (++slot == raw) { slot = 0; ++round; }
       }
     }
+    pdl_trigger();                                       // (not before: a dependent's waiting CTAs would keep a kernel of another stream off this SM)
     __syncwarp();
   }
 
@@ -585,7 +588,7 @@ int strict_raw_stages(int bn, bool long_c) {
 }
 
 template <int OP, bool LONG = false>
-cudaError_t launch(const StrictParams& p, bool after_own, cudaStream_t st) {
+cudaError_t launch(const StrictParams& p, cudaStream_t st) {
   const size_t stage = kATile + static_cast<size_t>(p.BN) * 128;
   const size_t smem = kStrictHeader + xpose_bytes(LONG) + (p.raw + kLoStages) * stage;
   cudaError_t err = ensure_smem_optin<strict_kernel<OP, LONG>>(static_cast<int>(kSmemMax));
@@ -597,7 +600,7 @@ cudaError_t launch(const StrictParams& p, bool after_own, cudaStream_t st) {
     }();
     if (regs * strict_threads(true) < (kProdWarps * kLongProdRegs + epi_warps(true) * kLongEpiRegs + 4 * kLongMmaRegs) * 32) return cudaErrorInvalidConfiguration;
   }
-  err = launch_kernel(strict_kernel<OP, LONG>, p.units < kSms ? p.units : kSms, strict_threads(LONG), smem, st, after_own, p);
+  err = launch_kernel(strict_kernel<OP, LONG>, p.units < kSms ? p.units : kSms, strict_threads(LONG), smem, st, true, p);
   count_launch();
   return err;
 }
@@ -618,14 +621,15 @@ cudaError_t launch_strict_rowgemm(const RowGemmParams& r, bool scatter, cudaStre
   p.nc = r.w_layout == EGS_W_NC;
   p.index_dtype = r.index_dtype;
   p.BN = r.BN; p.raw = r.stages;
+  p.after_own = r.after_own;
   p.tiles_m = (r.M + kTileM - 1) / kTileM;
   p.tiles_n = (r.N + r.BN - 1) / r.BN;
   const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.E;
   if (units > 2147483647ll) return cudaErrorInvalidValue;
   p.units = static_cast<int>(units);
   if (long_contraction(r.C))
-    return scatter ? launch<kOpScatter, true>(p, r.after_own != 0, st) : launch<kOpGather, true>(p, r.after_own != 0, st);
-  return scatter ? launch<kOpScatter>(p, r.after_own != 0, st) : launch<kOpGather>(p, r.after_own != 0, st);
+    return scatter ? launch<kOpScatter, true>(p, st) : launch<kOpGather, true>(p, st);
+  return scatter ? launch<kOpScatter>(p, st) : launch<kOpGather>(p, st);
 }
 
 void configure_strict_dweight(DWeightParams& p) {
@@ -651,13 +655,14 @@ cudaError_t launch_strict_dweight(const DWeightParams& r, cudaStream_t st) {
   p.B = r.B; p.T = r.T; p.E = r.E; p.K = r.K; p.M = r.M; p.C = r.FG; p.N = r.FD;
   p.index_dtype = r.index_dtype; p.out_layout = r.out_layout;
   p.BN = r.BN; p.raw = r.stages;
+  p.after_own = r.after_own;
   p.splits = r.splits; p.rows_per_split = r.rows_per_split;
   p.tiles_m = (r.FG + kTileM - 1) / kTileM;
   p.tiles_n = (r.FD + r.BN - 1) / r.BN;
   const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.E * p.splits;
   if (units > 2147483647ll) return cudaErrorInvalidValue;
   p.units = static_cast<int>(units);
-  return launch<kOpDweight>(p, r.after_own != 0, st);
+  return launch<kOpDweight>(p, st);
 }
 
 }  // namespace egs

@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_rowgemm_kern
   const bool run = (hdr->abort_flag == 0u);
 
   if (!run) {
-    // fall through to the common exit
+    pdl_wait();                          // (and fall through to the common exit)
   } else if (warp < kProducerWarps) {
     // =========================== producers ===========================
     const char* A = static_cast<const char*>(p.A);
@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(PersistShape<SCATTER>::kThreads, 1) tensor_row
   const bool run = (hdr->abort_flag == 0u);
 
   if (!run) {
-    // fall through to the common exit
+    pdl_wait();                          // (and fall through to the common exit)
   } else if (warp < kPersistProducerWarps) {
     // =========================== producers ===========================
     const char* A = static_cast<const char*>(p.A);
@@ -822,7 +822,7 @@ __global__ void __launch_bounds__(kThreads, MT == 2 ? 1 : 2) tensor_dweight_kern
   const bool run = (hdr->abort_flag == 0u);
 
   if (!run) {
-    // fall through to the common exit
+    pdl_wait();                          // (and fall through to the common exit)
   } else if (warp < kProducerWarps) {
     const char* Xs = static_cast<const char*>(p.Xsrc);
     const char* Ys = static_cast<const char*>(p.Ysrc);
@@ -1115,7 +1115,7 @@ __global__ void __launch_bounds__(17 * 32, 1) tensor_fused_pair_kernel(FusedPara
   const bool run = (hdr->abort_flag == 0u);
   const int ntot = nk1 + nk2;
   if (!run) {
-    // fall through to the common exit
+    pdl_wait();                          // (and fall through to the common exit)
   } else if (warp < kProdWarps) {
     // =========================== producers ===========================
     const char* Src = static_cast<const char*>(p.Src);

@@ -374,3 +374,32 @@ def test_scatter16_one_hot_row_rounds_all_rows_once(cuda_device, B, pair):
         Out = ops.gemm_scatter(Y.to(cuda_device), W.to(cuda_device), d_ind, T)
     ref = orc.np_scatter(Y, W, Ind, T)
     assert (np.abs(Out.cpu().double().numpy() - ref) <= 2.0 ** -8 * np.abs(ref) + 1e-5 * np.abs(ref).max()).all()
+
+
+# kernels become resident under the end of the ones before them: passes issued back to back, whose buffers torch hands from one to
+# the next, have to give what they give one by one (small integers: float32 sums are exact in any order)
+@pytest.mark.parametrize("B,T,E,K,I,J,bias", [(6, 128, 8, 32, 128, 64, False), (5, 33, 3, 13, 65, 95, False), (40, 300, 9, 40, 256, 128, True)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_passes_back_to_back(cuda_device, B, T, E, K, I, J, bias, dtype):
+    w = Workload("chain", B, T, E, K, I, J, dtype, "replace", 5)
+    ins = {k: v.to(cuda_device) for k, v in workloads.make_inputs(w, integer_valued=True).items() if torch.is_tensor(v)}
+    b = torch.randint(-2, 3, (E, J), device=cuda_device).to(dtype) if bias else None
+    Ws = ins["Ws"].sign()              # a token row's few contributions stay below 256: exact in 16 bits too
+
+    def step(i, sync):
+        X, wait = ins["X"].roll(i, 1), torch.cuda.synchronize if sync else (lambda: None)
+        wait()
+        csr = ops.build_index_csr(ins["Ind"], T)
+        wait()
+        Y = ops.gather_gemm(X, ins["Wg"], ins["Ind"], bias=b)
+        wait()
+        Out = ops.gemm_scatter(Y.clamp_(-1, 1), Ws, ins["Ind"], T, csr=csr)
+        wait()
+        dW = ops.dweight(Out.clamp_(-4, 4), Y, ins["Ind"], out_layout="direct_rows")
+        wait()
+        return Y, Out, dW, csr.entries
+    alone = [step(i, True) for i in range(6)]
+    together = [step(i, False) for i in range(6)]
+    ops.check_status()
+    for x, y in zip(alone, together):
+        assert all(torch.equal(p, q) for p, q in zip(x, y))
