@@ -11,7 +11,8 @@
 
 namespace egs {
 
-bool encode_tensor_map_16bit(TensorMap3* out, const void* base, int rank, const unsigned long long* dims, const unsigned* box) {
+static bool encode_tensor_map(TensorMap3* out, const void* base, int elem_bytes, int rank, const unsigned long long* dims, const unsigned* box,
+                              CUtensorMapSwizzle swizzle) {
   using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -35,18 +36,26 @@ bool encode_tensor_map_16bit(TensorMap3* out, const void* base, int rank, const 
   if (!encode || !out || !base || rank < 2 || rank > 4) return false;
   cuuint64_t gdim[4], gstride[3];
   cuuint32_t bdim[4], estride[4] = {1u, 1u, 1u, 1u};
-  cuuint64_t pitch = 2;                                  // bytes from one element of dimension i to the next
+  cuuint64_t pitch = elem_bytes;                         // bytes from one element of dimension i to the next
   for (int i = 0; i < rank; ++i) {
     gdim[i] = dims[i];
     bdim[i] = box[i];
     pitch *= dims[i];
     if (i + 1 < rank) gstride[i] = pitch;
   }
-  // CU_TENSOR_MAP_DATA_TYPE_UINT16: the loads only move bits, so one map type serves bf16 and fp16
-  const CUresult rc = encode(reinterpret_cast<CUtensorMap*>(out), CU_TENSOR_MAP_DATA_TYPE_UINT16, static_cast<cuuint32_t>(rank), const_cast<void*>(base), gdim,
-                             gstride, bdim, estride, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+  // integer types: the loads only move bits
+  const CUresult rc = encode(reinterpret_cast<CUtensorMap*>(out), elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT32, static_cast<cuuint32_t>(rank), const_cast<void*>(base), gdim,
+                             gstride, bdim, estride, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return rc == CUDA_SUCCESS;
+}
+bool encode_tensor_map_16bit(TensorMap3* out, const void* base, int rank, const unsigned long long* dims, const unsigned* box) {
+  return encode_tensor_map(out, base, 2, rank, dims, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+bool encode_tensor_map_32bit(TensorMap3* out, const void* base, int rank, const unsigned long long* dims, const unsigned* box, int swizzle) {
+  return encode_tensor_map(out, base, 4, rank, dims, box,
+                           swizzle == kMapSwizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B
+                           : swizzle == kMapSwizzle128Base32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 static std::atomic<long long> g_launches{0};
@@ -210,7 +219,7 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
   if (tensor) {
     p.expert_fastest = pick_expert_fastest(d, scatter, dtype);
     if (dtype == EGS_F32 && precision == EGS_PREC_STRICT) {
-      configure_strict_rowgemm(p);
+      configure_strict_rowgemm(p, scatter);
       err = launch_strict_rowgemm(p, scatter, st);
     } else if (path == EGS_PATH_PAIRED) {
       const size_t smem2 = configure_tensor_gather2(p);
@@ -623,7 +632,7 @@ int egs_describe_plan(int op, const egs_dims* dims, int w_layout, int dtype, int
   p.w_layout = w_layout;
   p.expert_fastest = pick_expert_fastest(d, op == 1, dtype);
   if (dtype != EGS_F32) configure_dense16_rowgemm(p, op == 1);
-  else if (precision == EGS_PREC_STRICT) configure_strict_rowgemm(p);
+  else if (precision == EGS_PREC_STRICT) configure_strict_rowgemm(p, op == 1);
   else configure_tensor_rowgemm(p, op == 1);
   out->tile_n = p.BN; out->stages = p.stages; out->row_tiles = p.row_tiles; out->persistent = p.persistent;
   out->expert_fastest = p.expert_fastest; out->pair = p.pair; out->slot_boxes = p.slot_boxes;

@@ -80,7 +80,7 @@ struct RowGemmParams {
   int row_tiles;      // tensor path: 128-row accumulator tiles per CTA (1 or 2)
   int persistent;     // tensor path: 1 = persistent warp-specialised variant
   int pair;           // 16-bit G, S: tiles of 256 rows on pairs of SMs
-  int slot_boxes;     // 16-bit S: slot rows come as TMA boxes
+  int slot_boxes;     // 16-bit and strict float32 S: slot rows come as TMA boxes
   int after_own;      // launched behind a kernel of the same call (fill, preparation): see launch_kernel
 };
 
@@ -103,7 +103,7 @@ struct DWeightParams {
   int after_own;      // launched behind the fill of `acc`: see launch_kernel
   int swap;           // 16-bit: the slot rows' features run along the accumulator's rows
   int pair;           // 16-bit: tiles of 256 rows on pairs of SMs
-  int slot_boxes;     // 16-bit: slot rows come as TMA boxes
+  int slot_boxes;     // 16-bit and strict float32: slot rows come as TMA boxes
 };
 
 // Fused pair G -> S (tensor path only):  Mid = gather(Src) x W1[e] is stored as slot rows AND fed, without leaving the
@@ -161,7 +161,7 @@ void configure_dense16_dweight(DWeightParams& p);
 cudaError_t launch_dense16_dweight(const DWeightParams& p, int dtype, cudaStream_t st);
 
 // Strict float32 (egs_strict.cu).  Long contractions are fine up to kStrictMaxContraction (see run_rowgemm).
-void configure_strict_rowgemm(RowGemmParams& p);
+void configure_strict_rowgemm(RowGemmParams& p, bool scatter);
 cudaError_t launch_strict_rowgemm(const RowGemmParams& p, bool scatter, cudaStream_t st);
 void configure_strict_dweight(DWeightParams& p);
 cudaError_t launch_strict_dweight(const DWeightParams& p, cudaStream_t st);
@@ -183,6 +183,9 @@ struct alignas(64) TensorMap3 {
   unsigned char bytes[128];
 };
 bool encode_tensor_map_16bit(TensorMap3* out, const void* base, int rank, const unsigned long long* dims, const unsigned* box);
+// The same for 32-bit elements.  kMapSwizzle128Base32: the XOR of the 128-byte swizzle acts on 32-byte pairs of chunks with the row modulo 4.
+enum { kMapSwizzleNone = 0, kMapSwizzle128 = 1, kMapSwizzle128Base32 = 2 };
+bool encode_tensor_map_32bit(TensorMap3* out, const void* base, int rank, const unsigned long long* dims, const unsigned* box, int swizzle);
 
 // Index preparation (egs_index.cu).  All index arrays are int32 on the device.
 cudaError_t launch_route_topk(const float* scores, void* ind, int index_dtype, int B, int T, int E, int K, cudaStream_t st);

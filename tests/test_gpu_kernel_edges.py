@@ -150,6 +150,31 @@ def test_strict_float32_edges(cuda_device, B, T, E, K, I, J):
         assert orc.rel_err(got[k], truth[k]) <= 1e-5, k
 
 
+# strict float32: tiles of 32 to 128 columns and their remainders, one step, fewer steps than split groups and many, row ranges of D, slot
+# rows as boxes (K = 1, 16, 32, 128) and gathered (K = 7, 43, 101), more units than SMs.  Small integers are exact as TF32 products.
+@pytest.mark.parametrize("B,T,E,K,I,J", [(1, 8, 1, 1, 4, 4), (3, 60, 2, 43, 36, 96), (5, 90, 3, 32, 132, 68), (9, 33, 2, 7, 100, 160),
+                                         (2, 300, 3, 128, 260, 32), (5, 300, 40, 101, 64, 516), (40, 64, 33, 16, 228, 200), (130, 20, 2, 16, 64, 136)])
+def test_strict_kernels_edges(cuda_device, B, T, E, K, I, J):
+    ins = workloads.make_inputs(Workload("strict", B, T, E, K, I, J, torch.float32, "replace", 31), integer_valued=True)
+    ins["Ind"][B - 1, E - 1, K - 1] = T           # out of range: left out
+    d = {k: v.to(cuda_device) for k, v in ins.items() if torch.is_tensor(v)}
+    known = (ins["Ind"] < T).unsqueeze(-1)
+    rows = lambda A, n: torch.gather(A.double(), 1, ins["Ind"].clamp(max=T - 1).reshape(B, E * K, 1).expand(-1, -1, n)).reshape(B, E, K, n) * known
+    Y = torch.randint(-3, 4, (B, E, K, J), generator=torch.Generator().manual_seed(1)).float()
+    contributions = torch.einsum("bekj,eji->beki", Y.double(), ins["Ws"].double()) * known
+    Out = torch.zeros(B, T, I, dtype=torch.float64).scatter_add_(1, ins["Ind"].clamp(max=T - 1).reshape(B, E * K, 1).expand(-1, -1, I), contributions.reshape(B, E * K, I))
+    P = torch.einsum("bekf,bekg->efg", rows(ins["X"], I), Y.double())
+    Yd, run = Y.to(cuda_device), dict(path="tensor", precision="strict")
+    same = lambda got, want: torch.equal(got.double().cpu(), want)
+    assert same(ops.gather_gemm(d["X"], d["Wg"], d["Ind"], **run), torch.einsum("beki,eij->bekj", rows(ins["X"], I), ins["Wg"].double()))
+    assert same(ops.gather_gemm(d["X"], d["Ws"], d["Ind"], w_layout="nc", **run), torch.einsum("beki,eji->bekj", rows(ins["X"], I), ins["Ws"].double()))
+    assert same(ops.gemm_scatter(Yd, d["Ws"], d["Ind"], T, **run), Out)
+    assert same(ops.gemm_scatter(Yd, d["Ws"].transpose(1, 2).contiguous(), d["Ind"], T, w_layout="nc", **run), Out)
+    assert same(ops.dweight(d["X"], Yd, d["Ind"], **run), P)
+    assert same(ops.dweight(d["X"], Yd, d["Ind"], out_layout="direct_rows", **run), P.transpose(1, 2))
+    ops.reset_status()
+
+
 # contractions beyond 512 on the tensor cores: no further from float64 than the float32 sums of the generic kernels
 @pytest.mark.parametrize("C", [516, 1024, 2048])
 @pytest.mark.parametrize("positive", [False, True])
