@@ -28,8 +28,8 @@
 // instruction (320 a stage of G), side by side with the TMA unit; a pair's gathers take the TMA units about as long.  Everything else has to stay out of the way: a satisfied barrier
 // wait takes 150 clocks and every dependent instruction of a lone warp 5-10, so nothing on a per-stage or per-tile path divides, the
 // issuing warps run converged (see mbar_wait_all) and ids are looked up elsewhere.
-// T=1024, E=64, K=64, I=1024, J=256, bf16: B=64 G 126-138 us, S 215, D 148-165; B=512 G 950 us, dY (weights [E, N, C]) 895 = 1.23
-// PFLOP/s, S 1450, D 1050, under the power cap.
+// T=1024, E=64, K=64, I=1024, J=256, bf16: B=64 G 126-138 us, S 180 (190 before), D 148-165; B=512 G 950 us, dY (weights [E, N, C]) 895 = 1.23
+// PFLOP/s, S 1150 (1240 before its rows stayed), D 1050, under the power cap; S without the fill of its output.
 #include <algorithm>
 #include <type_traits>
 
@@ -89,8 +89,15 @@ struct DenseParams {
   int nc;             // G, S: 1 = weights [E, N, C]
   int index_dtype;
   int BN, stages;
-  int tiles_m, tiles_n, units;
-  int r1, r2;                            // radices of the unit number, see Walk
+  int tiles_m, tiles_n, units;           // row blocks, column tiles
+  int full_waves;                        // S: units of all column tiles of a row block that every CTA (pair) has, before the others
+  int group, groups_n;                   // column tiles of one of the other units, units of a row block
+  int a_slots;                           // tiles of the 128-wide operand that are kept: `stages`, or a scatter's whole row block
+  int readers;                           // read-out warps
+  Div r1, r2;                            // radices of the unit number, see Walk
+  Div stride;                            // CTAs or pairs
+  Div by_k, by_group, by_tiles;          // K, groups_n, tiles_n
+  int step_full[3], step[4];             // digits of the stride: whole row blocks, other units
   int splits, rows_per_split;            // D
   int swap;           // D: 1 = the slot rows' features are the accumulator's rows
   int lane_rows;      // D: 1 = the output's rows are the accumulator's rows
@@ -110,39 +117,74 @@ struct Cursor {
   }
 };
 
-// The units of a CTA or pair, `stride` apart.  A unit is a number in a mixed radix - column tile; row block of a group, expert, group
-// (G, S) or row block, row range, expert (D) - and is advanced by adding the stride's digits: three divisions a unit (1000 clocks and
-// more) in the lanes that feed the tensor core were a fifth of the time of a tile with eight steps.
+// The tiles of a CTA or pair.  A unit is a number in a mixed radix - column tile; row block of a group, expert, group (G, S) or row block,
+// row range, expert (D) - units go out `stride` apart and are advanced by adding the stride's digits: three divisions a unit (1000
+// clocks and more) in the lanes that feed the tensor core were a fifth of the time of a tile with eight steps.
+// A scatter whose rows may stay has units of several column tiles: all of a row block's for as many whole waves as there are, and
+// groups of them, so that the last wave is even, for the row blocks that are left.
 template <int OP, bool PAIR>
 struct Walk {
   int left;                    // units to come, this one included
   int m0, n0, e, split;        // this CTA's 128 rows, the first column of the tile, expert, row range
-  int d0, d1, d2, d3, s0, s1, s2, s3;
+  int j, tiles, tile;          // tiles of the unit before this one, its tiles, this one's place among them
+  int full, d0, d1, d2, d3;
   const DenseParams& p;
   __device__ __forceinline__ explicit Walk(const DenseParams& q) : p(q) {
-    int u = PAIR ? blockIdx.x >> 1 : blockIdx.x, s = PAIR ? gridDim.x >> 1 : gridDim.x;
-    left = u < p.units ? (p.units - u + s - 1) / s : 0;
-    d0 = u % p.tiles_n; u /= p.tiles_n; s0 = s % p.tiles_n; s /= p.tiles_n;
-    d1 = u % p.r1; u /= p.r1; s1 = s % p.r1; s /= p.r1;
-    d2 = u % p.r2; d3 = u / p.r2; s2 = s % p.r2; s3 = s / p.r2;
+    const int c = PAIR ? blockIdx.x >> 1 : blockIdx.x, s = p.stride.d;
+    full = OP == kOpScatter ? p.full_waves : 0;
+    const int rest = p.units - full * s * p.groups_n;    // (p.units counts the units as if all were of the second kind)
+    left = full + (c < rest ? p.stride.quotient(rest - c + s - 1) : 0);
+    begin(0);
+  }
+  // the first unit of the row blocks from `block` on
+  __device__ __forceinline__ void begin(int block) {
+    int u = PAIR ? blockIdx.x >> 1 : blockIdx.x;
+    d0 = OP == kOpScatter && full > 0 ? 0 : p.by_group.remainder(u);
+    u += block;
+    d1 = p.r1.remainder(u);
+    d2 = p.r2.remainder(u);
+    d3 = u;
     place();
   }
   __device__ __forceinline__ void place() {
-    n0 = d0 * p.BN;
-    const int mt = OP == kOpDweight ? d1 : d3 * p.r1 + d1;
+    const int mt = OP == kOpDweight ? d1 : d3 * p.r1.d + d1;
     e = OP == kOpDweight ? d3 : d2;
     split = OP == kOpDweight ? d2 : 0;
     m0 = PAIR ? mt * 2 * kTileM + static_cast<int>(blockIdx.x & 1) * kTileM : mt * kTileM;
+    if (OP != kOpScatter) {
+      n0 = d0 * p.BN;
+      return;
+    }
+    // A scatter's units begin at different column tiles: CTAs in flight have experts of the same token rows, and additions that
+    // meet in one part of them hold each other up.
+    const int group = full > 0 ? p.tiles_n : p.group;
+    int turn = e;
+    j = 0;
+    tiles = min(group, p.tiles_n - d0 * group);
+    tile = p.by_tiles.remainder(turn);
+    if (tile >= tiles) tile = 0;
+    n0 = (d0 * group + tile) * p.BN;
   }
   __device__ __forceinline__ void next() {
+    if (OP == kOpScatter && ++j < tiles) {
+      const bool wrap = ++tile == tiles;
+      n0 += wrap ? (1 - tiles) * p.BN : p.BN;
+      if (wrap) tile = 0;
+      return;
+    }
     --left;
-    d0 += s0;
-    d1 += s1;
-    d2 += s2;
-    d3 += s3;
-    if (d0 >= p.tiles_n) { d0 -= p.tiles_n; ++d1; }
-    if (d1 >= p.r1) { d1 -= p.r1; ++d2; }
-    if (d2 >= p.r2) { d2 -= p.r2; ++d3; }
+    const bool whole = OP == kOpScatter && full > 0;
+    if (whole && --full == 0) {
+      begin(p.full_waves * p.stride.d);
+      return;
+    }
+    d0 += whole ? 0 : p.step[0];
+    d1 += whole ? p.step_full[0] : p.step[1];
+    d2 += whole ? p.step_full[1] : p.step[2];
+    d3 += whole ? p.step_full[2] : p.step[3];
+    if (!whole && d0 >= p.groups_n) { d0 -= p.groups_n; ++d1; }
+    if (d1 >= p.r1.d) { d1 -= p.r1.d; ++d2; }
+    if (d2 >= p.r2.d) { d2 -= p.r2.d; ++d3; }
     place();
   }
   __device__ __forceinline__ int steps() const {
@@ -174,14 +216,18 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
   const bool gathers = OP != kOpScatter || !p.tma_rows;
   const bool has_cp = !PAIR && gathers;
   const bool has_tma = PAIR || OP != kOpDweight || p.tma_rows;          // (in a pair it also announces what the producers gather)
-  const int readers = gathers ? kEpiWarps : kProdWarps + kEpiWarps;     // read-out warps: producers with nothing to gather join
-  const uint32_t ring0 = epi0 + epi_bytes(!gathers);
+  const int readers = p.readers;                                        // read-out warps: producers with nothing to gather may join
+  const uint32_t ring0 = epi0 + epi_bytes(readers > kEpiWarps);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool leader = !PAIR || (blockIdx.x & 1) == 0;
   const int nseg = (p.half + 63) >> 6;
   const uint32_t n_bytes = (OP != kOpDweight && p.nc) ? static_cast<uint32_t>(p.half) * 128u : static_cast<uint32_t>(nseg) * kSeg;
   const uint32_t stage_bytes = kMTile + n_bytes;
   const int stages = p.stages;
+  // a kept tile of the 128-wide operand: with the stages, those beyond their number behind them
+  auto a_tile = [&](int slot) {
+    return ring0 + (slot < stages ? static_cast<uint32_t>(slot) * stage_bytes : static_cast<uint32_t>(stages) * stage_bytes + static_cast<uint32_t>(slot - stages) * kMTile);
+  };
   const uint32_t acc_cols = tmem_cols_for(p.BN);
   const uint32_t tmem_cols = 2u * acc_cols;
   volatile uint32_t* abort_flag = &hdr->abort_flag;
@@ -243,7 +289,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     if constexpr (OP != kOpDweight) {
       constexpr int kQuads = kTileM / kProdWarps / 4;    // G, S: 16 rows a warp
       const int steps = (p.C + kStep - 1) / kStep;
-      int t = 0;
+      int t = 0, a_slot = 0;
       for (Walk<OP, PAIR> u(p); u.left > 0 && alive; u.next(), ++t) {
         alive = mbar_wait_all(smem_u32(&hdr->ids_full[t & 1]), (t >> 1) & 1, abort_flag, p.status.word);
         if (!alive) break;
@@ -256,8 +302,10 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           wait_free();
           if (!alive) break;
           const uint32_t bar = full0 + at.slot * 8u;
-          const uint32_t dst = ring0 + static_cast<uint32_t>(at.slot) * stage_bytes + static_cast<uint32_t>(warp * kQuads) * 512u;
           at.next(stages);
+          if (OP == kOpScatter && u.j > 0) continue;     // (the rows are there; every phase of a barrier has to be waited for all the same)
+          const uint32_t dst = a_tile(a_slot) + static_cast<uint32_t>(warp * kQuads) * 512u;
+          if (++a_slot == p.a_slots) a_slot = 0;
           if (elect_one()) {
 #pragma unroll
             for (int q = 0; q < kQuads; ++q) tma_gather4_pair(dst + q * 512u, &map_rows, k * kStep, row[q][0], row[q][1], row[q][2], row[q][3], bar);
@@ -465,6 +513,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     }
     cp_async_wait_all();
   } else if (warp < kMmaWarp) {
+    if (warp >= kProdWarps || readers > kEpiWarps) {
     // =========================== read-out ===========================
     const int ew = warp >= kProdWarps ? warp - kProdWarps : warp + kEpiWarps;
     const int lg = ew & 3, share = ew >> 2, shares = readers >> 2;       // TMEM lane group (warp number mod 4), share of the column blocks
@@ -593,6 +642,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       }
       if (!released) release();
     }
+    }
   } else if (warp == kMmaWarp) {
     // =========================== MMA issuer ===========================
     if (leader) {
@@ -601,10 +651,12 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       const uint64_t b_desc = (b_mn ? make_smem_desc(0u, kSeg, 1024u) : make_smem_desc(0u, 16u, 1024u)) + (kMTile >> 4);
       const uint32_t a_adv = (a_mn ? 16u * 128u : 32u) >> 4, b_adv = (b_mn ? 16u * 128u : 32u) >> 4;
       bool ok = true;
-      int t = 0;
+      int t = 0, a_first = 0, a_next = 0;                // slots of the row block's first tile and of the tile after its last
       Cursor at;
       for (Walk<OP, PAIR> u(p); u.left > 0 && ok; u.next(), ++t) {
         const int steps = u.steps();
+        if (u.j == 0) a_first = a_next;
+        a_next = a_first;
         const uint32_t idesc =
             make_idesc(Elem<T>::fmt, a_mn ? 1u : 0u, b_mn ? 1u : 0u, PAIR ? 2 * kTileM : kTileM, static_cast<uint32_t>(u.width()));
         const int buf = t & 1;
@@ -620,10 +672,12 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           const uint32_t empty = smem_u32(&hdr->empty[at.slot]);
           // (descriptors: 14 address bits in 16-byte units; shared memory is smaller)
           const uint32_t addr = (ring0 + static_cast<uint32_t>(at.slot) * stage_bytes) >> 4;
+          const uint32_t a_addr = OP == kOpScatter ? a_tile(a_next) >> 4 : addr;
+          if (OP == kOpScatter && ++a_next == p.a_slots) a_next = 0;
           at.next(stages);
           tc_fence_after();
           if (elect_one()) {
-            umma_f16_x4<PAIR>(d, a_desc + addr, b_desc + addr, a_adv, b_adv, idesc, ks > 0 ? 1u : 0u);
+            umma_f16_x4<PAIR>(d, a_desc + a_addr, b_desc + addr, a_adv, b_adv, idesc, ks > 0 ? 1u : 0u);
             umma_done<PAIR>(empty);
             if (ks + 1 == steps) umma_done<PAIR>(smem_u32(&hdr->acc_full[buf]));
           }
@@ -649,7 +703,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int m = u.m0 + lane + 32 * i;
-          b[i] = m / p.K;
+          b[i] = p.by_k.quotient(m);
           row[i] = m < p.M ? (b[i] * p.E + u.e) * p.K + (m - b[i] * p.K) : -1;
           id[i] = (row[i] >= 0 && (dst || OP == kOpGather)) ? load_index(p.Ind, p.index_dtype, row[i]) : 0;
         }
@@ -683,7 +737,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           for (int i = 0; i < kPer; ++i) {                 // all loads first
             const int m = m0 + it + i * kIndexWarps * 32;
             const bool on = m < m_end;
-            tok[i] = on ? m / p.K : 0;
+            tok[i] = on ? p.by_k.quotient(m) : 0;
             const int s = (tok[i] * p.E + u.e) * p.K + (on ? m - tok[i] * p.K : 0);
             t[i] = load_index(p.Ind, p.index_dtype, s);
             slot_row[i] = on ? s : -1;
@@ -711,12 +765,14 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     // a pair's stage is announced by the leader, for both CTAs and for what the producers gather
     const uint32_t bytes = PAIR ? 2u * stage_bytes : (OP != kOpDweight ? n_bytes : (p.swap ? kMTile : n_bytes)) + ((OP == kOpScatter && p.tma_rows) ? kMTile : 0u);
     bool ok = true;
+    int a_slot = 0;
     Cursor at;
     for (Walk<OP, PAIR> u(p); u.left > 0 && ok; u.next()) {
       const int steps = u.steps();
       const int n0 = u.first_column();
+      const bool rows_too = OP != kOpScatter || u.j == 0;       // a scatter's row block is loaded with its first column tile
       int m = OP == kOpDweight ? u.split * p.rows_per_split : u.m0;
-      int b = m / p.K, k = m - b * p.K;                // first slot row of the step
+      int b = p.by_k.quotient(m), k = m - b * p.K;     // first slot row of the step
       for (int ks = 0, c0 = 0; ks < steps; ++ks, c0 += kStep) {
         if (at.round > 0) {
           ok = mbar_wait_all(smem_u32(&hdr->empty[at.slot]), (at.round - 1) & 1, abort_flag, p.status.word);
@@ -734,9 +790,9 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           else tma_load_4d(dst, &map_rows, x, k, u.e, b, bar);
         };
         if (elect_one()) {
-          if (leader) mbar_arrive_expect_tx(own, bytes);
+          if (leader) mbar_arrive_expect_tx(own, rows_too ? bytes : (PAIR ? 2u : 1u) * n_bytes);
           if (OP != kOpDweight) {
-            if (OP == kOpScatter && p.tma_rows) box4(base, c0);
+            if (OP == kOpScatter && p.tma_rows && rows_too) box4(a_tile(a_slot), c0);
             if (p.nc) {
               box3(base + kMTile, c0, n0);
             } else {
@@ -752,6 +808,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
               if (s < ns) box4(dst + s * kSeg, x0 + s * 64);
           }
         }
+        if (OP == kOpScatter && rows_too && ++a_slot == p.a_slots) a_slot = 0;
         if (OP == kOpDweight) {
           k += kStep;                                  // 64 rows are parts of one batch element or whole ones
           while (k >= p.K) { k -= p.K; ++b; }
@@ -810,53 +867,105 @@ bool encode_slot_rows(TensorMap3* map, const void* base, int B, int E, int K, in
 // share of the copies, and the barriers of a step take 600 (800 in a scatter that gathers its rows).  Read-out takes epi clocks a
 // column beside the next tile's main loop; the additions of a scatter share the way to the L2 with the loads, and half of the shorter
 // one shows.  Units go out in waves of one per SM or pair of SMs; a pair starts and ends 2500 clocks slower.
+//
+// The rows of a scatter whose contraction is short enough stay in a pair's shared memory for several column tiles, and the loads hide better
+// beside the additions: a fifth of the shorter one shows, not half.  (B=512 as above, S without its fill: nothing taken out 1285 us, rows
+// loaded for the first column tile only 1115, no loads 820, no additions 840.)
+struct Ring {
+  int stages = 0, a_slots = 0, readers = kEpiWarps;
+};
 struct Tile {
   int bn = 256;
+  int group = 0, full_waves = 0;         // see Walk; 0: nothing stays
   bool pair = false;
   double cost = 1e30;
 };
-Tile pick_tile(int n, int m, long long groups, int steps, double lsu0, double lsu1, double epi, bool scatter) {
+size_t column_bytes(int half, bool nc_tile) { return nc_tile ? static_cast<size_t>(half) * 128 : static_cast<size_t>((half + 63) / 64) * kSeg; }
+// stages, with room for `keep` tiles of the 128-wide operand, in what `not_ring` bytes leave
+Ring fit_ring(int half, bool nc_tile, size_t not_ring, int keep) {
+  Ring r;
+  for (int s = kMaxStages; s > 0 && r.stages == 0; --s) {
+    const int slots = s > keep ? s : keep;
+    if (not_ring + slots * kMTile + s * column_bytes(half, nc_tile) <= kSmemMax) {
+      r.stages = s;
+      r.a_slots = slots;
+    }
+  }
+  return r;
+}
+// S: sixteen read-out warps where nothing is gathered; eight where their room is wanted for the rows that stay.  At least four stages,
+// or the rows cannot stay (stages = 0).  (On single CTAs, which stage twice the columns, rows that stayed gained nothing.)
+Ring fit_scatter(int half, bool nc_tile, bool boxes, int keep) {
+  const size_t fixed = kDenseHeader + kRowTable;
+  Ring r = fit_ring(half, nc_tile, fixed + epi_bytes(boxes), keep);
+  if (boxes) r.readers = kProdWarps + kEpiWarps;
+  if (keep == 0 || r.stages >= 4) return r;
+  if (boxes) r = fit_ring(half, nc_tile, fixed + epi_bytes(false), keep);
+  if (r.stages < 4) r.stages = 0;
+  return r;
+}
+Tile pick_tile(int n, int m, long long groups, int steps, double lsu0, double lsu1, double epi, bool scatter, bool nc_tile = false) {
   Tile best;
   for (int pair = 0; pair < 2; ++pair) {
     const int rows = pair ? 2 * kTileM : kTileM, sms = pair ? kSms / 2 : kSms, unit16 = pair ? 32 : 16;
     const double per_row = pair ? 2.0 : scatter ? 2.6 : 2.4, least = scatter && lsu0 > 0.0 ? 800.0 : 600.0;
     const long long row_units = (m + rows - 1) / rows * groups;
     const int top = n < 256 ? (n + unit16 - 1) / unit16 * unit16 : 256;
+    const bool boxes = lsu0 == 0.0;
     for (int bn = top; bn >= unit16; bn -= unit16) {
       const long long tiles = (n + bn - 1) / bn;
-      const long long units = row_units * tiles, waves = (units + sms - 1) / sms;
       const int staged = pair ? bn / 2 : bn;
       double step = per_row * (128 + staged);
       if (2.0 * bn > step) step = 2.0 * bn;
       if (lsu0 + lsu1 * staged > step) step = lsu0 + lsu1 * staged;
       if (step < least) step = least;
       const double loop = steps * step, out = epi * bn;
-      const double unit = (loop > out ? loop : out) + (scatter ? 0.5 * (loop > out ? out : loop) : 0.0);
-      const double cost = waves * (unit + 1000) + out + (pair ? 2500 : 0);
-      if (cost < best.cost * (pair && !best.pair ? 0.97 : 0.98)) {
-        best.bn = bn;
-        best.pair = pair != 0;
-        best.cost = cost;
+      const bool may_stay = scatter && tiles > 1 && pair != 0 && fit_scatter(staged, nc_tile, boxes, steps).stages > 0;
+      // (units of one tile; then, where rows may stay, whole waves of row blocks and the rest in one to eight units a row block)
+      for (long long per_block = 0; per_block <= (may_stay ? std::min(tiles, 8ll) : 0ll); ++per_block) {
+        const long long group = per_block == 0 ? 1 : (tiles + per_block - 1) / per_block, full = per_block == 0 ? 0 : row_units / sms;
+        const long long units = (row_units - full * sms) * ((tiles + group - 1) / group), waves = (units + sms - 1) / sms;
+        auto tile_cost = [&](long long stay) {
+          return (loop > out ? loop : out) + (scatter ? (0.2 + 0.3 / stay) * (loop > out ? out : loop) : 0.0) + 1000;
+        };
+        const double cost = full * tiles * tile_cost(tiles) + waves * group * tile_cost(group) + out + (pair ? 2500 : 0);
+        if (cost < best.cost * (pair && !best.pair ? 0.97 : bn != best.bn ? 0.98 : 1.0)) {
+          best.bn = bn;
+          best.group = per_block == 0 ? 0 : static_cast<int>(group);
+          best.full_waves = static_cast<int>(full);
+          best.pair = pair != 0;
+          best.cost = cost;
+        }
       }
     }
   }
   return best;
 }
 
-int ring_stages(int half, bool nc_tile, uint32_t not_ring) {
-  const size_t n_bytes = nc_tile ? static_cast<size_t>(half) * 128 : static_cast<size_t>((half + 63) / 64) * kSeg;
-  const size_t s = (kSmemMax - kDenseHeader - not_ring) / (kMTile + n_bytes);
-  return static_cast<int>(s > kMaxStages ? kMaxStages : s);
+// What Walk needs to know about the grid; r1 and r2 are set.
+void plan_walk(DenseParams& p, bool pair) {
+  const int most = pair ? kSms / 2 : kSms;
+  p.stride = Div(p.full_waves == 0 && p.units < most ? p.units : most);
+  p.by_k = Div(p.K);
+  p.by_group = Div(p.groups_n);
+  p.by_tiles = Div(p.tiles_n);
+  auto digits = [&](int u, int* to) {
+    to[0] = u % p.r1.d;
+    to[1] = u / p.r1.d % p.r2.d;
+    to[2] = u / p.r1.d / p.r2.d;
+  };
+  digits(p.stride.d, p.step_full);
+  p.step[0] = p.stride.d % p.groups_n;
+  digits(p.stride.d / p.groups_n, p.step + 1);
 }
 
 template <typename T, int OP, bool PAIR>
 cudaError_t launch(const DenseParams& p, const TensorMap3& mw, const TensorMap3& mr, cudaStream_t st) {
-  const size_t n_bytes = (OP != kOpDweight && p.nc) ? static_cast<size_t>(p.half) * 128 : static_cast<size_t>((p.half + 63) / 64) * kSeg;
-  const size_t smem = kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : kRowTable) + epi_bytes(OP == kOpScatter && p.tma_rows) +
-                      p.stages * (kMTile + n_bytes);
+  const size_t smem = kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : kRowTable) + epi_bytes(p.readers > kEpiWarps) +
+                      p.a_slots * kMTile + p.stages * column_bytes(p.half, OP != kOpDweight && p.nc);
   cudaError_t err = ensure_smem_optin<dense16_kernel<T, OP, PAIR>>(static_cast<int>(kSmemMax));
   if (err != cudaSuccess) return err;
-  const int grid = PAIR ? 2 * (p.units < kSms / 2 ? p.units : kSms / 2) : (p.units < kSms ? p.units : kSms);
+  const int grid = (PAIR ? 2 : 1) * p.stride.d;
   err = launch_kernel(dense16_kernel<T, OP, PAIR>, grid, kDenseThreads, smem, st, true, p, mw, mr);
   count_launch();
   return err;
@@ -871,11 +980,15 @@ cudaError_t launch_typed(const DenseParams& p, int dtype, const TensorMap3& mw, 
 void configure_dense16_rowgemm(RowGemmParams& p, bool scatter) {
   const int steps = (p.C + kStep - 1) / kStep;
   const bool cp_rows = !scatter || !rows_fit_boxes(p.K, 128);
-  const Tile t = pick_tile(p.N, p.M, p.E, steps, cp_rows ? 340.0 : 0.0, 0.0, 16.0, scatter);
+  const bool nc = p.w_layout == EGS_W_NC;
+  const Tile t = pick_tile(p.N, p.M, p.E, steps, cp_rows ? 340.0 : 0.0, 0.0, 16.0, scatter, nc);
   p.BN = t.bn;
   p.pair = t.pair ? 1 : 0;
+  p.tile_group = t.group;
+  p.full_waves = t.full_waves;
   p.slot_boxes = scatter && !cp_rows ? 1 : 0;
-  p.stages = ring_stages(p.pair ? p.BN / 2 : p.BN, p.w_layout == EGS_W_NC, kRowTable + epi_bytes(!cp_rows));
+  const Ring r = fit_scatter(p.pair ? p.BN / 2 : p.BN, nc, p.slot_boxes != 0, t.group > 0 ? steps : 0);
+  p.stages = r.stages;
   p.row_tiles = 1;
   p.persistent = 1;
 }
@@ -892,14 +1005,18 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
   const int rows = r.pair ? 2 * kTileM : kTileM;
   p.tiles_m = (r.M + rows - 1) / rows;
   p.tiles_n = (r.N + r.BN - 1) / r.BN;
-  p.r1 = p.tiles_m;
-  p.r2 = r.E;
-  if (r.expert_fastest) {
-    p.r1 = 1;
-  }
-  const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.E;
+  p.r1 = Div(r.expert_fastest ? 1 : p.tiles_m);
+  p.r2 = Div(r.E);
+  const Ring ring = fit_scatter(p.half, p.nc != 0, r.slot_boxes != 0, r.tile_group > 0 ? (r.C + kStep - 1) / kStep : 0);
+  p.a_slots = ring.a_slots;
+  p.readers = ring.readers;
+  p.group = r.tile_group > 0 ? r.tile_group : 1;
+  p.full_waves = r.full_waves;
+  p.groups_n = (p.tiles_n + p.group - 1) / p.group;
+  const long long units = static_cast<long long>(p.tiles_m) * p.groups_n * p.E;
   if (units > 2147483647ll - kSms) return cudaErrorInvalidValue;
   p.units = static_cast<int>(units);
+  plan_walk(p, r.pair != 0);
   TensorMap3 mw{}, mr{};
   const unsigned long long inner = p.nc ? r.C : r.N, outer = p.nc ? r.N : r.C;
   const unsigned long long dims[3] = {inner, outer, static_cast<unsigned long long>(r.E)};
@@ -951,7 +1068,7 @@ void configure_dense16_dweight(DWeightParams& p) {
       }
     }
   }
-  p.stages = ring_stages(p.pair ? p.BN / 2 : p.BN, false, table_bytes(slot_cp) + epi_bytes(false));
+  p.stages = fit_ring(p.pair ? p.BN / 2 : p.BN, false, kDenseHeader + table_bytes(slot_cp) + epi_bytes(false), 0).stages;
   p.row_tiles = 1;
   p.slot_boxes = slot_cp ? 0 : 1;
 }
@@ -971,11 +1088,17 @@ cudaError_t launch_dense16_dweight(const DWeightParams& r, int dtype, cudaStream
   const int rows = r.pair ? 2 * kTileM : kTileM;
   p.tiles_m = (p.C + rows - 1) / rows;
   p.tiles_n = (p.N + r.BN - 1) / r.BN;
-  p.r1 = p.tiles_m;
-  p.r2 = p.splits;
+  p.group = 1;
+  p.full_waves = 0;
+  p.groups_n = p.tiles_n;
+  p.a_slots = p.stages;
+  p.readers = kEpiWarps;
+  p.r1 = Div(p.tiles_m);
+  p.r2 = Div(p.splits);
   const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.E * p.splits;
   if (units > 2147483647ll - kSms) return cudaErrorInvalidValue;
   p.units = static_cast<int>(units);
+  plan_walk(p, r.pair != 0);
   TensorMap3 mw{}, mr{};
   p.tma_rows = r.slot_boxes;
   if (p.tma_rows && !encode_slot_rows(&mr, r.Ysrc, r.B, r.E, r.K, r.FD, kStep)) return cudaErrorInvalidValue;

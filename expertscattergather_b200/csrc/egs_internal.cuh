@@ -56,6 +56,26 @@ struct StatusRef {
 };
 StatusRef status_ref(int32_t* status_word);
 
+// Division of 0 <= n < 2^31 by a divisor known on the host: a multiplication, an addition and a shift (Granlund and Montgomery, "Division by
+// invariant integers using multiplication").  The compiler's sequence for a divisor it does not know takes 100 clocks and more, and ten
+// of those stood one after the other at the start of every role of the persistent kernels.
+struct Div {
+  uint32_t mul = 1, shift = 0;
+  int d = 1;
+  Div() = default;
+  explicit Div(int divisor) : d(divisor) {
+    while ((1ll << shift) < divisor) ++shift;
+    mul = static_cast<uint32_t>((((1ull << shift) - static_cast<uint64_t>(divisor)) << 32) / static_cast<uint64_t>(divisor)) + 1u;
+  }
+  __device__ __forceinline__ int quotient(int n) const { return static_cast<int>((__umulhi(mul, static_cast<uint32_t>(n)) + static_cast<uint32_t>(n)) >> shift); }
+  // divides n, returns the remainder
+  __device__ __forceinline__ int remainder(int& n) const {
+    const int q = quotient(n), r = n - q * d;
+    n = q;
+    return r;
+  }
+};
+
 // ------------------------------------------------------------------------------------------------
 // parameter blocks (validated on the host: every product below fits in int32 unless typed int64)
 // ------------------------------------------------------------------------------------------------
@@ -80,6 +100,8 @@ struct RowGemmParams {
   int row_tiles;      // tensor path: 128-row accumulator tiles per CTA (1 or 2)
   int persistent;     // tensor path: 1 = persistent warp-specialised variant
   int pair;           // 16-bit G, S: tiles of 256 rows on pairs of SMs
+  int tile_group;     // 16-bit S: column tiles that a row block stays in shared memory for (0: it is loaded for each)
+  int full_waves;     // ... and waves of row blocks that stay for all of them
   int slot_boxes;     // 16-bit and strict float32 S: slot rows come as TMA boxes
   int after_own;      // launched behind a kernel of the same call (fill, preparation): see launch_kernel
 };

@@ -94,6 +94,8 @@ struct StrictParams {
   int splits, rows_per_split;     // D
   int tiles_m, tiles_n;           // G, S: 128-row blocks per expert; D: 128-feature blocks; columns in BN
   int units;
+  Div by_tiles_n, by_tiles_m, by_splits, stride, by_k;       // see Walk; stride: CTAs
+  int step[4];                    // digits of the stride
   int slot_boxes;     // S, D: slot rows come as boxes
   int after_own;      // see launch_kernel
 };
@@ -104,15 +106,15 @@ template <int OP>
 struct Walk {
   int left;                       // units to come, this one included
   int e, m0, n0, split;
-  int d0, d1, d2, d3, s0, s1, s2, s3;
+  int d0, d1, d2, d3;
   const StrictParams& p;
   __device__ __forceinline__ explicit Walk(const StrictParams& q) : p(q) {
-    int u = blockIdx.x, s = gridDim.x;
-    left = u < p.units ? (p.units - u + s - 1) / s : 0;
-    const int r2 = OP == kOpDweight ? p.splits : 1;
-    d0 = u % p.tiles_n; u /= p.tiles_n; s0 = s % p.tiles_n; s /= p.tiles_n;
-    d1 = u % p.tiles_m; u /= p.tiles_m; s1 = s % p.tiles_m; s /= p.tiles_m;
-    d2 = u % r2; d3 = u / r2; s2 = s % r2; s3 = s / r2;
+    int u = blockIdx.x;
+    left = u < p.units ? p.stride.quotient(p.units - u + p.stride.d - 1) : 0;
+    d0 = p.by_tiles_n.remainder(u);
+    d1 = p.by_tiles_m.remainder(u);
+    d2 = OP == kOpDweight ? p.by_splits.remainder(u) : 0;
+    d3 = u;
     place();
   }
   __device__ __forceinline__ void place() {
@@ -123,10 +125,10 @@ struct Walk {
   }
   __device__ __forceinline__ void next() {
     --left;
-    d0 += s0;
-    d1 += s1;
-    d2 += s2;
-    d3 += s3;
+    d0 += p.step[0];
+    d1 += p.step[1];
+    d2 += p.step[2];
+    d3 += p.step[3];
     if (d0 >= p.tiles_n) { d0 -= p.tiles_n; ++d1; }
     if (d1 >= p.tiles_m) { d1 -= p.tiles_m; ++d2; }
     if (d2 >= (OP == kOpDweight ? p.splits : 1)) { d2 -= OP == kOpDweight ? p.splits : 1; ++d3; }
@@ -266,7 +268,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(const __grid_
       if (OP == kOpScatter && p.slot_boxes) {
         const int steps = (p.C + kStepElems - 1) / kStepElems;
         for (Walk<OP> u(p); warp == 0 && u.left > 0 && alive; u.next()) {
-          const int b = u.m0 / p.K, k = u.m0 - b * p.K;
+          const int b = p.by_k.quotient(u.m0), k = u.m0 - b * p.K;
           for (int ks = 0; ks < steps; ++ks) {
             const int slot = take();
             if (!alive) break;
@@ -657,7 +659,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(const __grid_
       for (Walk<OP> u(p); (OP != kOpDweight || p.slot_boxes) && u.left > 0 && ok; u.next()) {
         const int steps = u.steps();
         const int m = OP == kOpDweight ? u.split * p.rows_per_split : 0;
-        int b = m / p.K, k = m - b * p.K;                // D: first slot row of the step
+        int b = p.by_k.quotient(m), k = m - b * p.K;     // D: first slot row of the step
         for (int ks = 0, c0 = 0; ks < steps; ++ks, c0 += kStepElems) {
           if (at.round > 0) ok = mbar_wait_all(smem_u32(&hdr->b_empty[at.slot]), (at.round - 1) & 1, abort_flag, p.status.word);
           if (!ok) break;
@@ -695,7 +697,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(const __grid_
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int m = u.m0 + lane + 32 * i;
-            b[i] = m / p.K;
+            b[i] = p.by_k.quotient(m);
             row[i] = m < p.M ? (b[i] * p.E + u.e) * p.K + (m - b[i] * p.K) : -1;
             id[i] = (row[i] >= 0 && (dst || OP == kOpGather)) ? load_index(p.Ind, p.index_dtype, row[i]) : 0;
           }
@@ -729,7 +731,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(const __grid_
             for (int i = 0; i < 2; ++i) {                // both loads first
               const int m = m0 + it + i * 64;
               const bool on = m < m_end;
-              tok[i] = on ? m / p.K : 0;
+              tok[i] = on ? p.by_k.quotient(m) : 0;
               const int s = (tok[i] * p.E + u.e) * p.K + (on ? m - tok[i] * p.K : 0);
               t[i] = load_index(p.Ind, p.index_dtype, s);
               slot_row[i] = on ? s : -1;
@@ -802,6 +804,19 @@ bool encode_rows(TensorMap3* map, const void* base, long long rows, int width, i
   return encode_tensor_map_32bit(map, base, 2, dims, box, swizzle);
 }
 
+void plan_walk(StrictParams& p) {
+  p.by_tiles_n = Div(p.tiles_n);
+  p.by_tiles_m = Div(p.tiles_m);
+  p.by_splits = Div(p.splits > 0 ? p.splits : 1);
+  p.by_k = Div(p.K);
+  p.stride = Div(p.units < kSms ? p.units : kSms);
+  int s = p.stride.d;
+  p.step[0] = s % p.tiles_n; s /= p.tiles_n;
+  p.step[1] = s % p.tiles_m; s /= p.tiles_m;
+  p.step[2] = s % p.by_splits.d;
+  p.step[3] = s / p.by_splits.d;
+}
+
 template <int OP, bool LONG = false>
 cudaError_t launch(const StrictParams& p, const TensorMap3& ma, const TensorMap3& mb, cudaStream_t st) {
   const size_t smem = strict_smem(p.BN, p.raw_a, p.raw_b);
@@ -814,7 +829,7 @@ cudaError_t launch(const StrictParams& p, const TensorMap3& ma, const TensorMap3
     }();
     if (regs * kStrictThreads < kLongRegs * 32) return cudaErrorInvalidConfiguration;
   }
-  err = launch_kernel(strict_kernel<OP, LONG>, p.units < kSms ? p.units : kSms, kStrictThreads, smem, st, true, p, ma, mb);
+  err = launch_kernel(strict_kernel<OP, LONG>, p.stride.d, kStrictThreads, smem, st, true, p, ma, mb);
   count_launch();
   return err;
 }
@@ -842,6 +857,7 @@ cudaError_t launch_strict_rowgemm(const RowGemmParams& r, bool scatter, cudaStre
   const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.E;
   if (units > 2147483647ll) return cudaErrorInvalidValue;
   p.units = static_cast<int>(units);
+  plan_walk(p);
   p.slot_boxes = r.slot_boxes;
   TensorMap3 ma{}, mb{};
   const unsigned long long inner = p.nc ? r.C : r.N, outer = p.nc ? r.N : r.C;
@@ -887,6 +903,7 @@ cudaError_t launch_strict_dweight(const DWeightParams& r, cudaStream_t st) {
   const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.E * p.splits;
   if (units > 2147483647ll) return cudaErrorInvalidValue;
   p.units = static_cast<int>(units);
+  plan_walk(p);
   p.slot_boxes = r.slot_boxes;
   TensorMap3 ma{}, mb{};
   if (!encode_rows(&ma, r.Xsrc, static_cast<long long>(r.B) * r.T, r.FG, kTileM, kMapSwizzleNone) ||

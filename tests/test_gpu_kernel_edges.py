@@ -428,3 +428,24 @@ def test_passes_back_to_back(cuda_device, B, T, E, K, I, J, bias, dtype):
     ops.check_status()
     for x, y in zip(alone, together):
         assert all(torch.equal(p, q) for p, q in zip(x, y))
+
+
+# 16-bit scatters on pairs whose rows stay for several column tiles: whole waves of row blocks and a rest, a last tile of few columns, rows
+# as boxes and gathered, as many contraction steps as stages, more (eight read-out warps), and too many to stay.  Every row of Y has eight
+# entries of +-1, so a token row's sum stays below 256: exact in 16 bits in any order.
+@pytest.mark.parametrize("B,T,E,K,N,C", [(16, 700, 60, 64, 768, 256), (16, 700, 60, 64, 1032, 192), (20, 500, 50, 96, 776, 256), (13, 600, 160, 59, 504, 136),
+                                         (6, 900, 40, 128, 1032, 512), (6, 900, 40, 128, 520, 640), (32, 300, 60, 64, 1032, 72)])
+@pytest.mark.parametrize("w_layout", ["cn", "nc"])
+def test_scatter_rows_that_stay(cuda_device, B, T, E, K, N, C, w_layout):
+    g = torch.Generator(device=cuda_device).manual_seed(N)
+    ints = lambda *s: torch.randint(-1, 2, s, generator=g, device=cuda_device)
+    Ind = torch.rand(B, E, T, generator=g, device=cuda_device).topk(K, -1).indices
+    Y = torch.zeros(B, E, K, C, device=cuda_device).scatter_(-1, torch.rand(B, E, K, C, generator=g, device=cuda_device).topk(8, -1).indices,
+                                                             ints(B, E, K, 8).float())
+    W = ints(E, C, N).float()
+    assert ops.describe_plan("S", B, T, E, K, C, N, torch.bfloat16, w_layout=w_layout)["pair"] == 1
+    Out = torch.zeros(B, T, N, device=cuda_device).scatter_add_(1, Ind.reshape(B, E * K, 1).expand(-1, -1, N),
+                                                                torch.einsum("bekc,ecn->bekn", Y, W).reshape(B, E * K, N))
+    got = ops.gemm_scatter(Y.bfloat16(), (W if w_layout == "cn" else W.transpose(1, 2).contiguous()).bfloat16(), Ind, T, w_layout=w_layout)
+    assert torch.equal(got.float(), Out)
+    ops.check_status()
