@@ -15,11 +15,30 @@ namespace {
 // several CTAs share an SM.  Results leave through shared memory for the same reason: rows are written (or added to) 32
 // consecutive elements per instruction.  Tile widths are multiples of 32 chosen on the host so that little of a tile is
 // padding: the widths that come here are mostly odd and below 128.
-// 54855 routed rows, 83 -> 29 features, float32 (gather): 15 us; 45 us with fixed 64x64x16 tiles and no prefetch.
+// Products go two at a time (fma.rn.f32x2, each rounded like fmaf: the same bits): 77880 rows 101 -> 101 82 -> 74 us, 100000 rows 127 -> 63
+// 49 -> 41 us.  (Eight rows a thread, 64 threads a CTA and a ring of three cp.async stages read shared memory less and took 84 and 49:
+// there is more to gain from CTAs in flight, whose chain is id, row, product, store.)
+// 54855 routed rows, 83 -> 29 features, float32 (gather): 13 us; 45 us with fixed 64x64x16 tiles and no prefetch.
 constexpr int NTHREADS = 128;
 constexpr int TM = 64;          // rows per CTA of the row kernel
 constexpr int TK = 32;          // contraction step
 constexpr int APITCH = TK + 4;  // floats; rows 16-byte aligned, consecutive rows 4 banks apart
+
+// two products at a time
+__device__ __forceinline__ unsigned long long pair_of(float x, float y) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void fma2(unsigned long long& c, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float4 float4_of(unsigned long long a, unsigned long long b) {
+  float4 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.z), "=f"(r.w) : "l"(b));
+  return r;
+}
 
 // ------------------------------------------------------------------------------------------------
 // G and S:  tile[m, n] = sum_c A[row_a(m), c] * W(e, c, n);   G stores it, S adds it atomically
@@ -106,7 +125,7 @@ __global__ void __launch_bounds__(NTHREADS, NJ == 4 ? 3 : 4) generic_rowgemm_ker
     }
   };
 
-  float acc[4][4 * NJ] = {};
+  unsigned long long acc[4][2 * NJ] = {};
   fetch(0);
   for (int c0 = 0; c0 < p.C; c0 += TK) {
     stage();
@@ -122,14 +141,13 @@ __global__ void __launch_bounds__(NTHREADS, NJ == 4 ? 3 : 4) generic_rowgemm_ker
       for (int q = 0; q < 4; ++q) {
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
-          const float4 b = *reinterpret_cast<const float4*>(&Bs[(kk + q) * BPITCH + 32 * j + 4 * tx]);
+          const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(&Bs[(kk + q) * BPITCH + 32 * j + 4 * tx]);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const float av = q == 0 ? a[i].x : q == 1 ? a[i].y : q == 2 ? a[i].z : a[i].w;
-            acc[i][4 * j] = fmaf(av, b.x, acc[i][4 * j]);
-            acc[i][4 * j + 1] = fmaf(av, b.y, acc[i][4 * j + 1]);
-            acc[i][4 * j + 2] = fmaf(av, b.z, acc[i][4 * j + 2]);
-            acc[i][4 * j + 3] = fmaf(av, b.w, acc[i][4 * j + 3]);
+            const unsigned long long aa = pair_of(av, av);
+            fma2(acc[i][2 * j], aa, b.x);
+            fma2(acc[i][2 * j + 1], aa, b.y);
           }
         }
       }
@@ -144,7 +162,7 @@ __global__ void __launch_bounds__(NTHREADS, NJ == 4 ? 3 : 4) generic_rowgemm_ker
 #pragma unroll
     for (int i = 0; i < 4; ++i)
       *reinterpret_cast<float4*>(&As[(ty + 16 * i) * APITCH + 4 * tx]) =
-          make_float4(acc[i][4 * j], acc[i][4 * j + 1], acc[i][4 * j + 2], acc[i][4 * j + 3]);
+          float4_of(acc[i][2 * j], acc[i][2 * j + 1]);
     __syncthreads();
     const int n = n0 + 32 * j + lane;
     if (n < p.N) {
@@ -171,6 +189,7 @@ __global__ void __launch_bounds__(NTHREADS, NJ == 4 ? 3 : 4) generic_rowgemm_ker
 // (operator D: egs/triton_kernels.py:261-356 in the reference)
 // FI, GJ: tile size in units of 32 gathered / direct features.  Thread (ty, tx) owns features f = 32 i + 2 ty + {0, 1} and
 // g = 32 j + 4 tx .. + 3.  A tile is summed over `rows_per_split` rows and added to the float32 result where there are several.
+// For up to 32 direct features (GJ = 1); wider ones: the kernel after this.
 // ------------------------------------------------------------------------------------------------
 constexpr int kRowTable = 256;   // rows whose offsets are looked up at a time
 template <typename T, int FI, int GJ>
@@ -289,6 +308,162 @@ __global__ void __launch_bounds__(NTHREADS, FI * GJ > 4 ? 3 : 4) generic_dweight
       __syncthreads();
 #pragma unroll
       for (int r = warp; r < 32; r += 4) {
+        const int f = f0 + 32 * i + (fg ? r : lane), g = g0 + 32 * j + (fg ? lane : r);
+        if (f < p.FG && g < p.FD) {
+          const float v = fg ? tile[r * XP + lane] : tile[lane * XP + r];
+          const long long off = fg ? (static_cast<long long>(e) * p.FG + f) * p.FD + g : (static_cast<long long>(e) * p.FD + g) * p.FG + f;
+          if (p.splits > 1) atomicAdd(p.acc + off, v);
+          else out[off] = from_f32<T>(v);
+        }
+      }
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
+// D for more than 32 direct features: 64 threads as 8 (ty) x 8 (tx), each with features f = 32 i + 4 ty .. + 3 and g = 32 j + 4 tx .. + 3.
+// Twice the products of a thread of the kernel above for half as many more loads from shared memory, and a ring of three stages
+// of 16 rows filled by 4-byte cp.async (16-bit types: loads, conversions and stores), of which nothing lives in registers.
+// float32, from cold caches, 77880 rows 101 x 101: 113 -> 85 us; 100000 rows 127 x 63: 60 -> 46; 327152 rows 16 x 33: 80 -> 56.  (At 83 x 29 the kernel
+// above is faster, 21 against 26 us: half the threads a tile are too few there.)
+// ------------------------------------------------------------------------------------------------
+constexpr int kWideThreads = 64, kWideStep = 16, kWideStages = 3;
+
+// one element into shared memory, zero where it is masked (`safe`: any address that may be read)
+template <typename T>
+__device__ __forceinline__ void put(float* dst, const T* src, bool on, const T* safe) {
+  if constexpr (sizeof(T) == 4) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(on ? src : safe),
+                 "r"(on ? 4u : 0u)
+                 : "memory");
+  } else {
+    *dst = on ? to_f32<T>(*src) : 0.f;
+  }
+}
+__device__ __forceinline__ void stage_done() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kWideStages - 2) : "memory"); }
+
+template <typename T, int FI, int GJ>
+__global__ void __launch_bounds__(kWideThreads, FI * GJ > 6 ? 4 : FI * GJ > 3 ? 5 : 8) generic_dweight_wide_kernel(DWeightParams p) {
+  constexpr int FP = 32 * FI + 4, GP = 32 * GJ + 4, XP = 33;
+  __shared__ __align__(16) float tile[kWideStages * kWideStep * (FP + GP)];
+  __shared__ long long row_g[kRowTable];
+  __shared__ long long row_d[kRowTable];
+  static_assert(32 * XP <= kWideStages * kWideStep * (FP + GP), "the read-out goes through the ring");
+
+  const int e = blockIdx.z / p.splits;
+  const int split = blockIdx.z - e * p.splits;
+  const int f0 = blockIdx.x * 32 * FI;
+  const int g0 = blockIdx.y * 32 * GJ;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tx = tid & 7, ty = tid >> 3;
+  pdl_wait();
+  pdl_trigger();
+  const T* __restrict__ Xs = static_cast<const T*>(p.Xsrc);
+  const T* __restrict__ Ys = static_cast<const T*>(p.Ysrc);
+
+  const int m_begin = split * p.rows_per_split;
+  const int m_end = min(p.M, m_begin + p.rows_per_split);
+  unsigned long long acc[4 * FI][2 * GJ] = {};
+  auto fetch = [&](int step) {     // of the rows in the table
+    float* F = tile + step % kWideStages * (kWideStep * (FP + GP));
+    float* G = F + kWideStep * FP;
+#pragma unroll
+    for (int k = 0; k < kWideStep / 2; ++k) {
+      const int r = warp + 2 * k;
+      const long long og = row_g[step * kWideStep + r], od = row_d[step * kWideStep + r];
+#pragma unroll
+      for (int i = 0; i < FI; ++i) {
+        const int f = f0 + 32 * i + lane;
+        put<T>(F + r * FP + 32 * i + lane, Xs + og + f, og >= 0 && f < p.FG, Ys);
+      }
+#pragma unroll
+      for (int j = 0; j < GJ; ++j) {
+        const int g = g0 + 32 * j + lane;
+        put<T>(G + r * GP + 32 * j + lane, Ys + od + g, od >= 0 && g < p.FD, Ys);
+      }
+    }
+  };
+
+  for (int mt = m_begin; mt < m_end; mt += kRowTable) {
+    __syncthreads();
+#pragma unroll
+    for (int i = tid; i < kRowTable; i += kWideThreads) {
+      const int m = mt + i;
+      long long og = -1, od = -1;
+      if (m < m_end) {
+        const int b = m / p.K, k = m - b * p.K;
+        const long long slot = (static_cast<long long>(b) * p.E + e) * p.K + k;
+        const long long t = load_index(p.Ind, p.index_dtype, slot);
+        if (t >= 0 && t < p.T) {
+          og = (static_cast<long long>(b) * p.T + t) * p.FG;
+          od = slot * p.FD;
+        } else {
+          p.status.report(EGS_STATUS_INDEX_OUT_OF_RANGE);
+        }
+      }
+      row_g[i] = og;
+      row_d[i] = od;
+    }
+    __syncthreads();
+    const int steps = (min(kRowTable, m_end - mt) + kWideStep - 1) / kWideStep;
+#pragma unroll
+    for (int s = 0; s < kWideStages - 1; ++s) {
+      if (s < steps) fetch(s);
+      stage_done();
+    }
+    for (int s = 0; s < steps; ++s) {
+      stage_wait();
+      __syncthreads();
+      if (s + kWideStages - 1 < steps) fetch(s + kWideStages - 1);
+      stage_done();
+      const float* F = tile + s % kWideStages * (kWideStep * (FP + GP)) + 4 * ty;
+      const float* G = tile + s % kWideStages * (kWideStep * (FP + GP)) + kWideStep * FP + 4 * tx;
+#pragma unroll 4
+      for (int kk = 0; kk < kWideStep; ++kk) {
+        float4 a[FI];
+        ulonglong2 b[GJ];
+#pragma unroll
+        for (int i = 0; i < FI; ++i) a[i] = *reinterpret_cast<const float4*>(F + kk * FP + 32 * i);
+#pragma unroll
+        for (int j = 0; j < GJ; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(G + kk * GP + 32 * j);
+#pragma unroll
+        for (int i = 0; i < FI; ++i)
+#pragma unroll
+          for (int j = 0; j < GJ; ++j) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const float av = u == 0 ? a[i].x : u == 1 ? a[i].y : u == 2 ? a[i].z : a[i].w;
+              const unsigned long long aa = pair_of(av, av);
+              fma2(acc[4 * i + u][2 * j], aa, b[j].x);
+              fma2(acc[4 * i + u][2 * j + 1], aa, b[j].y);
+            }
+          }
+      }
+    }
+  }
+
+  // 32 x 32 blocks through shared memory, lanes along the contiguous direction of the output
+  T* __restrict__ out = static_cast<T*>(p.out);
+  const bool fg = p.out_layout == EGS_DW_GATHERED_ROWS;
+#pragma unroll
+  for (int i = 0; i < FI; ++i)
+#pragma unroll
+    for (int j = 0; j < GJ; ++j) {
+      if (f0 + 32 * i >= p.FG || g0 + 32 * j >= p.FD) continue;
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+{
+        const float4 x = float4_of(acc[4 * i + u][2 * j], acc[4 * i + u][2 * j + 1]);
+        float* to = tile + (4 * ty + u) * XP + 4 * tx;
+        to[0] = x.x;
+        to[1] = x.y;
+        to[2] = x.z;
+        to[3] = x.w;
+      }
+      __syncthreads();
+#pragma unroll 8
+      for (int r = warp; r < 32; r += 2) {
         const int f = f0 + 32 * i + (fg ? r : lane), g = g0 + 32 * j + (fg ? lane : r);
         if (f < p.FG && g < p.FD) {
           const float v = fg ? tile[r * XP + lane] : tile[lane * XP + r];
@@ -584,13 +759,14 @@ cudaError_t launch_generic_rowgemm(const RowGemmParams& p, bool scatter, int dty
   return err;
 }
 
-// Tile over FG x FD and the split of the contraction: about four CTAs per SM, and no fewer than 64 rows in a range, below which
-// adding the partial tile costs more than multiplying it.
+// Tile over FG x FD and the split of the contraction: about four CTAs per SM (eight of 64 threads with small tiles: 108000 rows 7 x 110 54 -> 42 us,
+// but 81 -> 89 at 101 x 101), and no fewer than 64 rows in a range, below which adding the partial tile costs more than multiplying it.
 void configure_generic_dweight(DWeightParams& p) {
   p.row_tiles = width_in_32s(p.FG, 4);
   p.BN = 32 * width_in_32s(p.FD, 2);
   const long long tiles = static_cast<long long>((p.FG + 32 * p.row_tiles - 1) / (32 * p.row_tiles)) * ((p.FD + p.BN - 1) / p.BN) * p.E;
-  long long want = (4 * 148 + tiles - 1) / tiles;
+  const long long ctas = p.BN > 32 && p.row_tiles <= 2 ? 8 * 148 : 4 * 148;
+  long long want = (ctas + tiles - 1) / tiles;
   const long long most = (p.M + 63) / 64;
   if (want > most) want = most;
   if (want < 1) want = 1;
@@ -606,8 +782,8 @@ cudaError_t launch_generic_dweight(const DWeightParams& p, int dtype, cudaStream
   cudaError_t err;
 #define EGS_LAUNCH_FI(TY, FIV)                                                           \
   do {                                                                                   \
-    if (gj == 1) err = launch_kernel(generic_dweight_kernel<TY, FIV, 1>, grid, NTHREADS, 0, st, true, p);       \
-    else err = launch_kernel(generic_dweight_kernel<TY, FIV, 2>, grid, NTHREADS, 0, st, true, p);               \
+    if (gj == 1) err = launch_kernel(generic_dweight_kernel<TY, FIV, 1>, grid, NTHREADS, 0, st, true, p);           \
+    else err = launch_kernel(generic_dweight_wide_kernel<TY, FIV, 2>, grid, kWideThreads, 0, st, true, p);          \
   } while (0)
 #define EGS_LAUNCH(TY)                       \
   do {                                       \
