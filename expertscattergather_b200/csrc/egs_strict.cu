@@ -18,7 +18,7 @@
 // splits in the same sixteen warps a step took 2150 clocks: the chain copy, wait, split, fence, multiply, free ran over two lo buffers.)
 // A split takes 1400 clocks from its first wait to its arrival, hence three groups.  A step takes 1200-1300 clocks, with an accumulator
 // per step 1600: eight warps then read and add 64 KB of tensor memory a step.
-// 32768 routed rows, E = 32, I = 1024, J = 256, from cold caches: S 142 -> 99 us, D 173 -> 96, G 157 -> 129; 65536 rows, E = 32, I = 128,
+// 32768 routed rows, E = 32, I = 1024, J = 256, from cold caches: S 142 -> 99 us, D 173 -> 94, G 157 -> 127; 65536 rows, E = 32, I = 128,
 // J = 64: 29 -> 23, 31 -> 23, 29 -> 23.
 // The tensor core adds product groups into its accumulator with truncation, an error that grows with the number of steps
 // (3.3e-5 of max|ref| at a contraction of 4096).  G and S up to a contraction of 512 and D, in ranges of at most 1024 rows, stay
@@ -192,10 +192,15 @@ __device__ __forceinline__ void load_quad(uint32_t addr, int (&r)[4]) {
   asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 
-__device__ __forceinline__ void add2(uint32_t& a0, uint32_t& a1, uint32_t b0, uint32_t b1) {
-  asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\tadd.rn.f32x2 a, a, b;\n\tmov.b64 {%0, %1}, a;\n\t}"
-      : "+r"(a0), "+r"(a1)
-      : "r"(b0), "r"(b1));
+// Sums of a long contraction, two in a 64-bit register, each rounded to nearest.  (Held as single words they had to be paired and taken
+// apart again at every addition: G 127 us against 132.)
+__device__ __forceinline__ void add2(unsigned long long& sum, uint32_t x0, uint32_t x1) {
+  asm("{\n\t.reg .b64 x;\n\tmov.b64 x, {%1, %2};\n\tadd.rn.f32x2 %0, %0, x;\n\t}" : "+l"(sum) : "r"(x0), "r"(x1));
+}
+__device__ __forceinline__ unsigned long long pair_of(uint32_t x0, uint32_t x1) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(x0), "r"(x1));
+  return r;
 }
 
 // map_a: rows of A one by one (gather4) or as boxes; map_b: weights, or D's slot rows one by one or as boxes
@@ -534,7 +539,7 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(const __grid_
         __syncwarp();
       };
       if (LONG) {
-        uint32_t v[kBlocks][32];                         // the sums of this thread's row
+        unsigned long long v[kBlocks][16];               // the sums of this thread's row, in pairs
         for (int ch = 0; ch < steps; ++ch) {
           const uint32_t acc = wait_full();
           if (!alive) break;
@@ -544,14 +549,12 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(const __grid_
               uint32_t x[32];
               tmem_ld32(acc + static_cast<uint32_t>((c * kShares + share) * 32), x);
               tmem_ld_wait();
+              if (ch == 0) {
 #pragma unroll
-              for (int i = 0; i < 32; i += 2) {
-                if (ch == 0) {
-                  v[c][i] = x[i];
-                  v[c][i + 1] = x[i + 1];
-                } else {
-                  add2(v[c][i], v[c][i + 1], x[i], x[i + 1]);
-                }
+                for (int i = 0; i < 16; ++i) v[c][i] = pair_of(x[2 * i], x[2 * i + 1]);
+              } else {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) add2(v[c][i], x[2 * i], x[2 * i + 1]);
               }
             }
           }
@@ -561,8 +564,11 @@ __global__ void __launch_bounds__(kStrictThreads, 1) strict_kernel(const __grid_
 #pragma unroll
         for (int c = 0; c < kBlocks; ++c) {
           if (c * kShares + share < nblk) {
-            again_if_nan(c * kShares + share, v[c]);
-            emit(c * kShares + share, v[c]);
+            uint32_t w[32];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) asm("mov.b64 {%0, %1}, %2;" : "=r"(w[2 * i]), "=r"(w[2 * i + 1]) : "l"(v[c][i]));
+            again_if_nan(c * kShares + share, w);
+            emit(c * kShares + share, w);
           }
         }
       } else {
