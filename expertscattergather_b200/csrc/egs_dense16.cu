@@ -905,7 +905,7 @@ Ring fit_scatter(int half, bool nc_tile, bool boxes, int keep) {
   return r;
 }
 Tile pick_tile(int n, int m, long long groups, int steps, double lsu0, double lsu1, double epi, bool scatter, bool nc_tile = false) {
-  Tile best;
+  Tile best, stay;                       // units of one tile; rows that stay
   for (int pair = 0; pair < 2; ++pair) {
     const int rows = pair ? 2 * kTileM : kTileM, sms = pair ? kSms / 2 : kSms, unit16 = pair ? 32 : 16;
     const double per_row = pair ? 2.0 : scatter ? 2.6 : 2.4, least = scatter && lsu0 > 0.0 ? 800.0 : 600.0;
@@ -929,17 +929,19 @@ Tile pick_tile(int n, int m, long long groups, int steps, double lsu0, double ls
           return (loop > out ? loop : out) + (scatter ? (0.2 + 0.3 / stay) * (loop > out ? out : loop) : 0.0) + 1000;
         };
         const double cost = full * tiles * tile_cost(tiles) + waves * group * tile_cost(group) + out + (pair ? 2500 : 0);
-        if (cost < best.cost * (pair && !best.pair ? 0.97 : bn != best.bn ? 0.98 : 1.0)) {
-          best.bn = bn;
-          best.group = per_block == 0 ? 0 : static_cast<int>(group);
-          best.full_waves = static_cast<int>(full);
-          best.pair = pair != 0;
-          best.cost = cost;
+        Tile& to = per_block == 0 ? best : stay;
+        if (cost < to.cost * (pair && !to.pair ? 0.97 : bn != to.bn ? 0.98 : 1.0)) {
+          to.bn = bn;
+          to.group = per_block == 0 ? 0 : static_cast<int>(group);
+          to.full_waves = static_cast<int>(full);
+          to.pair = pair != 0;
+          to.cost = cost;
         }
       }
     }
   }
-  return best;
+  // for a gain of 5.5 % and more: where 5.2 % were expected (2048 rows an expert, 192 -> 768 features) the scatter took 45 us instead of 43
+  return stay.cost < 0.945 * best.cost ? stay : best;
 }
 
 // What Walk needs to know about the grid; r1 and r2 are set.
