@@ -664,8 +664,9 @@ __global__ void __launch_bounds__(kPrepThreads) scatter_prepare_kernel(const voi
                                                                        int limit, int* __restrict__ plan, float* __restrict__ acc,
                                                                        T* __restrict__ out, size_t n, int zero_output, StatusRef status) {
   extern __shared__ int prep_cnt[];      // without `info` and `flags`
+  if (nflags > 0) pdl_trigger();         // (the counting kernel has waited: the scatter may begin under it)
   pdl_wait();
-  pdl_trigger();
+  if (nflags == 0) pdl_trigger();
   const int tid = threadIdx.x;
   int flag = 0;
   if (info) {
