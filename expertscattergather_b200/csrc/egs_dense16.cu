@@ -122,7 +122,7 @@ struct Cursor {
 // clocks and more) in the lanes that feed the tensor core were a fifth of the time of a tile with eight steps.
 // A scatter whose rows may stay has units of several column tiles: all of a row block's for as many whole waves as there are, and
 // groups of them, so that the last wave is even, for the row blocks that are left.
-template <int OP, bool PAIR>
+template <int OP, bool PAIR, bool KEEP>
 struct Walk {
   int left;                    // units to come, this one included
   int m0, n0, e, split;        // this CTA's 128 rows, the first column of the tile, expert, row range
@@ -131,7 +131,7 @@ struct Walk {
   const DenseParams& p;
   __device__ __forceinline__ explicit Walk(const DenseParams& q) : p(q) {
     const int c = PAIR ? blockIdx.x >> 1 : blockIdx.x, s = p.stride.d;
-    full = OP == kOpScatter ? p.full_waves : 0;
+    full = KEEP ? p.full_waves : 0;
     const int rest = p.units - full * s * p.groups_n;    // (p.units counts the units as if all were of the second kind)
     left = full + (c < rest ? p.stride.quotient(rest - c + s - 1) : 0);
     begin(0);
@@ -139,7 +139,7 @@ struct Walk {
   // the first unit of the row blocks from `block` on
   __device__ __forceinline__ void begin(int block) {
     int u = PAIR ? blockIdx.x >> 1 : blockIdx.x;
-    d0 = OP == kOpScatter && full > 0 ? 0 : p.by_group.remainder(u);
+    d0 = KEEP && full > 0 ? 0 : p.by_group.remainder(u);
     u += block;
     d1 = p.r1.remainder(u);
     d2 = p.r2.remainder(u);
@@ -151,7 +151,7 @@ struct Walk {
     e = OP == kOpDweight ? d3 : d2;
     split = OP == kOpDweight ? d2 : 0;
     m0 = PAIR ? mt * 2 * kTileM + static_cast<int>(blockIdx.x & 1) * kTileM : mt * kTileM;
-    if (OP != kOpScatter) {
+    if (!KEEP) {
       n0 = d0 * p.BN;
       return;
     }
@@ -166,14 +166,14 @@ struct Walk {
     n0 = (d0 * group + tile) * p.BN;
   }
   __device__ __forceinline__ void next() {
-    if (OP == kOpScatter && ++j < tiles) {
+    if (KEEP && ++j < tiles) {
       const bool wrap = ++tile == tiles;
       n0 += wrap ? (1 - tiles) * p.BN : p.BN;
       if (wrap) tile = 0;
       return;
     }
     --left;
-    const bool whole = OP == kOpScatter && full > 0;
+    const bool whole = KEEP && full > 0;
     if (whole && --full == 0) {
       begin(p.full_waves * p.stride.d);
       return;
@@ -206,7 +206,10 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* map, int x
       : "memory");
 }
 
-template <typename T, int OP, bool PAIR>
+// KEEP: a scatter whose rows stay for several column tiles (see pick_tile).  An instance of its own: with the slots of kept rows and the
+// walk over both kinds of units in the lanes that issue loads and MMAs, scatters that keep nothing took 3-7 % longer (bf16, 64 experts
+// of 5760 rows, 128 -> 520 features: 181 us without, 193 with).
+template <typename T, int OP, bool PAIR, bool KEEP>
 __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThreads, 1) dense16_kernel(const __grid_constant__ DenseParams p, const __grid_constant__ TensorMap3 map_w,
                                                                    const __grid_constant__ TensorMap3 map_rows) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -226,7 +229,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
   const int stages = p.stages;
   // a kept tile of the 128-wide operand: with the stages, those beyond their number behind them
   auto a_tile = [&](int slot) {
-    return ring0 + (slot < stages ? static_cast<uint32_t>(slot) * stage_bytes : static_cast<uint32_t>(stages) * stage_bytes + static_cast<uint32_t>(slot - stages) * kMTile);
+    return ring0 + (!KEEP || slot < stages ? static_cast<uint32_t>(slot) * stage_bytes : static_cast<uint32_t>(stages) * stage_bytes + static_cast<uint32_t>(slot - stages) * kMTile);
   };
   const uint32_t acc_cols = tmem_cols_for(p.BN);
   const uint32_t tmem_cols = 2u * acc_cols;
@@ -290,7 +293,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       constexpr int kQuads = kTileM / kProdWarps / 4;    // G, S: 16 rows a warp
       const int steps = (p.C + kStep - 1) / kStep;
       int t = 0, a_slot = 0;
-      for (Walk<OP, PAIR> u(p); u.left > 0 && alive; u.next(), ++t) {
+      for (Walk<OP, PAIR, KEEP> u(p); u.left > 0 && alive; u.next(), ++t) {
         alive = mbar_wait_all(smem_u32(&hdr->ids_full[t & 1]), (t >> 1) & 1, abort_flag, p.status.word);
         if (!alive) break;
         int row[kQuads][4];
@@ -301,11 +304,12 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
         for (int k = 0; k < steps; ++k) {
           wait_free();
           if (!alive) break;
-          const uint32_t bar = full0 + at.slot * 8u;
+          const int slot = at.slot;
+          const uint32_t bar = full0 + slot * 8u;
           at.next(stages);
-          if (OP == kOpScatter && u.j > 0) continue;     // (the rows are there; every phase of a barrier has to be waited for all the same)
-          const uint32_t dst = a_tile(a_slot) + static_cast<uint32_t>(warp * kQuads) * 512u;
-          if (++a_slot == p.a_slots) a_slot = 0;
+          if (KEEP && u.j > 0) continue;     // (the rows are there; every phase of a barrier has to be waited for all the same)
+          const uint32_t dst = a_tile(KEEP ? a_slot : slot) + static_cast<uint32_t>(warp * kQuads) * 512u;
+          if (KEEP && ++a_slot == p.a_slots) a_slot = 0;
           if (elect_one()) {
 #pragma unroll
             for (int q = 0; q < kQuads; ++q) tma_gather4_pair(dst + q * 512u, &map_rows, k * kStep, row[q][0], row[q][1], row[q][2], row[q][3], bar);
@@ -317,7 +321,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       const uint32_t g_dst = p.swap ? kMTile : 0u, s_dst = p.swap ? 0u : kMTile;
       const int g_seg = p.swap ? nseg : 2, s_seg = p.swap ? 2 : nseg;
       int batch = 0;
-      for (Walk<OP, PAIR> u(p); u.left > 0 && alive; u.next()) {
+      for (Walk<OP, PAIR, KEEP> u(p); u.left > 0 && alive; u.next()) {
         const int steps = u.steps(), n0 = u.first_column();
         const int gx = p.swap ? n0 : u.m0, sx = p.swap ? u.m0 : n0;
         for (int k = 0; k < steps; ++k) {
@@ -376,7 +380,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       // The index warps keep the rows of two units in shared memory.  A unit's are read one step ahead, before the copies of the
       // step before it are issued: a read behind a copy waits for it.
       const uint32_t table = smem0 + kDenseHeader + static_cast<uint32_t>(r0) * 4u;
-      const int units = Walk<OP, PAIR>(p).left, steps = (p.C + kStep - 1) / kStep;
+      const int units = Walk<OP, PAIR, KEEP>(p).left, steps = (p.C + kStep - 1) / kStep;
       int row[4];
       auto read_rows = [&](int t) {
         alive = mbar_wait_all(smem_u32(&hdr->ids_full[t & 1]), (t >> 1) & 1, abort_flag, p.status.word);
@@ -444,7 +448,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           }
         };
         int batch = 0;                                                             // batches begun by this CTA
-        Walk<OP, PAIR> u(p);
+        Walk<OP, PAIR, KEEP> u(p);
         if (u.left > 0) {
           alive = mbar_wait_all(smem_u32(&hdr->ids_full[0]), 0u, abort_flag, p.status.word);
           read_ids(table);
@@ -524,7 +528,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     pdl_wait();                                          // zeros the results are added to, the scatter's plan
     const bool f32_rows = OP == kOpScatter && *p.plan != 0;
     int t = 0;
-    for (Walk<OP, PAIR> u(p); u.left > 0 && alive; u.next(), ++t) {
+    for (Walk<OP, PAIR, KEEP> u(p); u.left > 0 && alive; u.next(), ++t) {
       const int bn = min(p.BN, p.N - u.n0);              // columns of this tile (a multiple of 8)
       const int n_end = u.n0 + bn;
       int my_ro = -1;                                    // G, S: destination row of tile row lg * 32 + lane
@@ -653,9 +657,9 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       bool ok = true;
       int t = 0, a_first = 0, a_next = 0;                // slots of the row block's first tile and of the tile after its last
       Cursor at;
-      for (Walk<OP, PAIR> u(p); u.left > 0 && ok; u.next(), ++t) {
+      for (Walk<OP, PAIR, KEEP> u(p); u.left > 0 && ok; u.next(), ++t) {
         const int steps = u.steps();
-        if (u.j == 0) a_first = a_next;
+        if (KEEP && u.j == 0) a_first = a_next;
         a_next = a_first;
         const uint32_t idesc =
             make_idesc(Elem<T>::fmt, a_mn ? 1u : 0u, b_mn ? 1u : 0u, PAIR ? 2 * kTileM : kTileM, static_cast<uint32_t>(u.width()));
@@ -672,8 +676,8 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           const uint32_t empty = smem_u32(&hdr->empty[at.slot]);
           // (descriptors: 14 address bits in 16-byte units; shared memory is smaller)
           const uint32_t addr = (ring0 + static_cast<uint32_t>(at.slot) * stage_bytes) >> 4;
-          const uint32_t a_addr = OP == kOpScatter ? a_tile(a_next) >> 4 : addr;
-          if (OP == kOpScatter && ++a_next == p.a_slots) a_next = 0;
+          const uint32_t a_addr = KEEP ? a_tile(a_next) >> 4 : addr;
+          if (KEEP && ++a_next == p.a_slots) a_next = 0;
           at.next(stages);
           tc_fence_after();
           if (elect_one()) {
@@ -697,7 +701,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       unsigned long long* full = dst ? hdr->dst_full : hdr->ids_full;
       unsigned long long* empty = dst ? hdr->dst_empty : hdr->ids_empty;
       int t = 0;
-      for (Walk<OP, PAIR> u(p); (dst || gathers) && u.left > 0 && alive; u.next(), ++t) {
+      for (Walk<OP, PAIR, KEEP> u(p); (dst || gathers) && u.left > 0 && alive; u.next(), ++t) {
         int row[4], b[4];
         long long id[4];
 #pragma unroll
@@ -727,7 +731,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     } else {
       constexpr int kPer = kBatch / (kIndexWarps * 32);
       int batch = 0;
-      for (Walk<OP, PAIR> u(p); u.left > 0 && alive; u.next()) {
+      for (Walk<OP, PAIR, KEEP> u(p); u.left > 0 && alive; u.next()) {
         const int m_begin = u.split * p.rows_per_split, m_end = min(p.M, m_begin + p.rows_per_split);
         const bool report = u.m0 == 0 && u.n0 == 0;
         for (int m0 = m_begin; m0 < m_end && alive; m0 += kBatch, ++batch) {
@@ -767,10 +771,10 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     bool ok = true;
     int a_slot = 0;
     Cursor at;
-    for (Walk<OP, PAIR> u(p); u.left > 0 && ok; u.next()) {
+    for (Walk<OP, PAIR, KEEP> u(p); u.left > 0 && ok; u.next()) {
       const int steps = u.steps();
       const int n0 = u.first_column();
-      const bool rows_too = OP != kOpScatter || u.j == 0;       // a scatter's row block is loaded with its first column tile
+      const bool rows_too = !KEEP || u.j == 0;       // a scatter's row block is loaded with its first column tile
       int m = OP == kOpDweight ? u.split * p.rows_per_split : u.m0;
       int b = p.by_k.quotient(m), k = m - b * p.K;     // first slot row of the step
       for (int ks = 0, c0 = 0; ks < steps; ++ks, c0 += kStep) {
@@ -792,7 +796,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
         if (elect_one()) {
           if (leader) mbar_arrive_expect_tx(own, rows_too ? bytes : (PAIR ? 2u : 1u) * n_bytes);
           if (OP != kOpDweight) {
-            if (OP == kOpScatter && p.tma_rows && rows_too) box4(a_tile(a_slot), c0);
+            if (OP == kOpScatter && p.tma_rows && rows_too) box4(KEEP ? a_tile(a_slot) : base, c0);
             if (p.nc) {
               box3(base + kMTile, c0, n0);
             } else {
@@ -808,7 +812,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
               if (s < ns) box4(dst + s * kSeg, x0 + s * 64);
           }
         }
-        if (OP == kOpScatter && rows_too && ++a_slot == p.a_slots) a_slot = 0;
+        if (KEEP && rows_too && ++a_slot == p.a_slots) a_slot = 0;
         if (OP == kOpDweight) {
           k += kStep;                                  // 64 rows are parts of one batch element or whole ones
           while (k >= p.K) { k -= p.K; ++b; }
@@ -961,20 +965,20 @@ void plan_walk(DenseParams& p, bool pair) {
   digits(p.stride.d / p.groups_n, p.step + 1);
 }
 
-template <typename T, int OP, bool PAIR>
+template <typename T, int OP, bool PAIR, bool KEEP>
 cudaError_t launch(const DenseParams& p, const TensorMap3& mw, const TensorMap3& mr, cudaStream_t st) {
   const size_t smem = kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : kRowTable) + epi_bytes(p.readers > kEpiWarps) +
                       p.a_slots * kMTile + p.stages * column_bytes(p.half, OP != kOpDweight && p.nc);
-  cudaError_t err = ensure_smem_optin<dense16_kernel<T, OP, PAIR>>(static_cast<int>(kSmemMax));
+  cudaError_t err = ensure_smem_optin<dense16_kernel<T, OP, PAIR, KEEP>>(static_cast<int>(kSmemMax));
   if (err != cudaSuccess) return err;
   const int grid = (PAIR ? 2 : 1) * p.stride.d;
-  err = launch_kernel(dense16_kernel<T, OP, PAIR>, grid, kDenseThreads, smem, st, true, p, mw, mr);
+  err = launch_kernel(dense16_kernel<T, OP, PAIR, KEEP>, grid, kDenseThreads, smem, st, true, p, mw, mr);
   count_launch();
   return err;
 }
-template <int OP, bool PAIR>
+template <int OP, bool PAIR, bool KEEP = false>
 cudaError_t launch_typed(const DenseParams& p, int dtype, const TensorMap3& mw, const TensorMap3& mr, cudaStream_t st) {
-  return dtype == EGS_F16 ? launch<__half, OP, PAIR>(p, mw, mr, st) : launch<__nv_bfloat16, OP, PAIR>(p, mw, mr, st);
+  return dtype == EGS_F16 ? launch<__half, OP, PAIR, KEEP>(p, mw, mr, st) : launch<__nv_bfloat16, OP, PAIR, KEEP>(p, mw, mr, st);
 }
 
 }  // namespace
@@ -1030,8 +1034,9 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
       !encode_gather(&mr, r.A, scatter ? static_cast<long long>(r.M) * r.E : static_cast<long long>(r.B) * r.T, r.C))
     return cudaErrorInvalidValue;
   if (scatter)
-    return r.pair ? launch_typed<kOpScatter, true>(p, dtype, mw, mr, st)
-                  : launch_typed<kOpScatter, false>(p, dtype, mw, mr, st);
+    return !r.pair           ? launch_typed<kOpScatter, false>(p, dtype, mw, mr, st)
+           : r.tile_group > 0 ? launch_typed<kOpScatter, true, true>(p, dtype, mw, mr, st)
+                              : launch_typed<kOpScatter, true>(p, dtype, mw, mr, st);
   return r.pair ? launch_typed<kOpGather, true>(p, dtype, mw, mr, st) : launch_typed<kOpGather, false>(p, dtype, mw, mr, st);
 }
 
