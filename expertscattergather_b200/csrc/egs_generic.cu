@@ -60,9 +60,9 @@ __global__ void __launch_bounds__(NTHREADS, NJ == 4 ? 3 : 4) generic_rowgemm_ker
   const int tx = tid & 7, ty = tid >> 3;
   pdl_wait();
   pdl_trigger();
-  const T* __restrict__ A = static_cast<const T*>(p.A);
-  const T* __restrict__ W = static_cast<const T*>(p.W) + static_cast<long long>(e) * p.C * p.N;
-  T* __restrict__ Out = static_cast<T*>(p.Out);
+  const T* A = static_cast<const T*>(p.A);
+  const T* W = static_cast<const T*>(p.W) + static_cast<long long>(e) * p.C * p.N;
+  T* Out = static_cast<T*>(p.Out);
 
   if (tid < TM) {
     const int m = m0 + tid;
@@ -210,8 +210,8 @@ __global__ void __launch_bounds__(NTHREADS, FI * GJ > 4 ? 3 : 4) generic_dweight
   const int tx = tid & 7, ty = tid >> 3;
   pdl_wait();
   pdl_trigger();
-  const T* __restrict__ Xs = static_cast<const T*>(p.Xsrc);
-  const T* __restrict__ Ys = static_cast<const T*>(p.Ysrc);
+  const T* Xs = static_cast<const T*>(p.Xsrc);
+  const T* Ys = static_cast<const T*>(p.Ysrc);
 
   const int m_begin = split * p.rows_per_split;
   const int m_end = min(p.M, m_begin + p.rows_per_split);
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(NTHREADS, FI * GJ > 4 ? 3 : 4) generic_dweight
   }
 
   // 32 x 32 blocks through shared memory, lanes along the contiguous direction of the output
-  T* __restrict__ out = static_cast<T*>(p.out);
+  T* out = static_cast<T*>(p.out);
   const bool fg = p.out_layout == EGS_DW_GATHERED_ROWS;
 #pragma unroll
   for (int i = 0; i < FI; ++i)
@@ -358,8 +358,8 @@ __global__ void __launch_bounds__(kWideThreads, FI * GJ > 6 ? 4 : FI * GJ > 3 ? 
   const int tx = tid & 7, ty = tid >> 3;
   pdl_wait();
   pdl_trigger();
-  const T* __restrict__ Xs = static_cast<const T*>(p.Xsrc);
-  const T* __restrict__ Ys = static_cast<const T*>(p.Ysrc);
+  const T* Xs = static_cast<const T*>(p.Xsrc);
+  const T* Ys = static_cast<const T*>(p.Ysrc);
 
   const int m_begin = split * p.rows_per_split;
   const int m_end = min(p.M, m_begin + p.rows_per_split);
@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(kWideThreads, FI * GJ > 6 ? 4 : FI * GJ > 3 ? 
   }
 
   // 32 x 32 blocks through shared memory, lanes along the contiguous direction of the output
-  T* __restrict__ out = static_cast<T*>(p.out);
+  T* out = static_cast<T*>(p.out);
   const bool fg = p.out_layout == EGS_DW_GATHERED_ROWS;
 #pragma unroll
   for (int i = 0; i < FI; ++i)
@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(kSumThreads) expert_row_sum_kernel(const T* __
 // ------------------------------------------------------------------------------------------------
 // zero fill and fp32 -> dtype conversion
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) fill_zero_kernel(uint4* __restrict__ p16, size_t n16, unsigned char* tail,
+__global__ void __launch_bounds__(256) fill_zero_kernel(uint4* p16, size_t n16, unsigned char* tail,
                                                        size_t ntail) {
   pdl_wait();
   pdl_trigger();
@@ -592,10 +592,10 @@ __global__ void __launch_bounds__(256) fill_zero_bytes_kernel(unsigned char* p, 
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) p[i] = 0;
 }
 
-template <typename T> __device__ __forceinline__ void convert8(const float* __restrict__ src, T* __restrict__ dst);
+template <typename T> __device__ __forceinline__ void convert8(const float* src, T* dst);
 
 template <typename T>
-__global__ void __launch_bounds__(256) convert_from_f32_kernel(const float* __restrict__ src, T* __restrict__ dst,
+__global__ void __launch_bounds__(256) convert_from_f32_kernel(const float* src, T* dst,
                                                               size_t n) {
   pdl_wait();
   pdl_trigger();
@@ -608,7 +608,7 @@ __global__ void __launch_bounds__(256) convert_from_f32_kernel(const float* __re
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) convert_to_f32_kernel(const T* __restrict__ src, float* __restrict__ dst,
+__global__ void __launch_bounds__(256) convert_to_f32_kernel(const T* src, float* dst,
                                                             size_t n) {
   pdl_wait();
   pdl_trigger();
@@ -636,7 +636,7 @@ constexpr int kPrepOwnIds = 8192;
 
 // whether a token row of batch elements b0 .. b0 + nb - 1 gets more than `limit` contributions, counted by the whole CTA;
 // cnt: [min(nb * T_, kPrepCounters)]
-__device__ __forceinline__ int has_hot_row(const void* __restrict__ ind, int index_dtype, int b0, int nb, int T_, int EK, int limit, int* cnt) {
+__device__ __forceinline__ int has_hot_row(const void* ind, int index_dtype, int b0, int nb, int T_, int EK, int limit, int* cnt) {
   const int tid = threadIdx.x, nc = static_cast<int>(min(static_cast<long long>(nb) * T_, static_cast<long long>(kPrepCounters)));
   for (int t = tid; t < nc; t += kPrepThreads) cnt[t] = 0;
   __syncthreads();
@@ -648,8 +648,8 @@ __device__ __forceinline__ int has_hot_row(const void* __restrict__ ind, int ind
   return __syncthreads_or(over);         // (and the counters may be used again)
 }
 
-__global__ void __launch_bounds__(kPrepThreads) scatter_count_kernel(const void* __restrict__ ind, int index_dtype, int B, int T_, int EK,
-                                                                     int limit, int* __restrict__ flags) {
+__global__ void __launch_bounds__(kPrepThreads) scatter_count_kernel(const void* ind, int index_dtype, int B, int T_, int EK,
+                                                                     int limit, int* flags) {
   extern __shared__ int prep_cnt[];
   pdl_wait();
   pdl_trigger();
@@ -659,10 +659,10 @@ __global__ void __launch_bounds__(kPrepThreads) scatter_count_kernel(const void*
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kPrepThreads) scatter_prepare_kernel(const void* __restrict__ ind, int index_dtype, int B, int T_, int EK,
-                                                                       const int* __restrict__ info, const int* __restrict__ flags, int nflags,
-                                                                       int limit, int* __restrict__ plan, float* __restrict__ acc,
-                                                                       T* __restrict__ out, size_t n, int zero_output, StatusRef status) {
+__global__ void __launch_bounds__(kPrepThreads) scatter_prepare_kernel(const void* ind, int index_dtype, int B, int T_, int EK,
+                                                                       const int* info, const int* flags, int nflags,
+                                                                       int limit, int* plan, float* acc,
+                                                                       T* out, size_t n, int zero_output, StatusRef status) {
   extern __shared__ int prep_cnt[];      // without `info` and `flags`
   if (nflags > 0) pdl_trigger();         // (the counting kernel has waited: the scatter may begin under it)
   pdl_wait();
@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(kPrepThreads) scatter_prepare_kernel(const voi
 
 // 8 float32 values -> 8 elements of T with vector loads and one 16-byte store (T is a 16-bit type)
 template <typename T>
-__device__ __forceinline__ void convert8(const float* __restrict__ src, T* __restrict__ dst) {
+__device__ __forceinline__ void convert8(const float* src, T* dst) {
   const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
   T v[8] = {from_f32<T>(a.x), from_f32<T>(a.y), from_f32<T>(a.z), from_f32<T>(a.w),
             from_f32<T>(b.x), from_f32<T>(b.y), from_f32<T>(b.z), from_f32<T>(b.w)};
@@ -702,8 +702,8 @@ __device__ __forceinline__ void convert8(const float* __restrict__ src, T* __res
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) scatter_finish_kernel(const int* __restrict__ plan, const float* __restrict__ acc,
-                                                            T* __restrict__ out, size_t n) {
+__global__ void __launch_bounds__(256) scatter_finish_kernel(const int* plan, const float* acc,
+                                                            T* out, size_t n) {
   pdl_wait();
   pdl_trigger();
   if (!*plan) return;

@@ -58,7 +58,7 @@ __device__ __forceinline__ unsigned expert_sum(unsigned v, unsigned* red, int pa
 }
 
 template <int WPE, int R>
-__global__ void __launch_bounds__(512) route_topk_regs_kernel(const float* __restrict__ scores, void* __restrict__ ind, int index_dtype,
+__global__ void __launch_bounds__(512) route_topk_regs_kernel(const float* scores, void* ind, int index_dtype,
                                                               int T, int E, int K, int eg_log2, int P) {
   constexpr int CT = WPE * 32 * kSelChunk;   // tokens per chunk
   extern __shared__ __align__(16) unsigned char sel_smem[];
@@ -317,8 +317,8 @@ __device__ __forceinline__ int cta_sum(int v, int* red) {
   return __reduce_add_sync(0xffffffffu, s);
 }
 
-__global__ void __launch_bounds__(kCsrBatchThreads) csr_batch_count_kernel(const void* __restrict__ ind, int index_dtype, int T, int EK,
-                                                                           int* __restrict__ counts, int4* __restrict__ partial) {
+__global__ void __launch_bounds__(kCsrBatchThreads) csr_batch_count_kernel(const void* ind, int index_dtype, int T, int EK,
+                                                                           int* counts, int4* partial) {
   extern __shared__ int cnt[];          // [T]
   __shared__ int red[32];
   const int b = blockIdx.x, tid = threadIdx.x;
@@ -356,10 +356,10 @@ __global__ void __launch_bounds__(kCsrBatchThreads) csr_batch_count_kernel(const
   }
 }
 
-__global__ void __launch_bounds__(kCsrBatchThreads) csr_batch_place_kernel(const void* __restrict__ ind, int index_dtype, int T, int EK,
-                                                                           const int* __restrict__ counts, const int4* __restrict__ partial,
-                                                                           int* __restrict__ offsets, int* __restrict__ entries,
-                                                                           int* __restrict__ info) {
+__global__ void __launch_bounds__(kCsrBatchThreads) csr_batch_place_kernel(const void* ind, int index_dtype, int T, int EK,
+                                                                           const int* counts, const int4* partial,
+                                                                           int* offsets, int* entries,
+                                                                           int* info) {
   extern __shared__ int csr_smem[];
   __shared__ int red[32];
   int* start = csr_smem;                // [T + 1] first entry of every row, local

@@ -236,6 +236,8 @@ void count_launch(int n = 1);
 //     its dependent from the start, which then only waits before it touches what the fill or the preparation wrote.  A preparation
 //     behind its call's counting kernel, which has waited before it triggered, may trigger at once: the scatter's contraction then
 //     runs under the counting too (4 batch elements of 16380 ids: 115 us a pass if not, 106 so).
+//   * it takes no `__restrict__` pointers: until the wait its inputs may still be written, and loads that are promised the contrary are
+//     not bound by it.  (Row sums, which are launched normally, keep theirs.  Without them nothing got slower by more than the runs differ.)
 // Launch and set-up of a kernel so run under the end of the one before, also across calls: 1-2 us a kernel (a training pass of ten
 // kernels 151 -> 145 us, one of fourteen 253 -> 241).  The persistent kernels trigger when their last tile has been issued: triggering
 // at their start let a dependent's waiting CTAs keep a kernel of another stream off an SM (253 -> 251 us only).
