@@ -188,7 +188,7 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
     }
     if (err != cudaSuccess) return fail_cuda(err, "scatter scratch init");
   } else if (scatter && zero_output) {
-    cudaError_t err = launch_fill_zero(Out, out_bytes, st);
+    cudaError_t err = launch_fill_zero(Out, out_bytes, st, tensor);
     if (err != cudaSuccess) return fail_cuda(err, "fill_zero");
     own = true;
   }
@@ -413,7 +413,7 @@ int egs_gather_scatter_pair(const void* Src, const void* W1, const void* W2, con
 
   if (dtype == EGS_F32) {
     if (zero_output && dst_bytes > 0) {
-      cudaError_t err = launch_fill_zero(Dst, dst_bytes, st);
+      cudaError_t err = launch_fill_zero(Dst, dst_bytes, st, true);
       if (err != cudaSuccess) return fail_cuda(err, "fill_zero");
       p.after_own = 1;
     }
@@ -531,7 +531,7 @@ static int dweight_impl(const void* Xsrc, const void* Ysrc, const void* Ind, voi
       p.acc = static_cast<float*>(workspace);
     }
     if (!(out_is_zero && dtype == EGS_F32)) {
-      err = launch_fill_zero(p.acc, n_out * sizeof(float), st);
+      err = launch_fill_zero(p.acc, n_out * sizeof(float), st, tensor);
       if (err != cudaSuccess) return fail_cuda(err, "fill_zero");
       p.after_own = 1;
     }

@@ -18,6 +18,11 @@ namespace {
 // Products go two at a time (fma.rn.f32x2, each rounded like fmaf: the same bits): 77880 rows 101 -> 101 82 -> 74 us, 100000 rows 127 -> 63
 // 49 -> 41 us.  (Eight rows a thread, 64 threads a CTA and a ring of three cp.async stages read shared memory less and took 84 and 49:
 // there is more to gain from CTAs in flight, whose chain is id, row, product, store.)
+// These kernels, the fills before them and the conversions after them do not trigger their dependents: those start when they have left.
+// CTAs of which an SM holds several settle on the SMs that the kernel before them leaves first, and stay there: a scatter of 48 CTAs
+// behind its fill (float32, 200 rows of 333 to 701 features for each of 2 experts) took 34 us with triggers at the start, 27
+// without dependent launches, 23 so; the operators of a training pass at 46 rows, 1025 and 305 features, 10 experts 233, 245 and 217 (265 with
+// triggers where the results are written), at 595 rows, 139 and 187, 11 experts 154, 155 and 127.
 // 54855 routed rows, 83 -> 29 features, float32 (gather): 13 us; 45 us with fixed 64x64x16 tiles and no prefetch.
 constexpr int NTHREADS = 128;
 constexpr int TM = 64;          // rows per CTA of the row kernel
@@ -59,7 +64,6 @@ __global__ void __launch_bounds__(NTHREADS, NJ == 4 ? 3 : 4) generic_rowgemm_ker
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tx = tid & 7, ty = tid >> 3;
   pdl_wait();
-  pdl_trigger();
   const T* A = static_cast<const T*>(p.A);
   const T* W = static_cast<const T*>(p.W) + static_cast<long long>(e) * p.C * p.N;
   T* Out = static_cast<T*>(p.Out);
@@ -209,7 +213,6 @@ __global__ void __launch_bounds__(NTHREADS, FI * GJ > 4 ? 3 : 4) generic_dweight
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tx = tid & 7, ty = tid >> 3;
   pdl_wait();
-  pdl_trigger();
   const T* Xs = static_cast<const T*>(p.Xsrc);
   const T* Ys = static_cast<const T*>(p.Ysrc);
 
@@ -357,7 +360,6 @@ __global__ void __launch_bounds__(kWideThreads, FI * GJ > 6 ? 4 : FI * GJ > 3 ? 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tx = tid & 7, ty = tid >> 3;
   pdl_wait();
-  pdl_trigger();
   const T* Xs = static_cast<const T*>(p.Xsrc);
   const T* Ys = static_cast<const T*>(p.Ysrc);
 
@@ -576,18 +578,18 @@ __global__ void __launch_bounds__(kSumThreads) expert_row_sum_kernel(const T* __
 // zero fill and fp32 -> dtype conversion
 // ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) fill_zero_kernel(uint4* p16, size_t n16, unsigned char* tail,
-                                                       size_t ntail) {
+                                                       size_t ntail, int early) {
   pdl_wait();
-  pdl_trigger();
+  if (early) pdl_trigger();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   const uint4 z = make_uint4(0, 0, 0, 0);
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n16; i += stride) p16[i] = z;
   if (blockIdx.x == 0 && threadIdx.x < ntail) tail[threadIdx.x] = 0;
 }
 
-__global__ void __launch_bounds__(256) fill_zero_bytes_kernel(unsigned char* p, size_t n) {
+__global__ void __launch_bounds__(256) fill_zero_bytes_kernel(unsigned char* p, size_t n, int early) {
   pdl_wait();
-  pdl_trigger();
+  if (early) pdl_trigger();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) p[i] = 0;
 }
@@ -598,7 +600,6 @@ template <typename T>
 __global__ void __launch_bounds__(256) convert_from_f32_kernel(const float* src, T* dst,
                                                               size_t n) {
   pdl_wait();
-  pdl_trigger();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   const size_t i0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const bool vec = sizeof(T) == 2 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0;
@@ -611,7 +612,6 @@ template <typename T>
 __global__ void __launch_bounds__(256) convert_to_f32_kernel(const T* src, float* dst,
                                                             size_t n) {
   pdl_wait();
-  pdl_trigger();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
     dst[i] = to_f32<T>(src[i]);
@@ -841,16 +841,16 @@ cudaError_t launch_expert_row_sum(const void* Src, const void* Ind, int index_dt
   return err;
 }
 
-cudaError_t launch_fill_zero(void* ptr, size_t bytes, cudaStream_t st) {
+cudaError_t launch_fill_zero(void* ptr, size_t bytes, cudaStream_t st, bool early) {
   if (bytes == 0) return cudaSuccess;
   const uintptr_t a = reinterpret_cast<uintptr_t>(ptr);
   cudaError_t err;
   if (a % 16 != 0) {
-    err = launch_kernel(fill_zero_bytes_kernel, grid_for(bytes, 256), 256, 0, st, true, static_cast<unsigned char*>(ptr), bytes);
+    err = launch_kernel(fill_zero_bytes_kernel, grid_for(bytes, 256), 256, 0, st, true, static_cast<unsigned char*>(ptr), bytes, early ? 1 : 0);
   } else {
     const size_t n16 = bytes / 16, ntail = bytes % 16;
     err = launch_kernel(fill_zero_kernel, grid_for(n16, 256 * 4), 256, 0, st, true, static_cast<uint4*>(ptr), n16,
-                        static_cast<unsigned char*>(ptr) + n16 * 16, ntail);
+                        static_cast<unsigned char*>(ptr) + n16 * 16, ntail, early ? 1 : 0);
   }
   count_launch();
   return err;
