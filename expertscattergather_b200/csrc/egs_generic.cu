@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(NTHREADS, NJ == 4 ? 3 : 4) generic_rowgemm_ker
 // (operator D: egs/triton_kernels.py:261-356 in the reference)
 // FI, GJ: tile size in units of 32 gathered / direct features.  Thread (ty, tx) owns features f = 32 i + 2 ty + {0, 1} and
 // g = 32 j + 4 tx .. + 3.  A tile is summed over `rows_per_split` rows and added to the float32 result where there are several.
-// For up to 32 direct features (GJ = 1); wider ones: the kernel after this.
+// For up to 32 direct features, and for wider ones of float32 where there are few CTAs; else the kernel after this.
 // ------------------------------------------------------------------------------------------------
 constexpr int kRowTable = 256;   // rows whose offsets are looked up at a time
 template <typename T, int FI, int GJ>
@@ -324,29 +324,19 @@ __global__ void __launch_bounds__(NTHREADS, FI * GJ > 4 ? 3 : 4) generic_dweight
 
 // ------------------------------------------------------------------------------------------------
 // D for more than 32 direct features: 64 threads as 8 (ty) x 8 (tx), each with features f = 32 i + 4 ty .. + 3 and g = 32 j + 4 tx .. + 3.
-// Twice the products of a thread of the kernel above for half as many more loads from shared memory, and a ring of three stages
-// of 16 rows filled by 4-byte cp.async (16-bit types: loads, conversions and stores), of which nothing lives in registers.
-// float32, from cold caches, 77880 rows 101 x 101: 113 -> 85 us; 100000 rows 127 x 63: 60 -> 46; 327152 rows 16 x 33: 80 -> 56.  (At 83 x 29 the kernel
-// above is faster, 21 against 26 us: half the threads a tile are too few there.)
+// Twice the products of a thread of the kernel above for half as many more loads from shared memory.  Shared memory is a ring of three
+// stages of 16 rows (two: 3 % slower); the rows two steps ahead are loaded into registers before the products of a step and stored
+// behind them.  Loaded, converted and stored at once, 16-bit types waited for memory in every step: 271 us for 79200 rows 101 x 101 in bf16, where
+// the kernel above takes 185 and this one 99.  4-byte cp.async, for float32 only, took 58 us at 100000 rows 127 x 63 and 95 at 196416
+// rows 111 x 33, this one 54 and 87, the kernel above 74 and 126.
+// Two warps keep two of an SM's four schedulers busy, so a float32 grid of less than two CTAs an SM takes the kernel above: 1416 rows
+// 107 x 119 12.6 us there and 17.7 here, 3212 of 1 x 63 6.8 and 8.8; from there on this one is the faster (15048 rows 25 x 557: 38 and 26), and for
+// 16-bit types always (1584 rows 95 x 445: 21.8 and 19.4, 3807 of 39 x 55 15.4 and 13.3).
 // ------------------------------------------------------------------------------------------------
 constexpr int kWideThreads = 64, kWideStep = 16, kWideStages = 3;
 
-// one element into shared memory, zero where it is masked (`safe`: any address that may be read)
-template <typename T>
-__device__ __forceinline__ void put(float* dst, const T* src, bool on, const T* safe) {
-  if constexpr (sizeof(T) == 4) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(on ? src : safe),
-                 "r"(on ? 4u : 0u)
-                 : "memory");
-  } else {
-    *dst = on ? to_f32<T>(*src) : 0.f;
-  }
-}
-__device__ __forceinline__ void stage_done() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kWideStages - 2) : "memory"); }
-
 template <typename T, int FI, int GJ>
-__global__ void __launch_bounds__(kWideThreads, FI * GJ > 6 ? 4 : FI * GJ > 3 ? 5 : 8) generic_dweight_wide_kernel(DWeightParams p) {
+__global__ void __launch_bounds__(kWideThreads, FI > 2 ? 4 : FI > 1 ? 5 : 8) generic_dweight_wide_kernel(DWeightParams p) {
   constexpr int FP = 32 * FI + 4, GP = 32 * GJ + 4, XP = 33;
   __shared__ __align__(16) float tile[kWideStages * kWideStep * (FP + GP)];
   __shared__ long long row_g[kRowTable];
@@ -366,23 +356,35 @@ __global__ void __launch_bounds__(kWideThreads, FI * GJ > 6 ? 4 : FI * GJ > 3 ? 
   const int m_begin = split * p.rows_per_split;
   const int m_end = min(p.M, m_begin + p.rows_per_split);
   unsigned long long acc[4 * FI][2 * GJ] = {};
-  auto fetch = [&](int step) {     // of the rows in the table
-    float* F = tile + step % kWideStages * (kWideStep * (FP + GP));
-    float* G = F + kWideStep * FP;
+  constexpr int kRows = kWideStep / 2;
+  T held[kRows][FI + GJ];
+  auto load = [&](int step) {      // this thread's elements of a step of the rows in the table, zero where they are masked
 #pragma unroll
-    for (int k = 0; k < kWideStep / 2; ++k) {
-      const int r = warp + 2 * k;
-      const long long og = row_g[step * kWideStep + r], od = row_d[step * kWideStep + r];
+    for (int k = 0; k < kRows; ++k) {
+      const int r = step * kWideStep + warp + 2 * k;
+      const long long og = row_g[r], od = row_d[r];
 #pragma unroll
       for (int i = 0; i < FI; ++i) {
         const int f = f0 + 32 * i + lane;
-        put<T>(F + r * FP + 32 * i + lane, Xs + og + f, og >= 0 && f < p.FG, Ys);
+        held[k][i] = og >= 0 && f < p.FG ? Xs[og + f] : from_f32<T>(0.f);
       }
 #pragma unroll
       for (int j = 0; j < GJ; ++j) {
         const int g = g0 + 32 * j + lane;
-        put<T>(G + r * GP + 32 * j + lane, Ys + od + g, od >= 0 && g < p.FD, Ys);
+        held[k][FI + j] = od >= 0 && g < p.FD ? Ys[od + g] : from_f32<T>(0.f);
       }
+    }
+  };
+  auto store = [&](int step) {
+    float* F = tile + step % kWideStages * (kWideStep * (FP + GP));
+    float* G = F + kWideStep * FP;
+#pragma unroll
+    for (int k = 0; k < kRows; ++k) {
+      const int r = warp + 2 * k;
+#pragma unroll
+      for (int i = 0; i < FI; ++i) F[r * FP + 32 * i + lane] = to_f32<T>(held[k][i]);
+#pragma unroll
+      for (int j = 0; j < GJ; ++j) G[r * GP + 32 * j + lane] = to_f32<T>(held[k][FI + j]);
     }
   };
 
@@ -410,14 +412,15 @@ __global__ void __launch_bounds__(kWideThreads, FI * GJ > 6 ? 4 : FI * GJ > 3 ? 
     const int steps = (min(kRowTable, m_end - mt) + kWideStep - 1) / kWideStep;
 #pragma unroll
     for (int s = 0; s < kWideStages - 1; ++s) {
-      if (s < steps) fetch(s);
-      stage_done();
+      if (s < steps) {
+        load(s);
+        store(s);
+      }
     }
     for (int s = 0; s < steps; ++s) {
-      stage_wait();
+      const int ahead = s + kWideStages - 1;             // (its stage was read in the step before this one)
       __syncthreads();
-      if (s + kWideStages - 1 < steps) fetch(s + kWideStages - 1);
-      stage_done();
+      if (ahead < steps) load(ahead);
       const float* F = tile + s % kWideStages * (kWideStep * (FP + GP)) + 4 * ty;
       const float* G = tile + s % kWideStages * (kWideStep * (FP + GP)) + kWideStep * FP + 4 * tx;
 #pragma unroll 4
@@ -441,6 +444,7 @@ __global__ void __launch_bounds__(kWideThreads, FI * GJ > 6 ? 4 : FI * GJ > 3 ? 
             }
           }
       }
+      if (ahead < steps) store(ahead);
     }
   }
 
@@ -454,8 +458,7 @@ __global__ void __launch_bounds__(kWideThreads, FI * GJ > 6 ? 4 : FI * GJ > 3 ? 
       if (f0 + 32 * i >= p.FG || g0 + 32 * j >= p.FD) continue;
       __syncthreads();
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-{
+      for (int u = 0; u < 4; ++u) {
         const float4 x = float4_of(acc[4 * i + u][2 * j], acc[4 * i + u][2 * j + 1]);
         float* to = tile + (4 * ty + u) * XP + 4 * tx;
         to[0] = x.x;
@@ -777,27 +780,22 @@ void configure_generic_dweight(DWeightParams& p) {
   p.splits = static_cast<int>((p.M + rows - 1) / rows);
 }
 
+template <typename T, int FI>
+static cudaError_t launch_dweight(const DWeightParams& p, cudaStream_t st) {
+  const dim3 grid((p.FG + 32 * FI - 1) / (32 * FI), (p.FD + p.BN - 1) / p.BN, p.E * p.splits);
+  if (p.BN == 32) return launch_kernel(generic_dweight_kernel<T, FI, 1>, grid, NTHREADS, 0, st, true, p);
+  if constexpr (sizeof(T) == 4) {        // see generic_dweight_wide_kernel
+    if (static_cast<long long>(grid.x) * grid.y * grid.z < 2 * 148) return launch_kernel(generic_dweight_kernel<T, FI, 2>, grid, NTHREADS, 0, st, true, p);
+  }
+  return launch_kernel(generic_dweight_wide_kernel<T, FI, 2>, grid, kWideThreads, 0, st, true, p);
+}
+template <typename T>
+static cudaError_t launch_dweight(const DWeightParams& p, cudaStream_t st) {
+  return p.row_tiles == 1 ? launch_dweight<T, 1>(p, st) : p.row_tiles == 2 ? launch_dweight<T, 2>(p, st) : p.row_tiles == 3 ? launch_dweight<T, 3>(p, st) : launch_dweight<T, 4>(p, st);
+}
+
 cudaError_t launch_generic_dweight(const DWeightParams& p, int dtype, cudaStream_t st) {
-  const int fi = p.row_tiles, gj = p.BN / 32;
-  dim3 grid((p.FG + 32 * fi - 1) / (32 * fi), (p.FD + p.BN - 1) / p.BN, p.E * p.splits);
-  cudaError_t err;
-#define EGS_LAUNCH_FI(TY, FIV)                                                           \
-  do {                                                                                   \
-    if (gj == 1) err = launch_kernel(generic_dweight_kernel<TY, FIV, 1>, grid, NTHREADS, 0, st, true, p);           \
-    else err = launch_kernel(generic_dweight_wide_kernel<TY, FIV, 2>, grid, kWideThreads, 0, st, true, p);          \
-  } while (0)
-#define EGS_LAUNCH(TY)                       \
-  do {                                       \
-    if (fi == 1) EGS_LAUNCH_FI(TY, 1);       \
-    else if (fi == 2) EGS_LAUNCH_FI(TY, 2);  \
-    else if (fi == 3) EGS_LAUNCH_FI(TY, 3);  \
-    else EGS_LAUNCH_FI(TY, 4);               \
-  } while (0)
-  if (dtype == EGS_F32) EGS_LAUNCH(float);
-  else if (dtype == EGS_F16) EGS_LAUNCH(__half);
-  else EGS_LAUNCH(__nv_bfloat16);
-#undef EGS_LAUNCH
-#undef EGS_LAUNCH_FI
+  const cudaError_t err = dtype == EGS_F32 ? launch_dweight<float>(p, st) : dtype == EGS_F16 ? launch_dweight<__half>(p, st) : launch_dweight<__nv_bfloat16>(p, st);
   count_launch();
   return err;
 }

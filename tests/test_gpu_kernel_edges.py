@@ -449,3 +449,23 @@ def test_scatter_rows_that_stay(cuda_device, B, T, E, K, N, C, w_layout):
     got = ops.gemm_scatter(Y.bfloat16(), (W if w_layout == "cn" else W.transpose(1, 2).contiguous()).bfloat16(), Ind, T, w_layout=w_layout)
     assert torch.equal(got.float(), Out)
     ops.check_status()
+
+
+# generic weight gradients of rows that are no multiples of 16 bytes: tiles of 32 to 128 gathered features with remainders, up to 32 direct
+# features and more, grids of few CTAs and of many, one row, remainders of the 16-row steps, the 256-row tables and the row ranges.  Small
+# integers: float32 sums are exact in any order, and a 16-bit result is rounded once.
+@pytest.mark.parametrize("B,T,E,K,FG,FD", [(1, 5, 1, 1, 1, 33), (3, 40, 2, 5, 31, 65), (2, 60, 5, 17, 33, 101), (7, 50, 3, 37, 65, 35), (1, 300, 2, 257, 97, 129),
+                                           (16, 300, 40, 16, 129, 67), (5, 90, 150, 9, 63, 35), (40, 70, 30, 33, 101, 103), (9, 64, 300, 3, 3, 77),
+                                           (30, 400, 12, 90, 127, 47), (6, 30, 4, 13, 15, 31)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("out_layout", ["gathered_rows", "direct_rows"])
+def test_generic_dweight_edges(cuda_device, B, T, E, K, FG, FD, dtype, out_layout):
+    g = torch.Generator(device=cuda_device).manual_seed(FG + FD)
+    X, Y = (torch.randint(-2, 3, s, generator=g, device=cuda_device).to(dtype) for s in ((B, T, FG), (B, E, K, FD)))
+    Ind = torch.randint(0, T, (B, E, K), generator=g, device=cuda_device)
+    Ind[B - 1, E - 1, K - 1] = T                  # out of range: left out
+    known = (Ind < T).unsqueeze(-1)
+    rows = torch.gather(X.double(), 1, Ind.clamp(max=T - 1).reshape(B, E * K, 1).expand(-1, -1, FG)).reshape(B, E, K, FG) * known
+    P = torch.einsum("bekf,bekg->efg" if out_layout == "gathered_rows" else "bekf,bekg->egf", rows, Y.double())
+    assert torch.equal(ops.dweight(X, Y, Ind, out_layout=out_layout, path="generic"), P.to(dtype))
+    ops.reset_status()
