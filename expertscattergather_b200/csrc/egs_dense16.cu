@@ -873,8 +873,13 @@ bool encode_slot_rows(TensorMap3* map, const void* base, int B, int E, int K, in
 // one shows.  Units go out in waves of one per SM or pair of SMs; a pair starts and ends 2500 clocks slower.
 //
 // The rows of a scatter whose contraction is short enough stay in a pair's shared memory for several column tiles, and the loads hide better
-// beside the additions: a fifth of the shorter one shows, not half.  (B=512 as above, S without its fill: nothing taken out 1285 us, rows
-// loaded for the first column tile only 1115, no loads 820, no additions 840.)
+// beside the additions: a fifth of the shorter one shows, not half, or 0.3 of it where only four stages are left.  (B=512 as above, S
+// without its fill: nothing taken out 1285 us, rows loaded for the first column tile only 1115, no loads 820, no additions 840.)
+// They stay where the estimate gains 2 % over single CTAs, whose gathers it takes for faster than they are, and 4 % over pairs.  Both
+// forms were measured for 159 sizes (bf16, whole calls, against rows loaded for every column tile): the 134 that stay take 0.966 of
+// the time in the median, a quarter 0.77 to 0.93, ten 1.03 to 1.07 - seven of those have weights beyond 64 MB and token rows beyond the L2,
+// where 0.94 to 1.07 came out, 0.99 in the mean; of the others one would gain 6 %, three 4 %.  All together 0.960 of the time; 0.965
+// with one margin of 5.5 % and no difference for four stages, 0.955 if every size took what is faster.
 struct Ring {
   int stages = 0, a_slots = 0, readers = kEpiWarps;
 };
@@ -923,29 +928,33 @@ Tile pick_tile(int n, int m, long long groups, int steps, double lsu0, double ls
       if (2.0 * bn > step) step = 2.0 * bn;
       if (lsu0 + lsu1 * staged > step) step = lsu0 + lsu1 * staged;
       if (step < least) step = least;
-      const double loop = steps * step, out = epi * bn;
-      const bool may_stay = scatter && tiles > 1 && pair != 0 && fit_scatter(staged, nc_tile, boxes, steps).stages > 0;
-      // (units of one tile; then, where rows may stay, whole waves of row blocks and the rest in one to eight units a row block)
-      for (long long per_block = 0; per_block <= (may_stay ? std::min(tiles, 8ll) : 0ll); ++per_block) {
-        const long long group = per_block == 0 ? 1 : (tiles + per_block - 1) / per_block, full = per_block == 0 ? 0 : row_units / sms;
-        const long long units = (row_units - full * sms) * ((tiles + group - 1) / group), waves = (units + sms - 1) / sms;
-        auto tile_cost = [&](long long stay) {
-          return (loop > out ? loop : out) + (scatter ? (0.2 + 0.3 / stay) * (loop > out ? out : loop) : 0.0) + 1000;
-        };
-        const double cost = full * tiles * tile_cost(tiles) + waves * group * tile_cost(group) + out + (pair ? 2500 : 0);
-        Tile& to = per_block == 0 ? best : stay;
-        if (cost < to.cost * (pair && !to.pair ? 0.97 : bn != to.bn ? 0.98 : 1.0)) {
-          to.bn = bn;
-          to.group = per_block == 0 ? 0 : static_cast<int>(group);
-          to.full_waves = static_cast<int>(full);
-          to.pair = pair != 0;
-          to.cost = cost;
-        }
+      const double loop = steps * step, out = epi * bn, more = loop > out ? loop : out, less = scatter ? (loop > out ? out : loop) : 0.0;
+      const double ends = out + (pair ? 2500 : 0);
+      auto consider = [&](Tile& to, double cost, long long group, long long full) {
+        if (cost >= to.cost * (pair && !to.pair ? 0.97 : bn != to.bn ? 0.98 : 1.0)) return;
+        to.bn = bn;
+        to.group = static_cast<int>(group);
+        to.full_waves = static_cast<int>(full);
+        to.pair = pair != 0;
+        to.cost = cost;
+      };
+      const long long units = row_units * tiles, waves = (units + sms - 1) / sms;
+      consider(best, waves * (more + 0.5 * less + 1000) + ends, 0, 0);
+      // Rows that stay: whole waves of row blocks, and the rest in one to eight units a row block.  At best that is as if all tiles
+      // were spread evenly, which most widths need not be looked at further for.
+      if (!scatter || pair == 0 || tiles == 1 || waves * (more + 0.2 * less + 1000) + ends >= 0.98 * stay.cost) continue;
+      const Ring ring = fit_scatter(staged, nc_tile, boxes, steps);
+      if (ring.stages == 0) continue;
+      const double shown = ring.stages == 4 ? 0.3 : 0.2;
+      auto tile_cost = [&](long long kept) { return more + (shown + 0.3 / kept) * less + 1000; };
+      const long long full = row_units / sms, rest = row_units - full * sms;
+      for (long long per_block = 1; per_block <= std::min(tiles, 8ll); ++per_block) {
+        const long long group = (tiles + per_block - 1) / per_block, rest_waves = (rest * ((tiles + group - 1) / group) + sms - 1) / sms;
+        consider(stay, full * tiles * tile_cost(tiles) + rest_waves * group * tile_cost(group) + ends, group, full);
       }
     }
   }
-  // for a gain of 5.5 % and more: where 5.2 % were expected (2048 rows an expert, 192 -> 768 features) the scatter took 45 us instead of 43
-  return stay.cost < 0.945 * best.cost ? stay : best;
+  return stay.cost < (best.pair ? 0.96 : 0.98) * best.cost ? stay : best;
 }
 
 // What Walk needs to know about the grid; r1 and r2 are set.

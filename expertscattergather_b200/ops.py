@@ -15,7 +15,7 @@ import torch
 from . import _lib
 
 __all__ = ["gather_gemm", "gemm_scatter", "gather_scatter_pair", "fused_pair_eligible", "fused_pair_preferred", "dweight", "fill_zero", "side_stream", "fill_stream", "set_precision", "get_precision", "set_path", "get_path",
-           "check_status", "reset_status", "publish_status", "launch_count", "dtype_to_type_id", "tensor_path_eligible", "describe_plan", "route_topk", "build_index_csr", "compact_index", "gemm_scatter_csr", "IndexCSR"]
+           "check_status", "reset_status", "publish_status", "launch_count", "dtype_to_type_id", "tensor_path_eligible", "describe_plan", "describe_kept_rows", "route_topk", "build_index_csr", "compact_index", "gemm_scatter_csr", "IndexCSR"]
 
 _PRECISIONS = {"strict": _lib.PREC_STRICT, "fp32": _lib.PREC_STRICT, "tf32": _lib.PREC_TF32}
 _PATHS = {"auto": _lib.PATH_AUTO, "generic": _lib.PATH_GENERIC, "tensor": _lib.PATH_TENSOR,
@@ -304,6 +304,15 @@ def describe_plan(op: str, B, T, E, K, C, N, dtype, *, w_layout="cn", precision=
                                dtype_to_type_id(dtype), prec, ctypes.byref(info))
     _lib.check(rc, "egs_describe_plan")
     return {n: int(getattr(info, n)) for n, _ in _lib.PlanInfo._fields_}
+
+
+def describe_kept_rows(B, T, E, K, C, N, dtype, *, w_layout="cn") -> tuple[int, int]:
+    """(kept_tiles, full_waves) of the 16-bit scatter 'auto' runs at these sizes (see ``egs_describe_kept_rows``)."""
+    dims, kept, full = _lib.Dims(B, T, E, K, C, N), ctypes.c_int(), ctypes.c_int()
+    rc = _lib.load().egs_describe_kept_rows(ctypes.byref(dims), _lib.W_CN if w_layout == "cn" else _lib.W_NC, dtype_to_type_id(dtype),
+                                            ctypes.byref(kept), ctypes.byref(full))
+    _lib.check(rc, "egs_describe_kept_rows")
+    return kept.value, full.value
 
 
 _TORCH_INDEX = {torch.int64: _lib.I64, torch.int32: _lib.I32, torch.int16: _lib.I16}

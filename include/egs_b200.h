@@ -283,6 +283,11 @@ typedef struct egs_plan_info {
 } egs_plan_info;
 int egs_describe_plan(int op, const egs_dims* dims, int w_layout, int dtype, int precision, egs_plan_info* out);
 
+/* The column tiles for which a row block's slot rows stay in shared memory in the 16-bit scatter that EGS_PATH_AUTO runs at these sizes:
+ * *full_waves units of every CTA pair keep them for all tiles, *kept_tiles is the most that any other unit keeps them for.  Both 0 where
+ * rows are loaded for every column tile, and for anything but 16-bit tensors on the tensor cores.  (Diagnostic, like egs_describe_plan.) */
+int egs_describe_kept_rows(const egs_dims* dims, int w_layout, int dtype, int* kept_tiles, int* full_waves);
+
 /*
  * Row sums per expert:  out[e, n] = sum over (b, k) of a row of Src.  Ind given: the token row Ind[b,e,k] of Src [B,T,N] (the
  * gradient of a per-slot scatter bias); Ind NULL: the slot row of Src [B,E,K,N] (the gradient of a gather bias).  Summed in

@@ -430,24 +430,50 @@ def test_passes_back_to_back(cuda_device, B, T, E, K, I, J, bias, dtype):
         assert all(torch.equal(p, q) for p, q in zip(x, y))
 
 
-# 16-bit scatters on pairs whose rows stay for several column tiles: whole waves of row blocks and a rest, a last tile of few columns, rows
-# as boxes and gathered, as many contraction steps as stages, more (eight read-out warps), and too many to stay.  Every row of Y has eight
-# entries of +-1, so a token row's sum stays below 256: exact in 16 bits in any order.
-@pytest.mark.parametrize("B,T,E,K,N,C", [(16, 700, 60, 64, 768, 256), (16, 700, 60, 64, 1032, 192), (20, 500, 50, 96, 760, 256), (13, 600, 160, 59, 504, 136),
-                                         (6, 900, 40, 128, 1032, 512), (6, 900, 40, 128, 520, 640), (16, 300, 60, 64, 1032, 136), (8, 300, 64, 32, 1000, 320)])
+# 16-bit scatters on pairs whose rows stay for `kept` column tiles: whole waves of row blocks and a rest, a last tile of few columns, rows as
+# boxes and gathered, as many contraction steps as stages, more (eight read-out warps, the last bytes of shared memory), and too many to
+# stay.  Every row of Y has eight entries of +-1, so a token row's sum stays below 256: exact in 16 bits in any order.
+def _sparse_scatter(dev, B, T, E, K, N, C):
+    g = torch.Generator(device=dev).manual_seed(N)
+    ints = lambda *s: torch.randint(-1, 2, s, generator=g, device=dev)
+    Ind = torch.rand(B, E, T, generator=g, device=dev).topk(K, -1).indices
+    Y = torch.zeros(B, E, K, C, device=dev).scatter_(-1, torch.rand(B, E, K, C, generator=g, device=dev).topk(8, -1).indices, ints(B, E, K, 8).float())
+    return Ind, Y, ints(E, C, N).float(), ints(E, N).float(), ints(B, T, N).float()
+
+
+def _scatter_sum(Ind, rows, out):
+    B, E, K, N = rows.shape
+    return out.scatter_add_(1, Ind.reshape(B, E * K, 1).expand(-1, -1, N), rows.reshape(B, E * K, N))
+
+
+@pytest.mark.parametrize("B,T,E,K,N,C,kept,full", [(16, 700, 60, 64, 768, 256, 1, 3), (16, 700, 60, 64, 1032, 192, 2, 3), (20, 500, 50, 96, 760, 256, 2, 5),
+                                                   (13, 600, 160, 59, 504, 136, 1, 6), (6, 900, 40, 128, 1032, 512, 2, 1), (6, 900, 40, 128, 520, 640, 0, 0),
+                                                   (16, 300, 60, 64, 1032, 136, 2, 3), (8, 300, 64, 32, 1000, 320, 4, 0), (16, 300, 16, 59, 1032, 512, 5, 0),
+                                                   (48, 300, 8, 59, 1032, 512, 2, 1)])
 @pytest.mark.parametrize("w_layout", ["cn", "nc"])
-def test_scatter_rows_that_stay(cuda_device, B, T, E, K, N, C, w_layout):
-    g = torch.Generator(device=cuda_device).manual_seed(N)
-    ints = lambda *s: torch.randint(-1, 2, s, generator=g, device=cuda_device)
-    Ind = torch.rand(B, E, T, generator=g, device=cuda_device).topk(K, -1).indices
-    Y = torch.zeros(B, E, K, C, device=cuda_device).scatter_(-1, torch.rand(B, E, K, C, generator=g, device=cuda_device).topk(8, -1).indices,
-                                                             ints(B, E, K, 8).float())
-    W = ints(E, C, N).float()
+def test_scatter_rows_that_stay(cuda_device, B, T, E, K, N, C, kept, full, w_layout):
+    Ind, Y, W, _, _ = _sparse_scatter(cuda_device, B, T, E, K, N, C)
+    assert ops.describe_kept_rows(B, T, E, K, C, N, torch.bfloat16, w_layout=w_layout) == (kept, full)
     assert ops.describe_plan("S", B, T, E, K, C, N, torch.bfloat16, w_layout=w_layout)["pair"] == 1
-    Out = torch.zeros(B, T, N, device=cuda_device).scatter_add_(1, Ind.reshape(B, E * K, 1).expand(-1, -1, N),
-                                                                torch.einsum("bekc,ecn->bekn", Y, W).reshape(B, E * K, N))
+    Out = _scatter_sum(Ind, torch.einsum("bekc,ecn->bekn", Y, W), torch.zeros(B, T, N, device=cuda_device))
     got = ops.gemm_scatter(Y.bfloat16(), (W if w_layout == "cn" else W.transpose(1, 2).contiguous()).bfloat16(), Ind, T, w_layout=w_layout)
     assert torch.equal(got.float(), Out)
+    ops.check_status()
+
+
+# ... and the other forms of the operator: a bias, an output that is added to, a hot token row (float32 rows), both 16-bit types
+@pytest.mark.parametrize("B,T,E,K,N,C", [(16, 700, 60, 64, 768, 256), (20, 500, 50, 96, 760, 256), (8, 300, 64, 32, 1000, 320)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("form", ["bias", "out", "hot", "bias out hot"])
+def test_scatter_rows_that_stay_in_every_form(cuda_device, B, T, E, K, N, C, dtype, form):
+    Ind, Y, W, bias, out = _sparse_scatter(cuda_device, B, T, E, K, N, C)
+    assert ops.describe_kept_rows(B, T, E, K, C, N, dtype)[0] > 0
+    if "hot" in form:
+        Ind[:, :, 0] = 3                          # 50 contributions and more: the call sums in float32 and rounds once
+    rows = torch.einsum("bekc,ecn->bekn", Y, W) + (bias[None, :, None] if "bias" in form else 0)
+    Out = _scatter_sum(Ind, rows, out.clone() if "out" in form else torch.zeros_like(out))
+    got = ops.gemm_scatter(Y.to(dtype), W.to(dtype), Ind, T, bias=bias.to(dtype) if "bias" in form else None, out=out.to(dtype) if "out" in form else None)
+    assert torch.equal(got, Out.to(dtype))
     ops.check_status()
 
 
