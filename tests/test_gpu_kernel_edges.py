@@ -9,6 +9,7 @@ import torch
 import expertscattergather_b200 as egs
 from expertscattergather_b200 import _lib, ops, workloads
 from expertscattergather_b200.workloads import Workload
+from expertscattergather_b200.step import train_step
 from gpu_util import STEP_KEYS, gpu_step
 from oracle import egs_oracle as orc
 
@@ -151,27 +152,36 @@ def test_strict_float32_edges(cuda_device, B, T, E, K, I, J):
 
 
 # strict float32: tiles of 32 to 128 columns and their remainders, one step, fewer steps than split groups and many, row ranges of D, slot
-# rows as boxes (K = 1, 16, 32, 128) and gathered (K = 7, 43, 101), more units than SMs.  Small integers are exact as TF32 products.
+# rows as boxes (K = 1, 16, 32, 128) and gathered (K = 7, 43, 101), more units than SMs.  Small integers are exact as TF32 products; `big`: one
+# operand is multiples of 5461 up to 14 bits, whose lo parts are not zero (those of both together would meet in the product that is left
+# out), and every sum stays an integer below 2^24.
 @pytest.mark.parametrize("B,T,E,K,I,J", [(1, 8, 1, 1, 4, 4), (3, 60, 2, 43, 36, 96), (5, 90, 3, 32, 132, 68), (9, 33, 2, 7, 100, 160),
                                          (2, 300, 3, 128, 260, 32), (5, 300, 40, 101, 64, 516), (40, 64, 33, 16, 228, 200), (130, 20, 2, 16, 64, 136)])
-def test_strict_kernels_edges(cuda_device, B, T, E, K, I, J):
+@pytest.mark.parametrize("big", ["none", "rows", "columns"])
+def test_strict_kernels_edges(cuda_device, B, T, E, K, I, J, big):
     ins = workloads.make_inputs(Workload("strict", B, T, E, K, I, J, torch.float32, "replace", 31), integer_valued=True)
     ins["Ind"][B - 1, E - 1, K - 1] = T           # out of range: left out
-    d = {k: v.to(cuda_device) for k, v in ins.items() if torch.is_tensor(v)}
     known = (ins["Ind"] < T).unsqueeze(-1)
-    rows = lambda A, n: torch.gather(A.double(), 1, ins["Ind"].clamp(max=T - 1).reshape(B, E * K, 1).expand(-1, -1, n)).reshape(B, E, K, n) * known
+    slots = ins["Ind"].clamp(max=T - 1).reshape(B, E * K, 1)
+    rows = lambda A: torch.gather(A.double(), 1, slots.expand(-1, -1, A.shape[-1])).reshape(B, E, K, -1) * known
+    a, b = 5461 if big == "rows" else 1, 5461 if big == "columns" else 1
     Y = torch.randint(-3, 4, (B, E, K, J), generator=torch.Generator().manual_seed(1)).float()
-    contributions = torch.einsum("bekj,eji->beki", Y.double(), ins["Ws"].double()) * known
-    Out = torch.zeros(B, T, I, dtype=torch.float64).scatter_add_(1, ins["Ind"].clamp(max=T - 1).reshape(B, E * K, 1).expand(-1, -1, I), contributions.reshape(B, E * K, I))
-    P = torch.einsum("bekf,bekg->efg", rows(ins["X"], I), Y.double())
-    Yd, run = Y.to(cuda_device), dict(path="tensor", precision="strict")
-    same = lambda got, want: torch.equal(got.double().cpu(), want)
-    assert same(ops.gather_gemm(d["X"], d["Wg"], d["Ind"], **run), torch.einsum("beki,eij->bekj", rows(ins["X"], I), ins["Wg"].double()))
-    assert same(ops.gather_gemm(d["X"], d["Ws"], d["Ind"], w_layout="nc", **run), torch.einsum("beki,eji->bekj", rows(ins["X"], I), ins["Ws"].double()))
-    assert same(ops.gemm_scatter(Yd, d["Ws"], d["Ind"], T, **run), Out)
-    assert same(ops.gemm_scatter(Yd, d["Ws"].transpose(1, 2).contiguous(), d["Ind"], T, w_layout="nc", **run), Out)
-    assert same(ops.dweight(d["X"], Yd, d["Ind"], **run), P)
-    assert same(ops.dweight(d["X"], Yd, d["Ind"], out_layout="direct_rows", **run), P.transpose(1, 2))
+    X, Wg, Ws = ins["X"] * a, ins["Wg"] * b, ins["Ws"] * b
+    dev, run = lambda t: t.contiguous().to(cuda_device), dict(path="tensor", precision="strict")
+
+    def same(got, want):
+        assert want.abs().max() < 2 ** 24 and torch.equal(got.double().cpu(), want)
+
+    contributions = torch.einsum("bekj,eji->beki", Y.double() * a, Ws.double()) * known
+    Out = torch.zeros(B, T, I, dtype=torch.float64).scatter_add_(1, slots.expand(-1, -1, I), contributions.reshape(B, E * K, I))
+    P = torch.einsum("bekf,bekg->efg", rows(X), Y.double() * b)
+    Ind = dev(ins["Ind"])
+    same(ops.gather_gemm(dev(X), dev(Wg), Ind, **run), torch.einsum("beki,eij->bekj", rows(X), Wg.double()))
+    same(ops.gather_gemm(dev(X), dev(Ws), Ind, w_layout="nc", **run), torch.einsum("beki,eji->bekj", rows(X), Ws.double()))
+    same(ops.gemm_scatter(dev(Y * a), dev(Ws), Ind, T, **run), Out)
+    same(ops.gemm_scatter(dev(Y * a), dev(Ws.transpose(1, 2)), Ind, T, w_layout="nc", **run), Out)
+    same(ops.dweight(dev(X), dev(Y * b), Ind, **run), P)
+    same(ops.dweight(dev(X), dev(Y * b), Ind, out_layout="direct_rows", **run), P.transpose(1, 2))
     ops.reset_status()
 
 
@@ -401,33 +411,56 @@ def test_scatter16_one_hot_row_rounds_all_rows_once(cuda_device, B, pair):
     assert (np.abs(Out.cpu().double().numpy() - ref) <= 2.0 ** -8 * np.abs(ref) + 1e-5 * np.abs(ref).max()).all()
 
 
-# kernels become resident under the end of the ones before them: passes issued back to back, whose buffers torch hands from one to
-# the next, have to give what they give one by one (small integers: float32 sums are exact in any order)
-@pytest.mark.parametrize("B,T,E,K,I,J,bias", [(6, 128, 8, 32, 128, 64, False), (5, 33, 3, 13, 65, 95, False), (40, 300, 9, 40, 256, 128, True)])
+# kernels become resident under the end of the ones before them: operators issued back to back, with nothing of torch between them, have to
+# give what they give one by one.  Each reads what the one before it has just written, or writes what it has just read: every family of
+# kernels, with and without prepared indices, more than one wave of tiles, the helper stream's fork and join.  A column of the weights has one
+# entry of +-1, so that all values are small integers: the same bits in any order, also in 16 bits.
+@pytest.mark.parametrize("B,T,E,K,I,J", [(6, 128, 8, 32, 128, 64), (5, 33, 3, 13, 65, 95), (40, 300, 9, 40, 256, 128), (64, 256, 32, 16, 128, 64),
+                                         (32, 512, 32, 32, 768, 192), (9, 200, 12, 43, 520, 72), (30, 90, 7, 20, 129, 121)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-def test_passes_back_to_back(cuda_device, B, T, E, K, I, J, bias, dtype):
-    w = Workload("chain", B, T, E, K, I, J, dtype, "replace", 5)
-    ins = {k: v.to(cuda_device) for k, v in workloads.make_inputs(w, integer_valued=True).items() if torch.is_tensor(v)}
-    b = torch.randint(-2, 3, (E, J), device=cuda_device).to(dtype) if bias else None
-    Ws = ins["Ws"].sign()              # a token row's few contributions stay below 256: exact in 16 bits too
+def test_operators_back_to_back(cuda_device, B, T, E, K, I, J, dtype):
+    g = torch.Generator(device=cuda_device).manual_seed(I)
+    ints = lambda *s: torch.randint(-1, 2, s, generator=g, device=cuda_device).to(dtype)
+    one = lambda n, m: torch.zeros(E, n, m, device=cuda_device, dtype=dtype).scatter_(1, torch.randint(0, n, (E, 1, m), generator=g, device=cuda_device),
+                                                                                      ints(E, 1, m))
+    Xs, G, Wg, Ws = [ints(B, T, I) for _ in range(4)], ints(B, T, I), one(I, J), one(J, I)
+    scores = torch.rand(B, T, E, generator=g, device=cuda_device)
+    Ind = torch.rand(B, E, T, generator=g, device=cuda_device).topk(K, -1).indices
+    bias = ints(E, J)
 
-    def step(i, sync):
-        X, wait = ins["X"].roll(i, 1), torch.cuda.synchronize if sync else (lambda: None)
+    def one_pass(X, sync):
+        wait = torch.cuda.synchronize if sync else (lambda: None)
+        out = []
+        def keep(t):
+            wait()
+            out.append(t)
+            return t
+        Y = keep(ops.gather_gemm(X, Wg, Ind))
+        Out = keep(ops.gemm_scatter(Y, Ws, Ind, T))                                    # reads Y; counts ids by itself
+        Y2 = keep(ops.gather_gemm(Out, Wg, Ind, bias=bias))                            # gathers what was just added
+        dW = keep(ops.dweight(Out, Y2, Ind))
+        dWd = keep(ops.dweight(X, Y2, Ind, out_layout="direct_rows"))
+        ops.fill_zero(Y)                                                               # overwrites what the scatter has read
         wait()
-        csr = ops.build_index_csr(ins["Ind"], T)
+        ind = keep(ops.route_topk(scores, K, index_dtype=torch.int32))
+        csr = ops.build_index_csr(ind, T)
+        keep(csr.entries)
+        Y3 = keep(ops.gather_gemm(X, Wg, ind))
+        O3 = keep(ops.gemm_scatter(Y3, Ws, ind, T, csr=csr))
+        ops.gemm_scatter(Y3, Ws, ind, T, out=O3)                                       # adds to what was just added to
         wait()
-        Y = ops.gather_gemm(X, ins["Wg"], ins["Ind"], bias=b)
+        step = train_step(X, Wg, Ws, Ind, G)
         wait()
-        Out = ops.gemm_scatter(Y.clamp_(-1, 1), Ws, ins["Ind"], T, csr=csr)
-        wait()
-        dW = ops.dweight(Out.clamp_(-4, 4), Y, ins["Ind"], out_layout="direct_rows")
-        wait()
-        return Y, Out, dW, csr.entries
-    alone = [step(i, True) for i in range(6)]
-    together = [step(i, False) for i in range(6)]
+        return [Y, Out, Y2, dW, dWd, ind, csr.entries, Y3, O3] + [step[k] for k in STEP_KEYS]
+    alone = [one_pass(X, True) for X in Xs]
+    together = [one_pass(X, False) for X in Xs]
+    for X in Xs * 2:                              # results dropped: torch hands their memory to the next operators
+        last = one_pass(X, False)
     ops.check_status()
-    for x, y in zip(alone, together):
-        assert all(torch.equal(p, q) for p, q in zip(x, y))
+    for x, y in zip(alone + [alone[-1]], together + [last]):
+        assert max(t.abs().max().item() for t in x[:3] + x[7:9]) <= 256
+        for i, (p, q) in enumerate(zip(x, y)):
+            assert torch.equal(p, q), i
 
 
 # 16-bit scatters on pairs whose rows stay for `kept` column tiles: whole waves of row blocks and a rest, a last tile of few columns, rows as
