@@ -528,3 +528,27 @@ def test_generic_dweight_edges(cuda_device, B, T, E, K, FG, FD, dtype, out_layou
     P = torch.einsum("bekf,bekg->efg" if out_layout == "gathered_rows" else "bekf,bekg->egf", rows, Y.double())
     assert torch.equal(ops.dweight(X, Y, Ind, out_layout=out_layout, path="generic"), P.to(dtype))
     ops.reset_status()
+
+
+# operands that begin 16 bytes into their storage (the least the tensor-core kernels and their boxes take) or at any element (generic kernels)
+@pytest.mark.parametrize("offset_bytes", [16, 4])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_operands_at_offsets(cuda_device, dtype, offset_bytes):
+    B, T, E, K, I, J = 6, 90, 3, 32, 136, 72
+    g = torch.Generator(device=cuda_device).manual_seed(2)
+    n = offset_bytes // dtype.itemsize
+
+    def at_offset(t):
+        whole = torch.empty(t.numel() + n, dtype=t.dtype, device=cuda_device)
+        return whole[n:].copy_(t.reshape(-1)).view(t.shape)
+    small = lambda *s: torch.randint(-1, 2, s, generator=g, device=cuda_device).to(dtype)
+    X, Y, Wg, Ws = small(B, T, I), small(B, E, K, J), small(E, I, J), small(E, J, I)
+    Ind = (torch.arange(B * E * K, device=cuda_device).view(B, E, K) * 7) % T
+    Xo, Yo, Wgo, Wso, Indo = (at_offset(t) for t in (X, Y, Wg, Ws, Ind.int()))
+    assert {t.data_ptr() % 32 for t in (Xo, Yo, Wgo, Wso)} == {offset_bytes}
+    assert torch.equal(ops.gather_gemm(Xo, Wgo, Indo), ops.gather_gemm(X, Wg, Ind))
+    assert torch.equal(ops.gather_gemm(Xo, Wso, Indo, w_layout="nc"), ops.gather_gemm(X, Ws, Ind, w_layout="nc"))
+    assert torch.equal(ops.gemm_scatter(Yo, Wso, Indo, T), ops.gemm_scatter(Y, Ws, Ind, T))
+    assert torch.equal(ops.gemm_scatter(Yo, Wgo, Indo, T, w_layout="nc"), ops.gemm_scatter(Y, Wg, Ind, T, w_layout="nc"))
+    assert torch.equal(ops.dweight(Xo, Yo, Indo), ops.dweight(X, Y, Ind))
+    ops.check_status()
