@@ -184,7 +184,7 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
                                    zero_output, dtype, status_ref(status), st);
       own = true;
     } else {
-      err = zero_output ? launch_fill_zero(acc, n_out * sizeof(float), st) : launch_convert_to_f32(Out, acc, n_out, dtype, st);
+      err = zero_output ? launch_fill_zero(acc, n_out * sizeof(float), st, false) : launch_convert_to_f32(Out, acc, n_out, dtype, st);
     }
     if (err != cudaSuccess) return fail_cuda(err, "scatter scratch init");
   } else if (scatter && zero_output) {
@@ -195,7 +195,7 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
   auto finish_rows = [&]() -> int {
     if (!f32_rows) return EGS_OK;
     cudaError_t err = plan ? launch_scatter_finish(plan, acc, Out, n_out, dtype, st)
-                           : launch_convert_from_f32(acc, Out, n_out, dtype, st);
+                           : launch_convert_from_f32(acc, Out, n_out, dtype, st, false);
     return err == cudaSuccess ? EGS_OK : fail_cuda(err, "scatter scratch convert");
   };
   if (no_work) return finish_rows();
@@ -413,7 +413,7 @@ int egs_gather_scatter_pair(const void* Src, const void* W1, const void* W2, con
 
   if (dtype == EGS_F32) {
     if (zero_output && dst_bytes > 0) {
-      cudaError_t err = launch_fill_zero(Dst, dst_bytes, st, true);
+      cudaError_t err = launch_fill_zero(Dst, dst_bytes, st);
       if (err != cudaSuccess) return fail_cuda(err, "fill_zero");
       p.after_own = 1;
     }
@@ -539,7 +539,7 @@ static int dweight_impl(const void* Xsrc, const void* Ysrc, const void* Ind, voi
   err = strict ? launch_strict_dweight(p, st) : dense16 ? launch_dense16_dweight(p, dtype, st) : tensor ? launch_tensor_dweight(p, smem, st) : launch_generic_dweight(p, dtype, st);
   if (err != cudaSuccess) return fail_cuda(err, "dweight launch");
   if (p.splits > 1 && dtype != EGS_F32) {
-    err = launch_convert_from_f32(p.acc, out, n_out, dtype, st);
+    err = launch_convert_from_f32(p.acc, out, n_out, dtype, st, tensor);
     if (err != cudaSuccess) return fail_cuda(err, "convert launch");
   }
   return EGS_OK;

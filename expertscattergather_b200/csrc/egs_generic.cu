@@ -9,7 +9,7 @@ namespace egs {
 
 namespace {
 
-// Both kernels: 128 threads as 16 (ty) x 8 (tx), operands converted to float32 in shared memory, contraction steps of 32.
+// The row kernel and the first weight-gradient kernel: 128 threads as 16 (ty) x 8 (tx), operands converted to float32 in shared memory, contraction steps of 32.
 // What bounds them is the chain of a step - load, barrier, multiply - so the next step's elements are fetched into registers
 // while the current one is multiplied, lanes run along the contiguous direction of every row (whole 128-byte segments), and
 // several CTAs share an SM.  Results leave through shared memory for the same reason: rows are written (or added to) 32
@@ -601,8 +601,9 @@ template <typename T> __device__ __forceinline__ void convert8(const float* src,
 
 template <typename T>
 __global__ void __launch_bounds__(256) convert_from_f32_kernel(const float* src, T* dst,
-                                                              size_t n) {
+                                                              size_t n, int early) {
   pdl_wait();
+  if (early) pdl_trigger();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   const size_t i0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const bool vec = sizeof(T) == 2 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0;
@@ -854,13 +855,13 @@ cudaError_t launch_fill_zero(void* ptr, size_t bytes, cudaStream_t st, bool earl
   return err;
 }
 
-cudaError_t launch_convert_from_f32(const float* src, void* dst, size_t n, int dtype, cudaStream_t st) {
+cudaError_t launch_convert_from_f32(const float* src, void* dst, size_t n, int dtype, cudaStream_t st, bool early) {
   if (n == 0) return cudaSuccess;
   const int grid = grid_for(n, 256 * 4);
   cudaError_t err;
-  if (dtype == EGS_F16) err = launch_kernel(convert_from_f32_kernel<__half>, grid, 256, 0, st, true, src, static_cast<__half*>(dst), n);
+  if (dtype == EGS_F16) err = launch_kernel(convert_from_f32_kernel<__half>, grid, 256, 0, st, true, src, static_cast<__half*>(dst), n, early ? 1 : 0);
   else if (dtype == EGS_BF16)
-    err = launch_kernel(convert_from_f32_kernel<__nv_bfloat16>, grid, 256, 0, st, true, src, static_cast<__nv_bfloat16*>(dst), n);
+    err = launch_kernel(convert_from_f32_kernel<__nv_bfloat16>, grid, 256, 0, st, true, src, static_cast<__nv_bfloat16*>(dst), n, early ? 1 : 0);
   else return cudaErrorInvalidValue;
   count_launch();
   return err;

@@ -160,9 +160,9 @@ cudaError_t launch_generic_dweight(const DWeightParams& p, int dtype, cudaStream
 // out[e, n] = sum over the slots of expert e of a row of Src: token rows through Ind, or slot rows where Ind is NULL
 cudaError_t launch_expert_row_sum(const void* Src, const void* Ind, int index_dtype, void* out, int B, int T, int E, int K, int N,
                                   int dtype, StatusRef status, cudaStream_t st);
-// early: the next kernel is one of the call's that has its SM for itself and may begin under the fill
-cudaError_t launch_fill_zero(void* ptr, size_t bytes, cudaStream_t st, bool early = false);
-cudaError_t launch_convert_from_f32(const float* src, void* dst, size_t n, int dtype, cudaStream_t st);
+// early: dependents may start with this kernel; false in front of and behind the generic kernels (see the top of egs_generic.cu)
+cudaError_t launch_fill_zero(void* ptr, size_t bytes, cudaStream_t st, bool early = true);
+cudaError_t launch_convert_from_f32(const float* src, void* dst, size_t n, int dtype, cudaStream_t st, bool early);
 cudaError_t launch_convert_to_f32(const void* src, float* dst, size_t n, int dtype, cudaStream_t st);
 // 16-bit scatter (see egs_generic.cu): prepare decides between direct additions (no token row gets more than `limit` contributions)
 // and float32 rows, and zeroes (or seeds) what the additions go to; finish rounds the float32 rows.
