@@ -50,8 +50,11 @@ __device__ __forceinline__ float4 float4_of(unsigned long long a, unsigned long 
 // (operator G: egs/triton_kernels.py:48-143, operator S: :156-247 in the reference)
 // NJ: tile width in units of 32 columns.  Thread (ty, tx) owns rows ty + 16 i and columns 32 j + 4 tx .. + 3.
 // ------------------------------------------------------------------------------------------------
-template <typename T, bool SCATTER, int NJ>
-__global__ void __launch_bounds__(NTHREADS, NJ == 4 ? 3 : 4) generic_rowgemm_kernel(RowGemmParams p) {
+// CTAS: CTAs that share an SM.  96 columns spill at four (float32), and a contraction of several steps pays for that: 32768 rows 1001 -> 257 of 16 experts
+// 549 us with four, 546 before products went in pairs, 483 with three; 960 rows 655 -> 67 70, 59 and 51.  A single step is over too soon: 60680 rows
+// 5 -> 177 24 us with four, 26 with three.
+template <typename T, bool SCATTER, int NJ, int CTAS>
+__global__ void __launch_bounds__(NTHREADS, CTAS) generic_rowgemm_kernel(RowGemmParams p) {
   constexpr int BN = 32 * NJ, BPITCH = BN + 4;
   __shared__ __align__(16) float As[TM * APITCH];
   __shared__ __align__(16) float Bs[TK * BPITCH];
@@ -743,17 +746,18 @@ cudaError_t launch_generic_rowgemm(const RowGemmParams& p, bool scatter, int dty
   const int nj = width_in_32s(p.N, 4);
   dim3 grid((p.M + TM - 1) / TM, (p.N + 32 * nj - 1) / (32 * nj), p.E);
   cudaError_t err;
-#define EGS_LAUNCH_NJ(TY, NJV)                                                             \
+#define EGS_LAUNCH_NJ(TY, NJV, CTAS)                                                       \
   do {                                                                                     \
-    if (scatter) err = launch_kernel(generic_rowgemm_kernel<TY, true, NJV>, grid, NTHREADS, 0, st, true, p);      \
-    else err = launch_kernel(generic_rowgemm_kernel<TY, false, NJV>, grid, NTHREADS, 0, st, true, p);             \
+    if (scatter) err = launch_kernel(generic_rowgemm_kernel<TY, true, NJV, CTAS>, grid, NTHREADS, 0, st, true, p);      \
+    else err = launch_kernel(generic_rowgemm_kernel<TY, false, NJV, CTAS>, grid, NTHREADS, 0, st, true, p);             \
   } while (0)
 #define EGS_LAUNCH(TY)                       \
   do {                                       \
-    if (nj == 1) EGS_LAUNCH_NJ(TY, 1);       \
-    else if (nj == 2) EGS_LAUNCH_NJ(TY, 2);  \
-    else if (nj == 3) EGS_LAUNCH_NJ(TY, 3);  \
-    else EGS_LAUNCH_NJ(TY, 4);               \
+    if (nj == 1) EGS_LAUNCH_NJ(TY, 1, 4);    \
+    else if (nj == 2) EGS_LAUNCH_NJ(TY, 2, 4);  \
+    else if (nj == 3 && p.C <= TK) EGS_LAUNCH_NJ(TY, 3, 4);  \
+    else if (nj == 3) EGS_LAUNCH_NJ(TY, 3, 3);  \
+    else EGS_LAUNCH_NJ(TY, 4, 3);            \
   } while (0)
   if (dtype == EGS_F32) EGS_LAUNCH(float);
   else if (dtype == EGS_F16) EGS_LAUNCH(__half);

@@ -552,3 +552,25 @@ def test_operands_at_offsets(cuda_device, dtype, offset_bytes):
     assert torch.equal(ops.gemm_scatter(Yo, Wgo, Indo, T, w_layout="nc"), ops.gemm_scatter(Y, Wg, Ind, T, w_layout="nc"))
     assert torch.equal(ops.dweight(Xo, Yo, Indo), ops.dweight(X, Y, Ind))
     ops.check_status()
+
+
+# generic row kernel: one to four times 32 columns a CTA with remainders; 65 to 96 columns have two forms, for one contraction step (up to 32
+# elements) and for more
+@pytest.mark.parametrize("C,N", [(1, 67), (31, 96), (32, 81), (33, 67), (65, 257), (101, 89), (97, 33), (33, 127), (5, 31)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("w_layout", ["cn", "nc"])
+def test_generic_rowgemm_edges(cuda_device, C, N, dtype, w_layout):
+    B, T, E, K = 3, 70, 4, 43
+    g = torch.Generator(device=cuda_device).manual_seed(C + N)
+    small = lambda *s: torch.randint(-1, 2, s, generator=g, device=cuda_device).to(dtype)
+    X, Y, W = small(B, T, C), small(B, E, K, C), small(E, C, N)
+    Wl = W if w_layout == "cn" else W.transpose(1, 2).contiguous()
+    Ind = torch.randint(0, T, (B, E, K), generator=g, device=cuda_device)
+    Ind[B - 1, E - 1, K - 1] = T                  # out of range: a row of zeros, and left out
+    known, slots = (Ind < T).unsqueeze(-1), Ind.clamp(max=T - 1).reshape(B, E * K, 1)
+    rows = torch.gather(X.double(), 1, slots.expand(-1, -1, C)).reshape(B, E, K, C) * known
+    assert torch.equal(ops.gather_gemm(X, Wl, Ind, w_layout=w_layout, path="generic"), torch.einsum("bekc,ecn->bekn", rows, W.double()).to(dtype))
+    products = torch.einsum("bekc,ecn->bekn", Y.double(), W.double()) * known
+    Out = torch.zeros(B, T, N, dtype=torch.float64, device=cuda_device).scatter_add_(1, slots.expand(-1, -1, N), products.reshape(B, E * K, N))
+    assert torch.equal(ops.gemm_scatter(Y, Wl, Ind, T, w_layout=w_layout, path="generic"), Out.to(dtype))
+    ops.reset_status()
