@@ -28,8 +28,9 @@
 // instruction (320 a stage of G), side by side with the TMA unit; a pair's gathers take the TMA units about as long.  Everything else has to stay out of the way: a satisfied barrier
 // wait takes 150 clocks and every dependent instruction of a lone warp 5-10, so nothing on a per-stage or per-tile path divides, the
 // issuing warps run converged (see mbar_wait_all) and ids are looked up elsewhere.
-// T=1024, E=64, K=64, I=1024, J=256, bf16: B=64 G 126-138 us, S 180 (190 before), D 148-165; B=512 G 950 us, dY (weights [E, N, C]) 895 = 1.23
-// PFLOP/s, S 1150 (1240 before its rows stayed), D 1050, under the power cap; S without the fill of its output.
+// T=1024, E=64, K=64, I=1024, J=256, bf16: B=64 G 126-138 us, D 148-165; B=512, under the power cap, G 850-990 us, dY (weights [E, N, C]) 840-900 = 1.23
+// PFLOP/s, D 1050-1200.  S as whole calls, its rows loaded for every column tile and kept, in turn: B=64 194 and 185 us, weights [E, N, C] 193 and
+// 185; B=512 1450 and 1361, 1577 and 1455 (about 200 of that fills the output).
 #include <algorithm>
 #include <type_traits>
 

@@ -240,8 +240,10 @@ void count_launch(int n = 1);
 //   * it takes no `__restrict__` pointers: until the wait its inputs may still be written, and loads that are promised the contrary are
 //     not bound by it.  (Row sums, which are launched normally, keep theirs.  Without them nothing got slower by more than the runs differ.)
 // Launch and set-up of a kernel so run under the end of the one before, also across calls: 1-2 us a kernel (a training pass of ten
-// kernels 151 -> 145 us, one of fourteen 253 -> 241).  The persistent kernels trigger when their last tile has been issued: triggering
-// at their start let a dependent's waiting CTAs keep a kernel of another stream off an SM (253 -> 251 us only).
+// kernels 151 -> 145 us, one of fourteen 253 -> 249).  The persistent kernels trigger when their last tile has been issued: triggering
+// at their start lets a dependent's waiting CTAs keep a kernel of another stream off an SM.  Kernels of which an SM holds several CTAs
+// (egs_generic.cu) do not trigger at all.  Ordinary launches: the bias row sums, the TF32 and fused kernels that no fill of their call precedes,
+// egs_gather2.cu, top-k of long sequences, the CSR of large batches and what reads it.
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
