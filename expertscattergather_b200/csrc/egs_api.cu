@@ -93,6 +93,10 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 constexpr long long kInt32Max = 2147483647LL;
 // 16-bit scatter adds directly into the output while no token row receives more contributions than this.
 constexpr int kDirect16Limit = 32;
+// 16-bit scatters of at most this many output elements round their float32 rows in the scatter kernel (its last CTA does it); a launch of its
+// own finds nothing to round after most calls.  Back to back, bf16, 64 tokens of 8 experts, 128 -> 512 features: 7.4 us a scatter with the
+// launch, 6.4 without; where a hot row selects float32 rows 9.4 and 12.1, at 64 Ki elements 10.5 and 16.6.  The host saves 2 us a launch.
+constexpr size_t kRoundInKernel = 64 << 10;
 // Longest contraction strict float32 runs on the tensor cores under EGS_PATH_AUTO (measured against float64 up to there, see
 // egs_strict.cu), and longest that one accumulator of the fused pair kernel sees.
 constexpr long long kStrictMaxContraction = 2048;
@@ -153,7 +157,7 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
   const bool no_work = (d.B * d.E * d.K == 0);
   if (!no_work && (!A || !W || !Ind) && d.C > 0) return EGS_ERR_INVALID_ARGUMENT;
 
-  // 16-bit scatter.  Workspace layout: [plan flag, 256 B][counting flags, room for B*T ints][float32 rows, B*T*N].  Generic
+  // 16-bit scatter.  Workspace layout: [plan, 256 B][counting flags, room for B*T ints][float32 rows, B*T*N].  Generic
   // kernels always sum in the float32 rows; the tensor-core path decides between those and direct 16-bit additions (see
   // egs_generic.cu).
   const bool f32_rows = scatter && dtype != EGS_F32;
@@ -180,7 +184,7 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
     if (tensor && !no_work && d.C > 0) {
       plan = reinterpret_cast<int*>(ws);
       err = launch_scatter_prepare(Ind, index_dtype, static_cast<int>(d.B), static_cast<int>(d.T), static_cast<int>(d.E),
-                                   static_cast<int>(d.K), csr_info, kDirect16Limit, plan + 64, plan, acc, Out, static_cast<int>(d.N),
+                                   static_cast<int>(d.K), csr_info, kDirect16Limit, plan + kPlanWords, plan, acc, Out, static_cast<int>(d.N),
                                    zero_output, dtype, status_ref(status), st);
       own = true;
     } else {
@@ -192,8 +196,9 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
     if (err != cudaSuccess) return fail_cuda(err, "fill_zero");
     own = true;
   }
+  const bool rounds = plan && n_out <= kRoundInKernel;
   auto finish_rows = [&]() -> int {
-    if (!f32_rows) return EGS_OK;
+    if (!f32_rows || rounds) return EGS_OK;
     cudaError_t err = plan ? launch_scatter_finish(plan, acc, Out, n_out, dtype, st)
                            : launch_convert_from_f32(acc, Out, n_out, dtype, st, false);
     return err == cudaSuccess ? EGS_OK : fail_cuda(err, "scatter scratch convert");
@@ -208,7 +213,7 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
   }
 
   RowGemmParams p{};
-  p.A = A; p.W = W; p.bias = bias; p.Ind = Ind; p.Out = Out; p.acc = acc; p.plan = plan; p.status = status_ref(status);
+  p.A = A; p.W = W; p.bias = bias; p.Ind = Ind; p.Out = Out; p.acc = acc; p.plan = plan; p.rounds = rounds ? 1 : 0; p.status = status_ref(status);
   p.B = static_cast<int>(d.B); p.T = static_cast<int>(d.T); p.E = static_cast<int>(d.E); p.K = static_cast<int>(d.K);
   p.C = static_cast<int>(d.C); p.N = static_cast<int>(d.N);
   p.M = static_cast<int>(d.B * d.K);
@@ -441,7 +446,7 @@ int egs_gather_scatter_pair(const void* Src, const void* W1, const void* W2, con
   const size_t counter_bytes = (static_cast<size_t>(B) * T * sizeof(int) + 255) & ~static_cast<size_t>(255);
   int* plan = reinterpret_cast<int*>(ws);
   float* acc = reinterpret_cast<float*>(ws + 256 + counter_bytes);
-  cudaError_t err = launch_scatter_prepare(Ind, index_dtype, p.B, p.T, p.E, p.K, nullptr, kDirect16Limit, plan + 64, plan, acc, Dst, p.N2, zero_output,
+  cudaError_t err = launch_scatter_prepare(Ind, index_dtype, p.B, p.T, p.E, p.K, nullptr, kDirect16Limit, plan + kPlanWords, plan, acc, Dst, p.N2, zero_output,
                                            dtype, status_ref(status_word), st);
   if (err != cudaSuccess) return fail_cuda(err, "scatter preparation");
   p.after_own = 1;

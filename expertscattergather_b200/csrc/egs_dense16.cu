@@ -73,6 +73,7 @@ struct __align__(16) DenseHeader {
   unsigned long long drain;
   uint32_t tmem_base;
   uint32_t abort_flag;
+  int added, last;                       // S: read-out warps that have added what they had to; 1: the grid's last, -1: others are to come
 };
 static_assert(sizeof(DenseHeader) <= kDenseHeader, "header does not fit");
 
@@ -83,7 +84,8 @@ struct DenseParams {
   const void* Ind;
   void* Out;          // G: slot rows; S: token rows; D: the gradient
   float* acc;         // S: float32 rows; D: float32 sums when splits > 1
-  const int* plan;    // S: see RowGemmParams::plan
+  int* plan;          // S: PlanWords
+  int rounds;         // S: the kernel rounds float32 rows itself
   StatusRef status;
   int B, T, E, K, M;
   int C, N;           // G, S: contraction and produced width; D: features of the operand along the accumulator's rows / columns
@@ -207,6 +209,48 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* map, int x
       : "memory");
 }
 
+// Rounds the float32 rows of a small scatter that sums in those: the CTA whose read-out warps are the last of the grid to have added what
+// they had to does it.  Nobody waits for another CTA, which may have yet to find room beside another stream's kernels.
+template <typename T>
+__device__ __noinline__ void round_rows(const DenseParams& p, DenseHeader* hdr, int warp, int lane) {
+  __threadfence();
+  __syncwarp();
+  if (lane == 0 && atomicAdd(&hdr->added, 1) == p.readers - 1) {
+    __threadfence();
+    const bool last = atomicAdd(p.plan + kPlanAdded, 1) == static_cast<int>(gridDim.x) - 1;
+    __threadfence();
+    *const_cast<volatile int*>(&hdr->last) = last ? 1 : -1;
+  }
+  const volatile int *verdict = &hdr->last;
+  const volatile uint32_t* abort_flag = &hdr->abort_flag;
+  __syncwarp();
+  while (__all_sync(0xffffffffu, *verdict == 0))
+    if (__any_sync(0xffffffffu, *abort_flag != 0u)) return;              // (a warp that gave up does not count)
+  if (__any_sync(0xffffffffu, *verdict < 0)) return;
+  __threadfence();
+  const int n = p.B * p.T * p.N;                     // (see kRoundInKernel)
+  T* out = static_cast<T*>(p.Out);
+  constexpr int kAtOnce = 8;
+  const int step = p.readers * 256;
+  for (int i0 = (warp * 32 + lane) * 8; i0 < n; i0 += kAtOnce * step) {
+    float4 v[2 * kAtOnce];
+#pragma unroll
+    for (int j = 0; j < kAtOnce; ++j) {
+      const float4* from = reinterpret_cast<const float4*>(p.acc + min(i0 + j * step, n - 8));
+      v[2 * j] = __ldcg(from);
+      v[2 * j + 1] = __ldcg(from + 1);
+    }
+#pragma unroll
+    for (int j = 0; j < kAtOnce; ++j) {
+      const float4 a = v[2 * j], b = v[2 * j + 1];
+      if (i0 + j * step < n)
+        *reinterpret_cast<uint4*>(out + i0 + j * step) =
+            make_uint4(pack2(out, __float_as_uint(a.x), __float_as_uint(a.y)), pack2(out, __float_as_uint(a.z), __float_as_uint(a.w)),
+                       pack2(out, __float_as_uint(b.x), __float_as_uint(b.y)), pack2(out, __float_as_uint(b.z), __float_as_uint(b.w)));
+    }
+  }
+}
+
 // KEEP: a scatter whose rows stay for several column tiles (see pick_tile).  An instance of its own: with the slots of kept rows and the
 // walk over both kinds of units in the lanes that issue loads and MMAs, scatters that keep nothing took 3-7 % longer (bf16, 64 experts
 // of 5760 rows, 128 -> 520 features: 181 us without, 193 with).
@@ -253,6 +297,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     fence_mbar_init();
     if (!p.after_own) pdl_wait();
     hdr->abort_flag = p.status.timed_out() ? 1u : 0u;
+    hdr->added = hdr->last = 0;
     if (smem_misaligned(smem_raw)) {
       hdr->abort_flag = 1u;
       p.status.report(EGS_STATUS_INTERNAL);
@@ -527,7 +572,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     T* out = static_cast<T*>(p.Out);
     bool alive = true;
     pdl_wait();                                          // zeros the results are added to, the scatter's plan
-    const bool f32_rows = OP == kOpScatter && *p.plan != 0;
+    const bool f32_rows = OP == kOpScatter && p.plan[kPlanHot] != 0;
     int t = 0;
     for (Walk<OP, PAIR, KEEP> u(p); u.left > 0 && alive; u.next(), ++t) {
       const int bn = min(p.BN, p.N - u.n0);              // columns of this tile (a multiple of 8)
@@ -647,6 +692,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       }
       if (!released) release();
     }
+    if (OP == kOpScatter && f32_rows && alive && p.rounds) round_rows<T>(p, hdr, ew, lane);
     }
   } else if (warp == kMmaWarp) {
     // =========================== MMA issuer ===========================
@@ -1011,7 +1057,7 @@ void configure_dense16_rowgemm(RowGemmParams& p, bool scatter) {
 
 cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dtype, cudaStream_t st) {
   DenseParams p{};
-  p.Rows = r.A; p.bias = r.bias; p.Ind = r.Ind; p.Out = r.Out; p.acc = r.acc; p.plan = r.plan; p.status = r.status;
+  p.Rows = r.A; p.bias = r.bias; p.Ind = r.Ind; p.Out = r.Out; p.acc = r.acc; p.plan = r.plan; p.rounds = r.rounds; p.status = r.status;
   p.B = r.B; p.T = r.T; p.E = r.E; p.K = r.K; p.M = r.M; p.C = r.C; p.N = r.N;
   p.nc = r.w_layout == EGS_W_NC;
   p.index_dtype = r.index_dtype;

@@ -701,7 +701,7 @@ __global__ void __launch_bounds__(kPrepThreads) scatter_prepare_kernel(const voi
   } else if (EK > limit) {
     flag = B == 1 ? has_hot_row<true>(ind, index_dtype, 0, 1, T_, EK, limit, prep_cnt) : has_hot_row<false>(ind, index_dtype, 0, B, T_, EK, limit, prep_cnt);
   }
-  if (blockIdx.x == 0 && tid == 0) *plan = flag;
+  if (blockIdx.x == 0 && tid <= kPlanAdded) plan[tid] = tid == kPlanHot ? flag : 0;
   const size_t stride = static_cast<size_t>(gridDim.x) * kPrepThreads, i0 = static_cast<size_t>(blockIdx.x) * kPrepThreads + tid;
   // (n is a multiple of 8 elements and both buffers are 16-byte aligned: tensor-core path only)
   if (flag && zero_output) {

@@ -79,14 +79,19 @@ struct Div {
 // ------------------------------------------------------------------------------------------------
 // parameter blocks (validated on the host: every product below fits in int32 unless typed int64)
 // ------------------------------------------------------------------------------------------------
+
+// The plan of a scatter with 16-bit tensors on the tensor cores, words on the device: whether its token rows accumulate in the float32 rows
+// (else additions go straight into the 16-bit output); CTAs that have added what they had to (zero at first).
+enum PlanWords { kPlanHot = 0, kPlanAdded = 1, kPlanWords = 64 };
+
 struct RowGemmParams {
   const void* A;      // G: token rows [B*T, C]      S: slot rows [B*E*K, C]
   const void* W;      // [E, C, N] (EGS_W_CN) or [E, N, C] (EGS_W_NC)
   const void* Ind;    // [B, E, K]
   void* Out;          // G: slot rows [B*E*K, N]     S: token rows [B*T, N]
   float* acc;         // S with 16-bit tensors: float32 accumulation rows [B*T, N]; otherwise unused
-  const int* plan;    // S with 16-bit tensors: a device flag, non-zero = token rows accumulate in the float32 rows, zero = direct
-                      // additions into the 16-bit output; NULL = always the float32 rows
+  int* plan;          // 16-bit S on the tensor cores: PlanWords
+  int rounds;         // ... and whether the kernel rounds the float32 rows itself
   const void* bias;   // optional [E, N] in the tensors' dtype: bias[e, :] is added to every produced row of expert e
                       // (G: to the stored row; S: to the row before it is added to its token row); NULL = none
   StatusRef status;    // optional device status word
@@ -138,7 +143,7 @@ struct FusedParams {
   void* Mid;           // slot rows [B*E*K, N1], overwritten
   float* Dst;          // float32 token rows [B*T, N2], added to (16-bit tensors: the accumulation rows of the scratch)
   void* Out16;         // 16-bit tensors: the output token rows [B*T, N2] that direct 16-bit additions go to
-  const int* plan;     // 16-bit tensors: device flag, see RowGemmParams::plan
+  const int* plan;     // 16-bit tensors: device flag, non-zero = token rows accumulate in the float32 rows, zero = direct additions
   StatusRef status;
   int B, T, E, K, C1, N1, N2;
   int M;               // B*K
@@ -165,7 +170,7 @@ cudaError_t launch_fill_zero(void* ptr, size_t bytes, cudaStream_t st, bool earl
 cudaError_t launch_convert_from_f32(const float* src, void* dst, size_t n, int dtype, cudaStream_t st, bool early);
 cudaError_t launch_convert_to_f32(const void* src, float* dst, size_t n, int dtype, cudaStream_t st);
 // 16-bit scatter (see egs_generic.cu): prepare decides between direct additions (no token row gets more than `limit` contributions)
-// and float32 rows, and zeroes (or seeds) what the additions go to; finish rounds the float32 rows.
+// and float32 rows, and zeroes (or seeds) what the additions go to; finish rounds the float32 rows for kernels that do not do that.
 // csr_info: the summary of a prepared CSR, whose heaviest row decides; NULL = the ids are counted.  flags: scratch of B ints.
 cudaError_t launch_scatter_prepare(const void* Ind, int index_dtype, int B, int T, int E, int K, const int* csr_info, int limit, int* flags,
                                    int* plan, float* acc, void* out16, int N, int zero_output, int dtype, StatusRef status, cudaStream_t st);

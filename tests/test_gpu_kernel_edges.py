@@ -411,6 +411,22 @@ def test_scatter16_one_hot_row_rounds_all_rows_once(cuda_device, B, pair):
     assert (np.abs(Out.cpu().double().numpy() - ref) <= 2.0 ** -8 * np.abs(ref) + 1e-5 * np.abs(ref).max()).all()
 
 
+# small outputs of float32 rows are rounded by the scatter's last CTA, those of more than 64 Ki elements by a launch of their own.  Small
+# integers: every sum is exact in float32, so the result is the exact one, rounded once.
+@pytest.mark.parametrize("B,T,E,K,C,N", [(1, 1, 1, 40, 8, 8), (1, 1, 40, 1, 32, 2064), (2, 512, 5, 16, 64, 64), (2, 513, 5, 16, 64, 64), (7, 24, 140, 2, 40, 376)])
+@pytest.mark.parametrize("form", ["plain", "out"])
+def test_scatter16_rounds_small_outputs(cuda_device, B, T, E, K, C, N, form):
+    g = torch.Generator().manual_seed(N)
+    Ind = torch.randint(0, T, (B, E, K), generator=g)
+    Ind.view(-1)[:40] = 0                                          # a hot row in the first batch element
+    Y = torch.randint(-7, 8, (B, E, K, C), generator=g).to(torch.bfloat16)
+    W = torch.randint(-7, 8, (E, C, N), generator=g).to(torch.bfloat16)
+    out = torch.randint(-64, 65, (B, T, N), generator=g).to(torch.bfloat16) if form == "out" else None
+    ref = orc.np_scatter(Y, W, Ind, T) + (0.0 if out is None else out.double().numpy())
+    got = ops.gemm_scatter(Y.to(cuda_device), W.to(cuda_device), Ind.to(cuda_device), T, out=None if out is None else out.to(cuda_device))
+    assert torch.equal(got.cpu(), torch.from_numpy(ref).to(torch.bfloat16))
+
+
 # kernels become resident under the end of the ones before them: operators issued back to back, with nothing of torch between them, have to
 # give what they give one by one.  Each reads what the one before it has just written, or writes what it has just read: every family of
 # kernels, with and without prepared indices, more than one wave of tiles, the helper stream's fork and join.  A column of the weights has one
