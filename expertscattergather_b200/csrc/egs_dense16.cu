@@ -324,19 +324,34 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     pdl_wait();                          // (and fall through to the common exit)
   } else if (PAIR && warp < kProdWarps && gathers) {
     // =========================== gather producers of a pair ===========================
-    // Every warp gathers the same rows of each stage, four at a time (tile::gather4).
+    // Rows come four at a time (tile::gather4).  Two groups of four warps take the stages in turn, a warp a quarter of a stage's rows,
+    // and load them segment by segment: a warp's loads one after the other go to one stretch of shared memory, and what a step costs a
+    // warp beside them - ids, the barrier, coordinates moved to uniform registers - it has two steps' time for.  With eight rows of both
+    // segments in turn for every stage, the gathers alone of a step of D took 860 clocks (with everything else 974, now 800), more than
+    // its MMAs: bf16, 64 experts of 1024 rows, 2048 x 512 features 132 us; eight rows segment by segment 120; in two groups 116.
+    constexpr int kGroups = 2, kParts = kProdWarps / kGroups;
+    const int group = warp & (kGroups - 1), part = warp / kGroups;
     const uint32_t table = smem0 + kDenseHeader;
     auto get4 = [](uint32_t a, int (&r)[4]) {
       asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
     };
     Cursor at;
     bool alive = true;
+    int turn = 0;
     auto wait_free = [&]() {             // for the stage at `at`; its barrier (the leader's) and its first byte here; moves on
       if (at.round > 0) alive = mbar_wait_all(smem_u32(&hdr->empty[at.slot]), (at.round - 1) & 1, abort_flag, p.status.word);
     };
+    // Whether the stage at `at` is this warp's, and then waits for it.  A warp must not skip phases of a barrier that it waits on: with
+    // an odd number of stages it meets each in turn with the other group, and waits for those as well.
+    auto wait_mine = [&]() -> bool {
+      const bool mine = turn == group;
+      turn ^= 1;
+      if (mine || (stages & 1)) wait_free();
+      return mine;
+    };
     const uint32_t full0 = map_to_cta(smem_u32(&hdr->full[0]), 0);
     if constexpr (OP != kOpDweight) {
-      constexpr int kQuads = kTileM / kProdWarps / 4;    // G, S: 16 rows a warp
+      constexpr int kQuads = kTileM / kParts / 4;        // G, S: 32 rows a warp
       const int steps = (p.C + kStep - 1) / kStep;
       int t = 0, a_slot = 0;
       for (Walk<OP, PAIR, KEEP> u(p); u.left > 0 && alive; u.next(), ++t) {
@@ -344,26 +359,26 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
         if (!alive) break;
         int row[kQuads][4];
 #pragma unroll
-        for (int q = 0; q < kQuads; ++q) get4(table + static_cast<uint32_t>((t & 1) * kTileM + (warp * kQuads + q) * 4) * 4u, row[q]);
+        for (int q = 0; q < kQuads; ++q) get4(table + static_cast<uint32_t>((t & 1) * kTileM + (part * kQuads + q) * 4) * 4u, row[q]);
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&hdr->ids_empty[t & 1]));
         for (int k = 0; k < steps; ++k) {
-          wait_free();
+          const bool mine = wait_mine();
           if (!alive) break;
           const int slot = at.slot;
           const uint32_t bar = full0 + slot * 8u;
           at.next(stages);
           if (KEEP && u.j > 0) continue;     // (the rows are there; every phase of a barrier has to be waited for all the same)
-          const uint32_t dst = a_tile(KEEP ? a_slot : slot) + static_cast<uint32_t>(warp * kQuads) * 512u;
+          const uint32_t dst = a_tile(KEEP ? a_slot : slot) + static_cast<uint32_t>(part * kQuads) * 512u;
           if (KEEP && ++a_slot == p.a_slots) a_slot = 0;
-          if (elect_one()) {
+          if (mine && elect_one()) {
 #pragma unroll
             for (int q = 0; q < kQuads; ++q) tma_gather4_pair(dst + q * 512u, &map_rows, k * kStep, row[q][0], row[q][1], row[q][2], row[q][3], bar);
           }
         }
       }
     } else {
-      constexpr int kQuads = kStep / kProdWarps / 4;     // 8 rows a warp
+      constexpr int kQuads = kStep / kParts / 4;         // 16 rows a warp
       const uint32_t g_dst = p.swap ? kMTile : 0u, s_dst = p.swap ? 0u : kMTile;
       const int g_seg = p.swap ? nseg : 2, s_seg = p.swap ? 2 : nseg;
       int batch = 0;
@@ -376,34 +391,40 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           if (in_batch == 0) alive = mbar_wait_all(smem_u32(&hdr->ids_full[batch & 1]), (batch >> 1) & 1, abort_flag, p.status.word);
           if (!alive) break;
           int tok[kQuads][4], slot_row[kQuads][4];
-          const uint32_t ids = table + static_cast<uint32_t>((batch & 1) * kBatch + in_batch * kStep + warp * kQuads * 4) * 4u;
+          const uint32_t ids = table + static_cast<uint32_t>((batch & 1) * kBatch + in_batch * kStep + part * kQuads * 4) * 4u;
+          if (turn == group) {
 #pragma unroll
-          for (int q = 0; q < kQuads; ++q) {
-            get4(ids + q * 16u, tok[q]);
-            if (!p.tma_rows) get4(ids + 2u * kBatch * 4u + q * 16u, slot_row[q]);
+            for (int q = 0; q < kQuads; ++q) {
+              get4(ids + q * 16u, tok[q]);
+              if (!p.tma_rows) get4(ids + 2u * kBatch * 4u + q * 16u, slot_row[q]);
+            }
           }
           if (in_batch == kBatchSteps - 1 || k + 1 == steps) {                     // this warp has read the batch
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&hdr->ids_empty[batch & 1]));
             ++batch;
           }
-          wait_free();
+          const bool mine = wait_mine();
           if (!alive) break;
           const uint32_t bar = full0 + at.slot * 8u;
-          const uint32_t dst = ring0 + static_cast<uint32_t>(at.slot) * stage_bytes + static_cast<uint32_t>(warp * kQuads) * 512u;
+          const uint32_t dst = ring0 + static_cast<uint32_t>(at.slot) * stage_bytes + static_cast<uint32_t>(part * kQuads) * 512u;
           at.next(stages);
-          if (elect_one()) {
+          if (mine && elect_one()) {
 #pragma unroll
-            for (int q = 0; q < kQuads; ++q) {
+            for (int s = 0; s < 2; ++s)
+              if (s < g_seg) {
+#pragma unroll
+                for (int q = 0; q < kQuads; ++q)
+                  tma_gather4_pair(dst + g_dst + s * kSeg + q * 512u, &map_w, gx + s * 64, tok[q][0], tok[q][1], tok[q][2], tok[q][3], bar);
+              }
+            if (!p.tma_rows) {
 #pragma unroll
               for (int s = 0; s < 2; ++s)
-                if (s < g_seg) tma_gather4_pair(dst + g_dst + s * kSeg + q * 512u, &map_w, gx + s * 64, tok[q][0], tok[q][1], tok[q][2], tok[q][3], bar);
-              if (!p.tma_rows) {
+                if (s < s_seg) {
 #pragma unroll
-                for (int s = 0; s < 2; ++s)
-                  if (s < s_seg)
+                  for (int q = 0; q < kQuads; ++q)
                     tma_gather4_pair(dst + s_dst + s * kSeg + q * 512u, &map_rows, sx + s * 64, slot_row[q][0], slot_row[q][1], slot_row[q][2], slot_row[q][3], bar);
-              }
+                }
             }
           }
         }
