@@ -196,7 +196,7 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
     if (err != cudaSuccess) return fail_cuda(err, "fill_zero");
     own = true;
   }
-  const bool rounds = plan && n_out <= kRoundInKernel;
+  bool rounds = false;                    // the scatter kernel rounds its float32 rows itself
   auto finish_rows = [&]() -> int {
     if (!f32_rows || rounds) return EGS_OK;
     cudaError_t err = plan ? launch_scatter_finish(plan, acc, Out, n_out, dtype, st)
@@ -213,7 +213,7 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
   }
 
   RowGemmParams p{};
-  p.A = A; p.W = W; p.bias = bias; p.Ind = Ind; p.Out = Out; p.acc = acc; p.plan = plan; p.rounds = rounds ? 1 : 0; p.status = status_ref(status);
+  p.A = A; p.W = W; p.bias = bias; p.Ind = Ind; p.Out = Out; p.acc = acc; p.plan = plan; p.status = status_ref(status);
   p.B = static_cast<int>(d.B); p.T = static_cast<int>(d.T); p.E = static_cast<int>(d.E); p.K = static_cast<int>(d.K);
   p.C = static_cast<int>(d.C); p.N = static_cast<int>(d.N);
   p.M = static_cast<int>(d.B * d.K);
@@ -232,6 +232,8 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
       err = launch_tensor_gather2(p, dtype, smem2, st);
     } else if (dtype != EGS_F32) {
       configure_dense16_rowgemm(p, scatter);
+      rounds = scatter && n_out <= kRoundInKernel && p.tile_group == 0;
+      p.rounds = rounds ? 1 : 0;
       err = launch_dense16_rowgemm(p, scatter, dtype, st);
     } else {
       const size_t smem = configure_tensor_rowgemm(p, scatter);

@@ -713,7 +713,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       }
       if (!released) release();
     }
-    if (OP == kOpScatter && f32_rows && alive && p.rounds) round_rows<T>(p, hdr, ew, lane);
+    if (OP == kOpScatter && !KEEP && f32_rows && alive && p.rounds) round_rows<T>(p, hdr, ew, lane);
     }
   } else if (warp == kMmaWarp) {
     // =========================== MMA issuer ===========================

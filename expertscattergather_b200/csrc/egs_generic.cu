@@ -582,14 +582,39 @@ __global__ void __launch_bounds__(kSumThreads) expert_row_sum_kernel(const T* __
 
 // ------------------------------------------------------------------------------------------------
 // zero fill and fp32 -> dtype conversion
+//
+// Both are bound by memory.  Large buffers are cut into stretches of kStretch (kConvert) vectors a thread with a CTA for each: handed out
+// in order as CTAs leave, the stretches in flight lie together, and 1.07 GB are zeroed in 147 us (7.3 TB/s), 128 MB in 24.6 and 64 MB in 14.3; by a
+// few waves of CTAs that stride over all of it 176, 26.6 and 16.4 us.  24 MB take those 8.3 us, stretches 9.0.  The kernel in front of
+// a 16-bit scatter has more to do in each CTA, and what follows it starts under a grid of few waves only: whole scatters of 134 MB take 172 us
+// with stretches and 170 without, of 268 MB 107 and 113, of 1.07 GB 1340 and 1367.
 // ------------------------------------------------------------------------------------------------
+constexpr int kStretch = 4;
+constexpr int kConvert = 2;                        // ... and twice as many 16-byte loads
+constexpr size_t kManyCtas = 32 << 20, kManyPrepCtas = 160 << 20;     // bytes from which on
+constexpr unsigned kFewCtas = 148 * 8;             // a few waves of the 148 SMs
+
+template <int THREADS>
+__device__ __forceinline__ void fill_vectors(uint4* p, size_t n, bool many) {
+  const uint4 z = make_uint4(0, 0, 0, 0);
+  if (many) {
+    for (size_t b = blockIdx.x; b * (THREADS * kStretch) < n; b += gridDim.x)
+#pragma unroll
+      for (int j = 0; j < kStretch; ++j) {
+        const size_t i = b * (THREADS * kStretch) + j * THREADS + threadIdx.x;
+        if (i < n) p[i] = z;
+      }
+  } else {
+    const size_t stride = static_cast<size_t>(gridDim.x) * THREADS;
+    for (size_t i = static_cast<size_t>(blockIdx.x) * THREADS + threadIdx.x; i < n; i += stride) p[i] = z;
+  }
+}
+
 __global__ void __launch_bounds__(256) fill_zero_kernel(uint4* p16, size_t n16, unsigned char* tail,
                                                        size_t ntail, int early) {
   pdl_wait();
   if (early) pdl_trigger();
-  const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-  const uint4 z = make_uint4(0, 0, 0, 0);
-  for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n16; i += stride) p16[i] = z;
+  fill_vectors<256>(p16, n16, gridDim.x > kFewCtas);
   if (blockIdx.x == 0 && threadIdx.x < ntail) tail[threadIdx.x] = 0;
 }
 
@@ -600,7 +625,18 @@ __global__ void __launch_bounds__(256) fill_zero_bytes_kernel(unsigned char* p, 
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) p[i] = 0;
 }
 
-template <typename T> __device__ __forceinline__ void convert8(const float* src, T* dst);
+// 8 float32 values -> 8 elements of T with vector loads and one 16-byte store (T is a 16-bit type)
+template <typename T>
+__device__ __forceinline__ void store8(const float4& a, const float4& b, T* dst) {
+  T v[8] = {from_f32<T>(a.x), from_f32<T>(a.y), from_f32<T>(a.z), from_f32<T>(a.w),
+            from_f32<T>(b.x), from_f32<T>(b.y), from_f32<T>(b.z), from_f32<T>(b.w)};
+  *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(v);
+}
+template <typename T>
+__device__ __forceinline__ void convert8(const float* src, T* dst) {
+  const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+  store8<T>(a, b, dst);
+}
 
 template <typename T>
 __global__ void __launch_bounds__(256) convert_from_f32_kernel(const float* src, T* dst,
@@ -611,7 +647,26 @@ __global__ void __launch_bounds__(256) convert_from_f32_kernel(const float* src,
   const size_t i0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const bool vec = sizeof(T) == 2 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0;
   const size_t n8 = vec ? n / 8 : 0;
-  for (size_t i = i0; i < n8; i += stride) convert8<T>(src + 8 * i, dst + 8 * i);
+  if (gridDim.x > kFewCtas) {
+    for (size_t b = blockIdx.x; b * (256 * kConvert) < n8; b += gridDim.x) {
+      float4 v[kConvert][2];
+#pragma unroll
+      for (int j = 0; j < kConvert; ++j) {
+        const size_t i = b * (256 * kConvert) + j * 256 + threadIdx.x;
+        if (i < n8) {
+          v[j][0] = *reinterpret_cast<const float4*>(src + 8 * i);
+          v[j][1] = *reinterpret_cast<const float4*>(src + 8 * i + 4);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kConvert; ++j) {
+        const size_t i = b * (256 * kConvert) + j * 256 + threadIdx.x;
+        if (i < n8) store8<T>(v[j][0], v[j][1], dst + 8 * i);
+      }
+    }
+  } else {
+    for (size_t i = i0; i < n8; i += stride) convert8<T>(src + 8 * i, dst + 8 * i);
+  }
   for (size_t i = n8 * 8 + i0; i < n; i += stride) dst[i] = from_f32<T>(src[i]);
 }
 
@@ -681,7 +736,8 @@ __global__ void __launch_bounds__(kPrepThreads) scatter_count_kernel(const void*
   if (threadIdx.x == 0) flags[blockIdx.x] = flag;
 }
 
-template <typename T>
+// COUNT: the CTAs count for themselves (an instance of its own: with the registers that counting takes an SM holds three CTAs, not four)
+template <typename T, bool COUNT>
 __global__ void __launch_bounds__(kPrepThreads) scatter_prepare_kernel(const void* ind, int index_dtype, int B, int T_, int EK,
                                                                        const int* info, const int* flags, int nflags,
                                                                        int limit, int* plan, float* acc,
@@ -698,30 +754,17 @@ __global__ void __launch_bounds__(kPrepThreads) scatter_prepare_kernel(const voi
   } else if (nflags > 0) {
     for (int i = tid; i < nflags; i += kPrepThreads) flag |= flags[i];
     flag = __syncthreads_or(flag);
-  } else if (EK > limit) {
+  } else if (COUNT) {
     flag = B == 1 ? has_hot_row<true>(ind, index_dtype, 0, 1, T_, EK, limit, prep_cnt) : has_hot_row<false>(ind, index_dtype, 0, B, T_, EK, limit, prep_cnt);
   }
   if (blockIdx.x == 0 && tid <= kPlanAdded) plan[tid] = tid == kPlanHot ? flag : 0;
-  const size_t stride = static_cast<size_t>(gridDim.x) * kPrepThreads, i0 = static_cast<size_t>(blockIdx.x) * kPrepThreads + tid;
   // (n is a multiple of 8 elements and both buffers are 16-byte aligned: tensor-core path only)
-  if (flag && zero_output) {
-    float4* a4 = reinterpret_cast<float4*>(acc);
-    for (size_t i = i0; i < n / 4; i += stride) a4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (zero_output) {
+    fill_vectors<kPrepThreads>(flag ? reinterpret_cast<uint4*>(acc) : reinterpret_cast<uint4*>(out), flag ? n / 4 : n / 8, gridDim.x > kFewCtas);
   } else if (flag) {                     // seed the float32 rows with what the output holds
-    for (size_t i = i0; i < n; i += stride) acc[i] = to_f32<T>(out[i]);
-  } else if (zero_output) {
-    uint4* o16 = reinterpret_cast<uint4*>(out);
-    for (size_t i = i0; i < n / 8; i += stride) o16[i] = make_uint4(0, 0, 0, 0);
+    const size_t stride = static_cast<size_t>(gridDim.x) * kPrepThreads;
+    for (size_t i = static_cast<size_t>(blockIdx.x) * kPrepThreads + tid; i < n; i += stride) acc[i] = to_f32<T>(out[i]);
   }
-}
-
-// 8 float32 values -> 8 elements of T with vector loads and one 16-byte store (T is a 16-bit type)
-template <typename T>
-__device__ __forceinline__ void convert8(const float* src, T* dst) {
-  const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
-  T v[8] = {from_f32<T>(a.x), from_f32<T>(a.y), from_f32<T>(a.z), from_f32<T>(a.w),
-            from_f32<T>(b.x), from_f32<T>(b.y), from_f32<T>(b.z), from_f32<T>(b.w)};
-  *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(v);
 }
 
 template <typename T>
@@ -734,10 +777,9 @@ __global__ void __launch_bounds__(256) scatter_finish_kernel(const int* plan, co
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n / 8; i += stride) convert8<T>(acc + 8 * i, out + 8 * i);
 }
 
-int grid_for(size_t work_items, int per_block) {
+int grid_for(size_t work_items, int per_block, bool many = false) {
   size_t blocks = (work_items + per_block - 1) / per_block;
-  const size_t cap = 148 * 8;   // a few waves of the 148 SMs; the kernels use grid-stride loops
-  if (blocks > cap) blocks = cap;
+  if (blocks > kFewCtas && !many) blocks = kFewCtas;
   if (blocks < 1) blocks = 1;
   return static_cast<int>(blocks);
 }
@@ -868,7 +910,7 @@ cudaError_t launch_fill_zero(void* ptr, size_t bytes, cudaStream_t st, bool earl
     err = launch_kernel(fill_zero_bytes_kernel, grid_for(bytes, 256), 256, 0, st, true, static_cast<unsigned char*>(ptr), bytes, early ? 1 : 0);
   } else {
     const size_t n16 = bytes / 16, ntail = bytes % 16;
-    err = launch_kernel(fill_zero_kernel, grid_for(n16, 256 * 4), 256, 0, st, true, static_cast<uint4*>(ptr), n16,
+    err = launch_kernel(fill_zero_kernel, grid_for(n16, 256 * kStretch, bytes > kManyCtas), 256, 0, st, true, static_cast<uint4*>(ptr), n16,
                         static_cast<unsigned char*>(ptr) + n16 * 16, ntail, early ? 1 : 0);
   }
   count_launch();
@@ -877,7 +919,7 @@ cudaError_t launch_fill_zero(void* ptr, size_t bytes, cudaStream_t st, bool earl
 
 cudaError_t launch_convert_from_f32(const float* src, void* dst, size_t n, int dtype, cudaStream_t st, bool early) {
   if (n == 0) return cudaSuccess;
-  const int grid = grid_for(n, 256 * 4);
+  const int grid = n * sizeof(float) > kManyCtas ? grid_for(n, 8 * 256 * kConvert, true) : grid_for(n, 256 * 4);
   cudaError_t err;
   if (dtype == EGS_F16) err = launch_kernel(convert_from_f32_kernel<__half>, grid, 256, 0, st, true, src, static_cast<__half*>(dst), n, early ? 1 : 0);
   else if (dtype == EGS_BF16)
@@ -905,16 +947,19 @@ static cudaError_t prepare(const void* Ind, int index_dtype, int B, int T_, int 
     count_launch();
     if (err != cudaSuccess) return err;
   }
-  // four CTAs per SM, each with at least 4 KB to zero and, where it counts, no more ids than half the elements it zeroes
+  // four CTAs per SM, or as many as there are stretches; each with at least 4 KB to zero and, where it counts, no more ids than half the
+  // elements it zeroes
   size_t grid = 4 * 148;
+  if (zero_output && n * sizeof(T) > kManyPrepCtas && !own_count) grid = (n / 8 + kPrepThreads * kStretch - 1) / (kPrepThreads * kStretch);
   const size_t by_bytes = n * sizeof(T) / 4096, by_count = own_count ? n / (2 * static_cast<size_t>(ids)) : grid;
   if (grid > by_bytes) grid = by_bytes;
   if (grid > by_count) grid = by_count;
   if (grid < 1) grid = 1;
-  if (own_count && smem > 48 * 1024) err = ensure_smem_optin<scatter_prepare_kernel<T>>(kPrepCounters * static_cast<int>(sizeof(int)));
+  if (own_count && smem > 48 * 1024) err = ensure_smem_optin<scatter_prepare_kernel<T, true>>(kPrepCounters * static_cast<int>(sizeof(int)));
   if (err != cudaSuccess) return err;
-  err = launch_kernel(scatter_prepare_kernel<T>, static_cast<unsigned>(grid), kPrepThreads, own_count ? smem : 0, st, true, Ind, index_dtype,
-                      B, T_, EK, info, flags, nflags, limit, plan, acc, static_cast<T*>(out16), n, zero_output, status);
+  err = launch_kernel(own_count ? scatter_prepare_kernel<T, true> : scatter_prepare_kernel<T, false>, static_cast<unsigned>(grid), kPrepThreads,
+                      own_count ? smem : 0, st, true, Ind, index_dtype, B, T_, EK, info, flags, nflags, limit, plan, acc, static_cast<T*>(out16), n,
+                      zero_output, status);
   count_launch();
   return err;
 }
@@ -932,7 +977,7 @@ cudaError_t launch_scatter_prepare(const void* Ind, int index_dtype, int B, int 
 
 cudaError_t launch_scatter_finish(const int* plan, const float* acc, void* out16, size_t n, int dtype, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  const int grid = grid_for(n, 256 * 8 * 4);             // four vectors per thread, a few waves of CTAs at most
+  const int grid = grid_for(n, 256 * 8 * 4);             // a few waves of CTAs: mostly they find nothing to do
   cudaError_t err;
   if (dtype == EGS_F16) err = launch_kernel(scatter_finish_kernel<__half>, grid, 256, 0, st, true, plan, acc, static_cast<__half*>(out16), n);
   else if (dtype == EGS_BF16)
