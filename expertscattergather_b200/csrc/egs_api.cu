@@ -12,7 +12,7 @@
 namespace egs {
 
 static bool encode_tensor_map(TensorMap3* out, const void* base, int elem_bytes, int rank, const unsigned long long* dims, const unsigned* box,
-                              CUtensorMapSwizzle swizzle) {
+                              CUtensorMapSwizzle swizzle, const unsigned long long* strides = nullptr) {
   using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -33,15 +33,15 @@ static bool encode_tensor_map(TensorMap3* out, const void* base, int elem_bytes,
     if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return false;
     has_context = true;
   }
-  if (!encode || !out || !base || rank < 2 || rank > 4) return false;
-  cuuint64_t gdim[4], gstride[3];
-  cuuint32_t bdim[4], estride[4] = {1u, 1u, 1u, 1u};
+  if (!encode || !out || !base || rank < 2 || rank > 5) return false;
+  cuuint64_t gdim[5], gstride[4];
+  cuuint32_t bdim[5], estride[5] = {1u, 1u, 1u, 1u, 1u};
   cuuint64_t pitch = elem_bytes;                         // bytes from one element of dimension i to the next
   for (int i = 0; i < rank; ++i) {
     gdim[i] = dims[i];
     bdim[i] = box[i];
     pitch *= dims[i];
-    if (i + 1 < rank) gstride[i] = pitch;
+    if (i + 1 < rank) gstride[i] = strides ? strides[i] : pitch;
   }
   // integer types: the loads only move bits
   const CUresult rc = encode(reinterpret_cast<CUtensorMap*>(out), elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT32, static_cast<cuuint32_t>(rank), const_cast<void*>(base), gdim,
@@ -51,6 +51,10 @@ static bool encode_tensor_map(TensorMap3* out, const void* base, int elem_bytes,
 }
 bool encode_tensor_map_16bit(TensorMap3* out, const void* base, int rank, const unsigned long long* dims, const unsigned* box) {
   return encode_tensor_map(out, base, 2, rank, dims, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+bool encode_tensor_map_16bit_strided(TensorMap3* out, const void* base, int rank, const unsigned long long* dims, const unsigned long long* strides,
+                                     const unsigned* box) {
+  return encode_tensor_map(out, base, 2, rank, dims, box, CU_TENSOR_MAP_SWIZZLE_128B, strides);
 }
 bool encode_tensor_map_32bit(TensorMap3* out, const void* base, int rank, const unsigned long long* dims, const unsigned* box, int swizzle) {
   return encode_tensor_map(out, base, 4, rank, dims, box,

@@ -105,6 +105,7 @@ struct DenseParams {
   int swap;           // D: 1 = the slot rows' features are the accumulator's rows
   int lane_rows;      // D: 1 = the output's rows are the accumulator's rows
   int tma_rows;       // S, D: slot rows come by TMA
+  int segs_at_once;   // boxes of all 64-column segments of a tile: of the weights [E, C, N], of D's slot rows (see whole_segments)
   int half;           // columns of a tile one CTA stages: BN, or BN / 2 in a pair
   int after_own;      // see launch_kernel
 };
@@ -251,6 +252,21 @@ __device__ __noinline__ void round_rows(const DenseParams& p, DenseHeader* hdr, 
   }
 }
 
+// (PAIR: counted by the leader's barrier, see tma_load_3d_pair)
+template <bool PAIR>
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const void* map, int x, int y, int z, int v, int w, uint32_t bar) {
+  if (PAIR)
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
+        "l"(map), "r"(x), "r"(y), "r"(z), "r"(v), "r"(w), "r"(bar)
+        : "memory");
+  else
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
+        "l"(map), "r"(x), "r"(y), "r"(z), "r"(v), "r"(w), "r"(bar)
+        : "memory");
+}
+
 // KEEP: a scatter whose rows stay for several column tiles (see pick_tile).  An instance of its own: with the slots of kept rows and the
 // walk over both kinds of units in the lanes that issue loads and MMAs, scatters that keep nothing took 3-7 % longer (bf16, 64 experts
 // of 5760 rows, 128 -> 520 features: 181 us without, 193 with).
@@ -324,12 +340,13 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     pdl_wait();                          // (and fall through to the common exit)
   } else if (PAIR && warp < kProdWarps && gathers) {
     // =========================== gather producers of a pair ===========================
-    // Rows come four at a time (tile::gather4).  Two groups of four warps take the stages in turn, a warp a quarter of a stage's rows,
-    // and load them segment by segment: a warp's loads one after the other go to one stretch of shared memory, and what a step costs a
-    // warp beside them - ids, the barrier, coordinates moved to uniform registers - it has two steps' time for.  With eight rows of both
-    // segments in turn for every stage, the gathers alone of a step of D took 860 clocks (with everything else 974, now 800), more than
-    // its MMAs: bf16, 64 experts of 1024 rows, 2048 x 512 features 132 us; eight rows segment by segment 120; in two groups 116.
-    constexpr int kGroups = 2, kParts = kProdWarps / kGroups;
+    // Rows come four at a time (tile::gather4).  In D two groups of four warps take the stages in turn, a warp a quarter of a stage's
+    // rows, and load them segment by segment: a warp's loads one after the other go to one stretch of shared memory, and what a step
+    // costs a warp beside them - ids, the barrier, coordinates moved to uniform registers - it has two steps' time for.  With eight
+    // rows of both segments in turn for every stage, the gathers alone of a step took 860 clocks (with everything else 974, now 800), more
+    // than its MMAs: bf16, 64 experts of 1024 rows, 2048 x 512 features 132 us; eight rows segment by segment 120; in two groups 116.
+    // G and S, whose warps keep their rows for a whole tile, gain nothing from groups.
+    constexpr int kGroups = OP == kOpDweight ? 2 : 1, kParts = kProdWarps / kGroups;
     const int group = warp & (kGroups - 1), part = warp / kGroups;
     const uint32_t table = smem0 + kDenseHeader;
     auto get4 = [](uint32_t a, int (&r)[4]) {
@@ -344,14 +361,14 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     // Whether the stage at `at` is this warp's, and then waits for it.  A warp must not skip phases of a barrier that it waits on: with
     // an odd number of stages it meets each in turn with the other group, and waits for those as well.
     auto wait_mine = [&]() -> bool {
-      const bool mine = turn == group;
+      const bool mine = kGroups == 1 || turn == group;
       turn ^= 1;
       if (mine || (stages & 1)) wait_free();
       return mine;
     };
     const uint32_t full0 = map_to_cta(smem_u32(&hdr->full[0]), 0);
     if constexpr (OP != kOpDweight) {
-      constexpr int kQuads = kTileM / kParts / 4;        // G, S: 32 rows a warp
+      constexpr int kQuads = kTileM / kParts / 4;        // G, S: 16 rows a warp
       const int steps = (p.C + kStep - 1) / kStep;
       int t = 0, a_slot = 0;
       for (Walk<OP, PAIR, KEEP> u(p); u.left > 0 && alive; u.next(), ++t) {
@@ -867,6 +884,9 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
             if (OP == kOpScatter && p.tma_rows && rows_too) box4(KEEP ? a_tile(a_slot) : base, c0);
             if (p.nc) {
               box3(base + kMTile, c0, n0);
+            } else if (p.segs_at_once) {
+              if (PAIR) tma_load_4d_pair(base + kMTile, &map_w, 0, c0, n0 >> 6, u.e, bar);
+              else tma_load_4d(base + kMTile, &map_w, 0, c0, n0 >> 6, u.e, bar);
             } else {
 #pragma unroll
               for (int s = 0; s < 4; ++s)
@@ -875,9 +895,13 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           } else if (p.tma_rows) {
             const int ns = p.swap ? 2 : nseg, x0 = p.swap ? u.m0 : n0;
             const uint32_t dst = base + (p.swap ? 0u : kMTile);
+            if (p.segs_at_once) {
+              tma_load_5d<PAIR>(dst, &map_rows, 0, k, b, x0 >> 6, u.e, bar);
+            } else {
 #pragma unroll
-            for (int s = 0; s < 4; ++s)
-              if (s < ns) box4(dst + s * kSeg, x0 + s * 64);
+              for (int s = 0; s < 4; ++s)
+                if (s < ns) box4(dst + s * kSeg, x0 + s * 64);
+            }
           }
         }
         if (KEEP && rows_too && ++a_slot == p.a_slots) a_slot = 0;
@@ -932,6 +956,11 @@ bool encode_slot_rows(TensorMap3* map, const void* base, int B, int E, int K, in
   const unsigned box[4] = {64u, kk, 1u, static_cast<unsigned>(rows) / kk};
   return encode_tensor_map_16bit(map, base, 4, dims, box);
 }
+
+// A tile whose rows are contraction elements comes 64 columns at a time, which is as wide as a swizzled box gets.  Seen as [rows, 64] matrices
+// side by side, the segments of a tile are one box of several of them, where segments are whole and a CTA's columns begin with one: one
+// load instead of two or four (bf16, G of 262144 rows of 64 experts, 1024 -> 256 features 114 -> 109 us, of 65536 rows, 2048 -> 512 104 -> 101).
+bool whole_segments(int width, int staged, bool pair) { return staged % 64 == 0 && width % (pair ? 128 : 64) == 0; }
 
 // One CTA per tile of 128 x BN or a pair of CTAs per tile of 256 x BN, and BN, by clocks.  A step writes and reads 128 + `staged`
 // rows of 128 bytes of a CTA's shared memory, 2 clocks a row at 128 bytes a clock (measured: 2.0 in pairs, 2.4 on single CTAs, 2.6 for
@@ -1104,7 +1133,14 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
   const unsigned long long inner = p.nc ? r.C : r.N, outer = p.nc ? r.N : r.C;
   const unsigned long long dims[3] = {inner, outer, static_cast<unsigned long long>(r.E)};
   const unsigned box[3] = {64u, p.nc ? static_cast<unsigned>(p.half) : static_cast<unsigned>(kStep), 1u};
-  if (!encode_tensor_map_16bit(&mw, r.W, 3, dims, box)) return cudaErrorInvalidValue;
+  p.segs_at_once = !p.nc && whole_segments(r.N, p.half, r.pair != 0);
+  if (p.segs_at_once) {
+    const unsigned long long segs[4] = {64ull, outer, inner / 64, static_cast<unsigned long long>(r.E)}, strides[3] = {inner * 2, 128ull, inner * outer * 2};
+    const unsigned seg_box[4] = {64u, static_cast<unsigned>(kStep), static_cast<unsigned>(p.half / 64), 1u};
+    if (!encode_tensor_map_16bit_strided(&mw, r.W, 4, segs, strides, seg_box)) return cudaErrorInvalidValue;
+  } else if (!encode_tensor_map_16bit(&mw, r.W, 3, dims, box)) {
+    return cudaErrorInvalidValue;
+  }
   p.tma_rows = r.slot_boxes;
   if (p.tma_rows && !encode_slot_rows(&mr, r.A, r.B, r.E, r.K, r.C, 128)) return cudaErrorInvalidValue;
   if (r.pair && !p.tma_rows &&
@@ -1185,7 +1221,17 @@ cudaError_t launch_dense16_dweight(const DWeightParams& r, int dtype, cudaStream
   plan_walk(p, r.pair != 0);
   TensorMap3 mw{}, mr{};
   p.tma_rows = r.slot_boxes;
-  if (p.tma_rows && !encode_slot_rows(&mr, r.Ysrc, r.B, r.E, r.K, r.FD, kStep)) return cudaErrorInvalidValue;
+  const int staged = r.swap ? kTileM : p.half;                 // columns of the slot rows that a CTA stages
+  p.segs_at_once = p.tma_rows && whole_segments(r.FD, staged, !r.swap && r.pair);
+  if (p.segs_at_once) {
+    const unsigned long long kk = static_cast<unsigned long long>(r.K), fd = static_cast<unsigned long long>(r.FD), e = static_cast<unsigned long long>(r.E);
+    const unsigned rows_k = static_cast<unsigned>(r.K < kStep ? r.K : kStep);
+    const unsigned long long segs[5] = {64ull, kk, static_cast<unsigned long long>(r.B), fd / 64, e}, strides[4] = {fd * 2, e * kk * fd * 2, 128ull, kk * fd * 2};
+    const unsigned seg_box[5] = {64u, rows_k, static_cast<unsigned>(kStep) / rows_k, static_cast<unsigned>(staged / 64), 1u};
+    if (!encode_tensor_map_16bit_strided(&mr, r.Ysrc, 5, segs, strides, seg_box)) return cudaErrorInvalidValue;
+  } else if (p.tma_rows && !encode_slot_rows(&mr, r.Ysrc, r.B, r.E, r.K, r.FD, kStep)) {
+    return cudaErrorInvalidValue;
+  }
   if (r.pair && (!encode_gather(&mw, r.Xsrc, static_cast<long long>(r.B) * r.T, r.FG) ||
                  (!p.tma_rows && !encode_gather(&mr, r.Ysrc, static_cast<long long>(r.M) * r.E, r.FD))))
     return cudaErrorInvalidValue;

@@ -211,6 +211,9 @@ struct alignas(64) TensorMap3 {
   unsigned char bytes[128];
 };
 bool encode_tensor_map_16bit(TensorMap3* out, const void* base, int rank, const unsigned long long* dims, const unsigned* box);
+// ... of up to five dimensions whose strides (bytes, of all but the first) are given
+bool encode_tensor_map_16bit_strided(TensorMap3* out, const void* base, int rank, const unsigned long long* dims, const unsigned long long* strides,
+                                     const unsigned* box);
 // The same for 32-bit elements.  kMapSwizzle128Base32: the XOR of the 128-byte swizzle acts on 32-byte pairs of chunks with the row modulo 4.
 enum { kMapSwizzleNone = 0, kMapSwizzle128 = 1, kMapSwizzle128Base32 = 2 };
 bool encode_tensor_map_32bit(TensorMap3* out, const void* base, int rank, const unsigned long long* dims, const unsigned* box, int swizzle);
