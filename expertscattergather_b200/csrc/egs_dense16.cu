@@ -965,7 +965,12 @@ bool whole_segments(int width, int staged, bool pair) { return staged % 64 == 0 
 // One CTA per tile of 128 x BN or a pair of CTAs per tile of 256 x BN, and BN, by clocks.  A step writes and reads 128 + `staged`
 // rows of 128 bytes of a CTA's shared memory, 2 clocks a row at 128 bytes a clock (measured: 2.0 in pairs, 2.4 on single CTAs, 2.6 for
 // their scatters), the tensor core multiplies BN columns in 2 * BN clocks, the load/store unit needs lsu0 + lsu1 * staged for its
-// share of the copies, and the barriers of a step take 600 (800 in a scatter that gathers its rows).  Read-out takes epi clocks a
+// share of the copies, and the barriers of a step take 600 (800 in a scatter that gathers its rows).  In G the copies of single CTAs, handed over
+// by their threads, hold a step up to 750 where there is more than one wave of them, and a pair's gathers beside less than 64 columns to
+// 850 (weights [E, N, C]: 750).  With 600 there all of these stayed on single CTAs: 512 rows of 256 experts, 512 -> 128 features, 33.3 us, on
+// pairs 30.3; 5724 of 10, 1056 -> 136, 41.5 and 37.4; 4515 of 45, 864 -> 104, 84 and 65; and these still do: 254 of 234, 592 -> 40, 21.3 and 23.1;
+// 104 of 10, 1408 -> 88, 12.6 and 13.3.  Of 320 calls of G, sizes drawn, the 50 that went to pairs take 0.74 to 1.04 of the time, 0.92 in the mean.
+// Read-out takes epi clocks a
 // column beside the next tile's main loop; the additions of a scatter share the way to the L2 with the loads, and half of the shorter
 // one shows.  Units go out in waves of one per SM or pair of SMs; a pair starts and ends 2500 clocks slower.
 //
@@ -1010,17 +1015,19 @@ Ring fit_scatter(int half, bool nc_tile, bool boxes, int keep) {
   if (r.stages < 4) r.stages = 0;
   return r;
 }
-Tile pick_tile(int n, int m, long long groups, int steps, double lsu0, double lsu1, double epi, bool scatter, bool nc_tile = false) {
+Tile pick_tile(int n, int m, long long groups, int steps, double lsu0, double lsu1, double epi, bool scatter, bool nc_tile = false, bool gather = false) {
   Tile best, stay;                       // units of one tile; rows that stay
   for (int pair = 0; pair < 2; ++pair) {
     const int rows = pair ? 2 * kTileM : kTileM, sms = pair ? kSms / 2 : kSms, unit16 = pair ? 32 : 16;
-    const double per_row = pair ? 2.0 : scatter ? 2.6 : 2.4, least = scatter && lsu0 > 0.0 ? 800.0 : 600.0;
+    const double per_row = pair ? 2.0 : scatter ? 2.6 : 2.4;
     const long long row_units = (m + rows - 1) / rows * groups;
     const int top = n < 256 ? (n + unit16 - 1) / unit16 * unit16 : 256;
     const bool boxes = lsu0 == 0.0;
     for (int bn = top; bn >= unit16; bn -= unit16) {
       const long long tiles = (n + bn - 1) / bn;
       const int staged = pair ? bn / 2 : bn;
+      const long long units = row_units * tiles, waves = (units + sms - 1) / sms;
+      const double least = scatter && lsu0 > 0.0 ? 800.0 : !gather ? 600.0 : pair ? (std::min(bn, n) >= 64 ? 600.0 : nc_tile ? 750.0 : 850.0) : waves > 1 ? 750.0 : 600.0;
       double step = per_row * (128 + staged);
       if (2.0 * bn > step) step = 2.0 * bn;
       if (lsu0 + lsu1 * staged > step) step = lsu0 + lsu1 * staged;
@@ -1035,7 +1042,6 @@ Tile pick_tile(int n, int m, long long groups, int steps, double lsu0, double ls
         to.pair = pair != 0;
         to.cost = cost;
       };
-      const long long units = row_units * tiles, waves = (units + sms - 1) / sms;
       consider(best, waves * (more + 0.5 * less + 1000) + ends, 0, 0);
       // Rows that stay: whole waves of row blocks, and the rest in one to eight units a row block.  At best that is as if all tiles
       // were spread evenly, which most widths need not be looked at further for.
@@ -1093,7 +1099,7 @@ void configure_dense16_rowgemm(RowGemmParams& p, bool scatter) {
   const int steps = (p.C + kStep - 1) / kStep;
   const bool cp_rows = !scatter || !rows_fit_boxes(p.K, 128);
   const bool nc = p.w_layout == EGS_W_NC;
-  const Tile t = pick_tile(p.N, p.M, p.E, steps, cp_rows ? 340.0 : 0.0, 0.0, 16.0, scatter, nc);
+  const Tile t = pick_tile(p.N, p.M, p.E, steps, cp_rows ? 340.0 : 0.0, 0.0, 16.0, scatter, nc, !scatter);
   p.BN = t.bn;
   p.pair = t.pair ? 1 : 0;
   p.tile_group = t.group;

@@ -585,13 +585,13 @@ __global__ void __launch_bounds__(kSumThreads) expert_row_sum_kernel(const T* __
 //
 // Both are bound by memory.  Large buffers are cut into stretches of kStretch (kConvert) vectors a thread with a CTA for each: handed out
 // in order as CTAs leave, the stretches in flight lie together, and 1.07 GB are zeroed in 147 us (7.3 TB/s), 128 MB in 24.6 and 64 MB in 14.3; by a
-// few waves of CTAs that stride over all of it 176, 26.6 and 16.4 us.  24 MB take those 8.3 us, stretches 9.0.  The kernel in front of
-// a 16-bit scatter has more to do in each CTA, and what follows it starts under a grid of few waves only: whole scatters of 134 MB take 172 us
-// with stretches and 170 without, of 268 MB 107 and 113, of 1.07 GB 1340 and 1367.
+// few waves of CTAs that stride over all of it 176, 26.6 and 16.4 us.  24 MB take those 8.3 us, stretches 9.0.  Where a kernel starts under the
+// fill it does so under a grid of few waves only, and the fill in front of a 16-bit scatter has more to do in each CTA: whole scatters of
+// 134 MB take 172 us with stretches and 170 without, of 268 MB 107 and 113, of 1.07 GB 1340 and 1367.
 // ------------------------------------------------------------------------------------------------
 constexpr int kStretch = 4;
 constexpr int kConvert = 2;                        // ... and twice as many 16-byte loads
-constexpr size_t kManyCtas = 32 << 20, kManyPrepCtas = 160 << 20;     // bytes from which on
+constexpr size_t kManyCtas = 32 << 20, kManyEarly = 160 << 20;     // bytes from which on; where dependents start early
 constexpr unsigned kFewCtas = 148 * 8;             // a few waves of the 148 SMs
 
 template <int THREADS>
@@ -910,7 +910,7 @@ cudaError_t launch_fill_zero(void* ptr, size_t bytes, cudaStream_t st, bool earl
     err = launch_kernel(fill_zero_bytes_kernel, grid_for(bytes, 256), 256, 0, st, true, static_cast<unsigned char*>(ptr), bytes, early ? 1 : 0);
   } else {
     const size_t n16 = bytes / 16, ntail = bytes % 16;
-    err = launch_kernel(fill_zero_kernel, grid_for(n16, 256 * kStretch, bytes > kManyCtas), 256, 0, st, true, static_cast<uint4*>(ptr), n16,
+    err = launch_kernel(fill_zero_kernel, grid_for(n16, 256 * kStretch, bytes > (early ? kManyEarly : kManyCtas)), 256, 0, st, true, static_cast<uint4*>(ptr), n16,
                         static_cast<unsigned char*>(ptr) + n16 * 16, ntail, early ? 1 : 0);
   }
   count_launch();
@@ -950,7 +950,7 @@ static cudaError_t prepare(const void* Ind, int index_dtype, int B, int T_, int 
   // four CTAs per SM, or as many as there are stretches; each with at least 4 KB to zero and, where it counts, no more ids than half the
   // elements it zeroes
   size_t grid = 4 * 148;
-  if (zero_output && n * sizeof(T) > kManyPrepCtas && !own_count) grid = (n / 8 + kPrepThreads * kStretch - 1) / (kPrepThreads * kStretch);
+  if (zero_output && n * sizeof(T) > kManyEarly && !own_count) grid = (n / 8 + kPrepThreads * kStretch - 1) / (kPrepThreads * kStretch);
   const size_t by_bytes = n * sizeof(T) / 4096, by_count = own_count ? n / (2 * static_cast<size_t>(ids)) : grid;
   if (grid > by_bytes) grid = by_bytes;
   if (grid > by_count) grid = by_count;
