@@ -279,11 +279,12 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
   const uint32_t epi0 = smem0 + kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : kRowTable);
   const bool gathers = OP != kOpScatter || !p.tma_rows;
   const bool has_cp = !PAIR && gathers;
-  const bool has_tma = PAIR || OP != kOpDweight || p.tma_rows;          // (in a pair it also announces what the producers gather)
   const int readers = p.readers;                                        // read-out warps: producers with nothing to gather may join
   const uint32_t ring0 = epi0 + epi_bytes(readers > kEpiWarps);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool leader = !PAIR || (blockIdx.x & 1) == 0;
+  // (in a pair the leader's also announces what the producers gather; a warp without a part in a stage must not follow the ring, see is_mine)
+  const bool has_tma = OP != kOpDweight || p.tma_rows || (PAIR && leader);
   const int nseg = (p.half + 63) >> 6;
   const uint32_t n_bytes = (OP != kOpDweight && p.nc) ? static_cast<uint32_t>(p.half) * 128u : static_cast<uint32_t>(nseg) * kSeg;
   const uint32_t stage_bytes = kMTile + n_bytes;
@@ -298,7 +299,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
 
   if (tid == 0) {
     for (int s = 0; s < kMaxStages; ++s) {
-      mbar_init(smem_u32(&hdr->full[s]), (has_cp ? kProdThreads : 0) + (has_tma ? 1 : 0));      // (a pair's: the leader's copy is used)
+      mbar_init(smem_u32(&hdr->full[s]), (has_cp ? kProdThreads : 0) + (PAIR || has_tma ? 1 : 0));      // (a pair's: the leader's copy is used)
       mbar_init(smem_u32(&hdr->empty[s]), 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -340,8 +341,8 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     pdl_wait();                          // (and fall through to the common exit)
   } else if (PAIR && warp < kProdWarps && gathers) {
     // =========================== gather producers of a pair ===========================
-    // Rows come four at a time (tile::gather4).  In D two groups of four warps take the stages in turn, a warp a quarter of a stage's
-    // rows, and load them segment by segment: a warp's loads one after the other go to one stretch of shared memory, and what a step
+    // Rows come four at a time (tile::gather4).  In D two groups of four warps share the stages, a warp has a quarter of a stage's
+    // rows, and loads them segment by segment: a warp's loads one after the other go to one stretch of shared memory, and what a step
     // costs a warp beside them - ids, the barrier, coordinates moved to uniform registers - it has two steps' time for.  With eight
     // rows of both segments in turn for every stage, the gathers alone of a step took 860 clocks (with everything else 974, now 800), more
     // than its MMAs: bf16, 64 experts of 1024 rows, 2048 x 512 features 132 us; eight rows segment by segment 120; in two groups 116.
@@ -354,18 +355,13 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     };
     Cursor at;
     bool alive = true;
-    int turn = 0;
     auto wait_free = [&]() {             // for the stage at `at`; its barrier (the leader's) and its first byte here; moves on
       if (at.round > 0) alive = mbar_wait_all(smem_u32(&hdr->empty[at.slot]), (at.round - 1) & 1, abort_flag, p.status.word);
     };
-    // Whether the stage at `at` is this warp's, and then waits for it.  A warp must not skip phases of a barrier that it waits on: with
-    // an odd number of stages it meets each in turn with the other group, and waits for those as well.
-    auto wait_mine = [&]() -> bool {
-      const bool mine = kGroups == 1 || turn == group;
-      turn ^= 1;
-      if (mine || (stages & 1)) wait_free();
-      return mine;
-    };
+    // Whether the stage at `at` is this warp's.  A group has every other slot of the ring, not every other step: with an odd number of stages
+    // the groups would meet each barrier in turn, and a warp that is late to look at a phase whose stage another group loads finds the one
+    // after it done as well, which a parity cannot tell from neither being done.
+    auto is_mine = [&]() { return kGroups == 1 || (at.slot & (kGroups - 1)) == group; };
     const uint32_t full0 = map_to_cta(smem_u32(&hdr->full[0]), 0);
     if constexpr (OP != kOpDweight) {
       constexpr int kQuads = kTileM / kParts / 4;        // G, S: 16 rows a warp
@@ -380,7 +376,8 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&hdr->ids_empty[t & 1]));
         for (int k = 0; k < steps; ++k) {
-          const bool mine = wait_mine();
+          const bool mine = is_mine();
+          if (mine) wait_free();
           if (!alive) break;
           const int slot = at.slot;
           const uint32_t bar = full0 + slot * 8u;
@@ -409,7 +406,8 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           if (!alive) break;
           int tok[kQuads][4], slot_row[kQuads][4];
           const uint32_t ids = table + static_cast<uint32_t>((batch & 1) * kBatch + in_batch * kStep + part * kQuads * 4) * 4u;
-          if (turn == group) {
+          const bool mine = is_mine();
+          if (mine) {
 #pragma unroll
             for (int q = 0; q < kQuads; ++q) {
               get4(ids + q * 16u, tok[q]);
@@ -421,7 +419,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
             if (lane == 0) mbar_arrive(smem_u32(&hdr->ids_empty[batch & 1]));
             ++batch;
           }
-          const bool mine = wait_mine();
+          if (mine) wait_free();
           if (!alive) break;
           const uint32_t bar = full0 + at.slot * 8u;
           const uint32_t dst = ring0 + static_cast<uint32_t>(at.slot) * stage_bytes + static_cast<uint32_t>(part * kQuads) * 512u;

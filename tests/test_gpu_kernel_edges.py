@@ -312,6 +312,27 @@ def test_dense16_dweight_sums_long_contractions_in_ranges(cuda_device, B, T, E, 
     assert torch.stack(bias).mean().abs().item() <= 8192 / 16 * 2.0 ** -23
 
 
+# weight gradients on pairs whose slot rows are gathered too, with an odd and an even number of stages (two groups of warps share the ring's
+# slots), widths whose last tile is narrow, ranges that end within a batch of ids.  Small integers: exact in float32, then rounded once.
+@pytest.mark.parametrize("B,T,E,K,FG,FD,stages", [(9, 300, 24, 101, 1000, 200, 5), (39, 80, 13, 21, 1936, 344, 5), (20, 90, 74, 45, 512, 520, 5), (15, 200, 74, 64, 512, 512, 6)])
+@pytest.mark.parametrize("out_layout", ["gathered_rows", "direct_rows"])
+def test_dense16_dweight_groups_share_the_ring(cuda_device, B, T, E, K, FG, FD, stages, out_layout):
+    plan = ops.describe_plan("D", B, T, E, K, FG, FD, torch.bfloat16)
+    assert plan["pair"] == 1 and plan["splits"] == 1 and plan["stages"] == stages, plan
+    g = torch.Generator().manual_seed(FG)
+    X = torch.randint(-2, 3, (B, T, FG), generator=g).to(torch.bfloat16)
+    Y = torch.randint(-2, 3, (B, E, K, FD), generator=g).to(torch.bfloat16)
+    Ind = torch.randint(0, T, (B, E, K), generator=g)
+    ref = torch.from_numpy(orc.np_dweight(X, Y, Ind))
+    if out_layout == "direct_rows":
+        ref = ref.transpose(1, 2)
+    d = [t.to(cuda_device) for t in (X, Y, Ind)]
+    for _ in range(10):
+        got = ops.dweight(*d, out_layout=out_layout)
+    ops.check_status()
+    assert torch.equal(got.cpu(), ref.to(torch.bfloat16))
+
+
 # the first CUDA call of a thread: boxes are described to the driver before anything else has made a context current there
 @pytest.mark.parametrize("op", ["G", "S", "D"])
 def test_dense16_first_call_of_a_thread(cuda_device, op):
