@@ -28,9 +28,9 @@
 // instruction (320 a stage of G), side by side with the TMA unit; a pair's gathers take the TMA units about as long.  Everything else has to stay out of the way: a satisfied barrier
 // wait takes 150 clocks and every dependent instruction of a lone warp 5-10, so nothing on a per-stage or per-tile path divides, the
 // issuing warps run converged (see mbar_wait_all) and ids are looked up elsewhere.
-// T=1024, E=64, K=64, I=1024, J=256, bf16: B=64 G 126-138 us, D 148-165; B=512, under the power cap, G 850-990 us, dY (weights [E, N, C]) 840-900 = 1.23
-// PFLOP/s, D 1050-1200.  S as whole calls, its rows loaded for every column tile and kept, in turn: B=64 194 and 185 us, weights [E, N, C] 193 and
-// 185; B=512 1450 and 1361, 1577 and 1455 (about 200 of that fills the output).
+// T=1024, E=64, K=64, I=1024, J=256, bf16: B=64 G and dY (weights [E, N, C]) 105-110 us, D 119-123 (138 before its gathers came in groups, segment by
+// segment); B=512, under the power cap, G and dY 850-950 us = 1.15-1.3 PFLOP/s, D 1050-1150.  S as whole calls: B=64 174 us, B=512 1340, 150 of which
+// fill the output (its rows loaded for every column tile instead of kept: 194 and 1450 before that fill took 30 us less).
 #include <algorithm>
 #include <type_traits>
 
@@ -105,7 +105,7 @@ struct DenseParams {
   int swap;           // D: 1 = the slot rows' features are the accumulator's rows
   int lane_rows;      // D: 1 = the output's rows are the accumulator's rows
   int tma_rows;       // S, D: slot rows come by TMA
-  int segs_at_once;   // boxes of all 64-column segments of a tile: of the weights [E, C, N], of D's slot rows (see whole_segments)
+  int whole, boxes;   // weights [E, C, N], D's slot rows: boxes of all 64-column segments of a tile (see whole_segments), boxes of a tile
   int half;           // columns of a tile one CTA stages: BN, or BN / 2 in a pair
   int after_own;      // see launch_kernel
 };
@@ -857,6 +857,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     for (Walk<OP, PAIR, KEEP> u(p); u.left > 0 && ok; u.next()) {
       const int steps = u.steps();
       const int n0 = u.first_column();
+      const int column = OP == kOpDweight && p.swap ? u.m0 : n0, x0 = p.whole ? 0 : column, z0 = p.whole ? column >> 6 : 0;
       const bool rows_too = !KEEP || u.j == 0;       // a scatter's row block is loaded with its first column tile
       int m = OP == kOpDweight ? u.split * p.rows_per_split : u.m0;
       int b = p.by_k.quotient(m), k = m - b * p.K;     // first slot row of the step
@@ -882,24 +883,19 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
             if (OP == kOpScatter && p.tma_rows && rows_too) box4(KEEP ? a_tile(a_slot) : base, c0);
             if (p.nc) {
               box3(base + kMTile, c0, n0);
-            } else if (p.segs_at_once) {
-              if (PAIR) tma_load_4d_pair(base + kMTile, &map_w, 0, c0, n0 >> 6, u.e, bar);
-              else tma_load_4d(base + kMTile, &map_w, 0, c0, n0 >> 6, u.e, bar);
             } else {
 #pragma unroll
               for (int s = 0; s < 4; ++s)
-                if (s < nseg) box3(base + kMTile + s * kSeg, n0 + s * 64, c0);
+                if (s < p.boxes) {
+                  if (PAIR) tma_load_4d_pair(base + kMTile + s * kSeg, &map_w, x0 + s * 64, c0, z0, u.e, bar);
+                  else tma_load_4d(base + kMTile + s * kSeg, &map_w, x0 + s * 64, c0, z0, u.e, bar);
+                }
             }
           } else if (p.tma_rows) {
-            const int ns = p.swap ? 2 : nseg, x0 = p.swap ? u.m0 : n0;
             const uint32_t dst = base + (p.swap ? 0u : kMTile);
-            if (p.segs_at_once) {
-              tma_load_5d<PAIR>(dst, &map_rows, 0, k, b, x0 >> 6, u.e, bar);
-            } else {
 #pragma unroll
-              for (int s = 0; s < 4; ++s)
-                if (s < ns) box4(dst + s * kSeg, x0 + s * 64);
-            }
+            for (int s = 0; s < 4; ++s)
+              if (s < p.boxes) tma_load_5d<PAIR>(dst + s * kSeg, &map_rows, x0 + s * 64, k, b, z0, u.e, bar);
           }
         }
         if (KEEP && rows_too && ++a_slot == p.a_slots) a_slot = 0;
@@ -1137,13 +1133,15 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
   const unsigned long long inner = p.nc ? r.C : r.N, outer = p.nc ? r.N : r.C;
   const unsigned long long dims[3] = {inner, outer, static_cast<unsigned long long>(r.E)};
   const unsigned box[3] = {64u, p.nc ? static_cast<unsigned>(p.half) : static_cast<unsigned>(kStep), 1u};
-  p.segs_at_once = !p.nc && whole_segments(r.N, p.half, r.pair != 0);
-  if (p.segs_at_once) {
-    const unsigned long long segs[4] = {64ull, outer, inner / 64, static_cast<unsigned long long>(r.E)}, strides[3] = {inner * 2, 128ull, inner * outer * 2};
-    const unsigned seg_box[4] = {64u, static_cast<unsigned>(kStep), static_cast<unsigned>(p.half / 64), 1u};
+  if (p.nc) {
+    if (!encode_tensor_map_16bit(&mw, r.W, 3, dims, box)) return cudaErrorInvalidValue;
+  } else {
+    p.whole = whole_segments(r.N, p.half, r.pair != 0);
+    p.boxes = p.whole ? 1 : (p.half + 63) / 64;
+    const unsigned long long segs[4] = {p.whole ? 64ull : inner, outer, p.whole ? inner / 64 : 1ull, static_cast<unsigned long long>(r.E)};
+    const unsigned long long strides[3] = {inner * 2, 128ull, inner * outer * 2};
+    const unsigned seg_box[4] = {64u, static_cast<unsigned>(kStep), p.whole ? static_cast<unsigned>(p.half / 64) : 1u, 1u};
     if (!encode_tensor_map_16bit_strided(&mw, r.W, 4, segs, strides, seg_box)) return cudaErrorInvalidValue;
-  } else if (!encode_tensor_map_16bit(&mw, r.W, 3, dims, box)) {
-    return cudaErrorInvalidValue;
   }
   p.tma_rows = r.slot_boxes;
   if (p.tma_rows && !encode_slot_rows(&mr, r.A, r.B, r.E, r.K, r.C, 128)) return cudaErrorInvalidValue;
@@ -1225,16 +1223,16 @@ cudaError_t launch_dense16_dweight(const DWeightParams& r, int dtype, cudaStream
   plan_walk(p, r.pair != 0);
   TensorMap3 mw{}, mr{};
   p.tma_rows = r.slot_boxes;
-  const int staged = r.swap ? kTileM : p.half;                 // columns of the slot rows that a CTA stages
-  p.segs_at_once = p.tma_rows && whole_segments(r.FD, staged, !r.swap && r.pair);
-  if (p.segs_at_once) {
+  if (p.tma_rows) {
+    const int staged = r.swap ? kTileM : p.half;               // columns of the slot rows that a CTA stages
+    p.whole = whole_segments(r.FD, staged, !r.swap && r.pair);
+    p.boxes = p.whole ? 1 : (staged + 63) / 64;
     const unsigned long long kk = static_cast<unsigned long long>(r.K), fd = static_cast<unsigned long long>(r.FD), e = static_cast<unsigned long long>(r.E);
     const unsigned rows_k = static_cast<unsigned>(r.K < kStep ? r.K : kStep);
-    const unsigned long long segs[5] = {64ull, kk, static_cast<unsigned long long>(r.B), fd / 64, e}, strides[4] = {fd * 2, e * kk * fd * 2, 128ull, kk * fd * 2};
-    const unsigned seg_box[5] = {64u, rows_k, static_cast<unsigned>(kStep) / rows_k, static_cast<unsigned>(staged / 64), 1u};
+    const unsigned long long segs[5] = {p.whole ? 64ull : fd, kk, static_cast<unsigned long long>(r.B), p.whole ? fd / 64 : 1ull, e};
+    const unsigned long long strides[4] = {fd * 2, e * kk * fd * 2, 128ull, kk * fd * 2};
+    const unsigned seg_box[5] = {64u, rows_k, static_cast<unsigned>(kStep) / rows_k, p.whole ? static_cast<unsigned>(staged / 64) : 1u, 1u};
     if (!encode_tensor_map_16bit_strided(&mr, r.Ysrc, 5, segs, strides, seg_box)) return cudaErrorInvalidValue;
-  } else if (p.tma_rows && !encode_slot_rows(&mr, r.Ysrc, r.B, r.E, r.K, r.FD, kStep)) {
-    return cudaErrorInvalidValue;
   }
   if (r.pair && (!encode_gather(&mw, r.Xsrc, static_cast<long long>(r.B) * r.T, r.FG) ||
                  (!p.tma_rows && !encode_gather(&mr, r.Ysrc, static_cast<long long>(r.M) * r.E, r.FD))))

@@ -683,7 +683,7 @@ __global__ void __launch_bounds__(256) convert_to_f32_kernel(const T* src, float
 // Adding straight into a bf16/fp16 output rounds at every addition, which is accurate enough only while few
 // contributions meet in one token row; summing in float32 rows and rounding once is always accurate but costs
 // a float32 fill, float32 atomics on a buffer twice the size and a conversion pass.  The choice is made on the
-// device, per call, from the actual indices: *plan != 0 selects the float32 rows.  One hot row anywhere selects them for every row
+// device, per call, from the actual indices: a plan's kPlanHot selects the float32 rows.  One hot row anywhere selects them for every row
 // of the call, so that what a row is summed in does not depend on its own luck alone.
 // The ids of a batch element are counted in shared memory by one CTA (4096 ids: about 2 us) of a kernel of their own, with a flag
 // per CTA; the kernel that zeroes what the additions go to starts under it (dependent launch) and collects the flags: 2 us of the
