@@ -108,6 +108,7 @@ struct DenseParams {
   int whole, boxes;   // weights [E, C, N], D's slot rows: boxes of all 64-column segments of a tile (see whole_segments), boxes of a tile
   int half;           // columns of a tile one CTA stages: BN, or BN / 2 in a pair
   int after_own;      // see launch_kernel
+  int tail, tail_bn;                     // G, D on pairs: units of half a tile in the last wave (0: none), width of the first half (see plan_tail)
 };
 
 // Position in the stage ring.
@@ -124,6 +125,7 @@ struct Cursor {
 // The tiles of a CTA or pair.  A unit is a number in a mixed radix - column tile; row block of a group, expert, group (G, S) or row block,
 // row range, expert (D) - units go out `stride` apart and are advanced by adding the stride's digits: three divisions a unit (1000
 // clocks and more) in the lanes that feed the tensor core were a fifth of the time of a tile with eight steps.
+// The last wave of G and D on pairs may be units of half a tile (see plan_tail).
 // A scatter whose rows may stay has units of several column tiles: all of a row block's for as many whole waves as there are, and
 // groups of them, so that the last wave is even, for the row blocks that are left.
 template <int OP, bool PAIR, bool KEEP>
@@ -132,19 +134,23 @@ struct Walk {
   int m0, n0, e, split;        // this CTA's 128 rows, the first column of the tile, expert, row range
   int j, tiles, tile;          // tiles of the unit before this one, its tiles, this one's place among them
   int full, d0, d1, d2, d3;
+  int bn;                      // width of the unit's tile
   const DenseParams& p;
+  static constexpr bool kTails = PAIR && OP != kOpScatter;
   __device__ __forceinline__ explicit Walk(const DenseParams& q) : p(q) {
     const int c = PAIR ? blockIdx.x >> 1 : blockIdx.x, s = p.stride.d;
-    full = KEEP ? p.full_waves : 0;
+    bn = p.BN;
+    full = KEEP || (kTails && p.tail > 0) ? p.full_waves : 0;
     const int rest = p.units - full * s * p.groups_n;    // (p.units counts the units as if all were of the second kind)
-    left = full + (c < rest ? p.stride.quotient(rest - c + s - 1) : 0);
+    left = kTails && full > 0 ? full + (c < p.tail ? 1 : 0) : full + (c < rest ? p.stride.quotient(rest - c + s - 1) : 0);
     begin(0);
   }
   // the first unit of the row blocks from `block` on
   __device__ __forceinline__ void begin(int block) {
     int u = PAIR ? blockIdx.x >> 1 : blockIdx.x;
+    if (!KEEP) u += block;               // (of which each has one unit here)
     d0 = KEEP && full > 0 ? 0 : p.by_group.remainder(u);
-    u += block;
+    if (KEEP) u += block;
     d1 = p.r1.remainder(u);
     d2 = p.r2.remainder(u);
     d3 = u;
@@ -177,6 +183,13 @@ struct Walk {
       return;
     }
     --left;
+    if (kTails && full > 0 && --full == 0) {
+      const int c = blockIdx.x >> 1, second = c & 1;
+      begin(p.full_waves * p.stride.d + (c >> 1) - c);
+      n0 += second * p.tail_bn;
+      bn = second ? p.BN - p.tail_bn : p.tail_bn;
+      return;
+    }
     const bool whole = KEEP && full > 0;
     if (whole && --full == 0) {
       begin(p.full_waves * p.stride.d);
@@ -198,8 +211,10 @@ struct Walk {
   // width of the tile's MMA (the last tile of a row may be narrower), and the first column this CTA stages
   __device__ __forceinline__ int width() const {
     const int rest = p.N - n0;
-    return min(p.BN, PAIR ? (rest + 31) & ~31 : (rest + 15) & ~15);
+    return min(kTails ? bn : p.BN, PAIR ? (rest + 31) & ~31 : (rest + 15) & ~15);
   }
+  // 64-column segments of the tile that a CTA stages
+  __device__ __forceinline__ int segs() const { return ((PAIR ? bn >> 1 : bn) + 63) >> 6; }
   __device__ __forceinline__ int first_column() const { return PAIR && (blockIdx.x & 1) ? n0 + width() / 2 : n0; }
 };
 
@@ -394,9 +409,9 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     } else {
       constexpr int kQuads = kStep / kParts / 4;         // 16 rows a warp
       const uint32_t g_dst = p.swap ? kMTile : 0u, s_dst = p.swap ? 0u : kMTile;
-      const int g_seg = p.swap ? nseg : 2, s_seg = p.swap ? 2 : nseg;
       int batch = 0;
       for (Walk<OP, PAIR, KEEP> u(p); u.left > 0 && alive; u.next()) {
+        const int segs = u.segs(), g_seg = p.swap ? segs : 2, s_seg = p.swap ? 2 : segs;
         const int steps = u.steps(), n0 = u.first_column();
         const int gx = p.swap ? n0 : u.m0, sx = p.swap ? u.m0 : n0;
         for (int k = 0; k < steps; ++k) {
@@ -611,7 +626,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     const bool f32_rows = OP == kOpScatter && p.plan[kPlanHot] != 0;
     int t = 0;
     for (Walk<OP, PAIR, KEEP> u(p); u.left > 0 && alive; u.next(), ++t) {
-      const int bn = min(p.BN, p.N - u.n0);              // columns of this tile (a multiple of 8)
+      const int bn = min(Walk<OP, PAIR, KEEP>::kTails ? u.bn : p.BN, p.N - u.n0);              // columns of this tile (a multiple of 8)
       const int n_end = u.n0 + bn;
       int my_ro = -1;                                    // G, S: destination row of tile row lg * 32 + lane
       if (OP != kOpDweight) {
@@ -859,6 +874,11 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       const int n0 = u.first_column();
       const int column = OP == kOpDweight && p.swap ? u.m0 : n0, x0 = p.whole ? 0 : column, z0 = p.whole ? column >> 6 : 0;
       const bool rows_too = !KEEP || u.j == 0;       // a scatter's row block is loaded with its first column tile
+      // (a half tile's columns come in boxes of a whole one where those are of whole segments or of weights [E, N, C]: the MMAs do not read
+      // the rest.  D's columns may be gathered: the boxes are the other operand's then.)
+      const bool less = Walk<OP, PAIR, KEEP>::kTails && u.bn < p.BN && (OP == kOpDweight ? p.swap || !p.whole : !p.whole && !p.nc);
+      const int boxes = less && !(OP == kOpDweight && p.swap) ? u.segs() : p.boxes;
+      const uint32_t unit_bytes = less ? 2u * (kMTile + static_cast<uint32_t>(u.segs()) * kSeg) : bytes;
       int m = OP == kOpDweight ? u.split * p.rows_per_split : u.m0;
       int b = p.by_k.quotient(m), k = m - b * p.K;     // first slot row of the step
       for (int ks = 0, c0 = 0; ks < steps; ++ks, c0 += kStep) {
@@ -878,7 +898,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           else tma_load_4d(dst, &map_rows, x, k, u.e, b, bar);
         };
         if (elect_one()) {
-          if (leader) mbar_arrive_expect_tx(own, rows_too ? bytes : (PAIR ? 2u : 1u) * n_bytes);
+          if (leader) mbar_arrive_expect_tx(own, rows_too ? unit_bytes : (PAIR ? 2u : 1u) * n_bytes);
           if (OP != kOpDweight) {
             if (OP == kOpScatter && p.tma_rows && rows_too) box4(KEEP ? a_tile(a_slot) : base, c0);
             if (p.nc) {
@@ -886,7 +906,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
             } else {
 #pragma unroll
               for (int s = 0; s < 4; ++s)
-                if (s < p.boxes) {
+                if (s < boxes) {
                   if (PAIR) tma_load_4d_pair(base + kMTile + s * kSeg, &map_w, x0 + s * 64, c0, z0, u.e, bar);
                   else tma_load_4d(base + kMTile + s * kSeg, &map_w, x0 + s * 64, c0, z0, u.e, bar);
                 }
@@ -895,7 +915,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
             const uint32_t dst = base + (p.swap ? 0u : kMTile);
 #pragma unroll
             for (int s = 0; s < 4; ++s)
-              if (s < p.boxes) tma_load_5d<PAIR>(dst + s * kSeg, &map_rows, x0 + s * 64, k, b, z0, u.e, bar);
+              if (s < boxes) tma_load_5d<PAIR>(dst + s * kSeg, &map_rows, x0 + s * 64, k, b, z0, u.e, bar);
           }
         }
         if (KEEP && rows_too && ++a_slot == p.a_slots) a_slot = 0;
@@ -1071,6 +1091,18 @@ void plan_walk(DenseParams& p, bool pair) {
   digits(p.stride.d / p.groups_n, p.step + 1);
 }
 
+// G, D on pairs: where the last wave would leave half of the pairs idle or more, its tiles are cut in two: a step of 128 columns takes 0.72 of the
+// time of one of 256, so that 3.46 waves take as long as 3.75, not four.  bf16, 32 experts of 2048 rows, 768 and 192 features: G 30.1 -> 28.2 us, D
+// 35.3 -> 33.3; 24 of 909, 1000 and 200: G 25.1 -> 23.0, D 27 -> 25; 64 of 4096, 1024 and 256: D 120 -> 116; 40 of 1280, 512 and 512: G 33 -> 30, D
+// 40 -> 34 (with the changes to its gathers).
+void plan_tail(DenseParams& p) {
+  const int pairs = kSms / 2, rest = p.units % pairs, first = (p.BN / 2 + 31) / 32 * 32, last = p.N - (p.tiles_n - 1) * p.BN;
+  if (p.units < pairs || rest == 0 || 2 * rest > pairs || p.BN < 128 || last <= first || (p.whole && first % 128 != 0)) return;
+  p.full_waves = p.units / pairs;
+  p.tail = 2 * rest;
+  p.tail_bn = first;
+}
+
 template <typename T, int OP, bool PAIR, bool KEEP>
 cudaError_t launch(const DenseParams& p, const TensorMap3& mw, const TensorMap3& mr, cudaStream_t st) {
   const size_t smem = kDenseHeader + (OP == kOpDweight ? table_bytes(!p.tma_rows) : kRowTable) + epi_bytes(p.readers > kEpiWarps) +
@@ -1152,6 +1184,7 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
     return !r.pair           ? launch_typed<kOpScatter, false>(p, dtype, mw, mr, st)
            : r.tile_group > 0 ? launch_typed<kOpScatter, true, true>(p, dtype, mw, mr, st)
                               : launch_typed<kOpScatter, true>(p, dtype, mw, mr, st);
+  if (r.pair) plan_tail(p);
   return r.pair ? launch_typed<kOpGather, true>(p, dtype, mw, mr, st) : launch_typed<kOpGather, false>(p, dtype, mw, mr, st);
 }
 
@@ -1237,6 +1270,7 @@ cudaError_t launch_dense16_dweight(const DWeightParams& r, int dtype, cudaStream
   if (r.pair && (!encode_gather(&mw, r.Xsrc, static_cast<long long>(r.B) * r.T, r.FG) ||
                  (!p.tma_rows && !encode_gather(&mr, r.Ysrc, static_cast<long long>(r.M) * r.E, r.FD))))
     return cudaErrorInvalidValue;
+  if (r.pair) plan_tail(p);
   return r.pair ? launch_typed<kOpDweight, true>(p, dtype, mw, mr, st)
                 : launch_typed<kOpDweight, false>(p, dtype, mw, mr, st);
 }

@@ -312,6 +312,27 @@ def test_dense16_dweight_sums_long_contractions_in_ranges(cuda_device, B, T, E, 
     assert torch.stack(bias).mean().abs().item() <= 8192 / 16 * 2.0 ** -23
 
 
+# G and D on pairs whose last wave is half empty or more: its tiles are cut in two.  Columns that come as boxes of whole segments and of
+# partial ones, gathered (either operand of D), weights of both layouts.  Small integers: exact in float32, then rounded once.
+@pytest.mark.parametrize("B,T,E,K,I,J", [(6, 100, 38, 101, 456, 192), (15, 100, 11, 32, 1032, 432), (11, 100, 52, 50, 400, 224), (7, 100, 56, 64, 704, 232),
+                                         (11, 100, 15, 64, 912, 640), (11, 100, 33, 50, 424, 248), (9, 100, 48, 45, 816, 256), (20, 90, 40, 64, 512, 512)])
+def test_dense16_last_wave_in_half_tiles(cuda_device, B, T, E, K, I, J):
+    plans = [ops.describe_plan(op, B, T, E, K, I, J, torch.bfloat16, w_layout=w) for op, w in (("G", "cn"), ("G", "nc"), ("D", "cn"))]
+    assert any(p["pair"] and p["tile_n"] >= 128 for p in plans), plans
+    g = torch.Generator().manual_seed(I)
+    X, Y = (torch.randint(-2, 3, s, generator=g).to(torch.bfloat16) for s in ((B, T, I), (B, E, K, J)))
+    W = torch.randint(-1, 2, (E, I, J), generator=g).to(torch.bfloat16)
+    Ind = torch.randint(0, T, (B, E, K), generator=g)
+    d = lambda t: t.to(cuda_device)
+    ref = torch.from_numpy(orc.np_gather(X, W, Ind)).to(torch.bfloat16)
+    assert torch.equal(ops.gather_gemm(d(X), d(W), d(Ind)).cpu(), ref)
+    assert torch.equal(ops.gather_gemm(d(X), d(W.transpose(1, 2).contiguous()), d(Ind), w_layout="nc").cpu(), ref)
+    ref = torch.from_numpy(orc.np_dweight(X, Y, Ind)).to(torch.bfloat16)
+    assert torch.equal(ops.dweight(d(X), d(Y), d(Ind)).cpu(), ref)
+    assert torch.equal(ops.dweight(d(X), d(Y), d(Ind), out_layout="direct_rows").cpu(), ref.transpose(1, 2))
+    ops.check_status()
+
+
 # weight gradients on pairs whose slot rows are gathered too, with an odd and an even number of stages (two groups of warps share the ring's
 # slots), widths whose last tile is narrow, ranges that end within a batch of ids.  Small integers: exact in float32, then rounded once.
 @pytest.mark.parametrize("B,T,E,K,FG,FD,stages", [(9, 300, 24, 101, 1000, 200, 5), (39, 80, 13, 21, 1936, 344, 5), (20, 90, 74, 45, 512, 520, 5), (15, 200, 74, 64, 512, 512, 6)])
