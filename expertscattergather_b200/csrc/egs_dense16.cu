@@ -108,7 +108,7 @@ struct DenseParams {
   int whole, boxes;   // weights [E, C, N], D's slot rows: boxes of all 64-column segments of a tile (see whole_segments), boxes of a tile
   int half;           // columns of a tile one CTA stages: BN, or BN / 2 in a pair
   int after_own;      // see launch_kernel
-  int tail, tail_bn;                     // G, D on pairs: units of half a tile in the last wave (0: none), width of the first half (see plan_tail)
+  int tail, tail_bn;                     // G on pairs: units of half a tile in the last wave (0: none), width of the first half (see plan_tail)
 };
 
 // Position in the stage ring.
@@ -125,7 +125,7 @@ struct Cursor {
 // The tiles of a CTA or pair.  A unit is a number in a mixed radix - column tile; row block of a group, expert, group (G, S) or row block,
 // row range, expert (D) - units go out `stride` apart and are advanced by adding the stride's digits: three divisions a unit (1000
 // clocks and more) in the lanes that feed the tensor core were a fifth of the time of a tile with eight steps.
-// The last wave of G and D on pairs may be units of half a tile (see plan_tail).
+// The last wave of G on pairs may be units of half a tile (see plan_tail).
 // A scatter whose rows may stay has units of several column tiles: all of a row block's for as many whole waves as there are, and
 // groups of them, so that the last wave is even, for the row blocks that are left.
 template <int OP, bool PAIR, bool KEEP>
@@ -136,7 +136,7 @@ struct Walk {
   int full, d0, d1, d2, d3;
   int bn;                      // width of the unit's tile
   const DenseParams& p;
-  static constexpr bool kTails = PAIR && OP != kOpScatter;
+  static constexpr bool kTails = PAIR && OP == kOpGather;
   __device__ __forceinline__ explicit Walk(const DenseParams& q) : p(q) {
     const int c = PAIR ? blockIdx.x >> 1 : blockIdx.x, s = p.stride.d;
     bn = p.BN;
@@ -409,9 +409,9 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     } else {
       constexpr int kQuads = kStep / kParts / 4;         // 16 rows a warp
       const uint32_t g_dst = p.swap ? kMTile : 0u, s_dst = p.swap ? 0u : kMTile;
+      const int g_seg = p.swap ? nseg : 2, s_seg = p.swap ? 2 : nseg;
       int batch = 0;
       for (Walk<OP, PAIR, KEEP> u(p); u.left > 0 && alive; u.next()) {
-        const int segs = u.segs(), g_seg = p.swap ? segs : 2, s_seg = p.swap ? 2 : segs;
         const int steps = u.steps(), n0 = u.first_column();
         const int gx = p.swap ? n0 : u.m0, sx = p.swap ? u.m0 : n0;
         for (int k = 0; k < steps; ++k) {
@@ -874,10 +874,9 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       const int n0 = u.first_column();
       const int column = OP == kOpDweight && p.swap ? u.m0 : n0, x0 = p.whole ? 0 : column, z0 = p.whole ? column >> 6 : 0;
       const bool rows_too = !KEEP || u.j == 0;       // a scatter's row block is loaded with its first column tile
-      // (a half tile's columns come in boxes of a whole one where those are of whole segments or of weights [E, N, C]: the MMAs do not read
-      // the rest.  D's columns may be gathered: the boxes are the other operand's then.)
-      const bool less = Walk<OP, PAIR, KEEP>::kTails && u.bn < p.BN && (OP == kOpDweight ? p.swap || !p.whole : !p.whole && !p.nc);
-      const int boxes = less && !(OP == kOpDweight && p.swap) ? u.segs() : p.boxes;
+      // (a half tile's columns come in boxes of a whole one where those are of whole segments or of weights [E, N, C]: the MMAs do not read the rest)
+      const bool less = Walk<OP, PAIR, KEEP>::kTails && u.bn < p.BN && !p.whole && !p.nc;
+      const int boxes = less ? u.segs() : p.boxes;
       const uint32_t unit_bytes = less ? 2u * (kMTile + static_cast<uint32_t>(u.segs()) * kSeg) : bytes;
       int m = OP == kOpDweight ? u.split * p.rows_per_split : u.m0;
       int b = p.by_k.quotient(m), k = m - b * p.K;     // first slot row of the step
@@ -1091,10 +1090,10 @@ void plan_walk(DenseParams& p, bool pair) {
   digits(p.stride.d / p.groups_n, p.step + 1);
 }
 
-// G, D on pairs: where the last wave would leave half of the pairs idle or more, its tiles are cut in two: a step of 128 columns takes 0.72 of the
-// time of one of 256, so that 3.46 waves take as long as 3.75, not four.  bf16, 32 experts of 2048 rows, 768 and 192 features: G 30.1 -> 28.2 us, D
-// 35.3 -> 33.3; 24 of 909, 1000 and 200: G 25.1 -> 23.0, D 27 -> 25; 64 of 4096, 1024 and 256: D 120 -> 116; 40 of 1280, 512 and 512: G 33 -> 30, D
-// 40 -> 34 (with the changes to its gathers).
+// G on pairs: where the last wave would leave half of the pairs idle or more, its tiles are cut in two: a step of 128 columns takes 0.72 of the time
+// of one of 256, so that 3.46 waves take as long as 3.75, not four.  bf16, 32 experts of 2048 rows, 768 -> 192 features 30.1 -> 28.2 us, 24 of 909,
+// 1000 -> 200 25.1 -> 23.0, 20 of 1024, 768 -> 512 25.1 -> 23.0.  D, which runs beside the dX / dY kernel and leaves it the idle pairs, keeps whole
+// tiles: alone 35.3 -> 33.3 us, but a training step of ragged sizes 139.5 -> 142.
 void plan_tail(DenseParams& p) {
   const int pairs = kSms / 2, rest = p.units % pairs, first = (p.BN / 2 + 31) / 32 * 32, last = p.N - (p.tiles_n - 1) * p.BN;
   if (p.units < pairs || rest == 0 || 2 * rest > pairs || p.BN < 128 || last <= first || (p.whole && first % 128 != 0)) return;
@@ -1270,7 +1269,6 @@ cudaError_t launch_dense16_dweight(const DWeightParams& r, int dtype, cudaStream
   if (r.pair && (!encode_gather(&mw, r.Xsrc, static_cast<long long>(r.B) * r.T, r.FG) ||
                  (!p.tma_rows && !encode_gather(&mr, r.Ysrc, static_cast<long long>(r.M) * r.E, r.FD))))
     return cudaErrorInvalidValue;
-  if (r.pair) plan_tail(p);
   return r.pair ? launch_typed<kOpDweight, true>(p, dtype, mw, mr, st)
                 : launch_typed<kOpDweight, false>(p, dtype, mw, mr, st);
 }

@@ -312,8 +312,8 @@ def test_dense16_dweight_sums_long_contractions_in_ranges(cuda_device, B, T, E, 
     assert torch.stack(bias).mean().abs().item() <= 8192 / 16 * 2.0 ** -23
 
 
-# G and D on pairs whose last wave is half empty or more: its tiles are cut in two.  Columns that come as boxes of whole segments and of
-# partial ones, gathered (either operand of D), weights of both layouts.  Small integers: exact in float32, then rounded once.
+# G on pairs whose last wave is half empty or more: its tiles are cut in two.  Columns that come as boxes of whole segments and of partial ones,
+# weights of both layouts; D on pairs beside it, with either operand gathered.  Small integers: exact in float32, then rounded once.
 @pytest.mark.parametrize("B,T,E,K,I,J", [(6, 100, 38, 101, 456, 192), (15, 100, 11, 32, 1032, 432), (11, 100, 52, 50, 400, 224), (7, 100, 56, 64, 704, 232),
                                          (11, 100, 15, 64, 912, 640), (11, 100, 33, 50, 424, 248), (9, 100, 48, 45, 816, 256), (20, 90, 40, 64, 512, 512)])
 def test_dense16_last_wave_in_half_tiles(cuda_device, B, T, E, K, I, J):
