@@ -73,6 +73,7 @@ struct __align__(16) DenseHeader {
   unsigned long long drain;
   uint32_t tmem_base;
   uint32_t abort_flag;
+  uint32_t freed;                        // S whose rows stay: steps whose slot the TMA warp has found free
   int added, last;                       // S: read-out warps that have added what they had to; 1: the grid's last, -1: others are to come
 };
 static_assert(sizeof(DenseHeader) <= kDenseHeader, "header does not fit");
@@ -330,6 +331,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     if (!p.after_own) pdl_wait();
     hdr->abort_flag = p.status.timed_out() ? 1u : 0u;
     hdr->added = hdr->last = 0;
+    hdr->freed = 0u;
     if (smem_misaligned(smem_raw)) {
       hdr->abort_flag = 1u;
       p.status.report(EGS_STATUS_INTERNAL);
@@ -377,6 +379,25 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     // the groups would meet each barrier in turn, and a warp that is late to look at a phase whose stage another group loads finds the one
     // after it done as well, which a parity cannot tell from neither being done.
     auto is_mine = [&]() { return kGroups == 1 || (at.slot & (kGroups - 1)) == group; };
+    // Rows that stay are loaded with their first column tile only; with the others these warps would follow phases that they have no part in.
+    // They ask the TMA warp, which has a part in every stage, how far the ring is.
+    uint32_t n = 0;                      // steps before this one
+    auto wait_turn = [&]() {
+      auto there = [&]() {
+        uint32_t freed;
+        asm volatile("ld.acquire.cta.shared::cta.b32 %0, [%1];" : "=r"(freed) : "r"(smem_u32(&hdr->freed)) : "memory");
+        return __all_sync(0xffffffffu, freed > n) != 0;
+      };
+      for (const long long t0 = clock64(); !there();) {
+        if (!__any_sync(0xffffffffu, *abort_flag != 0u || clock64() - t0 > kWaitLimitCycles)) continue;
+        if (lane == 0 && !*abort_flag) {
+          *abort_flag = 1u;
+          p.status.report(EGS_STATUS_PIPELINE_TIMEOUT);
+        }
+        alive = false;
+        break;
+      }
+    };
     const uint32_t full0 = map_to_cta(smem_u32(&hdr->full[0]), 0);
     if constexpr (OP != kOpDweight) {
       constexpr int kQuads = kTileM / kParts / 4;        // G, S: 16 rows a warp
@@ -392,12 +413,14 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
         if (lane == 0) mbar_arrive(smem_u32(&hdr->ids_empty[t & 1]));
         for (int k = 0; k < steps; ++k) {
           const bool mine = is_mine();
-          if (mine) wait_free();
+          if (!KEEP && mine) wait_free();
+          if (KEEP && u.j == 0) wait_turn();
           if (!alive) break;
           const int slot = at.slot;
           const uint32_t bar = full0 + slot * 8u;
           at.next(stages);
-          if (KEEP && u.j > 0) continue;     // (the rows are there; every phase of a barrier has to be waited for all the same)
+          ++n;
+          if (KEEP && u.j > 0) continue;     // (the rows are there)
           const uint32_t dst = a_tile(KEEP ? a_slot : slot) + static_cast<uint32_t>(part * kQuads) * 512u;
           if (KEEP && ++a_slot == p.a_slots) a_slot = 0;
           if (mine && elect_one()) {
@@ -868,6 +891,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     const uint32_t bytes = PAIR ? 2u * stage_bytes : (OP != kOpDweight ? n_bytes : (p.swap ? kMTile : n_bytes)) + ((OP == kOpScatter && p.tma_rows) ? kMTile : 0u);
     bool ok = true;
     int a_slot = 0;
+    uint32_t freed = 0;
     Cursor at;
     for (Walk<OP, PAIR, KEEP> u(p); u.left > 0 && ok; u.next()) {
       const int steps = u.steps();
@@ -897,6 +921,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           else tma_load_4d(dst, &map_rows, x, k, u.e, b, bar);
         };
         if (elect_one()) {
+          if (KEEP && gathers) asm volatile("st.release.cta.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hdr->freed)), "r"(freed + 1u) : "memory");
           if (leader) mbar_arrive_expect_tx(own, rows_too ? unit_bytes : (PAIR ? 2u : 1u) * n_bytes);
           if (OP != kOpDweight) {
             if (OP == kOpScatter && p.tma_rows && rows_too) box4(KEEP ? a_tile(a_slot) : base, c0);
@@ -918,6 +943,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           }
         }
         if (KEEP && rows_too && ++a_slot == p.a_slots) a_slot = 0;
+        ++freed;
         if (OP == kOpDweight) {
           k += kStep;                                  // 64 rows are parts of one batch element or whole ones
           while (k >= p.K) { k -= p.K; ++b; }
