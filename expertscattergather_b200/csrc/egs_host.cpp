@@ -360,8 +360,9 @@ Tensor gemm_scatter(const Tensor& Y, const Tensor& W, const Tensor& Ind, int64_t
   return out;
 }
 
-// on_stream: where the kernels go.  The buffers belong to the current stream either way: the caller forks and joins the two,
-// passes contiguous inputs, and keeps *shared_ws - the scratch, one buffer for the weight gradients of one pass, which run one
+// on_stream: where the kernels go.  The buffers belong to the current stream either way, and the other stream knows nothing of what the
+// current one does behind the fork: all that it writes is allocated before a temporary of a later operator could be freed and its block
+// handed out again, so work for it is issued right behind the fork.  The caller forks and joins the two, passes contiguous inputs, and keeps *shared_ws - the scratch, one buffer for the weight gradients of one pass, which run one
 // after the other and are of one size - until it has joined.
 Tensor dweight_on(const Tensor& Xsrc, const Tensor& Ysrc, const Tensor& Ind, int out_layout, int precision, int path, const OptTensor& zeroed,
                   std::optional<cudaStream_t> on_stream, Tensor* shared_ws) {
@@ -528,8 +529,11 @@ Grads gather_backward(const Tensor& X_, const Tensor& W, const Tensor& Ind_, con
     }
     g.w = dweight_on(X, dY, Ind, EGS_DW_GATHERED_ROWS, -1, -1, std::nullopt, on, &ws);
   }
+  auto bias_gradient = [&](std::optional<cudaStream_t> on) { g.b = expert_row_sum(dY, std::nullopt, dY.size(0), X.size(1), dY.size(1), dY.size(2), on); };
+  const auto sums_on = row_sum_stream(side, dY);
+  if (need_b && sums_on) bias_gradient(sums_on);                  // (before the dX kernel's scratch comes and goes, see dweight_on)
   if (need_x) g.in = gemm_scatter(dY, W, Ind, X.size(1), EGS_W_NC, std::nullopt, -1, -1, std::nullopt, std::nullopt);
-  if (need_b) g.b = expert_row_sum(dY, std::nullopt, dY.size(0), X.size(1), dY.size(1), dY.size(2), row_sum_stream(side, dY));
+  if (need_b && !sums_on) bias_gradient(std::nullopt);
   return g;
 }
 
@@ -546,8 +550,11 @@ Grads scatter_backward(const Tensor& Y_, const Tensor& W, const Tensor& Ind_, co
     }
     g.w = dweight_on(dOut, Y, Ind, EGS_DW_DIRECT_ROWS, -1, -1, std::nullopt, on, &ws);
   }
+  auto bias_gradient = [&](std::optional<cudaStream_t> on) { g.b = expert_row_sum(dOut, Ind, Y.size(0), dOut.size(1), Y.size(1), Y.size(2), on); };
+  const auto sums_on = row_sum_stream(side, dOut);
+  if (need_b && sums_on) bias_gradient(sums_on);                  // (before a copy of the weights comes and goes, see dweight_on)
   if (need_y) g.in = gather_gemm(dOut, W, Ind, EGS_W_NC, -1, -1, std::nullopt);
-  if (need_b) g.b = expert_row_sum(dOut, Ind, Y.size(0), dOut.size(1), Y.size(1), Y.size(2), row_sum_stream(side, dOut));
+  if (need_b && !sums_on) bias_gradient(std::nullopt);
   return g;
 }
 

@@ -85,3 +85,55 @@ def test_scatter_bias_reference_mode_is_the_broadcast_of_the_reference(cuda_devi
     Y3 = torch.zeros(4, 3, 8, w.J, device=cuda_device)
     with pytest.raises(RuntimeError):
         sm2(Y3, torch.zeros(4, 3, 8, dtype=torch.int64, device=cuda_device), w.T)
+
+
+# the bias gradient is summed on the helper stream while the dX / dY operator runs: with scratch and a copy of the weights in the pool that the bias
+# gradient's buffer comes from, that buffer has to be a block of its own.  Weights with one entry a row: every sum is a small integer, exact in bf16.
+@pytest.mark.parametrize("op", ["gather", "scatter"])
+@pytest.mark.parametrize("captured", [False, True])
+def test_bias_gradients_beside_the_input_gradient(cuda_device, op, captured):
+    B, T, E, K, I, J = 1, 128, 64, 16, 1024, 256
+    g = torch.Generator().manual_seed(5)
+    ints = lambda *s: torch.randint(-1, 2, s, generator=g).to(torch.bfloat16)
+    Ind = torch.rand(B, E, T, generator=g).topk(K, -1).indices
+    W = ints(E, I, J) * (torch.arange(I)[:, None] % J == torch.arange(J)[None])
+    rows, slots = ints(B, T, I), ints(B, E, K, J)               # X and dY, or dOut and Y
+    dw = torch.from_numpy(orc.np_dweight(rows, slots, Ind))
+    if op == "gather":
+        ref = [torch.from_numpy(orc.np_scatter(slots, W.transpose(1, 2), Ind, T)), dw, slots.double().sum((0, 2))]
+        args = [rows.to(cuda_device), W.to(cuda_device), Ind.to(cuda_device), slots.to(cuda_device)]
+    else:                                                       # (weights that are not contiguous: the dY kernel reads a copy)
+        ref = [torch.from_numpy(orc.np_gather(rows, W, Ind)), dw.transpose(1, 2), rows[0].double()[Ind[0]].sum(1)]
+        args = [slots.to(cuda_device), W.to(cuda_device).transpose(1, 2), Ind.to(cuda_device), rows.to(cuda_device)]
+    ref = [r.to(cuda_device).to(torch.bfloat16) for r in ref]
+    host = ops._host()
+    backward = lambda: (host.gather_backward if op == "gather" else host.scatter_backward)(*args, True, True, True)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    runs = []
+    if captured:
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            backward()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = backward()
+        for _ in range(5):
+            graph.replay()
+            runs.append([t.clone() for t in got])
+    else:
+        torch.cuda.memory._record_memory_history("all", context=None)
+        try:
+            first = backward()
+            trace = [(a["action"], a["addr"]) for a in torch.cuda.memory._snapshot()["device_traces"][cuda_device.index or 0]]
+        finally:
+            torch.cuda.memory._record_memory_history(None)
+        made = lambda t: trace.index(("alloc", t.data_ptr()))
+        assert not [a for a in trace[made(first[1]):made(first[2])] if a[0].startswith("free")]      # nothing that it could have got has been in use since the fork
+        runs = [first] + [backward() for _ in range(9)]
+    torch.cuda.synchronize()
+    ops.check_status()
+    for got in runs:
+        for a, b in zip(got, ref):
+            assert torch.equal(a, b)
