@@ -530,7 +530,7 @@ Grads gather_backward(const Tensor& X_, const Tensor& W, const Tensor& Ind_, con
     g.w = dweight_on(X, dY, Ind, EGS_DW_GATHERED_ROWS, -1, -1, std::nullopt, on, &ws);
   }
   auto bias_gradient = [&](std::optional<cudaStream_t> on) { g.b = expert_row_sum(dY, std::nullopt, dY.size(0), X.size(1), dY.size(1), dY.size(2), on); };
-  const auto sums_on = row_sum_stream(side, dY);
+  const auto sums_on = need_x ? row_sum_stream(side, dY) : std::nullopt;
   if (need_b && sums_on) bias_gradient(sums_on);                  // (before the dX kernel's scratch comes and goes, see dweight_on)
   if (need_x) g.in = gemm_scatter(dY, W, Ind, X.size(1), EGS_W_NC, std::nullopt, -1, -1, std::nullopt, std::nullopt);
   if (need_b && !sums_on) bias_gradient(std::nullopt);
@@ -551,7 +551,7 @@ Grads scatter_backward(const Tensor& Y_, const Tensor& W, const Tensor& Ind_, co
     g.w = dweight_on(dOut, Y, Ind, EGS_DW_DIRECT_ROWS, -1, -1, std::nullopt, on, &ws);
   }
   auto bias_gradient = [&](std::optional<cudaStream_t> on) { g.b = expert_row_sum(dOut, Ind, Y.size(0), dOut.size(1), Y.size(1), Y.size(2), on); };
-  const auto sums_on = row_sum_stream(side, dOut);
+  const auto sums_on = need_y ? row_sum_stream(side, dOut) : std::nullopt;
   if (need_b && sums_on) bias_gradient(sums_on);                  // (before a copy of the weights comes and goes, see dweight_on)
   if (need_y) g.in = gather_gemm(dOut, W, Ind, EGS_W_NC, -1, -1, std::nullopt);
   if (need_b && !sums_on) bias_gradient(std::nullopt);

@@ -137,3 +137,28 @@ def test_bias_gradients_beside_the_input_gradient(cuda_device, op, captured):
     for got in runs:
         for a, b in zip(got, ref):
             assert torch.equal(a, b)
+
+
+# ... and only there: without an input gradient the sum runs on the main stream, beside the weight gradient
+@pytest.mark.parametrize("op", ["gather", "scatter"])
+@pytest.mark.parametrize("need_input", [True, False])
+def test_where_bias_gradients_are_summed(cuda_device, op, need_input):
+    B, T, E, K, I, J = 2, 128, 32, 16, 512, 256
+    g = torch.Generator().manual_seed(6)
+    ints = lambda *s: torch.randint(-1, 2, s, generator=g).to(torch.bfloat16).to(cuda_device)
+    rows, slots, W, Ind = ints(B, T, I), ints(B, E, K, J), ints(E, I, J), torch.rand(B, E, T, generator=g).topk(K, -1).indices.to(cuda_device)
+    host = ops._host()
+    if op == "gather":
+        backward, args, ref = host.gather_backward, (rows, W, Ind, slots), slots.float().sum((0, 2))
+    else:
+        backward, args = host.scatter_backward, (slots, W.transpose(1, 2).contiguous(), Ind, rows)
+        ref = torch.stack([rows[b].float()[Ind[b]].sum(1) for b in range(B)]).sum(0)
+    backward(*args, need_input, True, True)
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        got = backward(*args, need_input, True, True)
+        torch.cuda.synchronize()
+    assert (got[0] is not None) == need_input and torch.equal(got[2].float(), ref)
+    streams = lambda name: {e.device_resource_id for e in prof.events() if name in e.name}
+    sums, weights = streams("expert_row_sum_kernel"), streams("dense16_kernel<__nv_bfloat16, 2")
+    assert len(sums) == len(weights) == 1 and (sums == weights) == need_input
