@@ -97,9 +97,11 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 constexpr long long kInt32Max = 2147483647LL;
 // 16-bit scatter adds directly into the output while no token row receives more contributions than this.
 constexpr int kDirect16Limit = 32;
-// 16-bit scatters of at most this many output elements round their float32 rows in the scatter kernel (its last CTA does it); a launch of its
-// own finds nothing to round after most calls.  Back to back, bf16, 64 tokens of 8 experts, 128 -> 512 features: 7.4 us a scatter with the
-// launch, 6.4 without; where a hot row selects float32 rows 9.4 and 12.1, at 64 Ki elements 10.5 and 16.6.  The host saves 2 us a launch.
+// 16-bit scatters of at most this many output elements may round their float32 rows in the scatter kernel (see round_rows); a launch of its own
+// finds nothing to round after most calls.  Back to back, bf16, 64 tokens of 8 experts, 128 -> 128 to 1024 features: 5.2 to 6.5 us a scatter with
+// the launch, 4.6 to 6.0 without; where a hot row selects float32 rows 6.9 to 8.4, and 8.2 to 8.9.  The host saves 2 us a launch.  So calls whose
+// rows get more than half of the limit's contributions in the mean, some row surely or likely more than the limit, keep the launch: 64 tokens of
+// 256 experts of 16, 128 -> 512 features, 18.0 us with it.
 constexpr size_t kRoundInKernel = 64 << 10;
 // Longest contraction strict float32 runs on the tensor cores under EGS_PATH_AUTO (measured against float64 up to there, see
 // egs_strict.cu), and longest that one accumulator of the fused pair kernel sees.
@@ -236,7 +238,8 @@ int run_rowgemm(bool scatter, const void* A, const void* W, const void* bias, co
       err = launch_tensor_gather2(p, dtype, smem2, st);
     } else if (dtype != EGS_F32) {
       configure_dense16_rowgemm(p, scatter);
-      rounds = scatter && n_out <= kRoundInKernel && p.tile_group == 0;
+      rounds = scatter && n_out <= kRoundInKernel && 2ll * d.E * d.K <= 1ll * kDirect16Limit * d.T && p.tile_group == 0 &&
+               (p.N + p.BN - 1) / p.BN < kPlanWords - kPlanAdded;
       p.rounds = rounds ? 1 : 0;
       err = launch_dense16_rowgemm(p, scatter, dtype, st);
     } else {

@@ -71,10 +71,11 @@ struct __align__(16) DenseHeader {
   unsigned long long dst_full[2];
   unsigned long long dst_empty[2];
   unsigned long long drain;
+  unsigned long long last;               // ... and the column tiles that this CTA was the last to add to
   uint32_t tmem_base;
   uint32_t abort_flag;
   uint32_t freed;                        // S whose rows stay: steps whose slot the TMA warp has found free
-  int added, last;                       // S: read-out warps that have added what they had to; 1: the grid's last, -1: others are to come
+  int rounds;                            // S: float32 rows are to be rounded here ...
 };
 static_assert(sizeof(DenseHeader) <= kDenseHeader, "header does not fit");
 
@@ -226,44 +227,46 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* map, int x
       : "memory");
 }
 
-// Rounds the float32 rows of a small scatter that sums in those: the CTA whose read-out warps are the last of the grid to have added what
-// they had to does it.  Nobody waits for another CTA, which may have yet to find room beside another stream's kernels.
-template <typename T>
-__device__ __noinline__ void round_rows(const DenseParams& p, DenseHeader* hdr, int warp, int lane) {
-  __threadfence();
-  __syncwarp();
-  if (lane == 0 && atomicAdd(&hdr->added, 1) == p.readers - 1) {
+// Rounds the float32 rows of a small scatter that sums in those, behind the barrier of the common exit.  A column tile is rounded by the CTA that
+// is the last to have added to it: one CTA for all of them took 1.5 us more at 16 Ki elements and 3.5 at 64 Ki.  Nobody waits for another CTA,
+// which may have yet to find room beside another stream's kernels.
+template <typename T, bool PAIR>
+__device__ __noinline__ void round_rows(const DenseParams& p, DenseHeader* hdr) {
+  const int tid = threadIdx.x;
+  if (tid < p.tiles_n) {
+    int added = 0;                                   // units of column tile `tid` that this CTA has had
+    for (int u = PAIR ? blockIdx.x >> 1 : blockIdx.x; u < p.units; u += p.stride.d) added += u % p.tiles_n == tid;
     __threadfence();
-    const bool last = atomicAdd(p.plan + kPlanAdded, 1) == static_cast<int>(gridDim.x) - 1;
+    const int all = p.units / p.tiles_n * (PAIR ? 2 : 1);
+    if (added > 0 && atomicAdd(p.plan + kPlanAdded + tid, added) + added == all) atomicOr(&hdr->last, 1ull << tid);
     __threadfence();
-    *const_cast<volatile int*>(&hdr->last) = last ? 1 : -1;
   }
-  const volatile int *verdict = &hdr->last;
-  const volatile uint32_t* abort_flag = &hdr->abort_flag;
-  __syncwarp();
-  while (__all_sync(0xffffffffu, *verdict == 0))
-    if (__any_sync(0xffffffffu, *abort_flag != 0u)) return;              // (a warp that gave up does not count)
-  if (__any_sync(0xffffffffu, *verdict < 0)) return;
-  __threadfence();
-  const int n = p.B * p.T * p.N;                     // (see kRoundInKernel)
+  __syncthreads();
   T* out = static_cast<T*>(p.Out);
-  constexpr int kAtOnce = 8;
-  const int step = p.readers * 256;
-  for (int i0 = (warp * 32 + lane) * 8; i0 < n; i0 += kAtOnce * step) {
-    float4 v[2 * kAtOnce];
+  for (unsigned long long tiles = hdr->last; tiles != 0; tiles &= tiles - 1) {
+    const int n0 = (__ffsll(static_cast<long long>(tiles)) - 1) * p.BN, chunks = min(p.BN, p.N - n0) / 8;      // of eight columns a row
+    const int n = p.B * p.T * chunks;                // (see kRoundInKernel)
+    constexpr int kAtOnce = 4;
+    for (int i0 = tid; i0 < n; i0 += kAtOnce * kDenseThreads) {
+      int at[kAtOnce];
+      float4 v[2 * kAtOnce];
 #pragma unroll
-    for (int j = 0; j < kAtOnce; ++j) {
-      const float4* from = reinterpret_cast<const float4*>(p.acc + min(i0 + j * step, n - 8));
-      v[2 * j] = __ldcg(from);
-      v[2 * j + 1] = __ldcg(from + 1);
-    }
+      for (int j = 0; j < kAtOnce; ++j) {
+        const int i = i0 + j * kDenseThreads, row = i / chunks;
+        at[j] = i < n ? row * p.N + n0 + (i - row * chunks) * 8 : -1;
+        if (at[j] >= 0) {
+          v[2 * j] = __ldcg(reinterpret_cast<const float4*>(p.acc + at[j]));
+          v[2 * j + 1] = __ldcg(reinterpret_cast<const float4*>(p.acc + at[j]) + 1);
+        }
+      }
 #pragma unroll
-    for (int j = 0; j < kAtOnce; ++j) {
-      const float4 a = v[2 * j], b = v[2 * j + 1];
-      if (i0 + j * step < n)
-        *reinterpret_cast<uint4*>(out + i0 + j * step) =
-            make_uint4(pack2(out, __float_as_uint(a.x), __float_as_uint(a.y)), pack2(out, __float_as_uint(a.z), __float_as_uint(a.w)),
-                       pack2(out, __float_as_uint(b.x), __float_as_uint(b.y)), pack2(out, __float_as_uint(b.z), __float_as_uint(b.w)));
+      for (int j = 0; j < kAtOnce; ++j) {
+        const float4 a = v[2 * j], b = v[2 * j + 1];
+        if (at[j] >= 0)
+          *reinterpret_cast<uint4*>(out + at[j]) =
+              make_uint4(pack2(out, __float_as_uint(a.x), __float_as_uint(a.y)), pack2(out, __float_as_uint(a.z), __float_as_uint(a.w)),
+                         pack2(out, __float_as_uint(b.x), __float_as_uint(b.y)), pack2(out, __float_as_uint(b.z), __float_as_uint(b.w)));
+      }
     }
   }
 }
@@ -330,7 +333,8 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     fence_mbar_init();
     if (!p.after_own) pdl_wait();
     hdr->abort_flag = p.status.timed_out() ? 1u : 0u;
-    hdr->added = hdr->last = 0;
+    hdr->rounds = 0;
+    hdr->last = 0ull;
     hdr->freed = 0u;
     if (smem_misaligned(smem_raw)) {
       hdr->abort_flag = 1u;
@@ -766,7 +770,10 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       }
       if (!released) release();
     }
-    if (OP == kOpScatter && !KEEP && f32_rows && alive && p.rounds) round_rows<T>(p, hdr, ew, lane);
+    if (OP == kOpScatter && !KEEP && f32_rows && p.rounds) {
+      __threadfence();                                   // (before the barrier of the common exit: what this thread has added)
+      if (tid == kProdThreads) hdr->rounds = 1;
+    }
     }
   } else if (warp == kMmaWarp) {
     // =========================== MMA issuer ===========================
@@ -956,6 +963,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
   // ---- common exit ----
   tc_fence_before();
   __syncthreads();
+  if (OP == kOpScatter && !KEEP && hdr->rounds && *abort_flag == 0u) round_rows<T, PAIR>(p, hdr);
   if (!PAIR) {
     if (warp == kMmaWarp) tmem_release(tmem_base, tmem_cols, smem_u32(&hdr->drain), abort_flag, p.status, lane);
   } else {

@@ -757,7 +757,7 @@ __global__ void __launch_bounds__(kPrepThreads) scatter_prepare_kernel(const voi
   } else if (COUNT) {
     flag = B == 1 ? has_hot_row<true>(ind, index_dtype, 0, 1, T_, EK, limit, prep_cnt) : has_hot_row<false>(ind, index_dtype, 0, B, T_, EK, limit, prep_cnt);
   }
-  if (blockIdx.x == 0 && tid <= kPlanAdded) plan[tid] = tid == kPlanHot ? flag : 0;
+  if (blockIdx.x == 0 && tid < kPlanWords) plan[tid] = tid == kPlanHot ? flag : 0;
   // (n is a multiple of 8 elements and both buffers are 16-byte aligned: tensor-core path only)
   if (zero_output) {
     fill_vectors<kPrepThreads>(flag ? reinterpret_cast<uint4*>(acc) : reinterpret_cast<uint4*>(out), flag ? n / 4 : n / 8, gridDim.x > kFewCtas);

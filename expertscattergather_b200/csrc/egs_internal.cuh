@@ -81,7 +81,7 @@ struct Div {
 // ------------------------------------------------------------------------------------------------
 
 // The plan of a scatter with 16-bit tensors on the tensor cores, words on the device: whether its token rows accumulate in the float32 rows
-// (else additions go straight into the 16-bit output); CTAs that have added what they had to (zero at first).
+// (else additions go straight into the 16-bit output); for each column tile the units that have been added (zero at first).
 enum PlanWords { kPlanHot = 0, kPlanAdded = 1, kPlanWords = 64 };
 
 struct RowGemmParams {

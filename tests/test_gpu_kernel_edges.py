@@ -469,6 +469,28 @@ def test_scatter16_rounds_small_outputs(cuda_device, B, T, E, K, C, N, form):
     assert torch.equal(got.cpu(), torch.from_numpy(ref).to(torch.bfloat16))
 
 
+# ... column tile by column tile in the scatter kernel, where no token row gets more than half of the limit's contributions in the mean and the
+# tiles have a counter each: launches of a call with a counting preparation.  CTAs of one unit and of several, one tile and many.
+@pytest.mark.parametrize("B,T,E,K,C,N,launches", [(1, 5, 2, 40, 8, 8, 2), (1, 5, 3, 27, 8, 8, 3), (1, 64, 64, 16, 128, 256, 2), (1, 64, 41, 25, 64, 256, 3), (1, 512, 5, 16, 64, 128, 2),
+                                                  (1, 513, 5, 16, 64, 128, 3), (1, 2048, 512, 64, 64, 32, 2), (1, 8, 2, 64, 32, 992, 2), (1, 8, 2, 64, 32, 1008, 3), (3, 100, 60, 8, 64, 200, 2)])
+@pytest.mark.parametrize("hot", [True, False])
+def test_scatter16_rounds_column_tiles(cuda_device, B, T, E, K, C, N, launches, hot):
+    g = torch.Generator().manual_seed(N)
+    Ind = torch.randint(0, T, (B, E, K), generator=g)
+    if hot:
+        Ind[B - 1].view(-1)[:40] = T - 1
+    Y = torch.randint(-7, 8, (B, E, K, C), generator=g).to(torch.bfloat16)
+    W = torch.randint(-7, 8, (E, C, N), generator=g).to(torch.bfloat16)
+    ref = torch.from_numpy(orc.np_scatter(Y, W, Ind, T)).to(torch.bfloat16)
+    d = [t.to(cuda_device) for t in (Y, W, Ind)]
+    n = ops.launch_count()
+    got = ops.gemm_scatter(*d, T)
+    assert ops.launch_count() - n == launches
+    if hot:
+        assert torch.equal(got.cpu(), ref)
+    ops.check_status()
+
+
 # kernels become resident under the end of the ones before them: operators issued back to back, with nothing of torch between them, have to
 # give what they give one by one.  Each reads what the one before it has just written, or writes what it has just read: every family of
 # kernels, with and without prepared indices, more than one wave of tiles, the helper stream's fork and join.  A column of the weights has one
