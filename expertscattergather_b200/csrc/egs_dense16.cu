@@ -74,7 +74,7 @@ struct __align__(16) DenseHeader {
   unsigned long long last;               // ... and the column tiles that this CTA was the last to add to
   uint32_t tmem_base;
   uint32_t abort_flag;
-  uint32_t freed;                        // S whose rows stay: steps whose slot the TMA warp has found free
+  uint32_t reached;                      // S whose rows stay: step that the TMA warp has come to, of those that begin a row block or follow the last
   int rounds;                            // S: float32 rows are to be rounded here ...
 };
 static_assert(sizeof(DenseHeader) <= kDenseHeader, "header does not fit");
@@ -335,7 +335,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     hdr->abort_flag = p.status.timed_out() ? 1u : 0u;
     hdr->rounds = 0;
     hdr->last = 0ull;
-    hdr->freed = 0u;
+    hdr->reached = 0u;
     if (smem_misaligned(smem_raw)) {
       hdr->abort_flag = 1u;
       p.status.report(EGS_STATUS_INTERNAL);
@@ -383,23 +383,24 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     // the groups would meet each barrier in turn, and a warp that is late to look at a phase whose stage another group loads finds the one
     // after it done as well, which a parity cannot tell from neither being done.
     auto is_mine = [&]() { return kGroups == 1 || (at.slot & (kGroups - 1)) == group; };
-    // Rows that stay are loaded with their first column tile only; with the others these warps would follow phases that they have no part in.
-    // They ask the TMA warp, which has a part in every stage, how far the ring is.
-    uint32_t n = 0;                      // steps before this one
-    auto wait_turn = [&]() {
-      auto there = [&]() {
-        uint32_t freed;
-        asm volatile("ld.acquire.cta.shared::cta.b32 %0, [%1];" : "=r"(freed) : "r"(smem_u32(&hdr->freed)) : "memory");
-        return __all_sync(0xffffffffu, freed > n) != 0;
-      };
-      for (const long long t0 = clock64(); !there();) {
+    // Rows that stay are loaded with their first column tile only.  With the others these warps have no part in the stages, and one that is late by
+    // a turn of the ring finds the phase after the one that it looks for done as well, which a parity cannot tell from neither being done.  It would
+    // wait forever, but the TMA warp, which has a part in every stage, says when it has come to the next row block: all phases before are done then.
+    auto wait_passed = [&](uint32_t next_block) {          // for the stage at `at`, or that the step of this number has been reached
+      if (at.round == 0) return;
+      const uint32_t bar = smem_u32(&hdr->empty[at.slot]), parity = (at.round - 1) & 1;
+      const long long t0 = clock64();
+      while (!__all_sync(0xffffffffu, mbar_try(bar, parity) != 0u)) {
+        uint32_t reached;
+        asm volatile("ld.acquire.cta.shared::cta.b32 %0, [%1];" : "=r"(reached) : "r"(smem_u32(&hdr->reached)) : "memory");
+        if (__all_sync(0xffffffffu, reached >= next_block)) return;
         if (!__any_sync(0xffffffffu, *abort_flag != 0u || clock64() - t0 > kWaitLimitCycles)) continue;
         if (lane == 0 && !*abort_flag) {
           *abort_flag = 1u;
           p.status.report(EGS_STATUS_PIPELINE_TIMEOUT);
         }
         alive = false;
-        break;
+        return;
       }
     };
     const uint32_t full0 = map_to_cta(smem_u32(&hdr->full[0]), 0);
@@ -407,6 +408,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       constexpr int kQuads = kTileM / kParts / 4;        // G, S: 16 rows a warp
       const int steps = (p.C + kStep - 1) / kStep;
       int t = 0, a_slot = 0;
+      uint32_t done = 0;                                 // steps up to the end of this tile
       for (Walk<OP, PAIR, KEEP> u(p); u.left > 0 && alive; u.next(), ++t) {
         alive = mbar_wait_all(smem_u32(&hdr->ids_full[t & 1]), (t >> 1) & 1, abort_flag, p.status.word);
         if (!alive) break;
@@ -415,15 +417,15 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
         for (int q = 0; q < kQuads; ++q) get4(table + static_cast<uint32_t>((t & 1) * kTileM + (part * kQuads + q) * 4) * 4u, row[q]);
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&hdr->ids_empty[t & 1]));
+        if (KEEP) done += steps;
         for (int k = 0; k < steps; ++k) {
           const bool mine = is_mine();
-          if (!KEEP && mine) wait_free();
-          if (KEEP && u.j == 0) wait_turn();
+          if (KEEP && u.j > 0) wait_passed(done + (u.tiles - u.j - 1) * steps);
+          else if (mine) wait_free();
           if (!alive) break;
           const int slot = at.slot;
           const uint32_t bar = full0 + slot * 8u;
           at.next(stages);
-          ++n;
           if (KEEP && u.j > 0) continue;     // (the rows are there)
           const uint32_t dst = a_tile(KEEP ? a_slot : slot) + static_cast<uint32_t>(part * kQuads) * 512u;
           if (KEEP && ++a_slot == p.a_slots) a_slot = 0;
@@ -898,7 +900,10 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
     const uint32_t bytes = PAIR ? 2u * stage_bytes : (OP != kOpDweight ? n_bytes : (p.swap ? kMTile : n_bytes)) + ((OP == kOpScatter && p.tma_rows) ? kMTile : 0u);
     bool ok = true;
     int a_slot = 0;
-    uint32_t freed = 0;
+    uint32_t n = 0;                      // steps before this tile
+    auto tell_reached = [&]() {
+      if (gathers && lane == 0) asm volatile("st.release.cta.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hdr->reached)), "r"(n) : "memory");
+    };
     Cursor at;
     for (Walk<OP, PAIR, KEEP> u(p); u.left > 0 && ok; u.next()) {
       const int steps = u.steps();
@@ -911,6 +916,10 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
       const uint32_t unit_bytes = less ? 2u * (kMTile + static_cast<uint32_t>(u.segs()) * kSeg) : bytes;
       int m = OP == kOpDweight ? u.split * p.rows_per_split : u.m0;
       int b = p.by_k.quotient(m), k = m - b * p.K;     // first slot row of the step
+      if (KEEP) {
+        if (u.j == 0) tell_reached();
+        n += steps;
+      }
       for (int ks = 0, c0 = 0; ks < steps; ++ks, c0 += kStep) {
         if (at.round > 0) {
           ok = mbar_wait_all(smem_u32(&hdr->empty[at.slot]), (at.round - 1) & 1, abort_flag, p.status.word);
@@ -928,7 +937,6 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           else tma_load_4d(dst, &map_rows, x, k, u.e, b, bar);
         };
         if (elect_one()) {
-          if (KEEP && gathers) asm volatile("st.release.cta.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hdr->freed)), "r"(freed + 1u) : "memory");
           if (leader) mbar_arrive_expect_tx(own, rows_too ? unit_bytes : (PAIR ? 2u : 1u) * n_bytes);
           if (OP != kOpDweight) {
             if (OP == kOpScatter && p.tma_rows && rows_too) box4(KEEP ? a_tile(a_slot) : base, c0);
@@ -950,13 +958,13 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(kDenseThr
           }
         }
         if (KEEP && rows_too && ++a_slot == p.a_slots) a_slot = 0;
-        ++freed;
         if (OP == kOpDweight) {
           k += kStep;                                  // 64 rows are parts of one batch element or whole ones
           while (k >= p.K) { k -= p.K; ++b; }
         }
       }
     }
+    if (KEEP && ok) tell_reached();
     __syncwarp();
   }
 

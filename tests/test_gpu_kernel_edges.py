@@ -574,6 +574,23 @@ def test_scatter_rows_that_stay(cuda_device, B, T, E, K, N, C, kept, full, w_lay
     ops.check_status()
 
 
+# ... gathered rows, which the gathering warps load with a row block's first column tile only: even and odd numbers of stages, row blocks of
+# fewer and of more steps than stages, and all of several results back to back
+@pytest.mark.parametrize("B,E,K,N,C,w_layout,stages", [(4, 50, 37, 512, 512, "cn", 4), (9, 37, 37, 512, 392, "nc", 5), (4, 31, 36, 992, 416, "nc", 5), (7, 50, 57, 616, 144, "cn", 6),
+                                                       (9, 52, 43, 624, 176, "nc", 7)])
+def test_gathered_scatter_rows_that_stay(cuda_device, B, E, K, N, C, w_layout, stages):
+    T = 300
+    Ind, Y, W, _, _ = _sparse_scatter(cuda_device, B, T, E, K, N, C)
+    plan = ops.describe_plan("S", B, T, E, K, C, N, torch.bfloat16, w_layout=w_layout)
+    assert ops.describe_kept_rows(B, T, E, K, C, N, torch.bfloat16, w_layout=w_layout)[0] > 1 and (plan["pair"], plan["slot_boxes"], plan["stages"]) == (1, 0, stages)
+    Out = _scatter_sum(Ind, torch.einsum("bekc,ecn->bekn", Y, W), torch.zeros(B, T, N, device=cuda_device)).bfloat16()
+    args = Y.bfloat16(), (W if w_layout == "cn" else W.transpose(1, 2).contiguous()).bfloat16(), Ind, T
+    got = [ops.gemm_scatter(*args, w_layout=w_layout) for _ in range(10)]
+    ops.check_status()
+    for x in got:
+        assert torch.equal(x, Out)
+
+
 # ... and the other forms of the operator: a bias, an output that is added to, a hot token row (float32 rows), both 16-bit types
 @pytest.mark.parametrize("B,T,E,K,N,C", [(16, 700, 60, 64, 768, 256), (20, 500, 50, 96, 760, 256), (8, 300, 64, 32, 1000, 320)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
