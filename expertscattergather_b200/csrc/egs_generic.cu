@@ -699,10 +699,10 @@ constexpr int kPrepOwnIds = 8192;
 // whether a token row of batch elements b0 .. b0 + nb - 1 gets more than `limit` contributions, counted by the whole CTA;
 // cnt: [min(nb * T_, kPrepCounters)].  Eight ids of a thread are on their way at a time: one after the other, the counting of 8 batch
 // elements of 8192 ids took 17 us of device time, all scatters of such sizes 8 us longer (bf16, T=2048, 64 experts, 512 -> 2048 features: 140 us,
-// now 132; 32 elements of 4096 ids, 128 -> 512 features: 54 and 50).
-template <bool ONE>
+// now 132; 32 elements of 4096 ids, 128 -> 512 features: 54 and 50).  Four where the CTAs that fill count for themselves (see
+// scatter_prepare_kernel).
+template <bool ONE, int kAtOnce>
 __device__ __forceinline__ int has_hot_row(const void* ind, int index_dtype, int b0, int nb, int T_, int EK, int limit, int* cnt) {
-  constexpr int kAtOnce = 8;
   const int tid = threadIdx.x, nc = static_cast<int>(min(static_cast<long long>(nb) * T_, static_cast<long long>(kPrepCounters)));
   for (int t = tid; t < nc; t += kPrepThreads) cnt[t] = 0;
   __syncthreads();
@@ -732,13 +732,16 @@ __global__ void __launch_bounds__(kPrepThreads) scatter_count_kernel(const void*
   pdl_wait();
   pdl_trigger();
   int flag = 0;
-  for (int b = blockIdx.x; b < B && !flag; b += gridDim.x) flag = has_hot_row<true>(ind, index_dtype, b, 1, T_, EK, limit, prep_cnt);
+  for (int b = blockIdx.x; b < B && !flag; b += gridDim.x) flag = has_hot_row<true, 8>(ind, index_dtype, b, 1, T_, EK, limit, prep_cnt);
   if (threadIdx.x == 0) flags[blockIdx.x] = flag;
 }
 
-// COUNT: the CTAs count for themselves (an instance of its own: with the registers that counting takes an SM holds three CTAs, not four)
+// COUNT: the CTAs count for themselves, an instance of its own.  Four CTAs of either are on an SM, as many as the grid counts on: with eight ids at a
+// time counting took registers for three, and the fourth quarter of the grid counted when the others had filled (bf16, whole scatters: 2
+// batch elements of 1956 tokens, 156 ids each, 120 -> 928 features 9.9 us without, 11.0 with eight ids, 10.0 with four; 1 of 5006, 448 ids, 480 -> 1632
+// 13.5, 14.4 and 13.3; 1 of 8192, 8192 ids, 256 -> 1024 26.3, 20.3 and 19.7).
 template <typename T, bool COUNT>
-__global__ void __launch_bounds__(kPrepThreads) scatter_prepare_kernel(const void* ind, int index_dtype, int B, int T_, int EK,
+__global__ void __launch_bounds__(kPrepThreads, 4) scatter_prepare_kernel(const void* ind, int index_dtype, int B, int T_, int EK,
                                                                        const int* info, const int* flags, int nflags,
                                                                        int limit, int* plan, float* acc,
                                                                        T* out, size_t n, int zero_output, StatusRef status) {
@@ -755,7 +758,7 @@ __global__ void __launch_bounds__(kPrepThreads) scatter_prepare_kernel(const voi
     for (int i = tid; i < nflags; i += kPrepThreads) flag |= flags[i];
     flag = __syncthreads_or(flag);
   } else if (COUNT) {
-    flag = B == 1 ? has_hot_row<true>(ind, index_dtype, 0, 1, T_, EK, limit, prep_cnt) : has_hot_row<false>(ind, index_dtype, 0, B, T_, EK, limit, prep_cnt);
+    flag = B == 1 ? has_hot_row<true, 4>(ind, index_dtype, 0, 1, T_, EK, limit, prep_cnt) : has_hot_row<false, 4>(ind, index_dtype, 0, B, T_, EK, limit, prep_cnt);
   }
   if (blockIdx.x == 0 && tid < kPlanWords) plan[tid] = tid == kPlanHot ? flag : 0;
   // (n is a multiple of 8 elements and both buffers are 16-byte aligned: tensor-core path only)
