@@ -1023,8 +1023,10 @@ bool whole_segments(int width, int staged, bool pair) { return staged % 64 == 0 
 // share of the copies, and the barriers of a step take 600 (800 in a scatter that gathers its rows).  In G the copies of single CTAs, handed over
 // by their threads, hold a step up to 750 where there is more than one wave of them, and a pair's gathers beside less than 64 columns to
 // 850 (weights [E, N, C]: 750).  With 600 there all of these stayed on single CTAs: 512 rows of 256 experts, 512 -> 128 features, 33.3 us, on
-// pairs 30.3; 5724 of 10, 1056 -> 136, 41.5 and 37.4; 4515 of 45, 864 -> 104, 84 and 65; and these still do: 254 of 234, 592 -> 40, 21.3 and 23.1;
-// 104 of 10, 1408 -> 88, 12.6 and 13.3.  Of 320 calls of G, sizes drawn, the 50 that went to pairs take 0.74 to 1.04 of the time, 0.92 in the mean.
+// pairs 30.3; 5724 of 10, 1056 -> 136, 41.5 and 37.4; 4515 of 45, 864 -> 104, 84 and 65.  Of 1600 calls of G, sizes drawn, 174 run otherwise than with 600
+// and take 0.91 of the time in the mean; the slowest 1.08 (1292 rows of 109 experts, 328 -> 280, on pairs), 1.06 (2400 of 12, 152 -> 304, tiles of 160, not
+// 112) and 1.05 (1085 of 20, 704 -> 88).  Widths that are held up alike cost the same here, but more columns still take longer: of those
+// that need as many waves only the narrowest is looked at (133 experts of 296 rows, 1432 -> 280: 80.8 us with tiles of 144, 88.2 with 176).
 // Read-out takes epi clocks a
 // column beside the next tile's main loop; the additions of a scatter share the way to the L2 with the loads, and half of the shorter
 // one shows.  Units go out in waves of one per SM or pair of SMs; a pair starts and ends 2500 clocks slower.
@@ -1082,6 +1084,7 @@ Tile pick_tile(int n, int m, long long groups, int steps, double lsu0, double ls
       const long long tiles = (n + bn - 1) / bn;
       const int staged = pair ? bn / 2 : bn;
       const long long units = row_units * tiles, waves = (units + sms - 1) / sms;
+      if (gather && !pair && waves > 1 && bn > unit16 && (row_units * ((n + bn - unit16 - 1) / (bn - unit16)) + sms - 1) / sms == waves) continue;
       const double least = scatter && lsu0 > 0.0 ? 800.0 : !gather ? 600.0 : pair ? (std::min(bn, n) >= 64 ? 600.0 : nc_tile ? 750.0 : 850.0) : waves > 1 ? 750.0 : 600.0;
       double step = per_row * (128 + staged);
       if (2.0 * bn > step) step = 2.0 * bn;

@@ -333,6 +333,15 @@ def test_dense16_last_wave_in_half_tiles(cuda_device, B, T, E, K, I, J):
     ops.check_status()
 
 
+# G on single CTAs: of the widths that need as many waves the narrowest; a wider one where it saves a wave; pairs where copies hold steps up
+@pytest.mark.parametrize("B,T,E,K,C,N,pair,tile_n", [(37, 388, 133, 8, 1432, 280, 0, 144), (15, 350, 85, 19, 504, 264, 0, 144), (1, 1021, 238, 69, 1240, 280, 0, 144), (2, 5283, 78, 13, 1840, 264, 0, 96),
+                                                     (5, 676, 56, 138, 152, 200, 0, 208), (1, 3265, 195, 75, 72, 128, 0, 128), (32, 1024, 256, 16, 512, 128, 1, 128)])
+@pytest.mark.parametrize("w_layout", ["cn", "nc"])
+def test_dense16_gather_tiles(cuda_device, B, T, E, K, C, N, pair, tile_n, w_layout):
+    plan = ops.describe_plan("G", B, T, E, K, C, N, torch.bfloat16, w_layout=w_layout)
+    assert (plan["pair"], plan["tile_n"]) == (pair, tile_n)
+
+
 # weight gradients on pairs whose slot rows are gathered too, with an odd and an even number of stages (two groups of warps share the ring's
 # slots), widths whose last tile is narrow, ranges that end within a batch of ids.  Small integers: exact in float32, then rounded once.
 @pytest.mark.parametrize("B,T,E,K,FG,FD,stages", [(9, 300, 24, 101, 1000, 200, 5), (39, 80, 13, 21, 1936, 344, 5), (20, 90, 74, 45, 512, 520, 5), (15, 200, 74, 64, 512, 512, 6)])
