@@ -28,7 +28,7 @@ EXPORTS = (
     "egs_version", "egs_status_string", "egs_last_cuda_error", "egs_gather_gemm", "egs_gemm_scatter",
     "egs_dweight", "egs_dweight_static_scratch", "egs_static_scratch_max_elements", "egs_dw_workspace_bytes", "egs_scatter_workspace_bytes", "egs_tensor_path_eligible", "egs_fill_zero", "egs_launch_count",
     "egs_gather_scatter_pair", "egs_fused_pair_eligible", "egs_dweight_prezeroed", "egs_selftest_wait_timeout",
-    "egs_describe_plan", "egs_describe_kept_rows", "egs_gather_gemm_bias", "egs_gemm_scatter_bias", "egs_route_topk", "egs_index_csr",
+    "egs_describe_plan", "egs_describe_kept_rows", "egs_describe_half_tiles", "egs_gather_gemm_bias", "egs_gemm_scatter_bias", "egs_route_topk", "egs_index_csr",
     "egs_index_csr_scratch_bytes", "egs_index_compact", "egs_gemm_scatter_prepared", "egs_gemm_scatter_csr",
     "egs_set_status_mirror", "egs_expert_row_sum",
 )
@@ -94,6 +94,8 @@ def _declare(lib: ctypes.CDLL) -> None:
     lib.egs_gemm_scatter_csr.argtypes = [vp, vp, vp, vp, vp, vp, ctypes.POINTER(Dims), i, i, i, vp]
     lib.egs_describe_kept_rows.restype = i
     lib.egs_describe_kept_rows.argtypes = [ctypes.POINTER(Dims), i, i, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]
+    lib.egs_describe_half_tiles.restype = i
+    lib.egs_describe_half_tiles.argtypes = [ctypes.POINTER(Dims), i, i, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]
     lib.egs_describe_plan.restype = i
     lib.egs_describe_plan.argtypes = [i, ctypes.POINTER(Dims), i, i, i, ctypes.POINTER(PlanInfo)]
     lib.egs_set_status_mirror.restype = i

@@ -669,6 +669,21 @@ int egs_describe_kept_rows(const egs_dims* dims, int w_layout, int dtype, int* k
   return EGS_OK;
 }
 
+int egs_describe_half_tiles(const egs_dims* dims, int w_layout, int dtype, int* units, int* first_columns) {
+  egs_plan_info info;
+  if (!units || !first_columns) return EGS_ERR_INVALID_ARGUMENT;
+  if (int rc = egs_describe_plan(0, dims, w_layout, dtype, EGS_PREC_STRICT, &info)) return rc;
+  *units = *first_columns = 0;
+  if (info.tile_n == 0 || dtype == EGS_F32) return EGS_OK;
+  RowGemmParams p{};
+  p.E = static_cast<int>(dims->E); p.K = static_cast<int>(dims->K); p.C = static_cast<int>(dims->C); p.N = static_cast<int>(dims->N);
+  p.M = static_cast<int>(dims->B * dims->K);
+  p.w_layout = w_layout;
+  configure_dense16_rowgemm(p, false);
+  dense16_half_tiles(p, units, first_columns);
+  return EGS_OK;
+}
+
 int egs_tensor_path_eligible(int op, const egs_dims* dims, int dtype, const void* const* pointers, int n_pointers) {
   if (!dims || !valid_dtype(dtype) || op < 0 || op > 2) return 0;
   if (!device_is_sm100()) return 0;

@@ -1139,12 +1139,17 @@ void plan_walk(DenseParams& p, bool pair) {
 // of one of 256, so that 3.46 waves take as long as 3.75, not four.  bf16, 32 experts of 2048 rows, 768 -> 192 features 30.1 -> 28.2 us, 24 of 909,
 // 1000 -> 200 25.1 -> 23.0, 20 of 1024, 768 -> 512 25.1 -> 23.0.  D, which runs beside the dX / dY kernel and leaves it the idle pairs, keeps whole
 // tiles: alone 35.3 -> 33.3 us, but a training step of ragged sizes 139.5 -> 142.
-void plan_tail(DenseParams& p) {
-  const int pairs = kSms / 2, rest = p.units % pairs, first = (p.BN / 2 + 31) / 32 * 32, last = p.N - (p.tiles_n - 1) * p.BN;
-  if (p.units < pairs || rest == 0 || 2 * rest > pairs || p.BN < 128 || last <= first || (p.whole && first % 128 != 0)) return;
-  p.full_waves = p.units / pairs;
-  p.tail = 2 * rest;
-  p.tail_bn = first;
+struct Tail {
+  int full_waves = 0, units = 0, first = 0;      // units of half a tile, columns of the first half
+};
+Tail plan_tail(int units, int bn, int n, bool whole) {
+  const int pairs = kSms / 2, rest = units % pairs, first = (bn / 2 + 31) / 32 * 32, last = n - (n - 1) / bn * bn;
+  Tail t;
+  if (units < pairs || rest == 0 || 2 * rest > pairs || bn < 128 || last <= first || (whole && first % 128 != 0)) return t;
+  t.full_waves = units / pairs;
+  t.units = 2 * rest;
+  t.first = first;
+  return t;
 }
 
 template <typename T, int OP, bool PAIR, bool KEEP>
@@ -1179,6 +1184,16 @@ void configure_dense16_rowgemm(RowGemmParams& p, bool scatter) {
   p.stages = r.stages;
   p.row_tiles = 1;
   p.persistent = 1;
+}
+
+void dense16_half_tiles(const RowGemmParams& r, int* units, int* first) {
+  *units = *first = 0;
+  if (!r.pair) return;
+  const long long all = static_cast<long long>((r.M + 2 * kTileM - 1) / (2 * kTileM)) * ((r.N + r.BN - 1) / r.BN) * r.E;
+  if (all > 2147483647ll - kSms) return;
+  const Tail t = plan_tail(static_cast<int>(all), r.BN, r.N, r.w_layout != EGS_W_NC && whole_segments(r.N, r.BN / 2, true));
+  *units = t.units;
+  *first = t.first;
 }
 
 cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dtype, cudaStream_t st) {
@@ -1228,7 +1243,12 @@ cudaError_t launch_dense16_rowgemm(const RowGemmParams& r, bool scatter, int dty
     return !r.pair           ? launch_typed<kOpScatter, false>(p, dtype, mw, mr, st)
            : r.tile_group > 0 ? launch_typed<kOpScatter, true, true>(p, dtype, mw, mr, st)
                               : launch_typed<kOpScatter, true>(p, dtype, mw, mr, st);
-  if (r.pair) plan_tail(p);
+  if (r.pair) {
+    const Tail t = plan_tail(p.units, p.BN, p.N, p.whole != 0);
+    if (t.units > 0) p.full_waves = t.full_waves;
+    p.tail = t.units;
+    p.tail_bn = t.first;
+  }
   return r.pair ? launch_typed<kOpGather, true>(p, dtype, mw, mr, st) : launch_typed<kOpGather, false>(p, dtype, mw, mr, st);
 }
 

@@ -184,6 +184,8 @@ cudaError_t launch_tensor_dweight(const DWeightParams& p, size_t smem_bytes, cud
 
 // 16-bit tensors (egs_dense16.cu): persistent kernels for G, S and D.
 void configure_dense16_rowgemm(RowGemmParams& p, bool scatter);
+// G as configured: units of half a tile in the last wave, columns of the first half (see plan_tail)
+void dense16_half_tiles(const RowGemmParams& p, int* units, int* first);
 cudaError_t launch_dense16_rowgemm(const RowGemmParams& p, bool scatter, int dtype, cudaStream_t st);
 void configure_dense16_dweight(DWeightParams& p);
 cudaError_t launch_dense16_dweight(const DWeightParams& p, int dtype, cudaStream_t st);

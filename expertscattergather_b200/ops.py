@@ -15,7 +15,7 @@ import torch
 from . import _lib
 
 __all__ = ["gather_gemm", "gemm_scatter", "gather_scatter_pair", "fused_pair_eligible", "fused_pair_preferred", "dweight", "fill_zero", "side_stream", "fill_stream", "set_precision", "get_precision", "set_path", "get_path",
-           "check_status", "reset_status", "publish_status", "launch_count", "dtype_to_type_id", "tensor_path_eligible", "describe_plan", "describe_kept_rows", "route_topk", "build_index_csr", "compact_index", "gemm_scatter_csr", "IndexCSR"]
+           "check_status", "reset_status", "publish_status", "launch_count", "dtype_to_type_id", "tensor_path_eligible", "describe_plan", "describe_kept_rows", "describe_half_tiles", "route_topk", "build_index_csr", "compact_index", "gemm_scatter_csr", "IndexCSR"]
 
 _PRECISIONS = {"strict": _lib.PREC_STRICT, "fp32": _lib.PREC_STRICT, "tf32": _lib.PREC_TF32}
 _PATHS = {"auto": _lib.PATH_AUTO, "generic": _lib.PATH_GENERIC, "tensor": _lib.PATH_TENSOR,
@@ -313,6 +313,15 @@ def describe_kept_rows(B, T, E, K, C, N, dtype, *, w_layout="cn") -> tuple[int, 
                                             ctypes.byref(kept), ctypes.byref(full))
     _lib.check(rc, "egs_describe_kept_rows")
     return kept.value, full.value
+
+
+def describe_half_tiles(B, T, E, K, C, N, dtype, *, w_layout="cn") -> tuple[int, int]:
+    """(units, first_columns) of the last wave of the 16-bit gather 'auto' runs at these sizes (see ``egs_describe_half_tiles``)."""
+    dims, units, first = _lib.Dims(B, T, E, K, C, N), ctypes.c_int(), ctypes.c_int()
+    rc = _lib.load().egs_describe_half_tiles(ctypes.byref(dims), _lib.W_CN if w_layout == "cn" else _lib.W_NC, dtype_to_type_id(dtype),
+                                             ctypes.byref(units), ctypes.byref(first))
+    _lib.check(rc, "egs_describe_half_tiles")
+    return units.value, first.value
 
 
 _TORCH_INDEX = {torch.int64: _lib.I64, torch.int32: _lib.I32, torch.int16: _lib.I16}

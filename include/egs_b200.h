@@ -288,6 +288,10 @@ int egs_describe_plan(int op, const egs_dims* dims, int w_layout, int dtype, int
  * rows are loaded for every column tile, and for anything but 16-bit tensors on the tensor cores.  (Diagnostic, like egs_describe_plan.) */
 int egs_describe_kept_rows(const egs_dims* dims, int w_layout, int dtype, int* kept_tiles, int* full_waves);
 
+/* The last wave of the 16-bit gather that EGS_PATH_AUTO runs on pairs of SMs at these sizes, where its tiles are cut in two: *units halves, the first
+ * of each *first_columns wide.  Both 0 where tiles stay whole, and for anything else.  (Diagnostic, like egs_describe_plan.) */
+int egs_describe_half_tiles(const egs_dims* dims, int w_layout, int dtype, int* units, int* first_columns);
+
 /*
  * Row sums per expert:  out[e, n] = sum over (b, k) of a row of Src.  Ind given: the token row Ind[b,e,k] of Src [B,T,N] (the
  * gradient of a per-slot scatter bias); Ind NULL: the slot row of Src [B,E,K,N] (the gradient of a gather bias).  Summed in

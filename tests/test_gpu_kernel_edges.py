@@ -312,11 +312,11 @@ def test_dense16_dweight_sums_long_contractions_in_ranges(cuda_device, B, T, E, 
     assert torch.stack(bias).mean().abs().item() <= 8192 / 16 * 2.0 ** -23
 
 
-# G on pairs whose last wave is half empty or more: its tiles are cut in two.  Columns that come as boxes of whole segments and of partial ones,
-# weights of both layouts; D on pairs beside it, with either operand gathered.  Small integers: exact in float32, then rounded once.
+# G and D at sizes of one to four waves, on pairs and on single CTAs; columns that come as boxes of whole segments and of partial ones, weights of
+# both layouts.  Small integers: exact in float32, then rounded once.
 @pytest.mark.parametrize("B,T,E,K,I,J", [(6, 100, 38, 101, 456, 192), (15, 100, 11, 32, 1032, 432), (11, 100, 52, 50, 400, 224), (7, 100, 56, 64, 704, 232),
                                          (11, 100, 15, 64, 912, 640), (11, 100, 33, 50, 424, 248), (9, 100, 48, 45, 816, 256), (20, 90, 40, 64, 512, 512)])
-def test_dense16_last_wave_in_half_tiles(cuda_device, B, T, E, K, I, J):
+def test_dense16_few_waves(cuda_device, B, T, E, K, I, J):
     plans = [ops.describe_plan(op, B, T, E, K, I, J, torch.bfloat16, w_layout=w) for op, w in (("G", "cn"), ("G", "nc"), ("D", "cn"))]
     assert any(p["pair"] and p["tile_n"] >= 128 for p in plans), plans
     g = torch.Generator().manual_seed(I)
@@ -342,6 +342,27 @@ def test_dense16_gather_tiles(cuda_device, B, T, E, K, C, N, pair, tile_n, w_lay
     assert (plan["pair"], plan["tile_n"]) == (pair, tile_n)
 
 
+# G on pairs whose last wave is half empty or more: its tiles are cut in two, into halves of 128 and 96, 96 and 96 or 64, 128 and 128 columns (fewer
+# in a row's last tile), boxes of whole segments and of partial ones.  Small integers: exact in float32, then rounded once.
+@pytest.mark.parametrize("B,E,K,I,J,first", [(27, 10, 70, 648, 152, 96), (23, 11, 76, 392, 320, 96), (20, 10, 94, 584, 192, 96), (20, 9, 73, 592, 360, 96), (19, 10, 97, 400, 216, 128),
+                                             (25, 9, 52, 424, 424, 128), (31, 10, 41, 400, 448, 128), (23, 10, 52, 392, 464, 128), (32, 9, 75, 400, 256, 128), (16, 11, 65, 416, 512, 128)])
+@pytest.mark.parametrize("dtype,bias", [(torch.bfloat16, False), (torch.float16, True)])
+def test_dense16_last_wave_in_half_tiles(cuda_device, B, E, K, I, J, first, dtype, bias):
+    T = 100
+    g = torch.Generator().manual_seed(I)
+    X, W = torch.randint(-2, 3, (B, T, I), generator=g).to(dtype), torch.randint(-1, 2, (E, I, J), generator=g).to(dtype)
+    Ind = torch.randint(0, T, (B, E, K), generator=g)
+    b = torch.randint(-5, 6, (E, J), generator=g).to(dtype) if bias else None
+    ref = orc.np_gather(X, W, Ind) + (b.double().numpy()[None, :, None] if bias else 0.0)
+    d = lambda t: None if t is None else t.to(cuda_device)
+    for w_layout in ("cn", "nc"):
+        units, first_columns = ops.describe_half_tiles(B, T, E, K, I, J, dtype, w_layout=w_layout)
+        assert units > 0 and first_columns == first
+        got = ops.gather_gemm(d(X), d(W if w_layout == "cn" else W.transpose(1, 2).contiguous()), d(Ind), w_layout=w_layout, bias=d(b))
+        assert torch.equal(got.cpu(), torch.from_numpy(ref).to(dtype))
+    ops.check_status()
+
+
 # weight gradients on pairs whose slot rows are gathered too, with an odd and an even number of stages (two groups of warps share the ring's
 # slots), widths whose last tile is narrow, ranges that end within a batch of ids.  Small integers: exact in float32, then rounded once.
 @pytest.mark.parametrize("B,T,E,K,FG,FD,stages", [(9, 300, 24, 101, 1000, 200, 5), (39, 80, 13, 21, 1936, 344, 5), (20, 90, 74, 45, 512, 520, 5), (15, 200, 74, 64, 512, 512, 6)])
@@ -357,10 +378,11 @@ def test_dense16_dweight_groups_share_the_ring(cuda_device, B, T, E, K, FG, FD, 
     if out_layout == "direct_rows":
         ref = ref.transpose(1, 2)
     d = [t.to(cuda_device) for t in (X, Y, Ind)]
-    for _ in range(10):
-        got = ops.dweight(*d, out_layout=out_layout)
+    got = [ops.dweight(*d, out_layout=out_layout) for _ in range(10)]
     ops.check_status()
-    assert torch.equal(got.cpu(), ref.to(torch.bfloat16))
+    ref = ref.to(torch.bfloat16).to(cuda_device)
+    for x in got:
+        assert torch.equal(x, ref)
 
 
 # the first CUDA call of a thread: boxes are described to the driver before anything else has made a context current there
@@ -497,6 +519,52 @@ def test_scatter16_rounds_column_tiles(cuda_device, B, T, E, K, C, N, launches, 
     assert ops.launch_count() - n == launches
     if hot:
         assert torch.equal(got.cpu(), ref)
+    ops.check_status()
+
+
+# what large buffers are zeroed and rounded by goes in stretches with a CTA each: sizes just beyond where that begins, last stretches that are not
+# whole.  The allocator hands out blocks that hold NaN.
+def _leave_nan_blocks(dev, *byte_counts):
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    blocks = [torch.full((n,), -1, dtype=torch.uint8, device=dev) for n in byte_counts]
+    torch.cuda.synchronize()
+    del blocks
+
+
+def test_fills_in_stretches(cuda_device):
+    for n in ((32 << 20) + 16, (32 << 20) + 3 * 16384 + 7 * 16 + 5):
+        x = torch.full((n + 64,), 255, dtype=torch.uint8, device=cuda_device)
+        ops.fill_zero(x[:n])
+        assert not x[:n].any().item() and (x[n:] == 255).all().item()
+
+
+@pytest.mark.parametrize("dtype,N", [(torch.float32, 808), (torch.bfloat16, 1608), (torch.float16, 1608)])
+@pytest.mark.parametrize("hot", [False, True])
+def test_scatter_into_zeros_in_stretches(cuda_device, dtype, N, hot):
+    B, T, E, K, C = 3, 17479, 4, 64, 64
+    n = B * T * N * (4 if dtype == torch.float32 else 2)
+    assert n > 160 << 20
+    Ind, Y, W, _, _ = _sparse_scatter(cuda_device, B, T, E, K, N, C)
+    if hot:
+        Ind[1, :, :10] = T - 1
+    Out = _scatter_sum(Ind, torch.einsum("bekc,ecn->bekn", Y, W), torch.zeros(B, T, N, device=cuda_device))
+    _leave_nan_blocks(cuda_device, n, 2 * n + (1 << 20))
+    got = ops.gemm_scatter(Y.to(dtype), W.to(dtype), Ind, T)
+    assert torch.equal(got, Out.to(dtype))
+    ops.check_status()
+
+
+def test_dweight_rounds_ranges_in_stretches(cuda_device):
+    B, T, E, K, FG, FD = 129, 70, 8, 64, 1064, 1000
+    assert 4 * E * FG * FD > 32 << 20 and ops.describe_plan("D", B, T, E, K, FG, FD, torch.bfloat16)["splits"] > 1
+    g = torch.Generator(device=cuda_device).manual_seed(9)
+    X, Y = (torch.randint(-2, 3, s, generator=g, device=cuda_device).float() for s in ((B, T, FG), (B, E, K, FD)))
+    Ind = torch.randint(0, T, (B, E, K), generator=g, device=cuda_device)
+    ref = torch.stack([torch.cat([X[b, Ind[b, e]] for b in range(B)]).T @ Y[:, e].reshape(B * K, FD) for e in range(E)])      # (sums below 2^24: exact)
+    _leave_nan_blocks(cuda_device, 2 * E * FG * FD, 4 * E * FG * FD + (1 << 20))
+    got = ops.dweight(X.bfloat16(), Y.bfloat16(), Ind)
+    assert torch.equal(got, ref.bfloat16())
     ops.check_status()
 
 

@@ -40,3 +40,10 @@ def test_dependent_kernels_promise_nothing_about_aliases(kernel):
     through `__restrict__` pointers are not bound by the wait."""
     file, name, params, body = kernel
     assert "__restrict__" not in params + body, f"{file}: {name}"
+
+
+def test_ctas_that_count_for_themselves_are_resident_together():
+    """The grid of the kernel that counts ids and fills has four CTAs for an SM; one that has to wait for the others counts and fills after them."""
+    text = open(os.path.join(CSRC, "egs_generic.cu")).read()
+    assert re.search(r"__launch_bounds__\(kPrepThreads, 4\)\s+scatter_prepare_kernel", text)
+    assert "size_t grid = 4 * 148;" in text
