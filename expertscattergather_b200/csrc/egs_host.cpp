@@ -651,9 +651,9 @@ std::tuple<Tensor, Tensor, bool> gather_scatter_forward(const Tensor& X, const T
 }
 
 // dX, dWg, dWs; those not needed stay undefined
-std::array<Tensor, 3> gather_scatter_backward(const Tensor& X_, const Tensor& Wg, const Tensor& Ws, const Tensor& Ind_, const Tensor& Y,
+std::array<Tensor, 3> gather_scatter_backward(const Tensor& X_, const Tensor& Wg, const Tensor& Ws, const Tensor& Ind_, const Tensor& Y_,
                                               const Tensor& dOut_, bool fused, bool need_x, bool need_wg, bool need_ws) {
-  const Tensor X = X_.contiguous(), dOut = dOut_.contiguous(), Ind = index_tensor(Ind_).t;
+  const Tensor X = X_.contiguous(), dOut = dOut_.contiguous(), Y = Y_.contiguous(), Ind = index_tensor(Ind_).t;
   Tensor dX, dWg, dWs, dY, ws;
   std::optional<SideStream> side;
   const bool fork = worth_a_side_stream(Y, Wg);
