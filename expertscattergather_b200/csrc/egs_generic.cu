@@ -587,7 +587,9 @@ __global__ void __launch_bounds__(kSumThreads) expert_row_sum_kernel(const T* __
 // in order as CTAs leave, the stretches in flight lie together, and 1.07 GB are zeroed in 147 us (7.3 TB/s), 128 MB in 24.6 and 64 MB in 14.3; by a
 // few waves of CTAs that stride over all of it 176, 26.6 and 16.4 us.  24 MB take those 8.3 us, stretches 9.0.  Where a kernel starts under the
 // fill it does so under a grid of few waves only, and the fill in front of a 16-bit scatter has more to do in each CTA: whole scatters of
-// 134 MB take 172 us with stretches and 170 without, of 268 MB 107 and 113, of 1.07 GB 1340 and 1367.
+// 134 MB take 172 us with stretches and 170 without, of 268 MB 107 and 113, of 1.07 GB 1340 and 1367.  From 160 MB on they take 0.93 to 1.01 of the
+// time without, 1.02 to 1.03 in front of a long contraction (171 MB, 504 -> 1352 features: 107.6 and 104.8), and 0.93 to 0.99 where a hot row
+// doubles the bytes.
 // ------------------------------------------------------------------------------------------------
 constexpr int kStretch = 4;
 constexpr int kConvert = 2;                        // ... and twice as many 16-byte loads

@@ -506,8 +506,10 @@ bool worth_a_side_stream(const Tensor& slot_rows, const Tensor& W) {      // [B,
   return slots * W.numel() > (tensor ? kSmallTensorWork : kSmallGenericWork);
 }
 // Bias gradients of 16-bit tensors follow the weight gradient there: their row sums read memory under the end of the dX / dY kernel, whose last
-// wave leaves SMs free, where they stood alone behind it before.  Forward and backward in bf16, on the main and on the helper stream: 32 experts,
-// 768 and 192 features 237 and 230 us, 64 experts, 512 and 64 431 and 407, 24 of ragged sizes 180 and 176, 16, 512 and 256 148.7 and 149.  The
+// wave leaves SMs free, where they stood alone behind it before.  Forward and backward in bf16 through both modules, on the main and on the helper
+// stream: 32 experts, 768 and 192 features 237 and 230 us, 64 experts, 512 and 64 431 and 407, 24 of ragged sizes 180 and 176, 16, 512 and 256 148.7
+// and 149; through the ExpertScatter alone, whose dY kernel may come first, 129 and 135, 246 and 244, 99 and 105.  Where there is no dX / dY
+// kernel the sum belongs on the main stream, beside the weight gradient (an ExpertGather alone 70.1 us, behind it on the helper stream 78.6).  The
 // float32 weight gradients take longer than the dX / dY kernels, and sums behind them 1-4 % of a large pass (1024 and 256 features 674 and 695 us).
 struct Grads {
   Tensor in, w, b;
