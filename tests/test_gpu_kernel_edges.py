@@ -316,7 +316,7 @@ def test_dense16_dweight_sums_long_contractions_in_ranges(cuda_device, B, T, E, 
 # both layouts.  Small integers: exact in float32, then rounded once.
 @pytest.mark.parametrize("B,T,E,K,I,J", [(6, 100, 38, 101, 456, 192), (15, 100, 11, 32, 1032, 432), (11, 100, 52, 50, 400, 224), (7, 100, 56, 64, 704, 232),
                                          (11, 100, 15, 64, 912, 640), (11, 100, 33, 50, 424, 248), (9, 100, 48, 45, 816, 256), (20, 90, 40, 64, 512, 512)])
-def test_dense16_few_waves(cuda_device, B, T, E, K, I, J):
+def test_dense16_last_wave_in_half_tiles(cuda_device, B, T, E, K, I, J):
     plans = [ops.describe_plan(op, B, T, E, K, I, J, torch.bfloat16, w_layout=w) for op, w in (("G", "cn"), ("G", "nc"), ("D", "cn"))]
     assert any(p["pair"] and p["tile_n"] >= 128 for p in plans), plans
     g = torch.Generator().manual_seed(I)
@@ -347,7 +347,7 @@ def test_dense16_gather_tiles(cuda_device, B, T, E, K, C, N, pair, tile_n, w_lay
 @pytest.mark.parametrize("B,E,K,I,J,first", [(27, 10, 70, 648, 152, 96), (23, 11, 76, 392, 320, 96), (20, 10, 94, 584, 192, 96), (20, 9, 73, 592, 360, 96), (19, 10, 97, 400, 216, 128),
                                              (25, 9, 52, 424, 424, 128), (31, 10, 41, 400, 448, 128), (23, 10, 52, 392, 464, 128), (32, 9, 75, 400, 256, 128), (16, 11, 65, 416, 512, 128)])
 @pytest.mark.parametrize("dtype,bias", [(torch.bfloat16, False), (torch.float16, True)])
-def test_dense16_last_wave_in_half_tiles(cuda_device, B, E, K, I, J, first, dtype, bias):
+def test_dense16_gather_in_half_tiles(cuda_device, B, E, K, I, J, first, dtype, bias):
     T = 100
     g = torch.Generator().manual_seed(I)
     X, W = torch.randint(-2, 3, (B, T, I), generator=g).to(dtype), torch.randint(-1, 2, (E, I, J), generator=g).to(dtype)
@@ -378,9 +378,24 @@ def test_dense16_dweight_groups_share_the_ring(cuda_device, B, T, E, K, FG, FD, 
     if out_layout == "direct_rows":
         ref = ref.transpose(1, 2)
     d = [t.to(cuda_device) for t in (X, Y, Ind)]
-    got = [ops.dweight(*d, out_layout=out_layout) for _ in range(10)]
+    for _ in range(10):
+        got = ops.dweight(*d, out_layout=out_layout)
     ops.check_status()
-    ref = ref.to(torch.bfloat16).to(cuda_device)
+    assert torch.equal(got.cpu(), ref.to(torch.bfloat16))
+
+
+# ... all of many results, launched back to back
+@pytest.mark.parametrize("B,T,E,K,FG,FD", [(39, 80, 13, 21, 1936, 344), (15, 200, 74, 64, 512, 512)])
+def test_dense16_dweight_groups_share_the_ring_every_time(cuda_device, B, T, E, K, FG, FD):
+    assert ops.describe_plan("D", B, T, E, K, FG, FD, torch.bfloat16)["pair"] == 1
+    g = torch.Generator().manual_seed(FD)
+    X = torch.randint(-2, 3, (B, T, FG), generator=g).to(torch.bfloat16)
+    Y = torch.randint(-2, 3, (B, E, K, FD), generator=g).to(torch.bfloat16)
+    Ind = torch.randint(0, T, (B, E, K), generator=g)
+    ref = torch.from_numpy(orc.np_dweight(X, Y, Ind)).to(torch.bfloat16).to(cuda_device)
+    d = [t.to(cuda_device) for t in (X, Y, Ind)]
+    got = [ops.dweight(*d) for _ in range(10)]
+    ops.check_status()
     for x in got:
         assert torch.equal(x, ref)
 
