@@ -362,8 +362,8 @@ Tensor gemm_scatter(const Tensor& Y, const Tensor& W, const Tensor& Ind, int64_t
 
 // on_stream: where the kernels go.  The buffers belong to the current stream either way, and the other stream knows nothing of what the
 // current one does behind the fork: all that it writes is allocated before a temporary of a later operator could be freed and its block
-// handed out again, so work for it is issued right behind the fork.  The caller forks and joins the two, passes contiguous inputs, and keeps *shared_ws - the scratch, one buffer for the weight gradients of one pass, which run one
-// after the other and are of one size - until it has joined.
+// handed out again, so work for it is issued right behind the fork.  The caller forks and joins the two, passes contiguous inputs, and keeps
+// *shared_ws - the scratch, one buffer for the weight gradients of one pass, which run one after the other and are of one size - until it has joined.
 Tensor dweight_on(const Tensor& Xsrc, const Tensor& Ysrc, const Tensor& Ind, int out_layout, int precision, int path, const OptTensor& zeroed,
                   std::optional<cudaStream_t> on_stream, Tensor* shared_ws) {
   if (Xsrc.dim() != 3 || Ysrc.dim() != 4 || Ind.dim() != 3) value_error("expected Xsrc[B,T,FG], Ysrc[B,E,K,FD], Ind[B,E,K]");
@@ -506,11 +506,13 @@ bool worth_a_side_stream(const Tensor& slot_rows, const Tensor& W) {      // [B,
   return slots * W.numel() > (tensor ? kSmallTensorWork : kSmallGenericWork);
 }
 // Bias gradients of 16-bit tensors follow the weight gradient there: their row sums read memory under the end of the dX / dY kernel, whose last
-// wave leaves SMs free, where they stood alone behind it before.  Forward and backward in bf16 through both modules, on the main and on the helper
-// stream: 32 experts, 768 and 192 features 237 and 230 us, 64 experts, 512 and 64 431 and 407, 24 of ragged sizes 180 and 176, 16, 512 and 256 148.7
-// and 149; through the ExpertScatter alone, whose dY kernel may come first, 129 and 135, 246 and 244, 99 and 105.  Where there is no dX / dY
-// kernel the sum belongs on the main stream, beside the weight gradient (an ExpertGather alone 70.1 us, behind it on the helper stream 78.6).  The
-// float32 weight gradients take longer than the dX / dY kernels, and sums behind them 1-4 % of a large pass (1024 and 256 features 674 and 695 us).
+// wave leaves SMs free, where they stood alone behind it before.  Forward and backward in bf16 through both modules, ten processes each, with
+// both sums on the main and both on the helper stream: 32 experts, 768 and 192 features 238 and 231 us, 192 and 768 265 and 264, 64 of 1024 and 128
+// 262 and 254, 24 of ragged sizes 179.5 and 181; with the scatter's alone on the main stream 239, 263, 254 and 179, in one process of ten 226, 257, 250
+// and 174.  Through the ExpertScatter alone, whose dY kernel ends before the weight gradient, the main stream would be the better one: 129 and
+// 134, 115 and 123, 142 and 148.  Where there is no dX / dY kernel the sum belongs on the main stream, beside the weight gradient (an ExpertGather
+// alone 70.1 us, behind it on the helper stream 78.6).  The float32 weight gradients take longer than the dX / dY kernels, and sums behind them
+// 1-4 % of a large pass (1024 and 256 features 674 and 695 us).
 struct Grads {
   Tensor in, w, b;
 };
