@@ -193,12 +193,17 @@ def test_modules_forward_and_backward_in_a_cuda_graph(cuda_device, dtype):
 
 
 def test_block_backward_from_saved_tensors_that_are_not_contiguous(cuda_device):
-    """What saved-tensor hooks hand back may lie otherwise in memory: the helper stream reads a copy that is made before it is forked."""
+    """What saved-tensor hooks hand back may lie otherwise in memory: the helper stream reads a copy that is made before it is forked.  Small integers and
+    weights with one entry a row: sums in 16 bits are exact in any order."""
     B, T, E, K, I, J = 4, 128, 16, 64, 256, 128
-    g = torch.Generator(device=cuda_device).manual_seed(8)
-    rand = lambda *s: torch.randn(s, generator=g, device=cuda_device).bfloat16()
+    g = torch.Generator().manual_seed(8)
+    ints = lambda *s: torch.randint(-1, 2, s, generator=g).to(torch.bfloat16).to(cuda_device)
     m = egs.ExpertGatherScatter(E, I, J).to(cuda_device).to(torch.bfloat16)
-    X, G, Ind = rand(B, T, I), rand(B, T, I), torch.rand(B, E, T, generator=g, device=cuda_device).topk(K, -1).indices
+    X, G, Ind = ints(B, T, I), ints(B, T, I), torch.rand(B, E, T, generator=g).topk(K, -1).indices.to(cuda_device)
+    one = (torch.arange(I)[:, None] % J == torch.arange(J)[None]).to(cuda_device)
+    with torch.no_grad():
+        m.gather.W.copy_(ints(E, I, J) * one)
+        m.scatter.W.copy_(ints(E, J, I) * one.T)
 
     def grads():
         m.zero_grad()
@@ -208,8 +213,9 @@ def test_block_backward_from_saved_tensors_that_are_not_contiguous(cuda_device):
 
     plain = grads()
     with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t.transpose(-1, -2).contiguous().transpose(-1, -2)):
-        moved = grads()
+        moved = [grads() for _ in range(5)]
     ops.check_status()
-    assert orc.rel_err(moved[0].cpu(), plain[0].cpu()) <= 1e-2       # (16-bit additions in any order)
-    for a, b in zip(moved[1:], plain[1:]):
-        assert torch.equal(a, b)
+    assert all(t.any().item() for t in plain)
+    for got in moved:
+        for a, b in zip(got, plain):
+            assert torch.equal(a, b)
